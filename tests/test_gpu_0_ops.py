@@ -122,6 +122,22 @@ def test_linear_wide_tensor_core_tiles(epi):
         close(y, ref, TOL[dt] / 2)
 
 
+@pytest.mark.parametrize("shape", [(129, 257, 64, 257), (300, 71, 72, 75), (65, 4097, 128, 4097), (2500, 5121, 64, 5121)])
+def test_linear_output_rows_off_the_16_byte_grid(shape):
+    """Plain stores of the tcgen05 GEMM to rows of any stride (an odd vocabulary), square and wide tiles; nothing is
+    written between the rows."""
+    from flash_stu_2_b200 import ops
+    M, N, K, ld = shape
+    torch.manual_seed(6)
+    x, W = torch.randn(M, K).bfloat16(), (torch.randn(N, K) / math.sqrt(K)).bfloat16()
+    buf = torch.full((M * ld + 1,), 7.0, dtype=torch.bfloat16, device=dev())
+    y = buf[1:].view(M, ld)   # two bytes off the grid as well
+    ops.linear(x.to(dev()), W.to(dev()), out=y[:, :N], backend=2)
+    ops.check_status()
+    close(y[:, :N], _lin_ref(x, W, None, None, 0, torch.bfloat16), 1e-2)
+    assert bool((y[:, N:] == 7.0).all()) and float(buf[0]) == 7.0
+
+
 def test_bounded_wait_expiry_is_reported_and_the_context_survives():
     """Failure detection inside the tcgen05 GEMM: with the copies of its first pipeline stage dropped (test hook) the
     consumer's bounded wait runs out after the shortened limit; the kernel reports status 3, frees its tensor memory
