@@ -93,7 +93,7 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
       if (!tc_ok) return STU_ERR_UNSUPPORTED;
       return gemm_tc_dispatch(x, x_row_stride, W, w_row_stride, W2, M, N, K, epilogue, causal, ep, st);
     case BACKEND_SIMT:
-      return gemm_simt_dispatch(x, x_row_stride, W, w_row_stride, w_k_stride, W2, M, N, K, epilogue, ep, dtype, st);
+      return gemm_simt_dispatch(x, x_row_stride, W, w_row_stride, w_k_stride, W2, M, N, K, epilogue, causal, ep, dtype, st);
   }
   return STU_ERR_UNSUPPORTED;
 }

@@ -1,89 +1,250 @@
 // General tiled GEMM on CUDA cores with fp32 accumulation: the path for fp32 models (where the
 // 1e-3 / bit-exact-greedy bar rules out tf32 tensor cores) and for shapes the tcgen05 path does
 // not take (tiny K, unaligned strides).  y = epilogue(x @ W^T).
+//
+// Bound: FFMA issue (74 TFLOP/s), and before that the number of CTAs: the prefill linears of a 512-wide fp32 model are
+// 256 x 512 x 6144.  64 x 64 tiles of 128 threads (8 x 4 outputs each: three 16-byte shared-memory reads per 32 FMAs)
+// with K split over a thread-block cluster of up to 8 CTAs until there are about two per SM (the partial tiles meet in
+// distributed shared memory, summed in rank order), 128 x 128 tiles (8 x 8 outputs) where those alone fill the chip.
+// Operand tiles pass through registers into a double-buffered, k-major shared-memory tile.  256 x 512 x 6144:
+// 531 us with 64 x 64 tiles of 4 x 4 outputs, no split and no overlap.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "epilogue.cuh"
 
-template <typename T, int EPI>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const T* __restrict__ A, long long lda,
-                                                        const T* __restrict__ B, long long ldb, long long skb,
-                                                        const T* __restrict__ B2, int M, int N, int K,
-                                                        EpiArgs<T> ep) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
-  __shared__ float Bs2[EPI == EPI_GELU_MUL ? BK : 1][BN + 4];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tx = tid & 15, ty = tid >> 4;  // thread computes rows ty*4.., cols tx*4..
-  float acc[4][4] = {}, acc2[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    // 64x16 tile: 1024 elements, 4 per thread; consecutive threads walk k for coalescing
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      int e = tid + i * 256;
-      int r = e >> 4, kk = e & 15;
-      int m = m0 + r, k = k0 + kk;
-      As[kk][r] = (m < M && k < K) ? Elem<T>::to_f(A[(size_t)m * lda + k]) : 0.f;
-      int n = n0 + r;
-      bool ok = (n < N && k < K);
-      Bs[kk][r] = ok ? Elem<T>::to_f(B[(size_t)n * ldb + (size_t)k * skb]) : 0.f;
-      if (EPI == EPI_GELU_MUL) Bs2[kk][r] = ok ? Elem<T>::to_f(B2[(size_t)n * ldb + (size_t)k * skb]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; kk++) {
-      float a[4], b[4], b2[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-      if (EPI == EPI_GELU_MUL) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) b2[j] = Bs2[kk][tx * 4 + j];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-          if (EPI == EPI_GELU_MUL) acc2[i][j] = fmaf(a[i], b2[j], acc2[i][j]);
-        }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-      if (m < M && n < N) epilogue_store<T, EPI>(ep, m, n, acc[i][j], acc2[i][j]);
-    }
+int device_sm_count();   // gemm_tc.cu
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+constexpr int BK = 16;
+
+// Four consecutive k of one row as fp32; vec: 16-byte (fp32) / 8-byte (bf16) aligned and inside the row.
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
+  const uint2 t = *reinterpret_cast<const uint2*>(p);
+  v[0] = __uint_as_float(t.x << 16);
+  v[1] = __uint_as_float(t.x & 0xffff0000u);
+  v[2] = __uint_as_float(t.y << 16);
+  v[3] = __uint_as_float(t.y & 0xffff0000u);
 }
 
-template <typename T>
-static int launch_simt(const void* A, long long lda, const void* B, long long ldb, long long skb, const void* B2,
-                       int M, int N, int K, int epi, const EpiArgs<T>& ep, cudaStream_t st) {
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
-#define LAUNCH(E)                                                                                          \
-  gemm_simt_kernel<T, E><<<grid, 256, 0, st>>>((const T*)A, lda, (const T*)B, ldb, skb, (const T*)B2, M, N, \
-                                               K, ep)
-  switch (epi) {
-    case EPI_STORE: LAUNCH(EPI_STORE); break;
-    case EPI_RESID: LAUNCH(EPI_RESID); break;
-    case EPI_GELU_MUL: LAUNCH(EPI_GELU_MUL); break;
-    case EPI_HIST: LAUNCH(EPI_HIST); break;
-    case EPI_BLOCKCOL: LAUNCH(EPI_BLOCKCOL); break;
-    default: return STU_ERR_UNSUPPORTED;
+// TM x TN outputs per thread, 16 threads across the columns.  KS > 1: cluster of KS CTAs along z.
+template <typename T, int EPI, int BM, int BN, int TM, int TN, int KS>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+    gemm_simt_kernel(const T* __restrict__ A, long long lda, const T* __restrict__ B, long long ldb, long long skb,
+                     const T* __restrict__ B2, int M, int N, int K, int causal, int vec_a, int vec_b, EpiArgs<T> ep) {
+  constexpr bool DUAL = (EPI == EPI_GELU_MUL);
+  constexpr int THREADS = (BM / TM) * (BN / TN), NB = DUAL ? 2 : 1;
+  constexpr int QA = BM * BK / 4 / THREADS, QB = BN * BK / 4 / THREADS;   // quads of k per thread and tile
+  static_assert(BN / TN == 16 && QA >= 1 && QB >= 1, "thread layout");
+  constexpr int PA = BM + 4, PB = BN + 4;
+  constexpr int TILE = BK * (PA + NB * PB);
+  constexpr int PART = KS > 1 ? BM * BN * NB : 0;
+  __shared__ __align__(16) float sm[2 * TILE > PART ? 2 * TILE : PART];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  // lower-triangular blocks of `causal` rows of B: nothing beyond the tile's last column
+  int k_end = causal && n0 % causal + BN <= causal ? min(K, n0 % causal + BN) : K;
+
+  const int nkb = (k_end + BK - 1) / BK, per = (nkb + KS - 1) / KS;
+  const int kb0 = KS > 1 ? (int)blockIdx.z * per : 0, kb1 = KS > 1 ? min(nkb, kb0 + per) : nkb;
+
+  float ra[QA][4], rb[NB][QB][4];
+  auto fetch = [&](int kb) {
+    const int k0 = kb * BK;
+#pragma unroll
+    for (int i = 0; i < QA; i++) {
+      const int e = tid + i * THREADS, r = e >> 2, k = k0 + (e & 3) * 4, m = m0 + r;
+      const T* p = A + (size_t)m * lda + k;
+      if (m < M && vec_a && k + 4 <= K) {
+        load4(p, ra[i]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) ra[i][j] = (m < M && k + j < K) ? Elem<T>::to_f(p[j]) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+#pragma unroll
+      for (int i = 0; i < QB; i++) {
+        const int e = tid + i * THREADS, r = e >> 2, k = k0 + (e & 3) * 4, n = n0 + r;
+        const T* p = (b ? B2 : B) + (size_t)n * ldb + (size_t)k * skb;
+        if (n < N && vec_b && k + 4 <= K) {
+          load4(p, rb[b][i]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) rb[b][i][j] = (n < N && k + j < K) ? Elem<T>::to_f(p[(size_t)j * skb]) : 0.f;
+        }
+      }
+  };
+  auto stage = [&](int buf) {
+    float* a = sm + buf * TILE;
+#pragma unroll
+    for (int i = 0; i < QA; i++) {
+      const int e = tid + i * THREADS, r = e >> 2, k = (e & 3) * 4;
+#pragma unroll
+      for (int j = 0; j < 4; j++) a[(k + j) * PA + r] = ra[i][j];
+    }
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+      float* bs = a + BK * PA + b * BK * PB;
+#pragma unroll
+      for (int i = 0; i < QB; i++) {
+        const int e = tid + i * THREADS, r = e >> 2, k = (e & 3) * 4;
+#pragma unroll
+        for (int j = 0; j < 4; j++) bs[(k + j) * PB + r] = rb[b][i][j];
+      }
+    }
+  };
+
+  float acc[NB][TM][TN];
+#pragma unroll
+  for (int b = 0; b < NB; b++)
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < TN; j++) acc[b][i][j] = 0.f;
+
+  if (kb0 < kb1) {
+    fetch(kb0);
+    stage(0);
   }
-#undef LAUNCH
+  __syncthreads();
+  for (int kb = kb0; kb < kb1; kb++) {
+    const int buf = (kb - kb0) & 1;
+    if (kb + 1 < kb1) fetch(kb + 1);   // in flight during the products below
+    const float* a = sm + buf * TILE + ty * TM;
+    const float* bs = sm + buf * TILE + BK * PA + tx * TN;
+#pragma unroll
+    for (int kk = 0; kk < BK; kk++) {
+      float av[TM], bv[NB][TN];
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4*>(av + i) = *reinterpret_cast<const float4*>(a + kk * PA + i);
+#pragma unroll
+      for (int b = 0; b < NB; b++)
+#pragma unroll
+        for (int j = 0; j < TN; j += 4)
+          *reinterpret_cast<float4*>(bv[b] + j) = *reinterpret_cast<const float4*>(bs + b * BK * PB + kk * PB + j);
+#pragma unroll
+      for (int b = 0; b < NB; b++)
+#pragma unroll
+        for (int i = 0; i < TM; i++)
+#pragma unroll
+          for (int j = 0; j < TN; j++) acc[b][i][j] = fmaf(av[i], bv[b][j], acc[b][i][j]);
+    }
+    if (kb + 1 < kb1) stage(buf ^ 1);   // the other buffer was last read before the barrier of the step before
+    __syncthreads();
+  }
+
+  if constexpr (KS == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < TN; j++) {
+        const int m = m0 + ty * TM + i, n = n0 + tx * TN + j;
+        if (m < M && n < N) epilogue_store<T, EPI>(ep, m, n, acc[0][i][j], DUAL ? acc[NB - 1][i][j] : 0.f);
+      }
+  } else {
+    cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j += 4)
+          *reinterpret_cast<float4*>(sm + (b * BM + ty * TM + i) * BN + tx * TN + j) =
+              make_float4(acc[b][i][j], acc[b][i][j + 1], acc[b][i][j + 2], acc[b][i][j + 3]);
+    cluster.sync();   // every partial tile is complete
+    const int rank = (int)cluster.block_rank();
+    const float* part[KS];
+#pragma unroll
+    for (int r = 0; r < KS; r++) part[r] = cluster.map_shared_rank(sm, r);
+    for (int e = tid; e < BM / KS * BN; e += THREADS) {   // every CTA finishes its share of the rows
+      const int row = rank + (e / BN) * KS, col = e % BN, m = m0 + row, n = n0 + col;
+      float s = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int r = 0; r < KS; r++) {
+        s += part[r][row * BN + col];
+        if (DUAL) s2 += part[r][(BM + row) * BN + col];
+      }
+      if (m < M && n < N) epilogue_store<T, EPI>(ep, m, n, s, s2);
+    }
+    cluster.sync();   // the other CTAs' tiles stay alive until read
+  }
+}
+
+struct Operands {
+  const void *A, *B, *B2;
+  long long lda, ldb, skb;
+  int M, N, K, causal, vec_a, vec_b;
+};
+
+template <typename T, int EPI, int BM, int BN, int TM, int TN, int KS>
+int launch_tile(const Operands& o, const EpiArgs<T>& ep, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((o.N + BN - 1) / BN, (o.M + BM - 1) / BM, KS);
+  cfg.blockDim = dim3((BM / TM) * (BN / TN));
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = KS;
+  cfg.attrs = at;
+  cfg.numAttrs = KS > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_simt_kernel<T, EPI, BM, BN, TM, TN, KS>, (const T*)o.A, o.lda,
+                                           (const T*)o.B, o.ldb, o.skb, (const T*)o.B2, o.M, o.N, o.K, o.causal, o.vec_a,
+                                           o.vec_b, ep);
+  if (e != cudaSuccess) return (int)e;
   STU_CHECK_LAUNCH();
   return STU_OK;
 }
 
+template <typename T, int EPI>
+int launch_simt(const Operands& o, const EpiArgs<T>& ep, cudaStream_t st) {
+  const long long sms = device_sm_count();
+  auto tiles = [&](int t) { return (long long)((o.M + t - 1) / t) * ((o.N + t - 1) / t); };
+  if constexpr (EPI != EPI_GELU_MUL) {
+    if (tiles(128) >= 2 * sms) return launch_tile<T, EPI, 128, 128, 8, 8, 1>(o, ep, st);
+  }
+  // split K while there are fewer than two CTAs per SM and every CTA keeps 64 of K
+  int ks = 1;
+  while (ks < 8 && tiles(64) * ks < 2 * sms && o.K / (2 * ks) >= 64) ks *= 2;
+  switch (ks) {
+    case 1: return launch_tile<T, EPI, 64, 64, 8, 4, 1>(o, ep, st);
+    case 2: return launch_tile<T, EPI, 64, 64, 8, 4, 2>(o, ep, st);
+    case 4: return launch_tile<T, EPI, 64, 64, 8, 4, 4>(o, ep, st);
+    default: return launch_tile<T, EPI, 64, 64, 8, 4, 8>(o, ep, st);
+  }
+}
+
+template <typename T>
+int launch_epi(const Operands& o, int epi, const EpiArgs<T>& ep, cudaStream_t st) {
+  switch (epi) {
+    case EPI_STORE: return launch_simt<T, EPI_STORE>(o, ep, st);
+    case EPI_RESID: return launch_simt<T, EPI_RESID>(o, ep, st);
+    case EPI_GELU_MUL: return launch_simt<T, EPI_GELU_MUL>(o, ep, st);
+    case EPI_HIST: return launch_simt<T, EPI_HIST>(o, ep, st);
+    case EPI_BLOCKCOL: return launch_simt<T, EPI_BLOCKCOL>(o, ep, st);
+  }
+  return STU_ERR_UNSUPPORTED;
+}
+
+}  // namespace
+
 int gemm_simt_dispatch(const void* A, long long lda, const void* B, long long ldb, long long skb, const void* B2,
-                       int M, int N, int K, int epi, const EpiArgsAny& ep, int dtype, cudaStream_t st) {
-  if (dtype == STU_F32) return launch_simt<float>(A, lda, B, ldb, skb, B2, M, N, K, epi, ep.as<float>(), st);
-  if (dtype == STU_BF16) return launch_simt<bf16>(A, lda, B, ldb, skb, B2, M, N, K, epi, ep.as<bf16>(), st);
+                       int M, int N, int K, int epi, int causal, const EpiArgsAny& ep, int dtype, cudaStream_t st) {
+  const uintptr_t quad = dtype == STU_F32 ? 15 : 7;   // bytes of four elements, less one
+  const bool vec_a = lda % 4 == 0 && !((uintptr_t)A & quad);
+  const bool vec_b = skb == 1 && ldb % 4 == 0 && !((uintptr_t)B & quad) && !((uintptr_t)B2 & quad);
+  const Operands o{A, B, B2, lda, ldb, skb, M, N, K, causal, vec_a, vec_b};
+  if (dtype == STU_F32) return launch_epi<float>(o, epi, ep.as<float>(), st);
+  if (dtype == STU_BF16) return launch_epi<bf16>(o, epi, ep.as<bf16>(), st);
   return STU_ERR_DTYPE;
 }

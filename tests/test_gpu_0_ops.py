@@ -122,6 +122,27 @@ def test_linear_wide_tensor_core_tiles(epi):
         close(y, ref, TOL[dt] / 2)
 
 
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(65, 64, 24, 0), (200, 65, 70, 2), (256, 512, 6144, 1), (300, 130, 264, 2), (64, 700, 3000, 0),
+                                   (2500, 2500, 40, 0), (100, 333, 1027, 1)])
+def test_linear_cuda_core_tiles(dt, shape):
+    """The CUDA-core GEMM at the edges of its tiles (64 and 128), K split over clusters of 1 to 8 CTAs, ragged K and rows off
+    the 16-byte grid; lower-triangular weights with the blocks above the diagonal skipped."""
+    from flash_stu_2_b200 import ops
+    M, N, K, epi = shape
+    torch.manual_seed(7)
+    x, W, W2 = torch.randn(M, K).to(dt), (torch.randn(N, K) / math.sqrt(K)).to(dt), (torch.randn(N, K) / math.sqrt(K)).to(dt)
+    resid = torch.randn(M, N).to(dt)
+    y = ops.linear(x.to(dev()), W.to(dev()), W2=W2.to(dev()) if epi == 2 else None,
+                   resid=resid.to(dev()) if epi == 1 else None, epilogue=epi, backend=1)
+    close(y, _lin_ref(x, W, W2, resid, epi, dt), TOL[dt] / 2)
+    if epi == 0:
+        Wl = torch.tril(W)
+        y = ops.linear(x.to(dev()), Wl.to(dev()), epilogue=ops.EPI_STORE | ops.EPI_FLAG_CAUSAL, backend=1)
+        close(y, _lin_ref(x, Wl, None, None, 0, dt), TOL[dt] / 2)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("shape", [(129, 257, 64, 257), (300, 71, 72, 75), (65, 4097, 128, 4097), (2500, 5121, 64, 5121)])
 def test_linear_output_rows_off_the_16_byte_grid(shape):
     """Plain stores of the tcgen05 GEMM to rows of any stride (an odd vocabulary), square and wide tiles; nothing is
