@@ -69,7 +69,8 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
 
   bool sk_ok = skinny_supported(x, x_row_stride, W, w_row_stride, w_k_stride, W2, M, N, K, epilogue, dtype);
   if (norm_w) {
-    if (!sk_ok || dtype != STU_BF16 || (backend != BACKEND_AUTO && backend != BACKEND_SKINNY))
+    // fp32: up to 8 rows (the kernel of stream.cu)
+    if (!sk_ok || (dtype != STU_BF16 && M > 8) || !aligned16(norm_w) || (backend != BACKEND_AUTO && backend != BACKEND_SKINNY))
       return STU_ERR_UNSUPPORTED;
     return skinny_dispatch(x, x_row_stride, W, w_row_stride, W2, M, N, K, epilogue, ep, norm_w, eps, dtype, pdl, st);
   }
@@ -120,7 +121,8 @@ extern "C" int stu_linear_push(const void* x, long long x_row_stride, const void
                          (cudaStream_t)stream);
 }
 
-// 1 when stu_linear would fuse the RMSNorm for this shape (decode path), else 0.
+// 1 when stu_linear would fuse the RMSNorm for this bf16 shape (decode path), else 0.  (fp32: stu_linear takes norm_w
+// up to 8 rows.)
 extern "C" int stu_linear_can_fuse_norm(int M, int N, int K, int epilogue, int dtype) {
   if (dtype != STU_BF16 || M < 1 || M > 64 || K % 8 || epilogue == EPI_HIST) return 0;
   if (prefers_tensor_gemm(M, N)) return 0;   // a separate norm kernel + the tcgen05 GEMM is faster there

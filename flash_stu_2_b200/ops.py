@@ -138,8 +138,9 @@ def embed(ids: torch.Tensor, table: torch.Tensor):
 
 
 def can_fuse_norm(M: int, N: int, K: int, epilogue: int, dtype: torch.dtype) -> bool:
-    code = 1 if dtype == torch.bfloat16 else 0
-    return bool(_lib.load().stu_linear_can_fuse_norm(M, N, K, epilogue, code))
+    if dtype == torch.float32:
+        return M <= 8 and K % 4 == 0 and epilogue in (EPI_STORE, EPI_RESID, EPI_GELU_MUL)
+    return bool(_lib.load().stu_linear_can_fuse_norm(M, N, K, epilogue, 1))
 
 
 def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = None,
