@@ -24,6 +24,24 @@ _lib = None
 
 _P = c_void_p
 _LL = c_longlong
+
+
+class StepLayer(ctypes.Structure):
+    """StuStepLayer of include/stu_b200.h."""
+    _fields_ = ([(n, c_int) for n in ("kind", "Lh", "W")] + [("eps1", c_float), ("eps2", c_float), ("reserved", c_int)]
+                + [(n, _P) for n in ("norm1", "w1", "wo", "norm2", "wg", "wu", "wd", "hist", "taps", "k_ring", "v_ring",
+                                     "slopes", "pos")])
+
+
+class StepArgs(ctypes.Structure):
+    """StuStepArgs of include/stu_b200.h."""
+    _fields_ = ([(n, c_int) for n in ("n_layers", "B", "d", "I", "H", "window", "V")]
+                + [("softcap", c_float), ("eps_final", c_float), ("reserved", c_int), ("ids", _P), ("ids_stride", _LL),
+                   ("embedding", _P), ("x", _P), ("norm_final", _P), ("lm_head", _P), ("logits", _P),
+                   ("ld_logits", _LL), ("workspace", _P), ("workspace_bytes", _LL), ("status", _P)])
+
+
+STEP_MAX_LAYERS = 40
 _SIGNATURES = {
     "stu_b200_version": ([], c_int),
     "stu_set_status_word": ([_P], c_int),
@@ -53,6 +71,11 @@ _SIGNATURES = {
     "stu_block_step_workspace_bytes": ([c_int, c_int], c_longlong),
     "stu_block_decode_step": ([_P, _LL, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _LL, c_int, c_int, c_int, c_int, c_float,
                                c_float, _P, _LL, c_int, _P, c_int, _P], c_int),
+    "stu_token_step_workspace_bytes": ([c_int, c_int, c_int, c_int], c_longlong),
+    "stu_token_step_supported": ([c_int, c_int, c_int, c_int, c_int, c_int], c_int),
+    "stu_token_step_plan_bytes": ([c_int], c_longlong),
+    "stu_token_step_plan": ([_P, _P, c_int, _P], c_int),
+    "stu_token_step": ([_P, c_int, _P, c_int, _P], c_int),
     "stu_to_history": ([_P, _LL, _LL, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_toeplitz": ([_P, _LL, c_int, _P, c_int, _LL, c_int, _P], c_int),
     "stu_full_combine": ([_P, _P, _LL, _P, _LL, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),

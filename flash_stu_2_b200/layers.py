@@ -85,7 +85,7 @@ class STULayer(nn.Module):
             if t + 1 > self.stu.capacity:
                 raise ValueError(f"sequence position {t + 1} exceeds the capacity {self.stu.capacity}")
             xp = ops.linear(h, self.stu.prepared()[0])
-            y = torch.empty(B, Hs, dtype=xc.dtype, device=xc.device)
+            y = ops.empty((B, Hs), xc.dtype, xc.device)
             ops.decode_approx_projected(None, xp, hist, taps8, pos, y, add_residual=False)
             pos._host_t = t + 1
         else:

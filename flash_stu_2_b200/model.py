@@ -8,6 +8,7 @@ can observe, all forced by the reference's own gaps:
   * sampling draws by inverse CDF from one uniform per sequence (optionally passed as
     `uniforms=[steps,B]` or drawn from `generator=`) instead of torch.multinomial.
 """
+import gc
 from typing import Any, Dict, Optional, Tuple
 
 import torch
@@ -21,6 +22,7 @@ from .config import FlashSTUConfig
 from .filters import get_spectral_filters, nearest_power_of_two
 from .layers import AttentionLayer, STULayer
 from .modules import STU, Attention, RMSNorm
+from .token_step import TokenStep
 
 
 class FlashSTU(PreTrainedModel):
@@ -151,9 +153,11 @@ class FlashSTU(PreTrainedModel):
         # logits rows padded to a multiple of 8 elements: the tensor-core GEMM needs 16-byte aligned output rows
         # and the vocabulary (50257) is odd
         Vp = (V + 7) // 8 * 8
-        logits = torch.empty(B, Vp, dtype=last.dtype, device=last.device)[:, :V]
+        logits = ops.empty((B, Vp), last.dtype, last.device)[:, :V]
         if ops.can_fuse_norm(B, V, last.shape[1], ops.EPI_STORE, last.dtype) and last.stride(1) == 1:
-            ops.linear(last, self.lm_head.weight, out=logits, norm_w=self.norm.weight, eps=self.norm.eps)
+            ov = ops.FLAG_OVERLAP if (x.shape[1] == 1 and ops.overlap_decode) else 0   # token step: weights fetched early
+            ops.linear(last, self.lm_head.weight, out=logits, norm_w=self.norm.weight, eps=self.norm.eps,
+                       epilogue=ops.EPI_STORE | ov)
         else:
             ops.linear(ops.rmsnorm(last.contiguous(), self.norm.weight, self.norm.eps), self.lm_head.weight, out=logits)
         return logits, cache
@@ -203,7 +207,8 @@ class FlashSTU(PreTrainedModel):
         # position from device memory): the step is ~100 small launches for a 24-layer model, which the interpreter
         # cannot issue as fast as the GPU retires them.  cuda_graph=False keeps the eager loop.
         capacity = min(self.config.seq_len, getattr(self.config, "cache_len", None) or self.config.seq_len)
-        use_graph = bool(kwargs.get("cuda_graph", True)) and use_cache and steps > 3 and max_length - 1 <= capacity
+        fits = use_cache and max_length - 1 <= capacity
+        use_graph = bool(kwargs.get("cuda_graph", True)) and fits and steps > 3
         # a sandwich layer's token step reads its position on the device only in the bf16 approx form
         for layer in self.layers:
             if getattr(layer, "stu_mlp_enabled", False) and not (
@@ -213,31 +218,40 @@ class FlashSTU(PreTrainedModel):
             if hasattr(layer, "stu") and layer.stu.use_approx and layer.stu.use_hankel_L:
                 use_graph = False   # the single-branch token step is a one-position prefill (host position)
         graph = None
+        stepper = None   # the persistent token-step kernel: small batches of layers that it computes
         for step in range(steps):
             cur = T0 + step
             u = None
             if do_sample:
                 u = uniforms[step].to(device=dev, dtype=torch.float32).contiguous() if uniforms is not None else \
                     torch.rand(B, device=dev, generator=generator)
-            if use_graph and past is not None and step >= 2:
-                if graph is None:
-                    tok_in = torch.empty(B, 1, dtype=torch.int64, device=dev)
-                    tok_out = torch.empty(B, 1, dtype=torch.int64, device=dev)
-                    u_buf = torch.zeros(B, dtype=torch.float32, device=dev)
-                    host_t = [getattr(e[-1], "_host_t", None) if e is not None else None for e in past]
-                    torch.cuda.synchronize(dev)
-                    graph = torch.cuda.CUDAGraph()
-                    with torch.cuda.graph(graph):
-                        logits_g, _ = self.last_logits(tok_in, past, True)
-                        ops.sample(logits_g, temperature, top_k, top_p, do_sample, u_buf if do_sample else None, tok_out,
-                                   out_stride=1)
-                    for e, t in zip(past, host_t):   # capturing ran the host bookkeeping, not the kernels
-                        if e is not None and t is not None:
-                            e[-1]._host_t = t
+            if step == 1 and fits and TokenStep.supported(self.layers, past, B, self.config.n_embd, self.config.torch_dtype):
+                x = torch.empty(B, self.config.n_embd, dtype=self.config.torch_dtype, device=dev)
+                stepper = TokenStep(self.layers, past, B, x, model=self)
+                V = self.lm_head.weight.shape[0]
+                if return_logits:   # the kernel writes every step's logits where the caller gets them
+                    first, all_logits = all_logits[0], torch.empty(B, steps, V, dtype=x.dtype, device=dev)
+                    all_logits[:, 0] = first
+                else:
+                    logits = torch.empty(B, V, dtype=x.dtype, device=dev)
+            if stepper is not None:
                 if timings is not None and ev_first is None:
                     ev_first = torch.cuda.Event(enable_timing=True)
                     ev_first.record()
-                tok_in.copy_(generated[:, cur - 1:cur])
+                if return_logits:
+                    logits = all_logits[:, step]
+                stepper.run(generated[:, cur - 1], logits)
+                ops.sample(logits, temperature, top_k, top_p, do_sample, u, generated[:, cur:], out_stride=max_length)
+                replayed += 1
+                continue
+            if use_graph and past is not None and step >= 2:
+                if graph is None:
+                    tok = generated[:, cur - 1:cur].clone()   # the step reads its token here and leaves the next one
+                    u_buf = torch.zeros(B, dtype=torch.float32, device=dev)
+                    graph, logits_g, buffers = self._capture_step(tok, past, temperature, top_k, top_p, do_sample, u_buf)
+                if timings is not None and ev_first is None:
+                    ev_first = torch.cuda.Event(enable_timing=True)
+                    ev_first.record()
                 if do_sample:
                     u_buf.copy_(u)
                 graph.replay()
@@ -245,7 +259,7 @@ class FlashSTU(PreTrainedModel):
                 for e in past:
                     if e is not None and getattr(e[-1], "_host_t", None) is not None:
                         e[-1]._host_t += 1
-                generated[:, cur:cur + 1].copy_(tok_out)
+                generated[:, cur:cur + 1].copy_(tok)
                 if return_logits:
                     all_logits.append(logits_g.clone())
                 continue
@@ -265,8 +279,40 @@ class FlashSTU(PreTrainedModel):
             timings["replayed_steps"] = replayed
             timings["replay_ms"] = ev_first.elapsed_time(ev_last)
         if return_logits:
-            return generated, torch.stack(all_logits, dim=1)
+            return generated, all_logits if stepper is not None else torch.stack(all_logits, dim=1)
         return generated
+
+    def _capture_step(self, tok, past, temperature, top_k, top_p, do_sample, u_buf):
+        """One cached token step (token in `tok`, next token left there) as a CUDA graph.  The step's outputs live in one
+        buffer of the caller, so that capturing needs neither a private memory pool nor the collection and cache flush
+        that go with one (together 0.1 to 0.8 s on a busy process)."""
+        B, d = tok.shape[0], self.config.n_embd
+        row = max(3 * d, d + max(layer.mlp.intermediate_size for layer in self.layers))
+        nbytes = (B * (6 * d + 2 * row) * (self.n_layers + 1) + B * (self.lm_head.weight.shape[0] + 64)) \
+            * self.lm_head.weight.element_size() + 4096 * (self.n_layers + 1)
+        buffer = torch.empty(nbytes, dtype=torch.uint8, device=tok.device)
+        host_t = [getattr(e[-1], "_host_t", None) if e is not None else None for e in past]
+        graph = torch.cuda.CUDAGraph()
+        stream, here = torch.cuda.Stream(tok.device), torch.cuda.current_stream(tok.device)
+        stream.wait_stream(here)
+        collecting = gc.isenabled()
+        gc.disable()   # a collection inside the capture could release objects whose destructors may not be captured
+        try:
+            with torch.cuda.stream(stream), ops.arena(buffer):
+                graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    logits, _ = self.last_logits(tok, past, True)
+                    ops.sample(logits, temperature, top_k, top_p, do_sample, u_buf if do_sample else None, tok, out_stride=1)
+                finally:
+                    graph.capture_end()
+        finally:
+            if collecting:
+                gc.enable()
+        here.wait_stream(stream)
+        for e, t in zip(past, host_t):   # capturing ran the host bookkeeping, not the kernels
+            if e is not None and t is not None:
+                e[-1]._host_t = t
+        return graph, logits, (buffer, stream)
 
     def prepare_inputs_for_generation(self, input_ids, past_key_values=None, attention_mask=None, use_cache=None,
                                       **kwargs) -> Dict[str, Any]:

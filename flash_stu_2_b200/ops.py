@@ -4,6 +4,9 @@ Every function takes CUDA tensors, launches on torch's current stream and return
 synchronising.  Device-side problems (bounded waits that ran out, out-of-range token ids or
 positions) are recorded in a per-process status word; `check_status()` reads it (one sync).
 """
+import ctypes
+import math
+import threading
 from typing import Optional
 
 import torch
@@ -83,7 +86,8 @@ STATUS_TEXT = {1: "token id outside the vocabulary", 2: "position outside the ca
                8: "the fused token-step kernel found no partial sums for the current position in its workspace",
                9: "a bounded pipeline wait ran out inside the tcgen05 prefill convolution",
                10: "a tensor-parallel rank waited in vain for another rank's sub-layer output",
-               11: "tcgen05 attention prefill: a bounded wait ran out, or a sequence was not at position 0"}
+               11: "tcgen05 attention prefill: a bounded wait ran out, or a sequence was not at position 0",
+               12: "a bounded grid-barrier wait ran out inside the token-step kernel"}
 
 
 def check_status(device=None):
@@ -96,13 +100,49 @@ def check_status(device=None):
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = RMS_EPS, out: Optional[torch.Tensor] = None):
+_local = threading.local()   # .arena: where this thread's outputs come from while an `arena` block is open
+
+
+class arena:
+    """Outputs of the ops called by this thread inside the block are consecutive pieces of `buffer` (a CUDA uint8
+    tensor) instead of allocations of their own: a captured step then owns its memory like any other tensor of the
+    caller, and capturing touches no allocator.  What does not fit is allocated as usual."""
+
+    def __init__(self, buffer: torch.Tensor):
+        self.buffer, self.used = buffer, 0
+
+    def __enter__(self):
+        self.outer, _local.arena = getattr(_local, "arena", None), self
+        return self
+
+    def __exit__(self, *exc):
+        _local.arena = self.outer
+
+    def take(self, shape, dtype):
+        n = math.prod(shape) * dtype.itemsize
+        if self.used + n > self.buffer.numel():
+            return None
+        piece = self.buffer[self.used:self.used + n].view(dtype).view(shape)
+        self.used += (n + 255) // 256 * 256
+        return piece
+
+
+def empty(shape, dtype: torch.dtype, device) -> torch.Tensor:
+    a = getattr(_local, "arena", None)
+    if a is not None:
+        t = a.take(shape, dtype)
+        if t is not None:
+            return t
+    return torch.empty(shape, dtype=dtype, device=device)
+
+
     _cuda(x, weight)
     d = x.shape[-1]
     x2 = x.reshape(-1, d)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     if out is None:
-        out = torch.empty(x2.shape, dtype=x.dtype, device=x.device)
+        out = empty(x2.shape, x.dtype, x.device)
     o2 = out.reshape(-1, d)
     rc = _lib.load().stu_rmsnorm(x2.data_ptr(), weight.data_ptr(), o2.data_ptr(), x2.shape[0], d, x2.stride(0),
                                  o2.stride(0), eps, _dt(x), _stream())
@@ -129,7 +169,7 @@ def bias_act(y: torch.Tensor, bias: Optional[torch.Tensor], act: int = ACT_NONE)
 def embed(ids: torch.Tensor, table: torch.Tensor):
     _cuda(ids, table)
     ids = ids.contiguous().to(torch.int64)
-    out = torch.empty(*ids.shape, table.shape[1], dtype=table.dtype, device=table.device)
+    out = empty((*ids.shape, table.shape[1]), table.dtype, table.device)
     rc = _lib.load().stu_embed(ids.data_ptr(), table.data_ptr(), out.data_ptr(), ids.numel(), table.shape[1],
                                table.shape[0], status_word(table.device).data_ptr(), _dt(table), _stream())
     _lib.check(rc, "stu_embed")
@@ -164,7 +204,7 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
         y_rs = 0
     else:
         if out is None:
-            out = torch.empty(M, N, dtype=x.dtype, device=x.device)
+            out = empty((M, N), x.dtype, x.device)
         assert out.shape == (M, N) and out.stride(1) == 1
         y_rs = out.stride(0)
     r_rs = 0
@@ -429,6 +469,14 @@ def to_history(x, hist, t0: int):
     """x [B,T,d] -> hist[b][c][t&1][t>>1] for t in [t0, t0+T)."""
     _cuda(x, hist)
     B, T, d = x.shape
+def token_step(plan: torch.Tensor, n_stages: int, args, bf16: bool):
+    """One token step of a stack of layers in one persistent kernel; plan: the device copy of stu_token_step_plan's
+    table, args a _lib.StepArgs whose tensors the caller keeps alive."""
+    rc = _lib.load().stu_token_step(plan.data_ptr(), n_stages, ctypes.addressof(args), int(bf16), _stream())
+    _lib.check(rc, "stu_token_step")
+    _count()
+
+
     assert hist.is_contiguous() and hist.shape[:3] == (B, d, 2) and x.stride(2) == 1
     rc = _lib.load().stu_to_history(x.data_ptr(), x.stride(0), x.stride(1), hist.data_ptr(), B, d, hist.shape[3], t0,
                                     t0 + T, _dt(x), _stream())
@@ -570,7 +618,7 @@ def swa_prefill_tc5(qkv, k_ring, v_ring, pos, slopes, H: int, window: int, softc
     assert not update_cache or (k_ring.shape == (B, W, d) and k_ring.is_contiguous() and v_ring.is_contiguous())
     lib = _lib.load()
     vt = torch.empty(lib.stu_swa_prefill_scratch_elems(B, Tn, H, 128), dtype=qkv.dtype, device=qkv.device)
-    out = torch.empty(B, Tn, d, dtype=qkv.dtype, device=qkv.device)
+    out = empty((B, Tn, d), qkv.dtype, qkv.device)
     rc = lib.stu_swa_prefill_tc5(qkv.data_ptr(), vt.data_ptr(), k_ring.data_ptr(), v_ring.data_ptr(), pos.data_ptr(),
                                  slopes.data_ptr(), out.data_ptr(), B, Tn, H, 128, W, window, float(softcap or 0.0),
                                  int(update_cache), status_word(qkv.device).data_ptr(), _dt(qkv), _stream())

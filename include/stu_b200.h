@@ -353,3 +353,59 @@ int stu_peer_exchange(const void* xchg, void* x, long long x_row_stride, const v
 }
 #endif
 #endif /* STU_B200_H */
+/* One token step of a stack of layers -- approx STU layers (flash_stu/layers/stu_layer.py:78-97) and sliding-window
+ * attention layers (flash_stu/layers/attention_layer.py:50-66) in any order, each with its MLP -- as ONE persistent
+ * cooperative kernel for up to 8 sequences at one common position: x = layers(x) in place, or, with `ids`, from the
+ * token ids, and with `lm_head` to the logits of the final norm (flash_stu/model.py:150-205).  Appends to every layer's
+ * cache and advances its positions.  All layers share d, I, and the attention layers H and window.  Status 6 when the
+ * cached positions differ, 2 beyond a history, 1 for an id outside the vocabulary, 12 when a grid barrier ran out. */
+#define STU_STEP_MAX_LAYERS 40
+#define STU_STEP_STU 0
+#define STU_STEP_ATTENTION 1
+
+typedef struct {
+  int kind;            /* STU_STEP_STU or STU_STEP_ATTENTION */
+  int Lh;              /* STU: positions per parity row of the history */
+  int W;               /* attention: slots of the key / value rings */
+  float eps1, eps2;    /* of the two norms */
+  int reserved;
+  const void* norm1;   /* [d] */
+  const void* w1;      /* STU: M_inputs^T [d][d]; attention: c_attn [3d][d] */
+  const void* wo;      /* attention: c_proj [d][d] */
+  const void* norm2;   /* [d] */
+  const void* wg;      /* [I][d] */
+  const void* wu;      /* [I][d] */
+  const void* wd;      /* [d][I] */
+  void* hist;          /* STU: [B][d][2][Lh] */
+  const void* taps;    /* STU: fp32 [d][Lh]; bf16 the reversed tables [8][d][Lh + 8] */
+  void* k_ring;        /* attention: [B][W][d] */
+  void* v_ring;
+  const float* slopes; /* attention: [H] */
+  int* pos;            /* [B][2] */
+} StuStepLayer;
+
+typedef struct {
+  int n_layers, B, d, I, H, window, V;
+  float softcap, eps_final;
+  int reserved;
+  const long long* ids; /* token of sequence b at ids[b * ids_stride], or NULL: x holds the input rows */
+  long long ids_stride;
+  const void* embedding; /* [V][d] */
+  void* x;               /* [B][d] residual stream, input (ids NULL) and output */
+  const void* norm_final; /* with lm_head */
+  const void* lm_head;    /* [V][d], or NULL: stop after the last layer */
+  void* logits;           /* [B] rows of V */
+  long long ld_logits;
+  void* workspace;        /* stu_token_step_workspace_bytes, 256-byte aligned, zeroed once */
+  long long workspace_bytes;
+  int* status;
+} StuStepArgs;
+
+long long stu_token_step_workspace_bytes(int d, int I, int H, int dtype);
+int stu_token_step_supported(int n_layers, int B, int d, int I, int H, int dtype);   /* 1: stu_token_step takes it */
+/* The plan (stu_token_step_plan_bytes bytes of HOST memory): checks the descriptors; returns the number of stages or an
+ * error (< 0).  The caller copies it to the device once; it holds addresses, so it serves as long as they do. */
+long long stu_token_step_plan_bytes(int n_layers);
+int stu_token_step_plan(const StuStepLayer* layers, const StuStepArgs* args, int dtype, void* plan);
+int stu_token_step(const void* plan_on_device, int n_stages, const StuStepArgs* args, int dtype, void* stream);
+

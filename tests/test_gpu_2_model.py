@@ -153,6 +153,36 @@ def test_graph_replayed_token_loop_equals_eager_loop(golden, tmp_path, name):
         assert torch.equal(la, lb)
 
 
+@pytest.mark.parametrize("dt,B,d,heads,mlp,window,T0", [
+    (torch.float32, 1, 48, 3, 4, 20, 9), (torch.float32, 2, 256, 4, 12, 64, 70), (torch.float32, 4, 772, 0, 3, 1, 33),
+    (torch.float32, 7, 512, 8, 1, 100, 130), (torch.bfloat16, 1, 1536, 12, 4, 90, 129), (torch.bfloat16, 2, 96, 3, 5, 7, 40),
+    (torch.bfloat16, 8, 1024, 16, 4, 300, 200), (torch.bfloat16, 3, 2048, 16, 1, 16, 35), (torch.bfloat16, 5, 264, 0, 2, 1, 20)])
+def test_token_step_kernel_against_full_prefix_logits(tmp_path, dt, B, d, heads, mlp, window, T0):
+    """generate() of small batches runs its cached steps as one persistent kernel: the logits of every step equal those
+    of the full-prefix forward over the generated ids.  Widths that leave the 148 CTAs ragged shares, one to eight
+    sequences, windows shorter and longer than the context, stacks with and without attention.  Bars: the model bars
+    of this file for bf16 (2e-2); fp32 sums of at most 4096 terms in another order, 1e-5 per layer."""
+    import flash_stu_2_b200 as F
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(d + B)
+    V, new = 1003, 12
+    cfg = F.FlashSTUConfig(n_embd=d, n_layers=4, n_heads=max(heads, 1), seq_len=256, window_size=window, vocab_size=V,
+                           mlp_scale=mlp, num_eigh=8, use_attn=heads > 0, torch_dtype=dt)
+    with torch.device(dev()):
+        m = F.FlashSTU(cfg)
+    with torch.no_grad():
+        for name, p in m.named_parameters():
+            if not name.endswith("norm.weight"):
+                p.normal_(0.0, 0.5 * p.shape[-1] ** -0.5)
+    m.eval()
+    ids, logits = m.generate(torch.randint(0, V, (B, T0), device=dev()), max_length=T0 + new, do_sample=False,
+                             return_logits=True)
+    with torch.no_grad():
+        want = m(ids, use_cache=False).logits[:, T0 - 1:-1]
+    ops.check_status()
+    close(logits, want, 4e-5 if dt == torch.float32 else 2e-2)
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for
