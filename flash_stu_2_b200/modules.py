@@ -429,7 +429,7 @@ class Attention(nn.Module):
         if norm_w is not None:
             qkv = ops.linear(xn.reshape(B * T, d), self.c_attn.weight, norm_w=norm_w, eps=eps).view(B, T, 3 * d)
         else:
-        ov = ops.FLAG_OVERLAP if (T == 1 and ops.overlap_decode) else 0   # token step: weights fetched early
+            ov = ops.FLAG_OVERLAP if (T == 1 and ops.overlap_decode) else 0   # token step: weights fetched early
             qkv = ops.linear(xn.reshape(B * T, d), self.c_attn.weight, epilogue=ops.EPI_STORE | ov).view(B, T, 3 * d)
         if entry is None and use_cache:
             entry = self.new_cache(B, xn.device)

@@ -99,7 +99,6 @@ def check_status(device=None):
             raise RuntimeError(f"flash_stu_2_b200 device status {v}: {STATUS_TEXT.get(v, 'unknown')}")
 
 
-def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = RMS_EPS, out: Optional[torch.Tensor] = None):
 _local = threading.local()   # .arena: where this thread's outputs come from while an `arena` block is open
 
 
@@ -136,6 +135,7 @@ def empty(shape, dtype: torch.dtype, device) -> torch.Tensor:
     return torch.empty(shape, dtype=dtype, device=device)
 
 
+def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = RMS_EPS, out: Optional[torch.Tensor] = None):
     _cuda(x, weight)
     d = x.shape[-1]
     x2 = x.reshape(-1, d)
@@ -465,10 +465,6 @@ def block_decode_step(x, stu_norm_w, MinT, hist, taps8, pos, mlp_norm_w, Wg, Wu,
     return out
 
 
-def to_history(x, hist, t0: int):
-    """x [B,T,d] -> hist[b][c][t&1][t>>1] for t in [t0, t0+T)."""
-    _cuda(x, hist)
-    B, T, d = x.shape
 def token_step(plan: torch.Tensor, n_stages: int, args, bf16: bool):
     """One token step of a stack of layers in one persistent kernel; plan: the device copy of stu_token_step_plan's
     table, args a _lib.StepArgs whose tensors the caller keeps alive."""
@@ -477,6 +473,10 @@ def token_step(plan: torch.Tensor, n_stages: int, args, bf16: bool):
     _count()
 
 
+def to_history(x, hist, t0: int):
+    """x [B,T,d] -> hist[b][c][t&1][t>>1] for t in [t0, t0+T)."""
+    _cuda(x, hist)
+    B, T, d = x.shape
     assert hist.is_contiguous() and hist.shape[:3] == (B, d, 2) and x.stride(2) == 1
     rc = _lib.load().stu_to_history(x.data_ptr(), x.stride(0), x.stride(1), hist.data_ptr(), B, d, hist.shape[3], t0,
                                     t0 + T, _dt(x), _stream())

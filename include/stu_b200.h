@@ -349,10 +349,6 @@ int stu_peer_exchange(const void* xchg, void* x, long long x_row_stride, const v
                       long long xn_row_stride, float eps, int rows, int d, int* status, int wait_ms, int dtype,
                       void* stream);
 
-#ifdef __cplusplus
-}
-#endif
-#endif /* STU_B200_H */
 /* One token step of a stack of layers -- approx STU layers (flash_stu/layers/stu_layer.py:78-97) and sliding-window
  * attention layers (flash_stu/layers/attention_layer.py:50-66) in any order, each with its MLP -- as ONE persistent
  * cooperative kernel for up to 8 sequences at one common position: x = layers(x) in place, or, with `ids`, from the
@@ -409,3 +405,7 @@ long long stu_token_step_plan_bytes(int n_layers);
 int stu_token_step_plan(const StuStepLayer* layers, const StuStepArgs* args, int dtype, void* plan);
 int stu_token_step(const void* plan_on_device, int n_stages, const StuStepArgs* args, int dtype, void* stream);
 
+#ifdef __cplusplus
+}
+#endif
+#endif /* STU_B200_H */
