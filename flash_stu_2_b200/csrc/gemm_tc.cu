@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* issued_ctr = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));
   int* consumed_ctr = issued_ctr + 1;
-  uint32_t* row_stage = reinterpret_cast<uint32_t*>(smem + STAGES * STAGE_BYTES + 256);   // [4][32][17], EPI_STORE
+  uint32_t* row_stage = reinterpret_cast<uint32_t*>(smem + STAGES * STAGE_BYTES + 256);   // [4][32][17], EPI_STORE and EPI_HIST_T
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = tiles_m * tiles_n;
@@ -274,7 +274,10 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
     // ---------------- epilogue warps: TMEM lane quarter = warp % 4
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
-    const bool unaligned = EPI == EPI_STORE && ((ep.ldy & 7) || (reinterpret_cast<uintptr_t>(ep.y) & 15));
+    // output that is off the 16-byte grid goes through shared memory: plain rows of any stride, and histories whose
+    // sequences or first position are no multiple of a 32-column block
+    const bool unaligned = EPI == EPI_STORE ? ((ep.ldy & 7) || (reinterpret_cast<uintptr_t>(ep.y) & 15))
+                                            : EPI == EPI_HIST_T && ((ep.Tseq & 31) || (ep.t0 & 15) || (ep.Lh & 7));
     int it = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, it++) {
       int tm, tn;
@@ -296,8 +299,9 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const int nb = n0 + cch * 32;
         if (unaligned) {
-          // output rows off the 16-byte grid (the logits of an odd vocabulary): the warp's 32 x 32 block goes through
-          // shared memory and leaves row by row, 64 consecutive bytes per store instruction
+          // the warp's 32 x 32 block leaves row by row: 64 consecutive bytes per store instruction, in a history (a row
+          // is a channel, a lane a token) 32 in each parity row.  (Stored by the threads that hold the rows, 2 bytes to
+          // each of 32 rows per instruction, the projection of 4 x 1999 tokens into a 1024-wide history took 90 us.)
           uint32_t* st = row_stage + quarter * (32 * 17);
           __syncwarp();
 #pragma unroll
@@ -307,16 +311,26 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
           }
           __syncwarp();
           const bf16* col = reinterpret_cast<const bf16*>(st) + lane;
-          bf16* yc = ep.y + (size_t)(m0 + quarter * 32) * ep.ldy + nb + lane;
-          const int rows = min(32, M - (m0 + quarter * 32));
-          if (nb + lane < N)
+          const int first = m0 + quarter * 32, rows = min(32, M - first), n = nb + lane;
+          if (n < N) {
+            bf16* yc;
+            size_t pitch;
+            if (EPI == EPI_HIST_T) {
+              const int b = n / ep.Tseq;
+              yc = ep.y + hist_off(b, first, ep.t0 + (n - b * ep.Tseq), (int)ep.ldy, ep.Lh);
+              pitch = (size_t)2 * ep.Lh;
+            } else {
+              yc = ep.y + (size_t)first * ep.ldy + n;
+              pitch = (size_t)ep.ldy;
+            }
 #pragma unroll 8
-            for (int i = 0; i < rows; i++) yc[(size_t)i * ep.ldy] = col[i * 34];
+            for (int i = 0; i < rows; i++) yc[i * pitch] = col[i * 34];
+          }
         } else if (m < M && nb < N) {
           if (EPI == EPI_HIST_T) {
             // row m = channel, columns = tokens nb..nb+31 of the flattened [B, T] batch
             const int d = (int)ep.ldy;
-            const bool fast = (ep.Tseq % 32 == 0) && (ep.t0 % 16 == 0) && (nb + 32 <= N) && (ep.Lh % 8 == 0);
+            const bool fast = nb + 32 <= N;   // (the rest of the alignment: see `unaligned`)
             if (fast) {
               const int b = nb / ep.Tseq, t = ep.t0 + (nb - b * ep.Tseq);  // t % 16 == 0
               float ev[16], od[16];
@@ -509,7 +523,7 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
   constexpr int BN = TN;
   constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2 * (DUAL ? 2 : 1);
-  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + (EPI == EPI_STORE ? 4 * 32 * 17 * 4 : 0);
+  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + (EPI == EPI_STORE || EPI == EPI_HIST_T ? 4 * 32 * 17 * 4 : 0);
   auto k = gemm_tc_kernel<EPI, STAGES, TN>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -867,12 +881,18 @@ bool gemm_tc_supported(const void* A, long long lda, const void* B, long long ld
   return get_encode_fn() != nullptr;
 }
 
-// 128 x 256 tiles when the output has at least two waves of them (rows x cols of the GEMM as the kernel sees it).
+// 128 x 256 tiles where their waves over the SMs take less time than those of 128 x 128 tiles: a wide tile costs 1.31
+// square ones (measured per 64 of K over 768 of them: 0.395 against 0.302 us; the square tile is bound by the
+// shared-memory reads of its operands).  Two waves of wide tiles against four of square ones: down projection
+// 7996 x 1024 x 4096 99 -> 66 us.
 // STU_B200_TILE_N=128 forces the square tiles.
 static bool wide_tiles(long long rows, long long cols) {
   static const char* env = getenv("STU_B200_TILE_N");
   if (env && atoi(env) == 128) return false;
-  return cols >= 512 && ((rows + BM - 1) / BM) * ((cols + 255) / 256) >= 2 * 148;
+  const long long sms = device_sm_count(), tiles_m = (rows + BM - 1) / BM;
+  const long long wide = (tiles_m * ((cols + 255) / 256) + sms - 1) / sms;
+  const long long square = (tiles_m * ((cols + 127) / 128) + sms - 1) / sms;
+  return 131 * wide < 100 * square;
 }
 
 int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N,

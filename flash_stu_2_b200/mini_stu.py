@@ -14,7 +14,7 @@ import torch.nn as nn
 
 from . import ops
 from .filters import get_spectral_filters, nearest_power_of_two
-from .modules import STU, new_pos, host_pos
+from .modules import STU, _sm_count, new_pos, host_pos
 
 LDS_PARAMS = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data", "lds_params.pt")
 
@@ -195,6 +195,17 @@ class MiniSTU(nn.Module):
             W = torch.cat([Q, T2], dim=2).to(self.dtype)
         return Vs.to(device), W.reshape(Ck * F_, -1).contiguous().to(device), R
 
+    def _lds_group(self, B: int, T: int, width: int, x) -> int:
+        """Sequences per contraction: as many as leave the fewest waves of 128 x 256 output tiles in all, within 2 GiB of
+        features (16 sequences of 6000 positions to 1024 outputs: groups of 3, 22 waves instead of 32)."""
+        sms = _sm_count(x.device)
+
+        def waves(n):
+            return -(-(-(-n * T // 128) * -(-self.output_dim // 256)) // sms)
+
+        most = max(1, min(B, (2 << 30) // max(1, T * width * x.element_size())))
+        return min(range(1, most + 1), key=lambda g: (B // g * waves(g) + (waves(B % g) if B % g else 0), g))
+
     def _forward_lds(self, x, past_key_value=None, use_cache=False):
         op = self._lds_prepared()
         A32, B32, Cm = self._lds_f32
@@ -234,10 +245,16 @@ class MiniSTU(nn.Module):
         h = torch.empty(B, d, D, dtype=torch.float64, device=x.device)
         ops.lds_chunk_scan(x, A32, B32, Vs, Z, h, Ck, unit_b=self._lds_unit_b)
         _, Mcat = op.prepared_full()
-        U2 = torch.empty(nch * Ck, F_ * d, dtype=x.dtype, device=x.device)
-        for b in range(B):
-            ops.lds_chunk_features(W, Z[b].view(nch * d, W.shape[1]), U2, d, Ck, F_)
-            ops.linear(U2[:T], Mcat, out=y[b])
+        # sequences of a group share the contraction (one alone leaves its last wave of output tiles nearly empty).  Their
+        # features follow one another T rows apart; the rows past T of a sequence's last chunk are overwritten by
+        # the next sequence's, or lie past the group's rows.
+        G = self._lds_group(B, T, F_ * d, x)
+        U2 = torch.empty((G - 1) * T + nch * Ck, F_ * d, dtype=x.dtype, device=x.device)
+        for b0 in range(0, B, G):
+            n = min(G, B - b0)
+            for b in range(b0, b0 + n):
+                ops.lds_chunk_features(W, Z[b].view(nch * d, W.shape[1]), U2[(b - b0) * T:(b - b0) * T + nch * Ck], d, Ck, F_)
+            ops.linear(U2[:n * T], Mcat, out=y[b0:b0 + n].view(n * T, self.output_dim))
         if not use_cache:
             return y
         pos = new_pos(B, x.device)

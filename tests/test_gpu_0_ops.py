@@ -159,6 +159,25 @@ def test_linear_output_rows_off_the_16_byte_grid(shape):
     assert bool((y[:, N:] == 7.0).all()) and float(buf[0]) == 7.0
 
 
+@pytest.mark.parametrize("shape", [(3, 70, 37, 0, 40), (2, 300, 129, 5, 72), (1, 2000, 64, 16, 48), (4, 1024, 1999, 0, 1000),
+                                   (2, 264, 96, 33, 67)])
+def test_projection_into_history_off_the_block_grid(shape):
+    """EPI_HIST of the tcgen05 GEMM for sequences, first positions and history pitches that are no multiple of its
+    32-token blocks, square and wide tiles: every new position lands in its parity row, nothing else is written."""
+    from flash_stu_2_b200 import ops
+    B, d, T, t0, Lh = shape
+    torch.manual_seed(8)
+    x, W = torch.randn(B, T, 64).bfloat16(), (torch.randn(d, 64) / 8).bfloat16()
+    hist = torch.full((B, d, 2, Lh), 7.0, dtype=torch.bfloat16, device=dev())
+    ops.linear(x.view(B * T, 64).to(dev()), W.to(dev()), out=hist, epilogue=ops.EPI_HIST, hist_T=T, hist_t0=t0,
+               hist_Lh=Lh, backend=2)
+    ops.check_status()
+    flat = hist.cpu().transpose(2, 3).reshape(B, d, 2 * Lh)
+    close(flat[:, :, t0:t0 + T], _lin_ref(x.view(B * T, 64), W, None, None, 0, torch.bfloat16).view(B, T, d).transpose(1, 2),
+          1e-2)
+    assert bool((flat[:, :, :t0] == 7.0).all()) and bool((flat[:, :, t0 + T:] == 7.0).all())
+
+
 def test_bounded_wait_expiry_is_reported_and_the_context_survives():
     """Failure detection inside the tcgen05 GEMM: with the copies of its first pipeline stage dropped (test hook) the
     consumer's bounded wait runs out after the shortened limit; the kernel reports status 3, frees its tensor memory
