@@ -504,6 +504,18 @@ def full_combine(E, Q, U, B: int, d: int, K: int, k: int, both_signs: bool, t0: 
     _count()
 
 
+def full_conv(hist, phi, U, both_signs: bool, t0: int, t_end: int):
+    """U+- of all filters (fp32): hist [B,d,2,Lh], phi [L,K] -> U [B*(t_end-t0), (1 or 2)*K*d]."""
+    _cuda(hist, phi, U)
+    B, d, _, Lh = hist.shape
+    L, K = phi.shape
+    assert hist.is_contiguous() and phi.is_contiguous() and U.stride(1) == 1 and U.shape[0] == B * (t_end - t0)
+    rc = _lib.load().stu_full_conv(hist.data_ptr(), Lh, phi.data_ptr(), L, K, U.data_ptr(), U.stride(0), B, d,
+                                   int(both_signs), t0, t_end, _dt(hist), _stream())
+    _lib.check(rc, "stu_full_conv")
+    _count()
+
+
 def full_decode_prepare(x2d, hist, phi, pos, PhiT):
     _cuda(x2d, hist, phi, pos, PhiT)
     B, d, _, Lh = hist.shape

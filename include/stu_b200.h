@@ -216,6 +216,10 @@ int stu_toeplitz(const void* f, long long f_stride, int L, void* out, int S, lon
  * order (the even-tap and odd-tap products of filter k). */
 int stu_full_combine(const void* E, const void* Q, long long ldE, void* U, long long ldU, int B, int d, int K, int k,
                      int both_signs, int t0, int t_end, int dtype, void* stream);
+/* The same operand for all K filters in one launch, from the history and the filters themselves (fp32 only):
+ * hist [B*d][2][Lh] holds the inputs of times [0, t_end), phi [L][K], Lh a multiple of 4. */
+int stu_full_conv(const void* hist, int Lh, const void* phi, int L, int K, void* U, long long ldU, int B, int d,
+                  int both_signs, int t0, int t_end, int dtype, void* stream);
 
 /* One cached decode step of the full variant, around one GEMM G = hist_rows @ PhiT^T (stu_linear, M = B*d*2,
  * N = 2K, K = Lh): prepare appends x_t at time pos[0] and rebuilds PhiT [2K][Lh] (time-reversed even / odd

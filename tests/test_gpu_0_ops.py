@@ -884,6 +884,35 @@ def test_full_variant_building_blocks(dt):
     assert torch.equal(U.cpu().view(B, T, 2, K, d), want)
 
 
+@pytest.mark.parametrize("shape", [(1, 7, 16, 5, 300, 0, 90), (1, 5, 27, 3, 97, 0, 97), (3, 24, 33, 4, 200, 61, 200),
+                                   (5, 1, 64, 2, 400, 128, 321), (2, 24, 96, 2, 130, 129, 130)])
+@pytest.mark.parametrize("both", [True, False])
+def test_full_convolution_of_all_filters(shape, both):
+    """The one-launch fp32 operand U against float64 sums: 4, 8 and 16 threads across the channels, tiles that hold several
+    sequences, odd channel counts, ranges that start inside the history, one position.  Bar: at most 200 fp32 roundings
+    of 2^-24 per sum."""
+    from flash_stu_2_b200 import ops
+    B, K, d, pad, L, t0, t_end = shape
+    torch.manual_seed(14)
+    Lh = ((t_end + 1) // 2 + pad + 7) // 8 * 8
+    x, phi = torch.randn(B, t_end, d), torch.randn(L, K) / 4
+    hist = torch.full((B, d, 2, Lh), float("nan"), device=dev())   # what lies past the last input is not read
+    ops.to_history(x.to(dev()), hist, 0)
+    U = torch.full((B * (t_end - t0), (2 if both else 1) * K * d + 4), 7.0, device=dev())
+    ops.full_conv(hist, phi.to(dev()), U, both, t0, t_end)
+    ops.check_status()
+    f = torch.zeros(max(L, t_end), K, dtype=torch.float64)
+    f[:L] = phi
+    lag = torch.arange(t_end)[:, None] - torch.arange(t_end)[None, :]
+    want = []
+    for sign in (1.0, -1.0)[: 2 if both else 1]:
+        taps = f * torch.where(torch.arange(f.shape[0]) % 2 == 1, sign, 1.0)[:, None]
+        T = torch.where((lag >= 0)[:, :, None], taps[lag.clamp_min(0)], torch.zeros((), dtype=torch.float64))
+        want.append(torch.einsum("tsk,bsi->btki", T, x.double())[:, t0:].reshape(B * (t_end - t0), K * d))
+    close(U[:, :-4], torch.cat(want, 1), 1e-5)
+    assert bool((U[:, -4:] == 7.0).all())
+
+
 @pytest.mark.parametrize("name,tol", [("std_full_float32", 1e-3), ("std_full_bfloat16", 2e-2),
                                        ("hankelL_full_float32", 1e-3), ("std_approx_float32", 1e-3),
                                        ("std_approx_bfloat16", 2e-2), ("hankelL_approx_float32", 1e-3),
