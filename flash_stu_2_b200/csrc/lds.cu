@@ -150,14 +150,21 @@ __global__ void __launch_bounds__(256) lds_decode_kernel(const T* __restrict__ x
 
 // Chunked scan: one CTA = 32 consecutive channels of one sequence (lane = channel), warp w owns modes
 // w*MPW .. w*MPW+MPW-1 of all 32 (state, A and B in registers, float64).  Per chunk: (1) the state carried into the
-// chunk is rotated, z_k = sum_n Vs[n][k] h[n] (Vs = V / sqrt(lambda), float64; every warp takes R/8 of the k through
-// a shared-memory copy of the state) and written as the leading columns of Z; (2) the chunk's inputs are staged in
-// shared memory, copied into the trailing Ck columns of Z (the Toeplitz operand) and (3) pushed through the
-// recurrence h = fma(A, h, B*x) position by position - the same expression, in the same order, as
-// lds_final_state_kernel, so the final state is bit-identical to that kernel's.
+// chunk is rotated, z_k = sum_n Vs[n][k] h[n] (Vs = V / sqrt(lambda), float64), and written as the leading columns of
+// Z; (2) the chunk's inputs are staged in shared memory, copied into the trailing Ck columns of Z (the Toeplitz
+// operand) and (3) pushed through the recurrence h = fma(A, h, B*x) position by position - the same expression, in the
+// same order, as lds_final_state_kernel, so the final state is bit-identical to that kernel's.
+// Bound: float64 FMAs (D per position and channel, D * R per chunk and channel).  The rotation is a [32 x D] . [D x R]
+// product on the float64 tensor path (m8n8k4; a warp owns 8 coordinates of all channels): one 8-byte read of Vs and
+// four of the state per 1024 FMAs.  As plain FMAs it read 16 bytes of Vs per two, the same ones in every lane, and the
+// load path took two thirds of the kernel; inputs were converted to float64 once per warp, now once.  16 sequences of
+// 6000 x 1024, D = 160, R = 64: 5.2 -> 2.5 ms.
 // Z: [B][nchunks][d][KZ] in the model dtype, KZ = 3*R + Ck (bf16: z_hi | z_lo | z_hi | x) or R + Ck (fp32: z | x).
 // UNITB: every B[n] == 1 (the distilled checkpoint's case): B*x is x, so the multiplication is dropped and the
 // result stays bit-identical to the general expression.
+constexpr int SCAN_X = 128;   // positions staged at a time
+constexpr int SCAN_HP = 36;   // distance of the state rows: the fragments' 4 modes x 8 channels fall on distinct banks
+
 template <typename T, int MPW, bool UNITB>
 __global__ void __launch_bounds__(256, UNITB ? 2 : 1) lds_chunk_scan_kernel(const T* __restrict__ x, long long x_bstride,
                                                              long long x_tstride, const double* __restrict__ A,
@@ -166,8 +173,9 @@ __global__ void __launch_bounds__(256, UNITB ? 2 : 1) lds_chunk_scan_kernel(cons
                                                              double* __restrict__ hfin, int d, int Tn, int D, int R,
                                                              int Ck, int KZ) {
   extern __shared__ __align__(16) unsigned char scan_smem[];
-  double* hs = reinterpret_cast<double*>(scan_smem);               // [D][33] state copy for the rotation
-  T* xs = reinterpret_cast<T*>(hs + (size_t)D * 33);               // [Ck][32] inputs of the chunk
+  const int Dp = (D + 3) & ~3;
+  double* hs = reinterpret_cast<double*>(scan_smem);   // [Dp][SCAN_HP] state copy for the rotation, zero rows past D
+  double* xs = hs + (size_t)Dp * SCAN_HP;              // [SCAN_X][33] inputs
   constexpr bool SPLIT = (sizeof(T) == 2);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nblk = (d + 31) >> 5;
@@ -183,73 +191,73 @@ __global__ void __launch_bounds__(256, UNITB ? 2 : 1) lds_chunk_scan_kernel(cons
     if (!UNITB) bb[m] = n < D ? Bv[n] : 0.0;
     h[m] = 0.0;
   }
+  for (int e = D * SCAN_HP + threadIdx.x; e < Dp * SCAN_HP; e += 256) hs[e] = 0.0;
+  const int r8 = lane >> 2, c4 = lane & 3;   // fragment coordinates
   for (int c = 0; c < nchunks; c++) {
     const int t0 = c * Ck;
-    T* zrow = Z + ((size_t)((size_t)b * nchunks + c) * d + (chok ? ch : 0)) * KZ;
+    T* zc = Z + ((size_t)((size_t)b * nchunks + c) * d + i0) * KZ;   // row of the first channel
     // ---- (1) rotate the carried state
 #pragma unroll
     for (int m = 0; m < MPW; m++) {
       const int n = warp * MPW + m;
-      if (n < D) hs[n * 33 + lane] = h[m];
+      if (n < D) hs[n * SCAN_HP + lane] = h[m];
     }
     __syncthreads();
-    // this warp's coordinates k0 .. k0+7 (groups of eight; R % 8 == 0): one pass over the modes with eight
-    // independent accumulators, the state value of a mode read once and the eight rotation entries as 16-byte
-    // warp-uniform loads
-    for (int k0 = warp * 8; k0 < R; k0 += 64) {
-      double z[8];
+    for (int k0 = warp * 8; k0 < R; k0 += 64) {   // this warp's coordinates k0 .. k0+7 (R % 8 == 0)
+      double z[4][2];   // channel 8j + r8, coordinates k0 + 2 c4 and the next
 #pragma unroll
-      for (int j = 0; j < 8; j++) z[j] = 0.0;
-#pragma unroll 2
-      for (int n = 0; n < D; n++) {
-        const double hv = hs[n * 33 + lane];
-        const double2* vr = reinterpret_cast<const double2*>(Vs + (size_t)n * R + k0);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const double2 v2 = __ldg(vr + j);
-          z[2 * j] = fma(v2.x, hv, z[2 * j]);
-          z[2 * j + 1] = fma(v2.y, hv, z[2 * j + 1]);
-        }
-      }
-      if (chok) {
-        float zf[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) zf[j] = (float)z[j];
-        if (SPLIT) {   // eight consecutive coordinates: one 16-byte store per copy
-          store_vec(zrow + k0, zf);           // rounds to the high parts
-          store_vec(zrow + 2 * R + k0, zf);
-#pragma unroll
-          for (int j = 0; j < 8; j++) zf[j] -= round_to<T>(zf[j]);
-          store_vec(zrow + R + k0, zf);       // low parts
-        } else {
-          store_vec(zrow + k0, zf);
-          store_vec(zrow + k0 + 4, zf + 4);
-        }
-      }
-    }
-    // ---- (2) stage the chunk's inputs (zero past the end of the sequence) and copy them into Z
-    const int zoff = SPLIT ? 3 * R : R;
-    for (int e = threadIdx.x; e < Ck * 32; e += 256) {
-      const int sg = e >> 5, cc = e & 31;
-      const int t = t0 + sg;
-      xs[e] = (t < Tn && i0 + cc < d) ? x[(size_t)b * x_bstride + (size_t)t * x_tstride + i0 + cc]
-                                      : Elem<T>::from_f(0.f);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < Ck * 32; e += 256) {   // consecutive threads write consecutive positions of a row
-      const int cc = e / Ck, sg = e - cc * Ck;
-      if (i0 + cc < d)
-        Z[((size_t)((size_t)b * nchunks + c) * d + i0 + cc) * KZ + zoff + sg] = xs[sg * 32 + cc];
-    }
-    // ---- (3) the recurrence over the chunk
-    const int lim = min(Ck, Tn - t0);
+      for (int j = 0; j < 4; j++) z[j][0] = z[j][1] = 0.0;
+      const double* hp = hs + c4 * SCAN_HP + r8;
+      const double* vp = Vs + (size_t)c4 * R + k0 + r8;
 #pragma unroll 4
-    for (int sg = 0; sg < lim; sg++) {
-      const double xv = (double)Elem<T>::to_f(xs[sg * 32 + lane]);
+      for (int n = 0; n < Dp; n += 4) {
+        const double v = n + c4 < D ? __ldg(vp + (size_t)n * R) : 0.0;
 #pragma unroll
-      for (int m = 0; m < MPW; m++) h[m] = UNITB ? fma(a[m], h[m], xv) : fma(a[m], h[m], bb[m] * xv);
+        for (int j = 0; j < 4; j++) dmma_884(z[j][0], z[j][1], hp[n * SCAN_HP + 8 * j], v);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (i0 + 8 * j + r8 < d) {
+          T* zr = zc + (size_t)(8 * j + r8) * KZ + k0 + 2 * c4;
+          const float z0 = (float)z[j][0], z1 = (float)z[j][1];
+          if constexpr (SPLIT) {
+            const __nv_bfloat162 hi = __floats2bfloat162_rn(z0, z1);
+            *reinterpret_cast<__nv_bfloat162*>(zr) = hi;
+            *reinterpret_cast<__nv_bfloat162*>(zr + R) =
+                __floats2bfloat162_rn(z0 - __bfloat162float(hi.x), z1 - __bfloat162float(hi.y));
+            *reinterpret_cast<__nv_bfloat162*>(zr + 2 * R) = hi;
+          } else {
+            *reinterpret_cast<float2*>(zr) = make_float2(z0, z1);
+          }
+        }
+      }
     }
-    __syncthreads();   // xs and hs are rewritten by the next chunk
+    const int zoff = SPLIT ? 3 * R : R;
+    for (int s0 = 0; s0 < Ck; s0 += SCAN_X) {   // (once for the chunks of 128 positions that the prefill uses)
+      const int ns = min(SCAN_X, Ck - s0);
+      // ---- (2) stage the chunk's inputs (zero past the end of the sequence) and copy them into Z
+      for (int e = threadIdx.x; e < ns * 32; e += 256) {
+        const int sg = e >> 5, cc = e & 31;
+        const int t = t0 + s0 + sg;
+        xs[sg * 33 + cc] = (t < Tn && i0 + cc < d)
+                               ? (double)Elem<T>::to_f(x[(size_t)b * x_bstride + (size_t)t * x_tstride + i0 + cc])
+                               : 0.0;
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < SCAN_X * 32; e += 256) {   // consecutive threads write consecutive positions of a row
+        const int cc = e / SCAN_X, sg = e % SCAN_X;
+        if (i0 + cc < d && sg < ns) zc[(size_t)cc * KZ + zoff + s0 + sg] = Elem<T>::from_f((float)xs[sg * 33 + cc]);
+      }
+      // ---- (3) the recurrence over them
+      const int lim = min(ns, Tn - t0 - s0);
+#pragma unroll 4
+      for (int sg = 0; sg < lim; sg++) {
+        const double xv = xs[sg * 33 + lane];
+#pragma unroll
+        for (int m = 0; m < MPW; m++) h[m] = UNITB ? fma(a[m], h[m], xv) : fma(a[m], h[m], bb[m] * xv);
+      }
+      __syncthreads();   // xs and hs are rewritten
+    }
   }
   if (chok) {
 #pragma unroll
@@ -276,9 +284,7 @@ extern "C" int stu_lds_chunk_scan(const void* x, long long x_bstride, long long 
     return STU_ERR_SHAPE;
   if (dtype != STU_F32 && dtype != STU_BF16) return STU_ERR_DTYPE;
   const int KZ = (dtype == STU_BF16 ? 3 * R : R) + Ck;
-  const size_t elem = dtype == STU_BF16 ? 2 : 4;
-  const size_t smem = (size_t)D * 33 * sizeof(double) + (size_t)Ck * 32 * elem;
-  if (smem > 200 * 1024) return STU_ERR_UNSUPPORTED;
+  const size_t smem = ((size_t)((D + 3) & ~3) * SCAN_HP + (size_t)SCAN_X * 33) * sizeof(double);
   const int grid = B * ((d + 31) / 32);
   cudaStream_t st = (cudaStream_t)stream;
   const int mpw = (D + 7) / 8;
