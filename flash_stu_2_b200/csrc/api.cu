@@ -46,7 +46,9 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
   if (M == 0) return STU_OK;
   const int causal = (epilogue & EPI_FLAG_CAUSAL) ? 1 : 0;
   const int pdl = epilogue & (STU_FLAG_OVERLAP | STU_FLAG_EARLY_TRIGGER);  // honoured by the skinny kernels only
-  epilogue &= ~(EPI_FLAG_CAUSAL | STU_FLAG_OVERLAP | STU_FLAG_EARLY_TRIGGER);
+  const bool kpos = (epilogue & EPI_FLAG_KPOS) != 0;   // honoured by the tcgen05 GEMM; the zeros are there all the same
+  epilogue &= ~(EPI_FLAG_CAUSAL | EPI_FLAG_KPOS | STU_FLAG_OVERLAP | STU_FLAG_EARLY_TRIGGER);
+  if (kpos && (epilogue != EPI_STORE || !resid)) return STU_ERR_UNSUPPORTED;
   if ((epilogue < EPI_STORE || epilogue > EPI_HIST) && epilogue != EPI_BLOCKCOL) return STU_ERR_UNSUPPORTED;
   // EPI_BLOCKCOL: hist_T = columns per block, resid_row_stride = distance between blocks (elements); resid unused
   if (epilogue == EPI_BLOCKCOL && (hist_T <= 0 || resid_row_stride <= 0)) return STU_ERR_SHAPE;
@@ -66,6 +68,10 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
   ep.t0 = hist_t0;
   ep.Lh = hist_Lh;
   ep.ld2 = (epilogue == EPI_BLOCKCOL) ? resid_row_stride : 0;
+  if (kpos) {
+    ep.kpos = (const int*)resid;
+    ep.resid = nullptr;
+  }
 
   bool sk_ok = skinny_supported(x, x_row_stride, W, w_row_stride, w_k_stride, W2, M, N, K, epilogue, dtype);
   if (norm_w) {

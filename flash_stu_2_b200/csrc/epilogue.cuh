@@ -15,6 +15,8 @@ enum {
 };
 // OR-ed into the epilogue code: W is lower triangular (W[n][k] = 0 for k > n); kernels may skip those blocks
 #define EPI_FLAG_CAUSAL 0x100
+// ... : W[n][k] = 0 for k > t / 2, t the position that `resid` (not a residual then) points to on the device
+#define EPI_FLAG_KPOS 0x1000
 
 template <typename T> struct EpiArgs {
   T* y;
@@ -24,6 +26,7 @@ template <typename T> struct EpiArgs {
   // EPI_HIST: row m of the GEMM is token (m / T) * .. + (m % T) of a [B,T] batch starting at time t0
   int Tseq, t0, Lh;
   long long ld2;  // EPI_BLOCKCOL: distance between column blocks
+  const int* kpos;       // EPI_STORE only, may be NULL: W is zero past column kpos[0] / 2 (EPI_FLAG_KPOS)
   const PeerDest* peer;  // EPI_STORE only, may be NULL: the rows go to every rank's inbox (row stride ldy) instead of y
 };
 
@@ -34,11 +37,13 @@ struct EpiArgsAny {
   long long ldr;
   int Tseq, t0, Lh;
   long long ld2 = 0;
+  const int* kpos = nullptr;
   const PeerDest* peer = nullptr;
   template <typename U> EpiArgs<U> as() const {
     EpiArgs<U> e;
     e.y = (U*)y; e.ldy = ldy; e.resid = (const U*)resid; e.ldr = ldr; e.Tseq = Tseq; e.t0 = t0; e.Lh = Lh;
     e.ld2 = ld2;
+    e.kpos = kpos;
     e.peer = peer;
     return e;
   }

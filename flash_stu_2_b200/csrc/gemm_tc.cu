@@ -180,7 +180,8 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = tiles_m * tiles_n;
-  const int num_kb = (K + BK - 1) / BK;
+  int num_kb = (K + BK - 1) / BK;
+  if (EPI == EPI_STORE && ep.kpos) num_kb = min(num_kb, max(__ldg(ep.kpos), 0) / (2 * BK) + 1);   // the rest of W is zero
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {

@@ -276,7 +276,8 @@ class STU(nn.Module):
             self._dec_scratch_key = key
         PhiT, G, U = self._dec_scratch
         ops.full_decode_prepare(xn2d, hist, phi, pos, PhiT)
-        ops.linear(hist.view(B * d * 2, Lh), PhiT, out=G)
+        # (PhiT is zero past the position: the history beyond it, here to the end of its capacity, is not read)
+        ops.linear(hist.view(B * d * 2, Lh), PhiT, out=G, kpos=pos)
         ops.full_decode_combine(G, pos, U, B, d, K, nsign == 2, Lh, advance=True)
         ops.linear(U, Mcat, resid=resid2d, out=out2d, epilogue=ops.EPI_RESID)
         pos._host_t = t + 1

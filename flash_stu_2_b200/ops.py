@@ -15,6 +15,7 @@ from . import _lib
 
 EPI_STORE, EPI_RESID, EPI_GELU_MUL, EPI_HIST = 0, 1, 2, 3
 EPI_FLAG_CAUSAL = 0x100  # OR-ed into the epilogue: the weight is lower triangular
+EPI_FLAG_KPOS = 0x1000   # ... the weight is zero past column t / 2 (linear(kpos=): the position t on the device)
 # Overlapped (programmatic dependent) launches of the decode kernels: OR-ed into the epilogue code of linear() and
 # passed as flags to decode_approx().  FLAG_OVERLAP: the kernel may start while its predecessor in the stream is
 # still running and fetches its constants (weights; history and taps) meanwhile; FLAG_EARLY_TRIGGER: it lets its
@@ -186,7 +187,8 @@ def can_fuse_norm(M: int, N: int, K: int, epilogue: int, dtype: torch.dtype) -> 
 def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = None,
            resid: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, epilogue: int = EPI_STORE,
            norm_w: Optional[torch.Tensor] = None, eps: float = RMS_EPS, backend: int = BACKEND_AUTO,
-           transposed_weight: bool = False, hist_T: int = 0, hist_t0: int = 0, hist_Lh: int = 0):
+           transposed_weight: bool = False, hist_T: int = 0, hist_t0: int = 0, hist_Lh: int = 0,
+           kpos: Optional[torch.Tensor] = None):
     """y = epilogue(x @ W^T) for x [M,K] and W [N,K] (or W [K,N] with transposed_weight=True)."""
     _cuda(x, W, W2, resid, out, norm_w)
     assert x.dim() == 2 and W.dim() == 2 and x.stride(1) == 1
@@ -211,6 +213,9 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
     if resid is not None:
         assert resid.shape == (M, N) and resid.stride(1) == 1
         r_rs = resid.stride(0)
+    if kpos is not None:
+        assert resid is None and epilogue == EPI_STORE and kpos.is_cuda and kpos.dtype == torch.int32
+        resid, epilogue = kpos, EPI_STORE | EPI_FLAG_KPOS
     status_word(x.device)   # the tcgen05 GEMM reports an expired device-side wait through the registered word
     rc = _lib.load().stu_linear(x.data_ptr(), x.stride(0), W.data_ptr(), w_rs, w_ks, _p(W2), _p(resid), r_rs,
                                 out.data_ptr(), y_rs, M, N, K, epilogue, hist_T, hist_t0, hist_Lh, _p(norm_w), eps,

@@ -77,7 +77,8 @@ int stu_embed(const long long* ids, const void* table, void* out, int rows, int 
 /* epilogue flags: 0x100 = W is lower triangular (k-blocks above the diagonal are skipped); 0x200 = launch with
  * programmatic stream serialization: the kernel fetches W (which the preceding kernel must not write) while that
  * kernel drains, and reads x only after it has completed (skinny shapes, M <= 64; ignored otherwise);
- * 0x400 = let the next 0x200 launch start at once. */
+ * 0x400 = let the next 0x200 launch start at once; 0x1000 (epilogue 0) = W is zero past column t / 2, `resid` points to
+ * the position t (int) on the device: those columns may be left unread. */
 int stu_linear(const void* x, long long x_row_stride, const void* W, long long w_row_stride, long long w_k_stride,
                const void* W2, const void* resid, long long resid_row_stride, void* y, long long y_row_stride,
                int M, int N, int K, int epilogue, int hist_T, int hist_t0, int hist_Lh, const void* norm_w,
