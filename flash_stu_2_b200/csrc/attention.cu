@@ -368,15 +368,16 @@ static bool launch_swa_decode(const void* qkv, void* k_ring, void* v_ring, int* 
   if (hd % VPL || !aligned16(qkv) || !aligned16(k_ring) || !aligned16(v_ring) || !aligned16(out)) return false;
   dim3 grid(H, B);
 #define STU_SWA_DEC(LPK_)                                                                                        \
-  cudaFuncSetAttribute(swa_decode_kernel<T, LPK_>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_RING_BYTES);    \
+  static SmemLimit limit##LPK_;                                                                                     \
+  allow_smem((const void*)swa_decode_kernel<T, LPK_>, DEC_RING_BYTES, limit##LPK_);                                 \
   launch_maybe_overlapped(swa_decode_kernel<T, LPK_>, grid, dim3(256), DEC_RING_BYTES, st, true, (const T*)qkv,     \
                           (T*)k_ring, (T*)v_ring, pos, slopes, (T*)out, B, H, W, window, scale, softcap,            \
                           update_cache)
   switch (hd / VPL) {
-    case 4: STU_SWA_DEC(4); return true;
-    case 8: STU_SWA_DEC(8); return true;
-    case 16: STU_SWA_DEC(16); return true;
-    case 32: STU_SWA_DEC(32); return true;
+    case 4: { STU_SWA_DEC(4); return true; }
+    case 8: { STU_SWA_DEC(8); return true; }
+    case 16: { STU_SWA_DEC(16); return true; }
+    case 32: { STU_SWA_DEC(32); return true; }
   }
 #undef STU_SWA_DEC
   return false;
@@ -644,9 +645,10 @@ extern "C" int stu_swa_forward(const void* qkv, void* k_ring, void* v_ring, int*
   dim3 g2(Tn < W ? Tn : W, B);
   const int hdp = (hd + 31) & ~31;
   const size_t smem = (size_t)(hdp * AT_QT + hdp * (AT_KT + 1) + AT_KT * hdp) * sizeof(float);
-  cudaError_t ea = cudaFuncSetAttribute(swa_attend_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-  if (ea == cudaSuccess)
-    ea = cudaFuncSetAttribute(swa_attend_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  static SmemLimit limit;
+  cudaError_t ea = allow_smem((const void*)swa_attend_kernel<float>, 64 * 1024, limit);
+  static SmemLimit limit16;
+  if (ea == cudaSuccess) ea = allow_smem((const void*)swa_attend_kernel<bf16>, 64 * 1024, limit16);
   if (ea != cudaSuccess) return (int)ea;
   if (dtype == STU_F32) {
     swa_attend_kernel<float><<<grid, 256, smem, st>>>((const float*)qkv, (const float*)k_ring, (const float*)v_ring, pos,
@@ -662,12 +664,14 @@ extern "C" int stu_swa_forward(const void* qkv, void* k_ring, void* v_ring, int*
       dim3 fg((Tn + FA_BM - 1) / FA_BM, H, B);
       const size_t fsm = (size_t)(FA_BM + 4 * FA_BN) * hd * sizeof(bf16);
       if (hd == 128) {
-        ea = cudaFuncSetAttribute(swa_flash_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm);
+        static SmemLimit limit;
+        ea = allow_smem((const void*)swa_flash_kernel<128>, fsm, limit);
         if (ea != cudaSuccess) return (int)ea;
         swa_flash_kernel<128><<<fg, 128, fsm, st>>>((const bf16*)qkv, (const bf16*)k_ring, (const bf16*)v_ring, pos,
                                                     slopes, (bf16*)out, Tn, H, W, window, scale, softcap);
       } else {
-        ea = cudaFuncSetAttribute(swa_flash_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm);
+        static SmemLimit limit;
+        ea = allow_smem((const void*)swa_flash_kernel<64>, fsm, limit);
         if (ea != cudaSuccess) return (int)ea;
         swa_flash_kernel<64><<<fg, 128, fsm, st>>>((const bf16*)qkv, (const bf16*)k_ring, (const bf16*)v_ring, pos,
                                                    slopes, (bf16*)out, Tn, H, W, window, scale, softcap);

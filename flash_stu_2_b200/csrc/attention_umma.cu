@@ -414,7 +414,8 @@ extern "C" int stu_swa_prefill_tc5(const void* qkv, void* vt_scratch, void* k_ri
     int rc = encode_sw128(&tmV, vt_scratch, 2, dims, str, box);
     if (rc != STU_OK) return rc;
   }
-  cudaError_t e = cudaFuncSetAttribute(swa_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)swa_umma_kernel, SMEM_BYTES, limit);
   if (e != cudaSuccess) return (int)e;
   const float scale = 1.0f / sqrtf((float)HD);
   swa_umma_kernel<<<dim3((Tn + BM - 1) / BM, H, B), 192, SMEM_BYTES, st>>>(tmQ, tmK, tmV, pos, slopes, (bf16*)out, Tn,

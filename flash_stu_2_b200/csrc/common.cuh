@@ -4,6 +4,9 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #define STU_OK 0
 #define STU_ERR_DTYPE (-1)
 #define STU_ERR_SHAPE (-2)
@@ -24,6 +27,27 @@ typedef __nv_bfloat16 bf16;
     cudaError_t e__ = cudaGetLastError();         \
     if (e__ != cudaSuccess) return (int)e__;      \
   } while (0)
+
+// Raises a kernel's dynamic shared memory limit on the current device to `bytes`.  The runtime call takes a lock and a
+// table look-up, more than a launch should pay each time, so it is made only when the limit grows; `limit` is a static
+// of the call site (one per kernel).
+struct SmemLimit {
+  std::mutex m;
+  std::atomic<int> bytes[STU_MAX_DEVICES] = {};
+};
+inline cudaError_t allow_smem(const void* kernel, size_t bytes, SmemLimit& limit) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= STU_MAX_DEVICES)
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (limit.bytes[dev].load(std::memory_order_acquire) >= (int)bytes) return cudaSuccess;
+  std::lock_guard<std::mutex> hold(limit.m);   // the limit only ever grows: a smaller request does not lower it again
+  if (limit.bytes[dev].load(std::memory_order_relaxed) >= (int)bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) limit.bytes[dev].store((int)bytes, std::memory_order_release);
+  return e;
+}
 
 template <typename T> struct Elem;
 template <> struct Elem<float> {

@@ -19,6 +19,7 @@
 #include "epilogue.cuh"
 
 int device_sm_count();   // SM count of the current device (cached per device)
+static int current_device();
 
 namespace cg = cooperative_groups;
 
@@ -526,7 +527,8 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2 * (DUAL ? 2 : 1);
   const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + (EPI == EPI_STORE || EPI == EPI_HIST_T ? 4 * 32 * 17 * 4 : 0);
   auto k = gemm_tc_kernel<EPI, STAGES, TN>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)k, smem, limit);
   if (e != cudaSuccess) return (int)e;
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
   const int sm_count = device_sm_count();
@@ -763,7 +765,8 @@ int launch_skinny_umma(const CUtensorMap& w, const CUtensorMap& w2, const CUtens
   if (!deep && nstages > 5) nstages = 5;
   const size_t smem = su_smem_bytes<SU_BN>(nstages);
   auto kern = skinny_umma_kernel<EPI, KSPLIT, SU_BN>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)kern, smem, limit);
   if (e != cudaSuccess) return (int)e;
   if (KSPLIT > 8) {   // clusters of 16 CTAs are outside the portable range
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -783,12 +786,15 @@ int launch_skinny_umma(const CUtensorMap& w, const CUtensorMap& w2, const CUtens
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (KSPLIT > 8) {   // can the GPU co-schedule a cluster of this size and footprint at all?  (the caller falls back)
+  static std::atomic<int> cosched[STU_MAX_DEVICES] = {};   // the most shared memory per CTA that was found to fit
+  const int dev = current_device();
+  if (KSPLIT > 8 && cosched[dev].load(std::memory_order_relaxed) < (int)smem) {   // can the GPU co-schedule a cluster of this size and footprint at all?  (the caller falls back)
     int clusters = 0;
     if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
       (void)cudaGetLastError();
       return STU_ERR_UNSUPPORTED;
     }
+    cosched[dev].store((int)smem, std::memory_order_relaxed);
   }
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, kern, w, w2, x, M, N, K, ep, status, early, g_wait_ns, nstages);
@@ -885,7 +891,7 @@ bool gemm_tc_supported(const void* A, long long lda, const void* B, long long ld
 // 128 x 256 tiles where their waves over the SMs take less time than those of 128 x 128 tiles: a wide tile costs 1.31
 // square ones (measured per 64 of K over 768 of them: 0.395 against 0.302 us; the square tile is bound by the
 // shared-memory reads of its operands).  Two waves of wide tiles against four of square ones: down projection
-// 7996 x 1024 x 4096 99 -> 66 us.
+// 7996 x 1024 x 4096 99 -> 69 us.
 // STU_B200_TILE_N=128 forces the square tiles.
 static bool wide_tiles(long long rows, long long cols) {
   static const char* env = getenv("STU_B200_TILE_N");

@@ -340,12 +340,14 @@ extern "C" int stu_lds_decode_features(const void* x, long long x_row_stride, do
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e;
   if (dtype == STU_F32) {
-    e = cudaFuncSetAttribute(lds_decode_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimit limit;
+    e = allow_smem((const void*)lds_decode_kernel<float>, smem, limit);
     if (e != cudaSuccess) return (int)e;
     lds_decode_kernel<float><<<(rows + 63) / 64, 256, smem, st>>>((const float*)x, x_row_stride, h, A, Bv,
                                                                 (const float*)C, (float*)U, B, d, D, F);
   } else if (dtype == STU_BF16) {
-    e = cudaFuncSetAttribute(lds_decode_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimit limit;
+    e = allow_smem((const void*)lds_decode_kernel<bf16>, smem, limit);
     if (e != cudaSuccess) return (int)e;
     lds_decode_kernel<bf16><<<(rows + 63) / 64, 256, smem, st>>>((const bf16*)x, x_row_stride, h, A, Bv, (const bf16*)C,
                                                                (bf16*)U, B, d, D, F);

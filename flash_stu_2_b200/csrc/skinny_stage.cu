@@ -222,7 +222,8 @@ int launch_stage(const void* A, long long lda, const void* B, long long ldb, con
   const size_t red_bytes = (size_t)NT * NW * MT * 128 * sizeof(float);
   const size_t smem = xs_bytes > red_bytes ? xs_bytes : red_bytes;
   auto kern = skinny_stage_kernel<EPI, MT, KSPLIT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)kern, smem, limit);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((N + NF - 1) / NF, KSPLIT);

@@ -195,7 +195,8 @@ int launch_wide_n(const void* A, long long lda, const void* B, long long ldb, in
                   const EpiArgs<bf16>& ep, const void* nw, float eps, cudaStream_t st) {
   const size_t smem = (size_t)(NT * NW * MT * 128 + (KSPLIT > 1 ? NT * MT * 128 : 0)) * sizeof(float);
   auto kern = skinny_wide_kernel<EPI, MT, KSPLIT, NORM>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)kern, smem, limit);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((N + 8 * NT - 1) / (8 * NT), KSPLIT);

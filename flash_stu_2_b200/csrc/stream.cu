@@ -212,14 +212,9 @@ int launch_bf16(const bf16* x, long long lda, const bf16* W, long long ldb, cons
   const size_t sums = (size_t)NW * NT * 128 * 4;
   const size_t smem = groups > 1 ? ring + sums : (ring > sums ? ring : sums);
   auto k = stream_bf16_kernel<EPI, NORM, NT, D>;
-  static bool once[STU_MAX_DEVICES] = {};   // the attribute is per function and device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= STU_MAX_DEVICES || !once[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    if (dev >= 0 && dev < STU_MAX_DEVICES) once[dev] = true;
-  }
+  static SmemLimit limit;
+  const cudaError_t granted = allow_smem((const void*)k, 160 * 1024, limit);
+  if (granted != cudaSuccess) return (int)granted;
   const cudaError_t e = launch_maybe_overlapped(k, dim3(grid), dim3(THREADS), smem, st, true, x, lda, W, ldb, W2, M, N, K,
                                                 ep, nw, eps, early, groups);
   if (e != cudaSuccess) return (int)e;
@@ -412,14 +407,9 @@ int launch_f32(const float* x, long long lda, const float* W, long long ldb, con
   const int groups = ((N + grid - 1) / grid + TF - 1) / TF;
   const size_t smem = (size_t)2 * (NR + M + (NORM ? 1 : 0)) * THREADS * 16 + (size_t)groups * wk * NV * 4;
   auto k = stream_f32_kernel<EPI, NORM, NR, MM>;
-  static bool once[STU_MAX_DEVICES] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= STU_MAX_DEVICES || !once[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    if (dev >= 0 && dev < STU_MAX_DEVICES) once[dev] = true;
-  }
+  static SmemLimit limit;
+  const cudaError_t granted = allow_smem((const void*)k, 200 * 1024, limit);
+  if (granted != cudaSuccess) return (int)granted;
   const cudaError_t e = launch_maybe_overlapped(k, dim3(grid), dim3(THREADS), smem, st, true, x, lda, W, ldb, W2, M, N, K,
                                                 ep, nw, eps, early, wk);
   if (e != cudaSuccess) return (int)e;

@@ -662,13 +662,10 @@ extern "C" int stu_block_decode_step(const void* x, long long x_row_stride, cons
   // down-projection unit (8 rows of I) two
   if ((long long)32 * d > MLP_SLOT || (long long)16 * I > 2 * MLP_SLOT) return STU_ERR_UNSUPPORTED;
   const size_t smem = (size_t)STAGES * STAGE_BYTES + MLP_BYTES + (2 * STAGES + 2 * MLP_SLOTS + 2) * sizeof(uint64_t) + 1024;
-  cudaError_t e =
-      cudaFuncSetAttribute(stu_block_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)stu_block_step_kernel, smem, limit);
   if (e != cudaSuccess) return (int)e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stu_block_step_kernel, NTHREADS, smem);
-  if (e != cudaSuccess) return (int)e;
-  if (per_sm < 1) return STU_ERR_UNSUPPORTED;
+  // (a footprint that leaves no CTA per SM is refused by the cooperative launch itself)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(device_sm_count());
   cfg.blockDim = dim3(NTHREADS);

@@ -345,14 +345,14 @@ extern "C" int stu_conv_prefill_approx(const void* hist, const void* taps, void*
     if (smem > 200 * 1024) return STU_ERR_UNSUPPORTED;
     dim3 grid(d, 2 * B);
     if (dtype == STU_F32) {
-      cudaError_t e = cudaFuncSetAttribute(conv_simt_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+      static SmemLimit limit;
+      cudaError_t e = allow_smem((const void*)conv_simt_kernel<float>, smem, limit);
       if (e != cudaSuccess) return (int)e;
       conv_simt_kernel<float><<<grid, 256, smem, st>>>((const float*)hist, (const float*)taps, (float*)yT, d, Lh, y_Lh,
                                                        t0, t_end);
     } else if (dtype == STU_BF16) {
-      cudaError_t e = cudaFuncSetAttribute(conv_simt_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+      static SmemLimit limit;
+      cudaError_t e = allow_smem((const void*)conv_simt_kernel<bf16>, smem, limit);
       if (e != cudaSuccess) return (int)e;
       conv_simt_kernel<bf16><<<grid, 256, smem, st>>>((const bf16*)hist, (const bf16*)taps, (bf16*)yT, d, Lh, y_Lh, t0,
                                                       t_end);
@@ -1015,10 +1015,9 @@ static int launch_rows8(const void* x, long long x_row_stride, const void* norm_
   const size_t dsm = (size_t)8 * (Lh + 8) * sizeof(bf16);
   dim3 gd(dch / 8, (B + 7) / 8);
   const bool two_per_sm = (size_t)gd.x * gd.y > 160 && 2 * (dsm + 8 * 1024) <= (size_t)220 * 1024;
-  cudaError_t ae = two_per_sm ? cudaFuncSetAttribute(stu_decode_rows8_kernel<16>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm)
-                              : cudaFuncSetAttribute(stu_decode_rows8_kernel<32>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
+  static SmemLimit limit16, limit32;
+  cudaError_t ae = two_per_sm ? allow_smem((const void*)stu_decode_rows8_kernel<16>, dsm, limit16)
+                              : allow_smem((const void*)stu_decode_rows8_kernel<32>, dsm, limit32);
   if (ae != cudaSuccess) return (int)ae;
   cudaError_t le =
       two_per_sm ? launch_maybe_overlapped(stu_decode_rows8_kernel<16>, gd, dim3(16 * 32), dsm, st,
@@ -1078,8 +1077,8 @@ extern "C" int stu_decode_approx(const void* x, long long x_row_stride, const vo
     const size_t dsm = (size_t)(Lh + 8) * sizeof(bf16);
     if (dsm > 48 * 1024) {
       if (dsm > 200 * 1024) return STU_ERR_UNSUPPORTED;
-      cudaError_t ae = cudaFuncSetAttribute(stu_decode_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)dsm);
+      static SmemLimit limit;
+      cudaError_t ae = allow_smem((const void*)stu_decode_diag_kernel, dsm, limit);
       if (ae != cudaSuccess) return (int)ae;
     }
     cudaError_t le = launch_maybe_overlapped(stu_decode_diag_kernel, gd, dim3(256), dsm, st,
@@ -1098,8 +1097,8 @@ extern "C" int stu_decode_approx(const void* x, long long x_row_stride, const vo
       return STU_ERR_ALIGN;
     size_t smem = (size_t)(Lh + 4) * sizeof(float);
     if (smem > 200 * 1024) return STU_ERR_UNSUPPORTED;
-    cudaError_t e = cudaFuncSetAttribute(stu_decode_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    static SmemLimit limit;
+    cudaError_t e = allow_smem((const void*)stu_decode_kernel<float>, smem, limit);
     if (e != cudaSuccess) return (int)e;
     stu_decode_kernel<float><<<grid, 256, smem, st>>>((const float*)x, x_row_stride, (const float*)norm_w,
                                                       (const float*)MinT, (float*)hist, (const float*)taps, pos,
@@ -1110,8 +1109,8 @@ extern "C" int stu_decode_approx(const void* x, long long x_row_stride, const vo
       return STU_ERR_ALIGN;
     size_t smem = (size_t)(Lh + 8) * sizeof(bf16);
     if (smem > 200 * 1024) return STU_ERR_UNSUPPORTED;
-    cudaError_t e = cudaFuncSetAttribute(stu_decode_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    static SmemLimit limit;
+    cudaError_t e = allow_smem((const void*)stu_decode_kernel<bf16>, smem, limit);
     if (e != cudaSuccess) return (int)e;
     stu_decode_kernel<bf16><<<grid, 256, smem, st>>>((const bf16*)x, x_row_stride, (const bf16*)norm_w,
                                                      (const bf16*)MinT, (bf16*)hist, (const bf16*)taps, pos,

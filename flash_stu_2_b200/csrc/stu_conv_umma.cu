@@ -435,7 +435,8 @@ extern "C" int stu_conv_prefill_approx_tc5(const void* hist, const void* taps8, 
     int rc = tma::encode_bf16(&tmH, hist, 5, dims, str, box, true);
     if (rc != STU_OK) return rc;
   }
-  cudaError_t e = cudaFuncSetAttribute(conv_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)conv_umma_kernel, SMEM_BYTES, limit);
   if (e != cudaSuccess) return (int)e;
   cudaStream_t st = (cudaStream_t)stream;
   const int units = d * g.nrg;   // channel tasks; each runs its superblocks

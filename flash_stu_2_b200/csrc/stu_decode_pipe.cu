@@ -400,7 +400,8 @@ static int launch_pipe(const void* x, long long x_row_stride, const void* norm_w
   P.xp_rstride = xp_row_stride;
 
   const size_t smem = (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * sizeof(uint64_t) + 1024;
-  cudaError_t e = cudaFuncSetAttribute(stu_decode_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limit;
+  cudaError_t e = allow_smem((const void*)stu_decode_pipe_kernel, smem, limit);
   if (e != cudaSuccess) return (int)e;
   const long long rows = (long long)((B + 7) / 8) * (d_ch / 8);
   const int sms = device_sm_count();

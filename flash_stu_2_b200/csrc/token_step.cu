@@ -807,14 +807,9 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
 template <typename T, int MM>
 int launch_step(const Params& P, size_t smem, cudaStream_t st) {
   auto k = token_step_kernel<T, MM>;
-  static bool once[STU_MAX_DEVICES] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= STU_MAX_DEVICES || !once[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, STEP_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    if (dev >= 0 && dev < STU_MAX_DEVICES) once[dev] = true;
-  }
+  static SmemLimit limit;
+  const cudaError_t granted = allow_smem((const void*)k, STEP_SMEM, limit);
+  if (granted != cudaSuccess) return (int)granted;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(device_sm_count());
   cfg.blockDim = dim3(THREADS);

@@ -4,7 +4,7 @@ import torch
 import torch.nn as nn
 
 from . import ops
-from .modules import MLP, STU, Attention, RMSNorm
+from .modules import MLP, STU, Attention, RMSNorm, child, host_pos, param, uniform_pos
 
 
 def _inplace_target(x: torch.Tensor):
@@ -42,9 +42,9 @@ class STULayer(nn.Module):
         history partial sums of the NEXT position in a workspace kept with the cache's position tensor; when the
         workspace holds none for the current position (first step after a prefill, a rewound or reordered cache) a
         mode-1 launch computes them first."""
-        from .modules import host_pos
         hist, pos = entry
-        stu = self.stu
+        stu, mlp = child(self, "stu"), child(self, "mlp")
+        stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
         MinT, taps, taps8 = stu.prepared()
         B, d = x2.shape
         t = host_pos(pos)
@@ -52,14 +52,15 @@ class STULayer(nn.Module):
             raise ValueError(f"sequence position {t + 1} exceeds the capacity {stu.capacity} (seq_len={stu.seq_len})")
         ahead = getattr(pos, "_ahead", None)
         if ahead is None or ahead[0].device != x2.device:
-            ahead = [ops.block_step_workspace(d, self.mlp.intermediate_size, x2.device), 0 if t == 0 else -1]
+            ahead = [ops.block_step_workspace(d, mlp.intermediate_size, x2.device), 0 if t == 0 else -1]
             pos._ahead = ahead
         ws = ahead[0]
-        args = (x2, self.stu_norm.weight, MinT, hist, taps8, pos, self.mlp_norm.weight, self.mlp.gate_proj.weight,
-                self.mlp.up_proj.weight, self.mlp.down_proj.weight, x2, ws)
+        args = (x2, param(stu_norm, "weight"), MinT, hist, taps8, pos, param(mlp_norm, "weight"),
+                param(child(mlp, "gate_proj"), "weight"), param(child(mlp, "up_proj"), "weight"),
+                param(child(mlp, "down_proj"), "weight"), x2, ws)
         if ahead[1] != t:
-            ops.block_decode_step(*args, mode=1, eps_stu=self.stu_norm.eps, eps_mlp=self.mlp_norm.eps)
-        ops.block_decode_step(*args, mode=0, eps_stu=self.stu_norm.eps, eps_mlp=self.mlp_norm.eps)
+            ops.block_decode_step(*args, mode=1, eps_stu=stu_norm.eps, eps_mlp=mlp_norm.eps)
+        ops.block_decode_step(*args, mode=0, eps_stu=stu_norm.eps, eps_mlp=mlp_norm.eps)
         ahead[1] = t + 1
         pos._host_t = t + 1
         return hist, pos
@@ -69,7 +70,6 @@ class STULayer(nn.Module):
         history of the hidden width.  Token steps on a bf16 batch at one position read their position on the device
         (the projection is a GEMM, the pipeline kernel appends and streams); other token steps are a one-position
         prefill, whose position is a host argument."""
-        from .modules import host_pos, uniform_pos
         B, T, d = xc.shape
         Hs = self.stu_mlp_hidden_size
         x2 = xc.view(B * T, d)
@@ -99,12 +99,12 @@ class STULayer(nn.Module):
         return entry
 
     def _can_fuse(self, x, entry):
-        from .modules import uniform_pos
         B, _, d = x.shape
         # the kernel passes the MLP weights through 32 KB shared-memory slots: 16 rows of d and 8 rows of I values
-        return (ops.fused_step and self.stu.use_approx and not self.stu.use_hankel_L and x.dtype == torch.bfloat16 and B <= 8 and d % 8 == 0
-                and d <= 1024 and self.mlp.intermediate_size <= 4096
-                and self.mlp.intermediate_size % 8 == 0 and STU.pipelined_decode and STU.tensor_core_decode
+        stu, mlp = child(self, "stu"), child(self, "mlp")
+        return (ops.fused_step and stu.use_approx and not stu.use_hankel_L and x.dtype == torch.bfloat16 and B <= 8 and d % 8 == 0
+                and d <= 1024 and mlp.intermediate_size <= 4096
+                and mlp.intermediate_size % 8 == 0 and STU.pipelined_decode and STU.tensor_core_decode
                 and STU.shared_tap_decode and uniform_pos(entry[1]))
 
     def _decode(self, x, entry):
@@ -116,16 +116,17 @@ class STULayer(nn.Module):
             self._scratch = {key: torch.empty(B, d, dtype=x.dtype, device=x.device)}
         mid = self._scratch[key]
         x2 = x.view(B, d)
-        if self.stu.use_approx:
-            entry = self.stu.decode_step(x2, self.stu_norm.weight, self.stu_norm.eps, entry, mid)
+        stu, mlp = child(self, "stu"), child(self, "mlp")
+        stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
+        if stu.use_approx:
+            entry = stu.decode_step(x2, param(stu_norm, "weight"), stu_norm.eps, entry, mid)
         else:
-            xn = ops.rmsnorm(x2, self.stu_norm.weight, self.stu_norm.eps)
-            entry = self.stu.full_decode_step(xn, x2, mid, entry)
-        inter = self.mlp.intermediate_size
-        if ops.can_fuse_norm(B, inter, d, ops.EPI_GELU_MUL, x.dtype):
-            self.mlp.apply_residual(mid, mid, x2, norm_w=self.mlp_norm.weight, eps=self.mlp_norm.eps, overlap=True)
+            xn = ops.rmsnorm(x2, param(stu_norm, "weight"), stu_norm.eps)
+            entry = stu.full_decode_step(xn, x2, mid, entry)
+        if ops.can_fuse_norm(B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype):
+            mlp.apply_residual(mid, mid, x2, norm_w=param(mlp_norm, "weight"), eps=mlp_norm.eps, overlap=True)
         else:
-            self.mlp.apply_residual(ops.rmsnorm(mid, self.mlp_norm.weight, self.mlp_norm.eps), mid, x2, overlap=True)
+            mlp.apply_residual(ops.rmsnorm(mid, param(mlp_norm, "weight"), mlp_norm.eps), mid, x2, overlap=True)
         return entry
 
     def forward(self, x: torch.Tensor, past_key_value=None, use_cache=False):
@@ -138,11 +139,12 @@ class STULayer(nn.Module):
         elif T == 1 and past_key_value is not None:
             entry = self._decode(xc, past_key_value)
         else:
-            xn = ops.rmsnorm(xc, self.stu_norm.weight, self.stu_norm.eps)
-            entry = self.stu.add_to_residual(xn, xc, past_key_value, use_cache)
+            stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
+            xn = ops.rmsnorm(xc, param(stu_norm, "weight"), stu_norm.eps)
+            entry = child(self, "stu").add_to_residual(xn, xc, past_key_value, use_cache)
             x2 = xc.view(B * T, d)
-            xn2 = ops.rmsnorm(x2, self.mlp_norm.weight, self.mlp_norm.eps)
-            self.mlp.apply_residual(xn2, x2, x2)
+            xn2 = ops.rmsnorm(x2, param(mlp_norm, "weight"), mlp_norm.eps)
+            child(self, "mlp").apply_residual(xn2, x2, x2)
         if xc is not x:
             x.copy_(xc)
         if use_cache:
@@ -163,19 +165,19 @@ class AttentionLayer(nn.Module):
         xc = _inplace_target(x)
         B, T, d = xc.shape
         x2 = xc.view(B * T, d)
+        attn, mlp = child(self, "attn"), child(self, "mlp")
+        attn_norm, mlp_norm = child(self, "attn_norm"), child(self, "mlp_norm")
         if T == 1 and ops.can_fuse_norm(B, 3 * d, d, ops.EPI_STORE, x.dtype):
-            y, entry = self.attn.attend(xc, past_key_value, use_cache, norm_w=self.attn_norm.weight,
-                                        eps=self.attn_norm.eps)
+            y, entry = attn.attend(xc, past_key_value, use_cache, norm_w=param(attn_norm, "weight"), eps=attn_norm.eps)
         else:
-            xn = ops.rmsnorm(xc, self.attn_norm.weight, self.attn_norm.eps)
-            y, entry = self.attn.attend(xn, past_key_value, use_cache)
+            xn = ops.rmsnorm(xc, param(attn_norm, "weight"), attn_norm.eps)
+            y, entry = attn.attend(xn, past_key_value, use_cache)
         ov = ops.FLAG_OVERLAP if (T == 1 and ops.overlap_decode) else 0   # token step: weights fetched early
-        ops.linear(y.view(B * T, d), self.attn.c_proj.weight, resid=x2, out=x2, epilogue=ops.EPI_RESID | ov)
-        inter = self.mlp.intermediate_size
-        if T == 1 and ops.can_fuse_norm(B, inter, d, ops.EPI_GELU_MUL, x.dtype):
-            self.mlp.apply_residual(x2, x2, x2, norm_w=self.mlp_norm.weight, eps=self.mlp_norm.eps, overlap=True)
+        ops.linear(y.view(B * T, d), param(child(attn, "c_proj"), "weight"), resid=x2, out=x2, epilogue=ops.EPI_RESID | ov)
+        if T == 1 and ops.can_fuse_norm(B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype):
+            mlp.apply_residual(x2, x2, x2, norm_w=param(mlp_norm, "weight"), eps=mlp_norm.eps, overlap=True)
         else:
-            self.mlp.apply_residual(ops.rmsnorm(x2, self.mlp_norm.weight, self.mlp_norm.eps), x2, x2, overlap=(T == 1))
+            mlp.apply_residual(ops.rmsnorm(x2, param(mlp_norm, "weight"), mlp_norm.eps), x2, x2, overlap=(T == 1))
         if xc is not x:
             x.copy_(xc)
         if use_cache:

@@ -56,6 +56,20 @@ def uniform_pos(pos: torch.Tensor) -> bool:
     return getattr(pos, "_uniform", False)
 
 
+def param(module: nn.Module, name: str):
+    """A parameter or buffer of a module.  nn.Module's attribute look-up runs in the interpreter for every one of them, two
+    dozen times per token step of a layer; replaced parameters (parametrisations) still go through it."""
+    t = module._parameters.get(name)
+    if t is None:
+        t = module._buffers.get(name)
+    return t if t is not None else getattr(module, name)
+
+
+def child(module: nn.Module, name: str) -> nn.Module:
+    m = module._modules.get(name)
+    return m if m is not None else getattr(module, name)
+
+
 class RMSNorm(nn.Module):
     """torch.nn.RMSNorm(dim, dtype) arithmetic (the reference's non-Triton branch,
     flash_stu/layers/stu_layer.py:17-36): fp32 statistics, eps = finfo(float32).eps."""
@@ -89,12 +103,13 @@ class MLP(nn.Module):
         """out = resid + down(gelu(gate(xn)) * up(xn)); with norm_w, xn is RMS-normalised inside the kernel.
         overlap (decode steps): both kernels fetch their weights while the kernel before them is still running."""
         ov = ops.FLAG_OVERLAP if (overlap and ops.overlap_decode) else 0
-        h = ops.linear(xn2d, self.gate_proj.weight, W2=self.up_proj.weight, epilogue=ops.EPI_GELU_MUL | ov,
-                       norm_w=norm_w, eps=eps)
+        h = ops.linear(xn2d, param(child(self, "gate_proj"), "weight"), W2=param(child(self, "up_proj"), "weight"),
+                       epilogue=ops.EPI_GELU_MUL | ov, norm_w=norm_w, eps=eps)
         # early_decode: the down projection releases its successor at once, so that an STU decode kernel that follows
         # streams its history while this kernel runs (the successor's projection still waits for this output)
         ovd = ov | (ops.FLAG_EARLY_TRIGGER if (ov and ops.early_decode) else 0)
-        return ops.linear(h, self.down_proj.weight, resid=resid2d, out=out2d, epilogue=ops.EPI_RESID | ovd)
+        return ops.linear(h, param(child(self, "down_proj"), "weight"), resid=resid2d, out=out2d,
+                          epilogue=ops.EPI_RESID | ovd)
 
     def forward(self, x):
         x2 = x.reshape(-1, x.shape[-1])
@@ -143,7 +158,7 @@ class STU(nn.Module):
     # ---- derived, cached per parameter version: M_inputs^T (K-major rows) and the even-tap table
     @property
     def seq_len(self) -> int:
-        return self.phi.shape[0]
+        return param(self, "phi").shape[0]
 
     @property
     def capacity(self) -> int:
@@ -157,8 +172,8 @@ class STU(nn.Module):
     def prepared(self):
         if not self.use_approx:
             return self.prepared_full()
-        key = (self.M_inputs._version, self.M_filters._version, self.phi._version, self.M_inputs.data_ptr(),
-               self.M_filters.data_ptr(), self.phi.data_ptr())
+        M_inputs, M_filters, phi = param(self, "M_inputs"), param(self, "M_filters"), param(self, "phi")
+        key = (M_inputs._version, M_filters._version, phi._version, M_inputs.data_ptr(), M_filters.data_ptr(), phi.data_ptr())
         if self._prep_key != key:
             with torch.no_grad():
                 # only the taps of positions a cache can hold are ever used
@@ -189,8 +204,9 @@ class STU(nn.Module):
     def prepared_full(self):
         """(phi [L,K] contiguous in the model dtype, Mcat [d_out, nsign*K*d_in]): the two M_phi tensors as one
         K-major weight whose column order (sign, k, i) matches the U operand the kernels build."""
-        mats = [self.M_phi_plus] + ([] if self.use_hankel_L else [self.M_phi_minus])
-        key = tuple(m._version for m in mats) + tuple(m.data_ptr() for m in mats) + (self.phi._version, self.phi.data_ptr())
+        mats = [param(self, "M_phi_plus")] + ([] if self.use_hankel_L else [param(self, "M_phi_minus")])
+        phi = param(self, "phi")
+        key = tuple(m._version for m in mats) + tuple(m.data_ptr() for m in mats) + (phi._version, phi.data_ptr())
         if self._prep_key != key:
             with torch.no_grad():
                 phi = self.phi.to(self.M_phi_plus.dtype).contiguous()
@@ -432,11 +448,12 @@ class Attention(nn.Module):
         """Heads merged, before c_proj: returns (y [B,T,d], entry).  With norm_w, xn is the un-normalised layer input
         and the RMSNorm is applied inside the c_attn kernel (token steps)."""
         B, T, d = xn.shape
+        c_attn = param(child(self, "c_attn"), "weight")
         if norm_w is not None:
-            qkv = ops.linear(xn.reshape(B * T, d), self.c_attn.weight, norm_w=norm_w, eps=eps).view(B, T, 3 * d)
+            qkv = ops.linear(xn.reshape(B * T, d), c_attn, norm_w=norm_w, eps=eps).view(B, T, 3 * d)
         else:
             ov = ops.FLAG_OVERLAP if (T == 1 and ops.overlap_decode) else 0   # token step: weights fetched early
-            qkv = ops.linear(xn.reshape(B * T, d), self.c_attn.weight, epilogue=ops.EPI_STORE | ov).view(B, T, 3 * d)
+            qkv = ops.linear(xn.reshape(B * T, d), c_attn, epilogue=ops.EPI_STORE | ov).view(B, T, 3 * d)
         if entry is None and use_cache:
             entry = self.new_cache(B, xn.device)
         if entry is not None:

@@ -61,7 +61,8 @@ def _cuda(*ts):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # (the stream's address without building a Stream object: a microsecond of every launch)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _p(t: Optional[torch.Tensor]):
@@ -69,6 +70,9 @@ def _p(t: Optional[torch.Tensor]):
 
 
 def status_word(device) -> torch.Tensor:
+    word = _status.get(device.index) if isinstance(device, torch.device) else None
+    if word is not None:
+        return word
     dev = torch.device(device)
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     if key not in _status:
