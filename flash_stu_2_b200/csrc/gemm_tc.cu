@@ -27,6 +27,7 @@ namespace {
 
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
+constexpr int SROW = 72;   // row distance of the epilogue's staging block: 16-byte accesses by rows and by columns conflict-free
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 enum { EPI_HIST_T = 4 };  // internal: rows = channels, columns = tokens (operands swapped by the host)
 
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* issued_ctr = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));
   int* consumed_ctr = issued_ctr + 1;
-  uint32_t* row_stage = reinterpret_cast<uint32_t*>(smem + STAGES * STAGE_BYTES + 256);   // [4][32][17], EPI_STORE and EPI_HIST_T
+  bf16* row_stage = reinterpret_cast<bf16*>(smem + STAGES * STAGE_BYTES + 256);   // [4 warps][32][SROW]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = tiles_m * tiles_n;
@@ -275,17 +276,22 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
   } else {
     // ---------------- epilogue warps: TMEM lane quarter = warp % 4
     const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    // output that is off the 16-byte grid goes through shared memory: plain rows of any stride, and histories whose
-    // sequences or first position are no multiple of a 32-column block
+    // The accumulator leaves in blocks of 32 rows x 64 columns per warp, through shared memory: a thread holds a row, but
+    // 16-byte stores by 32 threads to 32 rows cost 32 half-used sectors per instruction (4.6 us per 128 x 256 tile, more
+    // than its main loop below K = 768); 8 threads per row write whole lines.  Residual rows are read the same way, all
+    // eight loads ahead of the first use.  Histories (rows are channels, columns tokens): the even and the odd tokens of a
+    // block are 32 values each in their parity rows.
+    // Off the 16-byte grid (plain rows of any stride; histories whose sequences, first position or pitch are no multiples
+    // of the blocks) lanes store single values, side by side.
     const bool unaligned = EPI == EPI_STORE ? ((ep.ldy & 7) || (reinterpret_cast<uintptr_t>(ep.y) & 15))
-                                            : EPI == EPI_HIST_T && ((ep.Tseq & 31) || (ep.t0 & 15) || (ep.Lh & 7));
+                                            : EPI == EPI_HIST_T && ((ep.Tseq & 15) || (ep.t0 & 15) || (ep.Lh & 7));
+    bf16* st = row_stage + quarter * (32 * SROW);
     int it = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, it++) {
       int tm, tn;
       tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = tm * BM, n0 = tn * BN;
-      const int m = m0 + row;
+      const int first = m0 + quarter * 32, rows = min(32, M - first);   // this warp's rows
       const int buf = it & 1;
       const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
       bool ok = mbar_wait(&tmem_full[buf], ((uint32_t)it >> 1) & 1u, abort_flag, wait_ns);
@@ -293,115 +299,113 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-      for (int cch = 0; cch < BN / 32; cch++) {
-        uint32_t r[32], r2[32];
-        const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cch * 32);
-        tmem_ld32(taddr, r);
-        if (DUAL) tmem_ld32(taddr + BN, r2);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int nb = n0 + cch * 32;
-        if (unaligned) {
-          // the warp's 32 x 32 block leaves row by row: 64 consecutive bytes per store instruction, in a history (a row
-          // is a channel, a lane a token) 32 in each parity row.  (Stored by the threads that hold the rows, 2 bytes to
-          // each of 32 rows per instruction, the projection of 4 x 1999 tokens into a 1024-wide history took 90 us.)
-          uint32_t* st = row_stage + quarter * (32 * 17);
-          __syncwarp();
+      for (int nb = n0; nb < min(n0 + BN, N); nb += 64) {
+        const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {   // 32 columns of this thread's row
+          uint32_t r[32], r2[32];
+          tmem_ld32(taddr + h * 32, r);
+          if (DUAL) tmem_ld32(taddr + BN + h * 32, r2);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          bf16* dst = st + lane * SROW;
+          if (EPI == EPI_HIST_T && !unaligned) {
+            float par[2][16];
 #pragma unroll
-          for (int j = 0; j < 16; j++) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-            st[lane * 17 + j] = *reinterpret_cast<uint32_t*>(&h);
-          }
-          __syncwarp();
-          const bf16* col = reinterpret_cast<const bf16*>(st) + lane;
-          const int first = m0 + quarter * 32, rows = min(32, M - first), n = nb + lane;
-          if (n < N) {
-            bf16* yc;
-            size_t pitch;
-            if (EPI == EPI_HIST_T) {
-              const int b = n / ep.Tseq;
-              yc = ep.y + hist_off(b, first, ep.t0 + (n - b * ep.Tseq), (int)ep.ldy, ep.Lh);
-              pitch = (size_t)2 * ep.Lh;
-            } else {
-              yc = ep.y + (size_t)first * ep.ldy + n;
-              pitch = (size_t)ep.ldy;
-            }
-#pragma unroll 8
-            for (int i = 0; i < rows; i++) yc[i * pitch] = col[i * 34];
-          }
-        } else if (m < M && nb < N) {
-          if (EPI == EPI_HIST_T) {
-            // row m = channel, columns = tokens nb..nb+31 of the flattened [B, T] batch
-            const int d = (int)ep.ldy;
-            const bool fast = nb + 32 <= N;   // (the rest of the alignment: see `unaligned`)
-            if (fast) {
-              const int b = nb / ep.Tseq, t = ep.t0 + (nb - b * ep.Tseq);  // t % 16 == 0
-              float ev[16], od[16];
+            for (int j = 0; j < 32; j++) par[j & 1][j >> 1] = __uint_as_float(r[j]);
 #pragma unroll
-              for (int j = 0; j < 16; j++) {
-                ev[j] = __uint_as_float(r[2 * j]);
-                od[j] = __uint_as_float(r[2 * j + 1]);
-              }
-              bf16* pe = ep.y + ((size_t)((size_t)b * d + m) * 2 + 0) * ep.Lh + (t >> 1);
-              bf16* po = ep.y + ((size_t)((size_t)b * d + m) * 2 + 1) * ep.Lh + (t >> 1);
-              store_vec(pe, ev);
-              store_vec(pe + 8, ev + 8);
-              store_vec(po, od);
-              store_vec(po + 8, od + 8);
-            } else {
-              for (int j = 0; j < 32; j++) {
-                int n = nb + j;
-                if (n < N) {
-                  int b = n / ep.Tseq, t = ep.t0 + (n - b * ep.Tseq);
-                  ep.y[hist_off(b, m, t, d, ep.Lh)] = __float2bfloat16_rn(__uint_as_float(r[j]));
-                }
-              }
+            for (int q = 0; q < 2; q++) {
+              store_vec(dst + q * 32 + h * 16, par[q]);
+              store_vec(dst + q * 32 + h * 16 + 8, par[q] + 8);
             }
           } else {
-            bf16* yrow = ep.y + (size_t)m * ep.ldy + nb;
-            if (EPI == EPI_BLOCKCOL)   // columns in blocks of Tseq, ld2 elements apart
-              yrow = ep.y + (size_t)m * ep.ldy + (size_t)(nb / ep.Tseq) * ep.ld2 + (nb % ep.Tseq);
-            const bf16* rrow = (EPI == EPI_RESID) ? ep.resid + (size_t)m * ep.ldr + nb : nullptr;
-            const bool vec = (nb + 32 <= N) && (EPI != EPI_BLOCKCOL || ep.Tseq % 32 == 0);
 #pragma unroll
             for (int v8 = 0; v8 < 4; v8++) {
               float o[8];
-              if (EPI == EPI_RESID) {
-                float rs[8];
-                if (vec) {
-                  load_vec(rrow + v8 * 8, rs);
-                } else {
 #pragma unroll
-                  for (int j = 0; j < 8; j++) rs[j] = (nb + v8 * 8 + j < N) ? __bfloat162float(rrow[v8 * 8 + j]) : 0.f;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++) o[j] = rs[j] + round_to<bf16>(__uint_as_float(r[v8 * 8 + j]));
-              } else if (EPI == EPI_GELU_MUL) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                  float gte = round_to<bf16>(gelu_tanh_fast(round_to<bf16>(__uint_as_float(r[v8 * 8 + j]))));
-                  o[j] = gte * round_to<bf16>(__uint_as_float(r2[v8 * 8 + j]));
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++) o[j] = __uint_as_float(r[v8 * 8 + j]);
+              for (int j = 0; j < 8; j++) {
+                o[j] = __uint_as_float(r[v8 * 8 + j]);
+                if (EPI == EPI_GELU_MUL)
+                  o[j] = round_to<bf16>(gelu_tanh_fast(round_to<bf16>(o[j]))) *
+                         round_to<bf16>(__uint_as_float(r2[v8 * 8 + j]));
               }
-              if (vec) {
-                store_vec(yrow + v8 * 8, o);
-              } else if (EPI == EPI_BLOCKCOL) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                  const int n = nb + v8 * 8 + j;
-                  if (n < N)
-                    ep.y[(size_t)m * ep.ldy + (size_t)(n / ep.Tseq) * ep.ld2 + (n % ep.Tseq)] = __float2bfloat16_rn(o[j]);
-                }
+              store_vec(dst + h * 32 + v8 * 8, o);
+            }
+          }
+          if (unaligned) {   // 32 columns at a time: the stores of one half run beside the accumulator read of the next
+            __syncwarp();
+            const int n = nb + h * 32 + lane;
+            if (n < N) {
+              const bf16* col = st + h * 32 + lane;
+              if (EPI == EPI_HIST_T) {
+                const int b = n / ep.Tseq, pitch = 2 * ep.Lh;
+                bf16* yc = ep.y + hist_off(b, first, ep.t0 + (n - b * ep.Tseq), (int)ep.ldy, ep.Lh);
+#pragma unroll 8
+                for (int i = 0; i < rows; i++) yc[(size_t)i * pitch] = col[i * SROW];
               } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                  if (nb + v8 * 8 + j < N) yrow[v8 * 8 + j] = __float2bfloat16_rn(o[j]);
+                bf16* yc = ep.y + (size_t)first * ep.ldy + n;
+#pragma unroll 8
+                for (int i = 0; i < rows; i++) yc[(size_t)i * ep.ldy] = col[i * SROW];
               }
             }
           }
         }
+        __syncwarp();
+        if (!unaligned) {
+          const int piece = lane & 7, r0 = lane >> 3;   // 8 values of row r0, r0 + 4, ...
+          const int n = nb + piece * 8;
+          if (EPI == EPI_HIST_T) {
+            const int nt = nb + (piece & 3) * 16;   // first of the 16 tokens whose even or odd half this is
+            if (nt < N) {
+              const int b = nt / ep.Tseq, t = ep.t0 + (nt - b * ep.Tseq);
+              bf16* yc = ep.y + (((size_t)b * ep.ldy + first) * 2 + (piece >> 2)) * ep.Lh + (t >> 1);
+#pragma unroll
+              for (int i = 0; i < 8; i++)
+                if (r0 + i * 4 < rows)
+                  *reinterpret_cast<uint4*>(yc + (size_t)(r0 + i * 4) * 2 * ep.Lh) =
+                      *reinterpret_cast<const uint4*>(st + (r0 + i * 4) * SROW + piece * 8);
+            }
+          } else if (n + 8 <= N) {
+            bf16* yc = ep.y + (size_t)(first + r0) * ep.ldy +
+                       (EPI == EPI_BLOCKCOL ? (size_t)(n / ep.Tseq) * ep.ld2 + n % ep.Tseq : (size_t)n);   // Tseq % 8 == 0
+            if (EPI == EPI_RESID) {
+              const bf16* rc = ep.resid + (size_t)(first + r0) * ep.ldr + n;
+              uint4 res[8];
+#pragma unroll
+              for (int i = 0; i < 8; i++)
+                res[i] = r0 + i * 4 < rows ? *reinterpret_cast<const uint4*>(rc + (size_t)(i * 4) * ep.ldr)
+                                           : make_uint4(0, 0, 0, 0);
+#pragma unroll
+              for (int i = 0; i < 8; i++)
+                if (r0 + i * 4 < rows) {
+                  float o[8], rs[8];
+                  load_vec(st + (r0 + i * 4) * SROW + piece * 8, o);
+                  load_vec(reinterpret_cast<const bf16*>(&res[i]), rs);
+#pragma unroll
+                  for (int j = 0; j < 8; j++) o[j] += rs[j];
+                  store_vec(yc + (size_t)(i * 4) * ep.ldy, o);
+                }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; i++)
+                if (r0 + i * 4 < rows)
+                  *reinterpret_cast<uint4*>(yc + (size_t)(i * 4) * ep.ldy) =
+                      *reinterpret_cast<const uint4*>(st + (r0 + i * 4) * SROW + piece * 8);
+            }
+          } else {   // the last columns of a width that is no multiple of 8
+            for (int j = n; j < min(n + 8, N); j++)
+              for (int i = r0; i < rows; i += 4) {
+                const bf16 v = st[i * SROW + (j - nb)];
+                const size_t m = (size_t)(first + i);
+                if (EPI == EPI_RESID)
+                  ep.y[m * ep.ldy + j] = __float2bfloat16_rn(__bfloat162float(ep.resid[m * ep.ldr + j]) + __bfloat162float(v));
+                else if (EPI == EPI_BLOCKCOL)
+                  ep.y[m * ep.ldy + (size_t)(j / ep.Tseq) * ep.ld2 + j % ep.Tseq] = v;
+                else
+                  ep.y[m * ep.ldy + j] = v;
+              }
+          }
+        }
+        __syncwarp();   // the block has been read
       }
       // this thread's TMEM reads of the buffer are complete (wait::ld above): hand it back to the MMA warp
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -525,7 +529,7 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
   constexpr int BN = TN;
   constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2 * (DUAL ? 2 : 1);
-  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + (EPI == EPI_STORE || EPI == EPI_HIST_T ? 4 * 32 * 17 * 4 : 0);
+  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + 4 * 32 * SROW * sizeof(bf16);
   auto k = gemm_tc_kernel<EPI, STAGES, TN>;
   static SmemLimit limit;
   cudaError_t e = allow_smem((const void*)k, smem, limit);
