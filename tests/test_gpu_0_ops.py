@@ -842,6 +842,33 @@ def test_sampling_row_with_a_nan_logit_draws_uniformly():
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [4096, 4099, 50257, 65536])
+def test_sampling_by_a_cluster_equals_one_cta_per_row(dt, V):
+    """Up to 64 rows the greedy pick and a top-k of at most 256 run on a cluster of CTAs per row, more rows on one CTA per
+    row: the same tokens, with infinities, NaN, ties across the k-th place and more ties than the candidate list holds."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(10)
+    B = 65
+    z = torch.randn(B, V + 3) * 3
+    z[1, 5], z[2, 7], z[3, :] = float("nan"), float("inf"), -float("inf")
+    z[3, ::100] = torch.randn(z[3, ::100].shape)
+    z[4, 100:160] = 20.0
+    if V <= 51712:   # (a wider row with more ties than the list holds is refused with a status)
+        z[5, :] = 1.5
+        z[6, ::2] = 30.0
+    z = z.to(dt).to(dev())[:, :V]
+    u = torch.rand(B, device=dev())
+    u[7], u[8] = 0.0, 1.0 - 2 ** -24
+    for temp, k, p in [(1.0, None, None), (0.8, 40, None), (0.9, 100, 0.9), (1.0, 256, 0.5), (1.0, 1, None), (1.3, 50, 1.0)]:
+        one, many = (torch.full((n,), -1, dtype=torch.int64, device=dev()) for n in (B, 33))
+        ops.sample(z, temp, k, p, k is not None, u, one)
+        ops.sample(z[:33], temp, k, p, k is not None, u[:33], many)
+        ops.check_status()
+        assert torch.equal(one[:33], many), (temp, k, p)
+        assert bool((many >= 0).all()) and bool((many < V).all())
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_full_variant_building_blocks(dt):
     """to_history, the three Toeplitz matrices, the causal GEMM flag and the combine step against plain torch."""
     from flash_stu_2_b200 import ops
