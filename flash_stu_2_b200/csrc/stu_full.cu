@@ -72,17 +72,38 @@ extern "C" int stu_to_history(const void* x, long long x_bstride, long long x_ts
 //   kind 2 (odd taps, outputs of parity 0 from inputs of parity 1)   Tz[m][s] = f[2(m-s)-1]   m >  s
 // (time t = 2m+p reads input time t-j = 2s+p'; the tap index j follows.)  Entries past L and above the
 // diagonal are zero.
+//
+// Bound: the 3 S^2 values written.  A CTA writes 32 rows x 1024 columns: a row is the reversed filter at another offset,
+// so the filter's values are gathered once, into as many copies, each shifted by one value, as there are values in 16
+// bytes, and every row is 16-byte reads of the copy that its offset makes aligned and 16-byte stores.  (One value per
+// thread, gathered from the filter column each, took 18 us for S = 1504 in bf16.)
+constexpr int TZ_ROWS = 32, TZ_COLS = 1024;
 template <typename T>
-__global__ void toeplitz_kernel(const T* __restrict__ f, long long f_stride, int L, T* __restrict__ out, int S,
-                                long long ld) {
-  const int kind = blockIdx.z;
-  T* o = out + (size_t)kind * S * ld;
-  const int m = blockIdx.y;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
-    int j = 2 * (m - s) + (kind == 0 ? 0 : (kind == 1 ? 1 : -1));
-    T v = Elem<T>::from_f(0.f);
-    if (m >= s && j >= 0 && j < L) v = f[(size_t)j * f_stride];
-    o[(size_t)m * ld + s] = v;
+__global__ void __launch_bounds__(256) toeplitz_kernel(const T* __restrict__ f, long long f_stride, int L,
+                                                       T* __restrict__ out, int S, long long ld, int vec) {
+  constexpr int V = Elem<T>::VEC;
+  __shared__ __align__(16) T tab[V][TZ_COLS + TZ_ROWS];   // tab[c][y]: the value at m - s = m_last - s0 - (y + c)
+  const int kind = blockIdx.z, m0 = blockIdx.y * TZ_ROWS, s0 = blockIdx.x * TZ_COLS;
+  for (int y = threadIdx.x; y < TZ_COLS + TZ_ROWS; y += 256) {
+    const int i = m0 + TZ_ROWS - 1 - (s0 + y), j = 2 * i + (kind == 0 ? 0 : (kind == 1 ? 1 : -1));
+    const T v = i >= 0 && j >= 0 && j < L ? f[(size_t)j * f_stride] : Elem<T>::from_f(0.f);
+#pragma unroll
+    for (int c = 0; c < V; c++)
+      if (y >= c) tab[c][y - c] = v;
+  }
+  __syncthreads();
+  T* o = out + (size_t)kind * S * ld + s0;
+  const int cols = min(TZ_COLS, S - s0), rows = min(TZ_ROWS, S - m0);
+  for (int e = threadIdx.x; e < rows * (TZ_COLS / V); e += 256) {
+    const int r = e / (TZ_COLS / V), s = e % (TZ_COLS / V) * V, off = TZ_ROWS - 1 - r;   // row m0 + r starts at tab[0][off]
+    if (s >= cols) continue;
+    const T* src = &tab[off % V][s + off - off % V];
+    T* dst = o + (size_t)(m0 + r) * ld + s;
+    if (vec && s + V <= cols) {
+      *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+    } else {
+      for (int x = 0; x < V && s + x < cols; x++) dst[x] = src[x];
+    }
   }
 }
 
@@ -91,11 +112,14 @@ extern "C" int stu_toeplitz(const void* f, long long f_stride, int L, void* out,
   if (!f || !out) return STU_ERR_NULL;
   if (L <= 0 || S <= 0 || ld < S) return STU_ERR_SHAPE;
   cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid((S + 255) / 256 < 16 ? (S + 255) / 256 : 16, S, 3);
+  const long long rows = (S + TZ_ROWS - 1) / TZ_ROWS;
+  if (rows > 65535) return STU_ERR_UNSUPPORTED;
+  const dim3 grid((S + TZ_COLS - 1) / TZ_COLS, (unsigned)rows, 3);
+  const int vec = aligned16(out) && ld % (dtype == STU_F32 ? 4 : 8) == 0;
   if (dtype == STU_F32)
-    toeplitz_kernel<float><<<grid, 256, 0, st>>>((const float*)f, f_stride, L, (float*)out, S, ld);
+    toeplitz_kernel<float><<<grid, 256, 0, st>>>((const float*)f, f_stride, L, (float*)out, S, ld, vec);
   else if (dtype == STU_BF16)
-    toeplitz_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)f, f_stride, L, (bf16*)out, S, ld);
+    toeplitz_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)f, f_stride, L, (bf16*)out, S, ld, vec);
   else
     return STU_ERR_DTYPE;
   STU_CHECK_LAUNCH();
