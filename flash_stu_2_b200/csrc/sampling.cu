@@ -466,7 +466,8 @@ __global__ void __launch_bounds__(SP_T) sample_kernel(const T* __restrict__ logi
 // in 49 steps per pass, six passes.  Here a thread holds at most 8 entries, in registers, read once; the four radix
 // passes add the CTAs' histograms through distributed shared memory, every CTA for itself, and the survivors meet in
 // CTA 0, which cuts and draws as sample_row does: the same token.  More survivors than the list holds (ties): CTA 0
-// runs sample_row.  50257 entries: top-k 100 with a nucleus 79 -> 27 us, greedy fp32 17 -> 7.5 us.
+// runs sample_row.  50257 entries: top-k 100 with a nucleus 79 -> 27 us, 32 rows
+// of top-k 40 97 -> 38 us, greedy fp32 17 -> 7.5 us.
 constexpr int SPC = 8, SPC_PER = 8, SPC_TOPK = 256;
 constexpr int SPC_MAX_V = SPC * SP_T * SPC_PER;
 template <typename T>
@@ -619,9 +620,9 @@ extern "C" int stu_sample(const void* logits, long long ld, int B, int V, float 
   // greedy selection makes one pass only: nothing to keep
   const int cache = (do_sample && V <= SP_CACHE_MAX) ? 1 : 0;
   static const int variant = getenv("STU_SAMPLE_VARIANT") ? atoi(getenv("STU_SAMPLE_VARIANT")) : 2;
-  // A cluster per row where its 8 CTAs of all rows are resident together twice over at most (64 rows: 512 CTAs, two per
-  // SM) and the row fits its registers; shorter rows than 4096 are one CTA's work, and past SPC_TOPK the survivors of a
-  // bf16 row may well exceed the list.
+  // A cluster per row for up to 64 rows (512 CTAs, two per SM: under two rounds of 27 to 38 us against one of 80 to 100),
+  // where the row fits the cluster's registers; shorter rows than 4096 are one CTA's work, and past SPC_TOPK the survivors
+  // of a bf16 row may well exceed the list.
   if (V >= 4096 && V <= SPC_MAX_V && B <= 64 && (!do_sample || (top_k > 0 && top_k <= SPC_TOPK))) {
     const int full = V <= SP_CACHE_MAX;
     if (dtype == STU_F32)
