@@ -75,6 +75,7 @@ _SIGNATURES = {
     "stu_token_step_supported": ([c_int, c_int, c_int, c_int, c_int, c_int], c_int),
     "stu_token_step_plan_bytes": ([c_int], c_longlong),
     "stu_token_step_plan": ([_P, _P, c_int, _P], c_int),
+    "stu_token_step_walk": ([_P, c_int, _P, c_int], c_int),
     "stu_token_step": ([_P, c_int, _P, c_int, _P], c_int),
     "stu_to_history": ([_P, _LL, _LL, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_toeplitz": ([_P, _LL, c_int, _P, c_int, _LL, c_int, _P], c_int),

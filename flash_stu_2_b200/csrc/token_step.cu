@@ -109,8 +109,8 @@ struct Params {
   int xs_cols;         // columns of the activation rows in shared memory: max(d, I), or less, a multiple of d
   float scale;
 };
-__device__ __forceinline__ Range share_of(int N) {   // N < 2^24 (checked by the host)
-  return {(int)((unsigned)N * blockIdx.x / gridDim.x), (int)((unsigned)N * (blockIdx.x + 1) / gridDim.x)};
+__host__ __device__ inline Range share_of(int N, unsigned cta, unsigned ctas) {   // N < 2^24 (checked by the host)
+  return {(int)((unsigned)N * cta / ctas), (int)((unsigned)N * (cta + 1) / ctas)};
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -125,10 +125,18 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // fp32: warps that share a pair of rows (a power of two; the teams take the pairs in turn).
 __device__ __forceinline__ int team_warps(int rows) { return rows > 8 ? 1 : rows > 4 ? 2 : rows > 2 ? 4 : 8; }
 // `in_rows`: pieces of the activation rows that are in shared memory at a time; a unit lies inside them.
-__device__ __forceinline__ int unit_pieces(int rows, int pieces, int slots, bool packed, int in_rows) {
-  int p = packed ? max(1, min(min(pieces, in_rows), slots / (3 * rows))) : 1;
+__host__ __device__ inline int unit_pieces(int rows, int pieces, int slots, bool packed, int in_rows) {
+  int p = pieces < in_rows ? pieces : in_rows;
+  if (p > slots / (3 * rows)) p = slots / (3 * rows);
+  if (!packed || p < 1) p = 1;
   while (in_rows % p) p--;
   return p;
+}
+// Slots that a unit of n leaves unused in front of itself, from `head` to the end of the ring, because it does not wrap;
+// they count as its own until it is released.  Into an empty ring it goes without them: there they are free, and with
+// them a unit of 16 rows would fit no ring of fewer than 31 slots whenever it has to skip.
+__host__ __device__ inline int unit_skip(int head, int n, int slots, int used) {
+  return head + n > slots && used > 0 ? slots - head : 0;
 }
 template <typename T, int MM>
 __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_constant__ Params P) {
@@ -173,7 +181,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   }
   const int epoch = __ldcg(epoch_word);
   __syncthreads();
-  for (int i = tid; i < nst; i += THREADS) s_range[i] = share_of(tab[i].N);
+  for (int i = tid; i < nst; i += THREADS) s_range[i] = share_of(tab[i].N, blockIdx.x, gridDim.x);
   const int t = __ldcg(layers[0].pos);
   int bad = 0;
   for (int i = tid; i < a.n_layers * B; i += THREADS) {
@@ -205,13 +213,14 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
         const int pieces = s.pieces == 1 ? 1 : unit_pieces(rows, s.pieces, slots, packed, P.xs_cols / d);
         for (int k0 = 0, p0 = 0; k0 < s.K; k0 += pieces * d, p0 += pieces) {
           const int np = min(pieces, s.pieces - p0), n = rows * np;
-          const bool wrap = head + n > slots;
-          const int skip = wrap ? slots - head : 0;
+          const bool wrap = head + n > slots;   // (then the consumers go on at slot 0 as well)
+          int skip = unit_skip(head, n, slots, used);
           while (ok && (used + skip + n > slots || issued - freed == UNITS)) {
             ok = tma::mbar_wait_bounded(&empty_bar[freed % UNITS], (freed / UNITS) & 1u, &s_abort);
             ok = __all_sync(0xffffffffu, ok);
             used -= __shfl_sync(0xffffffffu, slots_of, freed % UNITS);
             freed++;
+            skip = unit_skip(head, n, slots, used);
           }
           if (!ok) break;
           if (wrap) head = 0;
@@ -306,7 +315,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   };
   // results: warp m finishes sequence m, lane n the features n, n + 32, ...; of the (at most 32) features of a d-wide
   // product that is one per thread, which also adds the residual
-  const Range own_r = share_of(d);
+  const Range own_r = share_of(d, blockIdx.x, gridDim.x);
   const int c0 = own_r.r0, own = own_r.r1 - c0, my_c = c0 + lane;
   const bool mine = warp < B && lane < own;
   int slot = 0;        // first slot of the next unit
@@ -856,8 +865,7 @@ extern "C" long long stu_token_step_workspace_bytes(int d, int I, int H, int dty
   return 512 + (32ll * d + 8ll * I) * e + (8ll * H + 160) * (hd + 4) * 4 + 256;
 }
 
-// 1 when stu_token_step takes a stack of these sizes, else 0.  H = 0: no attention layer.  The ring must hold a unit
-// of 16 rows and half another.
+// 1 when stu_token_step takes a stack of these sizes, else 0.  H = 0: no attention layer.
 extern "C" int stu_token_step_supported(int n_layers, int B, int d, int I, int H, int dtype) {
   if ((dtype != STU_BF16 && dtype != STU_F32) || n_layers < 1 || n_layers > MAXL) return 0;
   const int vec = dtype == STU_BF16 ? 8 : 4;
@@ -916,6 +924,46 @@ extern "C" int stu_token_step_plan(const StuStepLayer* layers, const StuStepArgs
   StuStepLayer* out = (StuStepLayer*)t;
   for (int l = 0; l < a.n_layers; l++) out[l] = layers[l];
   return nst;
+}
+
+// The producer's walk through the ring, on the host, for every CTA of the launch that stu_token_step would make of a plan
+// (in host memory): 0, or 1 + the stage at whose unit a CTA would wait for slots that nothing is left to release.
+extern "C" int stu_token_step_walk(const void* plan, int n_stages, const StuStepArgs* args, int dtype) {
+  if (!plan || !args) return STU_ERR_NULL;
+  const StuStepArgs& a = *args;
+  if (!stu_token_step_supported(a.n_layers, a.B, a.d, a.I, a.H, dtype)) return STU_ERR_UNSUPPORTED;
+  if (n_stages < 3 * a.n_layers || n_stages > 5 * a.n_layers + 1) return STU_ERR_SHAPE;
+  const Stage* tab = (const Stage*)plan;
+  const int slots = ring_slots(a.B, a.d, a.I, dtype), in_rows = held_cols(a.B, a.d, a.I, dtype) / a.d, sms = device_sm_count();
+  const bool packed = slot_pitch(a.d, dtype) == a.d * (dtype == STU_BF16 ? 2 : 4);
+  for (int cta = 0; cta < sms; cta++) {
+    int slots_of[UNITS], head = 0, used = 0;
+    unsigned issued = 0, freed = 0;
+    for (int st = 0; st < n_stages; st++) {
+      const Stage& s = tab[st];
+      if (!s.W) continue;
+      const bool dual = s.W2 != nullptr;
+      const Range r = share_of(s.N, cta, sms);
+      for (int f0 = r.r0, F = dual ? 8 : 16; f0 < r.r1; f0 += F) {
+        const int nf = F < r.r1 - f0 ? F : r.r1 - f0, rows = dual ? 2 * nf : nf;
+        const int pieces = s.pieces == 1 ? 1 : unit_pieces(rows, s.pieces, slots, packed, in_rows);
+        for (int p0 = 0; p0 < s.pieces; p0 += pieces) {
+          const int n = rows * (pieces < s.pieces - p0 ? pieces : s.pieces - p0);
+          int skip = unit_skip(head, n, slots, used);
+          while (used + skip + n > slots || issued - freed == UNITS) {
+            if (freed == issued) return st + 1;
+            used -= slots_of[freed++ % UNITS];
+            skip = unit_skip(head, n, slots, used);
+          }
+          if (head + n > slots) head = 0;
+          slots_of[issued++ % UNITS] = skip + n;
+          head += n;
+          used += skip + n;
+        }
+      }
+    }
+  }
+  return 0;
 }
 
 extern "C" int stu_token_step(const void* plan, int n_stages, const StuStepArgs* args, int dtype, void* stream) {

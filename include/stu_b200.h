@@ -408,6 +408,8 @@ int stu_token_step_supported(int n_layers, int B, int d, int I, int H, int dtype
  * error (< 0).  The caller copies it to the device once; it holds addresses, so it serves as long as they do. */
 long long stu_token_step_plan_bytes(int n_layers);
 int stu_token_step_plan(const StuStepLayer* layers, const StuStepArgs* args, int dtype, void* plan);
+/* Host check of a plan in host memory: 0, or 1 + the stage at which the weight stream of some CTA would wait for itself. */
+int stu_token_step_walk(const void* plan, int n_stages, const StuStepArgs* args, int dtype);
 int stu_token_step(const void* plan_on_device, int n_stages, const StuStepArgs* args, int dtype, void* stream);
 
 #ifdef __cplusplus

@@ -183,6 +183,13 @@ def test_token_step_kernel_against_full_prefix_logits(tmp_path, dt, B, d, heads,
     close(logits, want, 4e-5 if dt == torch.float32 else 2e-2)
 
 
+@pytest.mark.parametrize("dt,B,d,heads,mlp", [(torch.bfloat16, 1, 3072, 24, 4), (torch.bfloat16, 3, 2560, 20, 4),
+                                             (torch.bfloat16, 3, 2304, 36, 4), (torch.float32, 1, 1536, 12, 4)])
+def test_wide_models_of_few_sequences_against_full_prefix_logits(tmp_path, dt, B, d, heads, mlp):
+    """The same for models so wide that the weight ring of the token-step kernel holds fewer than two units of 16 rows."""
+    test_token_step_kernel_against_full_prefix_logits(tmp_path, dt, B, d, heads, mlp, 40, 50)
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for
