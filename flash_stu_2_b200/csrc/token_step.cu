@@ -229,7 +229,8 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
           if (lane == 0) tma::mbar_expect_tx(bar, row_bytes * rows);
           __syncwarp();
           // whole rows of a packed unit lie back to back: the gate rows (or all) and the up rows are one block each
-          const bool whole = packed && np == s.pieces;
+          // (rows that are no whole number of pieces leave the end of their slots unused: one copy per row)
+          const bool whole = packed && np == s.pieces && s.K == s.pieces * d;
           const int blocks = whole ? (dual ? 2 : 1) : rows;
           const uint32_t block = whole ? row_bytes * nf : row_bytes;
           const int cuts = (int)((block + COPY - 1) / COPY);   // copies per block

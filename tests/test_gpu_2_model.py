@@ -190,6 +190,38 @@ def test_wide_models_of_few_sequences_against_full_prefix_logits(tmp_path, dt, B
     test_token_step_kernel_against_full_prefix_logits(tmp_path, dt, B, d, heads, mlp, 40, 50)
 
 
+def _random_model(d, heads, dt, V=1003, layers=4, **kw):
+    import flash_stu_2_b200 as F
+    torch.manual_seed(d)
+    cfg = F.FlashSTUConfig(n_embd=d, n_layers=layers, n_heads=heads, seq_len=256, window_size=40, vocab_size=V, mlp_scale=2,
+                           num_eigh=8, torch_dtype=dt, **kw)
+    with torch.device(dev()):
+        m = F.FlashSTU(cfg)
+    with torch.no_grad():
+        for name, p in m.named_parameters():
+            if not name.endswith("norm.weight"):
+                p.normal_(0.0, 0.5 * p.shape[-1] ** -0.5)
+    return m.eval()
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hidden", [160, 200, 336, 1000])
+def test_token_step_kernel_hidden_sizes_off_the_width(dt, hidden):
+    """MLP widths below the layer width and no multiple of it: rows of the down projection that end inside a piece."""
+    from flash_stu_2_b200 import ops
+    m = _random_model(256, 4, dt)
+    with torch.no_grad():
+        for layer in m.layers:
+            layer.mlp.intermediate_size = hidden
+            for proj, shape in (("gate_proj", (hidden, 256)), ("up_proj", (hidden, 256)), ("down_proj", (256, hidden))):
+                getattr(layer.mlp, proj).weight = torch.nn.Parameter(
+                    (0.5 * shape[1] ** -0.5 * torch.randn(shape, device=dev())).to(dt))
+    ids, logits = m.generate(torch.randint(0, 1003, (2, 30), device=dev()), max_length=40, do_sample=False, return_logits=True)
+    want = m(ids, use_cache=False).logits[:, 29:-1]
+    ops.check_status()
+    close(logits, want, 4e-5 if dt == torch.float32 else 2e-2)   # the bars of the test above
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for
