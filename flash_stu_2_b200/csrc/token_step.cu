@@ -21,7 +21,9 @@
 // bf16: mma.sync m16n8k16, weights as the 16-row operand (gate/up: 8 gate and the 8 up rows of the same features),
 // sequences as the 8 columns.  fp32: FMAs.  All product code exists once (a stage switch picks operands and epilogue):
 // written out per product it outgrew the instruction cache and the step took 1.25 ms instead of the figure below.
-// Every wait is bounded: on expiry the status word is raised, outstanding copies are let land and every CTA returns.
+// Every wait is bounded: on expiry the status word is raised, outstanding copies are let land and every CTA returns.  The
+// caches, positions and outputs are then undefined, and the workspace is marked: launches on it return at once with the
+// same status (their barriers would start from a counter that was left half way) until it is zeroed.
 #include "common.cuh"
 #include "stu_step.cuh"
 #include "tma.cuh"
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   __shared__ uint64_t full_bar[UNITS], empty_bar[UNITS];
   __shared__ float s_part[8][NW], s_scale[8];
   __shared__ float s_hist[MAX_ROWS * 8];
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_go;
   const Stage* tab = reinterpret_cast<const Stage*>(s_plan);
   const StuStepLayer* layers = reinterpret_cast<const StuStepLayer*>(s_plan + nst * 2);
 
@@ -179,7 +181,8 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     s_abort = 0;
     tma::fence_barrier_init();
   }
-  const int epoch = __ldcg(epoch_word);
+  const int2 control = __ldcg(reinterpret_cast<const int2*>(ws));   // epoch, and whether a launch has given up
+  const int epoch = control.x;
   __syncthreads();
   for (int i = tid; i < nst; i += THREADS) s_range[i] = share_of(tab[i].N, blockIdx.x, gridDim.x);
   const int t = __ldcg(layers[0].pos);
@@ -190,9 +193,10 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     if (tl != t) bad = 6;
     if (tl < 0 || (L.kind == STU_STEP_STU && tl >= 2 * L.Lh)) bad = 2;
   }
-  const int any2 = __syncthreads_or(bad == 2), any6 = __syncthreads_or(bad == 6);
-  if (any2 || any6) {   // every CTA sees the same positions, none waits for another
-    if (tid == 0 && cta == 0 && a.status) atomicExch(a.status, any2 ? 2 : 6);
+  if (control.y) bad = 12;   // its barrier counter is not to be trusted any more
+  const int any2 = __syncthreads_or(bad == 2), any6 = __syncthreads_or(bad == 6), any12 = __syncthreads_or(bad == 12);
+  if (any2 || any6 || any12) {   // every CTA sees the same words, none waits for another
+    if (tid == 0 && cta == 0 && a.status) atomicExch(a.status, any12 ? 12 : any2 ? 2 : 6);
     return;
   }
   int* counter = (int*)(ws + 128 + 128 * (epoch & 1));
@@ -298,10 +302,11 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
         }
       }
       if (!ok) *(volatile int*)&s_abort = 1;
+      s_go = *(volatile int*)&s_abort == 0;   // one answer for the whole CTA: the producer may raise s_abort at any time
       if (waits == 1 && cta == 0) *(int*)(ws + 128 + 128 * ((epoch + 1) & 1)) = 0;   // the next launch's counter
     }
     cons_bar();
-    return *(volatile int*)&s_abort == 0;
+    return s_go;
   };
   // row m of the input of layer l
   auto input_row = [&](int l, int m, bool& ok) -> const T* {
@@ -807,7 +812,10 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   }
   __syncthreads();   // with the producer
   if (s_abort) {
-    if (tid == 0 && a.status) atomicExch(a.status, 12);
+    if (tid == 0) {
+      atomicExch(epoch_word + 1, 1);
+      if (a.status) atomicExch(a.status, 12);
+    }
   } else if (cta == 0) {   // every CTA has read the positions and the epoch long ago (it arrived at a barrier since)
     for (int i = tid; i < a.n_layers * B; i += CONS) layers[i / B].pos[2 * (i % B)] = t + 1;
     if (tid == 0) *epoch_word = epoch + 1;

@@ -278,6 +278,8 @@ class FlashSTU(PreTrainedModel):
             ev_last.synchronize()
             timings["replayed_steps"] = replayed
             timings["replay_ms"] = ev_first.elapsed_time(ev_last)
+        if stepper is not None:
+            stepper.check()   # tokens drawn from logits that no step has written are not returned
         if return_logits:
             return generated, all_logits if stepper is not None else torch.stack(all_logits, dim=1)
         return generated

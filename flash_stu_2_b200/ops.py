@@ -92,7 +92,7 @@ STATUS_TEXT = {1: "token id outside the vocabulary", 2: "position outside the ca
                9: "a bounded pipeline wait ran out inside the tcgen05 prefill convolution",
                10: "a tensor-parallel rank waited in vain for another rank's sub-layer output",
                11: "tcgen05 attention prefill: a bounded wait ran out, or a sequence was not at position 0",
-               12: "a bounded grid-barrier wait ran out inside the token-step kernel"}
+               12: "a bounded wait ran out inside the token-step kernel"}
 
 
 def check_status(device=None):

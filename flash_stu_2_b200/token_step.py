@@ -64,7 +64,7 @@ class TokenStep:
         self.n_stages = lib.stu_token_step_plan(ctypes.addressof(table), ctypes.addressof(a), code, ctypes.addressof(blob))
         _lib.check(min(self.n_stages, 0), "stu_token_step_plan")
         self.plan = torch.frombuffer(blob, dtype=torch.uint8).to(self.device)
-        self._keep = keep + [ws]
+        self._ws, self._keep = ws, keep
 
     @staticmethod
     def supported(layers: Sequence, past: Sequence, batch: int, d: int, dtype: torch.dtype) -> bool:
@@ -95,3 +95,9 @@ class TokenStep:
         ops.token_step(self.plan, self.n_stages, a, self.dtype == torch.bfloat16)
         for p in self.pos:
             p._host_t += 1
+
+    def check(self):
+        """Raises when a step has given up on a wait (the steps after it then did nothing).  Waits for the steps so far."""
+        if int(self._ws[4:8].view(torch.int32)):
+            ops.check_status(self.device)
+            raise RuntimeError(f"flash_stu_2_b200 device status 12: {ops.STATUS_TEXT[12]}")

@@ -222,6 +222,33 @@ def test_token_step_kernel_hidden_sizes_off_the_width(dt, hidden):
     close(logits, want, 4e-5 if dt == torch.float32 else 2e-2)   # the bars of the test above
 
 
+def test_token_step_that_gives_up_is_reported(monkeypatch):
+    """A grid barrier that is never complete (its counter starts far below zero): the bounded waits run out, status 12 is
+    raised, later steps on the workspace return at once, generate() raises instead of returning tokens, and the context
+    stays usable."""
+    import time
+    from flash_stu_2_b200 import ops, token_step
+    m = _random_model(256, 4, torch.float32, layers=2)
+    prompt = torch.randint(0, 1003, (2, 30), device=dev())
+    want = m.generate(prompt, max_length=40, do_sample=False)
+    make = token_step.TokenStep.__init__
+
+    def broken(self, *args, **kw):
+        make(self, *args, **kw)
+        self._ws[128:132].view(torch.int32).fill_(-1 << 20)
+
+    with monkeypatch.context() as mp:
+        mp.setattr(token_step.TokenStep, "__init__", broken)
+        torch.cuda.synchronize()
+        t = time.monotonic()
+        with pytest.raises(RuntimeError, match="device status 12"):
+            m.generate(prompt, max_length=60, do_sample=False)
+        assert time.monotonic() - t < 8   # one wait of two seconds, not one per token
+    ops.check_status()
+    assert torch.equal(m.generate(prompt, max_length=40, do_sample=False), want)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for
