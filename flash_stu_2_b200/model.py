@@ -225,7 +225,7 @@ class FlashSTU(PreTrainedModel):
             if do_sample:
                 u = uniforms[step].to(device=dev, dtype=torch.float32).contiguous() if uniforms is not None else \
                     torch.rand(B, device=dev, generator=generator)
-            if step == 1 and fits and TokenStep.supported(self.layers, past, B, self.config.n_embd, self.config.torch_dtype):
+            if step == 1 and fits and TokenStep.supported(self.layers, past, B, self.config.n_embd, self.config.torch_dtype, self):
                 x = torch.empty(B, self.config.n_embd, dtype=self.config.torch_dtype, device=dev)
                 stepper = TokenStep(self.layers, past, B, x, model=self)
                 V = self.lm_head.weight.shape[0]

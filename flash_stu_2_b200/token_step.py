@@ -16,6 +16,25 @@ def layer_supported(layer) -> bool:
     return hasattr(layer, "attn")
 
 
+def layer_weights(layer, d: int, inter: int):
+    """(field of the descriptor, tensor, shape) of the weights that the kernel reads of a layer (an STU layer's M_inputs it
+    reads as the derived transpose: no field)."""
+    mlp = layer.mlp
+    out = [("norm2", layer.mlp_norm.weight, (d,)), ("wg", mlp.gate_proj.weight, (inter, d)),
+           ("wu", mlp.up_proj.weight, (inter, d)), ("wd", mlp.down_proj.weight, (d, inter))]
+    if hasattr(layer, "stu"):
+        return out + [("norm1", layer.stu_norm.weight, (d,)), (None, layer.stu.M_inputs, (d, d))]
+    return out + [("norm1", layer.attn_norm.weight, (d,)), ("w1", layer.attn.c_attn.weight, (3 * d, d)),
+                  ("wo", layer.attn.c_proj.weight, (d, d))]
+
+
+def model_weights(model, d: int):
+    """The same for the embedding, the final norm and the LM head."""
+    head = model.lm_head.weight
+    return [("embedding", model.tok_emb.weight, (head.shape[0], d)), ("norm_final", model.norm.weight, (d,)),
+            ("lm_head", head, (head.shape[0], d))]
+
+
 class TokenStep:
     """The step of `layers` on the cache entries `past` (one per layer, all at one position).  run() advances the caches
     by one token; the object keeps every tensor that the descriptors point to."""
@@ -29,26 +48,23 @@ class TokenStep:
         d = x.shape[-1]
         heads = window = 0
         softcap = 0.0
+        inter = layers[0].mlp.intermediate_size
         for L, layer, entry in zip(table, layers, past):
-            mlp = layer.mlp
-            L.norm2, L.eps2 = layer.mlp_norm.weight.data_ptr(), layer.mlp_norm.eps
-            L.wg, L.wu, L.wd = (m.weight.data_ptr() for m in (mlp.gate_proj, mlp.up_proj, mlp.down_proj))
-            L.pos = entry[-1].data_ptr()
+            for field, w, _ in layer_weights(layer, d, inter):
+                if field:
+                    setattr(L, field, w.data_ptr())
+            L.eps2, L.pos = layer.mlp_norm.eps, entry[-1].data_ptr()
             if hasattr(layer, "stu"):
                 MinT, taps, taps8 = layer.stu.prepared()
                 keep += [MinT, taps, taps8]
                 L.kind, L.Lh = 0, entry[0].shape[3]
-                L.norm1, L.eps1 = layer.stu_norm.weight.data_ptr(), layer.stu_norm.eps
-                L.w1, L.hist = MinT.data_ptr(), entry[0].data_ptr()
+                L.eps1, L.w1, L.hist = layer.stu_norm.eps, MinT.data_ptr(), entry[0].data_ptr()
                 L.taps = (taps8 if self.dtype == torch.bfloat16 else taps).data_ptr()
             else:
                 attn = layer.attn
                 heads, window, softcap = attn.n_heads, attn.window, float(attn.softcap or 0.0)
-                L.kind, L.W = 1, entry[0].shape[1]
-                L.norm1, L.eps1 = layer.attn_norm.weight.data_ptr(), layer.attn_norm.eps
-                L.w1, L.wo = attn.c_attn.weight.data_ptr(), attn.c_proj.weight.data_ptr()
+                L.kind, L.W, L.eps1 = 1, entry[0].shape[1], layer.attn_norm.eps
                 L.k_ring, L.v_ring, L.slopes = entry[0].data_ptr(), entry[1].data_ptr(), attn.alibi_slopes.data_ptr()
-        inter = layers[0].mlp.intermediate_size
         code = 1 if self.dtype == torch.bfloat16 else 0
         nbytes = lib.stu_token_step_workspace_bytes(d, inter, heads, code)
         ws = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
@@ -58,8 +74,9 @@ class TokenStep:
         a.status = ops.status_word(self.device).data_ptr()
         if model is not None:
             a.V = model.lm_head.weight.shape[0]
-            a.embedding, a.lm_head = model.tok_emb.weight.data_ptr(), model.lm_head.weight.data_ptr()
-            a.norm_final, a.eps_final = model.norm.weight.data_ptr(), model.norm.eps
+            for field, w, _ in model_weights(model, d):
+                setattr(a, field, w.data_ptr())
+            a.eps_final = model.norm.eps
         blob = (ctypes.c_uint8 * lib.stu_token_step_plan_bytes(len(layers)))()
         self.n_stages = lib.stu_token_step_plan(ctypes.addressof(table), ctypes.addressof(a), code, ctypes.addressof(blob))
         _lib.check(min(self.n_stages, 0), "stu_token_step_plan")
@@ -67,7 +84,9 @@ class TokenStep:
         self._ws, self._keep = ws, keep
 
     @staticmethod
-    def supported(layers: Sequence, past: Sequence, batch: int, d: int, dtype: torch.dtype) -> bool:
+    def supported(layers: Sequence, past: Sequence, batch: int, d: int, dtype: torch.dtype, model=None) -> bool:
+        """Whether the kernel takes these layers and caches (and the model's embedding and head) as they are: whatever it
+        has no form of is the per-layer kernels' work."""
         if batch > 8 or len(layers) > _lib.STEP_MAX_LAYERS or dtype not in (torch.bfloat16, torch.float32):
             return False
         if any(e is None for e in past) or not all(layer_supported(layer) for layer in layers):
@@ -76,13 +95,17 @@ class TokenStep:
         if any(host_pos(e[-1]) != t or not uniform_pos(e[-1]) for e in past):
             return False
         inter = layers[0].mlp.intermediate_size
-        heads = {layer.attn.n_heads for layer in layers if hasattr(layer, "attn")}
-        if len(heads) > 1 or any(layer.mlp.intermediate_size != inter for layer in layers):
+        attn = [layer.attn for layer in layers if hasattr(layer, "attn")]
+        if any((a.n_heads, a.window, a.softcap) != (attn[0].n_heads, attn[0].window, attn[0].softcap) for a in attn):
             return False
-        params = [p for layer in layers for p in layer.parameters()]
-        if any(p.dtype != dtype or not p.is_contiguous() for p in params):
+        if model is not None and model.lm_head.weight.shape[0] >= 1 << 24:
             return False
-        return bool(_lib.load().stu_token_step_supported(len(layers), batch, d, inter, max(heads, default=0),
+        weights = [w for layer in layers for w in layer_weights(layer, d, inter)] + (model_weights(model, d) if model else [])
+        if any(w.dtype != dtype or tuple(w.shape) != shape for _, w, shape in weights):
+            return False
+        if any(field and (not w.is_contiguous() or w.data_ptr() % 16) for field, w, _ in weights):
+            return False
+        return bool(_lib.load().stu_token_step_supported(len(layers), batch, d, inter, attn[0].n_heads if attn else 0,
                                                          1 if dtype == torch.bfloat16 else 0))
 
     def run(self, ids: Optional[torch.Tensor] = None, logits: Optional[torch.Tensor] = None):

@@ -2,8 +2,11 @@
 import ctypes
 
 import pytest
+import torch
 
+import flash_stu_2_b200 as F
 from flash_stu_2_b200 import _lib
+from flash_stu_2_b200.token_step import TokenStep
 
 A = 1 << 20   # stands for an aligned device address: nothing here dereferences it
 
@@ -50,3 +53,43 @@ def test_weight_stream_never_waits_for_itself(bf16, B):
 def test_weight_stream_of_rings_of_24_to_30_slots(d, mlp, B, heads, bf16):
     if _lib.load().stu_token_step_supported(4, B, d, mlp * d, heads, int(bf16)):
         assert _stall(d, mlp * d, B, heads, bf16) == 0
+
+
+def _model(dt=torch.float32, **kw):
+    cfg = F.FlashSTUConfig(n_embd=64, n_layers=4, n_heads=2, seq_len=64, window_size=8, vocab_size=97, mlp_scale=4, num_eigh=8,
+                           torch_dtype=dt, **kw)
+    return F.FlashSTU(cfg).eval()
+
+
+def _takes(m, batch=2):
+    past = [(l.stu if hasattr(l, "stu") else l.attn).new_cache(batch, "cpu") for l in m.layers]
+    return TokenStep.supported(m.layers, past, batch, 64, m.config.torch_dtype, m)
+
+
+def _off_the_grid(w):
+    return torch.nn.Parameter(torch.zeros(w.numel() + 1, dtype=w.dtype)[1:].view(w.shape))
+
+
+def _narrow_mlp(m):
+    m.layers[2].mlp.gate_proj = torch.nn.Linear(64, 200, bias=False)
+    m.layers[2].mlp.up_proj = torch.nn.Linear(64, 200, bias=False)
+    m.layers[2].mlp.down_proj = torch.nn.Linear(200, 64, bias=False)
+
+
+@pytest.mark.parametrize("change", [
+    lambda m: setattr(m.layers[1].attn.c_attn, "weight", _off_the_grid(m.layers[1].attn.c_attn.weight)),
+    lambda m: setattr(m.layers[0].stu_norm, "weight", _off_the_grid(m.layers[0].stu_norm.weight)),
+    lambda m: setattr(m.lm_head, "weight", _off_the_grid(m.lm_head.weight)),
+    lambda m: setattr(m.tok_emb, "weight", _off_the_grid(m.tok_emb.weight)),
+    lambda m: setattr(m.norm, "weight", _off_the_grid(m.norm.weight)),
+    lambda m: setattr(m.lm_head, "weight", torch.nn.Parameter(m.lm_head.weight.bfloat16())),
+    lambda m: setattr(m.tok_emb, "weight", torch.nn.Parameter(torch.zeros(90, 64))),
+    lambda m: setattr(m.lm_head, "weight", torch.nn.Parameter(torch.zeros(64, 97).t())),
+    lambda m: setattr(m.layers[3].attn, "softcap", 7.0), lambda m: setattr(m.layers[3].attn, "window", 5), _narrow_mlp])
+def test_models_that_the_kernel_has_no_form_of_are_left_to_the_per_layer_kernels(change):
+    """Weights off the 16-byte grid, of another dtype or shape than the configuration's, attention layers that differ."""
+    m = _model()
+    assert _takes(m)
+    with torch.no_grad():
+        change(m)
+    assert not _takes(m)
