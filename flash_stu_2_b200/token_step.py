@@ -51,6 +51,7 @@ class TokenStep:
         inter = layers[0].mlp.intermediate_size
         for L, layer, entry in zip(table, layers, past):
             for field, w, _ in layer_weights(layer, d, inter):
+                keep.append(w)   # (a parametrised weight is a new tensor at every look-up)
                 if field:
                     setattr(L, field, w.data_ptr())
             L.eps2, L.pos = layer.mlp_norm.eps, entry[-1].data_ptr()
@@ -75,6 +76,7 @@ class TokenStep:
         if model is not None:
             a.V = model.lm_head.weight.shape[0]
             for field, w, _ in model_weights(model, d):
+                keep.append(w)
                 setattr(a, field, w.data_ptr())
             a.eps_final = model.norm.eps
         blob = (ctypes.c_uint8 * lib.stu_token_step_plan_bytes(len(layers)))()

@@ -249,6 +249,27 @@ def test_token_step_that_gives_up_is_reported(monkeypatch):
     ops.check_status()
 
 
+def test_token_step_kernel_with_parametrised_weights():
+    """A weight that is computed at every look-up lives as long as the steps that read it."""
+    from torch.nn.utils import parametrize
+    from flash_stu_2_b200 import ops
+
+    class Doubled(torch.nn.Module):
+        def forward(self, w):
+            return 2.0 * w
+
+    m = _random_model(256, 4, torch.float32)
+    for layer in m.layers:
+        parametrize.register_parametrization(layer.mlp.down_proj, "weight", Doubled())
+    for attn in (m.layers[1].attn, m.layers[3].attn):
+        parametrize.register_parametrization(attn.c_proj, "weight", Doubled())
+    ids, logits = m.generate(torch.randint(0, 1003, (2, 30), device=dev()), max_length=60, do_sample=False, return_logits=True)
+    with torch.no_grad():
+        want = m(ids, use_cache=False).logits[:, 29:-1]
+    ops.check_status()
+    close(logits, want, 4e-5)
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for
