@@ -208,6 +208,7 @@ class FlashSTU(PreTrainedModel):
         # cannot issue as fast as the GPU retires them.  cuda_graph=False keeps the eager loop.
         capacity = min(self.config.seq_len, getattr(self.config, "cache_len", None) or self.config.seq_len)
         fits = use_cache and max_length - 1 <= capacity
+        plain = all(getattr(getattr(self, n), "__func__", None) is getattr(FlashSTU, n) for n in ("last_logits", "_backbone"))
         use_graph = bool(kwargs.get("cuda_graph", True)) and fits and steps > 3
         # a sandwich layer's token step reads its position on the device only in the bf16 approx form
         for layer in self.layers:
@@ -225,7 +226,8 @@ class FlashSTU(PreTrainedModel):
             if do_sample:
                 u = uniforms[step].to(device=dev, dtype=torch.float32).contiguous() if uniforms is not None else \
                     torch.rand(B, device=dev, generator=generator)
-            if step == 1 and fits and TokenStep.supported(self.layers, past, B, self.config.n_embd, self.config.torch_dtype, self):
+            if step == 1 and fits and plain and TokenStep.supported(self.layers, past, B, self.config.n_embd,
+                                                                    self.config.torch_dtype, self):
                 x = torch.empty(B, self.config.n_embd, dtype=self.config.torch_dtype, device=dev)
                 stepper = TokenStep(self.layers, past, B, x, model=self)
                 V = self.lm_head.weight.shape[0]

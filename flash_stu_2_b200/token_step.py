@@ -6,11 +6,15 @@ from typing import Optional, Sequence
 import torch
 
 from . import _lib, ops
+from .layers import AttentionLayer, STULayer
 from .modules import host_pos, uniform_pos
 
 
 def layer_supported(layer) -> bool:
-    """Whether a layer's token step is one the kernel computes: a plain approx STU layer or an attention layer."""
+    """Whether a layer's token step is one the kernel computes: a plain approx STU layer or an attention layer, whose
+    forward() nobody overrides or listens to."""
+    if type(layer) not in (STULayer, AttentionLayer) or "forward" in vars(layer) or layer._forward_hooks or layer._forward_pre_hooks:
+        return False
     if hasattr(layer, "stu"):
         return layer.stu.use_approx and not layer.stu.use_hankel_L and not layer.stu_mlp_enabled
     return hasattr(layer, "attn")

@@ -270,6 +270,22 @@ def test_token_step_kernel_with_parametrised_weights():
     close(logits, want, 4e-5)
 
 
+def test_overridden_step_logits_reach_the_token_loop():
+    """last_logits() of a subclass decides every token."""
+    m = _random_model(64, 2, torch.float32)
+    base = type(m)
+
+    class Shifted(base):
+        def last_logits(self, *args, **kw):
+            logits, cache = super().last_logits(*args, **kw)
+            logits[:, 7] += 1000.0
+            return logits, cache
+
+    m.__class__ = Shifted
+    ids = m.generate(torch.randint(0, 1003, (2, 30), device=dev()), max_length=40, do_sample=False)
+    assert bool((ids[:, 30:] == 7).all())
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for

@@ -93,3 +93,21 @@ def test_models_that_the_kernel_has_no_form_of_are_left_to_the_per_layer_kernels
     with torch.no_grad():
         change(m)
     assert not _takes(m)
+
+
+def _own_forward(m):
+    layer = m.layers[2]
+    layer.forward = lambda *a, **kw: type(layer).forward(layer, *a, **kw)
+
+
+def _subclass(m):
+    m.layers[1].__class__ = type("Layer", (type(m.layers[1]),), {})
+
+
+@pytest.mark.parametrize("change", [lambda m: m.layers[0].register_forward_hook(lambda *a: None), _own_forward, _subclass,
+                                    lambda m: m.layers[3].register_forward_pre_hook(lambda *a: None)])
+def test_layers_that_somebody_overrides_or_listens_to_are_called(change):
+    m = _model()
+    assert _takes(m)
+    change(m)
+    assert not _takes(m)
