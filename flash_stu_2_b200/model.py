@@ -185,13 +185,14 @@ class FlashSTU(PreTrainedModel):
         floor(u * vocab_size) from its uniform (the reference draws a uniformly random token there);
         (4) prompts may be shorter than seq_len and steps read cached state (the reference recomputes the prefix);
         (5) nucleus filtering without top_k, and top_k above 1024, need the vocabulary row in shared memory (at
-        most 51712 entries; status 5 / 4 otherwise).  kwargs: uniforms, generator, return_logits, cuda_graph (replay
-        the cached steps from one captured graph, default True), timings (dict filled with the device time of the
-        replayed steps)."""
+        most 51712 entries; status 5 / 4 otherwise).  kwargs: uniforms, generator, return_logits, cuda_graph (True, the
+        default: the cached steps run as one persistent kernel each where there is one for the model and the batch,
+        else they are replayed from one captured graph; False: layer by layer, as forward() runs them), timings (dict
+        filled with the device time of the steps that one of the two forms ran)."""
         uniforms = kwargs.get("uniforms")
         generator = kwargs.get("generator")
         return_logits = kwargs.get("return_logits", False)
-        timings = kwargs.get("timings")   # optional dict: filled with the device time of the graph-replayed steps
+        timings = kwargs.get("timings")   # optional dict: filled with the device time of the steps not run layer by layer
         ev_first = ev_last = None
         replayed = 0
         B, T0 = input_ids.shape
@@ -203,13 +204,15 @@ class FlashSTU(PreTrainedModel):
         generated[:, :T0] = input_ids
         all_logits = []
         past = None
-        # Cached token steps after the first are replayed from one captured CUDA graph (every kernel reads its
-        # position from device memory): the step is ~100 small launches for a 24-layer model, which the interpreter
-        # cannot issue as fast as the GPU retires them.  cuda_graph=False keeps the eager loop.
+        # Cached token steps after the first are one launch of the persistent kernel (token_step.py), or replayed from
+        # one captured CUDA graph (every kernel reads its position from device memory): the step is ~100 small launches
+        # for a 24-layer model, which the interpreter cannot issue as fast as the GPU retires them.
+        # cuda_graph=False keeps the eager loop, ops.fused_step = False the kernels apart.
         capacity = min(self.config.seq_len, getattr(self.config, "cache_len", None) or self.config.seq_len)
         fits = use_cache and max_length - 1 <= capacity
         plain = all(getattr(getattr(self, n), "__func__", None) is getattr(FlashSTU, n) for n in ("last_logits", "_backbone"))
-        use_graph = bool(kwargs.get("cuda_graph", True)) and fits and steps > 3
+        eager = not kwargs.get("cuda_graph", True)
+        use_graph = not eager and fits and steps > 3
         # a sandwich layer's token step reads its position on the device only in the bf16 approx form
         for layer in self.layers:
             if getattr(layer, "stu_mlp_enabled", False) and not (
@@ -226,7 +229,7 @@ class FlashSTU(PreTrainedModel):
             if do_sample:
                 u = uniforms[step].to(device=dev, dtype=torch.float32).contiguous() if uniforms is not None else \
                     torch.rand(B, device=dev, generator=generator)
-            if step == 1 and fits and plain and TokenStep.supported(self.layers, past, B, self.config.n_embd,
+            if step == 1 and fits and plain and not eager and ops.fused_step and TokenStep.supported(self.layers, past, B, self.config.n_embd,
                                                                     self.config.torch_dtype, self):
                 x = torch.empty(B, self.config.n_embd, dtype=self.config.torch_dtype, device=dev)
                 stepper = TokenStep(self.layers, past, B, x, model=self)

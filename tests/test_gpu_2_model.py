@@ -286,6 +286,43 @@ def test_overridden_step_logits_reach_the_token_loop():
     assert bool((ids[:, 30:] == 7).all())
 
 
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kw", [dict(do_sample=False), dict(temperature=0.7, top_k=20), dict(top_k=50, top_p=0.8)])
+def test_the_three_forms_of_the_token_loop_agree(monkeypatch, dt, kw):
+    """The persistent kernel, the replayed graph (ops.fused_step off) and the eager loop (cuda_graph=False) on one model:
+    which one runs is what the caller asked for, and they draw the same tokens (fp32; bf16: logits within the bars)."""
+    from flash_stu_2_b200 import ops
+    m = _random_model(256, 4, dt)
+    prompt, u = torch.randint(0, 1003, (3, 33), device=dev()), torch.rand(12, 3)
+    calls = []
+    step = ops.token_step
+    monkeypatch.setattr(ops, "token_step", lambda *a: (calls.append(1), step(*a)))
+    captures = []
+    capture = type(m)._capture_step
+    monkeypatch.setattr(type(m), "_capture_step", lambda *a: (captures.append(1), capture(*a))[1])
+
+    def run(**more):
+        del calls[:], captures[:]
+        out = m.generate(prompt, max_length=45, uniforms=u, return_logits=True, **kw, **more)
+        return out + (len(calls), len(captures))
+
+    ids, logits, n, c = run()
+    assert (n, c) == (11, 0)
+    eager_ids, eager_logits, n, c = run(cuda_graph=False)
+    assert (n, c) == (0, 0)
+    monkeypatch.setattr(ops, "fused_step", False)
+    graph_ids, graph_logits, n, c = run()
+    assert (n, c) == (0, 1)
+    ops.check_status()
+    assert torch.equal(graph_ids, eager_ids) and torch.equal(graph_logits, eager_logits)
+    if dt == torch.float32:
+        assert torch.equal(ids, eager_ids)
+        close(logits, eager_logits, 4e-5)
+    else:   # up to the first token that rounding decides
+        same = int((ids == eager_ids).all(0).long().cumprod(0).sum()) - 33 + 1
+        close(logits[:, :same], eager_logits[:, :same], 2e-2)
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for
