@@ -140,6 +140,9 @@ def load(build_if_missing: bool = True):
     return lib
 
 
+ERR_UNSUPPORTED = -4
+
+
 def check(rc: int, what: str):
     if rc == 0:
         return

@@ -224,6 +224,9 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
     rc = _lib.load().stu_linear(x.data_ptr(), x.stride(0), W.data_ptr(), w_rs, w_ks, _p(W2), _p(resid), r_rs,
                                 out.data_ptr(), y_rs, M, N, K, epilogue, hist_T, hist_t0, hist_Lh, _p(norm_w), eps,
                                 _dt(x), backend, _stream())
+    if rc == _lib.ERR_UNSUPPORTED and norm_w is not None and x.dtype == torch.float32 and backend == BACKEND_AUTO:
+        # rows or weights off the 16-byte grid: the norm in a launch of its own, the product on the kernels that take them
+        return linear(rmsnorm(x, norm_w, eps), W, W2=W2, resid=resid, out=out, epilogue=epilogue)
     _lib.check(rc, "stu_linear")
     _count()
     return out

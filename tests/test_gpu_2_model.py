@@ -323,6 +323,26 @@ def test_the_three_forms_of_the_token_loop_agree(monkeypatch, dt, kw):
         close(logits[:, :same], eager_logits[:, :same], 2e-2)
 
 
+@pytest.mark.parametrize("where", ["attn_norm", "mlp_norm", "attn.c_attn", "mlp.gate_proj", "mlp.down_proj"])
+def test_fp32_steps_with_weights_off_the_16_byte_grid(where):
+    """fp32 steps fuse the norm into the linears, whose kernel reads 16 bytes at a time: parameters that start elsewhere (views
+    into one flat buffer) go to the kernels that read single values."""
+    from flash_stu_2_b200 import ops
+    m = _random_model(256, 4, torch.float32)
+    prompt = torch.randint(0, 1003, (2, 30), device=dev())
+    with torch.no_grad():
+        ids, want = m.generate(prompt, max_length=36, do_sample=False, return_logits=True, cuda_graph=False)
+        mod = m.layers[1].get_submodule(where)
+        flat = torch.zeros(mod.weight.numel() + 1, device=dev())
+        flat[1:] = mod.weight.reshape(-1)
+        mod.weight = torch.nn.Parameter(flat[1:].view(mod.weight.shape))
+        for graph in (False, True):
+            again, got = m.generate(prompt, max_length=36, do_sample=False, return_logits=True, cuda_graph=graph)
+            assert torch.equal(again, ids)
+            close(got, want, 4e-5)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("hd,B", [(64, 3), (128, 9)])
 def test_mid_size_hybrid_bf16_model_against_the_oracle(tmp_path, hd, B):
     """A bf16 hybrid model wide enough to reach the tensor-core kernels inside the model (head size 64 / 128 for
