@@ -49,8 +49,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   __shared__ __align__(16) float sm[2 * TILE > PART ? 2 * TILE : PART];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  // lower-triangular blocks of `causal` rows of B: nothing beyond the tile's last column
-  int k_end = causal && n0 % causal + BN <= causal ? min(K, n0 % causal + BN) : K;
+  const int k_end = causal ? min(K, n0 + BN) : K;   // a lower-triangular B has nothing beyond the tile's last column
 
   const int nkb = (k_end + BK - 1) / BK, per = (nkb + KS - 1) / KS;
   const int kb0 = KS > 1 ? (int)blockIdx.z * per : 0, kb1 = KS > 1 ? min(nkb, kb0 + per) : nkb;
