@@ -206,6 +206,18 @@ class MiniSTU(nn.Module):
         most = max(1, min(B, (2 << 30) // max(1, T * width * x.element_size())))
         return min(range(1, most + 1), key=lambda g: (B // g * waves(g) + (waves(B % g) if B % g else 0), g))
 
+    @staticmethod
+    def _lds_features(G: int, T: int, padded: int, width: int, x):
+        """(sequences per contraction, their feature rows [(G-1)*T + padded, width]): fewer sequences where the device has no
+        room for G, down to one."""
+        while True:
+            try:
+                return G, torch.empty((G - 1) * T + padded, width, dtype=x.dtype, device=x.device)
+            except torch.cuda.OutOfMemoryError:
+                if G == 1:
+                    raise
+                G = (G + 1) // 2
+
     def _forward_lds(self, x, past_key_value=None, use_cache=False):
         op = self._lds_prepared()
         A32, B32, Cm = self._lds_f32
@@ -248,8 +260,7 @@ class MiniSTU(nn.Module):
         # sequences of a group share the contraction (one alone leaves its last wave of output tiles nearly empty).  Their
         # features follow one another T rows apart; the rows past T of a sequence's last chunk are overwritten by
         # the next sequence's, or lie past the group's rows.
-        G = self._lds_group(B, T, F_ * d, x)
-        U2 = torch.empty((G - 1) * T + nch * Ck, F_ * d, dtype=x.dtype, device=x.device)
+        G, U2 = self._lds_features(self._lds_group(B, T, F_ * d, x), T, nch * Ck, F_ * d, x)
         for b0 in range(0, B, G):
             n = min(G, B - b0)
             for b in range(b0, b0 + n):

@@ -136,3 +136,22 @@ def test_block_power_iteration_reproduces_the_leading_hankel_eigenpairs():
     assert np.allclose(w.numpy()[-10:], wr[-10:], rtol=1e-9, atol=1e-15)
     assert (V[:, -8:].abs() - torch.tensor(Vr[:, -8:]).abs()).abs().max() < 1e-9
     assert torch.allclose(V.T @ V, torch.eye(K, dtype=torch.float64), atol=1e-10)
+
+
+def test_lds_feature_rows_shrink_to_the_memory_there_is(monkeypatch):
+    """The prefill of the distilled form holds the features of several sequences at once only where they fit."""
+    room, real = 5000, torch.empty
+
+    def empty(*shape, **kw):
+        if shape[0] > room:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return real(*shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    x = torch.zeros(8, 1000, 4)
+    for most, got in ((8, 4), (5, 3), (3, 3), (1, 1)):   # 8 -> 4, 5 -> 3
+        G, U = F.MiniSTU._lds_features(most, 1000, 1024, 16, x)
+        assert G == got and U.shape == ((G - 1) * 1000 + 1024, 16)
+    room = 1000
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        F.MiniSTU._lds_features(8, 1000, 1024, 16, x)
