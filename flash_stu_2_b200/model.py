@@ -9,6 +9,7 @@ can observe, all forced by the reference's own gaps:
     `uniforms=[steps,B]` or drawn from `generator=`) instead of torch.multinomial.
 """
 import gc
+import threading
 from typing import Any, Dict, Optional, Tuple
 
 import torch
@@ -23,6 +24,27 @@ from .filters import get_spectral_filters, nearest_power_of_two
 from .layers import AttentionLayer, STULayer
 from .modules import STU, Attention, RMSNorm
 from .token_step import TokenStep
+
+
+class _CollectionHeld:
+    """No garbage collection while any thread is inside: one inside a graph capture could release objects whose destructors
+    may not be captured.  The collector is the process's, so the last one out restores it as the first one found it."""
+    _lock, _inside, _was_on = threading.Lock(), 0, False
+
+    def __enter__(self):
+        cls = _CollectionHeld
+        with cls._lock:
+            if cls._inside == 0:
+                cls._was_on = gc.isenabled()
+                gc.disable()
+            cls._inside += 1
+
+    def __exit__(self, *exc):
+        cls = _CollectionHeld
+        with cls._lock:
+            cls._inside -= 1
+            if cls._inside == 0 and cls._was_on:
+                gc.enable()
 
 
 class FlashSTU(PreTrainedModel):
@@ -302,19 +324,13 @@ class FlashSTU(PreTrainedModel):
         graph = torch.cuda.CUDAGraph()
         stream, here = torch.cuda.Stream(tok.device), torch.cuda.current_stream(tok.device)
         stream.wait_stream(here)
-        collecting = gc.isenabled()
-        gc.disable()   # a collection inside the capture could release objects whose destructors may not be captured
-        try:
-            with torch.cuda.stream(stream), ops.arena(buffer):
-                graph.capture_begin(capture_error_mode="thread_local")
-                try:
-                    logits, _ = self.last_logits(tok, past, True)
-                    ops.sample(logits, temperature, top_k, top_p, do_sample, u_buf if do_sample else None, tok, out_stride=1)
-                finally:
-                    graph.capture_end()
-        finally:
-            if collecting:
-                gc.enable()
+        with _CollectionHeld(), torch.cuda.stream(stream), ops.arena(buffer):
+            graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                logits, _ = self.last_logits(tok, past, True)
+                ops.sample(logits, temperature, top_k, top_p, do_sample, u_buf if do_sample else None, tok, out_stride=1)
+            finally:
+                graph.capture_end()
         here.wait_stream(stream)
         for e, t in zip(past, host_t):   # capturing ran the host bookkeeping, not the kernels
             if e is not None and t is not None:

@@ -155,3 +155,22 @@ def test_lds_feature_rows_shrink_to_the_memory_there_is(monkeypatch):
     room = 1000
     with pytest.raises(torch.cuda.OutOfMemoryError):
         F.MiniSTU._lds_features(8, 1000, 1024, 16, x)
+
+
+def test_captures_of_two_threads_hold_the_collector_until_the_last_is_done():
+    import gc
+    from flash_stu_2_b200.model import _CollectionHeld
+    a, b = _CollectionHeld(), _CollectionHeld()
+    assert gc.isenabled()
+    a.__enter__(), b.__enter__()
+    a.__exit__()
+    assert not gc.isenabled()   # the other capture is still open
+    b.__exit__()
+    assert gc.isenabled()
+    gc.disable()
+    try:
+        with _CollectionHeld():
+            pass
+        assert not gc.isenabled()
+    finally:
+        gc.enable()
