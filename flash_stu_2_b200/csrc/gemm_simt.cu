@@ -5,7 +5,9 @@
 // Bound: FFMA issue (74 TFLOP/s), and before that the number of CTAs: the prefill linears of a 512-wide fp32 model are
 // 256 x 512 x 6144.  64 x 64 tiles of 128 threads (8 x 4 outputs each: three 16-byte shared-memory reads per 32 FMAs)
 // with K split over a thread-block cluster of up to 8 CTAs until there are about two per SM (the partial tiles meet in
-// distributed shared memory, summed in rank order), 128 x 128 tiles (8 x 8 outputs) where those alone fill the chip.
+// distributed shared memory, summed in rank order).  (128 x 128 tiles of 8 x 8 outputs where those alone fill the chip
+// are 2 to 5 % ahead only for the largest products, 4000 x 8192 x 4096 6.01 against 6.30 ms, and fall far behind on
+// short K, where the outputs leave in rows of 8: 8192 x 1024 x 24, the taps of an STU layer, 47 against 20 us.)
 // Operand tiles pass through registers into a double-buffered, k-major shared-memory tile.  256 x 512 x 6144:
 // 531 us with 64 x 64 tiles of 4 x 4 outputs, no split and no overlap.
 #include <cooperative_groups.h>
@@ -19,7 +21,8 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int BK = 16;
+constexpr int BM = 64, BN = 64, BK = 16;                  // tile
+constexpr int TM = 8, TN = 4, THREADS = BM / TM * (BN / TN);   // outputs of a thread, 16 threads across the columns
 
 // Four consecutive k of one row as fp32; vec: 16-byte (fp32) / 8-byte (bf16) aligned and inside the row.
 __device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
@@ -34,13 +37,13 @@ __device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
   v[3] = __uint_as_float(t.y & 0xffff0000u);
 }
 
-// TM x TN outputs per thread, 16 threads across the columns.  KS > 1: cluster of KS CTAs along z.
-template <typename T, int EPI, int BM, int BN, int TM, int TN, int KS>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+// KS > 1: cluster of KS CTAs along z.
+template <typename T, int EPI, int KS>
+__global__ void __launch_bounds__(THREADS)
     gemm_simt_kernel(const T* __restrict__ A, long long lda, const T* __restrict__ B, long long ldb, long long skb,
                      const T* __restrict__ B2, int M, int N, int K, int causal, int vec_a, int vec_b, EpiArgs<T> ep) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
-  constexpr int THREADS = (BM / TM) * (BN / TN), NB = DUAL ? 2 : 1;
+  constexpr int NB = DUAL ? 2 : 1;
   constexpr int QA = BM * BK / 4 / THREADS, QB = BN * BK / 4 / THREADS;   // quads of k per thread and tile
   static_assert(BN / TN == 16 && QA >= 1 && QB >= 1, "thread layout");
   constexpr int PA = BM + 4, PB = BN + 4;
@@ -184,11 +187,11 @@ struct Operands {
   int M, N, K, causal, vec_a, vec_b;
 };
 
-template <typename T, int EPI, int BM, int BN, int TM, int TN, int KS>
+template <typename T, int EPI, int KS>
 int launch_tile(const Operands& o, const EpiArgs<T>& ep, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((o.N + BN - 1) / BN, (o.M + BM - 1) / BM, KS);
-  cfg.blockDim = dim3((BM / TM) * (BN / TN));
+  cfg.blockDim = dim3(THREADS);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -197,7 +200,7 @@ int launch_tile(const Operands& o, const EpiArgs<T>& ep, cudaStream_t st) {
   at[0].val.clusterDim.z = KS;
   cfg.attrs = at;
   cfg.numAttrs = KS > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_simt_kernel<T, EPI, BM, BN, TM, TN, KS>, (const T*)o.A, o.lda,
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_simt_kernel<T, EPI, KS>, (const T*)o.A, o.lda,
                                            (const T*)o.B, o.ldb, o.skb, (const T*)o.B2, o.M, o.N, o.K, o.causal, o.vec_a,
                                            o.vec_b, ep);
   if (e != cudaSuccess) return (int)e;
@@ -207,19 +210,15 @@ int launch_tile(const Operands& o, const EpiArgs<T>& ep, cudaStream_t st) {
 
 template <typename T, int EPI>
 int launch_simt(const Operands& o, const EpiArgs<T>& ep, cudaStream_t st) {
-  const long long sms = device_sm_count();
-  auto tiles = [&](int t) { return (long long)((o.M + t - 1) / t) * ((o.N + t - 1) / t); };
-  if constexpr (EPI != EPI_GELU_MUL) {
-    if (tiles(128) >= 2 * sms) return launch_tile<T, EPI, 128, 128, 8, 8, 1>(o, ep, st);
-  }
+  const long long sms = device_sm_count(), tiles = (long long)((o.M + BM - 1) / BM) * ((o.N + BN - 1) / BN);
   // split K while there are fewer than two CTAs per SM and every CTA keeps 64 of K
   int ks = 1;
-  while (ks < 8 && tiles(64) * ks < 2 * sms && o.K / (2 * ks) >= 64) ks *= 2;
+  while (ks < 8 && tiles * ks < 2 * sms && o.K / (2 * ks) >= 64) ks *= 2;
   switch (ks) {
-    case 1: return launch_tile<T, EPI, 64, 64, 8, 4, 1>(o, ep, st);
-    case 2: return launch_tile<T, EPI, 64, 64, 8, 4, 2>(o, ep, st);
-    case 4: return launch_tile<T, EPI, 64, 64, 8, 4, 4>(o, ep, st);
-    default: return launch_tile<T, EPI, 64, 64, 8, 4, 8>(o, ep, st);
+    case 1: return launch_tile<T, EPI, 1>(o, ep, st);
+    case 2: return launch_tile<T, EPI, 2>(o, ep, st);
+    case 4: return launch_tile<T, EPI, 4>(o, ep, st);
+    default: return launch_tile<T, EPI, 8>(o, ep, st);
   }
 }
 

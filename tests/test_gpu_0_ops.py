@@ -126,7 +126,7 @@ def test_linear_wide_tensor_core_tiles(epi):
 @pytest.mark.parametrize("shape", [(65, 64, 24, 0), (200, 65, 70, 2), (256, 512, 6144, 1), (300, 130, 264, 2), (64, 700, 3000, 0),
                                    (2500, 2500, 40, 0), (100, 333, 1027, 1)])
 def test_linear_cuda_core_tiles(dt, shape):
-    """The CUDA-core GEMM at the edges of its tiles (64 and 128), K split over clusters of 1 to 8 CTAs, ragged K and rows off
+    """The CUDA-core GEMM at the edges of its 64 x 64 tiles, K split over clusters of 1 to 8 CTAs, ragged K and rows off
     the 16-byte grid; lower-triangular weights with and without the flag."""
     from flash_stu_2_b200 import ops
     M, N, K, epi = shape
@@ -146,13 +146,13 @@ def test_linear_cuda_core_tiles(dt, shape):
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(70, 512, 512), (65, 200, 333), (4000, 2500, 2500)])
 def test_linear_cuda_core_tiles_skip_what_a_triangular_weight_leaves_out(dt, shape):
-    """The CUDA-core GEMM reads nothing of a lower-triangular weight past the last column of a tile (64 or 128 wide, K split or
-    not): NaN from the next multiple of 128 on."""
+    """The CUDA-core GEMM reads nothing of a lower-triangular weight past the last column of a tile (64 wide, K split or not): NaN
+    from there on."""
     from flash_stu_2_b200 import ops
     M, N, K = shape
     torch.manual_seed(7)
     x, W = torch.randn(M, K).to(dt), torch.tril(torch.randn(N, K) / math.sqrt(K)).to(dt)
-    hole = torch.arange(K)[None, :] >= (torch.arange(N)[:, None] // 128 + 1) * 128
+    hole = torch.arange(K)[None, :] >= (torch.arange(N)[:, None] // 64 + 1) * 64
     y = ops.linear(x.to(dev()), W.masked_fill(hole, float("nan")).to(dev()), epilogue=ops.EPI_STORE | ops.EPI_FLAG_CAUSAL, backend=1)
     close(y, _lin_ref(x, W, None, None, 0, dt), TOL[dt] / 2)
     ops.check_status()
