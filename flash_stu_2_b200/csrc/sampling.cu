@@ -466,8 +466,7 @@ __global__ void __launch_bounds__(SP_T) sample_kernel(const T* __restrict__ logi
 // in 49 steps per pass, six passes.  Here a thread holds at most 8 entries, in registers, read once; the four radix
 // passes add the CTAs' histograms through distributed shared memory, every CTA for itself, and the survivors meet in
 // CTA 0, which cuts and draws as sample_row does: the same token.  More survivors than the list holds (ties): CTA 0
-// runs sample_row.  50257 entries: top-k 100 with a nucleus 79 -> 27 us, 32 rows
-// of top-k 40 97 -> 38 us, greedy fp32 17 -> 7.5 us.
+// runs sample_row.  The figures stand at the rule in stu_sample.
 constexpr int SPC = 8, SPC_PER = 8, SPC_TOPK = 256;
 constexpr int SPC_MAX_V = SPC * SP_T * SPC_PER;
 template <typename T>
@@ -620,10 +619,17 @@ extern "C" int stu_sample(const void* logits, long long ld, int B, int V, float 
   // greedy selection makes one pass only: nothing to keep
   const int cache = (do_sample && V <= SP_CACHE_MAX) ? 1 : 0;
   static const int variant = getenv("STU_SAMPLE_VARIANT") ? atoi(getenv("STU_SAMPLE_VARIANT")) : 2;
-  // A cluster per row for up to 64 rows (512 CTAs, two per SM: under two rounds of 27 to 38 us against one of 80 to 100),
-  // where the row fits the cluster's registers; shorter rows than 4096 are one CTA's work, and past SPC_TOPK the survivors
-  // of a bf16 row may well exceed the list.
-  if (V >= 4096 && V <= SPC_MAX_V && B <= 64 && (!do_sample || (top_k > 0 && top_k <= SPC_TOPK))) {
+  // A cluster per row where the row fits the cluster's registers and is long enough to pay for the cluster's barriers.  37
+  // rows are resident (two CTAs per SM), so its time grows with the rows and doubles past 37, while one CTA per row takes
+  // the same time for any number up to 148; past SPC_TOPK the survivors of a bf16 row may well exceed the list.
+  // Measured, us, one CTA and a cluster per row:
+  //   greedy     1 row: 16384 entries 5.9 and 7.1, 50257 13.0 and 7.7; 32 rows: 50257 13.0 and 13.2, 65536 15.8 and 13.4;
+  //              64 rows: 65536 15.9 and 24.0
+  //   top-k 40   1 row: 4096 entries 20.4 and 20.1, 16384 32.8 and 21.2; 32 rows: 4096 21.4 and 27.9, 16384 34.3 and 29.2;
+  //              64 rows: 16384 34.8 and 53.8, 50257 74.0 and 57.9
+  const bool wins = !do_sample ? B <= 32 && V >= 24576 + 768 * B
+                               : top_k > 0 && top_k <= SPC_TOPK && (B <= 32 ? V >= 6144 + 256 * B : B <= 64 && V >= 36864);
+  if (wins && V <= SPC_MAX_V) {
     const int full = V <= SP_CACHE_MAX;
     if (dtype == STU_F32)
       sample_cluster_kernel<float><<<B * SPC, SP_T, 0, st>>>((const float*)logits, ld, V, temperature, top_k, top_p,

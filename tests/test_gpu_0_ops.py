@@ -859,8 +859,19 @@ def test_sampling_row_with_a_nan_logit_draws_uniformly():
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("V", [4096, 4099, 50257, 65536])
 def test_sampling_by_a_cluster_equals_one_cta_per_row(dt, V):
-    """Up to 64 rows the greedy pick and a top-k of at most 256 run on a cluster of CTAs per row, more rows on one CTA per
-    row: the same tokens, with infinities, NaN, ties across the k-th place and more ties than the candidate list holds."""
+    """33 long rows run a top-k of at most 256 on a cluster of CTAs per row, 65 rows on one CTA per row: the same tokens, with
+    infinities, NaN, ties across the k-th place and more ties than the candidate list holds."""
+    _cluster_against_one_cta(dt, V, 33)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,V", [(9, 8447), (9, 8448), (9, 31487), (9, 31488), (32, 14336), (32, 49152), (32, 65536), (10, 10007)])
+def test_sampling_by_a_cluster_of_few_rows(dt, rows, V):
+    """The same on both sides of the lines from which on a cluster takes a row, the greedy pick among them."""
+    _cluster_against_one_cta(dt, V, rows)
+
+
+def _cluster_against_one_cta(dt, V, rows):
     from flash_stu_2_b200 import ops
     torch.manual_seed(10)
     B = 65
@@ -875,11 +886,11 @@ def test_sampling_by_a_cluster_equals_one_cta_per_row(dt, V):
     u = torch.rand(B, device=dev())
     u[7], u[8] = 0.0, 1.0 - 2 ** -24
     for temp, k, p in [(1.0, None, None), (0.8, 40, None), (0.9, 100, 0.9), (1.0, 256, 0.5), (1.0, 1, None), (1.3, 50, 1.0)]:
-        one, many = (torch.full((n,), -1, dtype=torch.int64, device=dev()) for n in (B, 33))
+        one, many = (torch.full((n,), -1, dtype=torch.int64, device=dev()) for n in (B, rows))
         ops.sample(z, temp, k, p, k is not None, u, one)
-        ops.sample(z[:33], temp, k, p, k is not None, u[:33], many)
+        ops.sample(z[:rows], temp, k, p, k is not None, u[:rows], many)
         ops.check_status()
-        assert torch.equal(one[:33], many), (temp, k, p)
+        assert torch.equal(one[:rows], many), (temp, k, p)
         assert bool((many >= 0).all()) and bool((many < V).all())
 
 
