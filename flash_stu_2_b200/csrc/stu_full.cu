@@ -73,19 +73,21 @@ extern "C" int stu_to_history(const void* x, long long x_bstride, long long x_ts
 // (time t = 2m+p reads input time t-j = 2s+p'; the tap index j follows.)  Entries past L and above the
 // diagonal are zero.
 //
-// Bound: the 3 S^2 values written.  A CTA writes 32 rows x 1024 columns: a row is the reversed filter at another offset,
+// Bound: the 3 S^2 values written.  A CTA writes ROWS rows x 1024 columns: a row is the reversed filter at another offset,
 // so the filter's values are gathered once, into as many copies, each shifted by one value, as there are values in 16
 // bytes, and every row is 16-byte reads of the copy that its offset makes aligned and 16-byte stores.  (One value per
-// thread, gathered from the filter column each, took 18 us for S = 1504 in bf16; this form takes 5.2 us.)
-constexpr int TZ_ROWS = 32, TZ_COLS = 1024;
-template <typename T>
+// thread, gathered from the filter column each, took 16 us for S = 1504 in bf16; this form takes 5.1 us.)
+constexpr int TZ_COLS = 1024;
+template <typename T, int ROWS>
 __global__ void __launch_bounds__(256) toeplitz_kernel(const T* __restrict__ f, long long f_stride, int L,
                                                        T* __restrict__ out, int S, long long ld, int vec) {
   constexpr int V = Elem<T>::VEC;
-  __shared__ __align__(16) T tab[V][TZ_COLS + TZ_ROWS];   // tab[c][y]: the value at m - s = m_last - s0 - (y + c)
-  const int kind = blockIdx.z, m0 = blockIdx.y * TZ_ROWS, s0 = blockIdx.x * TZ_COLS;
-  for (int y = threadIdx.x; y < TZ_COLS + TZ_ROWS; y += 256) {
-    const int i = m0 + TZ_ROWS - 1 - (s0 + y), j = 2 * i + (kind == 0 ? 0 : (kind == 1 ? 1 : -1));
+  static_assert(ROWS % V == 0, "the table's last row");
+  __shared__ __align__(16) T tab[V][TZ_COLS + ROWS];   // tab[c][y]: the value at m - s = m_last - s0 - (y + c)
+  const int kind = blockIdx.z, m0 = blockIdx.y * ROWS, s0 = blockIdx.x * TZ_COLS;
+  const int cols = min(TZ_COLS, S - s0), rows = min(ROWS, S - m0);
+  for (int y = threadIdx.x; y < (cols + V - 1) / V * V + ROWS; y += 256) {
+    const int i = m0 + ROWS - 1 - (s0 + y), j = 2 * i + (kind == 0 ? 0 : (kind == 1 ? 1 : -1));
     const T v = i >= 0 && j >= 0 && j < L ? f[(size_t)j * f_stride] : Elem<T>::from_f(0.f);
 #pragma unroll
     for (int c = 0; c < V; c++)
@@ -93,18 +95,33 @@ __global__ void __launch_bounds__(256) toeplitz_kernel(const T* __restrict__ f, 
   }
   __syncthreads();
   T* o = out + (size_t)kind * S * ld + s0;
-  const int cols = min(TZ_COLS, S - s0), rows = min(TZ_ROWS, S - m0);
-  for (int e = threadIdx.x; e < rows * (TZ_COLS / V); e += 256) {
-    const int r = e / (TZ_COLS / V), s = e % (TZ_COLS / V) * V, off = TZ_ROWS - 1 - r;   // row m0 + r starts at tab[0][off]
-    if (s >= cols) continue;
-    const T* src = &tab[off % V][s + off - off % V];
-    T* dst = o + (size_t)(m0 + r) * ld + s;
-    if (vec && s + V <= cols) {
-      *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-    } else {
-      for (int x = 0; x < V && s + x < cols; x++) dst[x] = src[x];
+  for (int r = threadIdx.x >> 5; r < rows; r += 8) {
+    const int off = ROWS - 1 - r;   // row m0 + r starts at tab[0][off]
+    const T* row = &tab[off % V][off - off % V];
+    T* dst = o + (size_t)(m0 + r) * ld;
+    for (int s = (threadIdx.x & 31) * V; s < cols; s += 32 * V) {
+      if (vec && s + V <= cols) {
+        *reinterpret_cast<uint4*>(dst + s) = *reinterpret_cast<const uint4*>(row + s);
+      } else {
+        for (int x = 0; x < V && s + x < cols; x++) dst[s + x] = row[s + x];
+      }
     }
   }
+}
+
+template <typename T>
+static int launch_toeplitz(const void* f, long long f_stride, int L, void* out, int S, long long ld, cudaStream_t st) {
+  const int vec = aligned16(out) && ld % Elem<T>::VEC == 0;
+  // Rows per CTA: 8 while 32 would leave most of the chip without a CTA (bf16, S = 504: 2.6 against 3.9 us; S = 1504: 6.9
+  // against 5.1)
+  const int per = S <= 1024 ? 8 : 32;
+  const long long tiles = ((long long)S + per - 1) / per;
+  if (tiles > 65535) return STU_ERR_UNSUPPORTED;
+  const dim3 grid((S + TZ_COLS - 1) / TZ_COLS, (unsigned)tiles, 3);
+  if (per == 8) toeplitz_kernel<T, 8><<<grid, 256, 0, st>>>((const T*)f, f_stride, L, (T*)out, S, ld, vec);
+  else toeplitz_kernel<T, 32><<<grid, 256, 0, st>>>((const T*)f, f_stride, L, (T*)out, S, ld, vec);
+  STU_CHECK_LAUNCH();
+  return STU_OK;
 }
 
 extern "C" int stu_toeplitz(const void* f, long long f_stride, int L, void* out, int S, long long ld, int dtype,
@@ -112,18 +129,9 @@ extern "C" int stu_toeplitz(const void* f, long long f_stride, int L, void* out,
   if (!f || !out) return STU_ERR_NULL;
   if (L <= 0 || S <= 0 || ld < S) return STU_ERR_SHAPE;
   cudaStream_t st = (cudaStream_t)stream;
-  const long long rows = (S + TZ_ROWS - 1) / TZ_ROWS;
-  if (rows > 65535) return STU_ERR_UNSUPPORTED;
-  const dim3 grid((S + TZ_COLS - 1) / TZ_COLS, (unsigned)rows, 3);
-  const int vec = aligned16(out) && ld % (dtype == STU_F32 ? 4 : 8) == 0;
-  if (dtype == STU_F32)
-    toeplitz_kernel<float><<<grid, 256, 0, st>>>((const float*)f, f_stride, L, (float*)out, S, ld, vec);
-  else if (dtype == STU_BF16)
-    toeplitz_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)f, f_stride, L, (bf16*)out, S, ld, vec);
-  else
-    return STU_ERR_DTYPE;
-  STU_CHECK_LAUNCH();
-  return STU_OK;
+  if (dtype == STU_F32) return launch_toeplitz<float>(f, f_stride, L, out, S, ld, st);
+  if (dtype == STU_BF16) return launch_toeplitz<bf16>(f, f_stride, L, out, S, ld, st);
+  return STU_ERR_DTYPE;
 }
 
 // U[(b, t - t0)][sign*K*d + k*d + i] = round(E[(b,i,p)][m] +- Q[(b,i,p)][m]),  t = 2m + p in [t0, t_end).

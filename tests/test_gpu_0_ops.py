@@ -1081,3 +1081,25 @@ def test_mini_stu_lds_prefill_and_recurrent_decode(golden, dt, tol, shape):
         with torch.no_grad():
             y2 = m2(g["x"].to(dt).to(dev()))
         close(y2, g["y"], 1e-3)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("S,ld,L", [(1, 1, 3), (7, 8, 40), (8, 8, 16), (9, 16, 9), (33, 35, 60), (264, 264, 700), (1024, 1024, 4096),
+                                    (1025, 1032, 900), (2056, 2060, 5000)])
+def test_toeplitz_matrices_of_any_size(dt, S, ld, L):
+    """The three matrices of a filter on both sides of the change from 8 to 32 rows per CTA, over several column tiles, with
+    rows on and off the 16-byte grid, filters shorter than the matrices; nothing is written between the rows."""
+    from flash_stu_2_b200 import _lib
+    torch.manual_seed(3)
+    phi = torch.randn(L, 3).to(dt)
+    out = torch.full((3, S, ld), 7.0, dtype=dt, device=dev())
+    col = phi.to(dev())[:, 1]
+    rc = _lib.load().stu_toeplitz(col.data_ptr(), 3, L, out.data_ptr(), S, ld, int(dt == torch.bfloat16),
+                                  torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    lag = torch.arange(S)[:, None] - torch.arange(S)[None, :]
+    for kind, tap in enumerate((2 * lag, 2 * lag + 1, 2 * lag - 1)):
+        f = phi[:, 1][tap.clamp(0, L - 1)]
+        want = torch.where((lag >= 0) & (tap >= 0) & (tap < L), f, torch.zeros((), dtype=dt))
+        assert torch.equal(out[kind, :, :S].cpu(), want), kind
+    assert bool((out[:, :, S:] == 7.0).all())
