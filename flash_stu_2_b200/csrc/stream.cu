@@ -397,15 +397,29 @@ template <int EPI, bool NORM, int NR, int MM>
 int launch_f32(const float* x, long long lda, const float* W, long long ldb, const float* W2, int M, int N, int K,
                const EpiArgs<float>& ep, const float* nw, float eps, int early, cudaStream_t st) {
   constexpr int TF = (EPI == EPI_GELU_MUL) ? NR / 2 : NR, NV = NR * MM;
-  const int nchunks = (K + 127) / 128;
-  int wk = 1;
-  while (wk < NW && wk < nchunks) wk *= 2;
-  // one CTA per SM; more only where its partial sums would need more than 64 KB
-  const int max_rows = 65536 / (wk * NV * 4) * TF;
-  int grid = N < device_sm_count() ? N : device_sm_count();
-  if ((N + grid - 1) / grid > max_rows) grid = (N + max_rows - 1) / max_rows;
-  const int groups = ((N + grid - 1) / grid + TF - 1) / TF;
-  const size_t smem = (size_t)2 * (NR + M + (NORM ? 1 : 0)) * THREADS * 16 + (size_t)groups * wk * NV * 4;
+  const int nchunks = (K + 127) / 128, sms = device_sm_count();
+  // the split that leaves the fewest chunks to the busiest warp: 6 chunks of K over 8 warps idle two of them, over 2 warps
+  // of 4 teams none (8 rows: 9216 x 768 16.9 -> 11.5 us, gate/up 34.1 -> 21.2; 1 row: 4608 x 1536 7.3 -> 6.7)
+  int wk = 1, grid = 1, groups = 1, least = 0;
+  for (int w = NW; w >= 1; w /= 2) {
+    if (w > 1 && w / 2 >= nchunks) continue;
+    // one CTA per SM; where its partial sums would need more than 64 KB, rounds of one per SM
+    const int max_rows = 65536 / (w * NV * 4) * TF;
+    int n = N < sms ? N : sms;
+    if ((N + n - 1) / n > max_rows) n = ((N + max_rows - 1) / max_rows + sms - 1) / sms * sms;
+    const int gr = ((N + n - 1) / n + TF - 1) / TF, teams = NW / w;
+    const int chunks = (n + sms - 1) / sms * ((gr + teams - 1) / teams) * ((nchunks + w - 1) / w);
+    if (least == 0 || chunks < least) {
+      least = chunks;
+      wk = w;
+      grid = n;
+      groups = gr;
+    }
+  }
+  size_t smem = (size_t)2 * (NR + M + (NORM ? 1 : 0)) * THREADS * 16 + (size_t)groups * wk * NV * 4;
+  // 128 rows per SM and more at 5 to 8 rows of x: one CTA per SM for certain.  Where two fit, CTAs that start behind a short
+  // kernel pair up on the SMs that are free first and others stay idle (8 rows, 40000 x 768 behind a norm: 70 us for 46)
+  if (MM == 8 && N > 128 * sms && smem < 116 * 1024) smem = 116 * 1024;
   auto k = stream_f32_kernel<EPI, NORM, NR, MM>;
   static SmemLimit limit;
   const cudaError_t granted = allow_smem((const void*)k, 200 * 1024, limit);
@@ -452,12 +466,16 @@ int dispatch_norm(const void* A, long long lda, const void* B, long long ldb, co
 // bf16: from 64 KB of weights and 31 features per SM on.  Below that the launch is latency and the 8-feature kernel,
 // which keeps nothing in shared memory, is as fast or faster (chain of dependent launches, 1 row: 1536 x 1536 2.9
 // against 2.5 us, 1024 x 4096 6.2 against 3.4 us; 8 rows: gate/up 4096 x 1024 a tie), above it this one is (1 row:
-// 4608 x 1536 7.4 -> 5.0 us, gate/up 6144 x 1536 14.7 -> 8.6 us = 4.4 TB/s; 8 rows: 8.3 -> 7.1 and 15.9 -> 11.4 us).  fp32: always (512-wide model, 2 rows: gate/up 6144 x 512 10.6 -> 7.2 us, down 7.8 -> 5.1 us).
+// 4608 x 1536 7.4 -> 5.0 us, gate/up 6144 x 1536 14.7 -> 8.6 us = 4.4 TB/s; 8 rows: 8.3 -> 7.1 and 15.9 -> 11.4 us).
+// fp32: all (512-wide model, 2 rows: gate/up 6144 x 512 10.6 -> 7.2 us, down 7.8 -> 5.1 us) but the widest gate/up products of
+// 5 to 8 rows, which the upkeep of the rings slows down (8 rows with the norm, us, this kernel and the one of skinny.cu
+// behind a norm kernel: 4608 x 1536 26.6 and 31.5, 6144 x 1536 34.6 and 32.0, 9216 x 768 26.3 and 23.2, 12288 x 3072
+// 117 and 90).  A caller that asks for the fused norm gets it, whatever the width.
 bool stream_takes(int M, int N, int K, int epi, int dtype, const void* norm_w, bool peer) {
   if (M > 8 || peer || (epi != EPI_STORE && epi != EPI_RESID && epi != EPI_GELU_MUL)) return false;
   if (norm_w && !aligned16(norm_w)) return false;
-  if (dtype == STU_F32) return true;
   const long long sms = device_sm_count();
+  if (dtype == STU_F32) return norm_w || epi != EPI_GELU_MUL || M <= 4 || N <= 37 * sms;
   return N > 30 * sms && (long long)N * K * (epi == EPI_GELU_MUL ? 4 : 2) >= 65536 * sms;
 }
 
