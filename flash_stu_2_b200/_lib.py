@@ -73,6 +73,7 @@ _SIGNATURES = {
                                c_float, _P, _LL, c_int, _P, c_int, _P], c_int),
     "stu_token_step_workspace_bytes": ([c_int, c_int, c_int, c_int], c_longlong),
     "stu_token_step_supported": ([c_int, c_int, c_int, c_int, c_int, c_int], c_int),
+    "stu_token_step_ring_slots": ([c_int, c_int, c_int, c_int], c_int),
     "stu_token_step_plan_bytes": ([c_int], c_longlong),
     "stu_token_step_plan": ([_P, _P, c_int, _P], c_int),
     "stu_token_step_walk": ([_P, c_int, _P, c_int], c_int),

@@ -891,6 +891,12 @@ extern "C" int stu_token_step_supported(int n_layers, int B, int d, int I, int H
   return ring_slots(B, d, I, dtype) >= 24 ? 1 : 0;
 }
 
+// Row slots of the weight ring that stu_token_step has for these sizes.
+extern "C" int stu_token_step_ring_slots(int B, int d, int I, int dtype) {
+  if ((dtype != STU_BF16 && dtype != STU_F32) || B < 1 || B > 8 || d < 1 || I < 1) return 0;
+  return ring_slots(B, d, I, dtype);
+}
+
 extern "C" long long stu_token_step_plan_bytes(int n_layers) {
   return n_layers < 1 || n_layers > MAXL ? 0 : (5ll * n_layers + 1) * sizeof(Stage) + (long long)n_layers * sizeof(StuStepLayer);
 }

@@ -251,8 +251,9 @@ class FlashSTU(PreTrainedModel):
             if do_sample:
                 u = uniforms[step].to(device=dev, dtype=torch.float32).contiguous() if uniforms is not None else \
                     torch.rand(B, device=dev, generator=generator)
-            if step == 1 and fits and plain and not eager and ops.fused_step and TokenStep.supported(self.layers, past, B, self.config.n_embd,
-                                                                    self.config.torch_dtype, self):
+            if step == 1 and fits and plain and not eager and ops.fused_step and TokenStep.supported(
+                    self.layers, past, B, self.config.n_embd, self.config.torch_dtype, self) and TokenStep.pays(
+                    self.layers, B, self.config.n_embd, self.config.torch_dtype, cur - 1, steps - 1):
                 x = torch.empty(B, self.config.n_embd, dtype=self.config.torch_dtype, device=dev)
                 stepper = TokenStep(self.layers, past, B, x, model=self)
                 V = self.lm_head.weight.shape[0]

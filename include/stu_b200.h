@@ -406,6 +406,7 @@ typedef struct {
 
 long long stu_token_step_workspace_bytes(int d, int I, int H, int dtype);
 int stu_token_step_supported(int n_layers, int B, int d, int I, int H, int dtype);   /* 1: stu_token_step takes it */
+int stu_token_step_ring_slots(int B, int d, int I, int dtype);   /* row slots of its weight ring: how deep the stream runs */
 /* The plan (stu_token_step_plan_bytes bytes of HOST memory): checks the descriptors; returns the number of stages or an
  * error (< 0).  The caller copies it to the device once; it holds addresses, so it serves as long as they do. */
 long long stu_token_step_plan_bytes(int n_layers);

@@ -111,3 +111,27 @@ def test_layers_that_somebody_overrides_or_listens_to_are_called(change):
     assert _takes(m)
     change(m)
     assert not _takes(m)
+
+
+@pytest.mark.parametrize("d,layers,heads,mlp,dt,B,t,steps,attn,want", [
+    (1024, 4, 16, 4, torch.bfloat16, 8, 12000, 64, False, False),    # a long history: the decode kernels stream it faster
+    (1024, 4, 16, 4, torch.bfloat16, 8, 100, 1000, False, False),    # the block step kernel, the capture long paid for
+    (1024, 4, 16, 4, torch.bfloat16, 8, 100, 12, False, True),       # ... and not
+    (1536, 24, 12, 4, torch.bfloat16, 1, 333, 64, True, True), (1536, 4, 12, 4, torch.bfloat16, 8, 12000, 64, False, False),
+    (512, 12, 8, 12, torch.float32, 2, 128, 127, True, True), (512, 4, 8, 4, torch.float32, 8, 4000, 64, False, False),
+    (3072, 4, 24, 4, torch.bfloat16, 1, 100, 64, True, False), (1536, 4, 24, 4, torch.float32, 4, 100, 64, True, False)])
+def test_form_of_the_step_follows_what_was_measured(d, layers, heads, mlp, dt, B, t, steps, attn, want):
+    class Attn:
+        n_heads, window = heads, 1024
+
+    class Mlp:
+        intermediate_size = mlp * d
+
+    class StuLayer:
+        mlp, stu = Mlp, None
+
+    class AttnLayer:
+        mlp, attn = Mlp, Attn
+
+    stack = [AttnLayer if attn and i % 2 else StuLayer for i in range(layers)]
+    assert TokenStep.pays(stack, B, d, dt, t, steps) is want
