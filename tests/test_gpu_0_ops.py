@@ -1103,3 +1103,22 @@ def test_toeplitz_matrices_of_any_size(dt, S, ld, L):
         want = torch.where((lag >= 0) & (tap >= 0) & (tap < L), f, torch.zeros((), dtype=dt))
         assert torch.equal(out[kind, :, :S].cpu(), want), kind
     assert bool((out[:, :, S:] == 7.0).all())
+
+
+@pytest.mark.parametrize("shape", [(8, 200, 768, 0), (5, 40001, 132, 0), (8, 19000, 772, 1), (1, 300, 1540, 0), (7, 5476, 260, 2), (7, 5477, 260, 2),
+                                   (3, 97, 1284, 1), (6, 64, 4, 0), (8, 1, 640, 0)])
+def test_fp32_linears_of_up_to_8_rows_at_the_edges_of_their_split(shape):
+    """1 to 13 chunks of K over 1 to 8 warps, one and several rounds of CTAs, the widths around which a product of 5 to 8 rows
+    changes kernels, with the norm fused and apart."""
+    from flash_stu_2_b200 import ops
+    M, N, K, epi = shape
+    torch.manual_seed(15)
+    x, nw = torch.randn(M, K), 1.0 + 0.1 * torch.randn(K)
+    W, W2, resid = torch.randn(N, K) / math.sqrt(K), torch.randn(N, K) / math.sqrt(K), torch.randn(M, N)
+    kw = dict(W2=W2.to(dev()) if epi == 2 else None, resid=resid.to(dev()) if epi == 1 else None, epilogue=epi)
+    y = ops.linear(x.to(dev()), W.to(dev()), **kw)
+    close(y, _lin_ref(x, W, W2, resid, epi, torch.float32), TOL[torch.float32] / 2)
+    xn = x * torch.rsqrt(x.pow(2).mean(1, keepdim=True) + ops.RMS_EPS) * nw
+    y = ops.linear(x.to(dev()), W.to(dev()), norm_w=nw.to(dev()), **kw)
+    close(y, _lin_ref(xn, W, W2, resid, epi, torch.float32), TOL[torch.float32] / 2)
+    ops.check_status()
