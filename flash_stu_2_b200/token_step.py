@@ -119,13 +119,14 @@ class TokenStep:
         """Whether `steps` steps from position t on take less time as persistent launches than replayed from a graph.
 
         A layer's part of the persistent step beyond (below zero: less than) its kernels', in microseconds, from 290 pairs
-        of 4-layer models on one B200 (d 256 to 3072, 1 to 8 sequences, positions 100 to 12000; the choice then costs 0.5 %
-        of the better form on average, 20 % at worst).  The tap sums over the history are what decides: the persistent
+        of 4-layer models on one B200 (d 256 to 3072, 1 to 8 sequences, positions 100 to 12000).  The tap sums over the history are what decides: the persistent
         kernel takes them at 2 TB/s (fp32: 1), the decode kernels at 5 and more.  bf16, STU layers only, 8 sequences, us per
         step, persistent and graph: d = 1024 at 100 117 and 93, at 12000 355 and 144; d = 1536 156 and 181, 550 and 278.
         Below two units of 16 rows in the weight ring the stream stops between units: d = 3072, 1 sequence 378 and 335;
         fp32 d = 1536, 1 sequence 209 and 274, 4 sequences 310 and 287.
-        Against that a graph's two eager steps, capture and instantiation cost 1.2 ms and 0.12 ms per layer."""
+        Against that a graph's two eager steps, capture and instantiation cost 1.2 ms and 0.12 ms per layer on an idle
+        host, and 20 to 170 ms now and then on a busy one, where the persistent steps take what they always take: it has
+        to gain twice the former."""
         bf16, inter = dtype == torch.bfloat16, layers[0].mlp.intermediate_size
         if _lib.load().stu_token_step_ring_slots(batch, d, inter, int(bf16)) < 31 and (bf16 or batch > 2):
             return False
@@ -146,7 +147,7 @@ class TokenStep:
                         beyond += 12
                 else:
                     beyond += 4.5 - 0.018 * keys + 0.0016 * batch * keys
-        return beyond * steps < 1200 + 120 * len(layers)
+        return beyond * steps < 2 * (1200 + 120 * len(layers))
 
     def run(self, ids: Optional[torch.Tensor] = None, logits: Optional[torch.Tensor] = None):
         """One token per sequence: ids [B] int64 (any stride; None: the rows are in x), logits [B,V] rows."""
