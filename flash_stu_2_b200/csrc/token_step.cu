@@ -24,8 +24,8 @@
 // Every wait is bounded: on expiry the status word is raised, outstanding copies are let land and every CTA returns.  The
 // caches, positions and outputs are then undefined, and the workspace is marked: launches on it return at once with the
 // same status (their barriers would start from a counter that was left half way) until it is zeroed.
+#include "../../include/stu_b200.h"   // the descriptors
 #include "common.cuh"
-#include "stu_step.cuh"
 #include "tma.cuh"
 
 int device_sm_count();   // gemm_tc.cu
@@ -102,6 +102,7 @@ struct Stage {
 struct Range { int r0, r1; };   // this CTA's features of a stage
 constexpr int MAX_STAGES = 5 * MAXL + 1;
 static_assert(sizeof(Stage) == 32 && sizeof(StuStepLayer) == 128, "the plan is copied in 16-byte pieces");
+static_assert(sizeof(StuStepArgs) == 128, "as in the Python binding");
 
 struct Params {
   StuStepArgs a;

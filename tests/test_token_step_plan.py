@@ -26,6 +26,17 @@ def _plan(d, inter, B, heads, bf16, V=50257, layers=4):
     return a, blob, n
 
 
+def test_descriptors_of_the_binding_have_the_layout_of_the_header():
+    """What the binding fills in is what the library copies out of it: sizes, and one field from each end."""
+    lib = _lib.load()
+    stages = 5 * 32
+    assert lib.stu_token_step_plan_bytes(2) - lib.stu_token_step_plan_bytes(1) - stages == ctypes.sizeof(_lib.StepLayer) == 128
+    a, blob, n = _plan(512, 2048, 2, 8, True)
+    table = (_lib.StepLayer * 4).from_buffer_copy(bytes(blob)[n * 32:n * 32 + 4 * 128])
+    assert [L.kind for L in table] == [0, 1, 0, 1] and all(L.Lh == 64 and L.W == 9 and L.norm1 == L.pos == A for L in table)
+    assert _lib.StepArgs.status.offset == ctypes.sizeof(_lib.StepArgs) - 8 == 120
+
+
 def _stall(d, inter, B, heads, bf16):
     a, blob, n = _plan(d, inter, B, heads, bf16)
     assert n > 0
