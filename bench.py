@@ -1060,8 +1060,8 @@ def run_model(a):
         res[graph] = (t_first, t_full, out)
     ops.check_status()
     t_first, t_full, out = res[True]
-    # token steps: device time of the graph-replayed steps alone (the two eager steps and the capture before them are
-    # host work that varies by milliseconds from run to run, which makes differences of whole-run times useless)
+    # token steps: device time of the persistent or graph-replayed steps alone (the eager steps and the capture before
+    # them are host work that varies by milliseconds from run to run, which makes differences of whole-run times useless)
     dec_ms = tm["replay_ms"] / tm["replayed_steps"] * (new - 1) if tm.get("replayed_steps") else t_full - t_first
     n_param = sum(p.numel() for p in model.parameters())
     print(json.dumps({
@@ -1069,7 +1069,7 @@ def run_model(a):
         "n_gpus": 1, "higher_is_better": True, "dtype": spec["dtype"], "data": "synthetic",
         "config": {"workload": f"FlashSTU.generate {a.model}: {cfg['n_layers']} layers d={cfg['n_embd']} "
                                f"V={cfg['vocab_size']} L={L} B={B} prompt {T0} +{new} tokens, {n_param / 1e6:.0f} M parameters",
-                   "sampling": spec["sampling"], "decode_launch": "one CUDA graph per token step"},
+                   "sampling": spec["sampling"], "decode_launch": "one persistent kernel or one CUDA graph per token step"},
         "decode_ms_per_token_step": dec_ms / (new - 1),
         "prefill": {"value": B * T0 / (t_first * 1e-3), "unit": "tokens/s", "ms": t_first},
         "eager_loop": {"decode_tokens_per_s": B * (new - 1) / ((res[False][1] - res[False][0]) * 1e-3),
