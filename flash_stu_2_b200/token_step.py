@@ -125,8 +125,8 @@ class TokenStep:
         Below two units of 16 rows in the weight ring the stream stops between units: d = 3072, 1 sequence 378 and 335;
         fp32 d = 1536, 1 sequence 209 and 274, 4 sequences 310 and 287.
         Against that a graph's two eager steps, capture and instantiation cost 1.2 ms and 0.12 ms per layer on an idle
-        host, and 20 to 170 ms now and then on a busy one, where the persistent steps take what they always take: it has
-        to gain twice the former."""
+        host, but 20 to 170 ms in one call of ten on a busy one, where the persistent steps take what they always take
+        (14 layers of d = 512, 54 steps: 21 to 173 ms against 20): four times the former is what it has to gain."""
         bf16, inter = dtype == torch.bfloat16, layers[0].mlp.intermediate_size
         if _lib.load().stu_token_step_ring_slots(batch, d, inter, int(bf16)) < 31 and (bf16 or batch > 2):
             return False
@@ -147,7 +147,7 @@ class TokenStep:
                         beyond += 12
                 else:
                     beyond += 4.5 - 0.018 * keys + 0.0016 * batch * keys
-        return beyond * steps < 2 * (1200 + 120 * len(layers))
+        return beyond * steps < 4 * (1200 + 120 * len(layers))
 
     def run(self, ids: Optional[torch.Tensor] = None, logits: Optional[torch.Tensor] = None):
         """One token per sequence: ids [B] int64 (any stride; None: the rows are in x), logits [B,V] rows."""
