@@ -398,11 +398,15 @@ int launch_f32(const float* x, long long lda, const float* W, long long ldb, con
                const EpiArgs<float>& ep, const float* nw, float eps, int early, cudaStream_t st) {
   constexpr int TF = (EPI == EPI_GELU_MUL) ? NR / 2 : NR, NV = NR * MM;
   const int nchunks = (K + 127) / 128, sms = device_sm_count();
-  // the split that leaves the fewest chunks to the busiest warp: 6 chunks of K over 8 warps idle two of them, over 2 warps
-  // of 4 teams none (8 rows: 9216 x 768 16.9 -> 11.5 us, gate/up 34.1 -> 21.2; 1 row: 4608 x 1536 7.3 -> 6.7)
+  // Of the splits over 8 and 4 warps the one that leaves the fewest chunks to the busiest warp: 12 chunks of K over 8 warps
+  // take two rounds of which half is idle, over 4 warps of 2 teams three full ones (8 rows: 4608 x 1536 13.4 -> 11.2 us,
+  // 50257 x 1536 186 -> 103 with whole rounds of CTAs; 1 row: 4608 x 1536 7.3 -> 6.7).  Beyond three
+  // chunks a warp, or over 2 warps, the results' error grows with the sums of a lane (K = 768 over 2 warps: 9.3e-8 for
+  // 8.8e-8, 2304 over 4: 1.07e-7 for 1.02e-7).
   int wk = 1, grid = 1, groups = 1, least = 0;
   for (int w = NW; w >= 1; w /= 2) {
     if (w > 1 && w / 2 >= nchunks) continue;
+    if (least && (w < 4 || nchunks > 3 * w)) break;
     // one CTA per SM; where its partial sums would need more than 64 KB, rounds of one per SM
     const int max_rows = 65536 / (w * NV * 4) * TF;
     int n = N < sms ? N : sms;
@@ -469,13 +473,19 @@ int dispatch_norm(const void* A, long long lda, const void* B, long long ldb, co
 // 4608 x 1536 7.4 -> 5.0 us, gate/up 6144 x 1536 14.7 -> 8.6 us = 4.4 TB/s; 8 rows: 8.3 -> 7.1 and 15.9 -> 11.4 us).
 // fp32: all (512-wide model, 2 rows: gate/up 6144 x 512 10.6 -> 7.2 us, down 7.8 -> 5.1 us) but the widest gate/up products of
 // 5 to 8 rows, which the upkeep of the rings slows down (8 rows with the norm, us, this kernel and the one of skinny.cu
-// behind a norm kernel: 4608 x 1536 26.6 and 31.5, 6144 x 1536 34.6 and 32.0, 9216 x 768 26.3 and 23.2, 12288 x 3072
-// 117 and 90).  A caller that asks for the fused norm gets it, whatever the width.
+// behind a norm kernel: 4608 x 1536 26.6 and 31.5, 5120 x 1280 29.0 and 26.1, 6144 x 1536 34.6 and 32.0, 9216 x 768 26.3 and 23.2, 12288 x 3072
+// 117 and 90) and wide heads of 5 to 8 rows whose K leaves a quarter of the warps idle (8 x 40000 x 768: 70 and 60).  A caller
+// that asks for the fused norm gets it, whatever the width.
 bool stream_takes(int M, int N, int K, int epi, int dtype, const void* norm_w, bool peer) {
   if (M > 8 || peer || (epi != EPI_STORE && epi != EPI_RESID && epi != EPI_GELU_MUL)) return false;
   if (norm_w && !aligned16(norm_w)) return false;
   const long long sms = device_sm_count();
-  if (dtype == STU_F32) return norm_w || epi != EPI_GELU_MUL || M <= 4 || N <= 37 * sms;
+  if (dtype == STU_F32) {
+    if (norm_w || M <= 4) return true;
+    if (epi == EPI_GELU_MUL) return N <= 32 * sms;
+    const int chunks = (K + 127) / 128, warps = chunks < 3 ? chunks : 4;   // see launch_f32
+    return N <= 128 * sms || 5 * chunks > 4 * ((chunks + warps - 1) / warps * warps);
+  }
   return N > 30 * sms && (long long)N * K * (epi == EPI_GELU_MUL ? 4 : 2) >= 65536 * sms;
 }
 

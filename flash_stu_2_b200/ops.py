@@ -184,9 +184,9 @@ def embed(ids: torch.Tensor, table: torch.Tensor):
 
 def can_fuse_norm(M: int, N: int, K: int, epilogue: int, dtype: torch.dtype) -> bool:
     if dtype == torch.float32:
-        # 5 to 8 rows: gate/up products from 37 features per SM on run on another kernel, and for wide heads the scaling
+        # 5 to 8 rows: gate/up products of more than 32 features per SM run on another kernel, and for wide heads the scaling
         # of every value by every warp costs more than a launch (8 rows, 50257 x 1536: 120 us fused, 106 apart)
-        wide = N > (5476 if epilogue == EPI_GELU_MUL else 18944)
+        wide = N > (4736 if epilogue == EPI_GELU_MUL else 18944)
         return M <= (4 if wide else 8) and K % 4 == 0 and epilogue in (EPI_STORE, EPI_RESID, EPI_GELU_MUL)
     return bool(_lib.load().stu_linear_can_fuse_norm(M, N, K, epilogue, 1))
 

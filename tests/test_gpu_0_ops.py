@@ -1105,8 +1105,8 @@ def test_toeplitz_matrices_of_any_size(dt, S, ld, L):
     assert bool((out[:, :, S:] == 7.0).all())
 
 
-@pytest.mark.parametrize("shape", [(8, 200, 768, 0), (5, 40001, 132, 0), (8, 19000, 772, 1), (1, 300, 1540, 0), (7, 5476, 260, 2), (7, 5477, 260, 2),
-                                   (3, 97, 1284, 1), (6, 64, 4, 0), (8, 1, 640, 0)])
+@pytest.mark.parametrize("shape", [(8, 200, 768, 0), (5, 40001, 132, 0), (8, 19000, 772, 1), (1, 300, 1540, 0), (7, 4736, 260, 2), (7, 4737, 260, 2),
+                                   (3, 97, 1284, 1), (6, 64, 4, 0), (8, 1, 640, 0), (6, 18945, 768, 0), (6, 18944, 768, 0)])
 def test_fp32_linears_of_up_to_8_rows_at_the_edges_of_their_split(shape):
     """1 to 13 chunks of K over 1 to 8 warps, one and several rounds of CTAs, the widths around which a product of 5 to 8 rows
     changes kernels, with the norm fused and apart."""
