@@ -247,9 +247,11 @@ class STU(nn.Module):
         U = torch.empty(B * T, nsign * K * d, dtype=xn.dtype, device=xn.device)
         if xn.dtype == torch.float32:
             # fp32 sums run on the CUDA cores: all filters in one launch (24 filters, 8 x 1000 positions of 64 channels:
-            # 122 launches, 1.35 ms -> 1 launch, 0.43 ms; products of bf16 models belong on the tensor cores, one filter at a time)
+            # 122 launches, 1.35 ms -> 1 launch, 0.43 ms)
             ops.full_conv(hist, phi, U, nsign == 2, t0, t0 + T)
-        else:
+        elif ops.full_conv_tc5_supported(hist):
+            ops.full_conv_tc5(hist, phi, U, nsign == 2, t0, t0 + T)
+        else:   # channels that are no whole 16 bytes: one filter at a time, through the GEMM
             S = _round_up((t0 + T + 1) // 2, 8)
             rows = hist.view(B * d * 2, Lh)[:, :S]
             even_in = hist.view(B * d, 2, Lh)[:, 0, :S]

@@ -531,6 +531,24 @@ def full_conv(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     _count()
 
 
+def full_conv_tc5_supported(hist) -> bool:
+    return hist.dtype == torch.bfloat16 and hist.shape[1] % 8 == 0 and hist.shape[3] % 8 == 0 and hist.data_ptr() % 16 == 0
+
+
+def full_conv_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
+    """full_conv for bf16 on the tcgen05 tensor cores."""
+    _cuda(hist, phi, U)
+    B, d, _, Lh = hist.shape
+    L, K = phi.shape
+    assert hist.is_contiguous() and phi.is_contiguous() and U.stride(1) == 1 and U.shape[0] == B * (t_end - t0)
+    lib = _lib.load()
+    tab = torch.empty(lib.stu_full_conv_tc5_scratch_elems(K, t_end), dtype=hist.dtype, device=hist.device)
+    rc = lib.stu_full_conv_tc5(hist.data_ptr(), Lh, phi.data_ptr(), L, K, tab.data_ptr(), U.data_ptr(), U.stride(0), B, d,
+                               int(both_signs), t0, t_end, status_word(hist.device).data_ptr(), _dt(hist), _stream())
+    _lib.check(rc, "stu_full_conv_tc5")
+    _count(2)
+
+
 def full_decode_prepare(x2d, hist, phi, pos, PhiT):
     _cuda(x2d, hist, phi, pos, PhiT)
     B, d, _, Lh = hist.shape

@@ -221,6 +221,11 @@ int stu_full_combine(const void* E, const void* Q, long long ldE, void* U, long 
  * hist [B*d][2][Lh] holds the inputs of times [0, t_end), phi [L][K], Lh a multiple of 4. */
 int stu_full_conv(const void* hist, int Lh, const void* phi, int L, int K, void* U, long long ldU, int B, int d,
                   int both_signs, int t0, int t_end, int dtype, void* stream);
+/* The same for bf16 on the tcgen05 tensor cores: d, Lh and ldU multiples of 8; scratch holds
+ * stu_full_conv_tc5_scratch_elems bf16 values (the taps of all filters as operand tables). */
+long long stu_full_conv_tc5_scratch_elems(int K, int t_end);
+int stu_full_conv_tc5(const void* hist, int Lh, const void* phi, int L, int K, void* scratch, void* U, long long ldU, int B,
+                      int d, int both_signs, int t0, int t_end, int* status, int dtype, void* stream);
 
 /* One cached decode step of the full variant, around one GEMM G = hist_rows @ PhiT^T (stu_linear, M = B*d*2,
  * N = 2K, K = Lh): prepare appends x_t at time pos[0] and rebuilds PhiT [2K][Lh] (time-reversed even / odd

@@ -966,6 +966,36 @@ def test_full_convolution_of_all_filters(shape, both):
     assert bool((U[:, -4:] == 7.0).all())
 
 
+@pytest.mark.parametrize("shape", [(1, 5, 40, 300, 0, 90), (3, 24, 72, 200, 61, 200), (2, 3, 136, 1400, 258, 1301),
+                                   (5, 2, 64, 700, 640, 641), (2, 24, 264, 900, 0, 777), (1, 24, 512, 512, 0, 512)])
+@pytest.mark.parametrize("both", [True, False])
+def test_full_convolution_on_tensor_cores(shape, both):
+    """The bf16 operand U against float64 sums: tiles of 64, 128 and 256 channels, fewer channels than a tile, tiles that hold
+    several sequences, one and several blocks of positions, ranges that start inside the history, one position.  Bar: E, Q
+    and their sum are each rounded to bf16 (2^-9 of each), and neither E nor Q exceeds 1.5 times the largest U of its row."""
+    from flash_stu_2_b200 import ops
+    B, K, d, L, t0, t_end = shape
+    torch.manual_seed(15)
+    Lh = ((t_end + 1) // 2 + 8 + 7) // 8 * 8
+    x, phi = torch.randn(B, t_end, d).bfloat16(), (torch.randn(L, K) / 4).bfloat16()
+    hist = torch.full((B, d, 2, Lh), 3.0, dtype=torch.bfloat16, device=dev())   # what lies past the last input has no effect
+    ops.to_history(x.to(dev()), hist, 0)
+    U = torch.full((B * (t_end - t0), (2 if both else 1) * K * d + 8), 7.0, dtype=torch.bfloat16, device=dev())
+    assert ops.full_conv_tc5_supported(hist)
+    ops.full_conv_tc5(hist, phi.to(dev()), U, both, t0, t_end)
+    ops.check_status()
+    f = torch.zeros(max(L, t_end), K, dtype=torch.float64)
+    f[:L] = phi
+    lag = torch.arange(t0, t_end)[:, None] - torch.arange(t_end)[None, :]
+    want = []
+    for sign in (1.0, -1.0)[: 2 if both else 1]:
+        taps = f * torch.where(torch.arange(f.shape[0]) % 2 == 1, sign, 1.0)[:, None]
+        T = torch.where((lag >= 0)[:, :, None], taps[lag.clamp_min(0)], torch.zeros((), dtype=torch.float64))
+        want.append(torch.einsum("tsk,bsi->btki", T, x.double()).reshape(B * (t_end - t0), K * d))
+    close(U[:, :-8], torch.cat(want, 1), 4 * 2 ** -9)
+    assert bool((U[:, -8:] == 7.0).all())
+
+
 @pytest.mark.parametrize("name,tol", [("std_full_float32", 1e-3), ("std_full_bfloat16", 2e-2),
                                        ("hankelL_full_float32", 1e-3), ("std_approx_float32", 1e-3),
                                        ("std_approx_bfloat16", 2e-2), ("hankelL_approx_float32", 1e-3),
