@@ -121,8 +121,7 @@ class STULayer(nn.Module):
         if stu.use_approx:
             entry = stu.decode_step(x2, param(stu_norm, "weight"), stu_norm.eps, entry, mid)
         else:
-            xn = ops.rmsnorm(x2, param(stu_norm, "weight"), stu_norm.eps)
-            entry = stu.full_decode_step(xn, x2, mid, entry)
+            entry = stu.full_decode_step(x2, x2, mid, entry, param(stu_norm, "weight"), stu_norm.eps)
         if ops.can_fuse_norm(B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype):
             mlp.apply_residual(mid, mid, x2, norm_w=param(mlp_norm, "weight"), eps=mlp_norm.eps, overlap=True)
         else:

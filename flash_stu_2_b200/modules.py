@@ -151,6 +151,7 @@ class STU(nn.Module):
                 self.M_phi_minus = nn.Parameter(torch.empty(self.K, self.d_in, self.d_out, dtype=dt))
         self._prep_key = None
         self._prep = None
+        self._taps_key = self._taps = None
         # optional cap on the positions a cache (and the tap tables) are laid out for: a model whose filters span
         # 32768 positions but that will only ever see 9216 keeps 9216-position histories (config.cache_len)
         self.cache_len = getattr(config, "cache_len", None)
@@ -277,8 +278,20 @@ class STU(nn.Module):
             return hist, pos
         return None
 
-    def full_decode_step(self, xn2d: torch.Tensor, resid2d: torch.Tensor, out2d: torch.Tensor, entry):
-        """One cached token of the full variant: out = resid + STU(xn) at the cached position."""
+    def step_taps(self):
+        """[8, 2K, Lh+8]: even and odd taps of the filters as the step kernel reads them, kept per version of phi."""
+        phi = param(self, "phi")
+        key = (phi._version, phi.data_ptr(), self.param_dtype)
+        if self._taps_key != key:
+            with torch.no_grad():
+                f = phi[:self.capacity].to(self.param_dtype).contiguous()
+                odd = ops.taps_even(f[1:], self.Lh) if f.shape[0] > 1 else torch.zeros_like(ops.taps_even(f, self.Lh))
+                self._taps, self._taps_key = ops.taps_rev8(torch.cat([ops.taps_even(f, self.Lh), odd])), key
+        return self._taps
+
+    def full_decode_step(self, x2d: torch.Tensor, resid2d: torch.Tensor, out2d: torch.Tensor, entry, norm_w=None,
+                         eps: float = ops.RMS_EPS):
+        """One cached token of the full variant: out = resid + STU(x) at the cached position (x normalised with norm_w)."""
         hist, pos = entry
         phi, Mcat = self.prepared_full()
         B, d, _, Lh = hist.shape
@@ -286,18 +299,24 @@ class STU(nn.Module):
         t = host_pos(pos)
         if t + 1 > self.capacity:
             raise ValueError(f"sequence position {t + 1} exceeds the capacity {self.capacity} (seq_len={self.seq_len})")
-        key = (B, xn2d.device, xn2d.dtype)
-        if getattr(self, "_dec_scratch_key", None) != key:
-            self._dec_scratch = (torch.zeros(2 * K, Lh, dtype=xn2d.dtype, device=xn2d.device),
-                                 torch.empty(B * d * 2, 2 * K, dtype=xn2d.dtype, device=xn2d.device),
-                                 torch.empty(B, nsign * K * d, dtype=xn2d.dtype, device=xn2d.device))
-            self._dec_scratch_key = key
-        PhiT, G, U = self._dec_scratch
-        ops.full_decode_prepare(xn2d, hist, phi, pos, PhiT)
-        # (PhiT is zero past the position: the history beyond it, here to the end of its capacity, is not read)
-        ops.linear(hist.view(B * d * 2, Lh), PhiT, out=G, kpos=pos)
-        ops.full_decode_combine(G, pos, U, B, d, K, nsign == 2, Lh, advance=True)
-        ops.linear(U, Mcat, resid=resid2d, out=out2d, epilogue=ops.EPI_RESID)
+        if Lh == self.Lh and ops.full_decode_step_supported(x2d, hist, K):
+            U = ops.empty((B, nsign * K * d), x2d.dtype, x2d.device)
+            ops.full_decode_step(x2d, norm_w, eps, hist, self.step_taps(), pos, U, self.capacity, nsign == 2)
+        else:   # fp32, more filters, rows off the 16-byte grid: tap matrices, a GEMM over all history rows, their combination
+            if norm_w is not None:
+                x2d = ops.rmsnorm(x2d, norm_w, eps)
+            key = (B, x2d.device, x2d.dtype)
+            if getattr(self, "_dec_scratch_key", None) != key:
+                self._dec_scratch = (torch.zeros(2 * K, Lh, dtype=x2d.dtype, device=x2d.device),
+                                     torch.empty(B * d * 2, 2 * K, dtype=x2d.dtype, device=x2d.device),
+                                     torch.empty(B, nsign * K * d, dtype=x2d.dtype, device=x2d.device))
+                self._dec_scratch_key = key
+            PhiT, G, U = self._dec_scratch
+            ops.full_decode_prepare(x2d, hist, phi, pos, PhiT)
+            # (PhiT is zero past the position: the history beyond it, here to the end of its capacity, is not read)
+            ops.linear(hist.view(B * d * 2, Lh), PhiT, out=G, kpos=pos)
+            ops.full_decode_combine(G, pos, U, B, d, K, nsign == 2, Lh, advance=True)
+        ops.linear(U, Mcat, resid=resid2d, out=out2d, epilogue=ops.EPI_RESID | (ops.FLAG_OVERLAP if ops.overlap_decode else 0))
         pos._host_t = t + 1
         return hist, pos
 

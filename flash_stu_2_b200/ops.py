@@ -549,6 +549,26 @@ def full_conv_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     _count(2)
 
 
+def full_decode_step_supported(x2d, hist, K: int) -> bool:
+    d = x2d.shape[1]
+    return (x2d.dtype == torch.bfloat16 and K <= 32 and d % 8 == 0 and hist.shape[3] % 8 == 0 and hist.data_ptr() % 16 == 0
+            and x2d.data_ptr() % 16 == 0 and x2d.stride(0) % 8 == 0)
+
+
+def full_decode_step(x2d, norm_w, eps: float, hist, taps8, pos, U, limit: int, both_signs: bool):
+    """U+- [B, (1 or 2)*K*d] of the position after the cached ones: x2d [B,d] (normalised first with norm_w) is appended to
+    hist [B,d,2,Lh], taps8 [8, 2K, Lh+8] holds the even and the odd taps of the filters; pos moves on."""
+    _cuda(x2d, norm_w, hist, taps8, pos, U)
+    B, d, _, Lh = hist.shape
+    K = taps8.shape[1] // 2
+    assert taps8.shape == (8, 2 * K, Lh + 8) and x2d.stride(1) == 1 and U.is_contiguous() and U.numel() == B * (1 + both_signs) * K * d
+    rc = _lib.load().stu_full_decode_step(x2d.data_ptr(), x2d.stride(0), norm_w.data_ptr() if norm_w is not None else None, eps,
+                                          hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), U.data_ptr(), B, d, K, Lh, limit,
+                                          int(both_signs), status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
+    _lib.check(rc, "stu_full_decode_step")
+    _count()
+
+
 def full_decode_prepare(x2d, hist, phi, pos, PhiT):
     _cuda(x2d, hist, phi, pos, PhiT)
     B, d, _, Lh = hist.shape

@@ -227,6 +227,13 @@ long long stu_full_conv_tc5_scratch_elems(int K, int t_end);
 int stu_full_conv_tc5(const void* hist, int Lh, const void* phi, int L, int K, void* scratch, void* U, long long ldU, int B,
                       int d, int both_signs, int t0, int t_end, int* status, int dtype, void* stream);
 
+/* One cached step of the full variant up to the contraction with M_phi, bf16, at most 32 filters: the optional RMSNorm of the
+ * rows x, their append at position t = pos[0], U+- [B][(1 or 2) K d] and pos + 1, in one kernel.  taps8 [8][2K][Lh+8]:
+ * stu_taps_rev8 of the K filters' even taps and of their odd taps ([2K][Lh], zero past the filters); t < limit <= 2 Lh. */
+int stu_full_decode_step(const void* x, long long x_rstride, const void* norm_w, float eps, void* hist, const void* taps8,
+                         int* pos, void* U, int B, int d, int K, int Lh, int limit, int both_signs, int* status, int dtype,
+                         void* stream);
+
 /* One cached decode step of the full variant, around one GEMM G = hist_rows @ PhiT^T (stu_linear, M = B*d*2,
  * N = 2K, K = Lh): prepare appends x_t at time pos[0] and rebuilds PhiT [2K][Lh] (time-reversed even / odd
  * taps for that position); combine forms U+- [B][2*K*d] from G and (advance != 0) moves every position on.

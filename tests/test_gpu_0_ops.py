@@ -1152,3 +1152,41 @@ def test_fp32_linears_of_up_to_8_rows_at_the_edges_of_their_split(shape):
     y = ops.linear(x.to(dev()), W.to(dev()), norm_w=nw.to(dev()), **kw)
     close(y, _lin_ref(xn, W, W2, resid, epi, torch.float32), TOL[torch.float32] / 2)
     ops.check_status()
+
+
+@pytest.mark.parametrize("B,d,K,L,signs", [(1, 40, 5, 64, 2), (3, 72, 24, 200, 2), (2, 264, 32, 96, 1), (8, 1024, 24, 520, 2), (9, 528, 16, 90, 2)])
+def test_full_variant_step_kernel(B, d, K, L, signs):
+    """The one-kernel step of the full variant against float64 sums at the first positions, around whole 8s and 32s of a parity
+    and at the last one: U, the appended input, the position; 16 and 32 channels per CTA, channels and filters that fill no
+    tile; what the cache holds past the position has no effect.  Bar: as for the prefill's U (E, Q and their sum rounded to bf16)."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(16)
+    Lh = ((L + 1) // 2 + 7) // 8 * 8
+    x, phi = (3 * torch.randn(B, L, d)).bfloat16(), (torch.randn(L, K) / 4).bfloat16()
+    w = (1 + 0.1 * torch.randn(d)).bfloat16()
+    xn = O.rmsnorm(x, w)
+    f = phi.to(dev())
+    taps8 = ops.taps_rev8(torch.cat([ops.taps_even(f, Lh), ops.taps_even(f[1:], Lh)]))
+    for t in sorted({0, 1, 2, 15, 16, 17, 31, 33, 62, 63, L - 2, L - 1}):
+        hist = torch.full((B, d, 2, Lh), float("nan"), dtype=torch.bfloat16, device=dev())
+        if t:
+            ops.to_history(xn[:, :t].to(dev()), hist, 0)
+        pos = torch.zeros(B, 2, dtype=torch.int32, device=dev())
+        pos[:, 0] = t
+        U = torch.full((B, signs * K * d), 7.0, dtype=torch.bfloat16, device=dev())
+        row = x[:, t].to(dev())
+        assert ops.full_decode_step_supported(row, hist, K)
+        ops.full_decode_step(row, w.to(dev()), ops.RMS_EPS, hist, taps8, pos, U, L, signs == 2)
+        ops.check_status()
+        assert pos.tolist() == [[t + 1, 0]] * B
+        close(hist[:, :, t & 1, t >> 1], xn[:, t], 2 ** -7)
+        past = xn[:, :t + 1].double().flip(1)
+        past[:, 0] = hist[:, :, t & 1, t >> 1].cpu().double()   # (its rounding may differ by one unit)
+        taps = phi[:t + 1].double()
+        want = [torch.einsum("tk,bti->bki", taps * (s ** torch.arange(t + 1))[:, None], past).reshape(B, K * d) for s in (1.0, -1.0)]
+        close(U, torch.cat(want[:signs], 1), 4 * 2 ** -9)
+    pos[:, 0] = L
+    ops.full_decode_step(row, w.to(dev()), ops.RMS_EPS, hist, taps8, pos, U, L, signs == 2)
+    with pytest.raises(RuntimeError, match="status 2"):
+        ops.check_status()
+    assert int(pos[0, 0]) == L
