@@ -1190,3 +1190,13 @@ def test_full_variant_step_kernel(B, d, K, L, signs):
     with pytest.raises(RuntimeError, match="status 2"):
         ops.check_status()
     assert int(pos[0, 0]) == L
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d", [(2368, 64), (2401, 264), (5000, 1024), (2500, 1536), (2400, 3072), (2999, 1000)])
+def test_rmsnorm_of_many_rows(dt, rows, d):
+    """A warp per row: widths that fill no round of the lanes, more rows than a multiple of the CTAs' warps."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(21)
+    x, w = (torch.randn(rows, d) * 3).to(dt), torch.randn(d).to(dt)
+    close(ops.rmsnorm(x.to(dev()), w.to(dev())), O.rmsnorm(x, w), 1e-6 if dt == torch.float32 else 2 ** -7)
