@@ -157,11 +157,13 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
 template <int EPI, int STAGES, int TN = 128>
 __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,
                                                          const __grid_constant__ CUtensorMap tmB,
-                                                         const __grid_constant__ CUtensorMap tmB2, int M, int N,
+                                                         const __grid_constant__ CUtensorMap tmB2,
+                                                         const __grid_constant__ CUtensorMap tmY, int by_copy, int M, int N,
                                                          int K, int tiles_m, int tiles_n, int group_m,
                                                          int causal, EpiArgs<bf16> ep, int* status,
                                                          int drop_first_copy, unsigned long long wait_ns) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
+  constexpr bool COPIES = (EPI == EPI_STORE || EPI == EPI_GELU_MUL || EPI == EPI_BLOCKCOL);   // outputs that nothing is added to
   static_assert(!DUAL || TN == 128, "the two-accumulator epilogue uses 128-wide tiles");
   constexpr int BN = TN;                       // shadows the file-level default inside the kernel
   constexpr int B_BYTES = BN * BK * 2;
@@ -178,7 +180,8 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* issued_ctr = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));
   int* consumed_ctr = issued_ctr + 1;
-  bf16* row_stage = reinterpret_cast<bf16*>(smem + STAGES * STAGE_BYTES + 256);   // [4 warps][32][SROW]
+  // per epilogue warp: [32][SROW], or, where the output leaves by tensor copies, two blocks of 32 x 64 in the 128-byte swizzle
+  bf16* row_stage = reinterpret_cast<bf16*>(smem + STAGES * STAGE_BYTES + 1024);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = tiles_m * tiles_n;
@@ -286,8 +289,10 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
     // of the blocks) lanes store single values, side by side.
     const bool unaligned = EPI == EPI_STORE ? ((ep.ldy & 7) || (reinterpret_cast<uintptr_t>(ep.y) & 15))
                                             : EPI == EPI_HIST_T && ((ep.Tseq & 15) || (ep.t0 & 15) || (ep.Lh & 7));
-    bf16* st = row_stage + quarter * (32 * SROW);
-    int it = 0;
+    // Plain outputs leave by tensor copies where they can: a warp puts a block of 32 x 64 into one of two swizzled buffers and one
+    // lane sends it off, edges clipped by the copy; the copy of one block runs beside the next block's accumulator reads.
+    bf16* st = row_stage + quarter * (COPIES ? 2 * 32 * 64 : 32 * SROW);
+    int it = 0, sent = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, it++) {
       int tm, tn;
       tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
@@ -299,6 +304,51 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (COPIES && by_copy) {
+#pragma unroll 1
+        for (int nb = n0; nb < min(n0 + BN, N); nb += 64, sent++) {
+          const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
+          unsigned char* blk = reinterpret_cast<unsigned char*>(st) + (sent & 1) * 4096;
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the block before last has left
+          __syncwarp();
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            uint32_t r[32], r2[32];
+            tmem_ld32(taddr + h * 32, r);
+            if (DUAL) tmem_ld32(taddr + BN + h * 32, r2);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int v8 = 0; v8 < 4; v8++) {
+              float o[8];
+#pragma unroll
+              for (int j = 0; j < 8; j++) {
+                o[j] = __uint_as_float(r[v8 * 8 + j]);
+                if (EPI == EPI_GELU_MUL)
+                  o[j] = round_to<bf16>(gelu_tanh_fast(round_to<bf16>(o[j]))) *
+                         round_to<bf16>(__uint_as_float(r2[v8 * 8 + j]));
+              }
+              store_vec(reinterpret_cast<bf16*>(blk + lane * 128 + (((h * 4 + v8) ^ (lane & 7)) << 4)), o);
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            if (rows <= 0) {
+            } else if (EPI == EPI_BLOCKCOL)
+              asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(&tmY),
+                           "r"(smem_u32(blk)), "r"(nb % ep.Tseq), "r"(first), "r"(nb / ep.Tseq)
+                           : "memory");
+            else
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&tmY),
+                           "r"(smem_u32(blk)), "r"(nb), "r"(first)
+                           : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        mbar_arrive(&tmem_empty[buf]);
+        continue;
+      }
 #pragma unroll 1
       for (int nb = n0; nb < min(n0 + BN, N); nb += 64) {
         const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
@@ -412,6 +462,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(&tmem_empty[buf]);
     }
+    if (COPIES && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // (none where nothing was sent)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   __syncthreads();
@@ -510,6 +561,19 @@ int make_map_uncached(CUtensorMap* map, const void* base, long long rows, long l
   return r == CUDA_SUCCESS ? STU_OK : STU_ERR_UNSUPPORTED;
 }
 
+// The same over an output, boxes of 32 rows x 64 columns: rows of ldy elements, or (column blocks) blocks of Tseq columns ld2 apart.
+int make_output_map(CUtensorMap* map, const EpiArgs<bf16>& ep, bool blocks, int M, int N) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return STU_ERR_UNSUPPORTED;
+  const cuuint64_t dims[3] = {(cuuint64_t)(blocks ? ep.Tseq : N), (cuuint64_t)M, (cuuint64_t)(blocks ? N / ep.Tseq : 1)};
+  const cuuint64_t strides[2] = {(cuuint64_t)ep.ldy * 2, (cuuint64_t)ep.ld2 * 2};
+  const cuuint32_t box[3] = {64, 32, 1}, estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, blocks ? 3 : 2, ep.y, dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? STU_OK : STU_ERR_UNSUPPORTED;
+}
+
 // Failure-detection test hooks (stu_test_inject_wait_expiry): drop the first operand copy of the next launch, and the
 // wall-time bound of every mbarrier wait.
 int g_drop_first_copy = 0;
@@ -530,7 +594,15 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
   constexpr int BN = TN;
   constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2 * (DUAL ? 2 : 1);
-  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + 4 * 32 * SROW * sizeof(bf16);
+  constexpr bool COPIES = (EPI == EPI_STORE || EPI == EPI_GELU_MUL || EPI == EPI_BLOCKCOL);
+  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 1024 + 4 * 32 * (COPIES ? 128 : SROW) * sizeof(bf16);
+  // The output by tensor copies: rows on the 16-byte grid and of whole 16 bytes (a copy clips at those), and (column blocks) 64
+  // columns inside one block of a whole number of them.  What gains is many outputs for little K: LDS features, 6144 x 48128 x
+  // 320, 237 -> 204 us; products of K = 1024 and more hide either form.
+  CUtensorMap y = a;
+  int by_copy = 0;
+  if (COPIES && !ep.peer && ep.ldy % 8 == 0 && N % 8 == 0 && aligned16(ep.y) && (EPI != EPI_BLOCKCOL || (ep.Tseq % 64 == 0 && N % ep.Tseq == 0)))
+    by_copy = make_output_map(&y, ep, EPI == EPI_BLOCKCOL, M, N) == STU_OK;
   auto k = gemm_tc_kernel<EPI, STAGES, TN>;
   static SmemLimit limit;
   cudaError_t e = allow_smem((const void*)k, smem, limit);
@@ -542,7 +614,7 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   const int drop = g_drop_first_copy;
   g_drop_first_copy = 0;   // the injected fault applies to one launch
   const int group_m = m_fast ? tiles_m : gemm_group_m(tiles_n, N, K, DUAL);
-  k<<<grid, 192, smem, st>>>(a, b, b2, M, N, K, tiles_m, tiles_n, group_m, causal, ep, status, drop, g_wait_ns);
+  k<<<grid, 192, smem, st>>>(a, b, b2, y, by_copy, M, N, K, tiles_m, tiles_n, group_m, causal, ep, status, drop, g_wait_ns);
   STU_CHECK_LAUNCH();
   return STU_OK;
 }

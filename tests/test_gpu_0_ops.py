@@ -1200,3 +1200,35 @@ def test_rmsnorm_of_many_rows(dt, rows, d):
     torch.manual_seed(21)
     x, w = (torch.randn(rows, d) * 3).to(dt), torch.randn(d).to(dt)
     close(ops.rmsnorm(x.to(dev()), w.to(dev())), O.rmsnorm(x, w), 1e-6 if dt == torch.float32 else 2 ** -7)
+
+
+@pytest.mark.parametrize("epi", [0, 2])
+@pytest.mark.parametrize("shape", [(33, 70, 64, 72), (129, 8, 72, 16), (300, 1000, 136, 1000), (2500, 5121, 64, 5128), (257, 64, 200, 64)])
+def test_linear_outputs_by_tensor_copies(shape, epi):
+    """Plain and gate/up outputs of the tcgen05 GEMM on rows of the 16-byte grid: last rows and columns that fill no block of 32 x
+    64, rows wider than the output; nothing beside it is written."""
+    from flash_stu_2_b200 import ops
+    M, N, K, ld = shape
+    torch.manual_seed(19)
+    x, W, W2 = torch.randn(M, K).bfloat16(), (torch.randn(N, K) / math.sqrt(K)).bfloat16(), (torch.randn(N, K) / math.sqrt(K)).bfloat16()
+    buf = torch.full((M + 64, ld), 7.0, dtype=torch.bfloat16, device=dev())
+    ops.linear(x.to(dev()), W.to(dev()), W2=W2.to(dev()) if epi else None, out=buf[:M, :N], epilogue=epi, backend=2)
+    ops.check_status()
+    close(buf[:M, :N], _lin_ref(x, W, W2, None, epi, torch.bfloat16), 1e-2)
+    assert bool((buf[:M, N:] == 7.0).all()) and bool((buf[M:] == 7.0).all())
+
+
+@pytest.mark.parametrize("d,chunks,rows,K", [(64, 3, 96, 72), (192, 2, 130, 320), (40, 5, 96, 64), (1024, 2, 6144, 320)])
+def test_lds_features_in_column_blocks(d, chunks, rows, K):
+    """The blocked output of the LDS features: blocks of whole 64s leave by tensor copies, others by the lanes."""
+    from flash_stu_2_b200 import ops
+    F = 6 if rows % 6 == 0 else 5
+    Ck = rows // F
+    torch.manual_seed(20)
+    W, Z = (torch.randn(Ck * F, K) / math.sqrt(K)).bfloat16(), torch.randn(chunks * d, K).bfloat16()
+    U = torch.full((chunks * Ck + 1, F * d), 7.0, dtype=torch.bfloat16, device=dev())
+    ops.lds_chunk_features(W.to(dev()), Z.to(dev()), U[:chunks * Ck], d, Ck, F)
+    ops.check_status()
+    want = (W.double() @ Z.double().t()).view(Ck, F, chunks, d).permute(2, 0, 1, 3).reshape(chunks * Ck, F * d)
+    close(U[:-1], want, 1e-2)
+    assert bool((U[-1] == 7.0).all())
