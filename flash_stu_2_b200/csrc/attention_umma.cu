@@ -1,20 +1,26 @@
-// Sliding-window attention prefill on the 5th-generation tensor cores (bf16, head dimension 128, sequences that
+// Sliding-window attention prefill on the 5th-generation tensor cores (bf16, head dimension 64 or 128, sequences that
 // start at position 0: every key of the call lies in the call's own qkv activations).
 //
 // Reference semantics (flash_stu/modules/attention.py:72-101 + the documented flash_attn_func contract): per head,
 // query i sees keys j in [i - w, i]; score = softcap * tanh(q.k * scale / softcap) - slope_h * (i - j); softmax; @ V.
 //
 // One CTA = 128 queries of one head of one sequence; key tiles of 64.  Per tile
-//   S = Q K^T        tcgen05.mma, M = 128 queries, N = 64 keys, K = 128 dims; Q (two 64-wide k-blocks) and the key tile
+//   S = Q K^T        tcgen05.mma, M = 128 queries, N = 64 keys, K = the head's dims; Q (64-wide k-blocks) and the key tile
 //                    come by cp.async.bulk.tensor with the 128-byte swizzle; S lands in tensor memory (two buffers)
-//   softmax          four warps, one query row per thread: tcgen05.ld of the row's 64 scores, soft cap (hardware
-//                    tanh), ALiBi, window / causal mask, exponentials in the exp2 domain against a LAZY reference
+//   softmax          four warps, one query row per thread: tcgen05.ld of the row's 64 scores, soft cap (see below),
+//                    ALiBi, window / causal mask, exponentials in the exp2 domain against a LAZY reference
 //                    maximum (moved only when the row maximum outgrows it by 2^8, then the O row in tensor memory is
 //                    rescaled with tcgen05.ld/st); P is rounded to bf16 and stored swizzled into shared memory
-//   O += P V         tcgen05.mma, M = 128 queries, N = 128 dims, K = 64 keys, accumulating in tensor memory; the value
+//   O += P V         tcgen05.mma, M = 128 queries, N = the head's dims, K = 64 keys, accumulating in tensor memory; the value
 //                    operand is a tile of V^T (keys contiguous), which a transpose kernel writes beforehand
+// Bound: the softmax, and in it the special-function unit, which takes 8 clocks a warp for every tanh and every exponential:
+// two of each score's three instruction streams waited for it.  A cap of 50 is far above the scores of a trained model, so where
+// every score of the warp's tile is below half the cap, tanh(y) = y p(y^2) with p of degree 2 (three coefficients, Chebyshev
+// interpolation on [0, 1/4], relative error 2.3e-5 against 2^-11 of the hardware's) on packed pairs; the tile goes through the
+// hardware tanh otherwise.  4 x 8192 positions of 24 heads of 128, window 2048: 1445 -> 1282 us; 4 x 1999 of 16 heads of 64,
+// window 512, 83 us (the mma.sync kernel 114).
 // O never leaves tensor memory until the last tile.  Warps: 0 producer (tensor copies), 1 MMA issuer, 2-5 softmax.
-// 96 KB of shared memory and 256 columns of tensor memory per CTA: two CTAs share an SM, one computes its softmax
+// 96 KB of shared memory (head dimension 64: 57) and 256 columns of tensor memory per CTA: two CTAs share an SM, one computes its softmax
 // while the other's MMAs run.  Every load is a plain single-CTA copy of this GPU's own memory; every wait is bounded
 // (status 11: a wait ran out or a sequence was not at position 0).
 #include <cuda.h>
@@ -28,12 +34,18 @@ int launch_kv_ring_write_bf16(const void* qkv, void* k_ring, void* v_ring, int* 
 
 namespace {
 
-constexpr int BM = 128, BN = 64, HD = 128;
-constexpr int Q_OFF = 0;                      // 2 k-blocks x [128 rows][64 dims]
-constexpr int K_OFF = 32768;                  // 2 stages x 2 k-blocks x [64 keys][64 dims]
-constexpr int V_OFF = K_OFF + 2 * 16384;      // [128 dims][64 keys]
-constexpr int P_OFF = V_OFF + 16384;          // [128 queries][64 keys]
-constexpr int SMEM_BYTES = P_OFF + 16384 + 1024;
+constexpr int BM = 128, BN = 64;
+template <int HD> struct Smem {
+  static constexpr int KB = HD / 64;                     // 64-dim k-blocks of a head
+  static constexpr int Q = 0;                            // KB x [128 rows][64 dims]
+  static constexpr int K_STAGE = KB * 8192;              // KB x [64 keys][64 dims]
+  static constexpr int K = KB * 16384;                   // two stages
+  static constexpr int V = K + 2 * K_STAGE;              // [HD dims][64 keys]
+  static constexpr int P = V + HD * 128;                 // [128 queries][64 keys]
+  static constexpr int BYTES = P + 16384 + 1024;
+};
+// tanh(y) = y (T0 + T1 y^2 + T2 y^4) for |y| <= 1/2
+constexpr float T0 = 0.999977239f, T1 = -0.331685329f, T2 = 0.115185198f;
 constexpr int STATUS_SWA = 11;
 constexpr float LOG2E = 1.4426950408889634f;
 
@@ -89,6 +101,30 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
         "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
+// pairs of fp32 values in 64-bit registers
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ f32x2 pair_of(uint32_t lo, uint32_t hi) { return (f32x2)hi << 32 | lo; }
+__device__ __forceinline__ void split(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ float fast_exp2(float x) {   // ex2.approx: exact 0 for -inf
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -101,6 +137,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 // Vt[b][h][c][t] = v of token t, head h, dim c; the pad t in [Tn, Tp) is written as zeros (a masked key's value is
 // multiplied by P = 0, which stale NaN bits would turn into NaN)
+template <int HD>
 __global__ void __launch_bounds__(256) v_transpose_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ vt, int Tn,
                                                           int Tp, int H) {
   __shared__ bf16 tile[64][HD + 2];
@@ -126,12 +163,14 @@ __global__ void __launch_bounds__(256) v_transpose_kernel(const bf16* __restrict
   }
 }
 
+template <int HD>
 __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                        const __grid_constant__ CUtensorMap tmK,
                                                        const __grid_constant__ CUtensorMap tmV,
                                                        const int* __restrict__ pos, const float* __restrict__ slopes,
                                                        bf16* __restrict__ out, int Tn, int H, int window, float scale,
                                                        float softcap, int* status) {
+  typedef Smem<HD> L;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ Ctl ctl;
@@ -165,31 +204,32 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = ctl.tmem_slot;
-  const uint32_t tm_s = tmem_base, tm_o = tmem_base + 128;   // S buffers at columns 0 and 64, O at 128..255
+  const uint32_t tm_s = tmem_base, tm_o = tmem_base + 128;   // S buffers at columns 0 and 64, O from 128 on
 
   if (!fresh) {
     // not a prefill from position 0: nothing is computed (the caller takes the general kernel for such calls)
   } else if (warp == 0) {
     if (lane == 0) {
       // ------------------------------------------------------------------ producer
-      tma::mbar_expect_tx(&ctl.q_full, 32768);
-      tma::load_3d(smem + Q_OFF, &tmQ, &ctl.q_full, h * HD, q0, b);
-      tma::load_3d(smem + Q_OFF + 16384, &tmQ, &ctl.q_full, h * HD + 64, q0, b);
+      tma::mbar_expect_tx(&ctl.q_full, L::KB * 16384);
+#pragma unroll
+      for (int kb = 0; kb < L::KB; kb++) tma::load_3d(smem + L::Q + kb * 16384, &tmQ, &ctl.q_full, h * HD + kb * 64, q0, b);
       auto load_k = [&](int t) {
         const int s = t & 1;
         if (!tma::mbar_wait_bounded(&ctl.k_empty[s], ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag)) return false;
-        unsigned char* dst = smem + K_OFF + s * 16384;
-        tma::mbar_expect_tx(&ctl.k_full[s], 16384);
-        tma::load_3d(dst, &tmK, &ctl.k_full[s], d + h * HD, j_lo + t * BN, b);
-        tma::load_3d(dst + 8192, &tmK, &ctl.k_full[s], d + h * HD + 64, j_lo + t * BN, b);
+        unsigned char* dst = smem + L::K + s * L::K_STAGE;
+        tma::mbar_expect_tx(&ctl.k_full[s], L::K_STAGE);
+#pragma unroll
+        for (int kb = 0; kb < L::KB; kb++)
+          tma::load_3d(dst + kb * 8192, &tmK, &ctl.k_full[s], d + h * HD + kb * 64, j_lo + t * BN, b);
         return true;
       };
       auto load_v = [&](int t) {
         if (t > 0 && !tma::mbar_wait_bounded(&ctl.pv_done, (uint32_t)(t - 1) & 1u, abort_flag)) return false;
-        tma::mbar_expect_tx(&ctl.v_full, 16384);
+        tma::mbar_expect_tx(&ctl.v_full, HD * 128);
         asm volatile(
             "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-            ::"r"(tma::smem_u32(smem + V_OFF)), "l"(&tmV), "r"(tma::smem_u32(&ctl.v_full)), "r"(j_lo + t * BN),
+            ::"r"(tma::smem_u32(smem + L::V)), "l"(&tmV), "r"(tma::smem_u32(&ctl.v_full)), "r"(j_lo + t * BN),
               "r"((b * H + h) * HD)
             : "memory");
         return true;
@@ -204,18 +244,18 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
   } else if (warp == 1) {
     if (lane == 0) {
       // ------------------------------------------------------------------ MMA issuer
-      const uint32_t q_s = tma::smem_u32(smem + Q_OFF), k_s = tma::smem_u32(smem + K_OFF),
-                     v_s = tma::smem_u32(smem + V_OFF), p_s = tma::smem_u32(smem + P_OFF);
+      const uint32_t q_s = tma::smem_u32(smem + L::Q), k_s = tma::smem_u32(smem + L::K),
+                     v_s = tma::smem_u32(smem + L::V), p_s = tma::smem_u32(smem + L::P);
       const uint32_t id_s = idesc_n(BN), id_o = idesc_n(HD);
       auto issue_s = [&](int t) {
         const int s = t & 1;
         if (!tma::mbar_wait_bounded(&ctl.k_full[s], (uint32_t)(t >> 1) & 1u, abort_flag)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int kb = 0; kb < 2; kb++)
+        for (int kb = 0; kb < L::KB; kb++)
 #pragma unroll
           for (int kk = 0; kk < 4; kk++)
-            umma(tm_s + s * BN, make_desc(q_s + kb * 16384) + 2 * kk, make_desc(k_s + s * 16384 + kb * 8192) + 2 * kk,
+            umma(tm_s + s * BN, make_desc(q_s + kb * 16384) + 2 * kk, make_desc(k_s + s * L::K_STAGE + kb * 8192) + 2 * kk,
                  id_s, (kb | kk) ? 1u : 0u);
         umma_commit(&ctl.s_full[s]);
         umma_commit(&ctl.k_empty[s]);
@@ -245,7 +285,11 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
     const float base_i = -c2 * (float)i;
     const float k0 = softcap > 0.f ? scale / softcap : 0.f;
     const float k1 = softcap > 0.f ? softcap * LOG2E : scale * LOG2E;
-    unsigned char* prow = smem + P_OFF + (row >> 3) * 1024 + (row & 7) * 128;
+    // tanh(s k0) k1 = s (cap0 + cap1 s^2 + cap2 s^4) while s^2 <= most_small
+    const float kk = k0 * k0, a0 = k0 * k1 * T0, a1 = k0 * k1 * kk * T1, a2 = k0 * k1 * kk * kk * T2;
+    const f32x2 cap0 = pair_of(a0, a0), cap1 = pair_of(a1, a1), cap2 = pair_of(a2, a2);
+    const float most_small = 0.25f / kk;
+    unsigned char* prow = smem + L::P + (row >> 3) * 1024 + (row & 7) * 128;
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
     for (int t = 0; t < nt; t++) {
@@ -264,24 +308,44 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
       const bool interior = (jt + BN - 1 <= q0) && (jt >= q0 + BM - 1 - window) && (q0 + BM - 1 <= i_last);
       const float base_t = fmaf(c2, (float)jt, base_i);
       float mx = -INFINITY;
+      if (softcap > 0.f) {
+        const f32x2 cc = pair_of(c2, c2), bt = pair_of(base_t, base_t);
+        float most = 0.f;   // the largest square
 #pragma unroll
-      for (int c = 0; c < 64; c++) {
-        float sc;
-        if (softcap > 0.f) {   // hardware tanh: relative error 2^-11, below the bf16 rounding of P
-          float th;
-          asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(__uint_as_float(sr[c]) * k0));
-          sc = fmaf(th, k1, fmaf(c2, (float)c, base_t));
-        } else {
-          sc = fmaf(__uint_as_float(sr[c]), k1, fmaf(c2, (float)c, base_t));
+        for (int c = 0; c < 64; c += 2) {
+          const f32x2 sv = pair_of(sr[c], sr[c + 1]), t2 = mul2(sv, sv);
+          float t0, t1, s0, s1;
+          split(t2, t0, t1);
+          most = fmaxf(most, fmaxf(t0, t1));
+          split(fma2(sv, fma2(t2, fma2(t2, cap2, cap1), cap0), fma2(cc, pair_of((float)c, (float)(c + 1)), bt)), s0, s1);
+          sr[c] = __float_as_uint(s0);
+          sr[c + 1] = __float_as_uint(s1);
         }
-        if (!interior) {
+        if (__any_sync(0xffffffffu, !(most <= most_small))) {   // (NaN included)
+          tmem_ld32(tm_s + lane_base + (t & 1) * BN, sr);
+          tmem_ld32(tm_s + lane_base + (t & 1) * BN + 32, sr + 32);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < 64; c++) {
+            float th;   // hardware tanh: relative error 2^-11, below the bf16 rounding of P
+            asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(__uint_as_float(sr[c]) * k0));
+            sr[c] = __float_as_uint(fmaf(th, k1, fmaf(c2, (float)c, base_t)));
+          }
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 64; c++) sr[c] = __float_as_uint(fmaf(__uint_as_float(sr[c]), k1, fmaf(c2, (float)c, base_t)));
+      }
+      if (!interior) {
+#pragma unroll
+        for (int c = 0; c < 64; c++) {
           const int j = jt + c;
           const bool valid = (j <= i) && (j >= i - window) && (i <= i_last);
-          sc = valid ? sc : -INFINITY;
+          sr[c] = valid ? sr[c] : 0xff800000u;   // -infinity
         }
-        sr[c] = __float_as_uint(sc);
-        mx = fmaxf(mx, sc);
       }
+#pragma unroll
+      for (int c = 0; c < 64; c += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])));
       // lazy reference maximum: moved (and the O row rescaled) only when some row of the warp outgrows it by 2^8
       const bool grow = (mx > m_ref + 8.f) || (m_ref == -INFINITY && mx > -INFINITY);
       float corr = 1.f;
@@ -294,13 +358,20 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
       }
       const float msafe = (m_ref == -INFINITY) ? 0.f : m_ref;
       uint32_t pk[32];
-      float psum = 0.f;
+      f32x2 psum2 = 0;
+      const f32x2 neg = pair_of(-msafe, -msafe);
 #pragma unroll
       for (int c = 0; c < 64; c += 2) {
-        const float p0 = fast_exp2(__uint_as_float(sr[c]) - msafe), p1 = fast_exp2(__uint_as_float(sr[c + 1]) - msafe);
-        psum += p0 + p1;
+        float p0, p1;
+        split(add2(pair_of(sr[c], sr[c + 1]), neg), p0, p1);
+        p0 = fast_exp2(p0);
+        p1 = fast_exp2(p1);
+        psum2 = add2(psum2, pair_of(p0, p1));
         pk[c >> 1] = pack_bf16(p0, p1);
       }
+      float psum, psum_odd;
+      split(psum2, psum, psum_odd);
+      psum += psum_odd;
       l += psum;
       // the previous tile's P V product has read P and finished accumulating into O
       if (t > 0) {
@@ -310,7 +381,7 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (rescale) {
 #pragma unroll 1
-          for (int cc = 0; cc < 4; cc++) {
+          for (int cc = 0; cc < HD / 32; cc++) {
             uint32_t o[32];
             tmem_ld32(tm_o + lane_base + cc * 32, o);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -338,7 +409,7 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       bf16* orow = out + ((size_t)b * Tn + i) * d + h * HD;
 #pragma unroll 1
-      for (int cc = 0; cc < 4; cc++) {
+      for (int cc = 0; cc < HD / 32; cc++) {
         uint32_t o[32];
         tmem_ld32(tm_o + lane_base + cc * 32, o);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -378,24 +449,15 @@ int encode_sw128(CUtensorMap* map, const void* base, int rank, const cuuint64_t*
 }  // namespace
 
 extern "C" long long stu_swa_prefill_scratch_elems(int B, int Tn, int H, int hd) {
-  if (B <= 0 || Tn <= 0 || H <= 0 || hd != HD) return -1;
-  return (long long)B * H * HD * ((Tn + 63) / 64 * 64);
+  if (B <= 0 || Tn <= 0 || H <= 0 || (hd != 64 && hd != 128)) return -1;
+  return (long long)B * H * hd * ((Tn + 63) / 64 * 64);
 }
 
-// Attention of a prefill that starts at position 0 (bf16, head dimension 128) on the tcgen05 tensor cores; the
-// sequences' keys and values then go into the rings and the positions advance by Tn, as stu_swa_forward does.
-// vt_scratch: stu_swa_prefill_scratch_elems() bf16 elements, 16-byte aligned (V transposed per head).
-extern "C" int stu_swa_prefill_tc5(const void* qkv, void* vt_scratch, void* k_ring, void* v_ring, int* pos,
-                                   const float* slopes, void* out, int B, int Tn, int H, int hd, int W, int window,
-                                   float softcap, int update_cache, int* status, int dtype, void* stream) {
-  if (!qkv || !vt_scratch || !pos || !slopes || !out || (update_cache && (!k_ring || !v_ring))) return STU_ERR_NULL;
-  if (dtype != STU_BF16) return STU_ERR_DTYPE;
-  if (hd != HD) return STU_ERR_UNSUPPORTED;
-  if (B <= 0 || Tn <= 0 || H <= 0 || window < 0 || (update_cache && W < window + 1)) return STU_ERR_SHAPE;
-  if (!aligned16(qkv) || !aligned16(vt_scratch) || !aligned16(out)) return STU_ERR_ALIGN;
-  cudaStream_t st = (cudaStream_t)stream;
+template <int HD>
+static int launch_prefill(const void* qkv, void* vt_scratch, const int* pos, const float* slopes, void* out, int B, int Tn, int H,
+                          int window, float softcap, int* status, cudaStream_t st) {
   const int d = H * HD, Tp = (Tn + 63) / 64 * 64;
-  v_transpose_kernel<<<dim3(Tp / 64, H, B), 256, 0, st>>>((const bf16*)qkv, (bf16*)vt_scratch, Tn, Tp, H);
+  v_transpose_kernel<HD><<<dim3(Tp / 64, H, B), 256, 0, st>>>((const bf16*)qkv, (bf16*)vt_scratch, Tn, Tp, H);
   STU_CHECK_LAUNCH();
   CUtensorMap tmQ, tmK, tmV;
   {
@@ -415,12 +477,29 @@ extern "C" int stu_swa_prefill_tc5(const void* qkv, void* vt_scratch, void* k_ri
     if (rc != STU_OK) return rc;
   }
   static SmemLimit limit;
-  cudaError_t e = allow_smem((const void*)swa_umma_kernel, SMEM_BYTES, limit);
+  cudaError_t e = allow_smem((const void*)swa_umma_kernel<HD>, Smem<HD>::BYTES, limit);
   if (e != cudaSuccess) return (int)e;
   const float scale = 1.0f / sqrtf((float)HD);
-  swa_umma_kernel<<<dim3((Tn + BM - 1) / BM, H, B), 192, SMEM_BYTES, st>>>(tmQ, tmK, tmV, pos, slopes, (bf16*)out, Tn,
-                                                                           H, window, scale, softcap, status);
+  swa_umma_kernel<HD><<<dim3((Tn + BM - 1) / BM, H, B), 192, Smem<HD>::BYTES, st>>>(tmQ, tmK, tmV, pos, slopes, (bf16*)out, Tn, H,
+                                                                                    window, scale, softcap, status);
   STU_CHECK_LAUNCH();
-  if (update_cache) return launch_kv_ring_write_bf16(qkv, k_ring, v_ring, pos, B, Tn, d, W, st);
   return STU_OK;
+}
+
+// Attention of a prefill that starts at position 0 (bf16, head dimension 64 or 128) on the tcgen05 tensor cores; the
+// sequences' keys and values then go into the rings and the positions advance by Tn, as stu_swa_forward does.
+// vt_scratch: stu_swa_prefill_scratch_elems() bf16 elements, 16-byte aligned (V transposed per head).
+extern "C" int stu_swa_prefill_tc5(const void* qkv, void* vt_scratch, void* k_ring, void* v_ring, int* pos,
+                                   const float* slopes, void* out, int B, int Tn, int H, int hd, int W, int window,
+                                   float softcap, int update_cache, int* status, int dtype, void* stream) {
+  if (!qkv || !vt_scratch || !pos || !slopes || !out || (update_cache && (!k_ring || !v_ring))) return STU_ERR_NULL;
+  if (dtype != STU_BF16) return STU_ERR_DTYPE;
+  if (hd != 64 && hd != 128) return STU_ERR_UNSUPPORTED;
+  if (B <= 0 || Tn <= 0 || H <= 0 || window < 0 || (update_cache && W < window + 1)) return STU_ERR_SHAPE;
+  if (!aligned16(qkv) || !aligned16(vt_scratch) || !aligned16(out)) return STU_ERR_ALIGN;
+  cudaStream_t st = (cudaStream_t)stream;
+  const int rc = hd == 128 ? launch_prefill<128>(qkv, vt_scratch, pos, slopes, out, B, Tn, H, window, softcap, status, st)
+                           : launch_prefill<64>(qkv, vt_scratch, pos, slopes, out, B, Tn, H, window, softcap, status, st);
+  if (rc != STU_OK || !update_cache) return rc;
+  return launch_kv_ring_write_bf16(qkv, k_ring, v_ring, pos, B, Tn, H * hd, W, st);
 }

@@ -1232,3 +1232,31 @@ def test_lds_features_in_column_blocks(d, chunks, rows, K):
     want = (W.double() @ Z.double().t()).view(Ck, F, chunks, d).permute(2, 0, 1, 3).reshape(chunks * Ck, F * d)
     close(U[:-1], want, 1e-2)
     assert bool((U[-1] == 7.0).all())
+
+
+@pytest.mark.parametrize("gain", [0.2, 3.0, 12.0])
+@pytest.mark.parametrize("cap", [50.0, 4.0, 0.0])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_prefill_soft_cap_small_and_large(hd, cap, gain):
+    """Scores far below the cap (polynomial), beyond it (hardware tanh) and mixed within a tile; no cap; both head dimensions.  Bar:
+    P and the output are rounded to bf16 (2^-9 each), the hardware tanh is off by 2^-11 of a score of at most cap."""
+    from flash_stu_2_b200 import ops
+    B, T, H, w = 2, 333, 3, 150
+    d = H * hd
+    torch.manual_seed(18)
+    qkv = torch.randn(B, T, 3 * d)
+    qkv[:, :, :2 * d] *= gain ** 0.5
+    qkv[:, 100:200, :d] *= 0.1
+    qkv = qkv.bfloat16().to(dev())
+    slopes = O.alibi_slopes(H).float().to(dev())
+    dummy = torch.zeros(1, 1, 1, dtype=torch.bfloat16, device=dev())
+    y = ops.swa_prefill_tc5(qkv, dummy, dummy, torch.zeros(B, 2, dtype=torch.int32, device=dev()), slopes, H, w, cap, update_cache=False)
+    ops.check_status()
+    q, k, v = [a.double().view(B, T, H, hd).transpose(1, 2) for a in qkv.split(d, dim=2)]
+    s = q @ k.transpose(2, 3) / math.sqrt(hd)
+    s = cap * torch.tanh(s / cap) if cap else s
+    lag = torch.arange(T, device=dev())[:, None] - torch.arange(T, device=dev())[None, :]
+    s = s - slopes.double()[None, :, None, None] * lag
+    s = s.masked_fill((lag < 0) | (lag > w), float("-inf"))
+    want = (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(B, T, d)
+    close(y, want, 1.5e-2 if cap != 50.0 or gain < 12 else 3e-2)
