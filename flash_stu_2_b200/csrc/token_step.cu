@@ -5,22 +5,26 @@
 //
 // Bound: HBM (every weight once per step: 1.8 GB = 283 us for the 24-layer 1536-wide bf16 model) against the chain of
 // dependent products (96 of them).  Launched kernel by kernel the chain wins: a dependent launch costs 2.5 us before
-// its first byte, and at most one kernel ahead can fetch its weights.  Here one CTA per SM runs the whole chain with
-// grid barriers between the products, and the weight stream does not stop at a barrier: a producer warp walks the
+// its first byte, and at most one kernel ahead can fetch its weights.  Here one CTA per SM runs the whole chain, and the weight
+// stream does not stop between two products: a producer warp walks the
 // weight rows of ALL products of ALL layers in order and brings them by bulk copies (one piece of d values each; pieces
 // below 2 KB are bound by the copy engine's request rate) into a ring of row slots (up to 180 KB per SM, 26 MB over
 // the chip), however far the arithmetic is.
 //
 //   product      a CTA owns N / 148 consecutive output features (no tile granularity), its 8 consumer warps split K
-//   activations  the input rows of a product (at most 8 x max(d, I)) are read from L2 into shared memory, normalised
-//                there when the product is behind a norm, and feed every feature of the CTA
+//   activations  the input rows of a product (at most 8 x max(d, I)) are read from L2 into shared memory, times the norm
+//                weight when the product is behind a norm, and feed every feature of the CTA
+//   hand-over    results travel as tagged words (below), which the readers poll: a grid barrier waits for the stores, for an
+//                atomic to arrive and for another read to see it before the first row can be read.  That model, 1 sequence: 771
+//                -> 683 us a step; 12 fp32 layers of 512, 2 sequences: 352 -> 311.  Barriers are left where the words would be
+//                read by everybody in bulk: the attention's partial sums, and the rows of wide down projections
 //   STU          a CTA's channels are projected, appended to the history and combined with their tap sums in place;
-//                the tap sums over the cached history need nothing of this step and are taken before the barrier
+//                the tap sums over the cached history need nothing of this step and are taken ahead of the wait
 //   attention    (sequence, head, key range) items over the CTAs; the ranges are merged by the readers
 //
 // bf16: mma.sync m16n8k16, weights as the 16-row operand (gate/up: 8 gate and the 8 up rows of the same features),
 // sequences as the 8 columns.  fp32: FMAs.  All product code exists once (a stage switch picks operands and epilogue):
-// written out per product it outgrew the instruction cache (that model, 1 sequence: 1.25 ms a step, 0.75 as it is).
+// written out per product it outgrew the instruction cache (that model, 1 sequence: 1.25 ms a step where this form took 0.75).
 // Every wait is bounded: on expiry the status word is raised, outstanding copies are let land and every CTA returns.  The
 // caches, positions and outputs are then undefined, and the workspace is marked: launches on it return at once with the
 // same status (their barriers would start from a counter that was left half way) until it is zeroed.
@@ -40,7 +44,10 @@ constexpr int RED_BYTES = TILES * NW * 128 * 4;
 constexpr uint32_t COPY = 4096;                // bytes of one bulk copy at most
 constexpr int UNITS = 32;                     // row groups in flight
 constexpr int MAX_ROWS = 32;                  // STU channels per CTA
-constexpr int NORM_VECS = 2;                  // norm weights of a row kept by a thread: d <= 2 * 256 vectors
+// Rows of the down projection are handed over as tagged words up to this size (every CTA reads all of them: twice the bytes of a
+// barrier's plain values).  2 fp32 rows of 6144, 98 KB: 12 layers 311 us a step, with the barrier 317; 1 bf16 row of 6144: a tie.
+constexpr long long TAGGED_H_BYTES = 100 * 1024;
+constexpr int NORM_VECS = 2;                  // rows behind a norm: d <= 2 * 256 vectors
 
 __device__ __forceinline__ void cons_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ uint4 ldcg16(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
@@ -73,6 +80,50 @@ __device__ __forceinline__ float ldcg_f(const float* p) { return __ldcg(p); }
 __device__ __forceinline__ float ldcg_f(const bf16* p) {
   return __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(p)) << 16);
 }
+// Tagged words: a value that one CTA hands to all others, and beside it in the same word the number of the use of its buffer
+// that it belongs to.  A reader polls the word itself: neither a fence nor a counter stands between the store and the load
+// that finds it.  bf16: 32 bits, the value above 16 bits of tag; fp32: 64 bits, the tag above the value.
+// (Every write of a word carries another tag than the write before: see tag_of in the kernel.)
+template <typename T> struct Tagged;
+template <> struct Tagged<bf16> {
+  static constexpr int BYTES = 4;
+  static __device__ __forceinline__ bool has(const uint4& w, uint32_t tag) {
+    return (((w.x ^ tag) | (w.y ^ tag) | (w.z ^ tag) | (w.w ^ tag)) & 0xffffu) == 0;
+  }
+  static __device__ __forceinline__ uint2 values(const uint4& w) {   // eight bytes of plain values
+    return make_uint2(__byte_perm(w.x, w.y, 0x7632), __byte_perm(w.z, w.w, 0x7632));
+  }
+  static __device__ __forceinline__ void put(char* row, int i, bf16 v, uint32_t tag) {
+    const uint32_t w = ((uint32_t)__bfloat16_as_ushort(v) << 16) | (tag & 0xffffu);
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(row + (size_t)i * 4), "r"(w) : "memory");
+  }
+};
+template <> struct Tagged<float> {
+  static constexpr int BYTES = 8;
+  static __device__ __forceinline__ bool has(const uint4& w, uint32_t tag) { return w.y == tag && w.w == tag; }
+  static __device__ __forceinline__ uint2 values(const uint4& w) { return make_uint2(w.x, w.z); }
+  static __device__ __forceinline__ void put(char* row, int i, float v, uint32_t tag) {
+    const uint64_t w = ((uint64_t)tag << 32) | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(row + (size_t)i * 8), "l"(w) : "memory");
+  }
+};
+__device__ __forceinline__ uint4 ld_tagged(const char* p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void unpack8(const uint2& v, float (&o)[4], bf16*) {   // the values of eight bytes
+  o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
+  o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+__device__ __forceinline__ void unpack8(const uint2& v, float (&o)[2], float*) {
+  o[0] = __uint_as_float(v.x); o[1] = __uint_as_float(v.y);
+}
+__device__ __forceinline__ uint2 pack8(const float (&v)[4], bf16*) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+__device__ __forceinline__ uint2 pack8(const float (&v)[2], float*) { return make_uint2(__float_as_uint(v[0]), __float_as_uint(v[1])); }
 // The sum over the warp of v[lane / (32 / NV)] (NV a power of two <= 32).
 template <int NV>
 __device__ __forceinline__ float fold(float (&v)[NV], int lane) {
@@ -111,6 +162,8 @@ struct Params {
   int slots, pitch;    // ring: row slots and their distance in bytes
   int xs_cols;         // columns of the activation rows in shared memory: max(d, I), or less, a multiple of d
   float scale;
+  int tagged_h;        // the rows of the down projection are handed over as tagged words too
+  int signature;       // of the sizes that the layout of the workspace follows from
 };
 __host__ __device__ inline Range share_of(int N, unsigned cta, unsigned ctas) {   // N < 2^24 (checked by the host)
   return {(int)((unsigned)N * cta / ctas), (int)((unsigned)N * (cta + 1) / ctas)};
@@ -147,6 +200,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   extern __shared__ __align__(128) unsigned char sm[];
   const StuStepArgs& a = P.a;
   const int slots = P.slots, pitch_w = P.pitch, nst = P.nst;
+  int nst_run = nst;
   const int xs_cols = P.xs_cols;
   const bool packed = pitch_w == a.d * (int)sizeof(T);
   unsigned char* ring = sm;
@@ -154,11 +208,12 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   unsigned char* xs = reinterpret_cast<unsigned char*>(red) + RED_BYTES;   // activation rows
   __shared__ uint4 s_plan[MAX_STAGES * 2 + MAXL * 8];
   __shared__ Range s_range[MAX_STAGES];
-  __shared__ const T* s_row[8];
+  __shared__ const T* s_row[8];   // rows of the first layer (null: an id outside the vocabulary)
   __shared__ uint64_t full_bar[UNITS], empty_bar[UNITS];
   __shared__ float s_part[8][NW], s_scale[8];
   __shared__ float s_hist[MAX_ROWS * 8];
-  __shared__ int s_abort, s_go;
+  __shared__ int s_abort, s_go[2];
+  __shared__ uint64_t s_start;
   const Stage* tab = reinterpret_cast<const Stage*>(s_plan);
   const StuStepLayer* layers = reinterpret_cast<const StuStepLayer*>(s_plan + nst * 2);
 
@@ -167,10 +222,13 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   const int hd = H > 0 ? d / H : V;
   unsigned char* ws = (unsigned char*)a.workspace;
   int* epoch_word = (int*)ws;
-  T* mid = (T*)(ws + 512);
-  T* qkv = mid + (size_t)8 * d;
-  T* hbuf = qkv + (size_t)24 * d;
-  float* att = (float*)(hbuf + (size_t)8 * I);                  // items of hd sums, then the maximum and the denominator
+  constexpr int TB = Tagged<T>::BYTES;
+  // tagged rows: X_ROWS the residual stream behind a layer, MID_ROWS in front of its MLP, QKV_ROWS, H_ROWS the rows of the
+  // down projection (plain values where P.tagged_h is 0); behind them the attention's items: hd sums, the maximum and the
+  // denominator
+  enum { X_ROWS = 0, MID_ROWS = 8, QKV_ROWS = 16, H_ROWS = 40 };
+  auto rows_at = [&](int k) { return (char*)a.workspace + 512 + (size_t)(k * d) * TB; };
+  auto att_at = [&]() { return (float*)(rows_at(H_ROWS) + (size_t)8 * I * TB); };
   T* xbuf = (T*)a.x;
 
   for (int i = tid; i < nst * 2 + a.n_layers * 8; i += THREADS) s_plan[i] = __ldg(P.plan + i);
@@ -180,9 +238,11 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
       tma::mbar_init(&empty_bar[i], NW);
     }
     s_abort = 0;
+    s_start = tma::global_ns();
     tma::fence_barrier_init();
   }
-  const int2 control = __ldcg(reinterpret_cast<const int2*>(ws));   // epoch, and whether a launch has given up
+  // epoch, whether a launch has given up, and the sizes that the tagged words were last written for
+  const int4 control = __ldcg(reinterpret_cast<const int4*>(ws));
   const int epoch = control.x;
   __syncthreads();
   for (int i = tid; i < nst; i += THREADS) s_range[i] = share_of(tab[i].N, blockIdx.x, gridDim.x);
@@ -200,7 +260,15 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     if (tid == 0 && cta == 0 && a.status) atomicExch(a.status, any12 ? 12 : any2 ? 2 : 6);
     return;
   }
-  int* counter = (int*)(ws + 128 + 128 * (epoch & 1));
+  int* counter = (int*)(ws + 128 + 128 * (epoch & 1));   // arrivals at the barriers; 16 words on: CTAs that have started
+  int* started = counter + 16;
+  if (tid == 0) {
+    if (cta == 0) {   // the next launch's (the last one that used them has ended)
+      int* next = (int*)(ws + 128 + 128 * ((epoch + 1) & 1));
+      next[0] = next[16] = 0;
+    }
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(started) : "memory");   // the control words and positions are read
+  }
 
   if (warp == NW) {
     // ================================================================ producer
@@ -277,94 +345,151 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   const int per = (nkeys + S - 1) / S;
   const int LPK = hd / V, KPW = 32 / LPK, sub = lane % LPK, grp = lane / LPK;   // lanes per key, keys per warp and load
 
-  int waits = 0;   // grid barriers passed
+  int target = 0;   // arrivals at the barriers so far
   auto arrive = [&]() {
     cons_bar();
     if (tid == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(counter) : "memory");
   };
-  auto wait = [&]() -> bool {   // every CTA has arrived `waits` times
-    waits++;
-    if (tid == 0) {
-      const int target = waits * G;
-      uint64_t start = 0;
-      bool ok = false;
-      for (uint32_t it = 0; it < (1u << 24); ++it) {
-        int v;
-        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-        if (v >= target) {
-          ok = true;
-          break;
-        }
-        if ((it & 63u) == 63u) {
-          if (*(volatile int*)&s_abort) break;
-          const uint64_t now = tma::global_ns();
-          if (start == 0) start = now;
-          else if (now - start > 2000000000ull) break;
-        }
-      }
-      if (!ok) *(volatile int*)&s_abort = 1;
-      s_go = *(volatile int*)&s_abort == 0;   // one answer for the whole CTA: the producer may raise s_abort at any time
-      if (waits == 1 && cta == 0) *(int*)(ws + 128 + 128 * ((epoch + 1) & 1)) = 0;   // the next launch's counter
+  // Whether this thread should stop waiting: another has given up, or the launch has taken two seconds (looked at every 64 polls).
+  auto give_up = [&](uint32_t polls) -> bool {
+    if ((polls & 63u) != 63u) return false;
+    if (*(volatile int*)&s_abort) return true;
+    if (tma::global_ns() - s_start < 2000000000ull && polls < (1u << 24)) return false;
+    *(volatile int*)&s_abort = 1;
+    return true;
+  };
+  auto poll_count = [&](const int* word, int least) {
+    for (uint32_t it = 0;; ++it) {
+      int v;
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+      if (v >= least || give_up(it)) return;
     }
+  };
+  // One answer for the whole CTA, behind a barrier (the producer may raise s_abort at any time)
+  unsigned asked = 0;   // (in turn in two words: nobody is two barriers behind)
+  auto go_on = [&]() -> bool {
+    int* go = s_go + (asked++ & 1u);
+    if (tid == 0) *go = *(volatile int*)&s_abort == 0;
     cons_bar();
-    return s_go;
+    return *go;
   };
-  // row m of the input of layer l
-  auto input_row = [&](int l, int m, bool& ok) -> const T* {
-    ok = true;
-    if (l == 0 && a.ids) {
-      const long long id = a.ids[(size_t)m * a.ids_stride];
-      ok = id >= 0 && id < a.V;
-      if (!ok && tid == 0 && cta == 0 && a.status) atomicExch(a.status, 1);
-      return (const T*)a.embedding + (size_t)(ok ? id : 0) * d;
+  auto wait = [&](int arrivals) -> bool {   // `arrivals` more CTAs have arrived than at the last barrier
+    target += arrivals;
+    if (tid == 0) poll_count(counter, target);
+    return go_on();
+  };
+  // The number of a layer's use of the row buffers.  Consecutive writes of a word differ in it, also in its low 16 bits: the
+  // next use is another layer of this launch or a layer of the next one (64 on for the same layer); none is 0 in its low
+  // 6 bits, which is what a zeroed word holds.
+  auto tag_of = [&](int layer) -> uint32_t { return (uint32_t)epoch * 64u + (uint32_t)layer + 1u; };
+  // The values [k0, k0 + len) of B tagged rows of K, eight bytes of them at a time: use(row, piece, values, extra),
+  // extra = more(piece) asked for ahead of the wait.
+  constexpr int VU = MM == 1 ? 4 : MM == 2 ? 2 : 1;   // pieces of a row on their way at a time
+  auto take = [&](const char* src, int K, int k0, int len, uint32_t tag, auto more, auto use) {
+    const int nv = len * (int)sizeof(T) / 8;
+    const char* base = src + (size_t)k0 * TB;
+#pragma unroll 1
+    for (int v0 = tid; v0 < nv; v0 += CONS * VU) {
+      uint4 w[MM][VU];
+      uint2 ex[VU];
+#pragma unroll
+      for (int u = 0; u < VU; u++) ex[u] = v0 + u * CONS < nv ? more(v0 + u * CONS) : make_uint2(0, 0);
+      for (uint32_t it = 0;; ++it) {
+        bool all = true;
+#pragma unroll
+        for (int m = 0; m < MM; m++)
+#pragma unroll
+          for (int u = 0; u < VU; u++)
+            if (m < B && v0 + u * CONS < nv) w[m][u] = ld_tagged(base + (size_t)m * K * TB + (size_t)(v0 + u * CONS) * 16);
+#pragma unroll
+        for (int m = 0; m < MM; m++)
+#pragma unroll
+          for (int u = 0; u < VU; u++)
+            if (m < B && v0 + u * CONS < nv) all = all && Tagged<T>::has(w[m][u], tag);
+        if (all || give_up(it)) break;
+      }
+#pragma unroll
+      for (int m = 0; m < MM; m++)
+#pragma unroll
+        for (int u = 0; u < VU; u++)
+          if (m < B && v0 + u * CONS < nv) use(m, v0 + u * CONS, Tagged<T>::values(w[m][u]), ex[u]);
     }
-    return xbuf + (size_t)m * d;
   };
-  // results: warp m finishes sequence m, lane n the features n, n + 32, ...; of the (at most 32) features of a d-wide
-  // product that is one per thread, which also adds the residual
+  // V values at a tagged word, by this thread alone
+  auto take_vec = [&](const char* p, uint32_t tag, uint4& out) {
+    constexpr int N = V * TB / 16;
+    uint4 w[N];
+    for (uint32_t it = 0;; ++it) {
+      bool all = true;
+#pragma unroll
+      for (int i = 0; i < N; i++) w[i] = ld_tagged(p + i * 16);
+#pragma unroll
+      for (int i = 0; i < N; i++) all = all && Tagged<T>::has(w[i], tag);
+      if (all || give_up(it)) break;
+    }
+    const uint2 lo = Tagged<T>::values(w[0]), hi = Tagged<T>::values(w[1]);
+    out = make_uint4(lo.x, lo.y, hi.x, hi.y);
+  };
+  static_assert(V * TB == 32, "two loads of tagged words per vector");
+  // A workspace that was last used for other sizes: whatever lies where the tagged words go is cleared first, as in a new one
+  if (control.z != P.signature) {
+    uint4* words = reinterpret_cast<uint4*>(rows_at(X_ROWS));
+    const size_t n = ((size_t)40 * d + (size_t)8 * I) * TB / 16;
+    for (size_t i = (size_t)cta * CONS + tid; i < n; i += (size_t)G * CONS) words[i] = make_uint4(0, 0, 0, 0);
+    arrive();
+  }
+  // row m of the input of the first layer
+  auto first_row = [&](int m) -> const T* {
+    if (!a.ids) return xbuf + (size_t)m * d;
+    const long long id = a.ids[(size_t)m * a.ids_stride];
+    if (id >= 0 && id < a.V) return (const T*)a.embedding + (size_t)id * d;
+    if (cta == 0 && a.status) atomicExch(a.status, 1);
+    return nullptr;
+  };
+  // Results: thread e finishes feature e % n of sequence e / n, n the features of the CTA; of a d-wide product that is at most
+  // one per thread, the same one in every layer: it keeps the residual stream there.
   const Range own_r = share_of(d, blockIdx.x, gridDim.x);
-  const int c0 = own_r.r0, own = own_r.r1 - c0, my_c = c0 + lane;
-  const bool mine = warp < B && lane < own;
+  const int c0 = own_r.r0, own = own_r.r1 - c0, my_m = own ? tid / own : 0, my_c = c0 + (own ? tid - my_m * own : 0);
+  const bool mine = own && tid < B * own;
+  if (tid < B) s_row[tid] = first_row(tid);
+  cons_bar();
+  float stream = mine && s_row[my_m] ? ldcg_f(s_row[my_m] + my_c) : 0.f;   // this thread's value of the residual stream
   int slot = 0;        // first slot of the next unit
   unsigned unit = 0;   // its index
 
-  // columns [k0, k0 + len) of B rows of K values, plain
-  auto load_rows = [&](const T* src, int K, int k0, int len, int pitch) {
+  // columns [k0, k0 + len) of the B rows of the down projection
+  auto load_h = [&](int layer, int k0, int len, int pitch) {
+    if (P.tagged_h) {
+      take(rows_at(H_ROWS), I, k0, len, tag_of(layer), [](int) { return make_uint2(0, 0); },
+           [&](int m, int v, const uint2& val, const uint2&) { *reinterpret_cast<uint2*>(xs + m * pitch + v * 8) = val; });
+      return;
+    }
+    const T* src = (const T*)rows_at(H_ROWS);
     const int nv = len / V;
-    if (B == 1) {
-#pragma unroll 4
-      for (int v = tid; v < nv; v += CONS) *reinterpret_cast<uint4*>(xs + v * 16) = ldcg16(src + k0 + v * V);
-    } else {
 #pragma unroll 1
-      for (int v = tid; v < nv; v += CONS) {
-        uint4 raw[8];
+    for (int v = tid; v < nv; v += CONS) {
+      uint4 raw[MM];
 #pragma unroll
-        for (int m = 0; m < 8; m++) raw[m] = m < B ? ldcg16(src + (size_t)m * K + k0 + v * V) : make_uint4(0, 0, 0, 0);
+      for (int m = 0; m < MM; m++) raw[m] = m < B ? ldcg16(src + (size_t)m * I + k0 + v * V) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int m = 0; m < 8; m++)
-          if (m < B) *reinterpret_cast<uint4*>(xs + m * pitch + v * 16) = raw[m];
-      }
+      for (int m = 0; m < MM; m++)
+        if (m < B) *reinterpret_cast<uint4*>(xs + m * pitch + v * 16) = raw[m];
     }
   };
+  const int down_rows = min(16, own), down_pieces = own > 0 ? unit_pieces(down_rows, (I + d - 1) / d, slots, packed, xs_cols / d) : 1;
+  const int items = B * H * S, owners = min(G, items);   // of the attention, and the CTAs that have any
+  if (control.z != P.signature && !wait(G)) nst_run = 0;
 
 #pragma unroll 1
-  for (int st = 0; st < nst; st++) {
+  for (int st = 0; st < nst_run; st++) {
     const Stage sg = tab[st];
     const int kind = sg.kind;
     const StuStepLayer& L = layers[min((int)sg.layer, a.n_layers - 1)];
     const bool normed = kind == ST_STU || kind == ST_QKV || kind == ST_GATE_UP || kind == ST_LM_HEAD;
     const int next_kind = st + 1 < nst ? tab[st + 1].kind : -1;
 
-    // ================================================================ before the barrier: what needs nothing of this step
-    uint4 nwv[NORM_VECS];
-    if (normed) {
-      const T* nw = (const T*)(kind == ST_LM_HEAD ? a.norm_final : kind == ST_GATE_UP ? L.norm2 : L.norm1);
-#pragma unroll
-      for (int i = 0; i < NORM_VECS; i++) {
-        const int v = tid + i * CONS;
-        nwv[i] = v * V < d ? ldnc16(nw + v * V) : make_uint4(0, 0, 0, 0);
-      }
-    }
+    // ================================================================ ahead of the wait: what needs nothing of this step
+    const int r0 = s_range[st].r0, r1 = s_range[st].r1;
     float tap0 = 0.f;
     if (kind == ST_STU) {   // tap sums over the cached history of this CTA's channels
       const T* taps = (const T*)L.taps;
@@ -442,20 +567,33 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
       }
     }
 
-    // ================================================================ every CTA's results of the stage before are there
-    if (st > 0 && !wait()) break;
 
     if (kind == ST_ATTEND) {
+      cons_bar();   // the sums of the product before have been read
       const T *kr = (const T*)L.k_ring, *vr = (const T*)L.v_ring;
       const int W = L.W;
       const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
 #pragma unroll 1
-      for (int it = cta; it < B * H * S; it += G) {
+      for (int it = cta; it < items; it += G) {
         const int b = it / (H * S), h = (it / S) % H, sp = it % S;
-        const T* cur = qkv + (size_t)b * 3 * d + h * hd;
+        const char* cur = rows_at(QKV_ROWS + 3 * b) + h * hd * TB;   // query, key and value of the new token
+        const uint32_t tag = tag_of(sg.layer);
         const int k0 = sp * per, k1 = min(nkeys, k0 + per);
         float qv[V], acc[V];
-        unpack(ldcg16(cur + sub * V), qv, (T*)nullptr);
+        T* fresh = reinterpret_cast<T*>(red + 4 * NW * 128);   // the new token's key and value of this head (behind the sums below)
+        if (sp == S - 1) {
+          if (tid < 2 * LPK) {   // ... and into the rings
+            const int which = tid >= LPK, i = (tid - which * LPK) * V;
+            uint4 v;
+            take_vec(cur + ((1 + which) * d + i) * TB, tag, v);
+            *reinterpret_cast<uint4*>((T*)(which ? L.v_ring : L.k_ring) + ((size_t)b * W + t % W) * d + h * hd + i) = v;
+            *reinterpret_cast<uint4*>(fresh + which * hd + i) = v;
+          }
+          cons_bar();
+        }
+        uint4 q_raw;
+        take_vec(cur + sub * V * TB, tag, q_raw);
+        unpack(q_raw, qv, (T*)nullptr);
 #pragma unroll
         for (int e = 0; e < V; e++) {
           qv[e] *= P.scale;
@@ -473,8 +611,8 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
             kv[u] = vv[u] = make_uint4(0, 0, 0, 0);
             if (kk < k1) {
               if (j == t) {   // the new token's key and value are still activations
-                kv[u] = ldcg16(cur + d + sub * V);
-                vv[u] = ldcg16(cur + 2 * d + sub * V);
+                kv[u] = *reinterpret_cast<const uint4*>(fresh + sub * V);
+                vv[u] = *reinterpret_cast<const uint4*>(fresh + hd + sub * V);
               } else {
                 const size_t off = ((size_t)b * W + j % W) * d + h * hd + sub * V;
                 kv[u] = ldnc16(kr + off);
@@ -541,9 +679,9 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
             dn = fmaf(gl[i], w, dn);
           }
           if (S == 1) {   // one range: the row of c_proj itself
-            ((T*)att)[(size_t)b * d + h * hd + tid] = Elem<T>::from_f(num / dn);
+            ((T*)att_at())[(size_t)b * d + h * hd + tid] = Elem<T>::from_f(num / dn);
           } else {
-            float* out = att + (size_t)it * (hd + 4);
+            float* out = att_at() + (size_t)it * (hd + 4);
             out[tid] = num;
             if (tid == 0) {
               out[hd] = M;
@@ -551,97 +689,68 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
             }
           }
         }
-        if (sp == S - 1) {   // this head's slice of the new key and value into the ring
-          const size_t at = ((size_t)b * W + t % W) * d + h * hd;
-          if (tid < LPK) *reinterpret_cast<uint4*>((T*)L.k_ring + at + tid * V) = ldcg16(cur + d + tid * V);
-          else if (tid < 2 * LPK)
-            *reinterpret_cast<uint4*>((T*)L.v_ring + at + (tid - LPK) * V) = ldcg16(cur + 2 * d + (tid - LPK) * V);
-        }
         cons_bar();
       }
-      arrive();
+      if (cta < owners) arrive();
       continue;
     }
 
     // ================================================================ the rows of the product, in shared memory
     // (bf16: rows 64 bytes past a multiple of 128 apart: conflict-free fragments)
-    const int N = sg.N, K = sg.K;
+    const int K = sg.K;
     const int pitch = sizeof(T) == 2 ? ((min(K, xs_cols) * 2 + 127) & ~127) + 64 : min(K, xs_cols) * 4;
-    float res = 0.f;   // the value that this thread's output feature is added to
-    if (mine && (kind == ST_STU || kind == ST_CPROJ || kind == ST_DOWN)) {
-      bool ok = true;
-      const T* row = kind == ST_DOWN ? mid + (size_t)warp * d : input_row(sg.layer, warp, ok);
-      res = ok ? ldcg_f(row + my_c) : 0.f;
+    if (kind == ST_CPROJ && !wait(owners)) break;
+    if (kind == ST_DOWN && !P.tagged_h && !wait(G)) break;
+    if (r0 >= r1) {   // no feature of this product: its rows may be gone before they are looked at
+      if (kind == ST_GATE_UP && !P.tagged_h) arrive();
+      continue;
     }
     if (normed) {
-      if (tid < B) {
-        bool ok = true;
-        const T* row = kind == ST_GATE_UP ? mid + (size_t)tid * d
-                       : kind == ST_LM_HEAD ? xbuf + (size_t)tid * d
-                                            : input_row(sg.layer, tid, ok);
-        s_row[tid] = ok ? row : nullptr;
-      }
-      cons_bar();
-      float ss[8];
+      // The rows go to shared memory times the norm weight; the factor of a row's mean square, which is known when all of it has
+      // been seen, goes onto its sums instead.
+      const T* nw = (const T*)(kind == ST_LM_HEAD ? a.norm_final : kind == ST_GATE_UP ? L.norm2 : L.norm1);
+      float ss[MM];
 #pragma unroll
-      for (int m = 0; m < 8; m++) ss[m] = 0.f;
-#pragma unroll 1
-      for (int v = tid; v * V < d; v += CONS) {
-        uint4 raw[8];   // every row's piece is requested before the first is used
+      for (int m = 0; m < MM; m++) ss[m] = 0.f;
+      auto more = [&](int v) { return __ldg(reinterpret_cast<const uint2*>(nw) + v); };
+      auto use = [&](int m, int v, const uint2& val, const uint2& w) {
+        float f[8 / sizeof(T)], g8[8 / sizeof(T)];
+        unpack8(val, f, (T*)nullptr);
+        unpack8(w, g8, (T*)nullptr);
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
-          const T* row = m < B ? s_row[m] : nullptr;
-          raw[m] = row ? ldcg16(row + v * V) : make_uint4(0, 0, 0, 0);
+        for (int j = 0; j < (int)(8 / sizeof(T)); j++) {
+#pragma unroll
+          for (int mm = 0; mm < MM; mm++)
+            if (mm == m) ss[mm] += f[j] * f[j];
+          f[j] *= g8[j];
         }
-#pragma unroll
-        for (int m = 0; m < 8; m++)
-          if (m < B) {
-            *reinterpret_cast<uint4*>(xs + m * pitch + v * 16) = raw[m];
-            float f[V];
-            unpack(raw[m], f, (T*)nullptr);
-#pragma unroll
-            for (int j = 0; j < V; j++) ss[m] += f[j] * f[j];
-          }
-      }
-      const float total = fold<8>(ss, lane);   // of row lane / 4
-      if ((lane & 3) == 0) s_part[lane >> 2][warp] = total;
-      cons_bar();
-      if (tid < 8) {
-        float s = 0.f;
-#pragma unroll
-        for (int w = 0; w < NW; w++) s += s_part[tid][w];
-        s_scale[tid] = rsqrtf(s / (float)d + (kind == ST_LM_HEAD ? a.eps_final : kind == ST_GATE_UP ? L.eps2 : L.eps1));
-      }
-      cons_bar();
+        *reinterpret_cast<uint2*>(xs + m * pitch + v * 8) = pack8(f, (T*)nullptr);
+      };
+      if (sg.layer == 0 && kind != ST_GATE_UP && kind != ST_LM_HEAD) {
 #pragma unroll 1
-      for (int m = 0; m < B; m++) {
-        const float r = s_scale[m];
+        for (int v = tid; v < d * (int)sizeof(T) / 8; v += CONS) {
+          const uint2 w = more(v);
 #pragma unroll
-        for (int i = 0; i < NORM_VECS; i++) {
-          const int v = tid + i * CONS;
-          if (v * V < d) {
-            uint4* p = reinterpret_cast<uint4*>(xs + m * pitch + v * 16);
-            if (sizeof(T) == 2) {
-              *p = norm_pack(*p, r, nwv[i]);
-            } else {
-              float f[4], w[4];
-              unpack(*p, f, (float*)nullptr);
-              unpack(nwv[i], w, (float*)nullptr);
-#pragma unroll
-              for (int j = 0; j < 4; j++) f[j] = f[j] * r * w[j];
-              *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
-            }
-          }
+          for (int m = 0; m < MM; m++)
+            if (m < B) use(m, v, s_row[m] ? __ldcg(reinterpret_cast<const uint2*>(s_row[m]) + v) : make_uint2(0, 0), w);
         }
+      } else {
+        take(rows_at(kind == ST_GATE_UP ? MID_ROWS : X_ROWS), d, 0, d, tag_of(kind == ST_GATE_UP ? sg.layer : sg.layer - 1), more, use);
       }
-    } else if (kind == ST_DOWN || S == 1) {
-      load_rows(kind == ST_DOWN ? hbuf : (const T*)att, K, 0, min(K, xs_cols), pitch);
+      const float total = fold<MM>(ss, lane);   // of row lane / (32 / MM)
+      if (lane % (32 / MM) == 0) s_part[lane / (32 / MM)][warp] = total;
+    } else if (kind == ST_DOWN) {
+      load_h(sg.layer, 0, min(K, xs_cols), pitch);
+    } else if (S == 1) {
+      const T* src = (const T*)att_at();
+      for (int v = tid; v < d / V; v += CONS)
+        for (int m = 0; m < B; m++) *reinterpret_cast<uint4*>(xs + m * pitch + v * 16) = ldcg16(src + (size_t)m * K + v * V);
     } else {   // ST_CPROJ: merge the key ranges of every head
       const int q4 = d / 4;
 #pragma unroll 1
       for (int i = tid; i < B * q4; i += CONS) {
         const int m = i / q4, e = (i - m * q4) * 4, h = e / hd;
-        const float* p = att + (size_t)(m * H + h) * S * (hd + 4);
+        const float* p = att_at() + (size_t)(m * H + h) * S * (hd + 4);
         float4 n4[8];
         float2 md[8];
 #pragma unroll
@@ -673,29 +782,50 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
         for (int j = 0; j < 4; j++) dst[j] = Elem<T>::from_f(y[j]);
       }
     }
-    cons_bar();
+    if (!go_on()) break;
+    if (normed && tid < B) {   // (read behind the barrier at the end of the product)
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < NW; w++) s += s_part[tid][w];
+      s_scale[tid] = rsqrtf(s / (float)d + (kind == ST_LM_HEAD ? a.eps_final : kind == ST_GATE_UP ? L.eps2 : L.eps1));
+    }
 
     // ================================================================ the product
+    const uint32_t tag = tag_of(sg.layer);
     auto finish = [&](int m, int n, float v, float v2) {   // m sequence, n feature; v2: the up projection
+      if (normed) {
+        v *= s_scale[m];
+        v2 *= s_scale[m];
+      }
       switch (kind) {
         case ST_STU: {
           const float xp = round_to<T>(v);
           ((T*)L.hist)[((size_t)((size_t)m * d + n) * 2 + par) * L.Lh + s_pos] = Elem<T>::from_f(xp);
-          const float y = round_to<T>(2.f * (s_hist[m * own + lane] + xp * tap0));
-          mid[(size_t)m * d + n] = Elem<T>::from_f(res + y);
+          stream = round_to<T>(stream + round_to<T>(2.f * (s_hist[tid] + xp * tap0)));
+          Tagged<T>::put(rows_at(MID_ROWS + m), n, Elem<T>::from_f(stream), tag);
           break;
         }
-        case ST_QKV: qkv[(size_t)m * N + n] = Elem<T>::from_f(v); break;
-        case ST_CPROJ: mid[(size_t)m * d + n] = Elem<T>::from_f(res + round_to<T>(v)); break;
-        case ST_GATE_UP:
-          hbuf[(size_t)m * N + n] = Elem<T>::from_f(round_to<T>(gelu_tanh(round_to<T>(v))) * round_to<T>(v2));
+        case ST_QKV: Tagged<T>::put(rows_at(QKV_ROWS + 3 * m), n, Elem<T>::from_f(v), tag); break;
+        case ST_CPROJ:
+          stream = round_to<T>(stream + round_to<T>(v));
+          Tagged<T>::put(rows_at(MID_ROWS + m), n, Elem<T>::from_f(stream), tag);
           break;
-        case ST_DOWN: xbuf[(size_t)m * d + n] = Elem<T>::from_f(res + round_to<T>(v)); break;
+        case ST_GATE_UP: {
+          const T h = Elem<T>::from_f(round_to<T>(gelu_tanh(round_to<T>(v))) * round_to<T>(v2));
+          if (P.tagged_h) Tagged<T>::put(rows_at(H_ROWS) + (size_t)m * I * TB, n, h, tag);
+          else ((T*)rows_at(H_ROWS))[(size_t)m * I + n] = h;
+          break;
+        }
+        case ST_DOWN:
+          stream = round_to<T>(stream + round_to<T>(v));
+          Tagged<T>::put(rows_at(X_ROWS + m), n, Elem<T>::from_f(stream), tag);
+          if (sg.layer == a.n_layers - 1) xbuf[(size_t)m * d + n] = Elem<T>::from_f(stream);
+          break;
         default: ((T*)a.logits)[(size_t)m * a.ld_logits + n] = Elem<T>::from_f(v);
       }
     };
     const bool dual = kind == ST_GATE_UP;
-    const int r0 = s_range[st].r0, r1 = s_range[st].r1, F = dual ? 8 : 16;
+    const int F = dual ? 8 : 16;
 #pragma unroll 1
     for (int base = r0; base < r1; base += TILES * F) {   // tiles whose sums fit the buffer
       const int feats = min(TILES * F, r1 - base);
@@ -703,18 +833,18 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
       for (int f = 0; f < feats; f += F) {
         const int nf = min(F, feats - f), rows = dual ? 2 * nf : nf;
         float* sums = red + (f / F) * (NW * 128);
-        float acc[2][4];
+        float acc[4][4];
 #pragma unroll
-        for (int c = 0; c < 4; c++) acc[0][c] = acc[1][c] = 0.f;
-        const int pieces = sg.pieces == 1 ? 1 : unit_pieces(rows, sg.pieces, slots, packed, xs_cols / d);
+        for (int c = 0; c < 4; c++) acc[0][c] = acc[1][c] = acc[2][c] = acc[3][c] = 0.f;
+        const int pieces = sg.pieces == 1 ? 1 : rows == down_rows ? down_pieces : unit_pieces(rows, sg.pieces, slots, packed, xs_cols / d);
 #pragma unroll 1
         for (int k0 = 0, p0 = 0; k0 < K; k0 += pieces * d, p0 += pieces, unit++) {
           const int np = min(pieces, sg.pieces - p0), n = rows * np, len = min(np * d, K - k0);
           if (slot + n > slots) slot = 0;
-          const int kx = sg.pieces == 1 ? 0 : k0 % xs_cols;   // column of the unit in the rows
+          const int kx = k0 < xs_cols ? k0 : k0 % xs_cols;   // column of the unit in the rows
           if (k0 && kx == 0) {   // the next columns of the rows (one tile only: own <= 32 features, see the host)
             cons_bar();
-            load_rows(hbuf, K, k0, min(xs_cols, K - k0), pitch);
+            load_h(sg.layer, k0, min(xs_cols, K - k0), pitch);
             cons_bar();
           }
           const unsigned char* rows0 = ring + (size_t)slot * pitch_w;
@@ -726,18 +856,26 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
             const int rh = (dual ? nf : 8) + g;
             const unsigned char* hi_row = rows0 + (rh < rows ? rh * row_pitch : 0);
             const unsigned char* xrow = xs + g * pitch + kx * 2;
-            const int nch = (len + 31) >> 5;
-#pragma unroll 3
-            for (int c = warp; c < nch; c += NW) {
-              const int k = c * 32 + q * 8;
-              uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, xv = lo;
-              if (k + 8 <= len) {
-                lo = *reinterpret_cast<const uint4*>(lo_row + k * 2);
-                hi = *reinterpret_cast<const uint4*>(hi_row + k * 2);
-                if (g < B) xv = *reinterpret_cast<const uint4*>(xrow + k * 2);
+            const int nch = (len + 31) >> 5, last = len - 8 - q * 8;
+            const unsigned char *lo_p = lo_row + q * 16, *hi_p = hi_row + q * 16, *x_p = xrow + q * 16;
+#pragma unroll 1
+            for (int c = warp; c < nch; c += 2 * NW) {
+              uint4 lo[2], hi[2], xv[2];
+#pragma unroll
+              for (int u = 0; u < 2; u++) {
+                lo[u] = hi[u] = xv[u] = make_uint4(0, 0, 0, 0);
+                if ((c + u * NW) * 32 <= last) {   // (the end of a row may lie inside a chunk)
+                  lo[u] = *reinterpret_cast<const uint4*>(lo_p + (c + u * NW) * 64);
+                  hi[u] = *reinterpret_cast<const uint4*>(hi_p + (c + u * NW) * 64);
+                  if (g < B) xv[u] = *reinterpret_cast<const uint4*>(x_p + (c + u * NW) * 64);
+                }
               }
-              mma_16816(acc[0], lo.x, hi.x, lo.y, hi.y, xv.x, xv.y);
-              mma_16816(acc[1], lo.z, hi.z, lo.w, hi.w, xv.z, xv.w);
+#pragma unroll
+              for (int u = 0; u < 2; u++)
+                if (c + u * NW < nch) {
+                  mma_16816(acc[2 * u & 3], lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
+                  mma_16816(acc[2 * u + 1 & 3], lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
+                }
             }
           } else {
             // pairs of rows over teams of warps, the chunks of the unit over the wk warps of a team
@@ -782,12 +920,12 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
         }
         if (sizeof(T) == 2)
 #pragma unroll
-          for (int c = 0; c < 4; c++) sums[warp * 128 + c * 32 + lane] = acc[0][c] + acc[1][c];
+          for (int c = 0; c < 4; c++) sums[warp * 128 + c * 32 + lane] = (acc[0][c] + acc[1][c]) + (acc[2][c] + acc[3][c]);
       }
       cons_bar();
 #pragma unroll 1
-      for (int n = lane; n < feats && warp < B; n += 32) {
-        const int m = warp, i = dual ? n >> 3 : n >> 4, row = n & (F - 1);
+      for (int e = tid; e < B * feats; e += CONS) {
+        const int m = B == 1 ? 0 : e / feats, n = e - m * feats, i = dual ? n >> 3 : n >> 4, row = n & (F - 1);
         const float* sums = red + i * (NW * 128);
         float v = 0.f, v2 = 0.f;
         if (sizeof(T) == 2) {
@@ -809,7 +947,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
       }
       if (base + feats < r1) cons_bar();   // the sums have been read
     }
-    if (st + 1 < nst) arrive();
+    if (kind == ST_GATE_UP && !P.tagged_h) arrive();
   }
   __syncthreads();   // with the producer
   if (s_abort) {
@@ -817,9 +955,14 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
       atomicExch(epoch_word + 1, 1);
       if (a.status) atomicExch(a.status, 12);
     }
-  } else if (cta == 0) {   // every CTA has read the positions and the epoch long ago (it arrived at a barrier since)
+  } else if (cta == 0) {   // once every CTA has read the positions and the control words (long ago, but for idle ones)
+    if (tid == 0) poll_count(started, G);
+    cons_bar();
     for (int i = tid; i < a.n_layers * B; i += CONS) layers[i / B].pos[2 * (i % B)] = t + 1;
-    if (tid == 0) *epoch_word = epoch + 1;
+    if (tid == 0) {
+      epoch_word[2] = P.signature;
+      *epoch_word = epoch + 1;
+    }
   }
 }
 
@@ -835,7 +978,7 @@ int launch_step(const Params& P, size_t smem, cudaStream_t st) {
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeCooperative;   // the grid barriers need every CTA resident
+  at[0].id = cudaLaunchAttributeCooperative;   // its CTAs wait for one another: all of them resident
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
@@ -871,8 +1014,8 @@ int ring_slots(int B, int d, int I, int dtype) {
 // the attention items.
 extern "C" long long stu_token_step_workspace_bytes(int d, int I, int H, int dtype) {
   if (d <= 0 || I <= 0 || H < 0) return 0;
-  const long long e = dtype == STU_BF16 ? 2 : 4, hd = H > 0 ? d / H : 0;
-  return 512 + (32ll * d + 8ll * I) * e + (8ll * H + 160) * (hd + 4) * 4 + 256;
+  const long long e = dtype == STU_BF16 ? Tagged<bf16>::BYTES : Tagged<float>::BYTES, hd = H > 0 ? d / H : 0;
+  return 512 + (40ll * d + 8ll * I) * e + (8ll * H + 160) * (hd + 4) * 4 + 256;
 }
 
 // 1 when stu_token_step takes a stack of these sizes, else 0.  H = 0: no attention layer.
@@ -1000,10 +1143,17 @@ extern "C" int stu_token_step(const void* plan, int n_stages, const StuStepArgs*
   P.xs_cols = held_cols(a.B, a.d, a.I, dtype);
   P.pitch = slot_pitch(a.d, dtype);
   P.scale = a.H > 0 ? 1.0f / sqrtf((float)(a.d / a.H)) : 1.f;
+  P.tagged_h = (long long)a.B * a.I * (dtype == STU_BF16 ? Tagged<bf16>::BYTES : Tagged<float>::BYTES) <= TAGGED_H_BYTES;
+  P.signature = (int)((((a.B * 64 + a.n_layers) * 1021 + a.H) * 65521u + (unsigned)a.d * 8191u + (unsigned)a.I) * 4u + (dtype == STU_BF16 ? 3u : 2u));
   const size_t smem = (((size_t)P.slots * P.pitch + 127) & ~(size_t)127) + RED_BYTES +
                       (size_t)a.B * row_pitch(P.xs_cols, dtype);
   cudaStream_t st = (cudaStream_t)stream;
-  if (dtype == STU_BF16) return launch_step<bf16, 8>(P, smem, st);
+  if (dtype == STU_BF16) {
+    if (a.B == 1) return launch_step<bf16, 1>(P, smem, st);
+    if (a.B == 2) return launch_step<bf16, 2>(P, smem, st);
+    if (a.B <= 4) return launch_step<bf16, 4>(P, smem, st);
+    return launch_step<bf16, 8>(P, smem, st);
+  }
   if (a.B == 1) return launch_step<float, 1>(P, smem, st);
   if (a.B == 2) return launch_step<float, 2>(P, smem, st);
   if (a.B <= 4) return launch_step<float, 4>(P, smem, st);

@@ -371,7 +371,7 @@ int stu_peer_exchange(const void* xchg, void* x, long long x_row_stride, const v
  * cooperative kernel for up to 8 sequences at one common position: x = layers(x) in place, or, with `ids`, from the
  * token ids, and with `lm_head` to the logits of the final norm (flash_stu/model.py:150-205).  Appends to every layer's
  * cache and advances its positions.  All layers share d, I, and the attention layers H and window.  Status 6 when the
- * cached positions differ, 2 beyond a history, 1 for an id outside the vocabulary.  12 when a grid barrier or a copy was
+ * cached positions differ, 2 beyond a history, 1 for an id outside the vocabulary.  12 when another CTA or a copy was
  * waited for in vain: caches, positions and outputs are undefined, the workspace's second word is set, and launches on
  * that workspace return with status 12 until it is zeroed. */
 #define STU_STEP_MAX_LAYERS 40

@@ -421,3 +421,28 @@ def test_checkpoint_written_with_the_reference_layout_loads_and_reproduces_its_l
     assert wider.shape[-1] == V + 7 and m2.lm_head.weight.data_ptr() == m2.tok_emb.weight.data_ptr()
     close(wider[..., :V], r["logits_full"], 1e-3)
     ops.check_status()
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_token_steps_of_two_models_on_one_workspace(monkeypatch, dt):
+    """The row buffers of the token step are polled for their contents: a workspace that was last used for other sizes holds
+    words that must not be taken for this launch's."""
+    from flash_stu_2_b200 import ops, token_step
+    models = [_random_model(256, 4, dt), _random_model(320, 5, dt, layers=3)]
+    prompt = torch.randint(0, 1003, (2, 30), device=dev())
+    want = [m.generate(prompt, max_length=40, do_sample=False, return_logits=True) for m in models]
+    shared = torch.zeros(1 << 22, dtype=torch.uint8, device=dev())
+    make = token_step.TokenStep.__init__
+
+    def on_shared(self, *args, **kw):
+        make(self, *args, **kw)
+        assert self._ws.numel() <= shared.numel()
+        self._ws = shared
+        self.args.workspace = shared.data_ptr()
+
+    monkeypatch.setattr(token_step.TokenStep, "__init__", on_shared)
+    for _ in range(3):
+        for m, (ids, logits) in zip(models, want):
+            got = m.generate(prompt, max_length=40, do_sample=False, return_logits=True)
+            assert torch.equal(got[0], ids) and torch.equal(got[1], logits)
+    ops.check_status()
