@@ -1,4 +1,5 @@
-"""Compile the CUDA sources under csrc/ into libstu_b200.so next to this file (nvcc, sm_100a only).
+"""Compile the CUDA sources under csrc/ into libstu_b200.so next to this file (nvcc, sm_100a only), and the extension
+module _native (csrc/native.cpp, the host compiler), through which the interpreter calls it.
 
 Every .cu file is compiled to an object of its own (in parallel, re-used while the source and the shared headers
 are older than it) and the objects are linked into the shared library; no device symbol crosses a file boundary,
@@ -6,12 +7,15 @@ so no relocatable device code is needed."""
 import glob
 import os
 import subprocess
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libstu_b200.so")
+NATIVE_SRC = os.path.join(CSRC, "native.cpp")
+NATIVE = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 
@@ -27,7 +31,28 @@ def stale() -> bool:
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(p) > t for p in sources() + headers())
+    return any(os.path.getmtime(p) > t for p in sources() + headers()) or native_stale()
+
+
+def native_stale() -> bool:
+    if not os.path.exists(NATIVE):
+        return True
+    t = os.path.getmtime(NATIVE)
+    return any(os.path.getmtime(p) > t for p in [NATIVE_SRC] + glob.glob(os.path.join(HERE, "..", "include", "*.h")))
+
+
+def build_native() -> str:
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
+           f"-I{cuda}/include", "-o", NATIVE, NATIVE_SRC, f"-L{HERE}", "-l:libstu_b200.so", f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+           "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("the host compiler failed on native.cpp:\n" + res.stdout + res.stderr)
+    return NATIVE
 
 
 def _nvcc():
@@ -58,6 +83,8 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("link failed:\n" + res.stdout + res.stderr)
     if verbose:
         print("".join(log for _, log in results))
+    if force or native_stale():
+        build_native()
     return LIB
 
 

@@ -144,6 +144,19 @@ def load(build_if_missing: bool = True):
     return lib
 
 
+_native = None
+
+
+def native():
+    """The same functions as an extension module (what ops.py launches): tensors or addresses for pointers, no ctypes between."""
+    global _native
+    if _native is None:
+        load()
+        from . import _native as module
+        _native = module
+    return _native
+
+
 ERR_UNSUPPORTED = -4
 
 

@@ -1,0 +1,250 @@
+// The C-ABI of include/stu_b200.h as functions of a Python extension module, and the two calls that every layer makes most, the
+// linear layer and the norm, from tensors in one step.  A launch through ctypes costs 4 us of argument conversion and 5 more of
+// checks in the interpreter, as much as the launch itself; token steps of small batches and short prefills are bound by that.
+//
+// Arguments are positional.  A pointer parameter takes a CUDA tensor (its first element), an address or None.  The lock of the
+// interpreter is released around the call.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <atomic>
+#include <stdexcept>
+#include <tuple>
+#include <utility>
+
+#include "../../include/stu_b200.h"
+
+namespace {
+
+struct BadArgument : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+
+template <typename T> T value_of(PyObject* o);
+template <> long long value_of<long long>(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw BadArgument("");
+  return v;
+}
+template <> int value_of<int>(PyObject* o) {
+  const long long v = value_of<long long>(o);
+  if (v != (int)v) {
+    PyErr_SetString(PyExc_OverflowError, "an int argument does not fit 32 bits");
+    throw BadArgument("");
+  }
+  return (int)v;
+}
+template <> float value_of<float>(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw BadArgument("");
+  return (float)v;
+}
+void* address_of(PyObject* o) {
+  if (o == Py_None) return nullptr;
+  if (THPVariable_Check(o)) {
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (!t.is_cuda()) {
+      PyErr_SetString(PyExc_RuntimeError, "flash_stu_2_b200 has no CPU path: tensors must live on a CUDA device");
+      throw BadArgument("");
+    }
+    return t.data_ptr();
+  }
+  void* p = PyLong_AsVoidPtr(o);
+  if (!p && PyErr_Occurred()) throw BadArgument("");
+  return p;
+}
+template <typename T> struct Convert {
+  static T from(PyObject* o) { return value_of<T>(o); }
+};
+template <typename T> struct Convert<T*> {
+  static T* from(PyObject* o) { return static_cast<T*>(const_cast<typename std::remove_const<T>::type*>(
+      static_cast<const T*>(address_of(o)))); }
+};
+
+template <auto F> struct Call;
+template <typename R, typename... A, R (*F)(A...)> struct Call<F> {
+  template <size_t... I>
+  static R run(PyObject* const* args, std::index_sequence<I...>) {
+    std::tuple<A...> a{Convert<A>::from(args[I])...};
+    R r;
+    Py_BEGIN_ALLOW_THREADS
+    r = F(std::get<I>(a)...);
+    Py_END_ALLOW_THREADS
+    return r;
+  }
+  static PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != (Py_ssize_t)sizeof...(A)) {
+      PyErr_Format(PyExc_TypeError, "%zd arguments expected, %zd given", (Py_ssize_t)sizeof...(A), n);
+      return nullptr;
+    }
+    try {
+      return PyLong_FromLongLong((long long)run(args, std::make_index_sequence<sizeof...(A)>()));
+    } catch (const BadArgument&) {
+      return nullptr;
+    } catch (const std::exception& e) {
+      PyErr_SetString(PyExc_RuntimeError, e.what());
+      return nullptr;
+    }
+  }
+};
+
+// Devices whose status word has been registered (ops.status_word)
+std::atomic<unsigned long long> g_ready{0};
+PyObject* status_ready(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  const long dev = n == 1 ? PyLong_AsLong(args[0]) : -1;
+  if (dev < 0 || dev >= 64) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "a device index is expected");
+    return nullptr;
+  }
+  g_ready.fetch_or(1ull << dev);
+  Py_RETURN_NONE;
+}
+
+int dtype_code(const at::Tensor& t) {
+  return t.scalar_type() == at::kBFloat16 ? 1 : t.scalar_type() == at::kFloat ? 0 : -1;
+}
+// A plain CUDA tensor or None (null); anything else: the caller's other path decides.
+bool plain(PyObject* o, const at::Tensor** t) {
+  *t = nullptr;
+  if (o == Py_None) return true;
+  if (!THPVariable_Check(o)) return false;
+  *t = &THPVariable_Unpack(o);
+  return (*t)->is_cuda();
+}
+void* data_of(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
+
+// linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed, hist_T, hist_t0, hist_Lh) -> y, or None where a check
+// fails or the library refuses: ops.linear then goes through its own checks, which raise what they raise.
+PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 13) {
+    PyErr_SetString(PyExc_TypeError, "13 arguments expected");
+    return nullptr;
+  }
+  try {
+    const at::Tensor *x, *W, *W2, *resid, *out, *norm_w;
+    if (!plain(args[0], &x) || !plain(args[1], &W) || !plain(args[2], &W2) || !plain(args[3], &resid) || !plain(args[4], &out) ||
+        !plain(args[6], &norm_w) || !x || !W)
+      Py_RETURN_NONE;
+    const int epi = value_of<int>(args[5]), code = dtype_code(*x), dev = x->device().index();
+    if (code < 0 || x->dim() != 2 || W->dim() != 2 || x->stride(1) != 1 || !(g_ready.load(std::memory_order_relaxed) >> dev & 1))
+      Py_RETURN_NONE;
+    const long long M = x->size(0), K = x->size(1);
+    const bool transposed = value_of<int>(args[9]) != 0;
+    if (W->size(transposed ? 0 : 1) != K) Py_RETURN_NONE;
+    const long long N = W->size(transposed ? 1 : 0), w_rs = W->stride(transposed ? 1 : 0), w_ks = W->stride(transposed ? 0 : 1);
+    if (M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) Py_RETURN_NONE;
+    if (W2 && (W2->sizes() != W->sizes() || W2->strides() != W->strides())) Py_RETURN_NONE;
+    if (resid && (resid->dim() != 2 || resid->size(0) != M || resid->size(1) != N || resid->stride(1) != 1)) Py_RETURN_NONE;
+    const bool hist = (epi & 0xff) == 3;
+    at::Tensor made;
+    long long y_rs = 0;
+    if (hist) {
+      if (!out) Py_RETURN_NONE;
+    } else {
+      if (!out) {
+        made = at::empty({M, N}, x->options());
+        out = &made;
+      }
+      if (out->dim() != 2 || out->size(0) != M || out->size(1) != N || out->stride(1) != 1) Py_RETURN_NONE;
+      y_rs = out->stride(0);
+    }
+    const float eps = value_of<float>(args[7]);
+    const int backend = value_of<int>(args[8]), hT = value_of<int>(args[10]), ht0 = value_of<int>(args[11]), hLh = value_of<int>(args[12]);
+    void *px = data_of(x), *pW = data_of(W), *pW2 = data_of(W2), *pr = data_of(resid), *py = data_of(out), *pn = data_of(norm_w);
+    const long long lda = x->stride(0), r_rs = resid ? resid->stride(0) : 0;
+    void* stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = stu_linear(px, lda, pW, w_rs, w_ks, pW2, pr, r_rs, py, y_rs, (int)M, (int)N, (int)K, epi, hT, ht0, hLh, pn, eps, code, backend, stream);
+    Py_END_ALLOW_THREADS
+    if (rc != 0) Py_RETURN_NONE;
+    if (made.defined()) return THPVariable_Wrap(std::move(made));
+    Py_INCREF(args[4]);
+    return args[4];
+  } catch (const BadArgument&) {
+    PyErr_Clear();
+  } catch (const std::exception&) {
+  }
+  Py_RETURN_NONE;
+}
+
+// rmsnorm(x, weight, eps) -> y, or None as above.
+PyObject* rmsnorm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3) {
+    PyErr_SetString(PyExc_TypeError, "3 arguments expected");
+    return nullptr;
+  }
+  try {
+    const at::Tensor *x, *w;
+    if (!plain(args[0], &x) || !plain(args[1], &w) || !x || !w) Py_RETURN_NONE;
+    const int code = dtype_code(*x);
+    if (code < 0 || x->dim() < 1 || !x->is_contiguous() || x->numel() == 0) Py_RETURN_NONE;
+    const long long d = x->size(-1), rows = x->numel() / d;
+    if (rows > INT32_MAX || d > INT32_MAX) Py_RETURN_NONE;
+    at::Tensor y = at::empty(x->sizes(), x->options());
+    void *px = data_of(x), *pw = data_of(w), *py = y.data_ptr(), *stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
+    const float eps = value_of<float>(args[2]);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = stu_rmsnorm(px, pw, py, (int)rows, (int)d, d, d, eps, code, stream);
+    Py_END_ALLOW_THREADS
+    if (rc == 0) return THPVariable_Wrap(std::move(y));
+  } catch (const BadArgument&) {
+    PyErr_Clear();
+  } catch (const std::exception&) {
+  }
+  Py_RETURN_NONE;
+}
+
+// what ops.py launches
+#define ENTRY(name) {#name, (PyCFunction)(void (*)(void))Call<&name>::call, METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    ENTRY(stu_bias_act),
+    ENTRY(stu_block_decode_step),
+    ENTRY(stu_block_step_workspace_bytes),
+    ENTRY(stu_conv_prefill_approx),
+    ENTRY(stu_conv_prefill_approx_static),
+    ENTRY(stu_conv_prefill_approx_tc5),
+    ENTRY(stu_decode_approx),
+    ENTRY(stu_decode_approx_pipelined),
+    ENTRY(stu_decode_approx_projected),
+    ENTRY(stu_decode_approx_push),
+    ENTRY(stu_decode_approx_shard),
+    ENTRY(stu_embed),
+    ENTRY(stu_full_combine),
+    ENTRY(stu_full_conv),
+    ENTRY(stu_full_decode_combine),
+    ENTRY(stu_full_conv_tc5),
+    ENTRY(stu_full_decode_prepare),
+    ENTRY(stu_full_decode_step),
+    ENTRY(stu_lds_chunk_scan),
+    ENTRY(stu_lds_decode_features),
+    ENTRY(stu_lds_final_state),
+    ENTRY(stu_linear),
+    ENTRY(stu_linear_can_fuse_norm),
+    ENTRY(stu_linear_push),
+    ENTRY(stu_peer_combine),
+    ENTRY(stu_peer_exchange),
+    ENTRY(stu_rmsnorm),
+    ENTRY(stu_sample),
+    ENTRY(stu_swa_forward),
+    ENTRY(stu_swa_prefill_scratch_elems),
+    ENTRY(stu_swa_prefill_tc5),
+    ENTRY(stu_taps_even),
+    ENTRY(stu_taps_rev8),
+    ENTRY(stu_to_history),
+    ENTRY(stu_toeplitz),
+    {"status_ready", (PyCFunction)(void (*)(void))status_ready, METH_FASTCALL, nullptr},
+    {"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, nullptr},
+    {"rmsnorm", (PyCFunction)(void (*)(void))rmsnorm, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }

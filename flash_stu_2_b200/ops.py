@@ -80,6 +80,7 @@ def status_word(device) -> torch.Tensor:
         _status[key] = w
         with torch.cuda.device(key):   # the library keeps one word per device, registered with that device current
             _lib.check(_lib.load().stu_set_status_word(w.data_ptr()), "stu_set_status_word")
+        _lib.native().status_ready(key)
     return _status[key]
 
 
@@ -141,6 +142,11 @@ def empty(shape, dtype: torch.dtype, device) -> torch.Tensor:
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = RMS_EPS, out: Optional[torch.Tensor] = None):
+    if out is None and getattr(_local, "arena", None) is None:
+        y = _lib.native().rmsnorm(x, weight, eps)
+        if y is not None:
+            _count()
+            return y
     _cuda(x, weight)
     d = x.shape[-1]
     x2 = x.reshape(-1, d)
@@ -149,7 +155,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = RMS_EPS, out: Op
     if out is None:
         out = empty(x2.shape, x.dtype, x.device)
     o2 = out.reshape(-1, d)
-    rc = _lib.load().stu_rmsnorm(x2.data_ptr(), weight.data_ptr(), o2.data_ptr(), x2.shape[0], d, x2.stride(0),
+    rc = _lib.native().stu_rmsnorm(x2.data_ptr(), weight.data_ptr(), o2.data_ptr(), x2.shape[0], d, x2.stride(0),
                                  o2.stride(0), eps, _dt(x), _stream())
     _lib.check(rc, "stu_rmsnorm")
     _count()
@@ -165,7 +171,7 @@ def bias_act(y: torch.Tensor, bias: Optional[torch.Tensor], act: int = ACT_NONE)
     cols = y.shape[-1]
     y2 = y.view(-1, cols)
     assert y2.stride(1) == 1 and (bias is None or (bias.shape == (cols,) and bias.is_contiguous()))
-    rc = _lib.load().stu_bias_act(y2.data_ptr(), _p(bias), y2.shape[0], cols, y2.stride(0), act, _dt(y), _stream())
+    rc = _lib.native().stu_bias_act(y2.data_ptr(), _p(bias), y2.shape[0], cols, y2.stride(0), act, _dt(y), _stream())
     _lib.check(rc, "stu_bias_act")
     _count()
     return y
@@ -175,7 +181,7 @@ def embed(ids: torch.Tensor, table: torch.Tensor):
     _cuda(ids, table)
     ids = ids.contiguous().to(torch.int64)
     out = empty((*ids.shape, table.shape[1]), table.dtype, table.device)
-    rc = _lib.load().stu_embed(ids.data_ptr(), table.data_ptr(), out.data_ptr(), ids.numel(), table.shape[1],
+    rc = _lib.native().stu_embed(ids.data_ptr(), table.data_ptr(), out.data_ptr(), ids.numel(), table.shape[1],
                                table.shape[0], status_word(table.device).data_ptr(), _dt(table), _stream())
     _lib.check(rc, "stu_embed")
     _count()
@@ -188,7 +194,7 @@ def can_fuse_norm(M: int, N: int, K: int, epilogue: int, dtype: torch.dtype) -> 
         # of every value by every warp costs more than a launch (8 rows, 50257 x 1536: 120 us fused, 106 apart)
         wide = N > (4736 if epilogue == EPI_GELU_MUL else 18944)
         return M <= (4 if wide else 8) and K % 4 == 0 and epilogue in (EPI_STORE, EPI_RESID, EPI_GELU_MUL)
-    return bool(_lib.load().stu_linear_can_fuse_norm(M, N, K, epilogue, 1))
+    return bool(_lib.native().stu_linear_can_fuse_norm(M, N, K, epilogue, 1))
 
 
 def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = None,
@@ -197,6 +203,12 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
            transposed_weight: bool = False, hist_T: int = 0, hist_t0: int = 0, hist_Lh: int = 0,
            kpos: Optional[torch.Tensor] = None):
     """y = epilogue(x @ W^T) for x [M,K] and W [N,K] (or W [K,N] with transposed_weight=True)."""
+    if kpos is None and (out is not None or getattr(_local, "arena", None) is None):
+        # checks, output and launch in one native call; None: whatever is out of the ordinary is looked at below
+        y = _lib.native().linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed_weight, hist_T, hist_t0, hist_Lh)
+        if y is not None:
+            _count()
+            return y
     _cuda(x, W, W2, resid, out, norm_w)
     assert x.dim() == 2 and W.dim() == 2 and x.stride(1) == 1
     M, K = x.shape
@@ -224,7 +236,7 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
         assert resid is None and epilogue == EPI_STORE and kpos.is_cuda and kpos.dtype == torch.int32
         resid, epilogue = kpos, EPI_STORE | EPI_FLAG_KPOS
     status_word(x.device)   # the tcgen05 GEMM reports an expired device-side wait through the registered word
-    rc = _lib.load().stu_linear(x.data_ptr(), x.stride(0), W.data_ptr(), w_rs, w_ks, _p(W2), _p(resid), r_rs,
+    rc = _lib.native().stu_linear(x.data_ptr(), x.stride(0), W.data_ptr(), w_rs, w_ks, _p(W2), _p(resid), r_rs,
                                 out.data_ptr(), y_rs, M, N, K, epilogue, hist_T, hist_t0, hist_Lh, _p(norm_w), eps,
                                 _dt(x), backend, _stream())
     if rc == _lib.ERR_UNSUPPORTED and norm_w is not None and x.dtype == torch.float32 and backend == BACKEND_AUTO:
@@ -241,7 +253,7 @@ def taps_even(fp: torch.Tensor, Lh: int):
     fp = fp.contiguous()
     L, d = fp.shape
     taps = torch.zeros(d, Lh, dtype=fp.dtype, device=fp.device)
-    rc = _lib.load().stu_taps_even(fp.data_ptr(), taps.data_ptr(), L, d, Lh, _dt(fp), _stream())
+    rc = _lib.native().stu_taps_even(fp.data_ptr(), taps.data_ptr(), L, d, Lh, _dt(fp), _stream())
     _lib.check(rc, "stu_taps_even")
     _count()
     return taps
@@ -252,7 +264,7 @@ def taps_rev8(taps: torch.Tensor):
     _cuda(taps)
     d, Lh = taps.shape
     out = torch.empty(8, d, Lh + 8, dtype=taps.dtype, device=taps.device)
-    rc = _lib.load().stu_taps_rev8(taps.data_ptr(), out.data_ptr(), d, Lh, _dt(taps), _stream())
+    rc = _lib.native().stu_taps_rev8(taps.data_ptr(), out.data_ptr(), d, Lh, _dt(taps), _stream())
     _lib.check(rc, "stu_taps_rev8")
     _count()
     return out
@@ -264,7 +276,7 @@ def conv_prefill_approx(hist, taps, yT, x, t0: int, t_end: int, use_tensor_cores
     B, d, _, Lh = hist.shape
     assert hist.is_contiguous() and yT.is_contiguous() and taps.shape == (d, Lh) and taps.is_contiguous()
     assert x.shape == (B, t_end - t0, d) and x.stride(2) == 1
-    rc = _lib.load().stu_conv_prefill_approx(hist.data_ptr(), taps.data_ptr(), yT.data_ptr(), x.data_ptr(),
+    rc = _lib.native().stu_conv_prefill_approx(hist.data_ptr(), taps.data_ptr(), yT.data_ptr(), x.data_ptr(),
                                              x.stride(0), x.stride(1), B, d, Lh, yT.shape[3], t0, t_end, _dt(x),
                                              int(use_tensor_cores), _stream())
     _lib.check(rc, "stu_conv_prefill_approx")
@@ -283,7 +295,7 @@ def conv_prefill_approx_tc5(hist, taps8, yT, x, t0: int, t_end: int):
     B, d, _, Lh = hist.shape
     assert hist.is_contiguous() and yT.is_contiguous() and taps8.shape == (8, d, Lh + 8) and taps8.is_contiguous()
     assert x.shape == (B, t_end - t0, d) and x.stride(2) == 1
-    rc = _lib.load().stu_conv_prefill_approx_tc5(hist.data_ptr(), taps8.data_ptr(), yT.data_ptr(), x.data_ptr(),
+    rc = _lib.native().stu_conv_prefill_approx_tc5(hist.data_ptr(), taps8.data_ptr(), yT.data_ptr(), x.data_ptr(),
                                                  x.stride(0), x.stride(1), B, d, Lh, yT.shape[3], t0, t_end,
                                                  status_word(x.device).data_ptr(), _dt(x), _stream())
     _lib.check(rc, "stu_conv_prefill_approx_tc5")
@@ -315,7 +327,7 @@ def conv_prefill_approx_static(hist, taps, x, t0: int, t_end: int, use_tensor_co
     B, d, _, Lh = hist.shape
     assert hist.is_contiguous() and taps.shape == (d, Lh) and taps.is_contiguous()
     assert x.shape == (B, t_end - t0, d) and x.stride(2) == 1
-    rc = _lib.load().stu_conv_prefill_approx_static(hist.data_ptr(), taps.data_ptr(), x.data_ptr(), x.stride(0),
+    rc = _lib.native().stu_conv_prefill_approx_static(hist.data_ptr(), taps.data_ptr(), x.data_ptr(), x.stride(0),
                                                     x.stride(1), B, d, Lh, t0, t_end, _dt(x), int(use_tensor_cores),
                                                     _stream())
     _lib.check(rc, "stu_conv_prefill_approx_static")
@@ -333,7 +345,7 @@ def decode_approx(x, norm_w, MinT, hist, taps, pos, out, eps: float = RMS_EPS, t
     assert x.shape == (B, d) and out.shape == (B, d) and x.stride(1) == 1 and out.stride(1) == 1
     assert pos.dtype == torch.int32 and pos.shape == (B, 2) and pos.is_contiguous()
     assert x.data_ptr() != out.data_ptr()
-    rc = _lib.load().stu_decode_approx(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(), hist.data_ptr(),
+    rc = _lib.native().stu_decode_approx(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(), hist.data_ptr(),
                                        taps.data_ptr(), _p(taps8), pos.data_ptr(), out.data_ptr(), out.stride(0), B, d,
                                        Lh, eps,
                                        status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
@@ -351,7 +363,7 @@ def decode_approx_shard(x, norm_w, MinT, hist, taps8, pos, out, eps: float = RMS
     d_in = x.shape[1]
     assert x.shape[0] == B and MinT.shape == (dch, d_in) and out.shape == (B, dch) and x.stride(1) == 1
     assert out.stride(1) == 1 and taps8.shape == (8, dch, Lh + 8) and pos.dtype == torch.int32
-    rc = _lib.load().stu_decode_approx_shard(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
+    rc = _lib.native().stu_decode_approx_shard(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
                                              hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), out.data_ptr(),
                                              out.stride(0), B, d_in, dch, Lh, eps, int(add_residual),
                                              status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
@@ -369,7 +381,7 @@ def decode_approx_projected(x, xp, hist, taps8, pos, out, add_residual: bool = T
     B, dch, _, Lh = hist.shape
     assert xp.shape == (B, dch) and out.shape == (B, dch) and xp.stride(1) == 1 and out.stride(1) == 1
     assert hist.is_contiguous() and taps8.is_contiguous() and (x is not None or not add_residual)
-    rc = _lib.load().stu_decode_approx_projected(_p(x), x.stride(0) if x is not None else 0, xp.data_ptr(),
+    rc = _lib.native().stu_decode_approx_projected(_p(x), x.stride(0) if x is not None else 0, xp.data_ptr(),
                                                  xp.stride(0), hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(),
                                                  out.data_ptr(), out.stride(0), B, dch, Lh, int(add_residual),
                                                  status_word(xp.device).data_ptr(), _dt(xp) | flags, _stream())
@@ -385,7 +397,7 @@ def linear_push(x: torch.Tensor, W: torch.Tensor, dest: int, dest_row_stride: in
     M, K = x.shape
     N = W.shape[0]
     assert W.shape[1] == K and x.stride(1) == 1 and W.stride(1) == 1
-    rc = _lib.load().stu_linear_push(x.data_ptr(), x.stride(0), W.data_ptr(), W.stride(0), M, N, K, dest,
+    rc = _lib.native().stu_linear_push(x.data_ptr(), x.stride(0), W.data_ptr(), W.stride(0), M, N, K, dest,
                                      dest_row_stride, _dt(x), _stream())
     _lib.check(rc, "stu_linear_push")
     _count()
@@ -397,7 +409,7 @@ def decode_approx_push(x, norm_w, MinT, hist, taps8, pos, dest: int, dest_row_st
     B, d_ch, _, Lh = hist.shape
     d_in = x.shape[1]
     assert MinT.shape == (d_ch, d_in) and MinT.is_contiguous() and hist.is_contiguous() and taps8.is_contiguous()
-    rc = _lib.load().stu_decode_approx_push(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
+    rc = _lib.native().stu_decode_approx_push(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
                                             hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), dest, dest_row_stride,
                                             B, d_in, d_ch, Lh, eps, status_word(x.device).data_ptr(), _dt(x),
                                             _stream())
@@ -411,7 +423,7 @@ def peer_combine(x, inbox: int, slot_stride: int, in_row_stride: int, slots: int
     _cuda(x)
     rows, d = x.shape
     assert x.stride(1) == 1 and (norm_w is None or (xn is not None and xn.shape == x.shape and xn.stride(1) == 1))
-    rc = _lib.load().stu_peer_combine(x.data_ptr(), x.stride(0), inbox, slot_stride, in_row_stride, slots, flags,
+    rc = _lib.native().stu_peer_combine(x.data_ptr(), x.stride(0), inbox, slot_stride, in_row_stride, slots, flags,
                                       n_ranks, epoch, _p(norm_w), _p(xn), xn.stride(0) if xn is not None else 0, eps,
                                       rows, d, status_word(x.device).data_ptr(), wait_ms, _dt(x), _stream())
     _lib.check(rc, "stu_peer_combine")
@@ -426,7 +438,7 @@ def peer_exchange(xchg: int, x, src, gather: bool, slot_stride: int, norm_w=None
     rows, d = x.shape
     assert src.shape[0] == rows and x.stride(1) == 1 and src.stride(1) == 1
     assert norm_w is None or (xn is not None and xn.shape == x.shape and xn.stride(1) == 1)
-    rc = _lib.load().stu_peer_exchange(xchg, x.data_ptr(), x.stride(0), src.data_ptr(), src.stride(0), src.shape[1],
+    rc = _lib.native().stu_peer_exchange(xchg, x.data_ptr(), x.stride(0), src.data_ptr(), src.stride(0), src.shape[1],
                                        int(gather), slot_stride, _p(norm_w), _p(xn),
                                        xn.stride(0) if xn is not None else 0, eps, rows, d,
                                        status_word(x.device).data_ptr(), wait_ms, _dt(x), _stream())
@@ -444,7 +456,7 @@ def decode_approx_pipelined(x, norm_w, MinT, hist, taps8, pos, out, eps: float =
     assert x.shape[0] == B and MinT.shape == (dch, d_in) and out.shape == (B, dch) and x.stride(1) == 1
     assert out.stride(1) == 1 and taps8.shape == (8, dch, Lh + 8) and pos.dtype == torch.int32 and pos.is_contiguous()
     assert hist.is_contiguous() and taps8.is_contiguous() and x.data_ptr() != out.data_ptr()
-    rc = _lib.load().stu_decode_approx_pipelined(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
+    rc = _lib.native().stu_decode_approx_pipelined(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
                                                  hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), out.data_ptr(),
                                                  out.stride(0), B, d_in, dch, Lh, eps, int(add_residual),
                                                  status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
@@ -456,7 +468,7 @@ def decode_approx_pipelined(x, norm_w, MinT, hist, taps8, pos, out, eps: float =
 def block_step_workspace(d: int, I: int, device) -> torch.Tensor:
     """Zeroed workspace of block_decode_step for one layer's cache (partial sums carried from one token step to the
     next, grid-barrier words, the step's intermediate rows)."""
-    n = int(_lib.load().stu_block_step_workspace_bytes(d, I))
+    n = int(_lib.native().stu_block_step_workspace_bytes(d, I))
     return torch.zeros((n + 255) // 256 * 256, dtype=torch.uint8, device=device)
 
 
@@ -470,7 +482,7 @@ def block_decode_step(x, stu_norm_w, MinT, hist, taps8, pos, mlp_norm_w, Wg, Wu,
     assert x.shape == (B, d) and out.shape == (B, d) and x.stride(1) == 1 and out.stride(1) == 1
     assert MinT.shape == (d, d) and Wg.shape == (I, d) and Wu.shape == (I, d) and Wd.shape == (d, I)
     assert all(w.is_contiguous() for w in (MinT, Wg, Wu, Wd, hist, taps8, pos)) and pos.dtype == torch.int32
-    rc = _lib.load().stu_block_decode_step(x.data_ptr(), x.stride(0), stu_norm_w.data_ptr(), MinT.data_ptr(),
+    rc = _lib.native().stu_block_decode_step(x.data_ptr(), x.stride(0), stu_norm_w.data_ptr(), MinT.data_ptr(),
                                            hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), mlp_norm_w.data_ptr(),
                                            Wg.data_ptr(), Wu.data_ptr(), Wd.data_ptr(), out.data_ptr(), out.stride(0),
                                            B, d, I, Lh, eps_stu, eps_mlp, workspace.data_ptr(), workspace.numel(), mode,
@@ -493,7 +505,7 @@ def to_history(x, hist, t0: int):
     _cuda(x, hist)
     B, T, d = x.shape
     assert hist.is_contiguous() and hist.shape[:3] == (B, d, 2) and x.stride(2) == 1
-    rc = _lib.load().stu_to_history(x.data_ptr(), x.stride(0), x.stride(1), hist.data_ptr(), B, d, hist.shape[3], t0,
+    rc = _lib.native().stu_to_history(x.data_ptr(), x.stride(0), x.stride(1), hist.data_ptr(), B, d, hist.shape[3], t0,
                                     t0 + T, _dt(x), _stream())
     _lib.check(rc, "stu_to_history")
     _count()
@@ -505,7 +517,7 @@ def toeplitz(phi, k: int, out):
     L, K = phi.shape
     assert phi.is_contiguous() and out.is_contiguous() and out.shape[0] == 3 and out.shape[1] == out.shape[2]
     col = phi[:, k]
-    rc = _lib.load().stu_toeplitz(col.data_ptr(), K, L, out.data_ptr(), out.shape[1], out.shape[2], _dt(phi), _stream())
+    rc = _lib.native().stu_toeplitz(col.data_ptr(), K, L, out.data_ptr(), out.shape[1], out.shape[2], _dt(phi), _stream())
     _lib.check(rc, "stu_toeplitz")
     _count()
 
@@ -513,7 +525,7 @@ def toeplitz(phi, k: int, out):
 def full_combine(E, Q, U, B: int, d: int, K: int, k: int, both_signs: bool, t0: int, t_end: int):
     _cuda(E, Q, U)
     assert E.shape == Q.shape and E.is_contiguous() and Q.is_contiguous() and U.stride(1) == 1
-    rc = _lib.load().stu_full_combine(E.data_ptr(), Q.data_ptr(), E.shape[1], U.data_ptr(), U.stride(0), B, d, K, k,
+    rc = _lib.native().stu_full_combine(E.data_ptr(), Q.data_ptr(), E.shape[1], U.data_ptr(), U.stride(0), B, d, K, k,
                                       int(both_signs), t0, t_end, _dt(E), _stream())
     _lib.check(rc, "stu_full_combine")
     _count()
@@ -525,7 +537,7 @@ def full_conv(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     B, d, _, Lh = hist.shape
     L, K = phi.shape
     assert hist.is_contiguous() and phi.is_contiguous() and U.stride(1) == 1 and U.shape[0] == B * (t_end - t0)
-    rc = _lib.load().stu_full_conv(hist.data_ptr(), Lh, phi.data_ptr(), L, K, U.data_ptr(), U.stride(0), B, d,
+    rc = _lib.native().stu_full_conv(hist.data_ptr(), Lh, phi.data_ptr(), L, K, U.data_ptr(), U.stride(0), B, d,
                                    int(both_signs), t0, t_end, _dt(hist), _stream())
     _lib.check(rc, "stu_full_conv")
     _count()
@@ -543,7 +555,7 @@ def full_conv_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     assert hist.is_contiguous() and phi.is_contiguous() and U.stride(1) == 1 and U.shape[0] == B * (t_end - t0)
     lib = _lib.load()
     tab = torch.empty(lib.stu_full_conv_tc5_scratch_elems(K, t_end), dtype=hist.dtype, device=hist.device)
-    rc = lib.stu_full_conv_tc5(hist.data_ptr(), Lh, phi.data_ptr(), L, K, tab.data_ptr(), U.data_ptr(), U.stride(0), B, d,
+    rc = _lib.native().stu_full_conv_tc5(hist.data_ptr(), Lh, phi.data_ptr(), L, K, tab.data_ptr(), U.data_ptr(), U.stride(0), B, d,
                                int(both_signs), t0, t_end, status_word(hist.device).data_ptr(), _dt(hist), _stream())
     _lib.check(rc, "stu_full_conv_tc5")
     _count(2)
@@ -562,7 +574,7 @@ def full_decode_step(x2d, norm_w, eps: float, hist, taps8, pos, U, limit: int, b
     B, d, _, Lh = hist.shape
     K = taps8.shape[1] // 2
     assert taps8.shape == (8, 2 * K, Lh + 8) and x2d.stride(1) == 1 and U.is_contiguous() and U.numel() == B * (1 + both_signs) * K * d
-    rc = _lib.load().stu_full_decode_step(x2d.data_ptr(), x2d.stride(0), norm_w.data_ptr() if norm_w is not None else None, eps,
+    rc = _lib.native().stu_full_decode_step(x2d.data_ptr(), x2d.stride(0), norm_w.data_ptr() if norm_w is not None else None, eps,
                                           hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), U.data_ptr(), B, d, K, Lh, limit,
                                           int(both_signs), status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
     _lib.check(rc, "stu_full_decode_step")
@@ -574,7 +586,7 @@ def full_decode_prepare(x2d, hist, phi, pos, PhiT):
     B, d, _, Lh = hist.shape
     L, K = phi.shape
     assert PhiT.shape == (2 * K, Lh) and PhiT.is_contiguous() and phi.is_contiguous() and x2d.stride(1) == 1
-    rc = _lib.load().stu_full_decode_prepare(x2d.data_ptr(), x2d.stride(0), hist.data_ptr(), phi.data_ptr(),
+    rc = _lib.native().stu_full_decode_prepare(x2d.data_ptr(), x2d.stride(0), hist.data_ptr(), phi.data_ptr(),
                                              pos.data_ptr(), PhiT.data_ptr(), B, d, K, L, Lh,
                                              status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
     _lib.check(rc, "stu_full_decode_prepare")
@@ -584,7 +596,7 @@ def full_decode_prepare(x2d, hist, phi, pos, PhiT):
 def full_decode_combine(G, pos, U, B: int, d: int, K: int, both_signs: bool, Lh: int, advance: bool = True):
     _cuda(G, pos, U)
     assert G.stride(1) == 1 and U.is_contiguous()
-    rc = _lib.load().stu_full_decode_combine(G.data_ptr(), G.stride(0), pos.data_ptr(), U.data_ptr(), B, d, K,
+    rc = _lib.native().stu_full_decode_combine(G.data_ptr(), G.stride(0), pos.data_ptr(), U.data_ptr(), B, d, K,
                                              int(both_signs), Lh, int(advance), _dt(G), _stream())
     _lib.check(rc, "stu_full_decode_combine")
     _count(2 if advance else 1)
@@ -595,7 +607,7 @@ def lds_final_state(hist, h, A32, B32, T: int):
     _cuda(hist, h, A32, B32)
     B, d, _, Lh = hist.shape
     assert hist.is_contiguous() and h.is_contiguous() and h.dtype == torch.float64 and A32.dtype == torch.float64
-    rc = _lib.load().stu_lds_final_state(hist.data_ptr(), h.data_ptr(), A32.data_ptr(), B32.data_ptr(), B, d, Lh, T,
+    rc = _lib.native().stu_lds_final_state(hist.data_ptr(), h.data_ptr(), A32.data_ptr(), B32.data_ptr(), B, d, Lh, T,
                                          h.shape[2], _dt(hist), _stream())
     _lib.check(rc, "stu_lds_final_state")
     _count()
@@ -613,7 +625,7 @@ def lds_chunk_scan(x, A64, B64, Vs, Z, hfin, Ck: int, unit_b: bool = False):
     assert A64.dtype == torch.float64 and Vs.dtype == torch.float64 and hfin.dtype == torch.float64
     KZ = (3 * R if x.dtype == torch.bfloat16 else R) + Ck
     assert Z.shape == (B, (T + Ck - 1) // Ck, d, KZ) and Z.dtype == x.dtype and hfin.shape == (B, d, D)
-    rc = _lib.load().stu_lds_chunk_scan(x.data_ptr(), x.stride(0), x.stride(1), A64.data_ptr(), B64.data_ptr(),
+    rc = _lib.native().stu_lds_chunk_scan(x.data_ptr(), x.stride(0), x.stride(1), A64.data_ptr(), B64.data_ptr(),
                                         Vs.data_ptr(), Z.data_ptr(), hfin.data_ptr(), B, d, T, D, R, Ck,
                                         _dt(x) | (0x1000 if unit_b else 0), _stream())
     _lib.check(rc, "stu_lds_chunk_scan")
@@ -629,7 +641,7 @@ def lds_chunk_features(W, Zb, U2, d: int, Ck: int, F: int):
     assert Mrows == Ck * F and Zb.shape[1] == KZ and W.is_contiguous() and Zb.is_contiguous() and U2.is_contiguous()
     assert N % d == 0 and U2.shape == (N // d * Ck, F * d) and U2.dtype == W.dtype == Zb.dtype
     status_word(W.device)
-    rc = _lib.load().stu_linear(W.data_ptr(), KZ, Zb.data_ptr(), KZ, 1, None, None, Ck * F * d, U2.data_ptr(), d,
+    rc = _lib.native().stu_linear(W.data_ptr(), KZ, Zb.data_ptr(), KZ, 1, None, None, Ck * F * d, U2.data_ptr(), d,
                                 Mrows, N, KZ, 5, d, 0, 0, None, 0.0, _dt(W), BACKEND_AUTO, _stream())
     _lib.check(rc, "stu_linear (LDS feature scatter)")
     _count()
@@ -642,7 +654,7 @@ def lds_decode_features(x2d, h, A32, B32, C, U):
     D, F = C.shape
     assert h.shape == (B, d, D) and h.is_contiguous() and h.dtype == torch.float64 and A32.dtype == torch.float64
     assert C.is_contiguous() and U.is_contiguous() and x2d.stride(1) == 1
-    rc = _lib.load().stu_lds_decode_features(x2d.data_ptr(), x2d.stride(0), h.data_ptr(), A32.data_ptr(), B32.data_ptr(),
+    rc = _lib.native().stu_lds_decode_features(x2d.data_ptr(), x2d.stride(0), h.data_ptr(), A32.data_ptr(), B32.data_ptr(),
                                              C.data_ptr(), U.data_ptr(), B, d, D, F, _dt(x2d), _stream())
     _lib.check(rc, "stu_lds_decode_features")
     _count()
@@ -657,7 +669,7 @@ def swa_forward(qkv, k_ring, v_ring, pos, slopes, H: int, window: int, softcap: 
     W = max(int(k_ring.shape[1]), window + 1)  # an uncached call passes a dummy ring that is never read
     assert not update_cache or (k_ring.shape == (B, W, d) and k_ring.is_contiguous() and v_ring.is_contiguous())
     out = torch.empty(B, Tn, d, dtype=qkv.dtype, device=qkv.device)
-    rc = _lib.load().stu_swa_forward(qkv.data_ptr(), k_ring.data_ptr(), v_ring.data_ptr(), pos.data_ptr(),
+    rc = _lib.native().stu_swa_forward(qkv.data_ptr(), k_ring.data_ptr(), v_ring.data_ptr(), pos.data_ptr(),
                                      slopes.data_ptr(), out.data_ptr(), B, Tn, H, d // H, W, window, float(softcap or 0.0),
                                      int(update_cache), _dt(qkv), _stream())
     _lib.check(rc, "stu_swa_forward")
@@ -698,7 +710,7 @@ def sample(logits, temperature: float, top_k: Optional[int], top_p: Optional[flo
     _cuda(logits, uniforms, out)
     B, V = logits.shape
     assert logits.stride(1) == 1 and out.dtype == torch.int64
-    rc = _lib.load().stu_sample(logits.data_ptr(), logits.stride(0), B, V, float(temperature), int(top_k or 0),
+    rc = _lib.native().stu_sample(logits.data_ptr(), logits.stride(0), B, V, float(temperature), int(top_k or 0),
                                 float(top_p if top_p is not None else -1.0), int(do_sample), _p(uniforms),
                                 out.data_ptr(), out_stride, status_word(logits.device).data_ptr(), _dt(logits),
                                 _stream())

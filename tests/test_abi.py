@@ -75,3 +75,32 @@ def test_ops_refuse_cpu_tensors():
     from flash_stu_2_b200 import ops
     with pytest.raises(RuntimeError, match="no CPU path"):
         ops.rmsnorm(torch.randn(2, 8), torch.ones(8))
+
+
+def test_extension_module_calls_the_same_functions():
+    """The entry points of the extension module return what ctypes gets, take None, addresses and keyword-free integers and
+    floats, and refuse a wrong number of arguments, values that do not convert and tensors that are not on a GPU."""
+    import torch
+    from flash_stu_2_b200 import _lib, ops
+    lib, native = _lib.load(), _lib.native()
+    assert native.stu_rmsnorm(None, None, None, 1, 8, 8, 8, 1e-6, 1, None) == lib.stu_rmsnorm(None, None, None, 1, 8, 8, 8, 1e-6, 1, None) == -5
+    assert native.stu_linear_can_fuse_norm(8, 4096, 1024, 2, True) == 1
+    a = 0x10000
+    args = (a, a, a + 2, a, 333 * 8, 8, 1, 8, 256, 168, 0, 333, None, 1, None)
+    assert native.stu_conv_prefill_approx_tc5(*args) == lib.stu_conv_prefill_approx_tc5(*args) == -3
+    with pytest.raises(TypeError, match="arguments expected"):
+        native.stu_linear_can_fuse_norm(8, 4096)
+    with pytest.raises(TypeError):
+        native.stu_linear_can_fuse_norm(8, 4096, 1024, 2, "bf16")
+    with pytest.raises(OverflowError):
+        native.stu_linear_can_fuse_norm(8, 1 << 40, 1024, 2, 1)
+    x = torch.zeros(2, 8)
+    with pytest.raises(RuntimeError, match="no CPU path"):
+        native.stu_rmsnorm(x, x, x, 2, 8, 8, 8, 1e-6, 0, None)
+    assert native.linear(x, x, None, None, None, 0, None, 1e-6, 0, False, 0, 0, 0) is None and native.rmsnorm(x, x, 1e-6) is None
+    for call in (lambda: ops.linear(x, x), lambda: ops.rmsnorm(x, x[0])):
+        with pytest.raises(RuntimeError, match="no CPU path"):
+            call()
+    exported = set(dir(native))
+    used = set(re.findall(r"_lib\.native\(\)\.(\w+)\(", open(os.path.join(ROOT, "flash_stu_2_b200", "ops.py")).read()))
+    assert used <= exported, used - exported

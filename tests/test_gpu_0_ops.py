@@ -1260,3 +1260,26 @@ def test_attention_prefill_soft_cap_small_and_large(hd, cap, gain):
     s = s.masked_fill((lag < 0) | (lag > w), float("-inf"))
     want = (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(B, T, d)
     close(y, want, 1.5e-2 if cap != 50.0 or gain < 12 else 3e-2)
+
+
+def test_linear_through_the_extension_module_checks_what_the_interpreter_checks():
+    """Shapes, strides and dtypes that the fast call does not take get the general path's answer."""
+    from flash_stu_2_b200 import ops
+    x, W = torch.randn(5, 64, device=dev()), torch.randn(32, 64, device=dev())
+    want = x @ W.t()
+    close(ops.linear(x, W), want, 1e-5)
+    close(ops.linear(x, W.t().contiguous(), transposed_weight=True), want, 1e-5)
+    close(ops.linear(torch.randn(7, 128, device=dev())[:5].copy_(torch.cat([x, x], 1))[:, 64:], W), want, 1e-5)   # rows of a wider tensor
+    buf = torch.full((5, 40), 7.0, device=dev())
+    assert ops.linear(x, W, out=buf[:, :32]).data_ptr() == buf.data_ptr() and bool((buf[:, 32:] == 7).all())
+    for bad in (lambda: ops.linear(x[:, :60], W), lambda: ops.linear(x, W, out=buf), lambda: ops.linear(x, W, W2=W[:16]),
+                lambda: ops.linear(x, W, resid=x, epilogue=ops.EPI_RESID), lambda: ops.linear(x.t(), W)):
+        with pytest.raises(AssertionError):
+            bad()
+    with pytest.raises(TypeError):
+        ops.linear(x.double(), W.double())
+    with pytest.raises(RuntimeError, match="no CPU path"):
+        ops.linear(x, W.cpu())
+    close(ops.rmsnorm(x.t(), torch.ones(5, device=dev())), O.rmsnorm(x.t().cpu(), torch.ones(5)), 1e-5)
+    with torch.inference_mode():
+        assert ops.linear(x, W).is_inference()
