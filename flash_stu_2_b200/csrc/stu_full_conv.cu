@@ -95,15 +95,18 @@ __global__ void __launch_bounds__(TX * 16, 32 / TX) full_conv_kernel(const float
       *reinterpret_cast<float4*>(xe) = *reinterpret_cast<const float4*>(&xs[buf][0][u][tx * 4]);
       *reinterpret_cast<float4*>(xo) = *reinterpret_cast<const float4*>(&xs[buf][1][u][tx * 4]);
       const float od[5] = {below, o[0], o[1], o[2], o[3]};
+      // (four in a row share the tap: its register is read once; with them interleaved a MiniSTU pass took 0.624 ms, so 0.597)
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < 4; i++) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          ee[i][j] = fmaf(t4[i], xe[j], ee[i][j]);
-          eo[i][j] = fmaf(t4[i], xo[j], eo[i][j]);
-          qo[i][j] = fmaf(od[i + 1], xe[j], qo[i][j]);
-          qe[i][j] = fmaf(od[i], xo[j], qe[i][j]);
-        }
+        for (int j = 0; j < 4; j++) ee[i][j] = fmaf(t4[i], xe[j], ee[i][j]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) eo[i][j] = fmaf(t4[i], xo[j], eo[i][j]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) qe[i][j] = fmaf(od[i], xo[j], qe[i][j]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) qo[i][j] = fmaf(od[i + 1], xe[j], qo[i][j]);
+      }
       t4[3] = t4[2]; t4[2] = t4[1]; t4[1] = t4[0]; t4[0] = te[-1 - u];
       o[3] = o[2]; o[2] = o[1]; o[1] = o[0]; o[0] = below;
     }

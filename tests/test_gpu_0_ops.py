@@ -1283,3 +1283,21 @@ def test_linear_through_the_extension_module_checks_what_the_interpreter_checks(
     close(ops.rmsnorm(x.t(), torch.ones(5, device=dev())), O.rmsnorm(x.t().cpu(), torch.ones(5)), 1e-5)
     with torch.inference_mode():
         assert ops.linear(x, W).is_inference()
+
+
+@pytest.mark.parametrize("epi", [0, 1, 2])
+@pytest.mark.parametrize("shape", [(130, 96, 72), (64, 16, 1000), (300, 33, 40), (70, 160, 3072), (1000, 32, 17)])
+def test_cuda_core_gemm_of_few_columns(shape, epi):
+    """fp32 tiles of 32 and 64 columns, ragged in every direction, K split over a cluster and not, against float64.  Bar: sums of K
+    products in fp32, each rounding at most 2^-24 of the sum of magnitudes (below 4 sqrt(K) of a result's size here)."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    torch.manual_seed(17)
+    x, W, W2, r = torch.randn(M, K), torch.randn(N, K) / math.sqrt(K), torch.randn(N, K) / math.sqrt(K), torch.randn(M, N)
+    y = ops.linear(x.to(dev()), W.to(dev()), W2=W2.to(dev()) if epi == 2 else None, resid=r.to(dev()) if epi == 1 else None,
+                   epilogue=epi, backend=1)
+    acc = x.double() @ W.double().t()
+    want = acc if epi == 0 else r.double() + acc if epi == 1 else \
+        torch.nn.functional.gelu(acc, approximate="tanh") * (x.double() @ W2.double().t())
+    close(y, want, 4 * math.sqrt(K) * 2 ** -22, row_tol=1e-4)
+    ops.check_status()
