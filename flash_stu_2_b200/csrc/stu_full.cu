@@ -1,6 +1,8 @@
 // STU spectral convolution, full variant (flash_stu/modules/stu.py:100-118; MiniSTU mini_stu/stu.py:240-269):
 //   U+-[b,t,k,i] = sum_j (+-1)^j phi[j,k] x[b,t-j,i]      (rounded to the model dtype)
 //   y[b,t,o]     = sum_{k,i} U+[b,t,k,i] M_phi_plus[k,i,o] + U-[b,t,k,i] M_phi_minus[k,i,o]
+// bf16 with channels in whole 16 bytes goes through stu_full_conv_umma.cu and stu_full_step.cu, fp32 prefills through
+// stu_full_conv.cu; this is the history's layout for all of them, and the general path of the rest.
 // Here the K filters are shared by all channels, so the convolutions are real GEMMs.  With the history of the
 // layer input kept parity-split and time-major per channel ([B][d][2][Lh], as for the approx variant):
 //   E_k[(b,i,p)][m] = sum_s phi[2(m-s),   k] * H[(b,i,p)][s]          even taps, same parity

@@ -8,8 +8,8 @@
 // four sums each: E and Q of both parities share the inputs xe[s] = x[2s], xo[s] = x[2s+1] and their taps
 //   E_even += f[2(m-s)] xe[s]   E_odd += f[2(m-s)] xo[s]   Q_odd += f[2(m-s)+1] xe[s]   Q_even += f[2(m-s)-1] xo[s].
 // A thread's taps slide by one as s advances, so a step of s costs 64 FMAs, two 16-byte reads of the inputs and two
-// words of taps.  Sums over s run in order, as the GEMMs' did.  24 filters, 8 x 1000 positions of 64 channels: 1.35 -> 0.43 ms
-// (27 TFLOP/s of the causal half).
+// words of taps.  Sums over s run in order, as the GEMMs' did.  24 filters, 8 x 1000 positions of 64 channels: 1.35 -> 0.40 ms
+// (29 TFLOP/s of the causal half).
 #include "common.cuh"
 
 namespace {
