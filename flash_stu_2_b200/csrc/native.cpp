@@ -118,6 +118,14 @@ bool plain(PyObject* o, const at::Tensor** t) {
 }
 void* data_of(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 
+// A CUDA error (rc > 0) raises as _lib.check does: the kernel may have gone out all the same (the error can be one that an earlier
+// call left behind), so the call must not be made a second time.  Refusals (rc < 0) come before any launch.
+bool raised(int rc, const char* what) {
+  if (rc <= 0) return false;
+  PyErr_Format(PyExc_RuntimeError, "%s: CUDA error %d", what, rc);
+  return true;
+}
+
 // linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed, hist_T, hist_t0, hist_Lh) -> y, or None where a check
 // fails or the library refuses: ops.linear then goes through its own checks, which raise what they raise.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -162,6 +170,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_BEGIN_ALLOW_THREADS
     rc = stu_linear(px, lda, pW, w_rs, w_ks, pW2, pr, r_rs, py, y_rs, (int)M, (int)N, (int)K, epi, hT, ht0, hLh, pn, eps, code, backend, stream);
     Py_END_ALLOW_THREADS
+    if (raised(rc, "stu_linear")) return nullptr;
     if (rc != 0) Py_RETURN_NONE;
     if (made.defined()) return THPVariable_Wrap(std::move(made));
     Py_INCREF(args[4]);
@@ -193,6 +202,7 @@ PyObject* rmsnorm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_BEGIN_ALLOW_THREADS
     rc = stu_rmsnorm(px, pw, py, (int)rows, (int)d, d, d, eps, code, stream);
     Py_END_ALLOW_THREADS
+    if (raised(rc, "stu_rmsnorm")) return nullptr;
     if (rc == 0) return THPVariable_Wrap(std::move(y));
   } catch (const BadArgument&) {
     PyErr_Clear();

@@ -1301,3 +1301,35 @@ def test_cuda_core_gemm_of_few_columns(shape, epi):
         torch.nn.functional.gelu(acc, approximate="tanh") * (x.double() @ W2.double().t())
     close(y, want, 4 * math.sqrt(K) * 2 ** -22, row_tol=1e-4)
     ops.check_status()
+
+
+def _leave_an_error_behind():
+    """A launch that the host refuses (more blocks along y than a grid has), nothing reaches the device: the error stays noted."""
+    from flash_stu_2_b200 import _lib, ops
+    t = torch.zeros(64, 8, dtype=torch.bfloat16, device=dev())
+    a = t.data_ptr()
+    assert _lib.load().stu_decode_approx(a, 8, a, a, a, a, a, a, a, 8, 1 << 20, 8, 8, 1e-6, a, 1, ops._stream()) > 0
+
+
+def test_an_error_left_behind_raises_and_a_product_in_place_is_made_at_most_once():
+    """A launch after which the library sees an error raises, even where the product itself went out; it is not made again, which
+    would add the branch to the residual twice.  The error is gone with that."""
+    from flash_stu_2_b200 import ops
+    x, W, w = torch.randn(5, 64, device=dev()), torch.randn(64, 64, device=dev()), torch.ones(64, device=dev())
+    y, branch = torch.randn(5, 64, device=dev()), x @ W.t()
+    before = y.clone()
+    for _ in range(2):   # (the first call registers the status word, the first native one loads the kernel, which clears errors)
+        ops.linear(x, W, resid=y, out=torch.empty_like(y), epilogue=ops.EPI_RESID)
+    _leave_an_error_behind()
+    with pytest.raises(RuntimeError, match="CUDA error"):
+        ops.linear(x, W, resid=y, out=y, epilogue=ops.EPI_RESID)
+    if not torch.equal(y, before):
+        close(y, before + branch, 1e-5)
+    y.copy_(before)
+    close(ops.linear(x, W, resid=y, out=y, epilogue=ops.EPI_RESID), before + branch, 1e-5)
+    ops.rmsnorm(x, w)
+    _leave_an_error_behind()
+    with pytest.raises(RuntimeError, match="CUDA error"):
+        ops.rmsnorm(x, w)
+    close(ops.rmsnorm(x, w), O.rmsnorm(x.cpu(), w.cpu()), 1e-5)
+    ops.check_status()
