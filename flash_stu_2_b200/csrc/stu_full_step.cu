@@ -52,9 +52,9 @@ __global__ void __launch_bounds__(THREADS, 2)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
   const int per_seq = (d + CH - 1) / CH, b = blockIdx.x / per_seq, i0 = (blockIdx.x - b * per_seq) * CH;
   const size_t pitch = (size_t)Lh + 8;
-  if (tid < 8 * NT) s_tap0[tid] = Elem<bf16>::to_f(taps[(size_t)min(tid, K - 1) * pitch + Lh - 1]);   // (constant over the steps)
-  pdl_wait();
+  pdl_wait();   // (the kernel in front may have just written the taps)
   pdl_trigger();
+  if (tid < 8 * NT) s_tap0[tid] = Elem<bf16>::to_f(taps[(size_t)min(tid, K - 1) * pitch + Lh - 1]);
   if (tid == 0) {
     const int t = *(volatile int*)pos;
     s_t = t;

@@ -1333,3 +1333,26 @@ def test_an_error_left_behind_raises_and_a_product_in_place_is_made_at_most_once
         ops.rmsnorm(x, w)
     close(ops.rmsnorm(x, w), O.rmsnorm(x.cpu(), w.cpu()), 1e-5)
     ops.check_status()
+
+
+def test_full_variant_step_right_behind_its_tap_table():
+    """The step is launched with the programmatic attribute: on a stream where the kernel directly in front writes the tap table,
+    what it takes of that table is the new one.  Other taps in the same buffer each time; the first position (U = x f[0]: E alone,
+    which is Q's zero added and subtracted), so that everything hangs on the tap at distance 0.  Bar: products rounded to bf16 once."""
+    from flash_stu_2_b200 import _lib, ops
+    B, d, K, Lh = 4, 256, 24, 512
+    torch.manual_seed(22)
+    x = torch.randn(B, d).bfloat16().to(dev())
+    taps = [torch.randn(2 * K, Lh).bfloat16().to(dev()) for _ in range(8)]
+    taps8 = ops.taps_rev8(taps[0])
+    hists = [torch.zeros(B, d, 2, Lh, dtype=torch.bfloat16, device=dev()) for _ in taps]
+    pos = [torch.zeros(B, 2, dtype=torch.int32, device=dev()) for _ in taps]
+    U = [torch.empty(B, 2 * K * d, dtype=torch.bfloat16, device=dev()) for _ in taps]
+    torch.cuda.synchronize()
+    for tp, h, p, u in zip(taps, hists, pos, U):
+        _lib.check(_lib.native().stu_taps_rev8(tp, taps8, 2 * K, Lh, 1, ops._stream()), "stu_taps_rev8")
+        ops.full_decode_step(x, None, 0.0, h, taps8, p, u, 2 * Lh, True)
+    ops.check_status()
+    for tp, u in zip(taps, U):
+        want = (tp[:K, 0].double()[None, :, None] * x.double()[:, None, :]).reshape(B, K * d)
+        close(u, torch.cat([want, want], 1), 2 ** -8)
