@@ -84,9 +84,16 @@ __device__ __forceinline__ float ldcg_f(const bf16* p) {
 // that it belongs to.  A reader polls the word itself: neither a fence nor a counter stands between the store and the load
 // that finds it.  bf16: 32 bits, the value above 16 bits of tag; fp32: 64 bits, the tag above the value.
 // (Every write of a word carries another tag than the write before: see tag_of in the kernel.)
+// The elements of a reader's 16-byte load are as wide as the stores: the parts of a vector access are accesses of their own, so only
+// a value and a tag of one element come from one store.
 template <typename T> struct Tagged;
 template <> struct Tagged<bf16> {
   static constexpr int BYTES = 4;
+  static __device__ __forceinline__ uint4 load(const char* p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+  }
   static __device__ __forceinline__ bool has(const uint4& w, uint32_t tag) {
     return (((w.x ^ tag) | (w.y ^ tag) | (w.z ^ tag) | (w.w ^ tag)) & 0xffffu) == 0;
   }
@@ -100,6 +107,11 @@ template <> struct Tagged<bf16> {
 };
 template <> struct Tagged<float> {
   static constexpr int BYTES = 8;
+  static __device__ __forceinline__ uint4 load(const char* p) {
+    uint64_t a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
+  }
   static __device__ __forceinline__ bool has(const uint4& w, uint32_t tag) { return w.y == tag && w.w == tag; }
   static __device__ __forceinline__ uint2 values(const uint4& w) { return make_uint2(w.x, w.z); }
   static __device__ __forceinline__ void put(char* row, int i, float v, uint32_t tag) {
@@ -107,11 +119,6 @@ template <> struct Tagged<float> {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(row + (size_t)i * 8), "l"(w) : "memory");
   }
 };
-__device__ __forceinline__ uint4 ld_tagged(const char* p) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ void unpack8(const uint2& v, float (&o)[4], bf16*) {   // the values of eight bytes
   o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
   o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
@@ -400,7 +407,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
         for (int m = 0; m < MM; m++)
 #pragma unroll
           for (int u = 0; u < VU; u++)
-            if (m < B && v0 + u * CONS < nv) w[m][u] = ld_tagged(base + (size_t)m * K * TB + (size_t)(v0 + u * CONS) * 16);
+            if (m < B && v0 + u * CONS < nv) w[m][u] = Tagged<T>::load(base + (size_t)m * K * TB + (size_t)(v0 + u * CONS) * 16);
 #pragma unroll
         for (int m = 0; m < MM; m++)
 #pragma unroll
@@ -422,7 +429,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     for (uint32_t it = 0;; ++it) {
       bool all = true;
 #pragma unroll
-      for (int i = 0; i < N; i++) w[i] = ld_tagged(p + i * 16);
+      for (int i = 0; i < N; i++) w[i] = Tagged<T>::load(p + i * 16);
 #pragma unroll
       for (int i = 0; i < N; i++) all = all && Tagged<T>::has(w[i], tag);
       if (all || give_up(it)) break;

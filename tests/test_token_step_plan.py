@@ -1,5 +1,7 @@
 """Host side of the persistent token-step kernel: its plan and the walk of its weight stream, without a GPU."""
 import ctypes
+import os
+import re
 
 import pytest
 import torch
@@ -146,3 +148,16 @@ def test_form_of_the_step_follows_what_was_measured(d, layers, heads, mlp, dt, B
 
     stack = [AttnLayer if attn and i % 2 else StuLayer for i in range(layers)]
     assert TokenStep.pays(stack, B, d, dt, t, steps) is want
+
+
+def test_tagged_words_are_read_in_elements_of_the_stores_width():
+    """A word's value and tag come from one store only if they lie in one element of the reader's vector load (a vector access is
+    as many accesses as it has elements): per type, every load of the words has elements as wide as the store."""
+    text = open(os.path.join(os.path.dirname(_lib.LIB_PATH), "csrc", "token_step.cu")).read()
+    for dt, bits in (("bf16", "32"), ("float", "64")):
+        body = text[text.index(f"struct Tagged<{dt}> {{"):]
+        body = body[:body.index("\n};")]
+        stores = re.findall(r"st\.relaxed\.gpu\.global\.[ub](\d+)", body)
+        loads = re.findall(r"ld\.relaxed\.gpu\.global\.v(\d)\.[ub](\d+)", body)
+        assert stores == [bits] and loads == [(str(128 // int(bits)), bits)], (dt, stores, loads)
+    assert len(re.findall(r"ld\.relaxed\.gpu\.global", text)) == 2   # nobody else reads them
