@@ -957,19 +957,19 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     if (kind == ST_GATE_UP && !P.tagged_h) arrive();
   }
   __syncthreads();   // with the producer
-  if (s_abort) {
-    if (tid == 0) {
-      atomicExch(epoch_word + 1, 1);
-      if (a.status) atomicExch(a.status, 12);
-    }
-  } else if (cta == 0) {   // once every CTA has read the positions and the control words (long ago, but for idle ones)
+  if (cta == 0 && !s_abort) {   // once every CTA has read the positions and the control words (long ago, but for idle ones)
     if (tid == 0) poll_count(started, G);
-    cons_bar();
-    for (int i = tid; i < a.n_layers * B; i += CONS) layers[i / B].pos[2 * (i % B)] = t + 1;
-    if (tid == 0) {
-      epoch_word[2] = P.signature;
-      *epoch_word = epoch + 1;
+    if (go_on()) {
+      for (int i = tid; i < a.n_layers * B; i += CONS) layers[i / B].pos[2 * (i % B)] = t + 1;
+      if (tid == 0) {
+        epoch_word[2] = P.signature;
+        *epoch_word = epoch + 1;
+      }
     }
+  }
+  if (tid == 0 && s_abort) {
+    atomicExch(epoch_word + 1, 1);
+    if (a.status) atomicExch(a.status, 12);
   }
 }
 

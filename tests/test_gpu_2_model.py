@@ -251,6 +251,33 @@ def test_token_step_that_gives_up_is_reported(monkeypatch):
     ops.check_status()
 
 
+def test_token_step_that_gives_up_on_its_last_wait_is_reported(monkeypatch):
+    """The count of CTAs that have started is never complete (it starts far below zero): the step computes its logits, but positions
+    and epoch do not move on past CTAs that may not have read them; status 12 and an exception as for any other wait."""
+    import time
+    from flash_stu_2_b200 import ops, token_step
+    m = _random_model(256, 4, torch.float32, layers=2)
+    prompt = torch.randint(0, 1003, (2, 30), device=dev())
+    want = m.generate(prompt, max_length=40, do_sample=False)
+    make, kept = token_step.TokenStep.__init__, []
+
+    def broken(self, *args, **kw):
+        make(self, *args, **kw)
+        kept.append(self)
+        self._ws[192:196].view(torch.int32).fill_(-1 << 20)
+
+    with monkeypatch.context() as mp:
+        mp.setattr(token_step.TokenStep, "__init__", broken)
+        torch.cuda.synchronize()
+        t = time.monotonic()
+        with pytest.raises(RuntimeError, match="device status 12"):
+            m.generate(prompt, max_length=60, do_sample=False)
+        assert time.monotonic() - t < 8
+    assert kept[0]._ws[:8].view(torch.int32).tolist() == [0, 1] and int(kept[0].pos[0][0, 0]) == 30
+    ops.check_status()
+    assert torch.equal(m.generate(prompt, max_length=40, do_sample=False), want)
+
+
 def test_token_step_kernel_with_parametrised_weights():
     """A weight that is computed at every look-up lives as long as the steps that read it."""
     from torch.nn.utils import parametrize
