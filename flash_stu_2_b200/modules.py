@@ -151,7 +151,7 @@ class STU(nn.Module):
                 self.M_phi_minus = nn.Parameter(torch.empty(self.K, self.d_in, self.d_out, dtype=dt))
         self._prep_key = None
         self._prep = None
-        self._taps_key = self._taps = None
+        self._taps_of = self._taps = None
         # optional cap on the positions a cache (and the tap tables) are laid out for: a model whose filters span
         # 32768 positions but that will only ever see 9216 keeps 9216-position histories (config.cache_len)
         self.cache_len = getattr(config, "cache_len", None)
@@ -279,15 +279,19 @@ class STU(nn.Module):
         return None
 
     def step_taps(self):
-        """[8, 2K, Lh+8]: even and odd taps of the filters as the step kernel reads them, kept per version of phi."""
+        """[8, 2K, Lh+8]: even and odd taps of the filters as the step kernel reads them, kept per version of phi and capacity.
+        (phi is kept beside them: another tensor at its address is not taken for it.)"""
         phi = param(self, "phi")
-        key = (phi._version, phi.data_ptr(), self.param_dtype)
-        if self._taps_key != key:
-            with torch.no_grad():
-                f = phi[:self.capacity].to(self.param_dtype).contiguous()
-                odd = ops.taps_even(f[1:], self.Lh) if f.shape[0] > 1 else torch.zeros_like(ops.taps_even(f, self.Lh))
-                self._taps, self._taps_key = ops.taps_rev8(torch.cat([ops.taps_even(f, self.Lh), odd])), key
-        return self._taps
+        of = (phi, phi._version, self.param_dtype, self.capacity)
+        if self._taps_of is not None and self._taps_of[0] is phi and self._taps_of[1:] == of[1:]:
+            return self._taps
+        with torch.no_grad():
+            f = phi[:self.capacity].to(self.param_dtype).contiguous()
+            odd = ops.taps_even(f[1:], self.Lh) if f.shape[0] > 1 else torch.zeros_like(ops.taps_even(f, self.Lh))
+            taps = ops.taps_rev8(torch.cat([ops.taps_even(f, self.Lh), odd]))
+        if not torch.cuda.is_current_stream_capturing():   # a table that only a graph's replay fills belongs to that graph
+            self._taps, self._taps_of = taps, of
+        return taps
 
     def full_decode_step(self, x2d: torch.Tensor, resid2d: torch.Tensor, out2d: torch.Tensor, entry, norm_w=None,
                          eps: float = ops.RMS_EPS):

@@ -312,3 +312,47 @@ def test_single_branch_approx_block_cached_steps_equal_prefill_rows(dt, tol):
     ops.check_status()
     assert int(cache[1][0, 0]) == L
     close(torch.cat(rows, 1).cpu(), want, tol)
+
+
+def _steps_of_full_block(blk, x, T1, n):
+    _, cache = blk(x[:, :T1].clone(), use_cache=True)
+    rows = []
+    for t in range(T1, T1 + n):
+        y, cache = blk(x[:, t:t + 1].clone(), past_key_value=cache, use_cache=True)
+        rows.append(y)
+    return torch.cat(rows, 1)
+
+
+def test_tap_table_of_the_full_variant_follows_the_capacity(golden):
+    """The step's tap table is laid out for the positions a cache can hold: another cap and a new cache get another table."""
+    from flash_stu_2_b200 import ops
+    r = dict(golden("blocks")["full_bfloat16"], _full=True)
+    blk, x = make_block(r, torch.bfloat16), r["x"].to(dev())
+    with torch.no_grad():
+        for cap in (None, 40, 24, None):
+            blk.layer.stu.cache_len = cap
+            close(_steps_of_full_block(blk, x, 9, 4).cpu(), r["y"][:, 9:13], 2e-2)
+            if cap is None:
+                close(_steps_of_full_block(blk, x, x.shape[1] - 3, 3).cpu(), r["y"][:, -3:], 2e-2)
+    ops.check_status()
+
+
+def test_a_captured_first_step_leaves_no_unwritten_tap_table_behind(golden):
+    """A step captured before any other has run records the building of the table, which only a replay does: an eager step after the
+    capture builds its own.  The replay then gives the next row."""
+    from flash_stu_2_b200 import ops
+    r = dict(golden("blocks")["full_bfloat16"], _full=True)
+    blk, x = make_block(r, torch.bfloat16), r["x"].to(dev())
+    T1 = 20
+    with torch.no_grad():
+        _, cache = blk(x[:, :T1].clone(), use_cache=True)
+        step, g = torch.empty_like(x[:, :1]), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g):
+            blk(step, past_key_value=cache, use_cache=True)
+        cache[1]._host_t = T1
+        y, cache = blk(x[:, T1:T1 + 1].clone(), past_key_value=cache, use_cache=True)
+        step.copy_(x[:, T1 + 1:T1 + 2])
+        g.replay()
+    ops.check_status()
+    close(torch.cat([y, step], 1).cpu(), r["y"][:, T1:T1 + 2], 2e-2)
