@@ -318,7 +318,10 @@ class FlashSTU(PreTrainedModel):
         that go with one (together 0.1 to 0.8 s on a busy process)."""
         B, d = tok.shape[0], self.config.n_embd
         row = max(3 * d, d + max(layer.mlp.intermediate_size for layer in self.layers))
-        nbytes = (B * (6 * d + 2 * row) * (self.n_layers + 1) + B * (self.lm_head.weight.shape[0] + 64)) \
+        # (full variant: U+-, the operand of the contraction with M_phi)
+        full = sum(layer.stu.K * layer.stu.d_in * (1 if layer.stu.use_hankel_L else 2) for layer in self.layers
+                   if hasattr(layer, "stu") and not layer.stu.use_approx)
+        nbytes = (B * (6 * d + 2 * row) * (self.n_layers + 1) + B * full + B * (self.lm_head.weight.shape[0] + 64)) \
             * self.lm_head.weight.element_size() + 4096 * (self.n_layers + 1)
         buffer = torch.empty(nbytes, dtype=torch.uint8, device=tok.device)
         host_t = [getattr(e[-1], "_host_t", None) if e is not None else None for e in past]

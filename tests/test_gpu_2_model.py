@@ -473,3 +473,45 @@ def test_token_steps_of_two_models_on_one_workspace(monkeypatch, dt):
             got = m.generate(prompt, max_length=40, do_sample=False, return_logits=True)
             assert torch.equal(got[0], ids) and torch.equal(got[1], logits)
     ops.check_status()
+
+
+@pytest.mark.parametrize("attn", [True, False])
+@pytest.mark.parametrize("kw", [dict(do_sample=False), dict(temperature=0.7, top_k=20)])
+def test_full_variant_bf16_generation_through_the_captured_graph(monkeypatch, attn, kw):
+    """FlashSTU(use_approx=False) in bf16: the replayed graph, which holds the one-kernel step of the full variant, draws the tokens
+    and gives the logits of the layer-by-layer loop; the logits follow those of the whole prefix.  The captured step's outputs
+    all fit the buffer that was allocated for them."""
+    import flash_stu_2_b200 as F
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(8)
+    cfg = F.FlashSTUConfig(n_embd=128, n_layers=4, n_heads=2, seq_len=256, window_size=40, vocab_size=203, mlp_scale=1,
+                           num_eigh=24, torch_dtype=torch.bfloat16, use_approx=False, use_attn=attn)
+    with torch.device(dev()):
+        m = F.FlashSTU(cfg).eval()
+    with torch.no_grad():
+        for name, p in m.named_parameters():
+            if "M_phi" in name:
+                p.normal_(0.0, 0.1 * p.shape[1] ** -0.5)
+            elif not name.endswith("norm.weight"):
+                p.normal_(0.0, 0.5 * p.shape[-1] ** -0.5)
+    prompt, u = torch.randint(0, 203, (4, 33), device=dev()), torch.rand(17, 4)
+    steps, refused = [], []
+    step, take = ops.full_decode_step, ops.arena.take
+    monkeypatch.setattr(ops, "full_decode_step", lambda *a: (steps.append(1), step(*a))[1])
+
+    def counted(self, shape, dtype):
+        piece = take(self, shape, dtype)
+        if piece is None:
+            refused.append(tuple(shape))
+        return piece
+
+    monkeypatch.setattr(ops.arena, "take", counted)
+    ids, logits = m.generate(prompt, max_length=50, uniforms=u, return_logits=True, **kw)
+    assert len(steps) == 2 * (2 if attn else 4)   # one eager step, one captured
+    assert not refused
+    eager_ids, eager_logits = m.generate(prompt, max_length=50, uniforms=u, return_logits=True, cuda_graph=False, **kw)
+    with torch.no_grad():
+        want = m(ids, use_cache=False).logits[:, 32:-1]
+    ops.check_status()
+    assert torch.equal(ids, eager_ids) and torch.equal(logits, eager_logits)
+    close(logits, want, 2e-2)
