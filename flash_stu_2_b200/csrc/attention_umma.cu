@@ -15,9 +15,9 @@
 //                    operand is a tile of V^T (keys contiguous), which a transpose kernel writes beforehand
 // Bound: the softmax, and in it the special-function unit, which takes 8 clocks a warp for every tanh and every exponential:
 // two of each score's three instruction streams waited for it.  A cap of 50 is far above the scores of a trained model, so where
-// every score of the warp's tile is below half the cap, tanh(y) = y p(y^2) with p of degree 2 (three coefficients, Chebyshev
-// interpolation on [0, 1/4], relative error 2.3e-5 against 2^-11 of the hardware's) on packed pairs; the tile goes through the
-// hardware tanh otherwise.  4 x 8192 positions of 24 heads of 128, window 2048: 1445 -> 1282 us; 4 x 1999 of 16 heads of 64,
+// every visible score of a row in the tile is below half the cap, tanh(y) = y p(y^2) with p of degree 2 (three coefficients, Chebyshev
+// interpolation on [0, 1/4], relative error 2.3e-5 against 2^-11 of the hardware's) on packed pairs; the row goes through the
+// hardware tanh otherwise.  (Masked scores, those of later keys above all, have no say in it.)  4 x 8192 positions of 24 heads of 128, window 2048: 1445 -> 1282 us; 4 x 1999 of 16 heads of 64,
 // window 512, 83 us (the mma.sync kernel 114).
 // O never leaves tensor memory until the last tile.  Warps: 0 producer (tensor copies), 1 MMA issuer, 2-5 softmax.
 // 96 KB of shared memory (head dimension 64: 57) and 256 columns of tensor memory per CTA: two CTAs share an SM, one computes its softmax
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
     const float base_i = -c2 * (float)i;
     const float k0 = softcap > 0.f ? scale / softcap : 0.f;
     const float k1 = softcap > 0.f ? softcap * LOG2E : scale * LOG2E;
-    // tanh(s k0) k1 = s (cap0 + cap1 s^2 + cap2 s^4) while s^2 <= most_small
+    // tanh(s k0) k1 = s (cap0 + cap1 s^2 + cap2 s^4) while s^2 < most_small
     const float kk = k0 * k0, a0 = k0 * k1 * T0, a1 = k0 * k1 * kk * T1, a2 = k0 * k1 * kk * kk * T2;
     const f32x2 cap0 = pair_of(a0, a0), cap1 = pair_of(a1, a1), cap2 = pair_of(a2, a2);
     const float most_small = 0.25f / kk;
@@ -310,7 +310,14 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
       float mx = -INFINITY;
       if (softcap > 0.f) {
         const f32x2 cc = pair_of(c2, c2), bt = pair_of(base_t, base_t);
-        float most = 0.f;   // the largest square
+        if (!interior) {   // a masked score decides nothing
+#pragma unroll
+          for (int c = 0; c < 64; c++) {
+            const int j = jt + c;
+            if (!((j <= i) && (j >= i - window) && (i <= i_last))) sr[c] = 0;
+          }
+        }
+        float most = 0.f;   // the largest square of the row (a NaN score is not in it: both forms carry it on)
 #pragma unroll
         for (int c = 0; c < 64; c += 2) {
           const f32x2 sv = pair_of(sr[c], sr[c + 1]), t2 = mul2(sv, sv);
@@ -321,15 +328,19 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
           sr[c] = __float_as_uint(s0);
           sr[c + 1] = __float_as_uint(s1);
         }
-        if (__any_sync(0xffffffffu, !(most <= most_small))) {   // (NaN included)
-          tmem_ld32(tm_s + lane_base + (t & 1) * BN, sr);
-          tmem_ld32(tm_s + lane_base + (t & 1) * BN + 32, sr + 32);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const bool large = !(most < most_small);   // (a row's own scores decide for it)
+        if (__any_sync(0xffffffffu, large)) {
 #pragma unroll
-          for (int c = 0; c < 64; c++) {
-            float th;   // hardware tanh: relative error 2^-11, below the bf16 rounding of P
-            asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(__uint_as_float(sr[c]) * k0));
-            sr[c] = __float_as_uint(fmaf(th, k1, fmaf(c2, (float)c, base_t)));
+          for (int h = 0; h < 2; h++) {
+            uint32_t raw[32];
+            tmem_ld32(tm_s + lane_base + (t & 1) * BN + h * 32, raw);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 32; c++) {
+              float th;   // hardware tanh: relative error 2^-11, below the bf16 rounding of P
+              asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(__uint_as_float(raw[c]) * k0));
+              if (large) sr[h * 32 + c] = __float_as_uint(fmaf(th, k1, fmaf(c2, (float)(h * 32 + c), base_t)));
+            }
           }
         }
       } else {

@@ -1356,3 +1356,22 @@ def test_full_variant_step_right_behind_its_tap_table():
     for tp, u in zip(taps, U):
         want = (tp[:K, 0].double()[None, :, None] * x.double()[:, None, :]).reshape(B, K * d)
         close(u, torch.cat([want, want], 1), 2 ** -8)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_prefill_rows_do_not_depend_on_later_tokens(hd):
+    """What follows a position changes no bit of its output, also where the later keys' scores lie beyond the soft cap (which takes
+    another tanh) in the tile that the position's own keys are in.  (Rows of one warp share a reference maximum: whole warps
+    of 32 positions in front of the change are compared.)"""
+    from flash_stu_2_b200 import ops
+    B, T, H, w = 1, 200, 2, 300
+    torch.manual_seed(23)
+    qkv = torch.randn(B, T, 3 * H * hd)
+    loud = qkv.clone()
+    loud[:, 97:] *= 40.0
+    slopes = O.alibi_slopes(H).float().to(dev())
+    dummy = torch.zeros(1, 1, 1, dtype=torch.bfloat16, device=dev())
+    a, b = [ops.swa_prefill_tc5(x.bfloat16().to(dev()), dummy, dummy, torch.zeros(B, 2, dtype=torch.int32, device=dev()), slopes, H, w,
+                                50.0, update_cache=False) for x in (qkv, loud)]
+    ops.check_status()
+    assert torch.equal(a[:, :96], b[:, :96]) and not torch.equal(a[:, 97:], b[:, 97:])
