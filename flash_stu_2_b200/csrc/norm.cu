@@ -104,8 +104,12 @@ static int launch_rmsnorm(const void* x, const void* w, void* y, int rows, int d
   bool vec = (d % V == 0) && (xs % V == 0) && (ys % V == 0) && aligned16(x) && aligned16(w) && aligned16(y);
   cudaError_t e;
   const int nv = (d + 32 * V - 1) / (32 * V);
-  // a warp per row from two rows per SM's warp on (fewer: a CTA per row is the shorter chain), rows of up to 12 vectors per lane
-  if (vec && nv <= 12 && rows >= 148 * 2 * NORM_WARPS) {
+  // A warp per row where the rows fill the SMs' warps often enough that its longer chain per row does not show: two rounds of 8
+  // warps per SM for rows of one or two vectors per lane, more for longer rows (fewer: a CTA per row is the shorter chain).  CTA and
+  // warp per row, us, bf16 (fp32 alike): 2368 x 512 2.9 and 2.0; 2368 x 1024 3.0 and 3.5, 4096 x 1024 4.8 and 3.8; 4096 x 2048 6.5 and
+  // 7.3, 6000 x 2048 8.4 and 7.9; 3000 x 3072 6.4 and 9.2, 8192 x 3072 15.4 and 17.3, 16384 x 3072 34.8 and 34.1.
+  const int rounds = nv <= 2 ? 2 : d <= 1024 ? 3 : d <= 2048 ? 5 : 10;
+  if (vec && nv <= 12 && rows >= 148 * NORM_WARPS * rounds) {
     const int ctas = (rows + NORM_WARPS - 1) / NORM_WARPS;
 #define STU_NORM_ROWS(NV_)                                                                                                 \
   e = launch_maybe_overlapped(rmsnorm_rows_kernel<T, NV_>, dim3(ctas), dim3(NORM_WARPS * 32), 0, st, true, (const T*)x,    \

@@ -1375,3 +1375,16 @@ def test_attention_prefill_rows_do_not_depend_on_later_tokens(hd):
                                 50.0, update_cache=False) for x in (qkv, loud)]
     ops.check_status()
     assert torch.equal(a[:, :96], b[:, :96]) and not torch.equal(a[:, 97:], b[:, 97:])
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d", [(2367, 256), (2368, 256), (2369, 512), (3551, 1000), (3552, 1000), (3555, 1024), (3552, 776), (5919, 1536),
+                                    (5920, 1536), (5921, 2048), (11839, 2056), (11840, 2056), (11841, 3072)])
+def test_rmsnorm_of_many_rows_on_both_sides_of_its_lines(dt, rows, d):
+    """Rows per warp and rows per CTA, in front of and behind the line of each width: a row's bits are those of a call of few rows."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(24)
+    x, w = (torch.randn(rows, d, device=dev()) * 3).to(dt), torch.randn(d, device=dev()).to(dt)
+    y = ops.rmsnorm(x, w)
+    assert torch.equal(y[-300:], ops.rmsnorm(x[-300:].contiguous(), w)) and torch.equal(y[:300], ops.rmsnorm(x[:300].contiguous(), w))
+    close(y[::97].cpu(), O.rmsnorm(x[::97].cpu(), w.cpu()), 1e-6 if dt == torch.float32 else 2 ** -7)
