@@ -5,6 +5,7 @@ Every .cu file is compiled to an object of its own (in parallel, re-used while t
 are older than it) and the objects are linked into the shared library; no device symbol crosses a file boundary,
 so no relocatable device code is needed."""
 import glob
+import importlib.util
 import os
 import subprocess
 import sysconfig
@@ -38,17 +39,22 @@ def native_stale() -> bool:
     if not os.path.exists(NATIVE):
         return True
     t = os.path.getmtime(NATIVE)
-    return any(os.path.getmtime(p) > t for p in [NATIVE_SRC] + glob.glob(os.path.join(HERE, "..", "include", "*.h")))
+    # (torch's own classes are on its boundary: another torch than the one that it was built for needs another)
+    torch_version = os.path.join(os.path.dirname(importlib.util.find_spec("torch").origin), "version.py")
+    return any(os.path.getmtime(p) > t for p in [NATIVE_SRC, torch_version] + glob.glob(os.path.join(HERE, "..", "include", "*.h")))
 
 
 def build_native() -> str:
     import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
-           f"-I{cuda}/include", "-o", NATIVE, NATIVE_SRC, f"-L{HERE}", "-l:libstu_b200.so", f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
-           "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    others = [f"{root}/include", f"{root}/include/torch/csrc/api/include", sysconfig.get_paths()["include"], f"{cuda}/include"]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wextra",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for path in others:   # (their warnings are not ours)
+        cmd += ["-isystem", path]
+    cmd += ["-o", NATIVE, NATIVE_SRC, f"-L{HERE}", "-l:libstu_b200.so", f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+            "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("the host compiler failed on native.cpp:\n" + res.stdout + res.stderr)

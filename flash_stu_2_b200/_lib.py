@@ -20,6 +20,9 @@ ERRORS = {
     -7: "the call needs more scratch than the library's built-in 32 MiB array",
 }
 
+MISSING = ("{} is missing and could not be built: the flash_stu_2_b200 ops have no CPU fallback; "
+           "run `python -c 'import __graft_entry__ as g; g.build()'` on a machine with nvcc")
+
 _lib = None
 
 _P = c_void_p
@@ -132,9 +135,7 @@ def load(build_if_missing: bool = True):
             if os.path.exists(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")):
                 _build.build_library()
     if not os.path.exists(LIB_PATH):
-        raise RuntimeError(
-            f"{LIB_PATH} is missing and could not be built: the flash_stu_2_b200 ops have no CPU fallback; "
-            "run `python -c 'import __graft_entry__ as g; g.build()'` on a machine with nvcc")
+        raise RuntimeError(MISSING.format(LIB_PATH))
     lib = ctypes.CDLL(LIB_PATH)
     for name, (argtypes, restype) in _SIGNATURES.items():
         fn = getattr(lib, name)
@@ -152,7 +153,10 @@ def native():
     global _native
     if _native is None:
         load()
-        from . import _native as module
+        try:
+            from . import _native as module
+        except ImportError as e:   # built on a machine with another interpreter or torch, or not at all
+            raise RuntimeError(MISSING.format(os.path.join(HERE, "_native")) + f" ({e})") from e
         _native = module
     return _native
 

@@ -104,3 +104,28 @@ def test_extension_module_calls_the_same_functions():
     exported = set(dir(native))
     used = set(re.findall(r"_lib\.native\(\)\.(\w+)\(", open(os.path.join(ROOT, "flash_stu_2_b200", "ops.py")).read()))
     assert used <= exported, used - exported
+
+
+def test_a_missing_extension_module_is_reported_like_a_missing_library(monkeypatch):
+    import sys
+    import flash_stu_2_b200
+    from flash_stu_2_b200 import _lib
+    _lib.native()
+    monkeypatch.setattr(_lib, "_native", None)
+    monkeypatch.delattr(flash_stu_2_b200, "_native", raising=False)
+    monkeypatch.setitem(sys.modules, "flash_stu_2_b200._native", None)   # its import fails
+    with pytest.raises(RuntimeError, match="no CPU fallback; run"):
+        _lib.native()
+
+
+def test_the_extension_module_is_stale_for_another_torch(monkeypatch):
+    """A torch installed after the module was built: it is built again."""
+    from flash_stu_2_b200 import _build, _lib
+    _lib.native()
+    assert not _build.native_stale()
+    import torch
+    real = os.path.getmtime
+    version = os.path.join(os.path.dirname(torch.__file__), "version.py")
+    assert os.path.exists(version)
+    monkeypatch.setattr(_build.os.path, "getmtime", lambda p: real(p) + (1e9 if os.path.samefile(p, version) else 0))
+    assert _build.native_stale()
