@@ -35,11 +35,40 @@ template <typename T> __device__ __forceinline__ float scaled_logit(const T* row
   return fminf(fmaxf(z, -1e4f), 1e4f);
 }
 
-// Sorts the n <= SP_T first entries, whole CTA; before(a, b): a ranks before b.  Every entry counts those in front of it (the
-// reads are broadcasts): two barriers, where a bitonic network of 128 entries has 28.  With the running sums read eight
-// ahead, and two radix passes in place of four for bf16 logits: one row of 50257 entries, top-k 100, top-p 0.9, 27 -> 17 us.
+// Sorts the n <= SP_T first entries, whole CTA; before(a, b): a ranks before b.  Up to SP_RANK of them every entry counts those
+// in front of it (the reads are broadcasts): two barriers, where a bitonic network of 128 entries has 28.  With the running sums
+// read eight ahead, and two radix passes in place of four for bf16 logits: one row of 50257 entries, top-k 100, top-p 0.9, 27 ->
+// 17 us.  The counts grow with the square: from there on the network, whose padding ranks last.  Counts and network, us, one row
+// of 50257, top-p 0.9: top-k 257 77 and 80, 400 87 and 84, 513 98 and 95, 700 110 and 100, 1000 134 and 107; without a nucleus
+// (one sort) 400 75 and 76, 700 96 and 91.
+constexpr int SP_RANK = 512;
 template <typename F> __device__ __forceinline__ void sort_candidates(float* s_val, int* s_idx, int n, F before) {
   const int tid = threadIdx.x;
+  if (n > SP_RANK) {
+    int width = 2 * SP_RANK;   // (a power of two)
+    while (width < n) width <<= 1;
+    if (tid >= n && tid < width) {
+      s_val[tid] = -INFINITY;
+      s_idx[tid] = 0x7fffffff;
+    }
+    __syncthreads();
+    for (int k = 2; k <= width; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        const int other = tid ^ j;
+        if (other > tid && other < width) {
+          const float va = s_val[tid], vb = s_val[other];
+          const int ia = s_idx[tid], ib = s_idx[other];
+          if (((tid & k) == 0) != before(va, ia, vb, ib)) {
+            s_val[tid] = vb;
+            s_val[other] = va;
+            s_idx[tid] = ib;
+            s_idx[other] = ia;
+          }
+        }
+        __syncthreads();
+      }
+    return;
+  }
   float v = 0.f;
   int id = 0, rank = 0;
   if (tid < n) {

@@ -1388,3 +1388,35 @@ def test_rmsnorm_of_many_rows_on_both_sides_of_its_lines(dt, rows, d):
     y = ops.rmsnorm(x, w)
     assert torch.equal(y[-300:], ops.rmsnorm(x[-300:].contiguous(), w)) and torch.equal(y[:300], ops.rmsnorm(x[:300].contiguous(), w))
     close(y[::97].cpu(), O.rmsnorm(x[::97].cpu(), w.cpu()), 1e-6 if dt == torch.float32 else 2 ** -7)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("k", [3, 255, 256, 257, 511, 512, 513, 700, 1000, 1024])
+@pytest.mark.parametrize("nucleus", [None, 0.3, 0.97])
+def test_draws_among_few_and_many_survivors(dt, k, nucleus):
+    """Top-k of up to 1024 entries, ties among them in bf16, with and without a nucleus: both sorts of the survivors.  Uniforms in the
+    middle of an entry's share of the running sum, a nucleus that ends in the middle of one: the entry itself is drawn
+    (shares of 10^-4 and more, fp32 sums of at most 1024 terms are off by less than 10^-5)."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(k)
+    z = (0.7 * torch.randn(3001)).to(dt)
+    if dt == torch.bfloat16:   # ties at the k-th place would add survivors: push what ties with it from outside below
+        first = torch.argsort(z.float(), descending=True, stable=True)
+        z[first[k:]] -= 1.0
+    w = z.double()
+    kept = (w >= torch.topk(w, k)[0][-1]).nonzero()[:, 0]
+    assert len(kept) == k
+    top_p = None
+    if nucleus is not None:
+        order = kept[torch.argsort(w[kept], descending=True, stable=True)]
+        share = torch.softmax(w[order], 0)
+        last = min(int((share.cumsum(0) < nucleus).sum()), k - 2)
+        top_p = float(share[:last].sum() + share[last] / 2)       # the mass in front of entry last + 1 is beyond it
+        kept = order[:last + 1].sort()[0]
+    share = torch.softmax(w[kept], 0)
+    picks = torch.randint(0, len(kept), (16,))
+    u = (share.cumsum(0) - share / 2)[picks].float()
+    out = torch.full((16,), -1, dtype=torch.int64, device=dev())
+    ops.sample(z.to(dev()).repeat(16, 1), 1.0, k, top_p, True, u.to(dev()), out)
+    ops.check_status()
+    assert torch.equal(out.cpu(), kept[picks])
