@@ -677,12 +677,23 @@ def swa_forward(qkv, k_ring, v_ring, pos, slopes, H: int, window: int, softcap: 
     return out
 
 
-swa_tc5 = True   # switch: prefills from position 0 with head dimension 128 (bf16) use the tcgen05 attention kernel
+swa_tc5 = True   # switch: prefills from position 0 with head dimension 64 or 128 (bf16) use the tcgen05 attention kernel
 
 
-def swa_prefill_tc5_supported(qkv, H: int, t0: int) -> bool:
-    d = qkv.shape[2] // 3
-    return swa_tc5 and qkv.dtype == torch.bfloat16 and d // H in (64, 128) and t0 == 0 and qkv.shape[1] >= 128
+def swa_prefill_tc5_supported(qkv, H: int, t0: int, window: int = 1 << 30) -> bool:
+    """Whether a prefill's attention runs on the tcgen05 kernel.  Heads of 64 have half the work per query, beside which the second
+    launch (the transpose of V), half as many CTAs and the keys that its wider tiles mask count: from 384 positions and keys on and
+    where the mma.sync kernel's CTAs of 64 queries are more than the SMs, shorter windows only with several CTAs per SM.  us,
+    tcgen05 and mma.sync: window 500, 1 sequence of 8 heads, 128 positions 12.3 and 10.1, 1024 26.3 and 21.8, 1536 26.8 and 27.1; 4 of
+    16 heads, 320 positions 23.6 and 20.9, 384 24.2 and 26.4, 2048 100 and 121; window 256, 4 of 16 heads, 768 positions 37.6 and 35.9,
+    2048 72 and 75; window 128, 2048 positions 59 and 51."""
+    B, Tn, d3 = qkv.shape
+    hd = d3 // 3 // H
+    if not (swa_tc5 and qkv.dtype == torch.bfloat16 and t0 == 0):
+        return False
+    if hd == 128:
+        return Tn >= 128
+    return hd == 64 and Tn >= 384 and window >= 256 and B * H * Tn >= (12288 if window >= 384 else 57344)
 
 
 def swa_prefill_tc5(qkv, k_ring, v_ring, pos, slopes, H: int, window: int, softcap: float, update_cache: bool):

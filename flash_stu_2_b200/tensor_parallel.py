@@ -221,7 +221,7 @@ class TensorParallelFlashSTU:
                 t0 = host_pos(pos)
                 xn = ops.rmsnorm(x2, self.sd[p + "attn_norm.weight"], self.eps)
                 qkv = ops.linear(xn, self.sd[p + "attn.c_attn.weight"]).view(B, T, 3 * dl)
-                attend = ops.swa_prefill_tc5 if ops.swa_prefill_tc5_supported(qkv, self.Hl, t0) else ops.swa_forward
+                attend = ops.swa_prefill_tc5 if ops.swa_prefill_tc5_supported(qkv, self.Hl, t0, self.window) else ops.swa_forward
                 y = attend(qkv, k_ring, v_ring, pos, self.slopes, self.Hl, self.window, self.cfg.softcap,
                            update_cache=True)
                 pos._host_t = t0 + T

@@ -1420,3 +1420,22 @@ def test_draws_among_few_and_many_survivors(dt, k, nucleus):
     ops.sample(z.to(dev()).repeat(16, 1), 1.0, k, top_p, True, u.to(dev()), out)
     ops.check_status()
     assert torch.equal(out.cpu(), kept[picks])
+
+
+@pytest.mark.parametrize("T", [128, 129, 383, 384, 385])
+@pytest.mark.parametrize("w", [100, 300, 700])
+def test_heads_of_64_on_both_attention_kernels(T, w):
+    """Around the line between the two prefill kernels for heads of 64: outputs, rings and positions of either agree.  Bar: P and the
+    output are rounded to bf16 in both, the hardware tanh and the polynomial are within 2^-11 of the function."""
+    from flash_stu_2_b200 import ops
+    B, H = 2, 3
+    torch.manual_seed(25)
+    qkv = torch.randn(B, T, 3 * H * 64).bfloat16().to(dev())
+    slopes = O.alibi_slopes(H).float().to(dev())
+    rings = [torch.zeros(2, B, w + 1, H * 64, dtype=torch.bfloat16, device=dev()) for _ in range(2)]
+    pos = [torch.zeros(B, 2, dtype=torch.int32, device=dev()) for _ in range(2)]
+    a, b = [f(qkv, r[0], r[1], p, slopes, H, w, 50.0, update_cache=True)
+            for f, r, p in zip((ops.swa_prefill_tc5, ops.swa_forward), rings, pos)]
+    ops.check_status()
+    close(a, b, 1.5e-2)
+    assert torch.equal(rings[0], rings[1]) and torch.equal(pos[0], pos[1]) and pos[0][:, 0].tolist() == [T] * B

@@ -174,3 +174,15 @@ def test_captures_of_two_threads_hold_the_collector_until_the_last_is_done():
         assert not gc.isenabled()
     finally:
         gc.enable()
+
+
+@pytest.mark.parametrize("hd,B,H,T,window,t0,takes", [
+    (128, 1, 1, 128, 16, 0, True), (128, 1, 1, 127, 16, 0, False), (128, 4, 8, 500, 500, 1, False),          # as heads of 128 were
+    (64, 4, 16, 384, 500, 0, True), (64, 4, 16, 383, 500, 0, False), (64, 1, 12, 1024, 1024, 0, True), (64, 1, 12, 1023, 1024, 0, False),
+    (64, 4, 16, 1999, 512, 0, True), (64, 4, 16, 800, 300, 0, False), (64, 4, 16, 896, 300, 0, True), (64, 4, 16, 4000, 200, 0, False),
+    (64, 4, 16, 1999, 512, 7, False), (32, 4, 16, 1999, 512, 0, False), (96, 4, 16, 1999, 512, 0, False)])
+def test_which_attention_kernel_takes_a_prefill(hd, B, H, T, window, t0, takes):
+    from flash_stu_2_b200 import ops
+    qkv = torch.empty(B, T, 3 * H * hd, dtype=torch.bfloat16, device="meta")
+    assert ops.swa_prefill_tc5_supported(qkv, H, t0, window) is takes
+    assert not ops.swa_prefill_tc5_supported(qkv.float(), H, t0, window)
