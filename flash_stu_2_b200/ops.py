@@ -567,6 +567,16 @@ def full_decode_step_supported(x2d, hist, K: int) -> bool:
             and x2d.data_ptr() % 16 == 0 and x2d.stride(0) % 8 == 0)
 
 
+def full_decode_step_pays(batch: int, d: int, K: int, t: int) -> bool:
+    """Whether the one-kernel step takes less time at position t than tap matrices, a GEMM over all history rows and a combine.  It
+    saves five launches and the tap matrices, but reads the taps in every CTA, on mma.sync: rows, filters and positions tell, and
+    with more sequences the rest of the step gains less from the launches that are saved (the lines are fits).  Layer step of 24 filters, us, replayed from a graph: 8 x 1024 at 1000 47.5 and 54.1, at 7000 72 and 76; 16 x 1024 at 1000 64 and 68,
+    at 2000 77 and 74, at 7000 136 and 102; 32 x 512 at 1000 50.5 and 50.3, at 2800 77 and 62; 32 x 1536 at 60 104 and 98, at 2800
+    214 and 144; 32 filters, 16 x 1024 at 60 70 and 70, at 2800 98 and 87."""
+    tiles = (K + 7) // 8
+    return batch * d * tiles <= 49152 and (batch * tiles) ** 2 * d * t <= 3.8e9
+
+
 def full_decode_step(x2d, norm_w, eps: float, hist, taps8, pos, U, limit: int, both_signs: bool):
     """U+- [B, (1 or 2)*K*d] of the position after the cached ones: x2d [B,d] (normalised first with norm_w) is appended to
     hist [B,d,2,Lh], taps8 [8, 2K, Lh+8] holds the even and the odd taps of the filters; pos moves on."""

@@ -356,3 +356,19 @@ def test_a_captured_first_step_leaves_no_unwritten_tap_table_behind(golden):
         g.replay()
     ops.check_status()
     close(torch.cat([y, step], 1).cpu(), r["y"][:, T1:T1 + 2], 2e-2)
+
+
+def test_full_variant_steps_change_their_form_on_one_cache(golden, monkeypatch):
+    """The two forms of the full variant's bf16 step work on the same cache: rows from a stream that changes between them at every
+    position are the reference's."""
+    from flash_stu_2_b200 import ops
+    r = dict(golden("blocks")["full_bfloat16"], _full=True)
+    blk, x = make_block(r, torch.bfloat16), r["x"].to(dev())
+    steps, step = [], ops.full_decode_step
+    monkeypatch.setattr(ops, "full_decode_step", lambda *a: (steps.append(1), step(*a))[1])
+    for odd in (0, 1):
+        monkeypatch.setattr(ops, "full_decode_step_pays", lambda B, d, K, t: t % 2 == odd)
+        with torch.no_grad():
+            close(_steps_of_full_block(blk, x, 100, 28).cpu(), r["y"][:, 100:], 2e-2)
+    ops.check_status()
+    assert len(steps) == 28

@@ -186,3 +186,11 @@ def test_which_attention_kernel_takes_a_prefill(hd, B, H, T, window, t0, takes):
     qkv = torch.empty(B, T, 3 * H * hd, dtype=torch.bfloat16, device="meta")
     assert ops.swa_prefill_tc5_supported(qkv, H, t0, window) is takes
     assert not ops.swa_prefill_tc5_supported(qkv.float(), H, t0, window)
+
+
+@pytest.mark.parametrize("batch,d,K,t,pays", [(1, 512, 24, 7000, True), (8, 1024, 24, 3000, True), (8, 1024, 24, 7000, False), (16, 1024, 24, 1000, True),
+                                             (16, 1024, 24, 2000, False), (16, 1024, 16, 4000, False), (16, 1024, 16, 2000, True), (32, 1536, 24, 0, False),
+                                             (16, 1024, 32, 0, False), (12, 1024, 32, 0, True)])
+def test_which_form_the_full_variants_step_takes(batch, d, K, t, pays):
+    from flash_stu_2_b200 import ops
+    assert ops.full_decode_step_pays(batch, d, K, t) is pays
