@@ -12,7 +12,7 @@
 // No Toeplitz matrix is materialised: in the un-swizzled K-major operand layout a 128 x 64 block is a grid of 8 x 8
 // core matrices, and with the row groups in descending order core matrix (q', kc) depends on q' + kc alone.  A table of
 // core matrices CM[X][r][w] = f[dist + 120 - 8 X + r - w] per filter and tap set (26 KB for 3000 positions) therefore holds
-// every block, and a stage of 64 columns brings 31 consecutive entries of it where a block would be 16 KB.
+// every block, and a stage of 64 columns brings 23 consecutive entries of it (3 KB) where a block would be 16 KB.
 //
 // Bound: the tensor pipe (2 * 2 S^2/2 multiply-adds per channel pair and filter) beside the 2 K d values written per
 // token.  E stays in registers, as the bf16 values it is rounded to, while Q is accumulated in the other half of tensor
@@ -370,12 +370,13 @@ extern "C" int stu_full_conv_tc5(const void* hist, int Lh, const void* phi, int 
   g.mb_first = (t0 >> 1) / BM;
   g.entries = table_entries(g.nb);
   const int sms = device_sm_count();
-  // the widest tile that leaves every SM two of them: a narrower one reads its table block for fewer channels
-  auto count = [&](int tn) { return (long long)(g.nb - g.mb_first) * ((rows + tn - 1) / tn) * 2 * K; };
+  // The widest tile that the rows fill more than half of: a narrower one reads its table block for fewer channels, which shows even
+  // where wide ones leave SMs idle.  us, tiles of 64, 128 and 256 channels, 24 filters: 1 x 512 of 100 positions 12.8, 11.5 and
+  // 11.4, of 700 33.6, 24.2 and 21.0; 4 x 1024 of 1500 626, 362 and 286; 8 x 1024 of 3000 4159, 2395 and 1886.
   g.tn = 256;
-  while (g.tn > 64 && (rows <= g.tn / 2 || count(g.tn) < 2 * sms)) g.tn /= 2;
+  while (g.tn > 64 && rows <= g.tn / 2) g.tn /= 2;
   g.n_ct = (int)((rows + g.tn - 1) / g.tn);
-  const long long tiles = count(g.tn);
+  const long long tiles = (long long)(g.nb - g.mb_first) * g.n_ct * 2 * K;
   if (tiles > 0x7fffffffll || (long long)g.entries * 8 * K > 0x7fffffffll) return STU_ERR_UNSUPPORTED;
   CUtensorMap tmH;
   {

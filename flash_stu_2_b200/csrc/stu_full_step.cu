@@ -220,7 +220,9 @@ extern "C" int stu_full_decode_step(const void* x, long long x_rstride, const vo
   if (norm_w && (d % 8 || x_rstride % 8 || !aligned16(x))) return STU_ERR_ALIGN;
   const bf16 *xp = (const bf16*)x, *np = (const bf16*)norm_w, *tp = (const bf16*)taps8;
   cudaStream_t st = (cudaStream_t)stream;
-  // 32 channels per CTA (the taps are read half as often) while that leaves no SM without one and the sums fit the registers
+  // 32 channels per CTA (the taps are read half as often) while that leaves no SM without one and the sums fit the registers.  us,
+  // 32 and 16 channels, 24 filters, position 1000: 192 CTAs of 32 (4 x 1536) 10.1 and 13.1, 128 (4 x 1024) 8.5 and 7.7; position
+  // 3000: 256 (8 x 1024) 16.3 and 20.4, 384 (12 x 1024) 32.0 and 32.2.
   const bool wide = (long long)B * ((d + 31) / 32) >= device_sm_count();
 #define STU_STEP(NT_, MT_) \
   return launch_step<NT_, MT_>(xp, x_rstride, np, eps, (bf16*)hist, tp, pos, (bf16*)U, B, d, K, Lh, limit, both_signs, status, st)

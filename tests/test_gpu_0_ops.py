@@ -1439,3 +1439,10 @@ def test_heads_of_64_on_both_attention_kernels(T, w):
     ops.check_status()
     close(a, b, 1.5e-2)
     assert torch.equal(rings[0], rings[1]) and torch.equal(pos[0], pos[1]) and pos[0][:, 0].tolist() == [T] * B
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 64, 300, 0, 300), (1, 3, 72, 300, 10, 299), (1, 2, 128, 130, 0, 129), (1, 2, 136, 90, 0, 90), (3, 2, 88, 700, 300, 700)])
+def test_full_convolution_tiles_of_64_128_and_256_channels(shape):
+    """Rows on both sides of half a tile (64, 72; 128, 136), and a last tile of 8 rows, few tiles for the SMs: the bars of the test of
+    the operand."""
+    test_full_convolution_on_tensor_cores(shape, True)
