@@ -17,7 +17,9 @@
 //   hand-over    results travel as tagged words (below), which the readers poll: a grid barrier waits for the stores, for an
 //                atomic to arrive and for another read to see it before the first row can be read.  That model, 1 sequence: 771
 //                -> 683 us a step; 12 fp32 layers of 512, 2 sequences: 352 -> 311.  Barriers are left where the words would be
-//                read by everybody in bulk: the attention's partial sums, and the rows of wide down projections
+//                read by everybody in bulk: the attention's partial sums, and rows of many bytes (TAGGED_X_BYTES).  With them and
+//                rows in fours, 5 to 8 sequences of 1536, 6 layers, take 281 to 296 us (339 to 359 with words alone, 268 to 278
+//                with barriers alone, in less code)
 //   STU          a CTA's channels are projected, appended to the history and combined with their tap sums in place;
 //                the tap sums over the cached history need nothing of this step and are taken ahead of the wait
 //   attention    (sequence, head, key range) items over the CTAs; the ranges are merged by the readers
@@ -44,10 +46,15 @@ constexpr int RED_BYTES = TILES * NW * 128 * 4;
 constexpr uint32_t COPY = 4096;                // bytes of one bulk copy at most
 constexpr int UNITS = 32;                     // row groups in flight
 constexpr int MAX_ROWS = 32;                  // STU channels per CTA
-// Rows of the down projection are handed over as tagged words up to this size (every CTA reads all of them: twice the bytes of a
-// barrier's plain values).  2 fp32 rows of 6144, 98 KB: 12 layers 311 us a step, with the barrier 317; 1 bf16 row of 6144: a tie.
-constexpr long long TAGGED_H_BYTES = 100 * 1024;
-constexpr int NORM_VECS = 2;                  // rows behind a norm: d <= 2 * 256 vectors
+// Rows are handed over as tagged words up to these sizes, by a barrier and as plain values above (every CTA reads all of a product's
+// rows: twice the bytes).  us a step, tagged and plain.  The residual stream, 32 KB: 24 KB (bf16, 4 rows of 1536, 6 layers) 233 and
+// 239, 32 KB (fp32, 4 rows of 1024, 6 layers) 234 and 243, (bf16, 8 of 1024, 10 layers) 365 and 376, 48 KB (8 of 1536) 299 and 297,
+// (fp32, 8 of 768, 10 layers) 455 and 447.  The rows of the down projection, 100 KB for one and two sequences, half of that for
+// more: 48 KB (bf16, 4 of 3072, 18 layers) 405 and 417, 96 KB (fp32, 2 of 6144, 8 layers) 207 and 210, (bf16, 4 of 6144, 6 layers)
+// 239 and 234, (fp32, 4 of 3072, 10 layers) 312 and 296, 128 KB (fp32, 4 of 4096, 6 layers) 249 and 243, 192 KB (bf16, 8 of 6144) 314
+// and 295.
+constexpr long long TAGGED_X_BYTES = 32 * 1024, TAGGED_H_BYTES = 100 * 1024;
+constexpr int MAX_VECS = 2 * CONS;            // 16-byte vectors of a row of the residual stream at most
 
 __device__ __forceinline__ void cons_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ uint4 ldcg16(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
@@ -169,7 +176,7 @@ struct Params {
   int slots, pitch;    // ring: row slots and their distance in bytes
   int xs_cols;         // columns of the activation rows in shared memory: max(d, I), or less, a multiple of d
   float scale;
-  int tagged_h;        // the rows of the down projection are handed over as tagged words too
+  int tagged_x, tagged_h;   // the rows of the residual stream, of the down projection, are handed over as tagged words
   int signature;       // of the sizes that the layout of the workspace follows from
 };
 __host__ __device__ inline Range share_of(int N, unsigned cta, unsigned ctas) {   // N < 2^24 (checked by the host)
@@ -389,37 +396,39 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   // next use is another layer of this launch or a layer of the next one (64 on for the same layer); none is 0 in its low
   // 6 bits, which is what a zeroed word holds.
   auto tag_of = [&](int layer) -> uint32_t { return (uint32_t)epoch * 64u + (uint32_t)layer + 1u; };
-  // The values [k0, k0 + len) of B tagged rows of K, eight bytes of them at a time: use(row, piece, values, extra),
-  // extra = more(piece) asked for ahead of the wait.
+  // The values [k0, k0 + len) of the tagged rows m0 .. m0 + RG - 1 (of B) of K, eight bytes of them at a time: use(row - m0, piece,
+  // values, extra), extra = more(piece) asked for ahead of the wait.
+  constexpr int RG = MM < 4 ? MM : 4;                 // rows on their way at a time (with eight the kernel spills 330 bytes and
+                                                      // takes 20 % longer)
   constexpr int VU = MM == 1 ? 4 : MM == 2 ? 2 : 1;   // pieces of a row on their way at a time
-  auto take = [&](const char* src, int K, int k0, int len, uint32_t tag, auto more, auto use) {
-    const int nv = len * (int)sizeof(T) / 8;
-    const char* base = src + (size_t)k0 * TB;
+  auto take = [&](const char* src, int K, int k0, int len, int m0, uint32_t tag, auto more, auto use) {
+    const int nv = len * (int)sizeof(T) / 8, rows = B - m0;
+    const char* base = src + ((size_t)m0 * K + k0) * TB;
 #pragma unroll 1
     for (int v0 = tid; v0 < nv; v0 += CONS * VU) {
-      uint4 w[MM][VU];
+      uint4 w[RG][VU];
       uint2 ex[VU];
 #pragma unroll
       for (int u = 0; u < VU; u++) ex[u] = v0 + u * CONS < nv ? more(v0 + u * CONS) : make_uint2(0, 0);
       for (uint32_t it = 0;; ++it) {
         bool all = true;
 #pragma unroll
-        for (int m = 0; m < MM; m++)
+        for (int m = 0; m < RG; m++)
 #pragma unroll
           for (int u = 0; u < VU; u++)
-            if (m < B && v0 + u * CONS < nv) w[m][u] = Tagged<T>::load(base + (size_t)m * K * TB + (size_t)(v0 + u * CONS) * 16);
+            if (m < rows && v0 + u * CONS < nv) w[m][u] = Tagged<T>::load(base + (size_t)m * K * TB + (size_t)(v0 + u * CONS) * 16);
 #pragma unroll
-        for (int m = 0; m < MM; m++)
+        for (int m = 0; m < RG; m++)
 #pragma unroll
           for (int u = 0; u < VU; u++)
-            if (m < B && v0 + u * CONS < nv) all = all && Tagged<T>::has(w[m][u], tag);
+            if (m < rows && v0 + u * CONS < nv) all = all && Tagged<T>::has(w[m][u], tag);
         if (all || give_up(it)) break;
       }
 #pragma unroll
-      for (int m = 0; m < MM; m++)
+      for (int m = 0; m < RG; m++)
 #pragma unroll
         for (int u = 0; u < VU; u++)
-          if (m < B && v0 + u * CONS < nv) use(m, v0 + u * CONS, Tagged<T>::values(w[m][u]), ex[u]);
+          if (m < rows && v0 + u * CONS < nv) use(m, v0 + u * CONS, Tagged<T>::values(w[m][u]), ex[u]);
     }
   };
   // V values at a tagged word, by this thread alone
@@ -464,24 +473,29 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
   int slot = 0;        // first slot of the next unit
   unsigned unit = 0;   // its index
 
-  // columns [k0, k0 + len) of the B rows of the down projection
-  auto load_h = [&](int layer, int k0, int len, int pitch) {
-    if (P.tagged_h) {
-      take(rows_at(H_ROWS), I, k0, len, tag_of(layer), [](int) { return make_uint2(0, 0); },
-           [&](int m, int v, const uint2& val, const uint2&) { *reinterpret_cast<uint2*>(xs + m * pitch + v * 8) = val; });
-      return;
-    }
-    const T* src = (const T*)rows_at(H_ROWS);
+  // columns [k0, k0 + len) of B plain rows of K values
+  auto load_plain = [&](const T* src, int K, int k0, int len, int pitch) {
     const int nv = len / V;
 #pragma unroll 1
     for (int v = tid; v < nv; v += CONS) {
       uint4 raw[MM];
 #pragma unroll
-      for (int m = 0; m < MM; m++) raw[m] = m < B ? ldcg16(src + (size_t)m * I + k0 + v * V) : make_uint4(0, 0, 0, 0);
+      for (int m = 0; m < MM; m++) raw[m] = m < B ? ldcg16(src + (size_t)m * K + k0 + v * V) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int m = 0; m < MM; m++)
         if (m < B) *reinterpret_cast<uint4*>(xs + m * pitch + v * 16) = raw[m];
     }
+  };
+  // columns [k0, k0 + len) of the B rows of the down projection
+  auto load_h = [&](int layer, int k0, int len, int pitch) {
+    if (P.tagged_h) {
+#pragma unroll 1
+      for (int m0 = 0; m0 < (RG < MM ? B : 1); m0 += RG)
+        take(rows_at(H_ROWS), I, k0, len, m0, tag_of(layer), [](int) { return make_uint2(0, 0); },
+             [&](int m, int v, const uint2& val, const uint2&) { *reinterpret_cast<uint2*>(xs + (m0 + m) * pitch + v * 8) = val; });
+      return;
+    }
+    load_plain((const T*)rows_at(H_ROWS), I, k0, len, pitch);
   };
   const int down_rows = min(16, own), down_pieces = own > 0 ? unit_pieces(down_rows, (I + d - 1) / d, slots, packed, xs_cols / d) : 1;
   const int items = B * H * S, owners = min(G, items);   // of the attention, and the CTAs that have any
@@ -706,52 +720,74 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     // (bf16: rows 64 bytes past a multiple of 128 apart: conflict-free fragments)
     const int K = sg.K;
     const int pitch = sizeof(T) == 2 ? ((min(K, xs_cols) * 2 + 127) & ~127) + 64 : min(K, xs_cols) * 4;
+    const bool first = sg.layer == 0 && (kind == ST_STU || kind == ST_QKV);   // the rows are the step's input
+    const bool arrives = kind == ST_GATE_UP ? !P.tagged_h : kind == ST_STU || kind == ST_CPROJ || kind == ST_DOWN ? !P.tagged_x : false;
     if (kind == ST_CPROJ && !wait(owners)) break;
     if (kind == ST_DOWN && !P.tagged_h && !wait(G)) break;
+    if (normed && !first && !P.tagged_x && !wait(G)) break;
     if (r0 >= r1) {   // no feature of this product: its rows may be gone before they are looked at
-      if (kind == ST_GATE_UP && !P.tagged_h) arrive();
+      if (arrives) arrive();
       continue;
     }
     if (normed) {
       // The rows go to shared memory times the norm weight; the factor of a row's mean square, which is known when all of it has
       // been seen, goes onto its sums instead.
       const T* nw = (const T*)(kind == ST_LM_HEAD ? a.norm_final : kind == ST_GATE_UP ? L.norm2 : L.norm1);
-      float ss[MM];
-#pragma unroll
-      for (int m = 0; m < MM; m++) ss[m] = 0.f;
       auto more = [&](int v) { return __ldg(reinterpret_cast<const uint2*>(nw) + v); };
-      auto use = [&](int m, int v, const uint2& val, const uint2& w) {
+      auto use = [&](float& ss, int m, int v, const uint2& val, const uint2& w) {
         float f[8 / sizeof(T)], g8[8 / sizeof(T)];
         unpack8(val, f, (T*)nullptr);
         unpack8(w, g8, (T*)nullptr);
 #pragma unroll
         for (int j = 0; j < (int)(8 / sizeof(T)); j++) {
-#pragma unroll
-          for (int mm = 0; mm < MM; mm++)
-            if (mm == m) ss[mm] += f[j] * f[j];
+          ss += f[j] * f[j];
           f[j] *= g8[j];
         }
         *reinterpret_cast<uint2*>(xs + m * pitch + v * 8) = pack8(f, (T*)nullptr);
       };
-      if (sg.layer == 0 && kind != ST_GATE_UP && kind != ST_LM_HEAD) {
+      if (first || !P.tagged_x) {
+        const T* rows = (const T*)rows_at(kind == ST_GATE_UP ? MID_ROWS : X_ROWS);
+        float ss[MM];
+#pragma unroll
+        for (int m = 0; m < MM; m++) ss[m] = 0.f;
 #pragma unroll 1
-        for (int v = tid; v < d * (int)sizeof(T) / 8; v += CONS) {
-          const uint2 w = more(v);
+        for (int v = tid; v < d / V; v += CONS) {
+          uint4 raw[MM];   // every row's piece is requested before the first is used
+#pragma unroll
+          for (int m = 0; m < MM; m++) {
+            const T* row = m >= B ? nullptr : first ? s_row[m] : rows + (size_t)m * d;
+            raw[m] = row ? ldcg16(row + v * V) : make_uint4(0, 0, 0, 0);
+          }
+          const uint2 w0 = more(2 * v), w1 = more(2 * v + 1);
 #pragma unroll
           for (int m = 0; m < MM; m++)
-            if (m < B) use(m, v, s_row[m] ? __ldcg(reinterpret_cast<const uint2*>(s_row[m]) + v) : make_uint2(0, 0), w);
+            if (m < B) {
+              use(ss[m], m, 2 * v, make_uint2(raw[m].x, raw[m].y), w0);
+              use(ss[m], m, 2 * v + 1, make_uint2(raw[m].z, raw[m].w), w1);
+            }
         }
+        const float total = fold<MM>(ss, lane);   // of row lane / (32 / MM)
+        if (lane % (32 / MM) == 0) s_part[lane / (32 / MM)][warp] = total;
       } else {
-        take(rows_at(kind == ST_GATE_UP ? MID_ROWS : X_ROWS), d, 0, d, tag_of(kind == ST_GATE_UP ? sg.layer : sg.layer - 1), more, use);
+#pragma unroll 1
+        for (int m0 = 0; m0 < (RG < MM ? B : 1); m0 += RG) {
+          float ss[RG];
+#pragma unroll
+          for (int m = 0; m < RG; m++) ss[m] = 0.f;
+          take(rows_at(kind == ST_GATE_UP ? MID_ROWS : X_ROWS), d, 0, d, m0, tag_of(kind == ST_GATE_UP ? sg.layer : sg.layer - 1), more,
+               [&](int m, int v, const uint2& val, const uint2& w) {
+#pragma unroll
+                 for (int mm = 0; mm < RG; mm++)
+                   if (mm == m) use(ss[mm], m0 + m, v, val, w);
+               });
+          const float total = fold<RG>(ss, lane);   // of row m0 + lane / (32 / RG)
+          if (lane % (32 / RG) == 0) s_part[m0 + lane / (32 / RG)][warp] = total;
+        }
       }
-      const float total = fold<MM>(ss, lane);   // of row lane / (32 / MM)
-      if (lane % (32 / MM) == 0) s_part[lane / (32 / MM)][warp] = total;
     } else if (kind == ST_DOWN) {
       load_h(sg.layer, 0, min(K, xs_cols), pitch);
     } else if (S == 1) {
-      const T* src = (const T*)att_at();
-      for (int v = tid; v < d / V; v += CONS)
-        for (int m = 0; m < B; m++) *reinterpret_cast<uint4*>(xs + m * pitch + v * 16) = ldcg16(src + (size_t)m * K + v * V);
+      load_plain((const T*)att_at(), K, 0, K, pitch);
     } else {   // ST_CPROJ: merge the key ranges of every head
       const int q4 = d / 4;
 #pragma unroll 1
@@ -799,6 +835,10 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
 
     // ================================================================ the product
     const uint32_t tag = tag_of(sg.layer);
+    auto hand_on = [&](int rows, int m, int n, T v, uint32_t tag) {   // a value of the residual stream
+      if (P.tagged_x) Tagged<T>::put(rows_at(rows + m), n, v, tag);
+      else ((T*)rows_at(rows))[(size_t)m * d + n] = v;
+    };
     auto finish = [&](int m, int n, float v, float v2) {   // m sequence, n feature; v2: the up projection
       if (normed) {
         v *= s_scale[m];
@@ -809,13 +849,13 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
           const float xp = round_to<T>(v);
           ((T*)L.hist)[((size_t)((size_t)m * d + n) * 2 + par) * L.Lh + s_pos] = Elem<T>::from_f(xp);
           stream = round_to<T>(stream + round_to<T>(2.f * (s_hist[tid] + xp * tap0)));
-          Tagged<T>::put(rows_at(MID_ROWS + m), n, Elem<T>::from_f(stream), tag);
+          hand_on(MID_ROWS, m, n, Elem<T>::from_f(stream), tag);
           break;
         }
         case ST_QKV: Tagged<T>::put(rows_at(QKV_ROWS + 3 * m), n, Elem<T>::from_f(v), tag); break;
         case ST_CPROJ:
           stream = round_to<T>(stream + round_to<T>(v));
-          Tagged<T>::put(rows_at(MID_ROWS + m), n, Elem<T>::from_f(stream), tag);
+          hand_on(MID_ROWS, m, n, Elem<T>::from_f(stream), tag);
           break;
         case ST_GATE_UP: {
           const T h = Elem<T>::from_f(round_to<T>(gelu_tanh(round_to<T>(v))) * round_to<T>(v2));
@@ -825,7 +865,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
         }
         case ST_DOWN:
           stream = round_to<T>(stream + round_to<T>(v));
-          Tagged<T>::put(rows_at(X_ROWS + m), n, Elem<T>::from_f(stream), tag);
+          hand_on(X_ROWS, m, n, Elem<T>::from_f(stream), tag);
           if (sg.layer == a.n_layers - 1) xbuf[(size_t)m * d + n] = Elem<T>::from_f(stream);
           break;
         default: ((T*)a.logits)[(size_t)m * a.ld_logits + n] = Elem<T>::from_f(v);
@@ -954,7 +994,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
       }
       if (base + feats < r1) cons_bar();   // the sums have been read
     }
-    if (kind == ST_GATE_UP && !P.tagged_h) arrive();
+    if (arrives) arrive();
   }
   __syncthreads();   // with the producer
   if (cta == 0 && !s_abort) {   // once every CTA has read the positions and the control words (long ago, but for idle ones)
@@ -1030,7 +1070,7 @@ extern "C" int stu_token_step_supported(int n_layers, int B, int d, int I, int H
   if ((dtype != STU_BF16 && dtype != STU_F32) || n_layers < 1 || n_layers > MAXL) return 0;
   const int vec = dtype == STU_BF16 ? 8 : 4;
   if (B < 1 || B > 8 || d < 1 || I < 1 || d % vec || I % vec || H < 0) return 0;
-  if (d > NORM_VECS * CONS * vec) return 0;
+  if (d > MAX_VECS * vec) return 0;
   if (H > 0) {
     if (d % H) return 0;
     const int lanes = d / H / vec;   // lanes per key
@@ -1150,7 +1190,8 @@ extern "C" int stu_token_step(const void* plan, int n_stages, const StuStepArgs*
   P.xs_cols = held_cols(a.B, a.d, a.I, dtype);
   P.pitch = slot_pitch(a.d, dtype);
   P.scale = a.H > 0 ? 1.0f / sqrtf((float)(a.d / a.H)) : 1.f;
-  P.tagged_h = (long long)a.B * a.I * (dtype == STU_BF16 ? Tagged<bf16>::BYTES : Tagged<float>::BYTES) <= TAGGED_H_BYTES;
+  P.tagged_x = (long long)a.B * a.d * (dtype == STU_BF16 ? Tagged<bf16>::BYTES : Tagged<float>::BYTES) <= TAGGED_X_BYTES;
+  P.tagged_h = (long long)a.B * a.I * (dtype == STU_BF16 ? Tagged<bf16>::BYTES : Tagged<float>::BYTES) <= (a.B <= 2 ? TAGGED_H_BYTES : TAGGED_H_BYTES / 2);
   P.signature = (int)((((a.B * 64 + a.n_layers) * 1021 + a.H) * 65521u + (unsigned)a.d * 8191u + (unsigned)a.I) * 4u + (dtype == STU_BF16 ? 3u : 2u));
   const size_t smem = (((size_t)P.slots * P.pitch + 127) & ~(size_t)127) + RED_BYTES +
                       (size_t)a.B * row_pitch(P.xs_cols, dtype);

@@ -192,6 +192,18 @@ def test_wide_models_of_few_sequences_against_full_prefix_logits(tmp_path, monke
     test_token_step_kernel_against_full_prefix_logits(tmp_path, dt, B, d, heads, mlp, 40, 50)
 
 
+@pytest.mark.parametrize("dt,B,d,heads,mlp", [
+    (torch.bfloat16, 8, 1024, 16, 3), (torch.bfloat16, 8, 1088, 17, 3), (torch.bfloat16, 5, 1536, 12, 2), (torch.bfloat16, 6, 1536, 24, 2),
+    (torch.float32, 4, 1024, 16, 2), (torch.float32, 5, 1024, 16, 2), (torch.float32, 8, 512, 8, 3), (torch.float32, 3, 512, 8, 4),
+    (torch.float32, 3, 512, 8, 5), (torch.float32, 2, 640, 5, 10), (torch.float32, 2, 640, 0, 11), (torch.bfloat16, 7, 256, 4, 4)])
+def test_token_step_rows_as_words_and_behind_barriers(tmp_path, monkeypatch, dt, B, d, heads, mlp):
+    """On both sides of the sizes up to which the residual stream (32 KB of words) and the rows of the down projection (100 KB, 50 KB
+    from three sequences on) travel as tagged words; with and without attention; two groups of rows."""
+    from flash_stu_2_b200.token_step import TokenStep
+    monkeypatch.setattr(TokenStep, "pays", staticmethod(lambda *a: True))
+    test_token_step_kernel_against_full_prefix_logits(tmp_path, dt, B, d, heads, mlp, 40, 50)
+
+
 def _random_model(d, heads, dt, V=1003, layers=4, **kw):
     import flash_stu_2_b200 as F
     torch.manual_seed(d)
