@@ -308,14 +308,19 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
       const bool interior = (jt + BN - 1 <= q0) && (jt >= q0 + BM - 1 - window) && (q0 + BM - 1 <= i_last);
       const float base_t = fmaf(c2, (float)jt, base_i);
       float mx = -INFINITY;
+      uint32_t seen[2] = {0xffffffffu, 0xffffffffu};   // the visible keys of this row
+      if (!interior) {
+        const int lo = max(0, i - window - jt), hi = i <= i_last ? min(BN - 1, i - jt) : -1;
+        const uint64_t bits = hi < lo ? 0ull : (~0ull >> (BN - 1 - (hi - lo))) << lo;
+        seen[0] = (uint32_t)bits;
+        seen[1] = (uint32_t)(bits >> 32);
+      }
       if (softcap > 0.f) {
         const f32x2 cc = pair_of(c2, c2), bt = pair_of(base_t, base_t);
         if (!interior) {   // a masked score decides nothing
 #pragma unroll
-          for (int c = 0; c < 64; c++) {
-            const int j = jt + c;
-            if (!((j <= i) && (j >= i - window) && (i <= i_last))) sr[c] = 0;
-          }
+          for (int c = 0; c < 64; c++)
+            if (!(seen[c >> 5] >> (c & 31) & 1u)) sr[c] = 0;
         }
         float most = 0.f;   // the largest square of the row (a NaN score is not in it: both forms carry it on)
 #pragma unroll
@@ -349,11 +354,8 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
       }
       if (!interior) {
 #pragma unroll
-        for (int c = 0; c < 64; c++) {
-          const int j = jt + c;
-          const bool valid = (j <= i) && (j >= i - window) && (i <= i_last);
-          sr[c] = valid ? sr[c] : 0xff800000u;   // -infinity
-        }
+        for (int c = 0; c < 64; c++)
+          if (!(seen[c >> 5] >> (c & 31) & 1u)) sr[c] = 0xff800000u;   // -infinity
       }
 #pragma unroll
       for (int c = 0; c < 64; c += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])));
