@@ -1446,3 +1446,26 @@ def test_full_convolution_tiles_of_64_128_and_256_channels(shape):
     """Rows on both sides of half a tile (64, 72; 128, 136), and a last tile of 8 rows, few tiles for the SMs: the bars of the test of
     the operand."""
     test_full_convolution_on_tensor_cores(shape, True)
+
+
+@pytest.mark.parametrize("gain", [1.0, 8.0, 30.0])
+def test_attention_prefill_of_heads_of_64_is_as_exact_as_the_running_maximum(gain):
+    """Error against float64 of the tcgen05 kernel, whose reference maximum lags, and of the mma.sync kernel, whose does not: on the same
+    inputs the former is no larger (by 1.01 at most: the two differ by which of 2 million roundings go which way)."""
+    from flash_stu_2_b200 import ops
+    T, H, w = 1024, 16, 512
+    torch.manual_seed(26)
+    qkv = torch.randn(1, T, 3 * H * 64, device=dev())
+    qkv[:, :, :2 * H * 64] *= gain ** 0.5
+    qkv = qkv.bfloat16()
+    slopes = O.alibi_slopes(H).float().to(dev())
+    dummy = torch.zeros(1, 1, 1, dtype=torch.bfloat16, device=dev())
+    q, k, v = [a.double().view(1, T, H, 64).transpose(1, 2) for a in qkv.split(H * 64, dim=2)]
+    s = 50 * torch.tanh(q @ k.transpose(2, 3) / 8 / 50)
+    lag = torch.arange(T, device=dev())[:, None] - torch.arange(T, device=dev())[None, :]
+    s = (s - slopes.double()[None, :, None, None] * lag).masked_fill((lag < 0) | (lag > w), float("-inf"))
+    want = (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(1, T, H * 64)
+    err = [float((f(qkv, dummy, dummy, torch.zeros(1, 2, dtype=torch.int32, device=dev()), slopes, H, w, 50.0, update_cache=False).double()
+                  - want).norm()) for f in (ops.swa_prefill_tc5, ops.swa_forward)]
+    ops.check_status()
+    assert err[0] <= 1.01 * err[1], err
