@@ -118,35 +118,39 @@ class TokenStep:
     def pays(layers: Sequence, batch: int, d: int, dtype: torch.dtype, t: int, steps: int) -> bool:
         """Whether `steps` steps from position t on take less time as persistent launches than replayed from a graph.
 
-        A layer's part of the persistent step beyond (below zero: less than) its kernels', in microseconds, from 290 pairs
-        of 4-layer models on one B200 (d 256 to 3072, 1 to 8 sequences, positions 100 to 12000).  The tap sums over the history are what decides: the persistent
-        kernel takes them at 2 TB/s (fp32: 1), the decode kernels at 5 and more.  bf16, STU layers only, 8 sequences, us per
-        step, persistent and graph: d = 1024 at 100 117 and 93, at 12000 355 and 144; d = 1536 156 and 181, 550 and 278.
-        Below two units of 16 rows in the weight ring the stream stops between units: d = 3072, 1 sequence 378 and 335;
-        fp32 d = 1536, 1 sequence 209 and 274, 4 sequences 310 and 287.
+        A layer's part of the persistent step beyond (below zero: less than) its kernels', in microseconds, fitted to 257 pairs
+        of models of 4 to 24 layers, 280 MB of weights and more, on one B200 (d 256 to 3072, 1 to 8 sequences, positions 100 to
+        12000).  The tap sums over the history are what decides: the persistent
+        kernel takes them at 2 TB/s (fp32: 1), the decode kernels at 5 and more.  us per step, persistent and graph: bf16, STU
+        layers only, 10 of d = 1024, 1 sequence at 1100 183 and 189, 8 sequences at 3000 394 and 225; 6 of d = 1536, 1 sequence at
+        100 148 and 206, 8 at 4000 397 and 319; with attention, 6 layers of d = 1536 at 400, 1 and 8 sequences 183 and 237, 296 and 311;
+        fp32, 8 layers of d = 512 with 6144 hidden values, 2 and 8 sequences 207 and 247, 398 and 307.
+        Below two units of 16 rows in the weight ring the stream stops between units: d = 3072, 1 sequence, 4 layers 359 and 348;
+        fp32 d = 1536, 1 sequence 196 and 264, 4 sequences 297 and 286.
         Against that a graph's two eager steps, capture and instantiation cost 1.2 ms and 0.12 ms per layer on an idle
         host, but 20 to 170 ms in one call of ten on a busy one, where the persistent steps take what they always take
-        (14 layers of d = 512, 54 steps: 21 to 173 ms against 20): four times the former is what it has to gain."""
+        (14 layers of d = 512, 54 steps: 21 to 173 ms against 20): four times the former is what it has to gain.  Counting that,
+        the pairs lose 1.0 % against the better choice over 30 to 1500 steps (2.6 % with the lines fitted to the kernel before)."""
         bf16, inter = dtype == torch.bfloat16, layers[0].mlp.intermediate_size
         if _lib.load().stu_token_step_ring_slots(batch, d, inter, int(bf16)) < 31 and (bf16 or batch > 2):
             return False
-        mid = t + steps // 2
+        mid, many = t + steps // 2, batch > 4   # (more than four sequences: another instance of the kernel)
         beyond = 0.0
         for layer in layers:
             if hasattr(layer, "stu"):
                 history = batch * d * (mid // 2) * (2e-6 if bf16 else 4e-6)   # MB
                 if bf16:   # (the block step kernel is the hard one to beat)
-                    beyond += (2 + 0.4 * batch if d <= 1024 and inter <= 4096 else batch - 14) + 0.47 * history
+                    beyond += 0.5 * history
+                    beyond += 0.14 * batch + 1.4 * many if d <= 1024 and inter <= 4096 else \
+                        -3 + 0.7 * batch + 2 * many - 0.021 * max(d - 1000, 0)
                 else:
-                    beyond += 4 - 0.017 * d + 0.4 * batch + (1 + 1 / batch) * history
+                    beyond += 4 - 0.022 * d + 0.5 * batch + 0.0008 * many * inter + 0.8 * (1 + 1 / batch) * history
             else:
                 keys = min(mid, layer.attn.window + 1, 1025)
                 if bf16:
-                    beyond += 6 + 0.9 * batch - 0.011 * keys if d <= 1024 else -2 - 0.004 * keys
-                    if batch * layer.attn.n_heads > 148 and keys > 512:   # a head's keys are not split over CTAs then
-                        beyond += 12
+                    beyond += 1.4 + 0.7 * batch + 6 * many - 0.023 * keys if d <= 1024 else -1.6 + 0.85 * batch + 3.5 * many - 0.01 * keys
                 else:
-                    beyond += 4.5 - 0.018 * keys + 0.0016 * batch * keys
+                    beyond += 3.3 + 0.7 * batch + 0.0017 * many * inter - 0.0055 * d - 0.036 * keys + 2.6e-6 * batch * keys * d
         return beyond * steps < 4 * (1200 + 120 * len(layers))
 
     def run(self, ids: Optional[torch.Tensor] = None, logits: Optional[torch.Tensor] = None):

@@ -150,6 +150,16 @@ def test_form_of_the_step_follows_what_was_measured(d, layers, heads, mlp, dt, B
     assert TokenStep.pays(stack, B, d, dt, t, steps) is want
 
 
+@pytest.mark.parametrize("d,layers,heads,mlp,dt,B,t,steps,attn,want", [
+    (512, 8, 8, 12, torch.float32, 2, 200, 400, True, True), (512, 8, 8, 12, torch.float32, 8, 200, 400, True, False),       # 207/245, 397/309
+    (768, 18, 12, 4, torch.bfloat16, 1, 400, 400, True, True), (768, 10, 12, 8, torch.bfloat16, 6, 4000, 400, False, False),   # 322/384, 436/286
+    (1024, 10, 8, 4, torch.bfloat16, 1, 4000, 400, True, True), (1536, 6, 12, 4, torch.bfloat16, 8, 4000, 400, False, False),  # 239/295, 405/327
+    (1536, 6, 12, 4, torch.bfloat16, 4, 400, 400, True, True)])                                                             # 233/271
+def test_form_of_the_step_follows_pairs_of_the_kernel_as_it_is(d, layers, heads, mlp, dt, B, t, steps, attn, want):
+    """us a step, persistent and graph, beside each case (up to the graph's capture, which 400 steps pay for)."""
+    test_form_of_the_step_follows_what_was_measured(d, layers, heads, mlp, dt, B, t, steps, attn, want)
+
+
 def test_tagged_words_are_read_in_elements_of_the_stores_width():
     """A word's value and tag come from one store only if they lie in one element of the reader's vector load (a vector access is
     as many accesses as it has elements): per type, every load of the words has elements as wide as the store."""
