@@ -156,7 +156,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = RMS_EPS, out: Op
         out = empty(x2.shape, x.dtype, x.device)
     o2 = out.reshape(-1, d)
     rc = _lib.native().stu_rmsnorm(x2.data_ptr(), weight.data_ptr(), o2.data_ptr(), x2.shape[0], d, x2.stride(0),
-                                 o2.stride(0), eps, _dt(x), _stream())
+                                   o2.stride(0), eps, _dt(x), _stream())
     _lib.check(rc, "stu_rmsnorm")
     _count()
     return out.reshape(x.shape)
@@ -182,7 +182,7 @@ def embed(ids: torch.Tensor, table: torch.Tensor):
     ids = ids.contiguous().to(torch.int64)
     out = empty((*ids.shape, table.shape[1]), table.dtype, table.device)
     rc = _lib.native().stu_embed(ids.data_ptr(), table.data_ptr(), out.data_ptr(), ids.numel(), table.shape[1],
-                               table.shape[0], status_word(table.device).data_ptr(), _dt(table), _stream())
+                                 table.shape[0], status_word(table.device).data_ptr(), _dt(table), _stream())
     _lib.check(rc, "stu_embed")
     _count()
     return out
@@ -237,8 +237,8 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
         resid, epilogue = kpos, EPI_STORE | EPI_FLAG_KPOS
     status_word(x.device)   # the tcgen05 GEMM reports an expired device-side wait through the registered word
     rc = _lib.native().stu_linear(x.data_ptr(), x.stride(0), W.data_ptr(), w_rs, w_ks, _p(W2), _p(resid), r_rs,
-                                out.data_ptr(), y_rs, M, N, K, epilogue, hist_T, hist_t0, hist_Lh, _p(norm_w), eps,
-                                _dt(x), backend, _stream())
+                                  out.data_ptr(), y_rs, M, N, K, epilogue, hist_T, hist_t0, hist_Lh, _p(norm_w), eps,
+                                  _dt(x), backend, _stream())
     if rc == _lib.ERR_UNSUPPORTED and norm_w is not None and x.dtype == torch.float32 and backend == BACKEND_AUTO:
         # rows or weights off the 16-byte grid: the norm in a launch of its own, the product on the kernels that take them
         return linear(rmsnorm(x, norm_w, eps), W, W2=W2, resid=resid, out=out, epilogue=epilogue)
@@ -277,8 +277,8 @@ def conv_prefill_approx(hist, taps, yT, x, t0: int, t_end: int, use_tensor_cores
     assert hist.is_contiguous() and yT.is_contiguous() and taps.shape == (d, Lh) and taps.is_contiguous()
     assert x.shape == (B, t_end - t0, d) and x.stride(2) == 1
     rc = _lib.native().stu_conv_prefill_approx(hist.data_ptr(), taps.data_ptr(), yT.data_ptr(), x.data_ptr(),
-                                             x.stride(0), x.stride(1), B, d, Lh, yT.shape[3], t0, t_end, _dt(x),
-                                             int(use_tensor_cores), _stream())
+                                               x.stride(0), x.stride(1), B, d, Lh, yT.shape[3], t0, t_end, _dt(x),
+                                               int(use_tensor_cores), _stream())
     _lib.check(rc, "stu_conv_prefill_approx")
     _count(2)
     return x
@@ -296,8 +296,8 @@ def conv_prefill_approx_tc5(hist, taps8, yT, x, t0: int, t_end: int):
     assert hist.is_contiguous() and yT.is_contiguous() and taps8.shape == (8, d, Lh + 8) and taps8.is_contiguous()
     assert x.shape == (B, t_end - t0, d) and x.stride(2) == 1
     rc = _lib.native().stu_conv_prefill_approx_tc5(hist.data_ptr(), taps8.data_ptr(), yT.data_ptr(), x.data_ptr(),
-                                                 x.stride(0), x.stride(1), B, d, Lh, yT.shape[3], t0, t_end,
-                                                 status_word(x.device).data_ptr(), _dt(x), _stream())
+                                                   x.stride(0), x.stride(1), B, d, Lh, yT.shape[3], t0, t_end,
+                                                   status_word(x.device).data_ptr(), _dt(x), _stream())
     _lib.check(rc, "stu_conv_prefill_approx_tc5")
     _count(2)
     return x
@@ -328,8 +328,8 @@ def conv_prefill_approx_static(hist, taps, x, t0: int, t_end: int, use_tensor_co
     assert hist.is_contiguous() and taps.shape == (d, Lh) and taps.is_contiguous()
     assert x.shape == (B, t_end - t0, d) and x.stride(2) == 1
     rc = _lib.native().stu_conv_prefill_approx_static(hist.data_ptr(), taps.data_ptr(), x.data_ptr(), x.stride(0),
-                                                    x.stride(1), B, d, Lh, t0, t_end, _dt(x), int(use_tensor_cores),
-                                                    _stream())
+                                                      x.stride(1), B, d, Lh, t0, t_end, _dt(x), int(use_tensor_cores),
+                                                      _stream())
     _lib.check(rc, "stu_conv_prefill_approx_static")
     _count(2)
     return x
@@ -346,9 +346,9 @@ def decode_approx(x, norm_w, MinT, hist, taps, pos, out, eps: float = RMS_EPS, t
     assert pos.dtype == torch.int32 and pos.shape == (B, 2) and pos.is_contiguous()
     assert x.data_ptr() != out.data_ptr()
     rc = _lib.native().stu_decode_approx(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(), hist.data_ptr(),
-                                       taps.data_ptr(), _p(taps8), pos.data_ptr(), out.data_ptr(), out.stride(0), B, d,
-                                       Lh, eps,
-                                       status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
+                                         taps.data_ptr(), _p(taps8), pos.data_ptr(), out.data_ptr(), out.stride(0), B, d,
+                                         Lh, eps,
+                                         status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
     _lib.check(rc, "stu_decode_approx")
     _count()
     return out
@@ -364,9 +364,9 @@ def decode_approx_shard(x, norm_w, MinT, hist, taps8, pos, out, eps: float = RMS
     assert x.shape[0] == B and MinT.shape == (dch, d_in) and out.shape == (B, dch) and x.stride(1) == 1
     assert out.stride(1) == 1 and taps8.shape == (8, dch, Lh + 8) and pos.dtype == torch.int32
     rc = _lib.native().stu_decode_approx_shard(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
-                                             hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), out.data_ptr(),
-                                             out.stride(0), B, d_in, dch, Lh, eps, int(add_residual),
-                                             status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
+                                               hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), out.data_ptr(),
+                                               out.stride(0), B, d_in, dch, Lh, eps, int(add_residual),
+                                               status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
     _lib.check(rc, "stu_decode_approx_shard")
     _count()
     return out
@@ -382,9 +382,9 @@ def decode_approx_projected(x, xp, hist, taps8, pos, out, add_residual: bool = T
     assert xp.shape == (B, dch) and out.shape == (B, dch) and xp.stride(1) == 1 and out.stride(1) == 1
     assert hist.is_contiguous() and taps8.is_contiguous() and (x is not None or not add_residual)
     rc = _lib.native().stu_decode_approx_projected(_p(x), x.stride(0) if x is not None else 0, xp.data_ptr(),
-                                                 xp.stride(0), hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(),
-                                                 out.data_ptr(), out.stride(0), B, dch, Lh, int(add_residual),
-                                                 status_word(xp.device).data_ptr(), _dt(xp) | flags, _stream())
+                                                   xp.stride(0), hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(),
+                                                   out.data_ptr(), out.stride(0), B, dch, Lh, int(add_residual),
+                                                   status_word(xp.device).data_ptr(), _dt(xp) | flags, _stream())
     _lib.check(rc, "stu_decode_approx_projected")
     _count()
     return out
@@ -398,7 +398,7 @@ def linear_push(x: torch.Tensor, W: torch.Tensor, dest: int, dest_row_stride: in
     N = W.shape[0]
     assert W.shape[1] == K and x.stride(1) == 1 and W.stride(1) == 1
     rc = _lib.native().stu_linear_push(x.data_ptr(), x.stride(0), W.data_ptr(), W.stride(0), M, N, K, dest,
-                                     dest_row_stride, _dt(x), _stream())
+                                       dest_row_stride, _dt(x), _stream())
     _lib.check(rc, "stu_linear_push")
     _count()
 
@@ -410,9 +410,9 @@ def decode_approx_push(x, norm_w, MinT, hist, taps8, pos, dest: int, dest_row_st
     d_in = x.shape[1]
     assert MinT.shape == (d_ch, d_in) and MinT.is_contiguous() and hist.is_contiguous() and taps8.is_contiguous()
     rc = _lib.native().stu_decode_approx_push(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
-                                            hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), dest, dest_row_stride,
-                                            B, d_in, d_ch, Lh, eps, status_word(x.device).data_ptr(), _dt(x),
-                                            _stream())
+                                              hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), dest, dest_row_stride,
+                                              B, d_in, d_ch, Lh, eps, status_word(x.device).data_ptr(), _dt(x),
+                                              _stream())
     _lib.check(rc, "stu_decode_approx_push")
     _count()
 
@@ -424,8 +424,8 @@ def peer_combine(x, inbox: int, slot_stride: int, in_row_stride: int, slots: int
     rows, d = x.shape
     assert x.stride(1) == 1 and (norm_w is None or (xn is not None and xn.shape == x.shape and xn.stride(1) == 1))
     rc = _lib.native().stu_peer_combine(x.data_ptr(), x.stride(0), inbox, slot_stride, in_row_stride, slots, flags,
-                                      n_ranks, epoch, _p(norm_w), _p(xn), xn.stride(0) if xn is not None else 0, eps,
-                                      rows, d, status_word(x.device).data_ptr(), wait_ms, _dt(x), _stream())
+                                        n_ranks, epoch, _p(norm_w), _p(xn), xn.stride(0) if xn is not None else 0, eps,
+                                        rows, d, status_word(x.device).data_ptr(), wait_ms, _dt(x), _stream())
     _lib.check(rc, "stu_peer_combine")
     _count()
 
@@ -439,9 +439,9 @@ def peer_exchange(xchg: int, x, src, gather: bool, slot_stride: int, norm_w=None
     assert src.shape[0] == rows and x.stride(1) == 1 and src.stride(1) == 1
     assert norm_w is None or (xn is not None and xn.shape == x.shape and xn.stride(1) == 1)
     rc = _lib.native().stu_peer_exchange(xchg, x.data_ptr(), x.stride(0), src.data_ptr(), src.stride(0), src.shape[1],
-                                       int(gather), slot_stride, _p(norm_w), _p(xn),
-                                       xn.stride(0) if xn is not None else 0, eps, rows, d,
-                                       status_word(x.device).data_ptr(), wait_ms, _dt(x), _stream())
+                                         int(gather), slot_stride, _p(norm_w), _p(xn),
+                                         xn.stride(0) if xn is not None else 0, eps, rows, d,
+                                         status_word(x.device).data_ptr(), wait_ms, _dt(x), _stream())
     _lib.check(rc, "stu_peer_exchange")
     _count()
 
@@ -457,9 +457,9 @@ def decode_approx_pipelined(x, norm_w, MinT, hist, taps8, pos, out, eps: float =
     assert out.stride(1) == 1 and taps8.shape == (8, dch, Lh + 8) and pos.dtype == torch.int32 and pos.is_contiguous()
     assert hist.is_contiguous() and taps8.is_contiguous() and x.data_ptr() != out.data_ptr()
     rc = _lib.native().stu_decode_approx_pipelined(x.data_ptr(), x.stride(0), norm_w.data_ptr(), MinT.data_ptr(),
-                                                 hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), out.data_ptr(),
-                                                 out.stride(0), B, d_in, dch, Lh, eps, int(add_residual),
-                                                 status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
+                                                   hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), out.data_ptr(),
+                                                   out.stride(0), B, d_in, dch, Lh, eps, int(add_residual),
+                                                   status_word(x.device).data_ptr(), _dt(x) | flags, _stream())
     _lib.check(rc, "stu_decode_approx_pipelined")
     _count()
     return out
@@ -483,10 +483,10 @@ def block_decode_step(x, stu_norm_w, MinT, hist, taps8, pos, mlp_norm_w, Wg, Wu,
     assert MinT.shape == (d, d) and Wg.shape == (I, d) and Wu.shape == (I, d) and Wd.shape == (d, I)
     assert all(w.is_contiguous() for w in (MinT, Wg, Wu, Wd, hist, taps8, pos)) and pos.dtype == torch.int32
     rc = _lib.native().stu_block_decode_step(x.data_ptr(), x.stride(0), stu_norm_w.data_ptr(), MinT.data_ptr(),
-                                           hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), mlp_norm_w.data_ptr(),
-                                           Wg.data_ptr(), Wu.data_ptr(), Wd.data_ptr(), out.data_ptr(), out.stride(0),
-                                           B, d, I, Lh, eps_stu, eps_mlp, workspace.data_ptr(), workspace.numel(), mode,
-                                           status_word(x.device).data_ptr(), _dt(x), _stream())
+                                             hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), mlp_norm_w.data_ptr(),
+                                             Wg.data_ptr(), Wu.data_ptr(), Wd.data_ptr(), out.data_ptr(), out.stride(0),
+                                             B, d, I, Lh, eps_stu, eps_mlp, workspace.data_ptr(), workspace.numel(), mode,
+                                             status_word(x.device).data_ptr(), _dt(x), _stream())
     _lib.check(rc, "stu_block_decode_step")
     _count()
     return out
@@ -506,7 +506,7 @@ def to_history(x, hist, t0: int):
     B, T, d = x.shape
     assert hist.is_contiguous() and hist.shape[:3] == (B, d, 2) and x.stride(2) == 1
     rc = _lib.native().stu_to_history(x.data_ptr(), x.stride(0), x.stride(1), hist.data_ptr(), B, d, hist.shape[3], t0,
-                                    t0 + T, _dt(x), _stream())
+                                      t0 + T, _dt(x), _stream())
     _lib.check(rc, "stu_to_history")
     _count()
 
@@ -526,7 +526,7 @@ def full_combine(E, Q, U, B: int, d: int, K: int, k: int, both_signs: bool, t0: 
     _cuda(E, Q, U)
     assert E.shape == Q.shape and E.is_contiguous() and Q.is_contiguous() and U.stride(1) == 1
     rc = _lib.native().stu_full_combine(E.data_ptr(), Q.data_ptr(), E.shape[1], U.data_ptr(), U.stride(0), B, d, K, k,
-                                      int(both_signs), t0, t_end, _dt(E), _stream())
+                                        int(both_signs), t0, t_end, _dt(E), _stream())
     _lib.check(rc, "stu_full_combine")
     _count()
 
@@ -538,7 +538,7 @@ def full_conv(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     L, K = phi.shape
     assert hist.is_contiguous() and phi.is_contiguous() and U.stride(1) == 1 and U.shape[0] == B * (t_end - t0)
     rc = _lib.native().stu_full_conv(hist.data_ptr(), Lh, phi.data_ptr(), L, K, U.data_ptr(), U.stride(0), B, d,
-                                   int(both_signs), t0, t_end, _dt(hist), _stream())
+                                     int(both_signs), t0, t_end, _dt(hist), _stream())
     _lib.check(rc, "stu_full_conv")
     _count()
 
@@ -556,7 +556,7 @@ def full_conv_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     lib = _lib.load()
     tab = torch.empty(lib.stu_full_conv_tc5_scratch_elems(K, t_end), dtype=hist.dtype, device=hist.device)
     rc = _lib.native().stu_full_conv_tc5(hist.data_ptr(), Lh, phi.data_ptr(), L, K, tab.data_ptr(), U.data_ptr(), U.stride(0), B, d,
-                               int(both_signs), t0, t_end, status_word(hist.device).data_ptr(), _dt(hist), _stream())
+                                         int(both_signs), t0, t_end, status_word(hist.device).data_ptr(), _dt(hist), _stream())
     _lib.check(rc, "stu_full_conv_tc5")
     _count(2)
 
@@ -570,9 +570,10 @@ def full_decode_step_supported(x2d, hist, K: int) -> bool:
 def full_decode_step_pays(batch: int, d: int, K: int, t: int) -> bool:
     """Whether the one-kernel step takes less time at position t than tap matrices, a GEMM over all history rows and a combine.  It
     saves five launches and the tap matrices, but reads the taps in every CTA, on mma.sync: rows, filters and positions tell, and
-    with more sequences the rest of the step gains less from the launches that are saved (the lines are fits).  Layer step of 24 filters, us, replayed from a graph: 8 x 1024 at 1000 47.5 and 54.1, at 7000 72 and 76; 16 x 1024 at 1000 64 and 68,
-    at 2000 77 and 74, at 7000 136 and 102; 32 x 512 at 1000 50.5 and 50.3, at 2800 77 and 62; 32 x 1536 at 60 104 and 98, at 2800
-    214 and 144; 32 filters, 16 x 1024 at 60 70 and 70, at 2800 98 and 87."""
+    with more sequences the rest of the step gains less from the launches that are saved (the lines are fits).  Layer step of 24
+    filters, us, replayed from a graph: 8 x 1024 at 1000 47.5 and 54.1, at 7000 72 and 76; 16 x 1024 at 1000 64 and 68, at 2000 77
+    and 74, at 7000 136 and 102; 32 x 512 at 1000 50.5 and 50.3, at 2800 77 and 62; 32 x 1536 at 60 104 and 98, at 2800 214 and
+    144; 32 filters, 16 x 1024 at 60 70 and 70, at 2800 98 and 87."""
     tiles = (K + 7) // 8
     return batch * d * tiles <= 49152 and (batch * tiles) ** 2 * d * t <= 3.8e9
 
@@ -585,8 +586,8 @@ def full_decode_step(x2d, norm_w, eps: float, hist, taps8, pos, U, limit: int, b
     K = taps8.shape[1] // 2
     assert taps8.shape == (8, 2 * K, Lh + 8) and x2d.stride(1) == 1 and U.is_contiguous() and U.numel() == B * (1 + both_signs) * K * d
     rc = _lib.native().stu_full_decode_step(x2d.data_ptr(), x2d.stride(0), norm_w.data_ptr() if norm_w is not None else None, eps,
-                                          hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), U.data_ptr(), B, d, K, Lh, limit,
-                                          int(both_signs), status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
+                                            hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), U.data_ptr(), B, d, K, Lh, limit,
+                                            int(both_signs), status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
     _lib.check(rc, "stu_full_decode_step")
     _count()
 
@@ -597,8 +598,8 @@ def full_decode_prepare(x2d, hist, phi, pos, PhiT):
     L, K = phi.shape
     assert PhiT.shape == (2 * K, Lh) and PhiT.is_contiguous() and phi.is_contiguous() and x2d.stride(1) == 1
     rc = _lib.native().stu_full_decode_prepare(x2d.data_ptr(), x2d.stride(0), hist.data_ptr(), phi.data_ptr(),
-                                             pos.data_ptr(), PhiT.data_ptr(), B, d, K, L, Lh,
-                                             status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
+                                               pos.data_ptr(), PhiT.data_ptr(), B, d, K, L, Lh,
+                                               status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
     _lib.check(rc, "stu_full_decode_prepare")
     _count()
 
@@ -607,7 +608,7 @@ def full_decode_combine(G, pos, U, B: int, d: int, K: int, both_signs: bool, Lh:
     _cuda(G, pos, U)
     assert G.stride(1) == 1 and U.is_contiguous()
     rc = _lib.native().stu_full_decode_combine(G.data_ptr(), G.stride(0), pos.data_ptr(), U.data_ptr(), B, d, K,
-                                             int(both_signs), Lh, int(advance), _dt(G), _stream())
+                                               int(both_signs), Lh, int(advance), _dt(G), _stream())
     _lib.check(rc, "stu_full_decode_combine")
     _count(2 if advance else 1)
 
@@ -618,7 +619,7 @@ def lds_final_state(hist, h, A32, B32, T: int):
     B, d, _, Lh = hist.shape
     assert hist.is_contiguous() and h.is_contiguous() and h.dtype == torch.float64 and A32.dtype == torch.float64
     rc = _lib.native().stu_lds_final_state(hist.data_ptr(), h.data_ptr(), A32.data_ptr(), B32.data_ptr(), B, d, Lh, T,
-                                         h.shape[2], _dt(hist), _stream())
+                                           h.shape[2], _dt(hist), _stream())
     _lib.check(rc, "stu_lds_final_state")
     _count()
 
@@ -636,8 +637,8 @@ def lds_chunk_scan(x, A64, B64, Vs, Z, hfin, Ck: int, unit_b: bool = False):
     KZ = (3 * R if x.dtype == torch.bfloat16 else R) + Ck
     assert Z.shape == (B, (T + Ck - 1) // Ck, d, KZ) and Z.dtype == x.dtype and hfin.shape == (B, d, D)
     rc = _lib.native().stu_lds_chunk_scan(x.data_ptr(), x.stride(0), x.stride(1), A64.data_ptr(), B64.data_ptr(),
-                                        Vs.data_ptr(), Z.data_ptr(), hfin.data_ptr(), B, d, T, D, R, Ck,
-                                        _dt(x) | (0x1000 if unit_b else 0), _stream())
+                                          Vs.data_ptr(), Z.data_ptr(), hfin.data_ptr(), B, d, T, D, R, Ck,
+                                          _dt(x) | (0x1000 if unit_b else 0), _stream())
     _lib.check(rc, "stu_lds_chunk_scan")
     _count()
 
@@ -652,7 +653,7 @@ def lds_chunk_features(W, Zb, U2, d: int, Ck: int, F: int):
     assert N % d == 0 and U2.shape == (N // d * Ck, F * d) and U2.dtype == W.dtype == Zb.dtype
     status_word(W.device)
     rc = _lib.native().stu_linear(W.data_ptr(), KZ, Zb.data_ptr(), KZ, 1, None, None, Ck * F * d, U2.data_ptr(), d,
-                                Mrows, N, KZ, 5, d, 0, 0, None, 0.0, _dt(W), BACKEND_AUTO, _stream())
+                                  Mrows, N, KZ, 5, d, 0, 0, None, 0.0, _dt(W), BACKEND_AUTO, _stream())
     _lib.check(rc, "stu_linear (LDS feature scatter)")
     _count()
 
@@ -665,7 +666,7 @@ def lds_decode_features(x2d, h, A32, B32, C, U):
     assert h.shape == (B, d, D) and h.is_contiguous() and h.dtype == torch.float64 and A32.dtype == torch.float64
     assert C.is_contiguous() and U.is_contiguous() and x2d.stride(1) == 1
     rc = _lib.native().stu_lds_decode_features(x2d.data_ptr(), x2d.stride(0), h.data_ptr(), A32.data_ptr(), B32.data_ptr(),
-                                             C.data_ptr(), U.data_ptr(), B, d, D, F, _dt(x2d), _stream())
+                                               C.data_ptr(), U.data_ptr(), B, d, D, F, _dt(x2d), _stream())
     _lib.check(rc, "stu_lds_decode_features")
     _count()
 
@@ -680,8 +681,8 @@ def swa_forward(qkv, k_ring, v_ring, pos, slopes, H: int, window: int, softcap: 
     assert not update_cache or (k_ring.shape == (B, W, d) and k_ring.is_contiguous() and v_ring.is_contiguous())
     out = torch.empty(B, Tn, d, dtype=qkv.dtype, device=qkv.device)
     rc = _lib.native().stu_swa_forward(qkv.data_ptr(), k_ring.data_ptr(), v_ring.data_ptr(), pos.data_ptr(),
-                                     slopes.data_ptr(), out.data_ptr(), B, Tn, H, d // H, W, window, float(softcap or 0.0),
-                                     int(update_cache), _dt(qkv), _stream())
+                                       slopes.data_ptr(), out.data_ptr(), B, Tn, H, d // H, W, window, float(softcap or 0.0),
+                                       int(update_cache), _dt(qkv), _stream())
     _lib.check(rc, "stu_swa_forward")
     _count(2 if update_cache else 1)
     return out
@@ -732,9 +733,9 @@ def sample(logits, temperature: float, top_k: Optional[int], top_p: Optional[flo
     B, V = logits.shape
     assert logits.stride(1) == 1 and out.dtype == torch.int64
     rc = _lib.native().stu_sample(logits.data_ptr(), logits.stride(0), B, V, float(temperature), int(top_k or 0),
-                                float(top_p if top_p is not None else -1.0), int(do_sample), _p(uniforms),
-                                out.data_ptr(), out_stride, status_word(logits.device).data_ptr(), _dt(logits),
-                                _stream())
+                                  float(top_p if top_p is not None else -1.0), int(do_sample), _p(uniforms),
+                                  out.data_ptr(), out_stride, status_word(logits.device).data_ptr(), _dt(logits),
+                                  _stream())
     _lib.check(rc, "stu_sample")
     _count()
     return out
