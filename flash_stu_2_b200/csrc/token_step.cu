@@ -55,6 +55,7 @@ constexpr int MAX_ROWS = 32;                  // STU channels per CTA
 // and 295.
 constexpr long long TAGGED_X_BYTES = 32 * 1024, TAGGED_H_BYTES = 100 * 1024;
 constexpr int MAX_VECS = 2 * CONS;            // 16-byte vectors of a row of the residual stream at most
+static_assert(2 * MAX_VECS * 32 <= TAGGED_X_BYTES, "one or two rows of the residual stream are always handed over as words");
 
 __device__ __forceinline__ void cons_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ uint4 ldcg16(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
@@ -498,6 +499,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     load_plain((const T*)rows_at(H_ROWS), I, k0, len, pitch);
   };
   const int down_rows = min(16, own), down_pieces = own > 0 ? unit_pieces(down_rows, (I + d - 1) / d, slots, packed, xs_cols / d) : 1;
+  const bool words_x = MM <= 2 || P.tagged_x;   // (one or two rows: at any width, see the host)
   const int items = B * H * S, owners = min(G, items);   // of the attention, and the CTAs that have any
   if (control.z != P.signature && !wait(G)) nst_run = 0;
 
@@ -721,10 +723,10 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     const int K = sg.K;
     const int pitch = sizeof(T) == 2 ? ((min(K, xs_cols) * 2 + 127) & ~127) + 64 : min(K, xs_cols) * 4;
     const bool first = sg.layer == 0 && (kind == ST_STU || kind == ST_QKV);   // the rows are the step's input
-    const bool arrives = kind == ST_GATE_UP ? !P.tagged_h : kind == ST_STU || kind == ST_CPROJ || kind == ST_DOWN ? !P.tagged_x : false;
+    const bool arrives = kind == ST_GATE_UP ? !P.tagged_h : kind == ST_STU || kind == ST_CPROJ || kind == ST_DOWN ? !words_x : false;
     if (kind == ST_CPROJ && !wait(owners)) break;
     if (kind == ST_DOWN && !P.tagged_h && !wait(G)) break;
-    if (normed && !first && !P.tagged_x && !wait(G)) break;
+    if (normed && !first && !words_x && !wait(G)) break;
     if (r0 >= r1) {   // no feature of this product: its rows may be gone before they are looked at
       if (arrives) arrive();
       continue;
@@ -745,8 +747,32 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
         }
         *reinterpret_cast<uint2*>(xs + m * pitch + v * 8) = pack8(f, (T*)nullptr);
       };
-      if (first || !P.tagged_x) {
-        const T* rows = (const T*)rows_at(kind == ST_GATE_UP ? MID_ROWS : X_ROWS);
+      const char* words = rows_at(kind == ST_GATE_UP ? MID_ROWS : X_ROWS);
+      const uint32_t tag_in = tag_of(kind == ST_GATE_UP ? sg.layer : sg.layer - 1);
+      if constexpr (MM <= 2) {
+        float ss[MM];
+#pragma unroll
+        for (int m = 0; m < MM; m++) ss[m] = 0.f;
+        auto add = [&](int m, int v, const uint2& val, const uint2& w) {
+#pragma unroll
+          for (int mm = 0; mm < MM; mm++)
+            if (mm == m) use(ss[mm], m, v, val, w);
+        };
+        if (first) {
+#pragma unroll 1
+          for (int v = tid; v < d * (int)sizeof(T) / 8; v += CONS) {
+            const uint2 w = more(v);
+#pragma unroll
+            for (int m = 0; m < MM; m++)
+              if (m < B) add(m, v, s_row[m] ? __ldcg(reinterpret_cast<const uint2*>(s_row[m]) + v) : make_uint2(0, 0), w);
+          }
+        } else {
+          take(words, d, 0, d, 0, tag_in, more, add);
+        }
+        const float total = fold<MM>(ss, lane);   // of row lane / (32 / MM)
+        if (lane % (32 / MM) == 0) s_part[lane / (32 / MM)][warp] = total;
+      } else if (first || !words_x) {
+        const T* rows = (const T*)words;
         float ss[MM];
 #pragma unroll
         for (int m = 0; m < MM; m++) ss[m] = 0.f;
@@ -774,7 +800,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
           float ss[RG];
 #pragma unroll
           for (int m = 0; m < RG; m++) ss[m] = 0.f;
-          take(rows_at(kind == ST_GATE_UP ? MID_ROWS : X_ROWS), d, 0, d, m0, tag_of(kind == ST_GATE_UP ? sg.layer : sg.layer - 1), more,
+          take(words, d, 0, d, m0, tag_in, more,
                [&](int m, int v, const uint2& val, const uint2& w) {
 #pragma unroll
                  for (int mm = 0; mm < RG; mm++)
@@ -836,7 +862,7 @@ __global__ void __launch_bounds__(THREADS, 1) token_step_kernel(const __grid_con
     // ================================================================ the product
     const uint32_t tag = tag_of(sg.layer);
     auto hand_on = [&](int rows, int m, int n, T v, uint32_t tag) {   // a value of the residual stream
-      if (P.tagged_x) Tagged<T>::put(rows_at(rows + m), n, v, tag);
+      if (words_x) Tagged<T>::put(rows_at(rows + m), n, v, tag);
       else ((T*)rows_at(rows))[(size_t)m * d + n] = v;
     };
     auto finish = [&](int m, int n, float v, float v2) {   // m sequence, n feature; v2: the up projection
