@@ -10,8 +10,8 @@
 // 32 channels, from L1 and L2.  A CTA owns 16 * MT channels of one sequence; its 8 warps take the 32-position chunks in
 // turn, their sums meet in shared memory.  As a kernel that rebuilt the K x Lh tap matrices, a GEMM against them (both
 // tap sets for both parities) and a kernel each to combine and to advance, behind the norm kernel, this was 5 launches: 8
-// sequences of 1024 channels near position 3000, the whole layer step 67 us; this form 59 (layer prefill and 64 steps 8.42 ->
-// 7.94 ms).
+// sequences of 1024 channels near position 2800, the whole layer step, replayed from a graph, 63.6 us; this form 55.9 (layer
+// prefill and 64 steps 8.42 -> 7.94 ms).  ops.full_decode_step_pays says where that form stays the faster one.
 #include "common.cuh"
 
 int device_sm_count();   // gemm_tc.cu
@@ -52,9 +52,8 @@ __global__ void __launch_bounds__(THREADS, 2)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
   const int per_seq = (d + CH - 1) / CH, b = blockIdx.x / per_seq, i0 = (blockIdx.x - b * per_seq) * CH;
   const size_t pitch = (size_t)Lh + 8;
-  pdl_wait();   // (the kernel in front may have just written the taps)
+  pdl_wait();
   pdl_trigger();
-  if (tid < 8 * NT) s_tap0[tid] = Elem<bf16>::to_f(taps[(size_t)min(tid, K - 1) * pitch + Lh - 1]);
   if (tid == 0) {
     const int t = *(volatile int*)pos;
     s_t = t;
@@ -161,6 +160,11 @@ __global__ void __launch_bounds__(THREADS, 2)
 #pragma unroll
     for (int w = 0; w < NW; w++) ss += s_part[w];
     r = rsqrtf(ss / (float)d + eps);
+  }
+  // (the taps at distance 0: behind the wait, since the kernel in front may have just written them)
+  if (tid >= THREADS - 8 * NT) {
+    const int k = tid - (THREADS - 8 * NT);
+    s_tap0[k] = Elem<bf16>::to_f(taps[(size_t)min(k, K - 1) * pitch + Lh - 1]);
   }
   if (tid < CH && i0 + tid < d) {
     const float v = Elem<bf16>::to_f(xr[i0 + tid]);
