@@ -1,15 +1,20 @@
 // Prefill linear layers on the 5th-generation tensor cores: D[M,N] = A[M,K] . B[N,K]^T in bf16 with
 // fp32 accumulators held in tensor memory (TMEM).
 //
-// One CTA computes 128 x 128 or 128 x 256 output tiles.  Warp 0 is the TMA producer (cp.async.bulk.tensor, 128-byte
-// swizzled 128x64 / 256x64 operand tiles into a ring of shared-memory stages), warp 1 allocates TMEM and
-// issues tcgen05.mma from one thread, warps 2..5 drain the accumulator with tcgen05.ld and run the
-// fused epilogue (store / residual add / tanh-GELU gate * up / transposed scatter into the projected
-// history).  The kernel is persistent (one CTA per SM walks the tile list) and the accumulator is
-// double-buffered in TMEM, so one tile's epilogue overlaps the next tile's main loop.  Every load is a plain
-// single-CTA TMA load of this GPU's own memory.
+// A pair of CTAs on neighbouring SMs computes 256 x 128 or 256 x 256 output tiles (gate/up: 256 x 128 of both accumulators) with
+// tcgen05.mma.cta_group::2: either CTA holds 128 rows of A, half the rows of B and the accumulator of its 128 rows.  What bounds
+// the large products is shared memory and power: a CTA alone on a 128 x 256 tile passes 96 KB through shared memory per 64 of K,
+// in a pair 64.  Warp 0 of either CTA is its TMA producer (cp.async.bulk.tensor, 128-byte swizzled tiles into a ring of stages,
+// counted on the first CTA's barriers), warp 1 allocates TMEM and, in the first CTA, issues the pair's tcgen05.mma; warps 2..9
+// drain the accumulator with tcgen05.ld and run the fused epilogue (store / residual add / tanh-GELU gate * up / transposed
+// scatter into the projected history).  The kernel is persistent (one pair per two SMs walks the tile list) and the accumulator is
+// double-buffered in TMEM, so one tile's epilogue overlaps the next tile's main loop.  Every load is a plain load of this GPU's
+// own memory into the loading CTA's shared memory.
+// One CTA per 128 x 256 or 128 x 128 tile, as it was before, and now (us, all back to back): 65536 x 1536 x 6144 938 -> 880,
+// gate/up 65536 x 6144 x 1536 1998 -> 1874, 65536 x 4608 x 1536 771 -> 656, 7996 x 3072 x 1024 47.3 -> 43.0, 1668 x 768 x 3072
+// 18.1 -> 12.0, 333 x 1536 x 6144 32.0 -> 18.3; smallest 4.3 -> 4.7 (256 x 256 x 64).
 //
-// Every wait on an mbarrier is bounded: on expiry the waiter raises the status word, the CTA drains
+// Every wait on an mbarrier is bounded: on expiry the waiter tells the other CTA and raises the status word, the pair drains
 // its outstanding bulk copies (bounded as well), frees its TMEM and returns.
 #include <cooperative_groups.h>
 #include <cuda.h>
@@ -27,7 +32,8 @@ namespace {
 
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int SROW = 72;   // row distance of the epilogue's staging block: 16-byte accesses by rows and by columns conflict-free
+constexpr int EPI_WARPS = 8;               // of the prefill kernel
+constexpr int BLOCK_BYTES = 32 * 64 * 2;   // an epilogue warp's block of 32 rows x 64 columns in shared memory
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 enum { EPI_HIST_T = 4 };  // internal: rows = channels, columns = tokens (operands swapped by the host)
 
@@ -45,6 +51,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Whether the phase is complete, without waiting for it.
+__device__ __forceinline__ bool mbar_ready(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(smem_u32(bar)), "r"(parity)
@@ -75,11 +93,57 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The same for a whole warp: one answer for all lanes.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned long long wait_ns) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, wait_ns));
+}
+// True in one lane of a converged warp.  The producer's and the issuer's loops are run by whole warps and only their
+// instructions by this lane: addresses and descriptors then are visibly the same for the warp and stay in uniform registers,
+// which tcgen05.mma and tensor copies take them from.  In a loop that one lane runs alone every operand goes through a
+// lane's register, and a k-block took 685 cycles to issue, whatever the size of its instructions (512 cycles for N = 256, 256 for
+// N = 128); now 605 and 440 (one pair of CTAs, 256 x 256 x 16384 without copies: 89.5 -> 78.8 us and 89.3 -> 56.8).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
+}
+
+// The same issued by either CTA of a pair: the tile lands in this CTA's shared memory, the bytes are counted on a barrier of
+// the pair's first CTA (`bar`: its shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+// shared::cluster address of the pair's first CTA's copy of a shared-memory object
+__device__ __forceinline__ uint32_t in_first_cta(const void* p) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+  return a;
+}
+__device__ __forceinline__ uint32_t load_from_cta(const volatile int* p, uint32_t cta) {
+  uint32_t a, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32((const void*)p)), "r"(cta));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_to_cta(const volatile int* p, uint32_t cta, int v) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32((const void*)p)), "r"(cta));
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// Both CTAs of the pair, all threads.  Orders no stores (that would wait for the outputs to arrive): barriers are made visible
+// by their own fence, the flag of a CTA that gave up by one ahead of this.
+__device__ __forceinline__ void pair_sync() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Shared-memory matrix descriptor for a K-major bf16 tile stored as rows of 128 bytes with the
@@ -105,6 +169,25 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t da, uint64_t db, 
       ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC), "r"(accumulate)
       : "memory");
 }
+// One instruction of a CTA pair: M = 256 (128 rows of A from each CTA's shared memory), the N rows of B half in either's.
+template <int BN_>
+__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+  constexpr uint32_t IDESC =
+      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN_ >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(IDESC), "r"(accumulate)
+      : "memory");
+}
+// Arrives at the barrier of both CTAs when the pair's instructions so far are done.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
@@ -121,8 +204,10 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr));
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+// A barrier of this pair (shared::cluster address).  At the default scope: a release for the cluster waits for all of the
+// thread's stores so far to arrive, which nothing here needs (the reads of tensor memory are done and fenced).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // tanh-GELU with the hardware tanh approximation (relative error ~2^-11, below the bf16 rounding that follows)
 __device__ __forceinline__ float gelu_tanh_fast(float x) {
@@ -130,6 +215,29 @@ __device__ __forceinline__ float gelu_tanh_fast(float x) {
   float t;
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(inner));
   return 0.5f * x * (1.0f + t);
+}
+
+// Two values rounded to bf16 and back: one conversion for both (the conversions bound the gate/up epilogue: 5250 -> 3300 cycles
+// of a tile).
+__device__ __forceinline__ void round_pair(float& a, float& b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&h);
+  a = __uint_as_float(w << 16);
+  b = __uint_as_float(w & 0xffff0000u);
+}
+// o = round(gelu(round(o))) * round(up), eight of them
+__device__ __forceinline__ void gelu_mul(float* o, const uint32_t* up) {
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) {
+    float u0 = __uint_as_float(up[j]), u1 = __uint_as_float(up[j + 1]);
+    round_pair(o[j], o[j + 1]);
+    round_pair(u0, u1);
+    o[j] = gelu_tanh_fast(o[j]);
+    o[j + 1] = gelu_tanh_fast(o[j + 1]);
+    round_pair(o[j], o[j + 1]);
+    o[j] *= u0;
+    o[j + 1] *= u1;
+  }
 }
 
 // With `causal` the B operand is lower triangular (B[n][k] = 0 for k > n, the Toeplitz matrices of the STU
@@ -150,40 +258,44 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tm = band * group_m + (r - tn * rows);
 }
 
-// Persistent kernel: CTA i handles tiles i, i + gridDim.x, ...  The accumulator is double-buffered in TMEM
+// k-blocks per stage of the ring.  Waiting for a stage, issuing and committing cost about 400 cycles whatever the size of the
+// instructions: more than the 256 that the four of a 128-column block take, less than the 512 of a 256-column one.  So the narrow
+// tiles take two blocks per stage (1536 x 6144 outputs' 333 rows 21.2 -> 18.9 us), the wide ones one, in twice as many stages
+// (gate/up of 65536 x 1536 1810 -> 1738 us).
+__host__ __device__ constexpr int stage_blocks(int mma_n) { return mma_n > 128 ? 1 : 2; }
+
+// Persistent kernel: pair i of CTAs handles tiles i, i + pairs, ...  The accumulator is double-buffered in TMEM
 // (2 x TN columns, or 2 x 256 for the two accumulators of the gate/up epilogue), so the MMA warp starts the next
-// tile while the epilogue warps drain the previous one.  TN = 256 (128 x 256 tiles) moves a third less operand
-// data per flop through shared memory than 128 x 128 and is used when the problem has enough wide tiles.
-template <int EPI, int STAGES, int TN = 128>
-__global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,
-                                                         const __grid_constant__ CUtensorMap tmB,
-                                                         const __grid_constant__ CUtensorMap tmB2,
-                                                         const __grid_constant__ CUtensorMap tmY, int by_copy, int M, int N,
-                                                         int K, int tiles_m, int tiles_n, int group_m,
-                                                         int causal, EpiArgs<bf16> ep, int* status,
-                                                         int drop_first_copy, unsigned long long wait_ns) {
+// tile while the epilogue warps drain the previous one.
+template <int EPI, int STAGES, int TN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS, 1)
+    gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmY, int by_copy, int M, int N,
+                   int K, int tiles_m, int tiles_n, int group_m, int causal, EpiArgs<bf16> ep, int* status,
+                   int drop_first_copy, unsigned long long wait_ns) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
   constexpr bool COPIES = (EPI == EPI_STORE || EPI == EPI_GELU_MUL || EPI == EPI_BLOCKCOL);   // outputs that nothing is added to
-  static_assert(!DUAL || TN == 128, "the two-accumulator epilogue uses 128-wide tiles");
-  constexpr int BN = TN;                       // shadows the file-level default inside the kernel
-  constexpr int B_BYTES = BN * BK * 2;
-  constexpr int STAGE_BYTES = A_BYTES + B_BYTES * (DUAL ? 2 : 1);
-  constexpr uint32_t ACC_COLS = DUAL ? 256 : (uint32_t)BN;
-  constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
+  constexpr int BN = TN;                       // output columns of a tile
+  constexpr int MMA_N = DUAL ? 2 * BN : BN;    // accumulator columns
+  constexpr int KBS = stage_blocks(MMA_N);
+  constexpr int KB_BYTES = A_BYTES + MMA_N / 2 * BK * 2;      // of one CTA: its rows of A, its half of B
+  constexpr int STAGE_BYTES = KBS * KB_BYTES;
+  constexpr uint32_t ACC_COLS = MMA_N;
+  constexpr uint32_t TMEM_COLS = MMA_N > 128 ? 512 : 256;     // two accumulators, a power of two
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);   // used in the pair's first CTA alone
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tmem_full = empty_bar + STAGES;   // [2]
-  uint64_t* tmem_empty = tmem_full + 2;       // [2]
+  uint64_t* tmem_empty = tmem_full + 2;       // [2], first CTA alone
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* issued_ctr = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);   // [2]: this CTA gave up, the other one did
+  int* issued_ctr = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 3));
   int* consumed_ctr = issued_ctr + 1;
-  // per epilogue warp: [32][SROW], or, where the output leaves by tensor copies, two blocks of 32 x 64 in the 128-byte swizzle
-  bf16* row_stage = reinterpret_cast<bf16*>(smem + STAGES * STAGE_BYTES + 1024);
+  unsigned char* blocks = smem + STAGES * STAGE_BYTES + 1024;   // one per epilogue warp, in the 128-byte swizzle
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int num_tiles = tiles_m * tiles_n;
   int num_kb = (K + BK - 1) / BK;
   if (EPI == EPI_STORE && ep.kpos) num_kb = min(num_kb, max(__ldg(ep.kpos), 0) / (2 * BK) + 1);   // the rest of W is zero
@@ -195,86 +307,112 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 128);
+      mbar_init(&tmem_empty[i], 2 * EPI_WARPS);   // of both CTAs
     }
-    *abort_flag = 0;
+    abort_flag[0] = abort_flag[1] = 0;
     *issued_ctr = 0;
     *consumed_ctr = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  pair_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer
-      int g = 0;  // k-blocks issued so far (ring position)
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-        int tm, tn;
-        tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
-        const int m0 = tm * BM, n0 = tn * BN;
-        const int kb_end = tile_kb(num_kb, n0, causal, BN);
-        for (int kb = 0; kb < kb_end; kb++, g++) {
-          const int s = g % STAGES;
-          const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
-          if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
+    // ---------------- TMA producer (of either CTA: its 128 rows of A, its half of the rows of B)
+    const bool leader = elect_one();
+    const CUtensorMap* mapB = DUAL && rank ? &tmB2 : &tmB;   // gate/up: the first CTA brings the gate rows, the second the up rows
+    const uint32_t full0 = in_first_cta(full_bar);
+    int g = 0, s = 0;  // stages issued so far, ring position
+    uint32_t ph = 1;
+    bool ok = true, ready = false;
+    for (int tile = pair; ok && tile < num_tiles; tile += pairs) {
+      int tm, tn;
+      tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
+      const int m0 = (2 * tm + rank) * BM, n0 = tn * BN + (DUAL ? 0 : rank * (BN / 2));
+      const int kb_end = tile_kb(num_kb, tn * BN, causal, BN);
+      for (int kb = 0; kb < kb_end; kb += KBS, g++) {
+        if (!ready) ok = warp_wait(&empty_bar[s], ph, abort_flag, wait_ns);
+        if (!ok) break;
+        const int s1 = s + 1 == STAGES ? 0 : s + 1;
+        const uint32_t ph1 = s1 ? ph : ph ^ 1u;
+        const bool ready1 = mbar_ready(&empty_bar[s1], ph1);   // asked for here, looked at behind the copies
+        if (leader) {
+          const int n = min(KBS, kb_end - kb);
           unsigned char* sa = smem + s * STAGE_BYTES;
-          mbar_expect_tx(&full_bar[s], STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * n * KB_BYTES);   // of both CTAs
           // drop_first_copy (failure-detection test only): the first stage's copies are never issued, so its
           // barrier never completes and the consumer's bounded wait has to run out
           if (!(drop_first_copy && g == 0)) {
-            tma_load_2d(sa, &tmA, &full_bar[s], kb * BK, m0);
-            tma_load_2d(sa + A_BYTES, &tmB, &full_bar[s], kb * BK, n0);
-            if (DUAL) tma_load_2d(sa + A_BYTES + B_BYTES, &tmB2, &full_bar[s], kb * BK, n0);
-            *issued_ctr = g + 1;
+            const uint32_t bar = full0 + s * (uint32_t)sizeof(uint64_t);
+#pragma unroll
+            for (int j = 0; j < KBS; j++)
+              if (j < n) {
+                tma_load_2d_pair(sa + j * KB_BYTES, &tmA, bar, (kb + j) * BK, m0);
+                tma_load_2d_pair(sa + j * KB_BYTES + A_BYTES, mapB, bar, (kb + j) * BK, n0);
+              }
           }
         }
+        ready = __all_sync(0xffffffffu, ready1);
+        s = s1, ph = ph1;
       }
     }
+    if (leader) *issued_ctr = g;
+    // the last stages' releases arrive in both CTAs: wait for them here, so that none is under way to a CTA that has left
+    for (int h = max(g - STAGES, 0); ok && h < g; h++)
+      ok = warp_wait(&empty_bar[h % STAGES], (uint32_t)(h / STAGES) & 1u, abort_flag, wait_ns);
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- MMA issuer
-      int g = 0, it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, it++) {
+    if (rank == 0) {
+      // ---------------- MMA issuer of the pair
+      const bool leader = elect_one();
+      const uint64_t da0 = make_smem_desc(smem_u32(smem)), db0 = make_smem_desc(smem_u32(smem) + A_BYTES);
+      int g = 0, s = 0, it = 0;
+      uint32_t ph = 0;
+      bool ok = true, ready = false;
+      for (int tile = pair; ok && tile < num_tiles; tile += pairs, it++) {
         const int buf = it & 1;
         const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
         int tm, tn;
         tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
         const int kb_end = tile_kb(num_kb, tn * BN, causal, BN);
-        if (!mbar_wait(&tmem_empty[buf], (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = 0; kb < kb_end; kb++, g++) {
-          const int s = g % STAGES;
-          const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
-          if (!mbar_wait(&full_bar[s], ph, abort_flag, wait_ns)) { ok = false; break; }
+        ok = warp_wait(&tmem_empty[buf], (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
+        if (!ok) break;
+        for (int kb = 0; kb < kb_end; kb += KBS, g++) {
+          if (!ready) ok = warp_wait(&full_bar[s], ph, abort_flag, wait_ns);
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + A_BYTES);
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; kk++) {
+          const int s1 = s + 1 == STAGES ? 0 : s + 1;
+          const uint32_t ph1 = s1 ? ph : ph ^ 1u;
+          const bool ready1 = mbar_ready(&full_bar[s1], ph1);   // asked for here, looked at behind the instructions
+          if (leader) {
+            const uint64_t da = da0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = db0 + (uint64_t)(s * (STAGE_BYTES >> 4));
             // advancing 16 bf16 = 32 bytes along K inside the swizzled row: +2 in the (>>4) address field
-            // gate/up: the two 128-row weight tiles lie back to back in the stage and form one 256-row B operand,
-            // so one N = 256 instruction fills both accumulators (columns 0..127 gate, 128..255 up) and the A tile
-            // is read from shared memory once instead of twice
-            if (DUAL)
-              umma<256>(acc_addr, da + 2 * kk, db + 2 * kk, (kb | kk) ? 1u : 0u);
-            else
-              umma<BN>(acc_addr, da + 2 * kk, db + 2 * kk, (kb | kk) ? 1u : 0u);
+            // gate/up: the B operand is the gate tile (first CTA) and the up tile (second), one N = 256 instruction fills
+            // both accumulators (columns 0..127 gate, 128..255 up)
+#pragma unroll
+            for (int j = 0; j < KBS; j++)
+              if (j == 0 || kb + j < kb_end) {
+#pragma unroll
+                for (int kk = 0; kk < BK / 16; kk++)
+                  umma_pair<MMA_N>(acc_addr, da + j * (KB_BYTES >> 4) + 2 * kk, db + j * (KB_BYTES >> 4) + 2 * kk,
+                                   (kb | j | kk) ? 1u : 0u);
+              }
+            umma_commit_pair(&empty_bar[s]);  // arrives when the MMAs above have finished reading this stage
           }
-          umma_commit(&empty_bar[s]);  // arrives when the MMAs above have finished reading this stage
-          *consumed_ctr = g + 1;
+          ready = __all_sync(0xffffffffu, ready1);
+          s = s1, ph = ph1;
         }
-        if (ok) umma_commit(&tmem_full[buf]);
+        if (ok && leader) umma_commit_pair(&tmem_full[buf]);
+        __syncwarp();
       }
+      if (leader) *consumed_ctr = g;
     }
   } else {
     // ---------------- epilogue warps: TMEM lane quarter = warp % 4
@@ -289,14 +427,19 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
     // of the blocks) lanes store single values, side by side.
     const bool unaligned = EPI == EPI_STORE ? ((ep.ldy & 7) || (reinterpret_cast<uintptr_t>(ep.y) & 15))
                                             : EPI == EPI_HIST_T && ((ep.Tseq & 15) || (ep.t0 & 15) || (ep.Lh & 7));
-    // Plain outputs leave by tensor copies where they can: a warp puts a block of 32 x 64 into one of two swizzled buffers and one
-    // lane sends it off, edges clipped by the copy; the copy of one block runs beside the next block's accumulator reads.
-    bf16* st = row_stage + quarter * (COPIES ? 2 * 32 * 64 : 32 * SROW);
-    int it = 0, sent = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, it++) {
+    // Plain outputs leave by tensor copies where they can: one lane sends the block off, edges clipped by the copy, which runs
+    // beside the next block's accumulator reads.
+    // Eight warps, two per quarter of the rows and either at every other 64 columns: four took 7400 cycles for a gate/up tile
+    // and 3900 for 256 columns, more than the main loop of K = 768 (6200) and all of it behind the last tile's.
+    bf16* st = reinterpret_cast<bf16*>(blocks + (warp - 2) * BLOCK_BYTES);
+    const int half = (warp - 2) >> 2;
+    auto at = [&](int row, int piece) { return st + row * 64 + ((piece ^ (row & 7)) << 3); };   // 8 values, 16 bytes
+    const uint32_t hand_back = in_first_cta(tmem_empty);
+    int it = 0;
+    for (int tile = pair; tile < num_tiles; tile += pairs, it++) {
       int tm, tn;
       tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
-      const int m0 = tm * BM, n0 = tn * BN;
+      const int m0 = (2 * tm + rank) * BM, n0 = tn * BN;
       const int first = m0 + quarter * 32, rows = min(32, M - first);   // this warp's rows
       const int buf = it & 1;
       const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
@@ -306,28 +449,25 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (COPIES && by_copy) {
 #pragma unroll 1
-        for (int nb = n0; nb < min(n0 + BN, N); nb += 64, sent++) {
+        for (int nb = n0 + 64 * half; nb < min(n0 + BN, N); nb += 128) {
           const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
-          unsigned char* blk = reinterpret_cast<unsigned char*>(st) + (sent & 1) * 4096;
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the block before last has left
-          __syncwarp();
 #pragma unroll
           for (int h = 0; h < 2; h++) {
             uint32_t r[32], r2[32];
             tmem_ld32(taddr + h * 32, r);
             if (DUAL) tmem_ld32(taddr + BN + h * 32, r2);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (h == 0) {
+              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the block before has left
+              __syncwarp();
+            }
 #pragma unroll
             for (int v8 = 0; v8 < 4; v8++) {
               float o[8];
 #pragma unroll
-              for (int j = 0; j < 8; j++) {
-                o[j] = __uint_as_float(r[v8 * 8 + j]);
-                if (EPI == EPI_GELU_MUL)
-                  o[j] = round_to<bf16>(gelu_tanh_fast(round_to<bf16>(o[j]))) *
-                         round_to<bf16>(__uint_as_float(r2[v8 * 8 + j]));
-              }
-              store_vec(reinterpret_cast<bf16*>(blk + lane * 128 + (((h * 4 + v8) ^ (lane & 7)) << 4)), o);
+              for (int j = 0; j < 8; j++) o[j] = __uint_as_float(r[v8 * 8 + j]);
+              if (DUAL) gelu_mul(o, r2 + v8 * 8);
+              store_vec(at(lane, h * 4 + v8), o);
             }
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -336,21 +476,22 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
             if (rows <= 0) {
             } else if (EPI == EPI_BLOCKCOL)
               asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(&tmY),
-                           "r"(smem_u32(blk)), "r"(nb % ep.Tseq), "r"(first), "r"(nb / ep.Tseq)
+                           "r"(smem_u32(st)), "r"(nb % ep.Tseq), "r"(first), "r"(nb / ep.Tseq)
                            : "memory");
             else
               asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&tmY),
-                           "r"(smem_u32(blk)), "r"(nb), "r"(first)
+                           "r"(smem_u32(st)), "r"(nb), "r"(first)
                            : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(&tmem_empty[buf]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(hand_back + buf * (uint32_t)sizeof(uint64_t));
         continue;
       }
 #pragma unroll 1
-      for (int nb = n0; nb < min(n0 + BN, N); nb += 64) {
+      for (int nb = n0 + 64 * half; nb < min(n0 + BN, N); nb += 128) {
         const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
 #pragma unroll 1
         for (int h = 0; h < 2; h++) {   // 32 columns of this thread's row
@@ -358,44 +499,39 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
           tmem_ld32(taddr + h * 32, r);
           if (DUAL) tmem_ld32(taddr + BN + h * 32, r2);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          bf16* dst = st + lane * SROW;
           if (EPI == EPI_HIST_T && !unaligned) {
             float par[2][16];
 #pragma unroll
             for (int j = 0; j < 32; j++) par[j & 1][j >> 1] = __uint_as_float(r[j]);
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-              store_vec(dst + q * 32 + h * 16, par[q]);
-              store_vec(dst + q * 32 + h * 16 + 8, par[q] + 8);
+              store_vec(at(lane, q * 4 + h * 2), par[q]);
+              store_vec(at(lane, q * 4 + h * 2 + 1), par[q] + 8);
             }
           } else {
 #pragma unroll
             for (int v8 = 0; v8 < 4; v8++) {
               float o[8];
 #pragma unroll
-              for (int j = 0; j < 8; j++) {
-                o[j] = __uint_as_float(r[v8 * 8 + j]);
-                if (EPI == EPI_GELU_MUL)
-                  o[j] = round_to<bf16>(gelu_tanh_fast(round_to<bf16>(o[j]))) *
-                         round_to<bf16>(__uint_as_float(r2[v8 * 8 + j]));
-              }
-              store_vec(dst + h * 32 + v8 * 8, o);
+              for (int j = 0; j < 8; j++) o[j] = __uint_as_float(r[v8 * 8 + j]);
+              if (DUAL) gelu_mul(o, r2 + v8 * 8);
+              store_vec(at(lane, h * 4 + v8), o);
             }
           }
           if (unaligned) {   // 32 columns at a time: the stores of one half run beside the accumulator read of the next
             __syncwarp();
             const int n = nb + h * 32 + lane;
             if (n < N) {
-              const bf16* col = st + h * 32 + lane;
+              const int piece = h * 4 + (lane >> 3), c = lane & 7;
               if (EPI == EPI_HIST_T) {
                 const int b = n / ep.Tseq, pitch = 2 * ep.Lh;
                 bf16* yc = ep.y + hist_off(b, first, ep.t0 + (n - b * ep.Tseq), (int)ep.ldy, ep.Lh);
 #pragma unroll 8
-                for (int i = 0; i < rows; i++) yc[(size_t)i * pitch] = col[i * SROW];
+                for (int i = 0; i < rows; i++) yc[(size_t)i * pitch] = at(i, piece)[c];
               } else {
                 bf16* yc = ep.y + (size_t)first * ep.ldy + n;
 #pragma unroll 8
-                for (int i = 0; i < rows; i++) yc[(size_t)i * ep.ldy] = col[i * SROW];
+                for (int i = 0; i < rows; i++) yc[(size_t)i * ep.ldy] = at(i, piece)[c];
               }
             }
           }
@@ -413,7 +549,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
               for (int i = 0; i < 8; i++)
                 if (r0 + i * 4 < rows)
                   *reinterpret_cast<uint4*>(yc + (size_t)(r0 + i * 4) * 2 * ep.Lh) =
-                      *reinterpret_cast<const uint4*>(st + (r0 + i * 4) * SROW + piece * 8);
+                      *reinterpret_cast<const uint4*>(at(r0 + i * 4, piece));
             }
           } else if (n + 8 <= N) {
             bf16* yc = ep.y + (size_t)(first + r0) * ep.ldy +
@@ -429,7 +565,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
               for (int i = 0; i < 8; i++)
                 if (r0 + i * 4 < rows) {
                   float o[8], rs[8];
-                  load_vec(st + (r0 + i * 4) * SROW + piece * 8, o);
+                  load_vec(at(r0 + i * 4, piece), o);
                   load_vec(reinterpret_cast<const bf16*>(&res[i]), rs);
 #pragma unroll
                   for (int j = 0; j < 8; j++) o[j] += rs[j];
@@ -440,12 +576,12 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
               for (int i = 0; i < 8; i++)
                 if (r0 + i * 4 < rows)
                   *reinterpret_cast<uint4*>(yc + (size_t)(i * 4) * ep.ldy) =
-                      *reinterpret_cast<const uint4*>(st + (r0 + i * 4) * SROW + piece * 8);
+                      *reinterpret_cast<const uint4*>(at(r0 + i * 4, piece));
             }
           } else {   // the last columns of a width that is no multiple of 8
             for (int j = n; j < min(n + 8, N); j++)
               for (int i = r0; i < rows; i += 4) {
-                const bf16 v = st[i * SROW + (j - nb)];
+                const bf16 v = at(i, piece)[j - n];
                 const size_t m = (size_t)(first + i);
                 if (EPI == EPI_RESID)
                   ep.y[m * ep.ldy + j] = __float2bfloat16_rn(__bfloat162float(ep.resid[m * ep.ldr + j]) + __bfloat162float(v));
@@ -458,20 +594,28 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
         }
         __syncwarp();   // the block has been read
       }
-      // this thread's TMEM reads of the buffer are complete (wait::ld above): hand it back to the MMA warp
+      // this warp's TMEM reads of the buffer are complete (wait::ld above): hand it back to the pair's MMA warp
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive(&tmem_empty[buf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(hand_back + buf * (uint32_t)sizeof(uint64_t));
     }
     if (COPIES && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // (none where nothing was sent)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
+  __syncwarp();
   __syncthreads();
-  if (*abort_flag) {
+  if (threadIdx.x == 0 && *abort_flag) {   // tell the other CTA
+    store_to_cta(abort_flag + 1, rank ^ 1, 1);
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  pair_sync();   // neither CTA leaves while the other's instructions, copies' barriers or arrivals still use its memory
+  if (abort_flag[0] || abort_flag[1]) {
     // A wait ran out.  Report it, then let copies that were issued but never consumed land (bounded)
-    // before shared memory is released.
-    if (threadIdx.x == 0) {
+    // before either CTA's shared memory is released.
+    if (rank == 0 && threadIdx.x == 0) {
       if (status) atomicExch(status, 3);
-      const int issued = *issued_ctr, consumed = *consumed_ctr;
+      const int issued = max(*issued_ctr, (int)load_from_cta(issued_ctr, 1)), consumed = *consumed_ctr;
       const uint64_t drain_start = global_ns();
       for (int g = consumed; g < issued; g++) {
         const int s = g % STAGES;
@@ -482,11 +626,12 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
         }
       }
     }
-    __syncthreads();
+    __syncwarp();
+    pair_sync();
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
   }
 }
 
@@ -585,17 +730,41 @@ unsigned long long g_wait_ns = 2000000000ull;
 // rows of A and 9 * 256 rows of B instead of all of B.  Gate/up of d = 3072 (75 MB of weights, 96 column tiles, 32768
 // rows): 4.6 -> 3.4 ms.  Below the lines the bands cost 1 % (gate/up of d = 1024) to 2.5 % (6000 x 1024 x 49152).
 int gemm_group_m(int tiles_n, int N, int K, bool dual) {
-  return tiles_n > 24 && (long long)N * K * (dual ? 4 : 2) > (48ll << 20) ? 16 : 1;
+  return tiles_n > 24 && (long long)N * K * (dual ? 4 : 2) > (48ll << 20) ? 8 : 1;
 }
 
-template <int EPI, int STAGES, int TN = 128>
+// Pairs of CTAs that the current device runs at a time.
+int device_pairs(const void* kernel, size_t smem) {
+  static std::atomic<int> found[STU_MAX_DEVICES] = {};
+  std::atomic<int>& n = found[current_device()];
+  if (n.load(std::memory_order_relaxed) == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * device_sm_count());
+    cfg.blockDim = dim3(64 + 32 * EPI_WARPS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+      (void)cudaGetLastError();
+      clusters = device_sm_count() / 2;
+    }
+    n.store(clusters, std::memory_order_relaxed);
+  }
+  return n.load(std::memory_order_relaxed);
+}
+
+template <int EPI, int STAGES, int TN>
 int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2, int M, int N, int K, int m_fast,
               int causal, const EpiArgs<bf16>& ep, int* status, cudaStream_t st) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
-  constexpr int BN = TN;
-  constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2 * (DUAL ? 2 : 1);
+  constexpr int STAGE_BYTES = stage_blocks(DUAL ? 2 * TN : TN) * (A_BYTES + (DUAL ? TN : TN / 2) * BK * 2);
   constexpr bool COPIES = (EPI == EPI_STORE || EPI == EPI_GELU_MUL || EPI == EPI_BLOCKCOL);
-  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 1024 + 4 * 32 * (COPIES ? 128 : SROW) * sizeof(bf16);
+  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 1024 + EPI_WARPS * BLOCK_BYTES;
   // The output by tensor copies: rows on the 16-byte grid and of whole 16 bytes (a copy clips at those), and (column blocks) 64
   // columns inside one block of a whole number of them.  What gains is many outputs for little K: LDS features, 6144 x 48128 x
   // 320, 237 -> 204 us; products of K = 1024 and more hide either form.
@@ -607,14 +776,13 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   static SmemLimit limit;
   cudaError_t e = allow_smem((const void*)k, smem, limit);
   if (e != cudaSuccess) return (int)e;
-  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
-  const int sm_count = device_sm_count();
-  const int tiles = tiles_m * tiles_n;
-  const int grid = tiles < sm_count ? tiles : sm_count;  // one persistent CTA per SM
+  const int tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + TN - 1) / TN;
+  const int tiles = tiles_m * tiles_n, pairs = device_pairs((const void*)k, smem);
+  const int grid = 2 * (tiles < pairs ? tiles : pairs);  // one persistent CTA per SM
   const int drop = g_drop_first_copy;
   g_drop_first_copy = 0;   // the injected fault applies to one launch
   const int group_m = m_fast ? tiles_m : gemm_group_m(tiles_n, N, K, DUAL);
-  k<<<grid, 192, smem, st>>>(a, b, b2, y, by_copy, M, N, K, tiles_m, tiles_n, group_m, causal, ep, status, drop, g_wait_ns);
+  k<<<grid, 64 + 32 * EPI_WARPS, smem, st>>>(a, b, b2, y, by_copy, M, N, K, tiles_m, tiles_n, group_m, causal, ep, status, drop, g_wait_ns);
   STU_CHECK_LAUNCH();
   return STU_OK;
 }
@@ -965,18 +1133,19 @@ bool gemm_tc_supported(const void* A, long long lda, const void* B, long long ld
   return get_encode_fn() != nullptr;
 }
 
-// 128 x 256 tiles where their waves over the SMs take less time than those of 128 x 128 tiles: a wide tile costs 1.31
-// square ones (measured per 64 of K over 768 of them: 0.395 against 0.302 us; the square tile is bound by the
-// shared-memory reads of its operands).  Two waves of wide tiles against four of square ones: down projection
-// 7996 x 1024 x 4096 99 -> 69 us.
-// STU_B200_TILE_N=128 forces the square tiles.
+// 256-column tiles where their waves over the pairs of SMs take less time than those of 128 columns: a wide tile costs 1.74
+// narrow ones where all pairs are busy (65536 x 1536 x 6144, 21 waves against 42: 900 and 1034 us; 1.87 where only one pair is:
+// 256 rows, K = 16384, 76.5 and 41.0).  One wave of either, 1668 x 768 x 3072: narrow 12.0 us, wide 18.3; two wide ones against
+// four narrow, 7996 x 1024 x 4096: 66.6 and 58.7.
+// STU_B200_TILE_N=128 and 256 force either.
 static bool wide_tiles(long long rows, long long cols) {
   static const char* env = getenv("STU_B200_TILE_N");
   if (env && atoi(env) == 128) return false;
-  const long long sms = device_sm_count(), tiles_m = (rows + BM - 1) / BM;
+  if (env && atoi(env) == 256) return true;
+  const long long sms = device_sm_count() / 2, tiles_m = (rows + 2 * BM - 1) / (2 * BM);
   const long long wide = (tiles_m * ((cols + 255) / 256) + sms - 1) / sms;
-  const long long square = (tiles_m * ((cols + 127) / 128) + sms - 1) / sms;
-  return 131 * wide < 100 * square;
+  const long long narrow = (tiles_m * ((cols + 127) / 128) + sms - 1) / sms;
+  return 174 * wide < 100 * narrow;
 }
 
 int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N,
@@ -989,29 +1158,29 @@ int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb,
     // one channel row of the history and writes whole 16-byte runs per parity
     const bool wide = wide_tiles(N, M);
     if ((rc = make_map(&ma, B, N, K, ldb)) != STU_OK) return rc;
-    if ((rc = make_map(&mb, A, M, K, lda, wide ? 256 : BM)) != STU_OK) return rc;
+    if ((rc = make_map(&mb, A, M, K, lda, wide ? 128 : 64)) != STU_OK) return rc;
     ep.ldy = N;  // channel count
-    if (wide) return launch_tc<EPI_HIST_T, 4, 256>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
-    return launch_tc<EPI_HIST_T, 6>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
+    if (wide) return launch_tc<EPI_HIST_T, 6, 256>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
+    return launch_tc<EPI_HIST_T, 4, 128>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
   }
   const bool wide = epi != EPI_GELU_MUL && wide_tiles(M, N);
   if ((rc = make_map(&ma, A, M, K, lda)) != STU_OK) return rc;
-  if ((rc = make_map(&mb, B, N, K, ldb, wide ? 256 : BM)) != STU_OK) return rc;
+  if ((rc = make_map(&mb, B, N, K, ldb, wide || epi == EPI_GELU_MUL ? 128 : 64)) != STU_OK) return rc;
   mb2 = mb;
   if (epi == EPI_GELU_MUL && (rc = make_map(&mb2, B2, N, K, ldb)) != STU_OK) return rc;
   if (wide) {
     switch (epi) {
-      case EPI_STORE: return launch_tc<EPI_STORE, 4, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
-      case EPI_RESID: return launch_tc<EPI_RESID, 4, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+      case EPI_STORE: return launch_tc<EPI_STORE, 6, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+      case EPI_RESID: return launch_tc<EPI_RESID, 6, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
       case EPI_BLOCKCOL:
-        return launch_tc<EPI_BLOCKCOL, 4, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+        return launch_tc<EPI_BLOCKCOL, 6, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
     }
   }
   switch (epi) {
-    case EPI_STORE: return launch_tc<EPI_STORE, 6>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
-    case EPI_RESID: return launch_tc<EPI_RESID, 6>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
-    case EPI_GELU_MUL: return launch_tc<EPI_GELU_MUL, 4>(ma, mb, mb2, M, N, K, 0, 0, ep, device_status_word(), st);
-    case EPI_BLOCKCOL: return launch_tc<EPI_BLOCKCOL, 6>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+    case EPI_STORE: return launch_tc<EPI_STORE, 4, 128>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+    case EPI_RESID: return launch_tc<EPI_RESID, 4, 128>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+    case EPI_GELU_MUL: return launch_tc<EPI_GELU_MUL, 6, 128>(ma, mb, mb2, M, N, K, 0, 0, ep, device_status_word(), st);
+    case EPI_BLOCKCOL: return launch_tc<EPI_BLOCKCOL, 4, 128>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
   }
   return STU_ERR_UNSUPPORTED;
 }

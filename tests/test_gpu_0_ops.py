@@ -43,6 +43,25 @@ def _lin_ref(x, W, W2, resid, epi, dt):
     return (g.float() * (x.double() @ W2.double().t()).to(dt).float()).to(dt)
 
 
+@pytest.mark.parametrize("epi", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 8), (128, 136, 64), (129, 256, 72), (255, 128, 136), (256, 264, 128), (257, 128, 192),
+                                   (512, 2560, 200), (2600, 2048, 64), (19200, 264, 128)])
+def test_linear_pair_tiles(M, N, K, epi):
+    """Tiles that a pair of CTAs computes: rows that fill one CTA's half, both, or a row of the next tile; both tile widths; K of
+    less than a block, of an odd number of blocks, of blocks and a piece; more tiles than pairs.  Sums in another order may round to
+    the next value, 2^-7 of the output at most: once in a plain output, twice with a residual, four times in gate/up."""
+    from flash_stu_2_b200 import ops
+    g = torch.Generator(device=dev()).manual_seed(M + N + K)
+    rand = lambda *s: torch.randn(*s, device=dev(), generator=g)
+    x, W, W2 = rand(M, K).bfloat16(), (rand(N, K) / math.sqrt(K)).bfloat16(), (rand(N, K) / math.sqrt(K)).bfloat16()
+    resid = rand(M, N).bfloat16()
+    y = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device=dev())
+    ops.linear(x, W, W2=W2 if epi == 2 else None, resid=resid if epi == 1 else None, out=y[:M], epilogue=epi, backend=ops.BACKEND_TCGEN05)
+    ops.check_status()
+    assert bool((y[M] == 7.0).all())
+    close(y[:M], _lin_ref(x, W, W2, resid, epi, torch.bfloat16), (1, 2, 4)[epi] * 2 ** -7)
+
+
 @pytest.mark.parametrize("backend", [1, 2, 3])
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("epi", [0, 1, 2])
