@@ -213,48 +213,55 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
   if (!fresh) {
     // not a prefill from position 0: nothing is computed (the caller takes the general kernel for such calls)
   } else if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ producer
-      tma::mbar_expect_tx(&ctl.q_full, L::KB * 16384);
+    const bool leader = elect_one();
+    // ------------------------------------------------------------------ producer
+    if (leader) tma::mbar_expect_tx(&ctl.q_full, L::KB * 16384);
 #pragma unroll
-      for (int kb = 0; kb < L::KB; kb++) tma::load_3d(smem + L::Q + kb * 16384, &tmQ, &ctl.q_full, h * HD + kb * 64, q0, b);
-      auto load_k = [&](int t) {
-        const int s = t & 1;
-        if (!tma::mbar_wait_bounded(&ctl.k_empty[s], ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag)) return false;
-        unsigned char* dst = smem + L::K + s * L::K_STAGE;
+    for (int kb = 0; kb < L::KB; kb++)
+      if (leader) tma::load_3d(smem + L::Q + kb * 16384, &tmQ, &ctl.q_full, h * HD + kb * 64, q0, b);
+    auto load_k = [&](int t) {
+      const int s = t & 1;
+      if (!tma::warp_wait_bounded(&ctl.k_empty[s], ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag)) return false;
+      unsigned char* dst = smem + L::K + s * L::K_STAGE;
+      if (leader) {
         tma::mbar_expect_tx(&ctl.k_full[s], L::K_STAGE);
 #pragma unroll
         for (int kb = 0; kb < L::KB; kb++)
           tma::load_3d(dst + kb * 8192, &tmK, &ctl.k_full[s], d + h * HD + kb * 64, j_lo + t * BN, b);
-        return true;
-      };
-      auto load_v = [&](int t) {
-        if (t > 0 && !tma::mbar_wait_bounded(&ctl.pv_done, (uint32_t)(t - 1) & 1u, abort_flag)) return false;
+      }
+      __syncwarp();
+      return true;
+    };
+    auto load_v = [&](int t) {
+      if (t > 0 && !tma::warp_wait_bounded(&ctl.pv_done, (uint32_t)(t - 1) & 1u, abort_flag)) return false;
+      if (leader) {
         tma::mbar_expect_tx(&ctl.v_full, HD * 128);
         asm volatile(
             "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
             ::"r"(tma::smem_u32(smem + L::V)), "l"(&tmV), "r"(tma::smem_u32(&ctl.v_full)), "r"(j_lo + t * BN),
               "r"((b * H + h) * HD)
             : "memory");
-        return true;
-      };
-      bool ok = load_k(0) && load_v(0);
-      if (ok && nt > 1) ok = load_k(1);
-      for (int t = 1; ok && t < nt; t++) {
-        ok = load_v(t);
-        if (ok && t + 1 < nt) ok = load_k(t + 1);
       }
+      __syncwarp();
+      return true;
+    };
+    bool ok = load_k(0) && load_v(0);
+    if (ok && nt > 1) ok = load_k(1);
+    for (int t = 1; ok && t < nt; t++) {
+      ok = load_v(t);
+      if (ok && t + 1 < nt) ok = load_k(t + 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
-      const uint32_t q_s = tma::smem_u32(smem + L::Q), k_s = tma::smem_u32(smem + L::K),
-                     v_s = tma::smem_u32(smem + L::V), p_s = tma::smem_u32(smem + L::P);
-      const uint32_t id_s = idesc_n(BN), id_o = idesc_n(HD);
-      auto issue_s = [&](int t) {
-        const int s = t & 1;
-        if (!tma::mbar_wait_bounded(&ctl.k_full[s], (uint32_t)(t >> 1) & 1u, abort_flag)) return false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const bool leader = elect_one();
+    // ------------------------------------------------------------------ MMA issuer
+    const uint32_t q_s = tma::smem_u32(smem + L::Q), k_s = tma::smem_u32(smem + L::K),
+                   v_s = tma::smem_u32(smem + L::V), p_s = tma::smem_u32(smem + L::P);
+    const uint32_t id_s = idesc_n(BN), id_o = idesc_n(HD);
+    auto issue_s = [&](int t) {
+      const int s = t & 1;
+      if (!tma::warp_wait_bounded(&ctl.k_full[s], (uint32_t)(t >> 1) & 1u, abort_flag)) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (leader) {
 #pragma unroll
         for (int kb = 0; kb < L::KB; kb++)
 #pragma unroll
@@ -263,21 +270,25 @@ __global__ void __launch_bounds__(192, 2) swa_umma_kernel(const __grid_constant_
                  id_s, (kb | kk) ? 1u : 0u);
         umma_commit(&ctl.s_full[s]);
         umma_commit(&ctl.k_empty[s]);
-        return true;
-      };
-      bool ok = tma::mbar_wait_bounded(&ctl.q_full, 0, abort_flag);
-      if (ok) ok = issue_s(0);
-      if (ok && nt > 1) ok = issue_s(1);
-      for (int t = 0; ok && t < nt; t++) {
-        if (!tma::mbar_wait_bounded(&ctl.p_full, (uint32_t)t & 1u, abort_flag)) { ok = false; break; }
-        if (!tma::mbar_wait_bounded(&ctl.v_full, (uint32_t)t & 1u, abort_flag)) { ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = tma::warp_wait_bounded(&ctl.q_full, 0, abort_flag);
+    if (ok) ok = issue_s(0);
+    if (ok && nt > 1) ok = issue_s(1);
+    for (int t = 0; ok && t < nt; t++) {
+      if (!tma::warp_wait_bounded(&ctl.p_full, (uint32_t)t & 1u, abort_flag)) { ok = false; break; }
+      if (!tma::warp_wait_bounded(&ctl.v_full, (uint32_t)t & 1u, abort_flag)) { ok = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (leader) {
 #pragma unroll
         for (int kk = 0; kk < 4; kk++)
           umma(tm_o, make_desc(p_s) + 2 * kk, make_desc(v_s) + 2 * kk, id_o, (t | kk) ? 1u : 0u);
         umma_commit(&ctl.pv_done);
-        if (t + 2 < nt) ok = issue_s(t + 2);   // its S buffer was read before p_full(t), its K stage freed by S(t)
       }
+      __syncwarp();
+      if (t + 2 < nt) ok = issue_s(t + 2);   // its S buffer was read before p_full(t), its K stage freed by S(t)
     }
   } else {
     // -------------------------------------------------------------------- softmax warps (TMEM lane quarter = warp % 4)

@@ -94,6 +94,17 @@ __device__ __forceinline__ void store_vec(bf16* p, const float* in) {
   *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// True in one lane of a converged warp.  The producer's and the issuer's loops are run by whole warps and only their
+// instructions by this lane: addresses and descriptors then are visibly the same for the warp and stay in uniform registers,
+// which tcgen05.mma and tensor copies take them from.  In a loop that one lane runs alone every operand goes through a
+// lane's register, and a k-block took 685 cycles to issue, whatever the size of its instructions (512 cycles for N = 256, 256 for
+// N = 128); now 605 and 440 (GEMM of a pair of CTAs, 256 x 256 x 16384 without copies: 89.5 -> 78.8 us and 89.3 -> 56.8).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
+
 // ---- programmatic dependent launch (overlap of a kernel's constant-data prefetch with its predecessor) ----
 // Flags OR-ed into the epilogue code of stu_linear and into the dtype code of stu_decode_approx:
 //   STU_FLAG_OVERLAP        the launch carries the programmatic-stream-serialization attribute: its CTAs may start

@@ -97,17 +97,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned long long wait_ns) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, wait_ns));
 }
-// True in one lane of a converged warp.  The producer's and the issuer's loops are run by whole warps and only their
-// instructions by this lane: addresses and descriptors then are visibly the same for the warp and stay in uniform registers,
-// which tcgen05.mma and tensor copies take them from.  In a loop that one lane runs alone every operand goes through a
-// lane's register, and a k-block took 685 cycles to issue, whatever the size of its instructions (512 cycles for N = 256, 256 for
-// N = 128); now 605 and 440 (one pair of CTAs, 256 x 256 x 16384 without copies: 89.5 -> 78.8 us and 89.3 -> 56.8).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
-  return ok != 0;
-}
-
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -861,56 +850,63 @@ __global__ void __launch_bounds__(192, 1)
   pdl_trigger();   // only now: this CTA holds its tensor memory
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer
-      auto load_w = [&](int s, int kb) {
-        unsigned char* sa = smem + s * stage_bytes;
-        if (DUAL) {   // 64 gate rows, then the 64 up rows of the same features
-          tma_load_2d(sa, &tmW, &full_bar[s], kb * BK, n0);
-          tma_load_2d(sa + A_BYTES / 2, &tmW2, &full_bar[s], kb * BK, n0);
-        } else {
-          tma_load_2d(sa, &tmW, &full_bar[s], kb * BK, n0);
-        }
-      };
-      auto load_x = [&](int s, int kb) {
-        tma_load_2d(smem + s * stage_bytes + A_BYTES, &tmX, &full_bar[s], kb * BK, 0);
-      };
-      const int pre = early_weights ? min(nstages, nkb) : 0;
-      for (int g = 0; g < pre; g++) {
+    // ---------------- TMA producer
+    const bool leader = elect_one();
+    auto load_w = [&](int s, int kb) {
+      unsigned char* sa = smem + s * stage_bytes;
+      if (DUAL) {   // 64 gate rows, then the 64 up rows of the same features
+        tma_load_2d(sa, &tmW, &full_bar[s], kb * BK, n0);
+        tma_load_2d(sa + A_BYTES / 2, &tmW2, &full_bar[s], kb * BK, n0);
+      } else {
+        tma_load_2d(sa, &tmW, &full_bar[s], kb * BK, n0);
+      }
+    };
+    auto load_x = [&](int s, int kb) {
+      tma_load_2d(smem + s * stage_bytes + A_BYTES, &tmX, &full_bar[s], kb * BK, 0);
+    };
+    const int pre = early_weights ? min(nstages, nkb) : 0;
+    for (int g = 0; g < pre; g++)
+      if (leader) {
         mbar_expect_tx(&full_bar[g], stage_bytes);
         load_w(g, kb0 + g);
-        *issued_ctr = g + 1;
       }
-      pdl_wait();   // the activations are the output of the kernel before this one
-      for (int g = 0; g < pre; g++) load_x(g, kb0 + g);
-      for (int g = pre; g < nkb; g++) {
-        const int s = g % nstages;
-        const uint32_t ph = (uint32_t)(g / nstages) & 1u;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, wait_ns)) break;
+    pdl_wait();   // the activations are the output of the kernel before this one
+    for (int g = 0; g < pre; g++)
+      if (leader) load_x(g, kb0 + g);
+    int g = pre, s = pre == nstages ? 0 : pre;
+    uint32_t ph = pre == nstages ? 0u : 1u;
+    for (; g < nkb; g++) {
+      if (!warp_wait(&empty_bar[s], ph, abort_flag, wait_ns)) break;
+      if (leader) {
         mbar_expect_tx(&full_bar[s], stage_bytes);
         load_w(s, kb0 + g);
         load_x(s, kb0 + g);
-        *issued_ctr = g + 1;
       }
+      if (++s == nstages) s = 0, ph ^= 1u;
     }
+    if (leader) *issued_ctr = g;
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- MMA issuer
-      bool ok = true;
-      for (int g = 0; ok && g < nkb; g++) {
-        const int s = g % nstages;
-        const uint32_t ph = (uint32_t)(g / nstages) & 1u;
-        if (!mbar_wait(&full_bar[s], ph, abort_flag, wait_ns)) { ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t sa = smem_u32(smem + s * stage_bytes);
-        const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + A_BYTES);
+    // ---------------- MMA issuer
+    const bool leader = elect_one();
+    const uint64_t da0 = make_smem_desc(smem_u32(smem)), db0 = make_smem_desc(smem_u32(smem) + A_BYTES);
+    bool ok = true;
+    int g = 0, s = 0;
+    uint32_t ph = 0;
+    for (; g < nkb; g++) {
+      ok = warp_wait(&full_bar[s], ph, abort_flag, wait_ns);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (leader) {
+        const uint64_t da = da0 + (uint64_t)(s * (stage_bytes >> 4)), db = db0 + (uint64_t)(s * (stage_bytes >> 4));
 #pragma unroll
         for (int kk = 0; kk < BK / 16; kk++) umma<SU_BN>(tmem_base, da + 2 * kk, db + 2 * kk, (g | kk) ? 1u : 0u);
-        umma_commit(&empty_bar[s]);
-        *consumed_ctr = g + 1;
+        if (g + nstages < nkb) umma_commit(&empty_bar[s]);   // (nobody waits for the last round's)
+        if (g + 1 == nkb) umma_commit(tmem_full);
       }
-      if (ok && nkb > 0) umma_commit(tmem_full);
+      __syncwarp();
+      if (++s == nstages) s = 0, ph ^= 1u;
     }
+    if (leader) *consumed_ctr = g;
   } else {
     // ---------------- accumulator drain: TMEM lane quarter = warp % 4, one weight row per thread
     const int quarter = warp & 3;

@@ -188,53 +188,59 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
   const uint32_t tmem_base = ctl->tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ producer: the history chunk of each phase
-      int pc = 0;
-      bool ok = true;
-      FOR_EACH_UNIT(task, msb, c, rg) {
+    // -------------------------------------------------------------------- producer: the history chunk of each phase
+    const bool leader = elect_one();
+    int pc = 0;
+    bool ok = true;
+    FOR_EACH_UNIT(task, msb, c, rg) {
+      if (!ok) break;
+      for (int ph = 0; ph <= 2 * msb; ph++, pc++) {
+        const int ssb = (ph == 2 * msb) ? msb : (ph >> 1);
+        const int s = pc & 1;
+        ok = tma::warp_wait_bounded(&ctl->stage_empty[s], ((uint32_t)(pc >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
         if (!ok) break;
-        for (int ph = 0; ph <= 2 * msb; ph++, pc++) {
-          const int ssb = (ph == 2 * msb) ? msb : (ph >> 1);
-          const int s = pc & 1;
-          if (!tma::mbar_wait_bounded(&ctl->stage_empty[s], ((uint32_t)(pc >> 1) & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
+        if (leader) {
           unsigned char* dst = smem + s * STAGE_BYTES;
           tma::mbar_expect_tx(&ctl->hist_full[s], HIST_BYTES);
           tma::load_5d(dst, &tmH, &ctl->hist_full[s], 0, 0, 8 * rg, SUP * ssb, c);
           tma::load_5d(dst + PLANE_BYTES, &tmH, &ctl->hist_full[s], 64, 0, 8 * rg, SUP * ssb, c);
-          ctl->issued_h = pc + 1;
         }
+        __syncwarp();
       }
     }
+    if (leader) ctl->issued_h = pc;
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
-      int pc = 0, uc = 0;
-      bool ok = true;
-      FOR_EACH_UNIT(task, msb, c, rg) {
+    // -------------------------------------------------------------------- MMA issuer
+    const bool leader = elect_one();
+    int pc = 0, uc = 0;
+    bool ok = true;
+    FOR_EACH_UNIT(task, msb, c, rg) {
+      if (!ok) break;
+      (void)c; (void)rg;
+      const int nb_m = min(SUP, g.nb_total - SUP * msb);
+      const int buf = uc & 1;
+      ok = tma::warp_wait_bounded(&ctl->tmem_empty[buf], ((uint32_t)(uc >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (leader) TL_STAMP(uc, 0);
+      for (int ph = 0; ph <= 2 * msb; ph++, pc++) {
+        const Phase P = phase_of(ph, msb, nb_m);
+        const int s = pc & 1;
+        ok = tma::warp_wait_bounded(&ctl->ready[s], (uint32_t)(pc >> 1) & 1u, abort_flag, wait_ns);
         if (!ok) break;
-        (void)c; (void)rg;
-        const int nb_m = min(SUP, g.nb_total - SUP * msb);
-        const int buf = uc & 1;
-        if (!tma::mbar_wait_bounded(&ctl->tmem_empty[buf], ((uint32_t)(uc >> 1) & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        TL_STAMP(uc, 0);
-        for (int ph = 0; ph <= 2 * msb; ph++, pc++) {
-          const Phase P = phase_of(ph, msb, nb_m);
-          const int s = pc & 1;
-          if (!tma::mbar_wait_bounded(&ctl->ready[s], (uint32_t)(pc >> 1) & 1u, abort_flag, wait_ns)) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (ph == 0) TL_STAMP(uc, 1);
-          const uint32_t hist_s = tma::smem_u32(smem + s * STAGE_BYTES), tab_s = hist_s + HIST_BYTES;
-          for (int st = 0; st < P.ndl; st++) {
-            const int dl = P.dl_lo + st;
-            const int mb_lo = max(0, dl), mb_hi = min(nb_m, SUP + dl);
-            if (mb_hi <= mb_lo) continue;
-            const uint32_t dcol = tmem_base + (uint32_t)(buf * ACC_COLS + 16 * mb_lo);
-            const uint32_t idesc = idesc_n(16 * (mb_hi - mb_lo));
-            // table entry of core matrix (q' = 0, kc = 0) of this distance: the table starts at the largest distance
-            const uint64_t da0 = make_desc_table(tab_s + 16 * (P.ndl - 1 - st) * 128);
-            const uint64_t db0 = make_desc_sw128(hist_s + (mb_lo - dl) * 2048);
+        if (ph == 0 && leader) TL_STAMP(uc, 1);
+        const uint32_t hist_s = tma::smem_u32(smem + s * STAGE_BYTES), tab_s = hist_s + HIST_BYTES;
+        for (int st = 0; st < P.ndl; st++) {
+          const int dl = P.dl_lo + st;
+          const int mb_lo = max(0, dl), mb_hi = min(nb_m, SUP + dl);
+          if (mb_hi <= mb_lo) continue;
+          const uint32_t dcol = tmem_base + (uint32_t)(buf * ACC_COLS + 16 * mb_lo);
+          const uint32_t idesc = idesc_n(16 * (mb_hi - mb_lo));
+          // table entry of core matrix (q' = 0, kc = 0) of this distance: the table starts at the largest distance
+          const uint64_t da0 = make_desc_table(tab_s + 16 * (P.ndl - 1 - st) * 128);
+          const uint64_t db0 = make_desc_sw128(hist_s + (mb_lo - dl) * 2048);
+          if (leader) {
 #pragma unroll
             for (int kk = 0; kk < 8; kk++) {
               const uint32_t acc = (ph == 0 && st == 0 && kk == 0) ? 0u : 1u;
@@ -242,15 +248,20 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
                    db0 + (uint64_t)(((kk >> 2) * PLANE_BYTES + (kk & 3) * 32) >> 4), idesc, acc);
             }
           }
-          umma_commit(&ctl->stage_empty[s]);
-          ctl->consumed_h = pc + 1;
+          __syncwarp();
         }
-        if (!ok) break;
+        if (leader) umma_commit(&ctl->stage_empty[s]);
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (leader) {
         TL_STAMP(uc, 2);
         umma_commit(&ctl->tmem_full[buf]);
-        uc++;
       }
+      __syncwarp();
+      uc++;
     }
+    if (leader) ctl->consumed_h = pc;
   } else if (warp < 6) {
     // -------------------------------------------------------------------- epilogue (TMEM lane quarter = warp % 4)
     // A lane holds one output position of 32 columns (two blocks x 16 parity rows).  Each 32 x 32 piece is turned

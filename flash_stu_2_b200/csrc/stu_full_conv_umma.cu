@@ -185,55 +185,65 @@ __global__ void __launch_bounds__(THREADS, 1) full_conv_umma_kernel(const __grid
   const uint32_t tmem_base = ctl->tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ producer
-      const uint32_t bytes = (uint32_t)g.tn * BK * 2 + A_BYTES;
-      int it = 0;
-      bool ok = true;
-      for (int i = blockIdx.x; ok && i < tiles; i += gridDim.x) {
-        const Tile t = tile_at(g, i);
-        for (int acc = 0; ok && acc < 2; acc++) {   // E, then Q
-          const int kind = acc == 0 ? 0 : (t.p ? 1 : 2);
-          const bf16* tk = tab + (size_t)(t.k * 3 + kind) * g.entries * 64;
-          for (int kb = 0; kb <= 2 * t.mb + 1; kb++, it++) {
-            const int s = it % STAGES;
-            if (!tma::mbar_wait_bounded(&ctl->empty[s], ((uint32_t)(it / STAGES) & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
+    // -------------------------------------------------------------------- producer
+    const bool leader = elect_one();
+    const uint32_t bytes = (uint32_t)g.tn * BK * 2 + A_BYTES;
+    int it = 0, s = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (int i = blockIdx.x; ok && i < tiles; i += gridDim.x) {
+      const Tile t = tile_at(g, i);
+      for (int acc = 0; ok && acc < 2; acc++) {   // E, then Q
+        const int kind = acc == 0 ? 0 : (t.p ? 1 : 2);
+        const bf16* tk = tab + (size_t)(t.k * 3 + kind) * g.entries * 64;
+        for (int kb = 0; kb <= 2 * t.mb + 1; kb++, it++) {
+          ok = tma::warp_wait_bounded(&ctl->empty[s], ph, abort_flag, wait_ns);
+          if (!ok) break;
+          if (leader) {
             tma::mbar_expect_tx(&ctl->full[s], bytes);
             tma::load_3d(smem + s * B_BYTES, &tmH, &ctl->full[s], kb * BK, t.p ^ acc, t.ct * g.tn);
             const int e0 = 16 * (g.nb - 1) - 16 * t.mb + 8 * kb;   // X = -(m0 - s0) / 8
             tma::bulk_load(smem + A_OFF + s * A_PITCH, tk + (size_t)e0 * 64, A_BYTES, &ctl->full[s]);
-            ctl->issued = it + 1;
           }
+          __syncwarp();
+          if (++s == STAGES) s = 0, ph ^= 1u;
         }
       }
     }
+    if (leader) ctl->issued = it;
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.tn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      int it = 0, n = 0;
-      bool ok = true;
-      for (int i = blockIdx.x; ok && i < tiles; i += gridDim.x, n++) {
-        const Tile t = tile_at(g, i);
-        for (int acc = 0; ok && acc < 2; acc++) {
-          if (!tma::mbar_wait_bounded(&ctl->acc_empty[acc], ((uint32_t)n & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
+    // -------------------------------------------------------------------- MMA issuer
+    const bool leader = elect_one();
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.tn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    int it = 0, n = 0, s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; ok && i < tiles; i += gridDim.x, n++) {
+      const Tile t = tile_at(g, i);
+      for (int acc = 0; ok && acc < 2; acc++) {
+        ok = tma::warp_wait_bounded(&ctl->acc_empty[acc], ((uint32_t)n & 1u) ^ 1u, abort_flag, wait_ns);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int kb = 0; kb <= 2 * t.mb + 1; kb++, it++) {
+          ok = tma::warp_wait_bounded(&ctl->full[s], ph, abort_flag, wait_ns);
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          for (int kb = 0; kb <= 2 * t.mb + 1; kb++, it++) {
-            const int s = it % STAGES;
-            if (!tma::mbar_wait_bounded(&ctl->full[s], (uint32_t)(it / STAGES) & 1u, abort_flag, wait_ns)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t da = make_desc_table(tma::smem_u32(smem + A_OFF + s * A_PITCH));
-            const uint64_t db = make_desc_sw128(tma::smem_u32(smem + s * B_BYTES));
+          const uint64_t da = make_desc_table(tma::smem_u32(smem + A_OFF + s * A_PITCH));
+          const uint64_t db = make_desc_sw128(tma::smem_u32(smem + s * B_BYTES));
+          if (leader) {
 #pragma unroll
             for (int kk = 0; kk < BK / 16; kk++)   // 16 columns: two core matrices of the table, 32 bytes of a history row
               umma(tmem_base + acc * 256, da + (uint64_t)(kk * 256 >> 4), db + (uint64_t)(kk * 32 >> 4), idesc, (kb | kk) ? 1u : 0u);
             umma_commit(&ctl->empty[s]);
-            ctl->consumed = it + 1;
           }
-          if (ok) umma_commit(&ctl->acc_full[acc]);
+          __syncwarp();
+          if (++s == STAGES) s = 0, ph ^= 1u;
         }
+        if (ok && leader) umma_commit(&ctl->acc_full[acc]);
+        __syncwarp();
       }
     }
+    if (leader) ctl->consumed = it;
   } else {
     // -------------------------------------------------------------------- epilogue (TMEM lane quarter = warp % 4)
     const int quarter = warp & 3, half = (warp - 2) >> 2;

@@ -168,4 +168,10 @@ static inline int encode_bf16(CUtensorMap* map, const void* base, int rank, cons
   return r == CUDA_SUCCESS ? STU_OK : STU_ERR_UNSUPPORTED;
 }
 
+// The same for a whole warp: one answer for all lanes.
+template <typename... Args>
+__device__ __forceinline__ bool warp_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag, Args... args) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, args...));
+}
+
 }  // namespace tma
