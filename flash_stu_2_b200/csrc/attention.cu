@@ -11,7 +11,11 @@
 // the score pass, lane = output dims for the P.V pass, online softmax per query.  Keys at positions
 // >= t0 (this call's tokens) come from the qkv activations, older ones from the ring.
 // kv_ring_write_kernel then stores this call's last W tokens into the ring and advances the positions.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 constexpr int AT_QT = 32;   // queries per CTA
 constexpr int AT_KT = 32;   // keys per tile
@@ -165,15 +169,18 @@ __global__ void __launch_bounds__(256) kv_ring_write_kernel(const T* __restrict_
 }
 
 // ------------------------------------------------------------------------------------------------
-// One new token per sequence (cached decode): memory-bound, one CTA per (head, sequence).
-// A key (or value) row of one head is hd elements = LPK lanes x 16 bytes, so a warp-wide load fetches 32/LPK
-// keys; each group of LPK lanes keeps its own online-softmax state (running maximum, sum, weighted values of
-// its 16-byte slice) over the keys it meets, with only the LPK-lane dot-product reduction per key, and the
-// 8 * 32/LPK groups of the CTA are merged once at the end through shared memory.  The new token's key and
-// value come from the qkv activations; the CTA then stores them into ring slot t % W for its head (no one reads
-// that slot in this launch: it held key t-W, outside the window), and the last CTA advances the positions.
-constexpr int DEC_U = 4;  // warp-wide key copies (and as many value copies) per round; two rounds in flight
-constexpr int DEC_RING_BYTES = 2 * DEC_U * 2 * 256 * 16;
+// One new token per sequence (cached decode): one CTA per (head, sequence), or a cluster of up to 8 that share its keys.
+// What bounds it is HBM where the grid is large (the keys and values once) and, before, the instructions per key: a key (or value)
+// row of one head is TV vectors of 16 bytes, held by 4 lanes (8 for 512-byte rows), so a warp works on 8 keys at a time and a dot
+// product takes two shuffles.  (16 lanes per key took four for two keys, and every copy a division for its ring slot; 16 sequences
+// of 12 heads of 128 over 1025 keys took as long as 32.)  Every group of lanes keeps its own softmax state (reference maximum,
+// sum, weighted values of its slice); the reference moves, and sum and values are rescaled, only where a score outgrows it
+// by 8, so that the rescale is rare (exp(8) is far from the end of fp32).  Groups are merged by shuffles, warps through shared
+// memory, CTAs of a cluster through distributed shared memory, in a fixed order.
+// The new token's key and value come from the qkv activations; the cluster's first CTA then stores them into ring slot t % W for its
+// head (no one reads that slot in this launch: it held key t-W, outside the window), and the last CTA advances the positions.
+constexpr int DEC_STAGE = 4 * 2 * 256;   // 16-byte vectors of a round: 4 of keys and 4 of values per thread
+constexpr int DEC_RING_BYTES = 2 * DEC_STAGE * 16;
 
 template <typename T> struct Vec16 {
   uint4 raw;
@@ -191,22 +198,24 @@ template <> __device__ __forceinline__ void Vec16<bf16>::unpack(float* f) const 
   }
 }
 
-template <typename T, int LPK>
-__global__ void __launch_bounds__(256) swa_decode_kernel(const T* __restrict__ qkv, T* __restrict__ k_ring,
+template <typename T, int TV>
+__global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict__ qkv, T* __restrict__ k_ring,
                                                          T* __restrict__ v_ring, int* __restrict__ pos,
                                                          const float* __restrict__ slopes, T* __restrict__ out, int B,
                                                          int H, int W, int window, float scale, float softcap,
-                                                         int update_cache) {
-  constexpr int VPL = 16 / sizeof(T);   // values per lane
-  constexpr int HD = LPK * VPL;         // head dimension
-  constexpr int KPW = 32 / LPK;         // keys per warp-wide load
-  constexpr int NG = 8 * KPW;           // softmax groups per CTA
-  __shared__ float s_m[NG], s_l[NG];
-  __shared__ float s_acc[NG][HD];
-  const int h = blockIdx.x, b = blockIdx.y;
+                                                         int update_cache, int splits) {
+  constexpr int VPL = 16 / sizeof(T);          // values per vector
+  constexpr int HD = TV * VPL;                 // head dimension
+  constexpr int G = TV >= 32 ? 8 : 4;          // lanes per key
+  constexpr int NV = TV / G;                   // vectors of a row per lane: sub, sub + G, ...
+  constexpr int U = 4 / NV;                    // keys of a lane per round
+  constexpr int KPW = 32 / G, KSTEP = 8 * KPW; // keys at a time: of a warp, of the CTA
+  __shared__ float s_m[8], s_l[8], s_acc[8][HD];
+  __shared__ float c_m, c_l, c_acc[HD];        // of this CTA, for the cluster
+  const int h = blockIdx.x / splits, part = blockIdx.x - h * splits, b = blockIdx.y;
   const int d = H * HD;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane % LPK, grp = lane / LPK;
+  const int sub = lane % G, grp = lane / G;
   pdl_trigger();   // launched with the programmatic attribute: resident while the qkv projection drains
   pdl_wait();
   const int t0 = pos[2 * b];
@@ -224,78 +233,82 @@ __global__ void __launch_bounds__(256) swa_decode_kernel(const T* __restrict__ q
     }
   }
   const T* cur = qkv + (size_t)b * 3 * d + h * HD;   // q | k | v of the new token, this head
-  float qv[VPL];
-  {
-    Vec16<T> q;
-    q.raw = *reinterpret_cast<const uint4*>(cur + sub * VPL);
-    q.unpack(qv);
-#pragma unroll
-    for (int e = 0; e < VPL; e++) qv[e] *= scale;
-  }
-  const float slope = slopes[h];
-  const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
   const int j_lo = max(0, t0 - window);
   const int nkeys = t0 - j_lo + 1;  // the new token included
-  float m = -INFINITY, l = 0.f, acc[VPL];
-#pragma unroll
-  for (int e = 0; e < VPL; e++) acc[e] = 0.f;
+  const int chunk = ((nkeys + splits - 1) / splits + 7) & ~7;
+  const int k_end = min(nkeys, (part + 1) * chunk);   // this CTA's keys: part * chunk .. k_end - 1
   const size_t ring_b = (size_t)b * W;
-  // Keys and values travel global -> shared memory by 16-byte asynchronous copies, two rounds of DEC_U keys (and
-  // values) in flight per thread: every thread copies into slots of its own and reads them back itself, so the ring
-  // needs no barrier, and the bytes in flight are bounded by shared memory (64 KB per CTA), not by registers.
-  extern __shared__ uint4 dec_ring[];   // [2 stages][DEC_U][key | value][256 threads]
-  const int first = warp * KPW;
-  const int niter = first < nkeys ? (nkeys - first + 8 * KPW * DEC_U - 1) / (8 * KPW * DEC_U) : 0;   // warp-uniform
+  // Keys and values travel global -> shared memory by 16-byte asynchronous copies, two rounds in flight per thread: every
+  // thread copies into slots of its own and reads them back itself, so the ring needs no barrier, and the bytes in
+  // flight are bounded by shared memory (64 KB per CTA), not by registers.
+  extern __shared__ uint4 dec_ring[];   // [2 stages][U][key | value][NV][256 threads]
+  const int base = part * chunk + warp * KPW;          // warp-uniform
+  const int niter = base < k_end ? (k_end - base + KSTEP * U - 1) / (KSTEP * U) : 0;
+  const int step = KSTEP % W;
+  int ik = base + grp, islot = (j_lo + ik) % W;        // key and ring slot of the next copy
   auto issue = [&](int it, int stage) {
     if (it < niter) {
 #pragma unroll
-      for (int u = 0; u < DEC_U; u++) {
-        const int kk = first + it * 8 * KPW * DEC_U + u * 8 * KPW + grp;
-        const bool ok = kk < nkeys;
-        const int j = j_lo + kk;
+      for (int u = 0; u < U; u++) {
+        const bool ok = ik < k_end;
         const T *ks, *vs;
-        if (ok && j == t0) {   // the new token's key and value come from the qkv activations
+        if (ik == nkeys - 1) {   // the new token's key and value come from the qkv activations
           ks = cur + d + sub * VPL;
           vs = cur + 2 * d + sub * VPL;
         } else {
-          const size_t off = (ring_b + (size_t)(ok ? j % W : 0)) * d + h * HD + sub * VPL;
+          const size_t off = (ring_b + (size_t)(ok ? islot : 0)) * d + h * HD + sub * VPL;
           ks = k_ring + off;
           vs = v_ring + off;
         }
         const unsigned nbytes = ok ? 16u : 0u;   // 0: the slot is filled with zeros
-        const unsigned kd = (unsigned)__cvta_generic_to_shared(&dec_ring[((stage * DEC_U + u) * 2 + 0) * 256 + threadIdx.x]);
-        const unsigned vd = (unsigned)__cvta_generic_to_shared(&dec_ring[((stage * DEC_U + u) * 2 + 1) * 256 + threadIdx.x]);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd), "l"(ks), "r"(nbytes) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd), "l"(vs), "r"(nbytes) : "memory");
+        const unsigned kd = (unsigned)__cvta_generic_to_shared(&dec_ring[stage * DEC_STAGE + (u * 2 * NV) * 256 + threadIdx.x]);
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + i * 4096), "l"(ks + i * G * VPL), "r"(nbytes) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + (NV + i) * 4096), "l"(vs + i * G * VPL), "r"(nbytes) : "memory");
+        }
+        ik += KSTEP;
+        islot += step;
+        if (islot >= W) islot -= W;
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");   // one group per call, empty past the end
   };
   issue(0, 0);
   issue(1, 1);
+  float qv[NV * VPL];
+#pragma unroll
+  for (int i = 0; i < NV; i++) {
+    Vec16<T> q;
+    q.raw = *reinterpret_cast<const uint4*>(cur + (i * G + sub) * VPL);
+    q.unpack(qv + i * VPL);
+  }
+#pragma unroll
+  for (int e = 0; e < NV * VPL; e++) qv[e] *= scale;
+  const float slope = slopes[h];
+  const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
+  float m = -INFINITY, l = 0.f, acc[NV * VPL];
+#pragma unroll
+  for (int e = 0; e < NV * VPL; e++) acc[e] = 0.f;
   for (int it = 0; it < niter; it++) {  // warp-uniform
-    const int base = first + it * 8 * KPW * DEC_U;
-    const int stage = it & 1;
+    const uint4* ring = dec_ring + (it & 1) * DEC_STAGE + threadIdx.x;
     asm volatile("cp.async.wait_group 1;" ::: "memory");   // round `it` has landed, round it + 1 may be in flight
-    Vec16<T> kr[DEC_U], vr[DEC_U];
+    float sc[U], mx = -INFINITY;
 #pragma unroll
-    for (int u = 0; u < DEC_U; u++) {
-      kr[u].raw = dec_ring[((stage * DEC_U + u) * 2 + 0) * 256 + threadIdx.x];
-      vr[u].raw = dec_ring[((stage * DEC_U + u) * 2 + 1) * 256 + threadIdx.x];
-    }
-    issue(it + 2, stage);   // refill the slots just read
-    // scores of the DEC_U keys of this group first, then ONE rescale of the running sums for all of them
-    float sc[DEC_U];
-#pragma unroll
-    for (int u = 0; u < DEC_U; u++) {
-      const int kk = base + u * 8 * KPW + grp;
-      float kf[VPL];
-      kr[u].unpack(kf);
+    for (int u = 0; u < U; u++) {
+      const int kk = base + grp + (it * U + u) * KSTEP;
       float dot = 0.f;
 #pragma unroll
-      for (int e = 0; e < VPL; e++) dot = fmaf(qv[e], kf[e], dot);
+      for (int i = 0; i < NV; i++) {
+        Vec16<T> k;
+        float kf[VPL];
+        k.raw = ring[(u * 2 * NV + i) * 256];
+        k.unpack(kf);
 #pragma unroll
-      for (int o = LPK / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        for (int e = 0; e < VPL; e++) dot = fmaf(qv[i * VPL + e], kf[e], dot);
+      }
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
       if (softcap > 0.f) {
         // bf16: hardware tanh, relative error 2^-11, below the bf16 rounding of the output (as in the prefill kernel)
         float th;
@@ -303,83 +316,152 @@ __global__ void __launch_bounds__(256) swa_decode_kernel(const T* __restrict__ q
         else th = tanhf(dot * inv_cap);
         dot = softcap * th;
       }
-      sc[u] = (kk < nkeys) ? dot - slope * (float)(nkeys - 1 - kk) : -INFINITY;   // ALiBi: i - j
+      sc[u] = (kk < k_end) ? dot - slope * (float)(nkeys - 1 - kk) : -INFINITY;   // ALiBi: i - j
+      mx = fmaxf(mx, sc[u]);
     }
-    float mnew = m;
-#pragma unroll
-    for (int u = 0; u < DEC_U; u++) mnew = fmaxf(mnew, sc[u]);
-    if (mnew > -INFINITY) {
-      const float corr = __expf(m - mnew);   // 0 while the group has seen no key yet
+    const bool grow = mx > m + 8.f || (m == -INFINITY && mx > -INFINITY);
+    if (__any_sync(0xffffffffu, grow)) {
+      const float corr = grow ? __expf(m - mx) : 1.f;   // 0 while the group has seen no key yet
+      if (grow) m = mx;
       l *= corr;
 #pragma unroll
-      for (int e = 0; e < VPL; e++) acc[e] *= corr;
+      for (int e = 0; e < NV * VPL; e++) acc[e] *= corr;
+    }
+    const float ref = m == -INFINITY ? 0.f : m;
 #pragma unroll
-      for (int u = 0; u < DEC_U; u++) {
-        const float pw = __expf(sc[u] - mnew);   // 0 for a key past the end
+    for (int u = 0; u < U; u++) {
+      const float pw = __expf(sc[u] - ref);   // 0 for a key past the end
+      l += pw;
+#pragma unroll
+      for (int i = 0; i < NV; i++) {
+        Vec16<T> v;
         float vf[VPL];
-        vr[u].unpack(vf);
-        l += pw;
+        v.raw = ring[(u * 2 * NV + NV + i) * 256];
+        v.unpack(vf);
 #pragma unroll
-        for (int e = 0; e < VPL; e++) acc[e] = fmaf(pw, vf[e], acc[e]);
+        for (int e = 0; e < VPL; e++) acc[i * VPL + e] = fmaf(pw, vf[e], acc[i * VPL + e]);
       }
-      m = mnew;
+    }
+    issue(it + 2, it & 1);   // refill the slots just read
+  }
+  {   // the groups of the warp: to their common maximum, then summed
+    float M = m;
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    const float w = m > -INFINITY ? __expf(m - M) : (l == l ? 0.f : l);   // (a group that saw NaN scores alone has no maximum)
+    l *= w;
+#pragma unroll
+    for (int e = 0; e < NV * VPL; e++) acc[e] *= w;
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) {
+      l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+      for (int e = 0; e < NV * VPL; e++) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+    }
+    if (lane == 0) {
+      s_m[warp] = M;
+      s_l[warp] = l;
+    }
+    if (grp == 0) {
+#pragma unroll
+      for (int i = 0; i < NV; i++)
+#pragma unroll
+        for (int e = 0; e < VPL; e++) s_acc[warp][(i * G + sub) * VPL + e] = acc[i * VPL + e];
     }
   }
-  const int gidx = warp * KPW + grp;
-  if (sub == 0) {
-    s_m[gidx] = m;
-    s_l[gidx] = l;
-  }
-#pragma unroll
-  for (int e = 0; e < VPL; e++) s_acc[gidx][sub * VPL + e] = acc[e];
-  if (update_cache) {  // this head's slice of the new key and value
+  if (update_cache && part == 0) {  // this head's slice of the new key and value
     const size_t slot = (ring_b + (size_t)(t0 % W)) * d + h * HD;
-    if (threadIdx.x < LPK)
+    if (threadIdx.x < TV)
       *reinterpret_cast<uint4*>(k_ring + slot + threadIdx.x * VPL) =
           *reinterpret_cast<const uint4*>(cur + d + threadIdx.x * VPL);
-    else if (threadIdx.x < 2 * LPK)
-      *reinterpret_cast<uint4*>(v_ring + slot + (threadIdx.x - LPK) * VPL) =
-          *reinterpret_cast<const uint4*>(cur + 2 * d + (threadIdx.x - LPK) * VPL);
+    else if (threadIdx.x < 2 * TV)
+      *reinterpret_cast<uint4*>(v_ring + slot + (threadIdx.x - TV) * VPL) =
+          *reinterpret_cast<const uint4*>(cur + 2 * d + (threadIdx.x - TV) * VPL);
   }
   __syncthreads();
+  float num = 0.f, den = 0.f, M = -INFINITY;
   if (threadIdx.x < HD) {
-    float M = -INFINITY;
 #pragma unroll
-    for (int g2 = 0; g2 < NG; g2++) M = fmaxf(M, s_m[g2]);
-    float num = 0.f, den = 0.f;
+    for (int g = 0; g < 8; g++) M = fmaxf(M, s_m[g]);
 #pragma unroll
-    for (int g2 = 0; g2 < NG; g2++) {
-      const float mg = s_m[g2];
-      if (mg > -INFINITY) {
-        const float w = __expf(mg - M);
-        num = fmaf(s_acc[g2][threadIdx.x], w, num);
-        den = fmaf(s_l[g2], w, den);
+    for (int g = 0; g < 8; g++) {
+      const float w = s_m[g] > -INFINITY ? __expf(s_m[g] - M) : (s_l[g] == s_l[g] ? 0.f : s_l[g]);
+      num = fmaf(s_acc[g][threadIdx.x], w, num);
+      den = fmaf(s_l[g], w, den);
+    }
+  }
+  if (splits > 1) {
+    if (threadIdx.x < HD) c_acc[threadIdx.x] = num;
+    if (threadIdx.x == 0) {
+      c_m = M;
+      c_l = den;
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    if (part == 0 && threadIdx.x < HD) {
+      float ms[8];
+      M = -INFINITY;
+      for (int r = 0; r < splits; r++) M = fmaxf(M, ms[r & 7] = *cluster.map_shared_rank(&c_m, r));
+      num = den = 0.f;
+      for (int r = 0; r < splits; r++) {
+        const float lr = *cluster.map_shared_rank(&c_l, r);
+        const float w = ms[r & 7] > -INFINITY ? __expf(ms[r & 7] - M) : (lr == lr ? 0.f : lr);
+        num = fmaf(cluster.map_shared_rank(c_acc, r)[threadIdx.x], w, num);
+        den = fmaf(lr, w, den);
       }
     }
-    out[(size_t)b * d + h * HD + threadIdx.x] = Elem<T>::from_f(num / den);
+    cluster.sync();   // the other CTAs' results stay alive until they are read
+    if (part) return;
   }
+  if (threadIdx.x < HD) out[(size_t)b * d + h * HD + threadIdx.x] = Elem<T>::from_f(num / den);
 }
+
+int device_sm_count();   // gemm_tc.cu
 
 template <typename T>
 static bool launch_swa_decode(const void* qkv, void* k_ring, void* v_ring, int* pos, const float* slopes, void* out,
                               int B, int H, int hd, int W, int window, float scale, float softcap, int update_cache,
-                              cudaStream_t st) {
+                              cudaStream_t st, int* rc) {
   constexpr int VPL = 16 / sizeof(T);
   if (hd % VPL || !aligned16(qkv) || !aligned16(k_ring) || !aligned16(v_ring) || !aligned16(out)) return false;
-  dim3 grid(H, B);
-#define STU_SWA_DEC(LPK_)                                                                                        \
-  static SmemLimit limit##LPK_;                                                                                     \
-  allow_smem((const void*)swa_decode_kernel<T, LPK_>, DEC_RING_BYTES, limit##LPK_);                                 \
-  launch_maybe_overlapped(swa_decode_kernel<T, LPK_>, grid, dim3(256), DEC_RING_BYTES, st, true, (const T*)qkv,     \
-                          (T*)k_ring, (T*)v_ring, pos, slopes, (T*)out, B, H, W, window, scale, softcap,            \
-                          update_cache)
+  // CTAs per (head, sequence): while the grid stays below three per SM, what shared memory holds, and each keeps 128 keys.  us, bf16 heads
+  // of 128, window 1024, 1 / 2 / 4 / 8 CTAs: 12 heads of 1 sequence 16.1 / 11.1 / 8.4 / 8.0, 8: 18.9 / 17.9 / 15.8 / 23.2, 16: 24.5 / 24.1 / 29.5, 24: 32.8 /
+  // 40.7, 32: 40.1 / 45.2; 129 keys of 4 heads of 32: 3.6 / 4.7.  (One CTA of the form with 16 lanes per key: 21.7, 24.6, 29.9, -, 41.1; 5.7.)
+  int splits = 1;
+  while (splits < 8 && 2 * splits * H * B <= 3 * device_sm_count() && (window + 1) / (2 * splits) >= 128) splits *= 2;
+  static SmemLimit limits[4];
+  auto launch = [&](auto kern, SmemLimit& limit) {
+    cudaError_t e = allow_smem((const void*)kern, DEC_RING_BYTES, limit);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(H * splits, B);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = DEC_RING_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    cfg.attrs = at;
+    if (splits > 1) {
+      at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+      at[cfg.numAttrs].val.clusterDim.x = splits;
+      at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+      cfg.numAttrs++;
+    }
+    if (pdl_enabled()) {
+      at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+      cfg.numAttrs++;
+    }
+    if (e == cudaSuccess)
+      e = cudaLaunchKernelEx(&cfg, kern, (const T*)qkv, (T*)k_ring, (T*)v_ring, pos, slopes, (T*)out, B, H, W, window, scale, softcap,
+                             update_cache, splits);
+    *rc = (int)e;
+    return true;
+  };
   switch (hd / VPL) {
-    case 4: { STU_SWA_DEC(4); return true; }
-    case 8: { STU_SWA_DEC(8); return true; }
-    case 16: { STU_SWA_DEC(16); return true; }
-    case 32: { STU_SWA_DEC(32); return true; }
+    case 4: return launch(swa_decode_kernel<T, 4>, limits[0]);
+    case 8: return launch(swa_decode_kernel<T, 8>, limits[1]);
+    case 16: return launch(swa_decode_kernel<T, 16>, limits[2]);
+    case 32: return launch(swa_decode_kernel<T, 32>, limits[3]);
   }
-#undef STU_SWA_DEC
   return false;
 }
 
@@ -628,15 +710,17 @@ extern "C" int stu_swa_forward(const void* qkv, void* k_ring, void* v_ring, int*
   const float scale = 1.0f / sqrtf((float)hd);
   if (Tn == 1) {  // cached decode: the memory-bound kernel (also stores the new key/value and advances pos)
     bool done = false;
+    int rc = 0;
     if (dtype == STU_F32)
       done = launch_swa_decode<float>(qkv, k_ring, v_ring, pos, slopes, out, B, H, hd, W, window, scale, softcap,
-                                      update_cache, st);
+                                      update_cache, st, &rc);
     else if (dtype == STU_BF16)
       done = launch_swa_decode<bf16>(qkv, k_ring, v_ring, pos, slopes, out, B, H, hd, W, window, scale, softcap,
-                                     update_cache, st);
+                                     update_cache, st, &rc);
     else
       return STU_ERR_DTYPE;
     if (done) {
+      if (rc != 0) return rc;
       STU_CHECK_LAUNCH();
       return STU_OK;
     }

@@ -43,6 +43,39 @@ def _lin_ref(x, W, W2, resid, epi, dt):
     return (g.float() * (x.double() @ W2.double().t()).to(dt).float()).to(dt)
 
 
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,H,hd,window,t", [(1, 4, 32, 255, 900), (1, 3, 64, 511, 3), (2, 5, 64, 1024, 1024), (1, 2, 128, 1024, 5000),
+                                             (3, 2, 128, 300, 301), (1, 1, 16, 2047, 1500), (40, 8, 64, 300, 120), (1, 2, 128, 1500, 127),
+                                             (2, 3, 32, 20, 21), (1, 2, 64, 0, 7)])
+def test_attention_decode_shares_keys(dt, B, H, hd, window, t):
+    """One cached token: keys of a head shared by 1 to 8 CTAs, some of them without any; rings that have wrapped and rings that are
+    not full; 64- to 512-byte rows.  Against the formula in float64 on the same rounded inputs; the output is rounded once (bf16: 2^-8
+    of its row's largest, and the hardware tanh's 2^-11 on scores up to 6)."""
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.modules import new_pos
+    if hd * torch.finfo(dt).bits // 128 not in (4, 8, 16, 32):
+        pytest.skip("rows of 64 to 512 bytes")
+    g = torch.Generator(device=dev()).manual_seed(B + hd + window + t)
+    rand = lambda *s: torch.randn(*s, device=dev(), generator=g).to(dt)
+    W, d, cap = window + 1, H * hd, 50.0
+    k_ring, v_ring, qkv = rand(B, W, d), rand(B, W, d), rand(B, 1, 3 * d)
+    slopes = torch.rand(H, device=dev(), generator=g) * 0.1
+    pos = new_pos(B, dev())
+    pos[:, 0] = t
+    keys = list(range(max(0, t - window), t))
+    slots = torch.tensor([j % W for j in keys], dtype=torch.long, device=dev())
+    q, kn, vn = (p.double().view(B, 1, H, hd) for p in qkv.split(d, dim=2))
+    k = torch.cat([k_ring[:, slots].double().view(B, -1, H, hd), kn], 1)
+    v = torch.cat([v_ring[:, slots].double().view(B, -1, H, hd), vn], 1)
+    s = cap * torch.tanh(torch.einsum("bqhc,bkhc->bhk", q, k) * hd ** -0.5 / cap)
+    s = s - slopes.double()[None, :, None] * (t - torch.tensor(keys + [t], device=dev(), dtype=torch.float64))
+    ref = torch.einsum("bhk,bkhc->bhc", s.softmax(-1), v).reshape(B, d)
+    y = ops.swa_forward(qkv, k_ring, v_ring, pos, slopes, H, window, cap, update_cache=True)
+    close(y.view(B, d), ref, 1e-5 if dt == torch.float32 else 1e-2)
+    assert pos[:, 0].tolist() == [t + 1] * B and pos[0, 1].item() == 0
+    assert torch.equal(k_ring[:, t % W], qkv[:, 0, d:2 * d]) and torch.equal(v_ring[:, t % W], qkv[:, 0, 2 * d:])
+
+
 @pytest.mark.parametrize("epi", [0, 1, 2])
 @pytest.mark.parametrize("M,N,K", [(1, 128, 8), (128, 136, 64), (129, 256, 72), (255, 128, 136), (256, 264, 128), (257, 128, 192),
                                    (512, 2560, 200), (2600, 2048, 64), (19200, 264, 128)])
