@@ -136,6 +136,9 @@ extern "C" int stu_linear_can_fuse_norm(int M, int N, int K, int epilogue, int d
   // gate/up kernel from its shared-memory copy); a separate norm kernel measured faster both times (24-layer model,
   // B = 32: 2.17 against 2.27 ms per token step, and 2.19 against 2.30 ms).  The kernels accept norm_w all the same.
   // (a fused norm inside the tcgen05 token-step kernel measured slower as well: 2.12-2.25 against 1.71-1.85 ms)
-  if (M > 16) return 0;
+  // 9..16 rows: the fused form is the weight-streaming kernel, the other the tcgen05 one behind a norm kernel, which is faster from
+  // 2.6 M weights on (us, 12 rows, fused and apart: 2304 x 768 4.1 and 5.0, gate/up 2048 x 512 3.6 and 5.1, 2560 x 640 6.7 and 5.7, 3072 x 768 7.4 and
+  // 6.0; 3072 x 1024 7.4 and 5.5, 4608 x 1536 16.8 and 7.4, gate/up 6144 x 1536 19.0 and 10.8)
+  if (M > 16 || (M > 8 && (long long)N * K * (epilogue == EPI_GELU_MUL ? 2 : 1) > 2600000)) return 0;
   return 1;
 }
