@@ -97,6 +97,8 @@ _SIGNATURES = {
                          _P], c_int),
     "stu_decode_approx_projected": ([_P, _LL, _P, _LL, _P, _P, _P, _P, _LL, c_int, c_int, c_int, c_int, _P, c_int, _P],
                                     c_int),
+    "stu_stream_ahead": ([_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, _P, c_int, _P], c_int),
+    "stu_stream_finish": ([_P, _P, _P, _P, _P, _P, _P, _P, c_float, _P, _P, c_int, c_int, c_int, _P, c_int, _P], c_int),
     "stu_peer_dest_bytes": ([], c_int),
     "stu_peer_alloc": ([_P, _LL], c_int),
     "stu_peer_free": ([_P], c_int),

@@ -222,7 +222,7 @@ PyMethodDef methods[] = {
     ENTRY(stu_conv_prefill_approx_tc5),
     ENTRY(stu_decode_approx),
     ENTRY(stu_decode_approx_pipelined),
-    ENTRY(stu_decode_approx_projected),
+    ENTRY(stu_decode_approx_projected), ENTRY(stu_stream_ahead), ENTRY(stu_stream_finish),
     ENTRY(stu_decode_approx_push),
     ENTRY(stu_decode_approx_shard),
     ENTRY(stu_embed),

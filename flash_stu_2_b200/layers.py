@@ -118,6 +118,11 @@ class STULayer(nn.Module):
         x2 = x.view(B, d)
         stu, mlp = child(self, "stu"), child(self, "mlp")
         stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
+        ahead = getattr(entry[1], "_stream_ahead", None)
+        if ahead is not None:   # a captured step whose history sums were computed beside the step before (stream_ahead.py)
+            xn = stu.stream_step(x2, param(stu_norm, "weight"), stu_norm.eps, entry, mid, ahead, param(mlp_norm, "weight"), mlp_norm.eps)
+            mlp.apply_residual(xn, mid, x2, overlap=True)
+            return entry
         if stu.use_approx:
             entry = stu.decode_step(x2, param(stu_norm, "weight"), stu_norm.eps, entry, mid)
         else:

@@ -8,6 +8,7 @@ can observe, all forced by the reference's own gaps:
   * sampling draws by inverse CDF from one uniform per sequence (optionally passed as
     `uniforms=[steps,B]` or drawn from `generator=`) instead of torch.multinomial.
 """
+import contextlib
 import gc
 import threading
 from typing import Any, Dict, Optional, Tuple
@@ -23,6 +24,7 @@ from .config import FlashSTUConfig
 from .filters import get_spectral_filters, nearest_power_of_two
 from .layers import AttentionLayer, STULayer
 from .modules import STU, Attention, RMSNorm
+from .stream_ahead import StreamAhead
 from .token_step import TokenStep
 
 
@@ -276,7 +278,8 @@ class FlashSTU(PreTrainedModel):
                 if graph is None:
                     tok = generated[:, cur - 1:cur].clone()   # the step reads its token here and leaves the next one
                     u_buf = torch.zeros(B, dtype=torch.float32, device=dev)
-                    graph, logits_g, buffers = self._capture_step(tok, past, temperature, top_k, top_p, do_sample, u_buf)
+                    graph, logits_g, buffers = self._capture_step(tok, past, temperature, top_k, top_p, do_sample, u_buf,
+                                                                  max_length - 2)
                 if timings is not None and ev_first is None:
                     ev_first = torch.cuda.Event(enable_timing=True)
                     ev_first.record()
@@ -312,10 +315,10 @@ class FlashSTU(PreTrainedModel):
             return generated, all_logits if stepper is not None else torch.stack(all_logits, dim=1)
         return generated
 
-    def _capture_step(self, tok, past, temperature, top_k, top_p, do_sample, u_buf):
-        """One cached token step (token in `tok`, next token left there) as a CUDA graph.  The step's outputs live in one
-        buffer of the caller, so that capturing needs neither a private memory pool nor the collection and cache flush
-        that go with one (together 0.1 to 0.8 s on a busy process)."""
+    def _capture_step(self, tok, past, temperature, top_k, top_p, do_sample, u_buf, last):
+        """One cached token step (token in `tok`, next token left there; to be replayed up to position `last`) as a CUDA graph.
+        The step's outputs live in one buffer of the caller, so that capturing needs neither a private memory pool nor the
+        collection and cache flush that go with one (together 0.1 to 0.8 s on a busy process)."""
         B, d = tok.shape[0], self.config.n_embd
         row = max(3 * d, d + max(layer.mlp.intermediate_size for layer in self.layers))
         # (full variant: U+-, the operand of the contraction with M_phi)
@@ -327,19 +330,25 @@ class FlashSTU(PreTrainedModel):
         host_t = [getattr(e[-1], "_host_t", None) if e is not None else None for e in past]
         graph = torch.cuda.CUDAGraph()
         stream, here = torch.cuda.Stream(tok.device), torch.cuda.current_stream(tok.device)
-        stream.wait_stream(here)
-        with _CollectionHeld(), torch.cuda.stream(stream), ops.arena(buffer):
-            graph.capture_begin(capture_error_mode="thread_local")
-            try:
-                logits, _ = self.last_logits(tok, past, True)
-                ops.sample(logits, temperature, top_k, top_p, do_sample, u_buf if do_sample else None, tok, out_stride=1)
-            finally:
-                graph.capture_end()
-        here.wait_stream(stream)
+        ahead = StreamAhead.plan(self.layers, past, B, last, sum(p.numel() * p.element_size() for p in self.parameters()))
+        with ahead if ahead is not None else contextlib.nullcontext():
+            stream.wait_stream(here)
+            with _CollectionHeld(), torch.cuda.stream(stream), ops.arena(buffer):
+                graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    if ahead is not None:
+                        ahead.branch(stream)
+                    logits, _ = self.last_logits(tok, past, True)
+                    ops.sample(logits, temperature, top_k, top_p, do_sample, u_buf if do_sample else None, tok, out_stride=1)
+                    if ahead is not None:
+                        ahead.join(stream)
+                finally:
+                    graph.capture_end()
+            here.wait_stream(stream)
         for e, t in zip(past, host_t):   # capturing ran the host bookkeeping, not the kernels
             if e is not None and t is not None:
                 e[-1]._host_t = t
-        return graph, logits, (buffer, stream)
+        return graph, logits, (buffer, stream, ahead)
 
     def prepare_inputs_for_generation(self, input_ids, past_key_values=None, attention_mask=None, use_cache=None,
                                       **kwargs) -> Dict[str, Any]:

@@ -391,12 +391,7 @@ class STU(nn.Module):
                 and STU.shared_tap_decode and taps8 is not None and uniform_pos(pos) and d % 8 == 0
                 and x2d.shape[1] % 8 == 0):
             # larger batches: the projection of the whole batch as one GEMM, then the pipeline kernel as a pure stream
-            if ops.can_fuse_norm(B, d, x2d.shape[1], ops.EPI_STORE, x2d.dtype):
-                xp = ops.linear(x2d, MinT, norm_w=norm_w, eps=eps)
-            else:
-                # token step: MinT is nobody's output here, so its tiles may be requested while the norm kernel runs
-                xp = ops.linear(ops.rmsnorm(x2d, norm_w, eps), MinT,
-                                epilogue=ops.EPI_STORE | (ops.FLAG_OVERLAP if ops.overlap_decode else 0))
+            xp = self.project_step(x2d, norm_w, eps, MinT)
             ops.decode_approx_projected(x2d, xp, hist, taps8, pos, out2d)
         elif (STU.pipelined_decode and STU.tensor_core_decode and STU.shared_tap_decode and taps8 is not None
                 and uniform_pos(pos) and d % 8 == 0 and x2d.shape[1] % 8 == 0
@@ -412,6 +407,24 @@ class STU(nn.Module):
                                     (ops.FLAG_UNIFORM_POS if (uniform_pos(pos) and STU.shared_tap_decode) else 0))
         pos._host_t = t + 1
         return hist, pos
+
+    @staticmethod
+    def project_step(x2d, norm_w, eps: float, MinT):
+        """The projected input of a token step of a larger batch, as one GEMM."""
+        if ops.can_fuse_norm(x2d.shape[0], MinT.shape[0], x2d.shape[1], ops.EPI_STORE, x2d.dtype):
+            return ops.linear(x2d, MinT, norm_w=norm_w, eps=eps)
+        # token step: MinT is nobody's output here, so its tiles may be requested while the norm kernel runs
+        return ops.linear(ops.rmsnorm(x2d, norm_w, eps), MinT,
+                          epilogue=ops.EPI_STORE | (ops.FLAG_OVERLAP if ops.overlap_decode else 0))
+
+    def stream_step(self, x2d, norm_w, eps: float, entry, out2d, ahead, next_norm_w, next_eps: float):
+        """decode_step where `ahead` = (part, ctl) holds the history sums of the position, with the norm behind it (returned)."""
+        hist, pos = entry
+        MinT, _, taps8 = self.prepared()
+        xp = self.project_step(x2d, norm_w, eps, MinT)
+        xn = ops.stream_finish(x2d, xp, hist, taps8, pos, *ahead, next_norm_w, next_eps, out2d)
+        pos._host_t = host_pos(pos) + 1
+        return xn
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if not self.use_approx:

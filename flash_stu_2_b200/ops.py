@@ -390,6 +390,39 @@ def decode_approx_projected(x, xp, hist, taps8, pos, out, add_residual: bool = T
     return out
 
 
+def stream_ahead(hists, taps8s, part, ctl, sms: int):
+    """Sums over the history of the next position (ctl[0]) of several approx STU layers at one position, on `sms` SMs; part
+    [layers,2,B,d] fp32, ctl [4] int32 (see stu_b200.h)."""
+    _cuda(part, ctl, *hists, *taps8s)
+    B, d, _, Lh = hists[0].shape
+    n = len(hists)
+    assert all(h.shape == hists[0].shape and h.is_contiguous() for h in hists) and part.shape == (n, 2, B, d)
+    assert all(w.shape == (8, d, Lh + 8) and w.is_contiguous() for w in taps8s) and len(taps8s) == n
+    assert part.is_contiguous() and part.dtype == torch.float32 and ctl.dtype == torch.int32 and ctl.numel() == 4
+    h = (ctypes.c_void_p * n)(*[t.data_ptr() for t in hists])
+    w = (ctypes.c_void_p * n)(*[t.data_ptr() for t in taps8s])
+    rc = _lib.native().stu_stream_ahead(ctypes.addressof(h), ctypes.addressof(w), n, part.data_ptr(), ctl.data_ptr(), B, d, Lh, sms,
+                                        status_word(part.device).data_ptr(), _dt(hists[0]), _stream())
+    _lib.check(rc, "stu_stream_ahead")
+    _count()
+
+
+def stream_finish(x, xp, hist, taps8, pos, part, ctl, norm_w, eps: float, out):
+    """The layer's own part of a token step whose history sums stream_ahead has left in `part` [2,B,d]: append, out = x + STU, and
+    the norm behind it, which is returned."""
+    _cuda(x, xp, hist, taps8, pos, part, ctl, norm_w, out)
+    B, d, _, Lh = hist.shape
+    assert x.shape == (B, d) and xp.shape == (B, d) and out.shape == (B, d) and part.shape == (2, B, d)
+    assert all(t.is_contiguous() for t in (x, xp, hist, taps8, pos, part, norm_w, out)) and pos.shape == (B, 2)
+    xn = empty((B, d), x.dtype, x.device)
+    rc = _lib.native().stu_stream_finish(x.data_ptr(), xp.data_ptr(), hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), part.data_ptr(),
+                                         ctl.data_ptr(), norm_w.data_ptr(), eps, out.data_ptr(), xn.data_ptr(), B, d, Lh,
+                                         status_word(x.device).data_ptr(), _dt(x), _stream())
+    _lib.check(rc, "stu_stream_finish")
+    _count()
+    return xn
+
+
 def linear_push(x: torch.Tensor, W: torch.Tensor, dest: int, dest_row_stride: int):
     """x[M,K] @ W[N,K]^T stored into every tensor-parallel rank's inbox through the exchange descriptor at device
     address `dest` (peer.PeerExchange.dest); M <= 64, bf16."""

@@ -295,6 +295,19 @@ int stu_decode_approx_projected(const void* x, long long x_row_stride, const voi
                                 void* hist, const void* taps8, int* pos, void* out, long long out_row_stride, int B,
                                 int d_ch, int Lh, int add_residual, int* status, int dtype, void* stream);
 
+/* The sums over the history of the NEXT position of `layers` approx STU layers (bf16, up to 64 of them, all of B sequences and d
+ * channels at one position), as one launch on `sms` SMs beside the current step: hist[i] / taps8[i] (host arrays of device
+ * pointers) as in stu_decode_approx_pipelined, part [layers][2][B][d] fp32, ctl [4] = {position to compute (advanced by the launch),
+ * 0, position that part[.][0] holds, the same for part[.][1]}; ctl[2 + (t & 1)] has to be t - 2 when position t is computed.
+ * stu_stream_finish is the layer's own part of the step, for the position t that ctl says `part` (the layer's, [2][B][d]) holds
+ * (status 8 otherwise): appends xp [B,d] (the projected input) to hist, out = x + round(2 * (part + xp * tap_0)),
+ * xn = rmsnorm(out) * norm_w, advances pos.  d <= 4096; x, xp, out, xn dense rows; the step of flash_stu/modules/stu.py:85-98,120. */
+int stu_stream_ahead(const void* const* hist, const void* const* taps8, int layers, float* part, int* ctl, int B, int d,
+                     int Lh, int sms, int* status, int dtype, void* stream);
+int stu_stream_finish(const void* x, const void* xp, void* hist, const void* taps8, int* pos, const float* part,
+                      const int* ctl, const void* norm_w, float eps, void* out, void* xn, int B, int d, int Lh,
+                      int* status, int dtype, void* stream);
+
 /* Attention of a prefill that starts at position 0 (every pos[2b] == 0, checked on the device: status 11 otherwise)
  * on the tcgen05 tensor cores: bf16, head dimension 64 or 128.  Same semantics and outputs as stu_swa_forward for that
  * case (flash_stu/modules/attention.py:72-101): 128 queries x one head per CTA, S = Q K^T and O += P V as

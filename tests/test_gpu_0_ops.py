@@ -667,6 +667,56 @@ def test_single_launch_exchange_kernel_with_the_other_ranks_stood_in_by_host_cop
             ex.close()
 
 
+@pytest.mark.parametrize("B,d,L,t,layers,sms", [(17, 64, 1100, 510, 3, 5), (16, 128, 600, 0, 1, 200), (8, 8, 2000, 1023, 2, 1), (33, 256, 1100, 1090, 2, 7),
+                                                (16, 1032, 300, 297, 1, 148)])
+def test_history_sums_ahead_of_the_step(B, d, L, t, layers, sms):
+    """stream_ahead + stream_finish against the pipeline kernel and the norm kernel, bit for bit, over four steps: sequences that
+    fill no group of eight, one to several slices, an odd number of rows per SM, positions up to the end of the capacity (where there
+    is no next one).  The history past the position holds NaN."""
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.modules import new_pos
+    g = torch.Generator(device=dev()).manual_seed(B + d + t)
+    rand = lambda *s: torch.randn(*s, device=dev(), generator=g).bfloat16()
+    Lh = (L // 2 + 7) // 8 * 8
+    cap = 2 * Lh
+    t = min(t, cap - 4) if t > 1024 else t
+    hists, taps8s = [], []
+    for _ in range(layers):
+        h = rand(B, d, 2, Lh)
+        h[:, :, 0, (t + 1) // 2:] = float("nan")
+        h[:, :, 1, t // 2:] = float("nan")
+        hists.append(h)
+        taps8s.append(ops.taps_rev8(rand(d, Lh)))
+    twins = [h.clone() for h in hists]
+    pos = [new_pos(B, dev()) for _ in range(2 * layers)]
+    for p in pos:
+        p[:, 0] = t
+    norm_w = rand(d)
+    part = torch.full((layers, 2, B, d), float("nan"), device=dev())
+    ctl = torch.tensor([t, 0] + ([t - 2, t - 1] if t % 2 == 0 else [t - 1, t - 2]), dtype=torch.int32, device=dev())
+    ops.stream_ahead(hists, taps8s, part, ctl, sms)
+    for step in range(4):
+        ops.stream_ahead(hists, taps8s, part, ctl, sms)      # of position t + step + 1: ahead of this step's appends
+        for i in range(layers):
+            x, xp = rand(B, d), rand(B, d)
+            want, out = torch.empty_like(x), torch.empty_like(x)
+            ops.decode_approx_projected(x, xp, twins[i], taps8s[i], pos[2 * i], want)
+            xn = ops.stream_finish(x, xp, hists[i], taps8s[i], pos[2 * i + 1], part[i], ctl, norm_w, 1e-6, out)
+            ops.check_status()
+            assert torch.equal(out, want) and torch.equal(xn, ops.rmsnorm(want, norm_w, 1e-6)), (step, i)
+            assert torch.equal(pos[2 * i], pos[2 * i + 1]) and pos[2 * i + 1][0].tolist() == [t + step + 1, 0]
+    for a, b in zip(hists, twins):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    # sums of another position are refused, nothing is appended
+    ctl[2:] = -1
+    if t + 4 < cap:
+        before = hists[0].clone()
+        ops.stream_finish(x, xp, hists[0], taps8s[0], pos[1], part[0], ctl, norm_w, 1e-6, out)
+        with pytest.raises(RuntimeError, match="status 8"):
+            ops.check_status()
+        assert torch.equal(hists[0].view(torch.int16), before.view(torch.int16)) and pos[1][0, 0].item() == t + 4
+
+
 @pytest.mark.parametrize("shape", [(17, 60, 256, 300), (32, 40, 128, 700), (9, 530, 64, 1100)])
 def test_decode_step_with_the_projection_done_by_the_caller(shape):
     """Larger batches: rmsnorm + one GEMM give the projected input of the whole batch, the pipeline kernel only appends

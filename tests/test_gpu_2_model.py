@@ -364,6 +364,31 @@ def test_the_three_forms_of_the_token_loop_agree(monkeypatch, dt, kw):
         close(logits[:, :same], eager_logits[:, :same], 2e-2)
 
 
+@pytest.mark.parametrize("B,T0,new,sms", [(17, 30, 34, 9), (19, 1, 63, 40), (32, 33, 12, 148)])
+def test_streams_beside_the_captured_step(monkeypatch, B, T0, new, sms):
+    """The captured step with its STU layers' history sums on a branch of their own draws the same tokens from the same logits as the
+    one whose layers stream for themselves, up to the last position of the capacity; a second call on the model does too.  (From 17
+    sequences on both forms norm in a kernel of its own.)"""
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.stream_ahead import StreamAhead
+    m = _random_model(256, 4, torch.bfloat16)
+    prompt = torch.randint(0, 1003, (B, T0), device=dev())
+    kw = dict(max_length=T0 + new, do_sample=False, return_logits=True)
+    monkeypatch.setattr(StreamAhead, "enabled", False)
+    want_ids, want = m.generate(prompt, **kw)
+    monkeypatch.setattr(StreamAhead, "enabled", True)
+    monkeypatch.setattr(StreamAhead, "sms", staticmethod(lambda *a: sms))
+    launches = []
+    ahead = ops.stream_ahead
+    monkeypatch.setattr(ops, "stream_ahead", lambda *a: (launches.append(a[-1]), ahead(*a)))
+    for _ in range(2):
+        del launches[:]
+        ids, logits = m.generate(prompt, **kw)
+        ops.check_status()
+        assert launches == [torch.cuda.get_device_properties(0).multi_processor_count, sms]
+        assert torch.equal(ids, want_ids) and torch.equal(logits, want)
+
+
 @pytest.mark.parametrize("where", ["attn_norm", "mlp_norm", "attn.c_attn", "mlp.gate_proj", "mlp.down_proj"])
 def test_fp32_steps_with_weights_off_the_16_byte_grid(where):
     """fp32 steps fuse the norm into the linears, whose kernel reads 16 bytes at a time: parameters that start elsewhere (views

@@ -171,3 +171,13 @@ def test_tagged_words_are_read_in_elements_of_the_stores_width():
         loads = re.findall(r"ld\.relaxed\.gpu\.global\.v(\d)\.[ub](\d+)", body)
         assert stores == [bits] and loads == [(str(128 // int(bits)), bits)], (dt, stores, loads)
     assert len(re.findall(r"ld\.relaxed\.gpu\.global", text)) == 2   # nobody else reads them
+
+
+def test_sms_for_the_streams_beside_a_step():
+    """What decides whether and on how many SMs a captured step's history streams run beside it: none for a few short streams, never
+    more than a third of the GPU, more for longer histories."""
+    from flash_stu_2_b200.stream_ahead import StreamAhead
+    big = lambda t: StreamAhead.sms(24, 12, 32, 1536, t, 1_800_000_000, 2_400_000_000, 148)
+    assert StreamAhead.sms(4, 2, 16, 512, 300, 60_000_000, 10_000_000, 148) == 0
+    assert 18 <= big(2176) <= 26 and big(500) == 8 and big(8000) == 49
+    assert all(0 < big(t) <= big(t + 512) for t in range(256, 7600, 256))
