@@ -482,6 +482,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
 #pragma unroll 1
       for (int nb = n0 + 64 * half; nb < min(n0 + BN, N); nb += 128) {
         const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
+        const bool shifted = EPI == EPI_STORE && unaligned && nb + 64 <= N && K <= 768;
 #pragma unroll 1
         for (int h = 0; h < 2; h++) {   // 32 columns of this thread's row
           uint32_t r[32], r2[32];
@@ -507,7 +508,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
               store_vec(at(lane, h * 4 + v8), o);
             }
           }
-          if (unaligned) {   // 32 columns at a time: the stores of one half run beside the accumulator read of the next
+          if (unaligned && !shifted) {   // 32 columns at a time: the stores of one half run beside the accumulator read of the next
             __syncwarp();
             const int n = nb + h * 32 + lane;
             if (n < N) {
@@ -526,6 +527,41 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
           }
         }
         __syncwarp();
+        if (shifted) {
+          // Plain rows off the 16-byte grid (an odd vocabulary): the 16-byte pieces of the row's memory lie s values into those of the
+          // block.  A lane takes its piece and its neighbour's and shifts out the eight values that one store takes; the s values
+          // ahead of the first such piece and the 8 - s behind the last are stored singly.  Logits of 834 x 50257 x 512 67 -> 58 us, 1668
+          // x 50257 x 768 136 -> 132; from K = 1024 on the main loop hides the single stores, which then cost less: 7996 x 50257 x 1024
+          // 724 us with them, 745 without.
+          const int piece = lane & 7, r0 = lane >> 3;
+          const size_t base = (reinterpret_cast<uintptr_t>(ep.y) >> 1) + nb;
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const int row = r0 + i * 4;
+            const size_t off = (size_t)(first + row) * ep.ldy;
+            const int s = (int)(8 - ((base + off) & 7)) & 7;
+            const uint4 v = *reinterpret_cast<const uint4*>(at(row, piece));
+            uint32_t w[8] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[4 + j] = __shfl_down_sync(0xffffffffu, w[j], 1);
+#pragma unroll
+            for (int j = 0; j < 6; j++) w[j] = s & 4 ? w[j + 2] : w[j];
+#pragma unroll
+            for (int j = 0; j < 5; j++) w[j] = s & 2 ? w[j + 1] : w[j];
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[j] = __funnelshift_r(w[j], w[j + 1], s & 1 ? 16 : 0);
+            if (row < rows && (s == 0 || piece < 7))
+              *reinterpret_cast<uint4*>(ep.y + off + nb + piece * 8 + s) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const int row = i * 4 + (lane >> 3), j = lane & 7;
+            const size_t off = (size_t)(first + row) * ep.ldy;
+            const int s = (int)(8 - ((base + off) & 7)) & 7;
+            const int col = j < s ? j : 56 + j;
+            if (row < rows && s != 0) ep.y[off + nb + col] = at(row, col >> 3)[col & 7];
+          }
+        }
         if (!unaligned) {
           const int piece = lane & 7, r0 = lane >> 3;   // 8 values of row r0, r0 + 4, ...
           const int n = nb + piece * 8;
@@ -715,11 +751,11 @@ unsigned long long g_wait_ns = 2000000000ull;
 
 // Row by row while the whole B operand stays in L2 (up to 48 MB, a share of the 126 MB that the rows of A and the
 // output leave alone) or has so few column tiles that the tiles in flight cover several row tiles anyway.  Otherwise
-// bands of 16 row tiles: the ~148 tiles in flight then cover 16 row tiles x 9 column tiles and a wave reads 16 * 128
-// rows of A and 9 * 256 rows of B instead of all of B.  Gate/up of d = 3072 (75 MB of weights, 96 column tiles, 32768
-// rows): 4.6 -> 3.4 ms.  Below the lines the bands cost 1 % (gate/up of d = 1024) to 2.5 % (6000 x 1024 x 49152).
+// bands of 16 row tiles of 256: a wave then reads 16 * 256 rows of A and few column tiles instead of all of B.  us, row by row and bands
+// of 8, 16, 32: gate/up 32768 x 12288 x 3072 4547, 3608, 3620, 3796; 32768 x 9216 x 3072 1413, 1406, 1354, 1415; 7996 x 50257 x 1024 967, 750,
+// 736, 725.  Below the lines bands of 16 cost 0 (gate/up of d = 1536) to 7 % (65536 x 1536 x 6144).
 int gemm_group_m(int tiles_n, int N, int K, bool dual) {
-  return tiles_n > 24 && (long long)N * K * (dual ? 4 : 2) > (48ll << 20) ? 8 : 1;
+  return tiles_n > 24 && (long long)N * K * (dual ? 4 : 2) > (48ll << 20) ? 16 : 1;
 }
 
 // Pairs of CTAs that the current device runs at a time.

@@ -210,6 +210,22 @@ def test_linear_cuda_core_tiles_skip_what_a_triangular_weight_leaves_out(dt, sha
     ops.check_status()
 
 
+@pytest.mark.parametrize("K", [768, 776])
+@pytest.mark.parametrize("N,ld,at", [(257, 259, 3), (640, 645, 7), (71, 77, 0), (320, 322, 1)])
+def test_linear_odd_rows_by_shifted_pieces_and_singly(N, ld, at, K):
+    """Rows off the 16-byte grid on either side of the K from which they are stored value by value: every phase of a row against the
+    16-byte pieces of memory, blocks of 64 columns and the columns behind the last; nothing is written between the rows."""
+    from flash_stu_2_b200 import ops
+    g = torch.Generator(device=dev()).manual_seed(N + K)
+    x, W = torch.randn(300, K, device=dev(), generator=g).bfloat16(), (torch.randn(N, K, device=dev(), generator=g) / math.sqrt(K)).bfloat16()
+    buf = torch.full((300 * ld + at,), 7.0, dtype=torch.bfloat16, device=dev())
+    y = buf[at:].view(300, ld)
+    ops.linear(x, W, out=y[:, :N], backend=ops.BACKEND_TCGEN05)
+    ops.check_status()
+    close(y[:, :N], _lin_ref(x, W, None, None, 0, torch.bfloat16), 2 ** -7)   # the next value of an output at most
+    assert bool((y[:, N:] == 7.0).all()) and bool((buf[:at] == 7.0).all())
+
+
 @pytest.mark.parametrize("shape", [(129, 257, 64, 257), (300, 71, 72, 75), (65, 4097, 128, 4097), (2500, 5121, 64, 5121)])
 def test_linear_output_rows_off_the_16_byte_grid(shape):
     """Plain stores of the tcgen05 GEMM to rows of any stride (an odd vocabulary), square and wide tiles; nothing is
