@@ -2,22 +2,34 @@
 // (flash_stu/modules/stu.py:100-118; MiniSTU mini_stu/stu.py:240-269):
 //   U+-[b,t,k,i] = E +- Q,   E = sum_{j even} phi[j,k] x[b,t-j,i],   Q the same over odd j.
 //
-// Bound: FFMA issue.  Filter by filter (Toeplitz matrices, three GEMMs with them, a combine pass) this was 120 launches
+// Bound: FMA issue.  Filter by filter (Toeplitz matrices, three GEMMs with them, a combine pass) this was 120 launches
 // of 3 to 16 us for 24 filters, E and Q went through memory, and a triangle's empty half was computed tile by tile.
 // Here a CTA owns 64 time indices m (t = 2m and 2m + 1) of 4 * TX channels under one filter, a thread 4 x 4 of them with
 // four sums each: E and Q of both parities share the inputs xe[s] = x[2s], xo[s] = x[2s+1] and their taps
 //   E_even += f[2(m-s)] xe[s]   E_odd += f[2(m-s)] xo[s]   Q_odd += f[2(m-s)+1] xe[s]   Q_even += f[2(m-s)-1] xo[s].
-// A thread's taps slide by one as s advances, so a step of s costs 64 FMAs, two 16-byte reads of the inputs and two
-// words of taps.  Sums over s run in order, as the GEMMs' did.  24 filters, 8 x 1000 positions of 64 channels: 1.35 -> 0.40 ms
-// (29 TFLOP/s of the causal half).
+// Two channels at a time (fma.rn.f32x2: inputs are pairs as they lie, taps are staged twice), which takes half the issue slots;
+// a thread's taps slide by one as s advances, so a step of s is 32 such instructions, two 16-byte reads of the inputs and two 8-byte
+// ones of the taps.  Sums over s run in order, as the GEMMs' did.  24 filters, 8 x 1000 positions of 64 channels: 1.35 ms; one product
+// at a time, 64 channels a CTA, copies' addresses worked out for every step 0.40; in pairs at 32 channels (three CTAs per SM) 0.36;
+// addresses once and all long sums ahead of all short ones 0.32; the 32 steps unrolled, so that the sliding costs no moves,
+// 0.28 (42 TFLOP/s of the causal half; the pairs' issue rate alone would be 0.20).
 #include "common.cuh"
 
 namespace {
 
+typedef unsigned long long f32x2;   // two fp32 values of one register pair
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) { return (f32x2)__float_as_uint(hi) << 32 | __float_as_uint(lo); }
+__device__ __forceinline__ float half_of(f32x2 v, int hi) { return __uint_as_float((uint32_t)(hi ? v >> 32 : v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 constexpr int MT = 64, ST = 32;   // time indices per CTA, inputs per step of the pipeline
 
 template <int TX>
-__global__ void __launch_bounds__(TX * 16, 32 / TX) full_conv_kernel(const float* __restrict__ hist, int Lh,
+__global__ void __launch_bounds__(TX * 16, 24 / TX) full_conv_kernel(const float* __restrict__ hist, int Lh,
                                                             const float* __restrict__ phi, int L, int K,
                                                             float* __restrict__ U, long long ldU, int rows, int d,
                                                             int both, int t0, int t_end, int tiles_m) {
@@ -27,32 +39,48 @@ __global__ void __launch_bounds__(TX * 16, 32 / TX) full_conv_kernel(const float
   constexpr int QT = (NT + THREADS - 1) / THREADS;
   static_assert(QX * 4 * THREADS == 2 * CT * ST, "thread layout");
   __shared__ __align__(16) float xs[2][2][ST][PX];   // [buffer][parity][s][channel]
-  __shared__ float taps[2][NT];
+  __shared__ f32x2 taps[2][NT];                      // each twice: both halves of an operand
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-  const int k = blockIdx.z, c0 = blockIdx.y * CT;
-  const int tm = tiles_m - 1 - (int)blockIdx.x;      // the longest sums first
+  const int k = blockIdx.x % K, c0 = blockIdx.x / K * CT;
+  const int tm = tiles_m - 1 - (int)blockIdx.y;      // the longest sums of all channels and filters first
   const int m0 = (t0 >> 1) + tm * MT;
   const int s_end = min(m0 + MT, (t_end + 1) >> 1);  // inputs that some output of the tile needs
 
+  // this thread's pieces: one channel, QX times four inputs; QT taps
   float rx[QX][4], rt[QT];
+  const bool mine = c0 + tid % CT < rows;
+  const float* src[QX];
+  int from[QX], tap_at[QT];
+  const float* tap[QT];
+#pragma unroll
+  for (int i = 0; i < QX; i++) {
+    const int q = (tid + i * THREADS) / CT, p = q / (ST / 4);
+    from[i] = 2 * (q % (ST / 4) * 4) + p;   // time of the first of the four inputs, less 2 s0
+    src[i] = hist + ((size_t)(c0 + (mine ? tid % CT : 0)) * 2 + p) * Lh + q % (ST / 4) * 4;
+  }
+#pragma unroll
+  for (int i = 0; i < QT; i++) {   // even[e] = f[2 (m0 - s0 - ST + e)], odd[e] = f[2 (m0 - s0 - ST + e) + 1]
+    const int e = tid + i * THREADS, odd = e >= MT + ST;
+    tap_at[i] = e < NT ? 2 * (m0 - ST + e - odd * (MT + ST)) + odd : -1;
+    tap[i] = phi + (long long)tap_at[i] * K + k;
+  }
   auto fetch = [&](int s0) {
+    if (2 * (s0 + ST) <= t_end) {   // (rows of the history are 16-byte aligned)
 #pragma unroll
-    for (int i = 0; i < QX; i++) {
-      const int e = tid + i * THREADS, c = e % CT, q = e / CT, p = q / (ST / 4), s = s0 + q % (ST / 4) * 4;
-      const float* src = hist + ((size_t)(c0 + c) * 2 + p) * Lh + s;
-      if (c0 + c < rows && 2 * (s + 3) + p < t_end) {   // (rows of the history are 16-byte aligned)
-        const float4 v = *reinterpret_cast<const float4*>(src);
+      for (int i = 0; i < QX; i++) {
+        const float4 v = mine ? *reinterpret_cast<const float4*>(src[i] + s0) : make_float4(0.f, 0.f, 0.f, 0.f);
         rx[i][0] = v.x; rx[i][1] = v.y; rx[i][2] = v.z; rx[i][3] = v.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; j++) rx[i][j] = (c0 + c < rows && 2 * (s + j) + p < t_end) ? src[j] : 0.f;
       }
+    } else {
+#pragma unroll
+      for (int i = 0; i < QX; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) rx[i][j] = (mine && from[i] + 2 * (s0 + j) < t_end) ? src[i][s0 + j] : 0.f;
     }
 #pragma unroll
-    for (int i = 0; i < QT; i++) {   // even[e] = f[2 (m0 - s0 - ST + e)], odd[e] = f[2 (m0 - s0 - ST + e) + 1]
-      const int e = tid + i * THREADS, odd = e >= MT + ST;
-      const int j = 2 * (m0 - s0 - ST + e - odd * (MT + ST)) + odd;
-      rt[i] = (e < NT && j >= 0 && j < L) ? phi[(size_t)j * K + k] : 0.f;
+    for (int i = 0; i < QT; i++) {
+      const int j = tap_at[i] - 2 * s0;
+      rt[i] = (j >= 0 && j < L) ? *(tap[i] - 2ll * s0 * K) : 0.f;
     }
   };
   auto stage = [&](int buf) {
@@ -64,14 +92,14 @@ __global__ void __launch_bounds__(TX * 16, 32 / TX) full_conv_kernel(const float
     }
 #pragma unroll
     for (int i = 0; i < QT; i++)
-      if (tid + i * THREADS < NT) taps[buf][tid + i * THREADS] = rt[i];
+      if (tid + i * THREADS < NT) taps[buf][tid + i * THREADS] = pair_of(rt[i], rt[i]);
   };
 
-  float ee[4][4], eo[4][4], qo[4][4], qe[4][4];   // [m][channel]
+  f32x2 ee[4][2], eo[4][2], qo[4][2], qe[4][2];   // [m][pair of channels]
 #pragma unroll
   for (int i = 0; i < 4; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) ee[i][j] = eo[i][j] = qo[i][j] = qe[i][j] = 0.f;
+    for (int j = 0; j < 2; j++) ee[i][j] = eo[i][j] = qo[i][j] = qe[i][j] = 0;
 
   fetch(0);
   stage(0);
@@ -80,32 +108,31 @@ __global__ void __launch_bounds__(TX * 16, 32 / TX) full_conv_kernel(const float
     const bool more = s0 + ST < s_end;
     if (more) fetch(s0 + ST);
     // taps of m = m0 + 4 ty + i against s = s0 + u: even[ST + 4 ty + i - u], odd the same index and the one below
-    const float* te = taps[buf] + ST + 4 * ty;
-    const float* to = te + MT + ST;
-    float t4[4], o[4];
+    const f32x2* te = taps[buf] + ST + 4 * ty;
+    const f32x2* to = te + MT + ST;
+    f32x2 t4[4], o[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       t4[i] = te[i];
       o[i] = to[i];
     }
-#pragma unroll 4
+#pragma unroll
     for (int u = 0; u < ST; u++) {
-      const float below = to[-1 - u];
-      float xe[4], xo[4];
-      *reinterpret_cast<float4*>(xe) = *reinterpret_cast<const float4*>(&xs[buf][0][u][tx * 4]);
-      *reinterpret_cast<float4*>(xo) = *reinterpret_cast<const float4*>(&xs[buf][1][u][tx * 4]);
-      const float od[5] = {below, o[0], o[1], o[2], o[3]};
-      // (four in a row share the tap: its register is read once; with them interleaved a MiniSTU pass took 0.624 ms, so 0.597)
+      const f32x2 below = to[-1 - u];
+      const ulonglong2 ve = *reinterpret_cast<const ulonglong2*>(&xs[buf][0][u][tx * 4]);
+      const ulonglong2 vo = *reinterpret_cast<const ulonglong2*>(&xs[buf][1][u][tx * 4]);
+      const f32x2 xe[2] = {ve.x, ve.y}, xo[2] = {vo.x, vo.y};
+      const f32x2 od[5] = {below, o[0], o[1], o[2], o[3]};
 #pragma unroll
       for (int i = 0; i < 4; i++) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) ee[i][j] = fmaf(t4[i], xe[j], ee[i][j]);
+        for (int j = 0; j < 2; j++) ee[i][j] = fma2(t4[i], xe[j], ee[i][j]);
 #pragma unroll
-        for (int j = 0; j < 4; j++) eo[i][j] = fmaf(t4[i], xo[j], eo[i][j]);
+        for (int j = 0; j < 2; j++) eo[i][j] = fma2(t4[i], xo[j], eo[i][j]);
 #pragma unroll
-        for (int j = 0; j < 4; j++) qe[i][j] = fmaf(od[i], xo[j], qe[i][j]);
+        for (int j = 0; j < 2; j++) qe[i][j] = fma2(od[i], xo[j], qe[i][j]);
 #pragma unroll
-        for (int j = 0; j < 4; j++) qo[i][j] = fmaf(od[i + 1], xe[j], qo[i][j]);
+        for (int j = 0; j < 2; j++) qo[i][j] = fma2(od[i + 1], xe[j], qo[i][j]);
       }
       t4[3] = t4[2]; t4[2] = t4[1]; t4[1] = t4[0]; t4[0] = te[-1 - u];
       o[3] = o[2]; o[2] = o[1]; o[1] = o[0]; o[0] = below;
@@ -125,7 +152,7 @@ __global__ void __launch_bounds__(TX * 16, 32 / TX) full_conv_kernel(const float
       float up[4], um[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const float E = p ? eo[i][j] : ee[i][j], Q = p ? qo[i][j] : qe[i][j];
+        const float E = half_of(p ? eo[i][j >> 1] : ee[i][j >> 1], j & 1), Q = half_of(p ? qo[i][j >> 1] : qe[i][j >> 1], j & 1);
         up[j] = E + Q;
         um[j] = E - Q;
       }
@@ -160,16 +187,15 @@ extern "C" int stu_full_conv(const void* hist, int Lh, const void* phi, int L, i
   if (dtype != STU_F32) return STU_ERR_DTYPE;
   if (Lh % 4 || !aligned16(hist)) return STU_ERR_ALIGN;
   const long long rows = (long long)B * d;
-  if (rows > (1 << 21)) return STU_ERR_UNSUPPORTED;   // the grid's second dimension
   const int tiles_m = (((t_end + 1) >> 1) - (t0 >> 1) + MT - 1) / MT;
+  if (rows > (1 << 21) || (rows + 31) / 32 * K > 0x7fffffffll || tiles_m > 65535) return STU_ERR_UNSUPPORTED;   // the grid
   cudaStream_t st = (cudaStream_t)stream;
-  // 64 channels per CTA; fewer where the last tile would be mostly padding (narrow layers of one sequence)
+  // 32 channels per CTA, 16 where half of them would be padding (narrow layers of one sequence)
 #define STU_FULL_CONV(TX_)                                                                                         \
-  full_conv_kernel<TX_><<<dim3(tiles_m, (unsigned)((rows + 4 * TX_ - 1) / (4 * TX_)), K), TX_ * 16, 0, st>>>(      \
+  full_conv_kernel<TX_><<<dim3((unsigned)((rows + 4 * TX_ - 1) / (4 * TX_) * K), tiles_m), TX_ * 16, 0, st>>>(     \
       (const float*)hist, Lh, (const float*)phi, L, K, (float*)U, ldU, (int)rows, d, both_signs, t0, t_end, tiles_m)
   if (rows <= 16) STU_FULL_CONV(4);
-  else if (rows <= 32) STU_FULL_CONV(8);
-  else STU_FULL_CONV(16);
+  else STU_FULL_CONV(8);
 #undef STU_FULL_CONV
   STU_CHECK_LAUNCH();
   return STU_OK;
