@@ -211,6 +211,60 @@ PyObject* rmsnorm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_RETURN_NONE;
 }
 
+// layer_step_f32(x, norm_w, MinT, hist, taps, pos, mid, mlp_norm_w, gate, up, down, eps, mlp_eps, decode_flags, gate_flags, down_flags,
+// status): one cached token of an approx layer in fp32, three launches: mid = x + STU(norm(x)); x = mid + MLP(norm(mid)).  Returns 3,
+// or 1 where the MLP was refused (mid is done; its kernels write nothing that they read, so the caller may run both again), or None
+// where nothing was launched.
+PyObject* layer_step_f32(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 17) {
+    PyErr_SetString(PyExc_TypeError, "17 arguments expected");
+    return nullptr;
+  }
+  try {
+    const at::Tensor* t[11];
+    for (int i = 0; i < 11; i++)
+      if (!plain(args[i], &t[i]) || !t[i] || !t[i]->is_contiguous() || t[i]->device() != t[0]->device() ||
+          t[i]->scalar_type() != (i == 5 ? at::kInt : at::kFloat))
+        Py_RETURN_NONE;
+    const at::Tensor &x = *t[0], &hist = *t[3], &gate = *t[8];
+    const int dev = x.device().index();
+    if (x.dim() != 2 || hist.dim() != 4 || gate.dim() != 2 || dev != c10::cuda::current_device() ||
+        !(g_ready.load(std::memory_order_relaxed) >> dev & 1))
+      Py_RETURN_NONE;
+    const int64_t B = x.size(0), d = x.size(1), Lh = hist.size(3), I = gate.size(0);
+    const auto is = [&](int i, at::IntArrayRef want) { return t[i]->sizes() == want; };
+    if (B < 1 || B > INT32_MAX || d > INT32_MAX || I > INT32_MAX || Lh > INT32_MAX || !is(1, {d}) || !is(2, {d, d}) || !is(3, {B, d, 2, Lh}) ||
+        !is(4, {d, Lh}) || !is(5, {B, 2}) || !is(6, {B, d}) || !is(7, {d}) || !is(8, {I, d}) || !is(9, {I, d}) || !is(10, {d, I}) ||
+        x.data_ptr() == t[6]->data_ptr())
+      Py_RETURN_NONE;
+    const float eps = value_of<float>(args[11]), mlp_eps = value_of<float>(args[12]);
+    const int decode_flags = value_of<int>(args[13]), gate_flags = value_of<int>(args[14]), down_flags = value_of<int>(args[15]);
+    int* status = static_cast<int*>(address_of(args[16]));
+    const at::Tensor h = at::empty({B, I}, x.options());
+    void* p[11];
+    for (int i = 0; i < 11; i++) p[i] = t[i]->data_ptr();
+    void *ph = h.data_ptr(), *stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
+    int rc, done = 0;
+    Py_BEGIN_ALLOW_THREADS
+    rc = stu_decode_approx(p[0], d, p[1], p[2], p[3], p[4], nullptr, (int*)p[5], p[6], d, (int)B, (int)d, (int)Lh, eps, status, decode_flags,
+                           stream);
+    if (rc == 0) {
+      done = 1;
+      rc = stu_linear(p[6], d, p[8], d, 1, p[9], nullptr, 0, ph, I, (int)B, (int)I, (int)d, 2 | gate_flags, 0, 0, 0, p[7], mlp_eps, 0, 0, stream);
+    }
+    if (rc == 0)
+      rc = stu_linear(ph, I, p[10], I, 1, nullptr, p[6], d, p[0], d, (int)B, (int)d, (int)I, 1 | down_flags, 0, 0, 0, nullptr, 0.f, 0, 0, stream);
+    Py_END_ALLOW_THREADS
+    if (raised(rc, "layer_step_f32")) return nullptr;
+    if (rc == 0) done = 3;
+    if (done) return PyLong_FromLong(done);
+  } catch (const BadArgument&) {
+    PyErr_Clear();
+  } catch (const std::exception&) {
+  }
+  Py_RETURN_NONE;
+}
+
 // what ops.py launches
 #define ENTRY(name) {#name, (PyCFunction)(void (*)(void))Call<&name>::call, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
@@ -251,6 +305,7 @@ PyMethodDef methods[] = {
     ENTRY(stu_toeplitz),
     {"status_ready", (PyCFunction)(void (*)(void))status_ready, METH_FASTCALL, nullptr},
     {"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, nullptr},
+    {"layer_step_f32", (PyCFunction)(void (*)(void))layer_step_f32, METH_FASTCALL, nullptr},
     {"rmsnorm", (PyCFunction)(void (*)(void))rmsnorm, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

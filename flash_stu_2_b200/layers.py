@@ -118,6 +118,13 @@ class STULayer(nn.Module):
         x2 = x.view(B, d)
         stu, mlp = child(self, "stu"), child(self, "mlp")
         stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
+        if x.dtype == torch.float32 and stu.use_approx and not stu.use_hankel_L and ops.can_fuse_norm(
+                B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype):
+            done = stu.layer_step_f32(x2, mid, entry, stu_norm, mlp_norm, mlp)
+            if done == 1:
+                mlp.apply_residual(mid, mid, x2, norm_w=param(mlp_norm, "weight"), eps=mlp_norm.eps, overlap=True)
+            if done:
+                return entry
         ahead = getattr(entry[1], "_stream_ahead", None)
         if ahead is not None:   # a captured step whose history sums were computed beside the step before (stream_ahead.py)
             xn = stu.stream_step(x2, param(stu_norm, "weight"), stu_norm.eps, entry, mid, ahead, param(mlp_norm, "weight"), mlp_norm.eps)

@@ -408,6 +408,21 @@ class STU(nn.Module):
         pos._host_t = t + 1
         return hist, pos
 
+    def layer_step_f32(self, x2d, mid, entry, stu_norm, mlp_norm, mlp) -> int:
+        """decode_step of an fp32 layer and the MLP behind it as one native call; see ops.layer_step_f32."""
+        hist, pos = entry
+        MinT, taps, _ = self.prepared()
+        t = host_pos(pos)
+        if t + 1 > self.capacity:
+            raise ValueError(f"sequence position {t + 1} exceeds the capacity {self.capacity} (seq_len={self.seq_len})")
+        done = ops.layer_step_f32(x2d, param(stu_norm, "weight"), MinT, hist, taps, pos, mid, param(mlp_norm, "weight"),
+                                  param(child(mlp, "gate_proj"), "weight"), param(child(mlp, "up_proj"), "weight"),
+                                  param(child(mlp, "down_proj"), "weight"), stu_norm.eps, mlp_norm.eps,
+                                  uniform_pos(pos) and STU.shared_tap_decode)
+        if done:
+            pos._host_t = t + 1
+        return done
+
     @staticmethod
     def project_step(x2d, norm_w, eps: float, MinT):
         """The projected input of a token step of a larger batch, as one GEMM."""

@@ -354,6 +354,23 @@ def decode_approx(x, norm_w, MinT, hist, taps, pos, out, eps: float = RMS_EPS, t
     return out
 
 
+def layer_step_f32(x, norm_w, MinT, hist, taps, pos, mid, mlp_norm_w, gate, up, down, eps: float, mlp_eps: float, uniform: bool) -> int:
+    """One cached token of an approx layer in fp32, up to 8 sequences: decode_approx into `mid`, then the MLP from there into x, issued in
+    one native call (the interpreter takes as long for the three calls apart as the kernels do).  3: done; 1: the MLP is left to the
+    caller; 0: nothing was launched."""
+    if getattr(_local, "arena", None) is not None:
+        return 0
+    ov = FLAG_OVERLAP if overlap_decode else 0
+    early = FLAG_EARLY_TRIGGER if overlap_decode else 0
+    done = _lib.native().layer_step_f32(x, norm_w, MinT, hist, taps, pos, mid, mlp_norm_w, gate, up, down, eps, mlp_eps,
+                                        early | (FLAG_UNIFORM_POS if uniform else 0), ov, ov | (early if early_decode else 0),
+                                        status_word(x.device))
+    if done is None:
+        return 0
+    _count(done)
+    return done
+
+
 def decode_approx_shard(x, norm_w, MinT, hist, taps8, pos, out, eps: float = RMS_EPS, add_residual: bool = False,
                         flags: int = 0):
     """Fused decode step for the d_ch channels of a tensor-parallel rank: x [B,d_in] (full layer input), MinT

@@ -372,3 +372,43 @@ def test_full_variant_steps_change_their_form_on_one_cache(golden, monkeypatch):
             close(_steps_of_full_block(blk, x, 100, 28).cpu(), r["y"][:, 100:], 2e-2)
     ops.check_status()
     assert len(steps) == 28
+
+
+@pytest.mark.parametrize("off", [None, "gate_proj", "down_proj"])
+@pytest.mark.parametrize("B,d", [(1, 64), (3, 36), (8, 128)])
+def test_fp32_layer_step_in_one_native_call(monkeypatch, B, d, off):
+    """The step of an fp32 layer issued in one call, against its three launches made one by one: the same bits in the outputs and the
+    cache; gate weights that start off the 16-byte grid, which the fused norm is refused for, leave the MLP to the other path."""
+    import flash_stu_2_b200 as F
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(d)
+    cfg = F.FlashSTUConfig(n_embd=d, seq_len=64, num_eigh=8, use_attn=False, mlp_scale=4, torch_dtype=torch.float32, n_layers=1, vocab_size=1,
+                           n_heads=1)
+    blk = F.FlashSTUBlock(config=cfg, phi=F.get_spectral_filters(64, 8, device="cpu", dtype=torch.float32))
+    for p in blk.parameters():
+        torch.nn.init.normal_(p, std=0.2)
+    blk = blk.to("cuda:0").eval()
+    if off:
+        lin = getattr(blk.layer.mlp, off)
+        flat = torch.empty(lin.weight.numel() + 1, device="cuda:0")
+        flat[1:].copy_(lin.weight.detach().flatten())
+        lin.weight = torch.nn.Parameter(flat[1:].view_as(lin.weight))
+    x, rows = torch.randn(B, 9, d, device="cuda:0"), torch.randn(5, B, 1, d, device="cuda:0")
+    step, returned = ops.layer_step_f32, []
+
+    def run():
+        with torch.no_grad():
+            _, cache = blk(x.clone(), use_cache=True)
+            out = []
+            for r in rows:
+                y, cache = blk(r.clone(), past_key_value=cache, use_cache=True)
+                out.append(y)
+        ops.check_status()
+        return torch.stack(out), cache[0], cache[1]
+
+    monkeypatch.setattr(ops, "layer_step_f32", lambda *a: returned.append(step(*a)) or returned[-1])
+    got = run()
+    assert returned == [1 if off == "gate_proj" else 3] * 5
+    monkeypatch.setattr(ops, "layer_step_f32", lambda *a: 0)
+    for a, b in zip(got, run()):
+        assert torch.equal(a, b)
