@@ -93,6 +93,7 @@ _SIGNATURES = {
     "stu_lds_final_state": ([_P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_lds_chunk_scan": ([_P, _LL, _LL, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_lds_decode_features": ([_P, _LL, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P], c_int),
+    "stu_lds_decode_step": ([_P, _LL, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_swa_forward": ([_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
                          _P], c_int),
     "stu_decode_approx_projected": ([_P, _LL, _P, _LL, _P, _P, _P, _P, _LL, c_int, c_int, c_int, c_int, _P, c_int, _P],

@@ -287,7 +287,7 @@ PyMethodDef methods[] = {
     ENTRY(stu_full_decode_prepare),
     ENTRY(stu_full_decode_step),
     ENTRY(stu_lds_chunk_scan),
-    ENTRY(stu_lds_decode_features),
+    ENTRY(stu_lds_decode_step),
     ENTRY(stu_lds_final_state),
     ENTRY(stu_linear),
     ENTRY(stu_linear_can_fuse_norm),

@@ -219,6 +219,7 @@ class MiniSTU(nn.Module):
                 G = (G + 1) // 2
 
     def _forward_lds(self, x, past_key_value=None, use_cache=False):
+        before = self._lds_key
         op = self._lds_prepared()
         A32, B32, Cm = self._lds_f32
         B, T, d = x.shape
@@ -229,11 +230,13 @@ class MiniSTU(nn.Module):
                 raise NotImplementedError("the LDS backend continues a cache one token at a time")
             h, pos = past_key_value
             t = host_pos(pos)
-            U = torch.empty(B, F_ * d, dtype=x.dtype, device=x.device)
-            ops.lds_decode_features(x.view(B, d), h, A32, B32, Cm, U)
+            known = op._prep_key
             _, Mcat = op.prepared_full()
-            y = ops.linear(U, Mcat).view(B, 1, self.output_dim)
-            pos[:, 0] += 1
+            # constants that were there before this call are read ahead of the kernels in front: M's tiles while the state kernel runs
+            overlap = ops.overlap_decode and before is self._lds_key and known is op._prep_key
+            U = torch.empty(B, F_ * d, dtype=x.dtype, device=x.device)
+            ops.lds_decode_features(x.view(B, d), h, A32, B32, Cm, U, pos, overlap)
+            y = ops.linear(U, Mcat, epilogue=ops.EPI_STORE | (ops.FLAG_OVERLAP if overlap else 0)).view(B, 1, self.output_dim)
             pos._host_t = t + 1
             return (y, (h, pos)) if use_cache else y
         y = torch.empty(B, T, self.output_dim, dtype=x.dtype, device=x.device)

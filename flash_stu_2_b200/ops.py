@@ -708,16 +708,18 @@ def lds_chunk_features(W, Zb, U2, d: int, Ck: int, F: int):
     _count()
 
 
-def lds_decode_features(x2d, h, A32, B32, C, U):
-    """One recurrent LDS step for every channel: h <- A*h + B*x; U[b, f*d+i] = (h @ C)[f]."""
-    _cuda(x2d, h, A32, B32, C, U)
+def lds_decode_features(x2d, h, A32, B32, C, U, pos=None, overlap: bool = False):
+    """One recurrent LDS step for every channel: h <- A*h + B*x; U[b, f*d+i] = (h @ C)[f]; positions in pos move on.  overlap: the
+    constants A, B and C were not written by the kernel before this one."""
+    _cuda(x2d, h, A32, B32, C, U, pos)
     B, d = x2d.shape
     D, F = C.shape
     assert h.shape == (B, d, D) and h.is_contiguous() and h.dtype == torch.float64 and A32.dtype == torch.float64
     assert C.is_contiguous() and U.is_contiguous() and x2d.stride(1) == 1
-    rc = _lib.native().stu_lds_decode_features(x2d.data_ptr(), x2d.stride(0), h.data_ptr(), A32.data_ptr(), B32.data_ptr(),
-                                               C.data_ptr(), U.data_ptr(), B, d, D, F, _dt(x2d), _stream())
-    _lib.check(rc, "stu_lds_decode_features")
+    assert pos is None or (pos.shape == (B, 2) and pos.dtype == torch.int32 and pos.is_contiguous())
+    rc = _lib.native().stu_lds_decode_step(x2d.data_ptr(), x2d.stride(0), h.data_ptr(), A32.data_ptr(), B32.data_ptr(), C.data_ptr(),
+                                           U.data_ptr(), _p(pos), B, d, D, F, _dt(x2d) | (FLAG_OVERLAP if overlap else 0), _stream())
+    _lib.check(rc, "stu_lds_decode_step")
     _count()
 
 

@@ -268,6 +268,10 @@ int stu_lds_chunk_scan(const void* x, long long x_bstride, long long x_tstride, 
 /* One recurrent step (mini_stu/lds.py:95-101): h updated in place, U [B][F*d] = features in the row order of M. */
 int stu_lds_decode_features(const void* x, long long x_row_stride, double* h, const double* A, const double* Bv,
                             const void* C, void* U, int B, int d, int D, int F, int dtype, void* stream);
+/* The same, and every sequence's position in pos [B][2] moves on (pos may be NULL).  With STU_FLAG_OVERLAP (0x200) in dtype A, Bv and C
+ * are read while the kernel before this one in the stream may still be running: it must not be what writes them. */
+int stu_lds_decode_step(const void* x, long long x_row_stride, double* h, const double* A, const double* Bv, const void* C,
+                        void* U, int* pos, int B, int d, int D, int F, int dtype, void* stream);
 
 /* Sliding-window attention for the Tn new tokens in qkv [B,Tn,3*H*hd] (c_attn output) against a ring
  * cache of W >= window+1 slots ([B][W][H*hd] each; token t in slot t % W), ALiBi slopes [H] (fp32) and tanh
