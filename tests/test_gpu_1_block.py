@@ -412,3 +412,32 @@ def test_fp32_layer_step_in_one_native_call(monkeypatch, B, d, off):
     monkeypatch.setattr(ops, "layer_step_f32", lambda *a: 0)
     for a, b in zip(got, run()):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T", [1, 63, 96, 97, 126, 127, 128])
+def test_a_new_cache_is_zero_behind_the_prefill(T):
+    """Histories and rings are allocated without zeros where the prefill writes over them: what lies behind it is zero whatever the
+    memory held."""
+    import flash_stu_2_b200 as F
+    torch.manual_seed(T)
+    phi = F.get_spectral_filters(128, 8, device="cpu", dtype=torch.bfloat16)
+    for attn in (False, True):
+        cfg = F.FlashSTUConfig(n_embd=64, seq_len=128, num_eigh=8, use_attn=attn, mlp_scale=2, torch_dtype=torch.bfloat16, n_layers=1, vocab_size=1,
+                               n_heads=1, window_size=62)
+        blk = F.FlashSTUBlock(config=cfg, phi=phi)
+        for p in blk.parameters():
+            torch.nn.init.normal_(p, std=0.2)
+        blk = blk.to("cuda:0").eval()
+        poison = [torch.full((2, 64, 2, 64), float("nan"), dtype=torch.bfloat16, device="cuda:0") for _ in range(64)]
+        poison += [torch.full((2, 63, 64), float("nan"), dtype=torch.bfloat16, device="cuda:0") for _ in range(64)]
+        torch.cuda.synchronize()
+        del poison
+        with torch.no_grad():
+            _, cache = blk(torch.randn(2, T, 64, device="cuda:0").bfloat16(), use_cache=True)
+        if attn:
+            for ring in cache[:2]:
+                assert bool((ring[:, min(T, 63):] == 0).all()) and bool(torch.isfinite(ring).all())
+        else:
+            for parity in (0, 1):
+                n = (T + 1 - parity) // 2
+                assert bool((cache[0][:, :, parity, n:] == 0).all()) and bool(torch.isfinite(cache[0][:, :, parity, :n]).all())
