@@ -51,7 +51,9 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
   if (kpos && (epilogue != EPI_STORE || !resid)) return STU_ERR_UNSUPPORTED;
   if ((epilogue < EPI_STORE || epilogue > EPI_HIST) && epilogue != EPI_BLOCKCOL) return STU_ERR_UNSUPPORTED;
   // EPI_BLOCKCOL: hist_T = columns per block, resid_row_stride = distance between blocks (elements); resid unused
-  if (epilogue == EPI_BLOCKCOL && (hist_T <= 0 || resid_row_stride <= 0)) return STU_ERR_SHAPE;
+  // (hist_Lh > 0: row m of x is zero from column K - hist_Lh + m / hist_t0 + 1 on; the tcgen05 GEMM skips what it can)
+  if (epilogue == EPI_BLOCKCOL && (hist_T <= 0 || resid_row_stride <= 0 || hist_Lh < 0 || hist_Lh > K || (hist_Lh && hist_t0 <= 0)))
+    return STU_ERR_SHAPE;
   if (epilogue == EPI_GELU_MUL && !W2) return STU_ERR_NULL;
   if (epilogue == EPI_RESID && !resid) return STU_ERR_NULL;
   if (epilogue == EPI_HIST && (hist_T <= 0 || hist_Lh <= 0 || hist_t0 < 0 || (M % hist_T) != 0 ||

@@ -267,7 +267,8 @@ class MiniSTU(nn.Module):
         for b0 in range(0, B, G):
             n = min(G, B - b0)
             for b in range(b0, b0 + n):
-                ops.lds_chunk_features(W, Z[b].view(nch * d, W.shape[1]), U2[(b - b0) * T:(b - b0) * T + nch * Ck], d, Ck, F_)
+                ops.lds_chunk_features(W, Z[b].view(nch * d, W.shape[1]), U2[(b - b0) * T:(b - b0) * T + nch * Ck], d, Ck, F_,
+                                       causal=True)
             ops.linear(U2[:n * T], Mcat, out=y[b0:b0 + n].view(n * T, self.output_dim))
         if not use_cache:
             return y

@@ -693,9 +693,10 @@ def lds_chunk_scan(x, A64, B64, Vs, Z, hfin, Ck: int, unit_b: bool = False):
     _count()
 
 
-def lds_chunk_features(W, Zb, U2, d: int, Ck: int, F: int):
+def lds_chunk_features(W, Zb, U2, d: int, Ck: int, F: int, causal: bool = False):
     """U2[c*Ck + tau, f*d + i] = sum_k W[tau*F + f, k] * Zb[c*d + i, k]: the LDS features of one sequence, one GEMM over
-    all its chunks, scattered straight into the [tokens, F*d] operand of the contraction with M."""
+    all its chunks, scattered straight into the [tokens, F*d] operand of the contraction with M.  causal: the last Ck columns of W
+    are a Toeplitz matrix, zero behind column tau of them (those blocks are skipped)."""
     _cuda(W, Zb, U2)
     Mrows, KZ = W.shape
     N = Zb.shape[0]
@@ -703,7 +704,8 @@ def lds_chunk_features(W, Zb, U2, d: int, Ck: int, F: int):
     assert N % d == 0 and U2.shape == (N // d * Ck, F * d) and U2.dtype == W.dtype == Zb.dtype
     status_word(W.device)
     rc = _lib.native().stu_linear(W.data_ptr(), KZ, Zb.data_ptr(), KZ, 1, None, None, Ck * F * d, U2.data_ptr(), d,
-                                  Mrows, N, KZ, 5, d, 0, 0, None, 0.0, _dt(W), BACKEND_AUTO, _stream())
+                                  Mrows, N, KZ, 5, d, F if causal else 0, Ck if causal else 0, None, 0.0, _dt(W), BACKEND_AUTO,
+                                  _stream())
     _lib.check(rc, "stu_linear (LDS feature scatter)")
     _count()
 

@@ -258,7 +258,8 @@ int stu_lds_final_state(const void* hist, double* h, const double* A, const doub
  * state, rotated into a balanced basis (z = Vs^T h, Vs [D][R] float64), and the chunk's inputs into
  * Z [B][ceil(Tn/Ck)][d][KZ] (bf16: z_hi | z_lo | z_hi | x, KZ = 3R+Ck; fp32: z | x, KZ = R+Ck), and the final state into
  * hfin [B*d][D] (bit-identical to stu_lds_final_state).  The features of all chunks of a sequence are then ONE
- * stu_linear call with epilogue 5 on Z (see flash_stu_2_b200/mini_stu.py for the constant operand).  R % 8 == 0,
+ * stu_linear call with epilogue 5 on Z (hist_t0 = F and hist_Lh = Ck there say that row m of the operand is zero behind
+ * column K - Ck + m / F, so that those blocks may be skipped; 0, 0: nothing is known) (see flash_stu_2_b200/mini_stu.py for the constant operand).  R % 8 == 0,
  * Ck % 8 == 0, D <= 256.  dtype | 0x1000: the caller has checked that every Bv[n] is exactly 1 (faster kernel, same
  * bits). */
 int stu_lds_chunk_scan(const void* x, long long x_bstride, long long x_tstride, const double* A, const double* Bv,

@@ -1336,6 +1336,26 @@ def test_linear_outputs_by_tensor_copies(shape, epi):
     assert bool((buf[:M, N:] == 7.0).all()) and bool((buf[M:] == 7.0).all())
 
 
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,nch,Ck,F,K", [(64, 3, 128, 48, 320), (128, 2, 64, 40, 200), (64, 1, 32, 8, 32), (72, 2, 128, 5, 136)])
+def test_lds_features_skip_what_a_toeplitz_operand_leaves_out(dt, d, nch, Ck, F, K):
+    """Features whose operand is zero behind its diagonal: the blocks that are skipped take nothing from the sums (the same bits as with
+    them), wherever the last row of a tile lies."""
+    from flash_stu_2_b200 import ops
+    g = torch.Generator(device=dev()).manual_seed(K)
+    W = torch.randn(Ck * F, K, device=dev(), generator=g) / math.sqrt(K)
+    tau, col = torch.arange(Ck * F, device=dev()) // F, torch.arange(K, device=dev())
+    W = W.masked_fill(col[None, :] > (K - Ck + tau)[:, None], 0.0).to(dt).contiguous()
+    Z = torch.randn(nch * d, K, device=dev(), generator=g).to(dt)
+    a, b = (torch.full((nch * Ck, F * d), 7.0, dtype=dt, device=dev()) for _ in range(2))
+    ops.lds_chunk_features(W, Z, a, d, Ck, F, causal=True)
+    ops.lds_chunk_features(W, Z, b, d, Ck, F)
+    ops.check_status()
+    assert torch.equal(a, b)
+    want = (W.double() @ Z.double().t()).view(Ck, F, nch, d).permute(2, 0, 1, 3).reshape(nch * Ck, F * d)
+    close(a, want, 1e-5 if dt == torch.float32 else 2 ** -8)
+
+
 @pytest.mark.parametrize("d,chunks,rows,K", [(64, 3, 96, 72), (192, 2, 130, 320), (40, 5, 96, 64), (1024, 2, 6144, 320)])
 def test_lds_features_in_column_blocks(d, chunks, rows, K):
     """The blocked output of the LDS features: blocks of whole 64s leave by tensor copies, others by the lanes."""
