@@ -295,7 +295,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
   const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int num_tiles = tiles_m * tiles_n;
   int num_kb = (K + BK - 1) / BK;
-  if (EPI == EPI_STORE && ep.kpos) num_kb = min(num_kb, max(__ldg(ep.kpos), 0) / (2 * BK) + 1);   // the rest of W is zero
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -321,6 +320,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
   pair_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  // launched programmatically: everything so far ran beside the end of the kernel in front; the next kernel may be made resident now
+  // that this one holds its tensor memory
+  pdl_trigger();
+  pdl_wait();
+  if (EPI == EPI_STORE && ep.kpos) num_kb = min(num_kb, max(__ldg(ep.kpos), 0) / (2 * BK) + 1);   // the rest of W is zero
 
   if (warp == 0) {
     // ---------------- TMA producer (of either CTA: its 128 rows of A, its half of the rows of B)
@@ -815,7 +819,9 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   const int drop = g_drop_first_copy;
   g_drop_first_copy = 0;   // the injected fault applies to one launch
   const int group_m = m_fast ? tiles_m : gemm_group_m(tiles_n, N, K, DUAL);
-  k<<<grid, 64 + 32 * EPI_WARPS, smem, st>>>(a, b, b2, y, by_copy, M, N, K, tiles_m, tiles_n, group_m, causal, ep, status, drop, g_wait_ns);
+  e = launch_maybe_overlapped(k, dim3(grid), dim3(64 + 32 * EPI_WARPS), smem, st, true, a, b, b2, y, by_copy, M, N, K, tiles_m, tiles_n, group_m,
+                              causal, ep, status, drop, g_wait_ns);
+  if (e != cudaSuccess) return (int)e;
   STU_CHECK_LAUNCH();
   return STU_OK;
 }
