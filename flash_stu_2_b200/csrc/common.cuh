@@ -108,8 +108,8 @@ __device__ __forceinline__ bool elect_one() {
 // ---- programmatic dependent launch (overlap of a kernel's constant-data prefetch with its predecessor) ----
 // Flags OR-ed into the epilogue code of stu_linear and into the dtype code of stu_decode_approx:
 //   STU_FLAG_OVERLAP        the launch carries the programmatic-stream-serialization attribute: its CTAs may start
-//                           while the preceding kernel of the stream is still running; everything the kernel
-//                           reads before griddepcontrol.wait must be data that kernel does not write
+//                           while kernels before it in the stream are still running; everything the kernel
+//                           reads before griddepcontrol.wait must be data that none of them writes (see PdlTrigger, epilogue.cuh)
 //   STU_FLAG_EARLY_TRIGGER  the kernel lets its own successor start as soon as all its CTAs are resident
 //                           (otherwise: right after its own wait, i.e. once its predecessor has completed)
 // Both instructions are no-ops in a launch without programmatic neighbours.

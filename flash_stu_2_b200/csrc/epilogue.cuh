@@ -13,6 +13,18 @@ enum {
                      // elements after the last (the distilled-LDS features: rows (tau, f), columns (chunk, channel),
                      // written straight into the [tokens, F*d] operand of the contraction with M)
 };
+
+// What may still be running when a kernel starts.  A kernel that triggers AHEAD of its wait lets its successor start while its own
+// predecessor runs, and a chain of such kernels that far back; one that triggers BEHIND its wait starts its successor
+// with everything but itself complete.  stu_decode_pipe_kernel reads ahead of its wait (under STU_FLAG_OVERLAP) positions and
+// history that the layer's previous step wrote: every chain from one step of a layer to its next has to hold a kernel of the
+// second kind, or one that is launched plainly.  These are: every tcgen05 GEMM (gemm_tc_kernel), every linear that is launched with
+// neither flag, and every gate/up product (a layer's MLP follows its STU; the down projection behind it still asks for its
+// weights beside the whole of the gate/up kernel).
+template <int EPI> struct PdlTrigger {
+  static constexpr bool ahead_of_wait = EPI != EPI_GELU_MUL;
+};
+
 // OR-ed into the epilogue code: W is lower triangular (W[n][k] = 0 for k > n); kernels may skip those blocks
 #define EPI_FLAG_CAUSAL 0x100
 // ... : W[n][k] = 0 for k > t / 2, t the position that `resid` (not a residual then) points to on the device

@@ -321,10 +321,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
   pair_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  // launched programmatically: everything so far ran beside the end of the kernel in front; the next kernel may be made resident now
-  // that this one holds its tensor memory
-  pdl_trigger();
+  // launched programmatically: everything so far ran beside the end of the kernel in front; the next kernel may be made resident
+  // once that one is complete (see PdlTrigger, epilogue.cuh) and this one holds its tensor memory
   pdl_wait();
+  pdl_trigger();
   if (EPI == EPI_STORE && ep.kpos) num_kb = min(num_kb, max(__ldg(ep.kpos), 0) / (2 * BK) + 1);   // the rest of W is zero
 
   if (warp == 0) {
@@ -839,7 +839,8 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
 // share of the tokens in a fixed order through distributed shared memory and runs their epilogue (coalesced along
 // the features).
 // Launched with the programmatic attribute: the successor is released once tensor memory has been allocated (a
-// co-resident successor that allocated first could otherwise block this kernel's allocation while waiting for it);
+// co-resident successor that allocated first could otherwise block this kernel's allocation while waiting for it), in gate/up and
+// without early_weights once the kernel in front is complete (PdlTrigger, epilogue.cuh);
 // with early_weights (the caller's promise that the preceding kernel does not write the weights) the weight tiles of
 // the first stages are requested before griddepcontrol.wait, the activation tiles after it.
 
@@ -898,7 +899,8 @@ __global__ void __launch_bounds__(192, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();   // only now: this CTA holds its tensor memory
+  const bool early_trigger = early_weights && PdlTrigger<EPI>::ahead_of_wait;
+  if (early_trigger) pdl_trigger();   // only now: this CTA holds its tensor memory
 
   if (warp == 0) {
     // ---------------- TMA producer
@@ -922,6 +924,7 @@ __global__ void __launch_bounds__(192, 1)
         load_w(g, kb0 + g);
       }
     pdl_wait();   // the activations are the output of the kernel before this one
+    if (!early_trigger) pdl_trigger();
     for (int g = 0; g < pre; g++)
       if (leader) load_x(g, kb0 + g);
     int g = pre, s = pre == nstages ? 0 : pre;

@@ -84,7 +84,8 @@ __global__ void __launch_bounds__(NW * 32, 1) skinny_stage_kernel(const bf16* __
     nvalid[j] = n < N;
     wrow[j] = ((DUAL && j >= 2) ? W2 : W) + (size_t)(nvalid[j] ? n : 0) * ldb;
   }
-  pdl_trigger();
+  const bool early_trigger = early_weights && PdlTrigger<EPI>::ahead_of_wait;
+  if (early_trigger) pdl_trigger();
   if (!early_weights) pdl_wait();
   uint4 wv[U][NT];
 #pragma unroll
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(NW * 32, 1) skinny_stage_kernel(const bf16* __
   }
   __syncthreads();
   if (early_weights) pdl_wait();   // the activations are the output of the kernel before this one
+  if (!early_trigger) pdl_trigger();
   if (threadIdx.x == 0 && nch > 0) {
     tma::mbar_expect_tx(&s_bar, (uint32_t)M * nch * 64);
     for (int m = 0; m < M; m++)

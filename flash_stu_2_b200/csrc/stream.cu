@@ -130,11 +130,13 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
   };
 
-  pdl_trigger();
+  const bool early_trigger = early && PdlTrigger<EPI>::ahead_of_wait;
+  if (early_trigger) pdl_trigger();
   if (!early) pdl_wait();
 #pragma unroll
   for (int s = 0; s < D; s++) issue_w(s);
   if (early) pdl_wait();
+  if (!early_trigger) pdl_trigger();
 #pragma unroll
   for (int s = 0; s < D; s++) {
     issue_x(s);
@@ -323,11 +325,13 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
   };
 
-  pdl_trigger();
+  const bool early_trigger = early && PdlTrigger<EPI>::ahead_of_wait;
+  if (early_trigger) pdl_trigger();
   if (!early) pdl_wait();
 #pragma unroll
   for (int s = 0; s < D; s++) issue_w(s);
   if (early) pdl_wait();
+  if (!early_trigger) pdl_trigger();
 #pragma unroll
   for (int s = 0; s < D; s++) {
     issue_x(s);

@@ -22,7 +22,8 @@
 //     never wait for them (two hand-over slots), so the projection of a row runs under the stream of that row.
 // No cross-CTA reduction, no workspace: a row is summed inside one CTA, slices in order.
 // In an overlapped (programmatic) launch only the projection group waits for the preceding kernel: history, taps and
-// positions were written by this layer's previous step, which has completed by the time this kernel can start.
+// positions were written by this layer's previous step, which has completed by the time this kernel can start (a kernel between the two
+// sees to that: PdlTrigger, epilogue.cuh).
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises status 7, lets its outstanding copies land (bounded) and
 // returns.

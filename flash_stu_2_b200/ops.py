@@ -392,7 +392,8 @@ def decode_approx_shard(x, norm_w, MinT, hist, taps8, pos, out, eps: float = RMS
 def decode_approx_projected(x, xp, hist, taps8, pos, out, add_residual: bool = True):
     """Decode step of an approx STU sub-layer whose projected input xp [B, d_ch] the caller computed as one GEMM:
     appends xp to the cache, out = (x +) taps . history.  With overlap_decode the kernel starts its history stream
-    while the projection before it is still running and lets its own successor start at once."""
+    while the projection before it is still running and lets its own successor start at once: between two steps on one
+    cache there has to be a launch that does not do so before it has waited, such as a linear() without launch flags."""
     _cuda(xp, hist, taps8, pos, out)
     flags = (FLAG_OVERLAP | FLAG_EARLY_TRIGGER) if overlap_decode else 0
     B, dch, _, Lh = hist.shape

@@ -128,8 +128,11 @@ int stu_conv_prefill_approx_tc5(const void* hist, const void* taps8, void* yT, v
  * programmatic-stream-serialization attribute: each fetches its weights while the kernel before it drains and waits
  * (griddepcontrol.wait) before it touches anything that kernel writes.  stu_set_programmatic_launch(0) turns the
  * launches that follow back into plain stream-ordered ones (as STU_B200_DISABLE_PDL=1 does from the start) and
- * returns the previous setting; a captured CUDA graph keeps what it was captured with.  No counterpart in the
- * reference. */
+ * returns the previous setting; a captured CUDA graph keeps what it was captured with.  Most of them let their own successor start
+ * before they have waited themselves, so that several kernels may be under way: what a launch with 0x200 reads ahead of its wait
+ * (weights and constants; positions and history in stu_decode_approx_pipelined, _push and _projected) may be written by none of them.
+ * Everything before its predecessor is complete where that is a plain launch, a stu_linear without 0x200 and 0x400, one with
+ * epilogue 2 or one of more than 64 rows.  No counterpart in the reference. */
 int stu_set_programmatic_launch(int on);
 
 /* Profiling aid of stu_conv_prefill_approx_tc5: while a device buffer of 128 64-bit words is registered, CTA 0 of

@@ -173,6 +173,29 @@ def test_tagged_words_are_read_in_elements_of_the_stores_width():
     assert len(re.findall(r"ld\.relaxed\.gpu\.global", text)) == 2   # nobody else reads them
 
 
+def test_kernels_that_end_a_chain_of_early_launches():
+    """The STU decode kernel reads positions and history ahead of its programmatic wait, which the layer's previous step wrote: a
+    kernel between the two has to wait before it lets its successor start.  The tcgen05 GEMM always does, gate/up products and linears
+    whose caller vouches for no weights do in every form."""
+    csrc = os.path.join(os.path.dirname(_lib.LIB_PATH), "csrc")
+    body = {}
+    for name, kernel in (("gemm_tc", "gemm_tc_kernel"), ("gemm_tc", "skinny_umma_kernel"), ("skinny_stage", "skinny_stage_kernel"),
+                         ("skinny_wide", "skinny_wide_kernel"), ("stream", "stream_bf16_kernel"), ("stream", "stream_f32_kernel")):
+        text = open(os.path.join(csrc, name + ".cu")).read()
+        body[kernel] = text[text.index("__global__", text.index(f"{kernel}(") - 400):]
+        body[kernel] = body[kernel][:body[kernel].index("\n}\n")]
+    for kernel, text in body.items():
+        triggers = [text[:m.start()] for m in re.finditer(r"pdl_trigger\(\)", text)]
+        early = [t for t in triggers if t.endswith("if (early_trigger) ")]
+        if kernel in ("gemm_tc_kernel", "skinny_wide_kernel"):
+            assert not early
+        else:
+            assert re.search(r"early_trigger = early(_weights)? && PdlTrigger<EPI>::ahead_of_wait", text), kernel
+        late = [t for t in triggers if t not in early]
+        assert len(late) == 1 and "pdl_wait()" in late[0], kernel
+        assert not re.search(r"if \(early(_weights)?\) pdl_trigger", text)
+
+
 def test_sms_for_the_streams_beside_a_step():
     """What decides whether and on how many SMs a captured step's history streams run beside it: none for a few short streams, never
     more than a third of the GPU, more for longer histories."""
