@@ -183,17 +183,18 @@ struct FinishParams {
   const int* ctl;
   int* pos;
   int* status;
-  int B, d, Lh;
+  int B, d, Lh, overlap;
   float eps;
 };
 
-// One CTA per sequence: the new token's term, the residual, the append and the norm behind them.  Everything that the step before left
-// (sums, taps, position) is read ahead of the wait for the projection.
+// One CTA per sequence: the new token's term, the residual, the append and the norm behind them.  Under STU_FLAG_OVERLAP everything that
+// the step before left (sums, taps, position) is read ahead of the wait for the projection: the caller's word that no kernel
+// which may still be under way writes it (the steps of a replayed graph, which begin when the replay before is complete).
 __global__ void __launch_bounds__(128) stu_stream_finish_kernel(const FinishParams P) {
   constexpr int NV = 4;   // vectors of 8 channels per thread: d up to 4096
   const int b = blockIdx.x, d = P.d, Lh = P.Lh;
   const size_t LP = (size_t)Lh + 8;
-  pdl_trigger();
+  if (P.overlap) pdl_trigger();
   const int t = P.pos[2 * b], p = t & 1, s = t >> 1;
   const bool ok = t >= 0 && t < 2 * Lh && P.ctl[2 + p] == t;
   float y[NV][8], w0[NV][8];
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(128) stu_stream_finish_kernel(const FinishPara
     }
   }
   pdl_wait();   // the projection is the kernel before this one
+  if (!P.overlap) pdl_trigger();
   if (!ok) {
     if (threadIdx.x == 0 && P.status) atomicExch(P.status, t < 0 || t >= 2 * Lh ? 2 : 8);
     return;
@@ -296,12 +298,14 @@ extern "C" int stu_stream_finish(const void* x, const void* xp, void* hist, cons
                                  const int* ctl, const void* norm_w, float eps, void* out, void* xn, int B, int d, int Lh,
                                  int* status, int dtype, void* stream) {
   if (!x || !xp || !hist || !taps8 || !pos || !part || !ctl || !norm_w || !out || !xn) return STU_ERR_NULL;
+  const bool overlap = (dtype & STU_FLAG_OVERLAP) != 0;
+  dtype &= ~STU_FLAG_OVERLAP;
   if (B <= 0 || d <= 0 || Lh <= 0 || d % 8 || Lh % 8) return STU_ERR_SHAPE;
   if (dtype != STU_BF16 || d > 4096) return STU_ERR_UNSUPPORTED;
   if (!aligned16(x) || !aligned16(xp) || !aligned16(part) || !aligned16(norm_w) || !aligned16(out) || !aligned16(xn)) return STU_ERR_ALIGN;
   FinishParams P{(const bf16*)x, (const bf16*)xp, (const bf16*)taps8, (const bf16*)norm_w, (bf16*)hist, (bf16*)out, (bf16*)xn,
-                 part, ctl, pos, status, B, d, Lh, eps};
-  const cudaError_t e = launch_maybe_overlapped(stu_stream_finish_kernel, dim3(B), dim3(128), 0, (cudaStream_t)stream, pdl_enabled(), P);
+                 part, ctl, pos, status, B, d, Lh, overlap ? 1 : 0, eps};
+  const cudaError_t e = launch_maybe_overlapped(stu_stream_finish_kernel, dim3(B), dim3(128), 0, (cudaStream_t)stream, overlap, P);
   if (e != cudaSuccess) return (int)e;
   STU_CHECK_LAUNCH();
   return STU_OK;

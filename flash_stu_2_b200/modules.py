@@ -445,7 +445,8 @@ class STU(nn.Module):
         hist, pos = entry
         MinT, _, taps8 = self.prepared()
         xp = self.project_step(x2d, norm_w, eps, MinT)
-        xn = ops.stream_finish(x2d, xp, hist, taps8, pos, *ahead, next_norm_w, next_eps, out2d)
+        # (the step of the replay before, which wrote what is read early here, is complete when a replay begins)
+        xn = ops.stream_finish(x2d, xp, hist, taps8, pos, *ahead, next_norm_w, next_eps, out2d, overlap=ops.overlap_decode)
         pos._host_t = host_pos(pos) + 1
         return xn
 

@@ -425,9 +425,10 @@ def stream_ahead(hists, taps8s, part, ctl, sms: int):
     _count()
 
 
-def stream_finish(x, xp, hist, taps8, pos, part, ctl, norm_w, eps: float, out):
+def stream_finish(x, xp, hist, taps8, pos, part, ctl, norm_w, eps: float, out, overlap: bool = False):
     """The layer's own part of a token step whose history sums stream_ahead has left in `part` [2,B,d]: append, out = x + STU, and
-    the norm behind it, which is returned."""
+    the norm behind it, which is returned.  overlap: pos, part, ctl and taps8 were not written by a kernel that may still be under way
+    (a step of a replayed graph): they are read while the projection before this kernel runs."""
     _cuda(x, xp, hist, taps8, pos, part, ctl, norm_w, out)
     B, d, _, Lh = hist.shape
     assert x.shape == (B, d) and xp.shape == (B, d) and out.shape == (B, d) and part.shape == (2, B, d)
@@ -435,7 +436,7 @@ def stream_finish(x, xp, hist, taps8, pos, part, ctl, norm_w, eps: float, out):
     xn = empty((B, d), x.dtype, x.device)
     rc = _lib.native().stu_stream_finish(x.data_ptr(), xp.data_ptr(), hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), part.data_ptr(),
                                          ctl.data_ptr(), norm_w.data_ptr(), eps, out.data_ptr(), xn.data_ptr(), B, d, Lh,
-                                         status_word(x.device).data_ptr(), _dt(x), _stream())
+                                         status_word(x.device).data_ptr(), _dt(x) | (FLAG_OVERLAP if overlap else 0), _stream())
     _lib.check(rc, "stu_stream_finish")
     _count()
     return xn

@@ -309,7 +309,9 @@ int stu_decode_approx_projected(const void* x, long long x_row_stride, const voi
  * 0, position that part[.][0] holds, the same for part[.][1]}; ctl[2 + (t & 1)] has to be t - 2 when position t is computed.
  * stu_stream_finish is the layer's own part of the step, for the position t that ctl says `part` (the layer's, [2][B][d]) holds
  * (status 8 otherwise): appends xp [B,d] (the projected input) to hist, out = x + round(2 * (part + xp * tap_0)),
- * xn = rmsnorm(out) * norm_w, advances pos.  d <= 4096; x, xp, out, xn dense rows; the step of flash_stu/modules/stu.py:85-98,120. */
+ * xn = rmsnorm(out) * norm_w, advances pos.  d <= 4096; x, xp, out, xn dense rows; the step of flash_stu/modules/stu.py:85-98,120.
+ * With STU_FLAG_OVERLAP (0x200) in its dtype pos, ctl, part and taps8 are read while kernels before it in the stream may still be
+ * running (see stu_set_programmatic_launch): none of them may write these. */
 int stu_stream_ahead(const void* const* hist, const void* const* taps8, int layers, float* part, int* ctl, int B, int d,
                      int Lh, int sms, int* status, int dtype, void* stream);
 int stu_stream_finish(const void* x, const void* xp, void* hist, const void* taps8, int* pos, const float* part,

@@ -196,6 +196,29 @@ def test_kernels_that_end_a_chain_of_early_launches():
         assert not re.search(r"if \(early(_weights)?\) pdl_trigger", text)
 
 
+def test_early_reads_of_the_finish_kernel_are_the_callers_choice(monkeypatch):
+    """stream_finish starts beside the kernels in front, and reads what the step before wrote ahead of its wait, only where it is told
+    to; the captured step is what tells it."""
+    from types import SimpleNamespace
+
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.modules import STU
+    calls = []
+    monkeypatch.setattr(ops, "_cuda", lambda *a: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "status_word", lambda dev: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(_lib, "native", lambda: SimpleNamespace(stu_stream_finish=lambda *a: calls.append(a[-2]) or 0))
+    rows = lambda: torch.zeros(2, 8, dtype=torch.bfloat16)
+    hist, taps8, part = torch.zeros(2, 8, 2, 8), torch.zeros(8, 8, 16), torch.zeros(2, 2, 8)
+    pos, ctl = torch.zeros(2, 2, dtype=torch.int32), torch.zeros(4, dtype=torch.int32)
+    pos._host_t = 0
+    ops.stream_finish(rows(), rows(), hist, taps8, pos, part, ctl, torch.zeros(8), 1e-6, rows())
+    monkeypatch.setattr(STU, "project_step", staticmethod(lambda x, *a: rows()))
+    stu = SimpleNamespace(prepared=lambda: (None, None, taps8), project_step=STU.project_step)
+    STU.stream_step(stu, rows(), None, 1e-6, (hist, pos), rows(), (part, ctl), torch.zeros(8), 1e-6)
+    assert calls == [1, 1 | ops.FLAG_OVERLAP]
+
+
 def test_sms_for_the_streams_beside_a_step():
     """What decides whether and on how many SMs a captured step's history streams run beside it: none for a few short streams, never
     more than a third of the GPU, more for longer histories."""
