@@ -311,6 +311,8 @@ class FlashSTU(PreTrainedModel):
             timings["replay_ms"] = ev_first.elapsed_time(ev_last)
         if stepper is not None:
             stepper.check()   # tokens drawn from logits that no step has written are not returned
+        if graph is not None and buffers[-1] is not None:
+            buffers[-1].check()
         if return_logits:
             return generated, all_logits if stepper is not None else torch.stack(all_logits, dim=1)
         return generated

@@ -95,3 +95,10 @@ class StreamAhead:
 
     def join(self, stream):
         stream.wait_stream(self.stream)
+
+    def check(self):
+        """Raises when a launch of the sums has given up on a wait: the steps from the position behind it on wrote nothing.  Waits for
+        the steps so far."""
+        if int(self.ctl[2:].min()) < 0:   # (a half that holds no position stays so)
+            ops.check_status(self.part.device)
+            raise RuntimeError(f"flash_stu_2_b200 device status 8: {ops.STATUS_TEXT[8]}")

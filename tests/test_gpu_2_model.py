@@ -389,6 +389,32 @@ def test_streams_beside_the_captured_step(monkeypatch, B, T0, new, sms):
         assert torch.equal(ids, want_ids) and torch.equal(logits, want)
 
 
+@pytest.mark.parametrize("half", [0, 1])
+def test_captured_step_without_its_history_sums_is_reported(monkeypatch, half):
+    """Sums that a launch beside the step could not finish stay unannounced, and every later step of the call writes nothing: tokens
+    drawn from what the buffers held are not returned.  (What a launch leaves that gave up is put there by the host.)"""
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.stream_ahead import StreamAhead
+    m = _random_model(256, 4, torch.bfloat16)
+    prompt = torch.randint(0, 1003, (17, 30), device=dev())
+    monkeypatch.setattr(StreamAhead, "sms", staticmethod(lambda *a: 16))
+    want = m.generate(prompt, max_length=40, do_sample=False)
+    launch, n = StreamAhead.launch, []
+
+    def gave_up(self, sms):
+        n.append(sms)
+        if len(n) == 2:   # being captured: the halves are marked in every replay
+            self.ctl[2 + half].fill_(-1)
+        launch(self, sms)
+
+    monkeypatch.setattr(StreamAhead, "launch", gave_up)
+    with pytest.raises(RuntimeError, match="status 8"):
+        m.generate(prompt, max_length=40, do_sample=False)
+    monkeypatch.setattr(StreamAhead, "launch", launch)
+    assert torch.equal(m.generate(prompt, max_length=40, do_sample=False), want)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("where", ["attn_norm", "mlp_norm", "attn.c_attn", "mlp.gate_proj", "mlp.down_proj"])
 def test_fp32_steps_with_weights_off_the_16_byte_grid(where):
     """fp32 steps fuse the norm into the linears, whose kernel reads 16 bytes at a time: parameters that start elsewhere (views
