@@ -4,7 +4,7 @@ import torch
 import torch.nn as nn
 
 from . import ops
-from .modules import MLP, STU, Attention, RMSNorm, child, host_pos, param, uniform_pos
+from .modules import MLP, STU, Attention, RMSNorm, child, host_pos, own, param, uniform_pos
 
 
 def _inplace_target(x: torch.Tensor):
@@ -119,7 +119,7 @@ class STULayer(nn.Module):
         stu, mlp = child(self, "stu"), child(self, "mlp")
         stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
         if x.dtype == torch.float32 and stu.use_approx and not stu.use_hankel_L and ops.can_fuse_norm(
-                B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype):
+                B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype) and own(stu, STU, "decode_step") and own(mlp, MLP, "apply_residual"):
             done = stu.layer_step_f32(x2, mid, entry, stu_norm, mlp_norm, mlp)
             if done == 1:
                 mlp.apply_residual(mid, mid, x2, norm_w=param(mlp_norm, "weight"), eps=mlp_norm.eps, overlap=True)

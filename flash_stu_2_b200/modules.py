@@ -70,6 +70,11 @@ def child(module: nn.Module, name: str) -> nn.Module:
     return m if m is not None else getattr(module, name)
 
 
+def own(module: nn.Module, cls, *methods: str) -> bool:
+    """Whether these methods of a module are the class's own: nobody who overrides one is passed by."""
+    return all(getattr(type(module), m, None) is getattr(cls, m) and m not in vars(module) for m in methods)
+
+
 class RMSNorm(nn.Module):
     """torch.nn.RMSNorm(dim, dtype) arithmetic (the reference's non-Triton branch,
     flash_stu/layers/stu_layer.py:17-36): fp32 statistics, eps = finfo(float32).eps."""

@@ -7,7 +7,8 @@ branch of the graph, on a few SMs, and in the chain adds the new token's own ter
 import torch
 
 from . import ops
-from .modules import STU, _sm_count, host_pos, uniform_pos
+from .layers import STULayer
+from .modules import STU, _sm_count, host_pos, own, uniform_pos
 
 MAX_LAYERS = 64
 
@@ -30,7 +31,8 @@ class StreamAhead:
 
     @staticmethod
     def supported(layers, past, B: int) -> bool:
-        """bf16 approx layers of one size at one position, where the token's projection is a GEMM of its own."""
+        """bf16 approx layers of one size at one position, where the token's projection is a GEMM of its own and nobody overrides the
+        steps that this form of it takes the place of."""
         stus = [(layer, e) for layer, e in zip(layers, past) if hasattr(layer, "stu")]
         if not stus or len(stus) > MAX_LAYERS or B < STU.projected_decode_min_batch or not StreamAhead.enabled:
             return False
@@ -39,6 +41,8 @@ class StreamAhead:
         shape, t = stus[0][1][0].shape, host_pos(stus[0][1][1])
         for layer, (hist, pos) in stus:
             stu = layer.stu
+            if not (own(layer, STULayer, "forward", "_decode") and own(stu, STU, "decode_step")):
+                return False
             if (layer.stu_mlp_enabled or not stu.use_approx or stu.use_hankel_L or hist.dtype != torch.bfloat16 or hist.shape != shape
                     or not hist.is_contiguous() or not uniform_pos(pos) or host_pos(pos) != t or hist.shape[1] % 8 or hist.shape[1] > 4096
                     or stu.prepared()[2] is None):

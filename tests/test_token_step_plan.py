@@ -8,6 +8,9 @@ import torch
 
 import flash_stu_2_b200 as F
 from flash_stu_2_b200 import _lib
+from flash_stu_2_b200.layers import STULayer
+from flash_stu_2_b200.modules import STU
+from flash_stu_2_b200.stream_ahead import StreamAhead
 from flash_stu_2_b200.token_step import TokenStep
 
 A = 1 << 20   # stands for an aligned device address: nothing here dereferences it
@@ -202,7 +205,6 @@ def test_early_reads_of_the_finish_kernel_are_the_callers_choice(monkeypatch):
     from types import SimpleNamespace
 
     from flash_stu_2_b200 import ops
-    from flash_stu_2_b200.modules import STU
     calls = []
     monkeypatch.setattr(ops, "_cuda", lambda *a: None)
     monkeypatch.setattr(ops, "_stream", lambda: 0)
@@ -219,10 +221,50 @@ def test_early_reads_of_the_finish_kernel_are_the_callers_choice(monkeypatch):
     assert calls == [1, 1 | ops.FLAG_OVERLAP]
 
 
+def _sub_stu(m):
+    m.layers[2].stu.__class__ = type("Stu", (STU,), {"decode_step": lambda self, *a: STU.decode_step(self, *a)})
+
+
+def _sub_layer(m):
+    m.layers[2].__class__ = type("Layer", (STULayer,), {"_decode": lambda self, *a: STULayer._decode(self, *a)})
+
+
+def _foreign_layer(m):
+    m.layers[0] = torch.nn.Module()
+    m.layers[0].stu, m.layers[0].stu_mlp_enabled = m.layers[2].stu, False
+
+
+@pytest.mark.parametrize("change", [lambda m: setattr(m.layers[0].stu, "decode_step", lambda *a: None), _own_forward, _sub_stu, _sub_layer,
+                                    _foreign_layer])
+def test_overridden_steps_are_not_streamed_beside_the_chain(monkeypatch, change):
+    m = _model().bfloat16()
+    monkeypatch.setattr(STU, "prepared", lambda self: (None, None, True))
+    pos = torch.zeros(16, 2, dtype=torch.int32)
+    pos._host_t, pos._uniform = 3, True
+    past = [(torch.zeros(16, 64, 2, 8, dtype=torch.bfloat16), pos) for _ in m.layers]
+    assert StreamAhead.supported(m.layers, past, 16)
+    change(m)
+    assert not StreamAhead.supported(m.layers, past, 16)
+
+
+@pytest.mark.parametrize("where,name", [("stu", "decode_step"), ("mlp", "apply_residual")])
+def test_overridden_parts_of_an_fp32_step_are_called(monkeypatch, where, name):
+    """The native call for a whole fp32 layer step takes the place of decode_step and apply_residual where they are the classes' own."""
+    layer = _model().layers[0]
+    taken, called = [], []
+    monkeypatch.setattr(STU, "layer_step_f32", lambda self, *a: taken.append(1) or 3)
+    entry, x = (torch.zeros(2, 64, 2, 8), torch.zeros(2, 2, dtype=torch.int32)), torch.zeros(2, 1, 64)
+    assert layer._decode(x, entry) is entry and taken == [1]
+    monkeypatch.setattr(STU, "decode_step", lambda self, *a: entry)
+    monkeypatch.setattr(type(layer.mlp), "apply_residual", lambda self, *a, **k: None)
+    part = getattr(layer, where)
+    setattr(part, name, lambda *a, **k: called.append(name) or entry)
+    assert layer._decode(x, entry) is entry and taken == [1] and called == [name]
+
+
 def test_sms_for_the_streams_beside_a_step():
     """What decides whether and on how many SMs a captured step's history streams run beside it: none for a few short streams, never
     more than a third of the GPU, more for longer histories."""
-    from flash_stu_2_b200.stream_ahead import StreamAhead
     big = lambda t: StreamAhead.sms(24, 12, 32, 1536, t, 1_800_000_000, 2_400_000_000, 148)
     assert StreamAhead.sms(4, 2, 16, 512, 300, 60_000_000, 10_000_000, 148) == 0
     assert 18 <= big(2176) <= 26 and big(500) == 8 and big(8000) == 49
