@@ -75,6 +75,11 @@ def own(module: nn.Module, cls, *methods: str) -> bool:
     return all(getattr(type(module), m, None) is getattr(cls, m) and m not in vars(module) for m in methods)
 
 
+def _cache_for_prefill(op, cls, batch: int, device, filled: int):
+    """op.new_cache for a prefill of `filled` positions (an override takes a batch and a device)."""
+    return op.new_cache(batch, device, filled) if own(op, cls, "new_cache") else op.new_cache(batch, device)
+
+
 class RMSNorm(nn.Module):
     """torch.nn.RMSNorm(dim, dtype) arithmetic (the reference's non-Triton branch,
     flash_stu/layers/stu_layer.py:17-36): fp32 statistics, eps = finfo(float32).eps."""
@@ -348,7 +353,7 @@ class STU(nn.Module):
             hist, pos = entry
             t0 = host_pos(pos)
         elif use_cache:
-            hist, pos = self.new_cache(B, xn.device, T if T <= self.capacity else 0)
+            hist, pos = _cache_for_prefill(self, STU, B, xn.device, T if T <= self.capacity else 0)
         else:
             pos = None
             hist = torch.empty(B, d, 2, self.Lh, dtype=xn.dtype, device=xn.device)
@@ -522,7 +527,7 @@ class Attention(nn.Module):
             ov = ops.FLAG_OVERLAP if (T == 1 and ops.overlap_decode) else 0   # token step: weights fetched early
             qkv = ops.linear(xn.reshape(B * T, d), c_attn, epilogue=ops.EPI_STORE | ov).view(B, T, 3 * d)
         if entry is None and use_cache:
-            entry = self.new_cache(B, xn.device, T)
+            entry = _cache_for_prefill(self, Attention, B, xn.device, T)
         if entry is not None:
             k_ring, v_ring, pos = entry
             t0 = host_pos(pos)

@@ -414,6 +414,25 @@ def test_fp32_layer_step_in_one_native_call(monkeypatch, B, d, off):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("attn", [False, True])
+def test_an_overridden_new_cache_is_called_as_it_was(attn):
+    """Subclasses make caches from a batch and a device."""
+    import flash_stu_2_b200 as F
+    phi = F.get_spectral_filters(128, 8, device="cpu", dtype=torch.bfloat16)
+    cfg = F.FlashSTUConfig(n_embd=64, seq_len=128, num_eigh=8, use_attn=attn, mlp_scale=2, torch_dtype=torch.bfloat16, n_layers=1, vocab_size=1,
+                           n_heads=1, window_size=20)
+    blk = F.FlashSTUBlock(config=cfg, phi=phi).to("cuda:0").eval()
+    for p in blk.parameters():
+        torch.nn.init.normal_(p, std=0.2)
+    x = torch.randn(2, 100, 64, device="cuda:0").bfloat16()
+    with torch.no_grad():
+        y, cache = blk(x.clone(), use_cache=True)
+        op = blk.layer.attn if attn else blk.layer.stu
+        op.__class__ = type("Op", (type(op),), {"new_cache": lambda self, batch, device: super(type(self), self).new_cache(batch, device)})
+        y2, cache2 = blk(x.clone(), use_cache=True)
+    assert torch.equal(y, y2) and all(torch.equal(a, b) for a, b in zip(cache, cache2))
+
+
 @pytest.mark.parametrize("T", [1, 63, 96, 97, 126, 127, 128])
 def test_a_new_cache_is_zero_behind_the_prefill(T):
     """Histories and rings are allocated without zeros where the prefill writes over them: what lies behind it is zero whatever the
