@@ -41,8 +41,10 @@ __global__ void __launch_bounds__(TX * 16, 24 / TX) full_conv_kernel(const float
   __shared__ __align__(16) float xs[2][2][ST][PX];   // [buffer][parity][s][channel]
   __shared__ f32x2 taps[2][NT];                      // each twice: both halves of an operand
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-  const int k = blockIdx.x % K, c0 = blockIdx.x / K * CT;
-  const int tm = tiles_m - 1 - (int)blockIdx.y;      // the longest sums of all channels and filters first
+  // one dimension holds any number of tiles; the longest sums of all channels and filters first
+  const unsigned per_tile = gridDim.x / (unsigned)tiles_m, at = blockIdx.x % per_tile;
+  const int k = at % K, c0 = at / K * CT;
+  const int tm = tiles_m - 1 - (int)(blockIdx.x / per_tile);
   const int m0 = (t0 >> 1) + tm * MT;
   const int s_end = min(m0 + MT, (t_end + 1) >> 1);  // inputs that some output of the tile needs
 
@@ -188,13 +190,15 @@ extern "C" int stu_full_conv(const void* hist, int Lh, const void* phi, int L, i
   if (Lh % 4 || !aligned16(hist)) return STU_ERR_ALIGN;
   const long long rows = (long long)B * d;
   const int tiles_m = (((t_end + 1) >> 1) - (t0 >> 1) + MT - 1) / MT;
-  if (rows > (1 << 21) || (rows + 31) / 32 * K > 0x7fffffffll || tiles_m > 65535) return STU_ERR_UNSUPPORTED;   // the grid
+  const int ct = rows <= 16 ? 16 : 32;   // channels per CTA
+  const long long ctas = (rows + ct - 1) / ct * K * tiles_m;
+  if (rows > (1 << 21) || ctas > 0x7fffffffll) return STU_ERR_UNSUPPORTED;   // the grid (its outputs would be 500 GB)
   cudaStream_t st = (cudaStream_t)stream;
   // 32 channels per CTA, 16 where half of them would be padding (narrow layers of one sequence)
 #define STU_FULL_CONV(TX_)                                                                                         \
-  full_conv_kernel<TX_><<<dim3((unsigned)((rows + 4 * TX_ - 1) / (4 * TX_) * K), tiles_m), TX_ * 16, 0, st>>>(     \
+  full_conv_kernel<TX_><<<(unsigned)ctas, TX_ * 16, 0, st>>>(                                                      \
       (const float*)hist, Lh, (const float*)phi, L, K, (float*)U, ldU, (int)rows, d, both_signs, t0, t_end, tiles_m)
-  if (rows <= 16) STU_FULL_CONV(4);
+  if (ct == 16) STU_FULL_CONV(4);
   else STU_FULL_CONV(8);
 #undef STU_FULL_CONV
   STU_CHECK_LAUNCH();

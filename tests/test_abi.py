@@ -106,6 +106,16 @@ def test_extension_module_calls_the_same_functions():
     assert used <= exported, used - exported
 
 
+def test_long_inputs_of_the_fp32_convolutions_are_not_refused():
+    """More tiles of positions than a grid's second dimension holds.  (The addresses are dummies: only where no launch can reach them.)"""
+    import torch
+    from flash_stu_2_b200 import _lib
+    if torch.cuda.is_available():
+        pytest.skip("would be launched")
+    call = lambda t_end: _lib.load().stu_full_conv(0x10000, t_end // 2 + 4 & ~3, 0x10000, 64, 2, 0x10000, 16, 1, 8, 0, 0, t_end, 0, None)
+    assert call(1000) > 0 and call(9_000_000) == call(1000)   # CUDA's own error: no device
+
+
 def test_a_missing_extension_module_is_reported_like_a_missing_library(monkeypatch):
     import sys
     import flash_stu_2_b200
