@@ -12,6 +12,13 @@ def _inplace_target(x: torch.Tensor):
     return x if x.is_contiguous() else x.contiguous()
 
 
+def _own_step(stu, mlp) -> bool:
+    """Whether the parts of a token step are the classes' own (asked in every step of a small layer, so by type where that will do)."""
+    if type(stu) is STU and type(mlp) is MLP:
+        return "decode_step" not in stu.__dict__ and "apply_residual" not in mlp.__dict__
+    return own(stu, STU, "decode_step") and own(mlp, MLP, "apply_residual")
+
+
 class STULayer(nn.Module):
     def __init__(self, config, phi, n):
         super().__init__()
@@ -119,7 +126,7 @@ class STULayer(nn.Module):
         stu, mlp = child(self, "stu"), child(self, "mlp")
         stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
         if x.dtype == torch.float32 and stu.use_approx and not stu.use_hankel_L and ops.can_fuse_norm(
-                B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype) and own(stu, STU, "decode_step") and own(mlp, MLP, "apply_residual"):
+                B, mlp.intermediate_size, d, ops.EPI_GELU_MUL, x.dtype) and _own_step(stu, mlp):
             done = stu.layer_step_f32(x2, mid, entry, stu_norm, mlp_norm, mlp)
             if done == 1:
                 mlp.apply_residual(mid, mid, x2, norm_w=param(mlp_norm, "weight"), eps=mlp_norm.eps, overlap=True)

@@ -72,7 +72,11 @@ def child(module: nn.Module, name: str) -> nn.Module:
 
 def own(module: nn.Module, cls, *methods: str) -> bool:
     """Whether these methods of a module are the class's own: nobody who overrides one is passed by."""
-    return all(getattr(type(module), m, None) is getattr(cls, m) and m not in vars(module) for m in methods)
+    of, mine = type(module), module.__dict__
+    for m in methods:
+        if m in mine or (of is not cls and getattr(of, m, None) is not getattr(cls, m)):
+            return False
+    return True
 
 
 def _cache_for_prefill(op, cls, batch: int, device, filled: int):
