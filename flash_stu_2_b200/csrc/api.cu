@@ -16,6 +16,7 @@ enum { BACKEND_AUTO = 0, BACKEND_SIMT = 1, BACKEND_TCGEN05 = 2, BACKEND_SKINNY =
 //               starting at time hist_t0, N channels, hist_Lh elements per parity row)
 //            5: y[m*y_row_stride + (n / hist_T) * resid_row_stride + (n % hist_T)] = acc  (columns in blocks of hist_T,
 //               blocks resid_row_stride elements apart; resid itself is not read)
+//            +0x2000 (with 5): row m of x is zero behind column K - hist_Lh + m / hist_t0
 // norm_w != NULL asks for x to be RMS-normalised (eps) on the way in; only the decode (skinny) path
 // fuses this, other shapes return STU_ERR_UNSUPPORTED so that the caller normalises separately.
 static int g_pdl = -1;   // -1: not decided yet (environment), 0 off, 1 on
@@ -47,13 +48,15 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
   const int causal = (epilogue & EPI_FLAG_CAUSAL) ? 1 : 0;
   const int pdl = epilogue & (STU_FLAG_OVERLAP | STU_FLAG_EARLY_TRIGGER);  // honoured by the skinny kernels only
   const bool kpos = (epilogue & EPI_FLAG_KPOS) != 0;   // honoured by the tcgen05 GEMM; the zeros are there all the same
-  epilogue &= ~(EPI_FLAG_CAUSAL | EPI_FLAG_KPOS | STU_FLAG_OVERLAP | STU_FLAG_EARLY_TRIGGER);
+  const bool toeplitz = (epilogue & EPI_FLAG_TOEPLITZ) != 0;   // honoured by the tcgen05 GEMM, like kpos
+  epilogue &= ~(EPI_FLAG_CAUSAL | EPI_FLAG_KPOS | EPI_FLAG_TOEPLITZ | STU_FLAG_OVERLAP | STU_FLAG_EARLY_TRIGGER);
   if (kpos && (epilogue != EPI_STORE || !resid)) return STU_ERR_UNSUPPORTED;
   if ((epilogue < EPI_STORE || epilogue > EPI_HIST) && epilogue != EPI_BLOCKCOL) return STU_ERR_UNSUPPORTED;
   // EPI_BLOCKCOL: hist_T = columns per block, resid_row_stride = distance between blocks (elements); resid unused
-  // (hist_Lh > 0: row m of x is zero from column K - hist_Lh + m / hist_t0 + 1 on; the tcgen05 GEMM skips what it can)
-  if (epilogue == EPI_BLOCKCOL && (hist_T <= 0 || resid_row_stride <= 0 || hist_Lh < 0 || hist_Lh > K || (hist_Lh && hist_t0 <= 0)))
-    return STU_ERR_SHAPE;
+  if (epilogue == EPI_BLOCKCOL && (hist_T <= 0 || resid_row_stride <= 0)) return STU_ERR_SHAPE;
+  // EPI_FLAG_TOEPLITZ: hist_Lh = width of the triangular part, hist_t0 = rows per position
+  if (toeplitz && epilogue != EPI_BLOCKCOL) return STU_ERR_UNSUPPORTED;
+  if (toeplitz && (hist_Lh <= 0 || hist_Lh > K || hist_t0 <= 0)) return STU_ERR_SHAPE;
   if (epilogue == EPI_GELU_MUL && !W2) return STU_ERR_NULL;
   if (epilogue == EPI_RESID && !resid) return STU_ERR_NULL;
   if (epilogue == EPI_HIST && (hist_T <= 0 || hist_Lh <= 0 || hist_t0 < 0 || (M % hist_T) != 0 ||
@@ -70,6 +73,7 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
   ep.t0 = hist_t0;
   ep.Lh = hist_Lh;
   ep.ld2 = (epilogue == EPI_BLOCKCOL) ? resid_row_stride : 0;
+  if (epilogue == EPI_BLOCKCOL && !toeplitz) ep.t0 = ep.Lh = 0;
   if (kpos) {
     ep.kpos = (const int*)resid;
     ep.resid = nullptr;

@@ -29,6 +29,8 @@ template <int EPI> struct PdlTrigger {
 #define EPI_FLAG_CAUSAL 0x100
 // ... : W[n][k] = 0 for k > t / 2, t the position that `resid` (not a residual then) points to on the device
 #define EPI_FLAG_KPOS 0x1000
+// ... (EPI_BLOCKCOL): row m of x is zero behind column K - hist_Lh + m / hist_t0
+#define EPI_FLAG_TOEPLITZ 0x2000
 
 template <typename T> struct EpiArgs {
   T* y;

@@ -238,7 +238,7 @@ __device__ __forceinline__ int tile_kb(int num_kb, int n0, int causal, int bn) {
   return need < num_kb ? need : num_kb;
 }
 
-// Column blocks with ep.Lh > 0: row m of A is zero from column K - Lh + m / t0 + 1 on (the Toeplitz part of the distilled-LDS features,
+// Column blocks with ep.Lh > 0 (EPI_FLAG_TOEPLITZ): row m of A is zero from column K - Lh + m / t0 + 1 on (the Toeplitz part of the distilled-LDS features,
 // t0 rows per position): the k-blocks behind the last row's are skipped (6144 x 48128 x 320, half of whose rows need 256: 184 -> 174 us).
 template <int EPI>
 __device__ __forceinline__ int row_kb(int kb, const EpiArgs<bf16>& ep, int tm, int M, int K) {

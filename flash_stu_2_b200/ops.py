@@ -15,6 +15,7 @@ from . import _lib
 
 EPI_STORE, EPI_RESID, EPI_GELU_MUL, EPI_HIST = 0, 1, 2, 3
 EPI_FLAG_CAUSAL = 0x100  # OR-ed into the epilogue: the weight is lower triangular
+EPI_FLAG_TOEPLITZ = 0x2000   # ... the last columns of x are a Toeplitz matrix's lower triangle (lds_chunk_features)
 EPI_FLAG_KPOS = 0x1000   # ... the weight is zero past column t / 2 (linear(kpos=): the position t on the device)
 # Overlapped (programmatic dependent) launches of the decode kernels: OR-ed into the epilogue code of linear() and
 # passed as flags to decode_approx().  FLAG_OVERLAP: the kernel may start while its predecessor in the stream is
@@ -707,7 +708,7 @@ def lds_chunk_features(W, Zb, U2, d: int, Ck: int, F: int, causal: bool = False)
     assert N % d == 0 and U2.shape == (N // d * Ck, F * d) and U2.dtype == W.dtype == Zb.dtype
     status_word(W.device)
     rc = _lib.native().stu_linear(W.data_ptr(), KZ, Zb.data_ptr(), KZ, 1, None, None, Ck * F * d, U2.data_ptr(), d,
-                                  Mrows, N, KZ, 5, d, F if causal else 0, Ck if causal else 0, None, 0.0, _dt(W), BACKEND_AUTO,
+                                  Mrows, N, KZ, 5 | (EPI_FLAG_TOEPLITZ if causal else 0), d, F, Ck, None, 0.0, _dt(W), BACKEND_AUTO,
                                   _stream())
     _lib.check(rc, "stu_linear (LDS feature scatter)")
     _count()

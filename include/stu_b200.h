@@ -78,7 +78,8 @@ int stu_embed(const long long* ids, const void* table, void* out, int rows, int 
  * programmatic stream serialization: the kernel fetches W (which the preceding kernel must not write) while that
  * kernel drains, and reads x only after it has completed (skinny shapes, M <= 64; ignored otherwise);
  * 0x400 = let the next 0x200 launch start at once; 0x1000 (epilogue 0) = W is zero past column t / 2, `resid` points to
- * the position t (int) on the device: those columns may be left unread. */
+ * the position t (int) on the device: those columns may be left unread; 0x2000 (epilogue 5) = row m of x is zero behind column
+ * K - hist_Lh + m / hist_t0: those columns may be left unread (without it hist_t0 and hist_Lh are not looked at). */
 int stu_linear(const void* x, long long x_row_stride, const void* W, long long w_row_stride, long long w_k_stride,
                const void* W2, const void* resid, long long resid_row_stride, void* y, long long y_row_stride,
                int M, int N, int K, int epilogue, int hist_T, int hist_t0, int hist_Lh, const void* norm_w,
@@ -261,8 +262,8 @@ int stu_lds_final_state(const void* hist, double* h, const double* A, const doub
  * state, rotated into a balanced basis (z = Vs^T h, Vs [D][R] float64), and the chunk's inputs into
  * Z [B][ceil(Tn/Ck)][d][KZ] (bf16: z_hi | z_lo | z_hi | x, KZ = 3R+Ck; fp32: z | x, KZ = R+Ck), and the final state into
  * hfin [B*d][D] (bit-identical to stu_lds_final_state).  The features of all chunks of a sequence are then ONE
- * stu_linear call with epilogue 5 on Z (hist_t0 = F and hist_Lh = Ck there say that row m of the operand is zero behind
- * column K - Ck + m / F, so that those blocks may be skipped; 0, 0: nothing is known) (see flash_stu_2_b200/mini_stu.py for the constant operand).  R % 8 == 0,
+ * stu_linear call with epilogue 5 | 0x2000, hist_t0 = F and hist_Lh = Ck (see flash_stu_2_b200/mini_stu.py for the
+ * constant operand).  R % 8 == 0,
  * Ck % 8 == 0, D <= 256.  dtype | 0x1000: the caller has checked that every Bv[n] is exactly 1 (faster kernel, same
  * bits). */
 int stu_lds_chunk_scan(const void* x, long long x_bstride, long long x_tstride, const double* A, const double* Bv,

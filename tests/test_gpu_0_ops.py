@@ -1349,9 +1349,12 @@ def test_lds_features_skip_what_a_toeplitz_operand_leaves_out(dt, d, nch, Ck, F,
     Z = torch.randn(nch * d, K, device=dev(), generator=g).to(dt)
     a, b = (torch.full((nch * Ck, F * d), 7.0, dtype=dt, device=dev()) for _ in range(2))
     ops.lds_chunk_features(W, Z, a, d, Ck, F, causal=True)
-    ops.lds_chunk_features(W, Z, b, d, Ck, F)
+    ops.lds_chunk_features(W, Z, b, d, Ck, F)   # (says nothing of W: its hist_t0 and hist_Lh are not looked at)
     ops.check_status()
     assert torch.equal(a, b)
+    full = torch.randn(Ck * F, K, device=dev(), generator=g).to(dt)
+    ops.lds_chunk_features(full, Z, b, d, Ck, F)
+    close(b, (full.double() @ Z.double().t()).view(Ck, F, nch, d).permute(2, 0, 1, 3).reshape(nch * Ck, F * d), 1e-5 if dt == torch.float32 else 2 ** -8)
     want = (W.double() @ Z.double().t()).view(Ck, F, nch, d).permute(2, 0, 1, 3).reshape(nch * Ck, F * d)
     close(a, want, 1e-5 if dt == torch.float32 else 2 ** -8)
 
