@@ -181,6 +181,11 @@ __global__ void __launch_bounds__(256) kv_ring_write_kernel(const T* __restrict_
 // head (no one reads that slot in this launch: it held key t-W, outside the window), and the last CTA advances the positions.
 constexpr int DEC_STAGE = 4 * 2 * 256;   // 16-byte vectors of a round: 4 of keys and 4 of values per thread
 constexpr int DEC_RING_BYTES = 2 * DEC_STAGE * 16;
+// Keys that one CTA takes alone, and at least where several share them.  What a cluster's meeting and every CTA's merge cost shows
+// where keys are few: us, 12 heads of 128 of 4 sequences, 2, 61, 161 and 251 keys shared by all 8 CTAs whatever their number 7.0, 7.1, 7.1 and
+// 7.3; at least 128 keys each 3.4, 5.1, 7.3 and 8.2; this rule 3.4, 5.1, 6.8 and 7.1 (1 sequence 5.4, 5.4, 5.4, 5.5 and 3.1, 3.8, 5.0, 5.2; one CTA
+// of the form with 16 lanes per key 2.5, 3.5, 5.4 and 6.7).
+constexpr int DEC_ALONE = 128, DEC_PART_KEYS = 64;
 
 template <typename T> struct Vec16 {
   uint4 raw;
@@ -195,6 +200,25 @@ template <> __device__ __forceinline__ void Vec16<bf16>::unpack(float* f) const 
   for (int i = 0; i < 4; i++) {
     f[2 * i] = __uint_as_float(w[i] << 16);
     f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+
+// Sums acc[0 .. N - 1] over the lanes that differ in the bits O, 2 O, .. 16, each of them keeping a share: the values from the returned
+// index on end up in acc[0 ..].  (Every lane summing all of them took 96 shuffles for 32 values, this takes 28.)
+template <int N, int O> __device__ __forceinline__ int sum_shares(float* acc, int lane) {
+  if constexpr (O >= 32) {
+    return 0;
+  } else if constexpr (N == 1) {
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], O);
+    return sum_shares<1, 2 * O>(acc, lane);
+  } else {
+    const bool upper = (lane & O) != 0;
+#pragma unroll
+    for (int e = 0; e < N / 2; e++) {
+      const float give = upper ? acc[e] : acc[N / 2 + e];
+      acc[e] = (upper ? acc[N / 2 + e] : acc[e]) + __shfl_xor_sync(0xffffffffu, give, O);
+    }
+    return (upper ? N / 2 : 0) + sum_shares<N / 2, 2 * O>(acc, lane);
   }
 }
 
@@ -235,7 +259,10 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
   const T* cur = qkv + (size_t)b * 3 * d + h * HD;   // q | k | v of the new token, this head
   const int j_lo = max(0, t0 - window);
   const int nkeys = t0 - j_lo + 1;  // the new token included
-  const int chunk = ((nkeys + splits - 1) / splits + 7) & ~7;
+  // few keys are not worth a meeting: the CTAs past the first `parts` of the cluster leave (its barrier waits for none that has)
+  const int parts = nkeys <= DEC_ALONE ? 1 : min(splits, (nkeys + DEC_PART_KEYS - 1) / DEC_PART_KEYS);
+  if (part >= parts) return;
+  const int chunk = ((nkeys + parts - 1) / parts + 7) & ~7;
   const int k_end = min(nkeys, (part + 1) * chunk);   // this CTA's keys: part * chunk .. k_end - 1
   const size_t ring_b = (size_t)b * W;
   // Keys and values travel global -> shared memory by 16-byte asynchronous copies, two rounds in flight per thread: every
@@ -344,7 +371,14 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
     }
     issue(it + 2, it & 1);   // refill the slots just read
   }
-  {   // the groups of the warp: to their common maximum, then summed
+  if (niter == 0) {   // (warp-uniform)
+    if (lane == 0) {
+      s_m[warp] = -INFINITY;
+      s_l[warp] = 0.f;
+    }
+#pragma unroll
+    for (int e = lane; e < HD; e += 32) s_acc[warp][e] = 0.f;
+  } else {   // the groups of the warp: to their common maximum, then summed, every group keeping its share of the values
     float M = m;
 #pragma unroll
     for (int o = G; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
@@ -353,21 +387,15 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
 #pragma unroll
     for (int e = 0; e < NV * VPL; e++) acc[e] *= w;
 #pragma unroll
-    for (int o = G; o < 32; o <<= 1) {
-      l += __shfl_xor_sync(0xffffffffu, l, o);
-#pragma unroll
-      for (int e = 0; e < NV * VPL; e++) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-    }
+    for (int o = G; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    const int first = sum_shares<NV * VPL, G>(acc, lane);
     if (lane == 0) {
       s_m[warp] = M;
       s_l[warp] = l;
     }
-    if (grp == 0) {
+    constexpr int SHARE = NV * VPL > KPW ? NV * VPL / KPW : 1;
 #pragma unroll
-      for (int i = 0; i < NV; i++)
-#pragma unroll
-        for (int e = 0; e < VPL; e++) s_acc[warp][(i * G + sub) * VPL + e] = acc[i * VPL + e];
-    }
+    for (int e = 0; e < SHARE; e++) s_acc[warp][((first + e) / VPL * G + sub) * VPL + (first + e) % VPL] = acc[e];
   }
   if (update_cache && part == 0) {  // this head's slice of the new key and value
     const size_t slot = (ring_b + (size_t)(t0 % W)) * d + h * HD;
@@ -390,7 +418,7 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
       den = fmaf(s_l[g], w, den);
     }
   }
-  if (splits > 1) {
+  if (parts > 1) {
     if (threadIdx.x < HD) c_acc[threadIdx.x] = num;
     if (threadIdx.x == 0) {
       c_m = M;
@@ -401,9 +429,9 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
     if (part == 0 && threadIdx.x < HD) {
       float ms[8];
       M = -INFINITY;
-      for (int r = 0; r < splits; r++) M = fmaxf(M, ms[r & 7] = *cluster.map_shared_rank(&c_m, r));
+      for (int r = 0; r < parts; r++) M = fmaxf(M, ms[r & 7] = *cluster.map_shared_rank(&c_m, r));
       num = den = 0.f;
-      for (int r = 0; r < splits; r++) {
+      for (int r = 0; r < parts; r++) {
         const float lr = *cluster.map_shared_rank(&c_l, r);
         const float w = ms[r & 7] > -INFINITY ? __expf(ms[r & 7] - M) : (lr == lr ? 0.f : lr);
         num = fmaf(cluster.map_shared_rank(c_acc, r)[threadIdx.x], w, num);
@@ -424,7 +452,8 @@ static bool launch_swa_decode(const void* qkv, void* k_ring, void* v_ring, int* 
                               cudaStream_t st, int* rc) {
   constexpr int VPL = 16 / sizeof(T);
   if (hd % VPL || !aligned16(qkv) || !aligned16(k_ring) || !aligned16(v_ring) || !aligned16(out)) return false;
-  // CTAs per (head, sequence): while the grid stays below three per SM, what shared memory holds, and each keeps 128 keys.  us, bf16 heads
+  // CTAs per (head, sequence), of which the kernel uses those that the keys of the moment are worth: while the grid stays below three
+  // per SM, what shared memory holds, and each keeps 128 keys of a full window.  us, bf16 heads
   // of 128, window 1024, 1 / 2 / 4 / 8 CTAs: 12 heads of 1 sequence 16.1 / 11.1 / 8.4 / 8.0, 8: 18.9 / 17.9 / 15.8 / 23.2, 16: 24.5 / 24.1 / 29.5, 24: 32.8 /
   // 40.7, 32: 40.1 / 45.2; 129 keys of 4 heads of 32: 3.6 / 4.7.  (One CTA of the form with 16 lanes per key: 21.7, 24.6, 29.9, -, 41.1; 5.7.)
   int splits = 1;

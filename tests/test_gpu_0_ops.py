@@ -46,9 +46,10 @@ def _lin_ref(x, W, W2, resid, epi, dt):
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B,H,hd,window,t", [(1, 4, 32, 255, 900), (1, 3, 64, 511, 3), (2, 5, 64, 1024, 1024), (1, 2, 128, 1024, 5000),
                                              (3, 2, 128, 300, 301), (1, 1, 16, 2047, 1500), (40, 8, 64, 300, 120), (1, 2, 128, 1500, 127),
-                                             (2, 3, 32, 20, 21), (1, 2, 64, 0, 7)])
+                                             (2, 3, 32, 20, 21), (1, 2, 64, 0, 7), (1, 2, 128, 1500, 128), (2, 2, 64, 1024, 0),
+                                             (1, 4, 128, 1024, 320), (1, 1, 32, 2047, 190), (2, 1, 16, 1024, 5)])
 def test_attention_decode_shares_keys(dt, B, H, hd, window, t):
-    """One cached token: keys of a head shared by 1 to 8 CTAs, some of them without any; rings that have wrapped and rings that are
+    """One cached token: keys of a head shared by 1 to 8 CTAs, some of them without any, all of a cluster or its first ones; rings that have wrapped and rings that are
     not full; 64- to 512-byte rows.  Against the formula in float64 on the same rounded inputs; the output is rounded once (bf16: 2^-8
     of its row's largest, and the hardware tanh's 2^-11 on scores up to 6)."""
     from flash_stu_2_b200 import ops
