@@ -72,8 +72,10 @@ __global__ void __launch_bounds__(256) lds_final_state_kernel(const T* __restric
 // state per channel read and written (whole sectors), 6 MMAs for 48 features.  (The first form of this kernel gave a
 // warp one channel and its lanes the features: 2 * D float64 FMAs per lane, each with a shared-memory read of C and a
 // float -> double conversion; the 12-layer stack spent most of its token step there.)
-// The constants are staged ahead of the wait for the kernel in front (programmatic launch), the next 16 states of a lane are under way
-// while the last are multiplied, and positions move on here: 16 x 1024 channels with the contraction behind it 59.1 -> 54.6 us a step.
+// Under STU_FLAG_OVERLAP the constants are staged ahead of the wait for the kernel in front (programmatic launch).  The next 16 states of
+// a lane are under way while the last are multiplied, and positions move on here.  us, alone and with the contraction behind it: 16 x 1024
+// channels 21.0 and 46.1 (one launch after the other, the states in three rounds 24.0 and 54.3), 8 x 1024 14.2 and 40.7 (18.7 and 45.1).  Constants
+// staged one load after the other cost 7 us of it: 28.7 and 21.9 alone.
 constexpr int LDS_NTF = LDS_MAXF / 8;   // n-tiles of 8 features
 
 __device__ __forceinline__ void dmma_884(double& c0, double& c1, double a, double b) {
@@ -86,15 +88,30 @@ template <typename T>
 __global__ void __launch_bounds__(256) lds_decode_kernel(const T* __restrict__ x, long long x_rstride,
                                                          double* __restrict__ h, const double* __restrict__ A,
                                                          const double* __restrict__ Bv, const T* __restrict__ C,
-                                                         T* __restrict__ U, int* __restrict__ pos, int B, int d, int D, int F) {
+                                                         T* __restrict__ U, int* __restrict__ pos, int B, int d, int D, int F, int overlap) {
   extern __shared__ __align__(16) unsigned char lds_smem[];
   const int Dp = (D + 3) & ~3, Fp = 8 * ((F + 7) / 8) + 4;
   double* Cs = reinterpret_cast<double*>(lds_smem);   // [Dp][Fp], zero outside [D][F]
   double* As = Cs + (size_t)Dp * Fp;                  // [Dp]
   double* Bs = As + Dp;                               // [Dp]
-  pdl_trigger();   // the constants come in while the kernel before this one drains; inputs and states behind the wait
-  for (int n = threadIdx.x >> 5; n < Dp; n += 8)
-    for (int f = threadIdx.x & 31; f < Fp; f += 32) Cs[n * Fp + f] = (n < D && f < F) ? (double)Elem<T>::to_f(C[n * F + f]) : 0.0;
+  if (overlap) pdl_trigger();   // the constants come in while the kernel before this one drains; inputs and states behind the wait
+  {   // (eight loads of a thread under way at a time)
+    const int sn = 256 / Fp, sf = 256 - sn * Fp;
+    int n = threadIdx.x / Fp, f = threadIdx.x - n * Fp;
+    for (int e0 = threadIdx.x; e0 < Dp * Fp; e0 += 8 * 256) {
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        v[k] = (n < D && f < F) ? Elem<T>::to_f(C[n * F + f]) : 0.f;
+        n += sn;
+        f += sf;
+        if (f >= Fp) f -= Fp, n++;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (e0 + k * 256 < Dp * Fp) Cs[e0 + k * 256] = (double)v[k];
+    }
+  }
   for (int n = threadIdx.x; n < Dp; n += 256) {
     As[n] = n < D ? A[n] : 0.0;
     Bs[n] = n < D ? Bv[n] : 0.0;
@@ -367,13 +384,13 @@ extern "C" int stu_lds_decode_step(const void* x, long long x_row_stride, double
     e = allow_smem((const void*)lds_decode_kernel<float>, smem, limit);
     if (e != cudaSuccess) return (int)e;
     e = launch_maybe_overlapped(lds_decode_kernel<float>, dim3((rows + 63) / 64), dim3(256), smem, st, overlap, (const float*)x,
-                                x_row_stride, h, A, Bv, (const float*)C, (float*)U, pos, B, d, D, F);
+                                x_row_stride, h, A, Bv, (const float*)C, (float*)U, pos, B, d, D, F, overlap ? 1 : 0);
   } else if (dtype == STU_BF16) {
     static SmemLimit limit;
     e = allow_smem((const void*)lds_decode_kernel<bf16>, smem, limit);
     if (e != cudaSuccess) return (int)e;
     e = launch_maybe_overlapped(lds_decode_kernel<bf16>, dim3((rows + 63) / 64), dim3(256), smem, st, overlap, (const bf16*)x,
-                                x_row_stride, h, A, Bv, (const bf16*)C, (bf16*)U, pos, B, d, D, F);
+                                x_row_stride, h, A, Bv, (const bf16*)C, (bf16*)U, pos, B, d, D, F, overlap ? 1 : 0);
   } else {
     return STU_ERR_DTYPE;
   }

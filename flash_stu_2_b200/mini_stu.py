@@ -218,6 +218,19 @@ class MiniSTU(nn.Module):
                     raise
                 G = (G + 1) // 2
 
+    @staticmethod
+    def _lds_early(B: int, d: int, dtype: torch.dtype):
+        """Whether a step's state kernel and its contraction start beside the kernels in front of them.  Up to 8 rows the contraction is one
+        wave of CTAs that share its SMs evenly only if they come to an idle GPU: beside the state kernel's CTAs (64 channels each) some
+        SMs get two and others none.  That pays while those are few, and for the tensor-core contraction of more rows, whose CTAs are short.
+        us a step, neither and both: bf16 to d outputs, 16 x 1024 49.3 and 46.1, 9 x 1024 40.6 and 39.0, 1 x 1024 40.2 and 36.3, 5 x 256 19.6 and 15.6, 6 x 256
+        19.7 and 21.7, 3 x 512 23.4 and 25.4, 8 x 1024 40.7 and 43.4; fp32 the state kernel alone: 8 x 128 20.3 and 16.4, 1 x 1024 56.0 and 51.8 (both:
+        62.0), 4 x 256 23.9 and 24.4, 2 x 1024 54.6 and 52.1, 4 x 1024 56.7 and 61.7, 8 x 1024 84.8 and 122."""
+        ctas = -(-B * d // 64)
+        if dtype == torch.bfloat16:
+            return (B > 8 or B == 1 or ctas <= 20,) * 2
+        return ctas <= 16, False
+
     def _forward_lds(self, x, past_key_value=None, use_cache=False):
         before = self._lds_key
         op = self._lds_prepared()
@@ -233,10 +246,11 @@ class MiniSTU(nn.Module):
             known = op._prep_key
             _, Mcat = op.prepared_full()
             # constants that were there before this call are read ahead of the kernels in front: M's tiles while the state kernel runs
-            overlap = ops.overlap_decode and before is self._lds_key and known is op._prep_key
+            there = ops.overlap_decode and before is self._lds_key and known is op._prep_key
+            state, contraction = (there and early for early in self._lds_early(B, d, x.dtype))
             U = torch.empty(B, F_ * d, dtype=x.dtype, device=x.device)
-            ops.lds_decode_features(x.view(B, d), h, A32, B32, Cm, U, pos, overlap)
-            y = ops.linear(U, Mcat, epilogue=ops.EPI_STORE | (ops.FLAG_OVERLAP if overlap else 0)).view(B, 1, self.output_dim)
+            ops.lds_decode_features(x.view(B, d), h, A32, B32, Cm, U, pos, state)
+            y = ops.linear(U, Mcat, epilogue=ops.EPI_STORE | (ops.FLAG_OVERLAP if contraction else 0)).view(B, 1, self.output_dim)
             pos._host_t = t + 1
             return (y, (h, pos)) if use_cache else y
         y = torch.empty(B, T, self.output_dim, dtype=x.dtype, device=x.device)

@@ -274,7 +274,7 @@ int stu_lds_chunk_scan(const void* x, long long x_bstride, long long x_tstride, 
 int stu_lds_decode_features(const void* x, long long x_row_stride, double* h, const double* A, const double* Bv,
                             const void* C, void* U, int B, int d, int D, int F, int dtype, void* stream);
 /* The same, and every sequence's position in pos [B][2] moves on (pos may be NULL).  With STU_FLAG_OVERLAP (0x200) in dtype A, Bv and C
- * are read while the kernel before this one in the stream may still be running: it must not be what writes them. */
+ * are read while kernels before this one in the stream may still be running (see stu_set_programmatic_launch): none of them may write these. */
 int stu_lds_decode_step(const void* x, long long x_row_stride, double* h, const double* A, const double* Bv, const void* C,
                         void* U, int* pos, int B, int d, int D, int F, int dtype, void* stream);
 

@@ -1233,6 +1233,29 @@ def test_mini_stu_lds_prefill_and_recurrent_decode(golden, dt, tol, shape):
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,d,D,F", [(1, 7, 160, 48), (2, 64, 161, 64), (3, 65, 3, 1), (1, 200, 256, 9), (5, 24, 64, 33), (2, 96, 100, 50)])
+def test_lds_state_step_of_any_size(dt, B, d, D, F):
+    """The recurrent step's state and features against float64, over its limits of modes and features: constants of sizes that divide
+    neither the block nor its staging rounds, channels that fill no CTA; two steps, plain and beside the kernels in front."""
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.modules import new_pos
+    g = torch.Generator(device=dev()).manual_seed(D + F)
+    rand = lambda *s: torch.randn(*s, device=dev(), generator=g, dtype=torch.float64)
+    A, Bv, C, h = rand(D).tanh(), rand(D), rand(D, F).to(dt), rand(B, d, D)
+    want = h.clone()
+    pos = new_pos(B, dev())
+    torch.cuda.synchronize()
+    for overlap in (False, True):
+        x, U = rand(B, d).to(dt), torch.full((B, F * d), 7.0, dtype=dt, device=dev())
+        ops.lds_decode_features(x, h, A, Bv, C, U, pos, overlap)
+        want = torch.addcmul(A * want, Bv, x.double()[..., None])
+        assert (h - want).abs().max() <= 1e-14 * want.abs().max()   # fma against product and sum
+        close(U.view(B, F, d), (h @ C.double()).transpose(1, 2), 1e-6 if dt == torch.float32 else 2 ** -8)
+    ops.check_status()
+    assert pos[:, 0].tolist() == [2] * B
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("S,ld,L", [(1, 1, 3), (7, 8, 40), (8, 8, 16), (9, 16, 9), (33, 35, 60), (264, 264, 700), (1024, 1024, 4096),
                                     (1025, 1032, 900), (2056, 2060, 5000)])
 def test_toeplitz_matrices_of_any_size(dt, S, ld, L):

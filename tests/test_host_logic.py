@@ -157,6 +157,14 @@ def test_lds_feature_rows_shrink_to_the_memory_there_is(monkeypatch):
         F.MiniSTU._lds_features(8, 1000, 1024, 16, x)
 
 
+@pytest.mark.parametrize("B,d,dt,early", [
+    (16, 1024, torch.bfloat16, (True, True)), (9, 64, torch.bfloat16, (True, True)), (8, 1024, torch.bfloat16, (False, False)),
+    (1, 2048, torch.bfloat16, (True, True)), (5, 256, torch.bfloat16, (True, True)), (6, 256, torch.bfloat16, (False, False)),
+    (8, 128, torch.float32, (True, False)), (4, 1024, torch.float32, (False, False)), (1, 1024, torch.float32, (True, False))])
+def test_which_lds_steps_start_beside_the_kernels_in_front(B, d, dt, early):
+    assert F.MiniSTU._lds_early(B, d, dt) == early
+
+
 def test_captures_of_two_threads_hold_the_collector_until_the_last_is_done():
     import gc
     from flash_stu_2_b200.model import _CollectionHeld
