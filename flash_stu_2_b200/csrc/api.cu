@@ -32,6 +32,7 @@ extern "C" int stu_set_programmatic_launch(int on) {
   return prev;
 }
 
+int device_sm_count();   // gemm_tc.cu
 bool skinny_umma_takes(int M, int N, int K, int epi, bool norm, bool peer);   // gemm_tc.cu
 
 // Small-M shapes for which the tcgen05 GEMM beats the weight-streaming kernel.
@@ -142,9 +143,14 @@ extern "C" int stu_linear_can_fuse_norm(int M, int N, int K, int epilogue, int d
   // gate/up kernel from its shared-memory copy); a separate norm kernel measured faster both times (24-layer model,
   // B = 32: 2.17 against 2.27 ms per token step, and 2.19 against 2.30 ms).  The kernels accept norm_w all the same.
   // (a fused norm inside the tcgen05 token-step kernel measured slower as well: 2.12-2.25 against 1.71-1.85 ms)
-  // 9..16 rows: the fused form is the weight-streaming kernel, the other the tcgen05 one behind a norm kernel, which is faster from
-  // 2.6 M weights on (us, 12 rows, fused and apart: 2304 x 768 4.1 and 5.0, gate/up 2048 x 512 3.6 and 5.1, 2560 x 640 6.7 and 5.7, 3072 x 768 7.4 and
-  // 6.0; 3072 x 1024 7.4 and 5.5, 4608 x 1536 16.8 and 7.4, gate/up 6144 x 1536 19.0 and 10.8)
-  if (M > 16 || (M > 8 && (long long)N * K * (epilogue == EPI_GELU_MUL ? 2 : 1) > 2600000)) return 0;
-  return 1;
+  if (M > 16) return 0;
+  if (M <= 8) return 1;
+  // 9..16 rows: the fused form is the weight-streaming kernel of 8 features per CTA, the other the tcgen05 one behind a norm kernel.  The
+  // former is the faster one while its CTAs are one wave, two per SM (one, of 16 warps, for K > 1024 without gate/up), and rows
+  // are not long.  us, 9 rows, fused and apart: gate/up 2368 x 768 4.3 and 5.8, 2432 x 768 6.2 and 5.8, 2048..2304 x 1024 4.8 and 6.4, 2304 x 1280 6.5
+  // and 7.6, 1536 x 1536 6.8 and 6.5; plain 2368 x 1024 4.1 and 5.6, 2432 x 1024 6.3 and 5.5, 1024 x 1152 4.0 and 5.5, 1536 x 1152 7.1 and 5.5, 1024 x 2048 5.0
+  // and 5.9, 1024 x 3072 6.9 and 6.8, 4608 x 1536 15.7 and 7.4
+  const long long wave = 8ll * device_sm_count();
+  if (epilogue == EPI_GELU_MUL) return N <= 2 * wave && K <= 1280;
+  return (N <= 2 * wave && K <= 1024) || (N <= wave && K <= 2048);
 }

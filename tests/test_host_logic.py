@@ -165,6 +165,15 @@ def test_which_lds_steps_start_beside_the_kernels_in_front(B, d, dt, early):
     assert F.MiniSTU._lds_early(B, d, dt) == early
 
 
+@pytest.mark.parametrize("M,N,K,epi,fused", [
+    (8, 50000, 4096, 0, True), (17, 512, 512, 0, False), (9, 2304, 768, 2, True), (16, 2048, 1024, 2, True), (12, 2440, 768, 2, False),
+    (12, 1536, 1536, 2, False), (9, 2304, 1024, 0, True), (16, 2440, 512, 0, False), (9, 1024, 2048, 0, True), (9, 1536, 1536, 0, False),
+    (16, 1024, 3072, 0, False), (12, 4608, 1536, 0, False)])
+def test_which_linears_fuse_their_norm(M, N, K, epi, fused):
+    from flash_stu_2_b200 import ops
+    assert ops.can_fuse_norm(M, N, K, epi, torch.bfloat16) is fused
+
+
 def test_captures_of_two_threads_hold_the_collector_until_the_last_is_done():
     import gc
     from flash_stu_2_b200.model import _CollectionHeld
