@@ -9,7 +9,8 @@
 // drain the accumulator with tcgen05.ld and run the fused epilogue (store / residual add / tanh-GELU gate * up / transposed
 // scatter into the projected history).  The kernel is persistent (one pair per two SMs walks the tile list) and the accumulator is
 // double-buffered in TMEM, so one tile's epilogue overlaps the next tile's main loop.  Every load is a plain load of this GPU's
-// own memory into the loading CTA's shared memory.
+// own memory into the loading CTA's shared memory.  Where tiles of 256 rows would fill their last wave badly, CTAs alone on tiles of
+// 128 x 256 take their place (tile_form).
 // One CTA per 128 x 256 or 128 x 128 tile, as it was before, and now (us, all back to back): 65536 x 1536 x 6144 938 -> 880,
 // gate/up 65536 x 6144 x 1536 1998 -> 1874, 65536 x 4608 x 1536 771 -> 656, 7996 x 3072 x 1024 47.3 -> 43.0, 1668 x 768 x 3072
 // 18.1 -> 12.0, 333 x 1536 x 6144 32.0 -> 18.3; smallest 4.3 -> 4.7 (256 x 256 x 64), before the launch became programmatic: barriers and tensor memory
@@ -147,7 +148,7 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
   d |= (uint64_t)2 << 61;                 // 128-byte swizzle
   return d;
 }
-// Instruction descriptor: D fp32, A/B bf16, both K-major, M = 128, N = the tile width (128 or 256).
+// Instruction descriptor: D fp32, A/B bf16, both K-major, M = 128, N = 256 (tiles of single CTAs) or the 16, 32 or 64 rows of a token step.
 template <int BN_>
 __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
   constexpr uint32_t IDESC =
@@ -241,9 +242,9 @@ __device__ __forceinline__ int tile_kb(int num_kb, int n0, int causal, int bn) {
 // Column blocks with ep.Lh > 0 (EPI_FLAG_TOEPLITZ): row m of A is zero from column K - Lh + m / t0 + 1 on (the Toeplitz part of the distilled-LDS features,
 // t0 rows per position): the k-blocks behind the last row's are skipped (6144 x 48128 x 320, half of whose rows need 256: 184 -> 174 us).
 template <int EPI>
-__device__ __forceinline__ int row_kb(int kb, const EpiArgs<bf16>& ep, int tm, int M, int K) {
+__device__ __forceinline__ int row_kb(int kb, const EpiArgs<bf16>& ep, int last_row, int K) {
   if (EPI != EPI_BLOCKCOL || ep.Lh <= 0) return kb;
-  return min(kb, (K - ep.Lh + (min((tm + 1) * 2 * BM, M) - 1) / ep.t0 + BK) / BK);
+  return min(kb, (K - ep.Lh + last_row / ep.t0 + BK) / BK);
 }
 
 // Tile order: bands of group_m row tiles, rows first inside a band (group_m = 1: row by row; tiles_m: column by
@@ -265,8 +266,10 @@ __host__ __device__ constexpr int stage_blocks(int mma_n) { return mma_n > 128 ?
 // Persistent kernel: pair i of CTAs handles tiles i, i + pairs, ...  The accumulator is double-buffered in TMEM
 // (2 x TN columns, or 2 x 256 for the two accumulators of the gate/up epilogue), so the MMA warp starts the next
 // tile while the epilogue warps drain the previous one.
-template <int EPI, int STAGES, int TN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS, 1)
+// CTAS = 1: the same with a CTA in the place of a pair, tiles of 128 rows (cta_group::1, all rows of B in its shared memory), for
+// products whose tiles of 256 rows would fill their last wave badly (see tile_form).
+template <int EPI, int STAGES, int TN, int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmY, int by_copy, int M, int N,
                    int K, int tiles_m, int tiles_n, int group_m, int causal, EpiArgs<bf16> ep, int* status,
@@ -276,7 +279,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
   constexpr int BN = TN;                       // output columns of a tile
   constexpr int MMA_N = DUAL ? 2 * BN : BN;    // accumulator columns
   constexpr int KBS = stage_blocks(MMA_N);
-  constexpr int KB_BYTES = A_BYTES + MMA_N / 2 * BK * 2;      // of one CTA: its rows of A, its half of B
+  constexpr bool PAIR = CTAS == 2;
+  constexpr int KB_BYTES = A_BYTES + MMA_N / CTAS * BK * 2;   // of one CTA: its rows of A, its half of B (or all of it)
   constexpr int STAGE_BYTES = KBS * KB_BYTES;
   constexpr uint32_t ACC_COLS = MMA_N;
   constexpr uint32_t TMEM_COLS = MMA_N > 128 ? 512 : 256;     // two accumulators, a power of two
@@ -293,7 +297,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
   unsigned char* blocks = smem + STAGES * STAGE_BYTES + 1024;   // one per epilogue warp, in the 128-byte swizzle
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int rank = PAIR ? blockIdx.x & 1 : 0, pair = blockIdx.x / CTAS, pairs = gridDim.x / CTAS;
   const int num_tiles = tiles_m * tiles_n;
   int num_kb = (K + BK - 1) / BK;
 
@@ -304,7 +308,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 2 * EPI_WARPS);   // of both CTAs
+      mbar_init(&tmem_empty[i], CTAS * EPI_WARPS);   // of both CTAs
     }
     abort_flag[0] = abort_flag[1] = 0;
     *issued_ctr = 0;
@@ -312,13 +316,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  pair_sync();
+  if constexpr (PAIR) pair_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   // launched programmatically: everything so far ran beside the end of the kernel in front; the next kernel may be made resident
@@ -338,8 +346,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
     for (int tile = pair; ok && tile < num_tiles; tile += pairs) {
       int tm, tn;
       tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
-      const int m0 = (2 * tm + rank) * BM, n0 = tn * BN + (DUAL ? 0 : rank * (BN / 2));
-      const int kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, tm, M, K);
+      const int m0 = (CTAS * tm + rank) * BM, n0 = tn * BN + (DUAL ? 0 : rank * (BN / 2));
+      const int kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, min((tm + 1) * CTAS * BM, M) - 1, K);
       for (int kb = 0; kb < kb_end; kb += KBS, g++) {
         if (!ready) ok = warp_wait(&empty_bar[s], ph, abort_flag, wait_ns);
         if (!ok) break;
@@ -349,7 +357,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
         if (leader) {
           const int n = min(KBS, kb_end - kb);
           unsigned char* sa = smem + s * STAGE_BYTES;
-          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * n * KB_BYTES);   // of both CTAs
+          if (rank == 0) mbar_expect_tx(&full_bar[s], CTAS * n * KB_BYTES);   // of both CTAs
           // drop_first_copy (failure-detection test only): the first stage's copies are never issued, so its
           // barrier never completes and the consumer's bounded wait has to run out
           if (!(drop_first_copy && g == 0)) {
@@ -357,8 +365,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
 #pragma unroll
             for (int j = 0; j < KBS; j++)
               if (j < n) {
-                tma_load_2d_pair(sa + j * KB_BYTES, &tmA, bar, (kb + j) * BK, m0);
-                tma_load_2d_pair(sa + j * KB_BYTES + A_BYTES, mapB, bar, (kb + j) * BK, n0);
+                unsigned char* sj = sa + j * KB_BYTES;
+                if constexpr (PAIR) {
+                  tma_load_2d_pair(sj, &tmA, bar, (kb + j) * BK, m0);
+                  tma_load_2d_pair(sj + A_BYTES, mapB, bar, (kb + j) * BK, n0);
+                } else {
+                  tma_load_2d(sj, &tmA, &full_bar[s], (kb + j) * BK, m0);
+                  tma_load_2d(sj + A_BYTES, &tmB, &full_bar[s], (kb + j) * BK, n0);
+                  if (DUAL) tma_load_2d(sj + A_BYTES + BN * BK * 2, &tmB2, &full_bar[s], (kb + j) * BK, n0);   // gate rows, up rows
+                }
               }
           }
         }
@@ -383,7 +398,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
         const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
         int tm, tn;
         tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
-        const int kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, tm, M, K);
+        const int kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, min((tm + 1) * CTAS * BM, M) - 1, K);
         ok = warp_wait(&tmem_empty[buf], (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
         if (!ok) break;
         for (int kb = 0; kb < kb_end; kb += KBS, g++) {
@@ -402,16 +417,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
             for (int j = 0; j < KBS; j++)
               if (j == 0 || kb + j < kb_end) {
 #pragma unroll
-                for (int kk = 0; kk < BK / 16; kk++)
-                  umma_pair<MMA_N>(acc_addr, da + j * (KB_BYTES >> 4) + 2 * kk, db + j * (KB_BYTES >> 4) + 2 * kk,
-                                   (kb | j | kk) ? 1u : 0u);
+                for (int kk = 0; kk < BK / 16; kk++) {
+                  const uint64_t dak = da + j * (KB_BYTES >> 4) + 2 * kk, dbk = db + j * (KB_BYTES >> 4) + 2 * kk;
+                  if constexpr (PAIR) umma_pair<MMA_N>(acc_addr, dak, dbk, (kb | j | kk) ? 1u : 0u);
+                  else umma<MMA_N>(acc_addr, dak, dbk, (kb | j | kk) ? 1u : 0u);
+                }
               }
-            umma_commit_pair(&empty_bar[s]);  // arrives when the MMAs above have finished reading this stage
+            // arrives when the MMAs above have finished reading this stage
+            if constexpr (PAIR) umma_commit_pair(&empty_bar[s]);
+            else umma_commit(&empty_bar[s]);
           }
           ready = __all_sync(0xffffffffu, ready1);
           s = s1, ph = ph1;
         }
-        if (ok && leader) umma_commit_pair(&tmem_full[buf]);
+        if (ok && leader) {
+          if constexpr (PAIR) umma_commit_pair(&tmem_full[buf]);
+          else umma_commit(&tmem_full[buf]);
+        }
         __syncwarp();
       }
       if (leader) *consumed_ctr = g;
@@ -441,7 +463,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
     for (int tile = pair; tile < num_tiles; tile += pairs, it++) {
       int tm, tn;
       tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
-      const int m0 = (2 * tm + rank) * BM, n0 = tn * BN;
+      const int m0 = (CTAS * tm + rank) * BM, n0 = tn * BN;
       const int first = m0 + quarter * 32, rows = min(32, M - first);   // this warp's rows
       const int buf = it & 1;
       const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
@@ -642,18 +664,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
   }
   __syncwarp();
   __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag) {   // tell the other CTA
-    store_to_cta(abort_flag + 1, rank ^ 1, 1);
-    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  if constexpr (PAIR) {
+    if (threadIdx.x == 0 && *abort_flag) {   // tell the other CTA
+      store_to_cta(abort_flag + 1, rank ^ 1, 1);
+      asm volatile("fence.acq_rel.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    pair_sync();   // neither CTA leaves while the other's instructions, copies' barriers or arrivals still use its memory
   }
-  __syncwarp();
-  pair_sync();   // neither CTA leaves while the other's instructions, copies' barriers or arrivals still use its memory
   if (abort_flag[0] || abort_flag[1]) {
     // A wait ran out.  Report it, then let copies that were issued but never consumed land (bounded)
     // before either CTA's shared memory is released.
     if (rank == 0 && threadIdx.x == 0) {
       if (status) atomicExch(status, 3);
-      const int issued = max(*issued_ctr, (int)load_from_cta(issued_ctr, 1)), consumed = *consumed_ctr;
+      const int issued = PAIR ? max(*issued_ctr, (int)load_from_cta(issued_ctr, 1)) : *issued_ctr, consumed = *consumed_ctr;
       const uint64_t drain_start = global_ns();
       for (int g = consumed; g < issued; g++) {
         const int s = g % STAGES;
@@ -665,11 +689,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS,
       }
     }
     __syncwarp();
-    pair_sync();
+    if constexpr (PAIR) pair_sync();
+    else __syncthreads();
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
   }
 }
 
@@ -771,11 +797,23 @@ int gemm_group_m(int tiles_n, int N, int K, bool dual) {
   return tiles_n > 24 && (long long)N * K * (dual ? 4 : 2) > (48ll << 20) ? 16 : 1;
 }
 
-// Pairs of CTAs that the current device runs at a time.
-int device_pairs(const void* kernel, size_t smem) {
+template <int EPI, int STAGES, int TN, int CTAS>
+constexpr size_t tc_smem() {
+  constexpr bool DUAL = (EPI == EPI_GELU_MUL);
+  constexpr size_t stage = (size_t)stage_blocks(DUAL ? 2 * TN : TN) * (A_BYTES + (DUAL ? 2 * TN : TN) / CTAS * BK * 2);
+  constexpr size_t bytes = STAGES * stage + 1024 + 1024 + EPI_WARPS * BLOCK_BYTES;
+  static_assert(bytes > 114 * 1024 && bytes <= 227 * 1024, "one CTA per SM, whatever the form: device_pairs");
+  return bytes;
+}
+
+// Pairs of CTAs that the current device runs at a time (every form of the kernel fills an SM).
+int device_pairs() {
   static std::atomic<int> found[STU_MAX_DEVICES] = {};
   std::atomic<int>& n = found[current_device()];
   if (n.load(std::memory_order_relaxed) == 0) {
+    const void* kernel = (const void*)gemm_tc_kernel<EPI_STORE, 6, 256, 2>;
+    constexpr size_t smem = tc_smem<EPI_STORE, 6, 256, 2>();
+    static SmemLimit limit;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * device_sm_count());
     cfg.blockDim = dim3(64 + 32 * EPI_WARPS);
@@ -787,7 +825,7 @@ int device_pairs(const void* kernel, size_t smem) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+    if (allow_smem(kernel, smem, limit) != cudaSuccess || cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
       (void)cudaGetLastError();
       clusters = device_sm_count() / 2;
     }
@@ -796,13 +834,12 @@ int device_pairs(const void* kernel, size_t smem) {
   return n.load(std::memory_order_relaxed);
 }
 
-template <int EPI, int STAGES, int TN>
+template <int EPI, int STAGES, int TN, int CTAS = 2>
 int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2, int M, int N, int K, int m_fast,
               int causal, const EpiArgs<bf16>& ep, int* status, cudaStream_t st) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
-  constexpr int STAGE_BYTES = stage_blocks(DUAL ? 2 * TN : TN) * (A_BYTES + (DUAL ? TN : TN / 2) * BK * 2);
   constexpr bool COPIES = (EPI == EPI_STORE || EPI == EPI_GELU_MUL || EPI == EPI_BLOCKCOL);
-  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 1024 + EPI_WARPS * BLOCK_BYTES;
+  constexpr size_t smem = tc_smem<EPI, STAGES, TN, CTAS>();
   // The output by tensor copies: rows on the 16-byte grid and of whole 16 bytes (a copy clips at those), and (column blocks) 64
   // columns inside one block of a whole number of them.  What gains is many outputs for little K: LDS features, 6144 x 48128 x
   // 320, 237 -> 204 us; products of K = 1024 and more hide either form.
@@ -810,13 +847,13 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   int by_copy = 0;
   if (COPIES && !ep.peer && ep.ldy % 8 == 0 && N % 8 == 0 && aligned16(ep.y) && (EPI != EPI_BLOCKCOL || (ep.Tseq % 64 == 0 && N % ep.Tseq == 0)))
     by_copy = make_output_map(&y, ep, EPI == EPI_BLOCKCOL, M, N) == STU_OK;
-  auto k = gemm_tc_kernel<EPI, STAGES, TN>;
+  auto k = gemm_tc_kernel<EPI, STAGES, TN, CTAS>;
   static SmemLimit limit;
   cudaError_t e = allow_smem((const void*)k, smem, limit);
   if (e != cudaSuccess) return (int)e;
-  const int tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + TN - 1) / TN;
-  const int tiles = tiles_m * tiles_n, pairs = device_pairs((const void*)k, smem);
-  const int grid = 2 * (tiles < pairs ? tiles : pairs);  // one persistent CTA per SM
+  const int tiles_m = (M + CTAS * BM - 1) / (CTAS * BM), tiles_n = (N + TN - 1) / TN;
+  const int tiles = tiles_m * tiles_n, most = CTAS == 2 ? device_pairs() : device_sm_count();
+  const int grid = CTAS * (tiles < most ? tiles : most);  // one persistent CTA per SM
   const int drop = g_drop_first_copy;
   g_drop_first_copy = 0;   // the injected fault applies to one launch
   const int group_m = m_fast ? tiles_m : gemm_group_m(tiles_n, N, K, DUAL);
@@ -1187,15 +1224,28 @@ bool gemm_tc_supported(const void* A, long long lda, const void* B, long long ld
 // narrow ones where all pairs are busy (65536 x 1536 x 6144, 21 waves against 42: 900 and 1034 us; 1.87 where only one pair is:
 // 256 rows, K = 16384, 76.5 and 41.0).  One wave of either, 1668 x 768 x 3072: narrow 12.0 us, wide 18.3; two wide ones against
 // four narrow, 7996 x 1024 x 4096: 66.6 and 58.7.
-// STU_B200_TILE_N=128 and 256 force either.
-static bool wide_tiles(long long rows, long long cols) {
-  static const char* env = getenv("STU_B200_TILE_N");
-  if (env && atoi(env) == 128) return false;
-  if (env && atoi(env) == 256) return true;
-  const long long sms = device_sm_count() / 2, tiles_m = (rows + 2 * BM - 1) / (2 * BM);
-  const long long wide = (tiles_m * ((cols + 255) / 256) + sms - 1) / sms;
-  const long long narrow = (tiles_m * ((cols + 127) / 128) + sms - 1) / sms;
-  return 174 * wide < 100 * narrow;
+// Tiles of 128 x 256 by single CTAs where those of 256 rows fill their last wave badly (M mod 256 up to 128, one wave against two): a wave of
+// them costs 1.10 to 1.17 of the pairs' wide ones (shared memory, see the head of this file), counted as 1.24 because it gains less
+// than its waves say where there are many.  us, pairs and single: gate/up 300 x 6144 x 1536 20.5 and 15.0 (1 wave for 2), 100 x 10240 x 2560 32.6 and
+// 24.6, 300 x 12288 x 3072 55.6 and 51.6 (2 for 3), 1030 x 6144 x 1536 43.4 and 40.4 (3 for 4), 1030 x 12288 x 3072 127 and 137 (6 for 7: pairs);
+// plain 300 x 12288 x 4096 45.9 and 34.8, 1030 x 7680 x 2560 42.7 and 36.9, 300 x 50257 x 2560 102 and 92; residual 3661 x 2560 x 10240 196 and 152;
+// with as many waves 7996 x 4096 x 1024 gate/up 108 and 129.  (16.7, 26.6, 50.9, 41.0, 130; 34.3, 37.4, 94; 147; 120 when all tiles were single CTAs'.)
+// STU_B200_TILE_N=128 and 256 force either, STU_B200_TILE_CTAS=1 and 2 the last form or the others.
+enum { TILE_NARROW, TILE_WIDE, TILE_SINGLE };
+static int tile_form(long long rows, long long cols, bool dual, bool single_built) {
+  static const char* env_n = getenv("STU_B200_TILE_N");
+  static const char* env_c = getenv("STU_B200_TILE_CTAS");
+  const long long pairs = device_pairs(), sms = device_sm_count(), rows2 = (rows + 2 * BM - 1) / (2 * BM);
+  const auto waves = [](long long tiles, long long at_a_time) { return (tiles + at_a_time - 1) / at_a_time; };
+  const long long wide = 174 * waves(rows2 * ((cols + 255) / 256), pairs);
+  const long long narrow = 100 * waves(rows2 * ((cols + 127) / 128), pairs);
+  const long long single_waves = waves((rows + BM - 1) / BM * ((cols + 255) / 256), sms), single = 215 * single_waves;
+  int form = dual || wide < narrow ? TILE_WIDE : TILE_NARROW;
+  if (env_n && !dual) form = atoi(env_n) == 128 ? TILE_NARROW : TILE_WIDE;
+  if (!single_built || (env_c && atoi(env_c) == 2)) return form;
+  if (env_c && atoi(env_c) == 1) return TILE_SINGLE;
+  if (rows <= BM && single_waves > 1) return form;   // weights from HBM bound either (128 x 50257 x 1024 27.4 and 29.9 us)
+  return single < (form == TILE_WIDE ? wide : narrow) ? TILE_SINGLE : form;
 }
 
 int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N,
@@ -1206,19 +1256,27 @@ int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb,
   if (epi == EPI_HIST) {
     // swap operands: rows = channels (the weight), columns = tokens, so that each epilogue thread owns
     // one channel row of the history and writes whole 16-byte runs per parity
-    const bool wide = wide_tiles(N, M);
+    const bool wide = tile_form(N, M, false, false) == TILE_WIDE;
     if ((rc = make_map(&ma, B, N, K, ldb)) != STU_OK) return rc;
     if ((rc = make_map(&mb, A, M, K, lda, wide ? 128 : 64)) != STU_OK) return rc;
     ep.ldy = N;  // channel count
     if (wide) return launch_tc<EPI_HIST_T, 6, 256>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
     return launch_tc<EPI_HIST_T, 4, 128>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
   }
-  const bool wide = epi != EPI_GELU_MUL && wide_tiles(M, N);
+  const bool dual = epi == EPI_GELU_MUL;
+  const int form = tile_form(M, dual ? 2ll * N : N, dual, epi != EPI_BLOCKCOL);
   if ((rc = make_map(&ma, A, M, K, lda)) != STU_OK) return rc;
-  if ((rc = make_map(&mb, B, N, K, ldb, wide || epi == EPI_GELU_MUL ? 128 : 64)) != STU_OK) return rc;
+  if ((rc = make_map(&mb, B, N, K, ldb, form == TILE_NARROW ? 64 : form == TILE_SINGLE && !dual ? 256 : 128)) != STU_OK) return rc;
   mb2 = mb;
-  if (epi == EPI_GELU_MUL && (rc = make_map(&mb2, B2, N, K, ldb)) != STU_OK) return rc;
-  if (wide) {
+  if (dual && (rc = make_map(&mb2, B2, N, K, ldb)) != STU_OK) return rc;
+  if (form == TILE_SINGLE) {
+    switch (epi) {
+      case EPI_STORE: return launch_tc<EPI_STORE, 4, 256, 1>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+      case EPI_RESID: return launch_tc<EPI_RESID, 4, 256, 1>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
+      case EPI_GELU_MUL: return launch_tc<EPI_GELU_MUL, 4, 128, 1>(ma, mb, mb2, M, N, K, 0, 0, ep, device_status_word(), st);
+    }
+  }
+  if (form == TILE_WIDE && !dual) {
     switch (epi) {
       case EPI_STORE: return launch_tc<EPI_STORE, 6, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);
       case EPI_RESID: return launch_tc<EPI_RESID, 6, 256>(ma, mb, mb2, M, N, K, 0, causal, ep, device_status_word(), st);

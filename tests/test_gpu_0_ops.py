@@ -96,6 +96,27 @@ def test_linear_pair_tiles(M, N, K, epi):
     close(y[:M], _lin_ref(x, W, W2, resid, epi, torch.bfloat16), (1, 2, 4)[epi] * 2 ** -7)
 
 
+@pytest.mark.parametrize("M,N,K,epi,pad", [(300, 6144, 72, 2, 0), (257, 10240, 64, 2, 8), (100, 10248, 200, 2, 0), (1030, 2048, 512, 2, 0), (300, 12288, 72, 0, 0),
+                                           (384, 12296, 136, 1, 8), (129, 18950, 64, 0, 3), (270, 12301, 776, 0, 0), (1030, 7680, 64, 1, 0), (128, 9480, 8, 2, 0)])
+def test_linear_tiles_of_single_ctas(M, N, K, epi, pad):
+    """Products whose tiles of 256 rows would fill their last wave badly are computed by single CTAs: the same bits as by pairs (rows that the
+    pairs' tiles hold, in pieces of 256), whole and ragged tiles, gate/up, residuals, rows on and off the 16-byte grid."""
+    from flash_stu_2_b200 import ops
+    g = torch.Generator(device=dev()).manual_seed(M + N + K)
+    rand = lambda *s: torch.randn(*s, device=dev(), generator=g)
+    x, W, W2 = rand(M, K).bfloat16(), (rand(N, K) / math.sqrt(K)).bfloat16(), (rand(N, K) / math.sqrt(K)).bfloat16()
+    resid = rand(M, N).bfloat16()
+    kw = lambda r: dict(W2=W2 if epi == 2 else None, resid=resid[r] if epi == 1 else None, epilogue=epi, backend=ops.BACKEND_TCGEN05)
+    y = torch.full((M + 1, N + pad), 7.0, dtype=torch.bfloat16, device=dev())
+    ops.linear(x, W, out=y[:M, :N], **kw(slice(0, M)))
+    few = ops.linear(x, W[:2048], W2=W2[:2048] if epi == 2 else None, resid=resid[:, :2048].contiguous() if epi == 1 else None, epilogue=epi,
+                     backend=ops.BACKEND_TCGEN05)   # one wave of pairs
+    ops.check_status()
+    assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())
+    close(y[:M, :N], _lin_ref(x, W, W2, resid, epi, torch.bfloat16), (1, 2, 4)[epi] * 2 ** -7)   # as of the pairs' tiles
+    assert torch.equal(y[:M, :2048], few) or M > 1000   # (1030 rows: several waves either way)
+
+
 @pytest.mark.parametrize("backend", [1, 2, 3])
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("epi", [0, 1, 2])
