@@ -22,6 +22,8 @@
 #include <cuda.h>
 #include <stdlib.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "epilogue.cuh"
 
@@ -1232,7 +1234,7 @@ bool gemm_tc_supported(const void* A, long long lda, const void* B, long long ld
 // with as many waves 7996 x 4096 x 1024 gate/up 108 and 129.  (16.7, 26.6, 50.9, 41.0, 130; 34.3, 37.4, 94; 147; 120 when all tiles were single CTAs'.)
 // STU_B200_TILE_N=128 and 256 force either, STU_B200_TILE_CTAS=1 and 2 the last form or the others.
 enum { TILE_NARROW, TILE_WIDE, TILE_SINGLE };
-static int tile_form(long long rows, long long cols, bool dual, bool single_built) {
+static int tile_form(long long rows, long long cols, bool dual, bool single_built, long long* cost = nullptr) {
   static const char* env_n = getenv("STU_B200_TILE_N");
   static const char* env_c = getenv("STU_B200_TILE_CTAS");
   const long long pairs = device_pairs(), sms = device_sm_count(), rows2 = (rows + 2 * BM - 1) / (2 * BM);
@@ -1241,11 +1243,19 @@ static int tile_form(long long rows, long long cols, bool dual, bool single_buil
   const long long narrow = 100 * waves(rows2 * ((cols + 127) / 128), pairs);
   const long long single_waves = waves((rows + BM - 1) / BM * ((cols + 255) / 256), sms), single = 215 * single_waves;
   int form = dual || wide < narrow ? TILE_WIDE : TILE_NARROW;
+  if (cost) *cost = std::min(wide, std::min(narrow, single));
   if (env_n && !dual) form = atoi(env_n) == 128 ? TILE_NARROW : TILE_WIDE;
   if (!single_built || (env_c && atoi(env_c) == 2)) return form;
   if (env_c && atoi(env_c) == 1) return TILE_SINGLE;
   if (rows <= BM && single_waves > 1) return form;   // weights from HBM bound either (128 x 50257 x 1024 27.4 and 29.9 us)
   return single < (form == TILE_WIDE ? wide : narrow) ? TILE_SINGLE : form;
+}
+
+// What the tiles of a plain product of this many rows and columns take, in hundredths of a wave of the narrow ones.
+extern "C" long long stu_linear_tile_cost(int M, int N) {
+  long long cost = 0;
+  if (M > 0 && N > 0) tile_form(M, N, false, true, &cost);
+  return cost;
 }
 
 int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N,

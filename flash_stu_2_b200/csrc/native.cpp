@@ -291,6 +291,7 @@ PyMethodDef methods[] = {
     ENTRY(stu_lds_final_state),
     ENTRY(stu_linear),
     ENTRY(stu_linear_can_fuse_norm),
+    ENTRY(stu_linear_tile_cost),
     ENTRY(stu_linear_push),
     ENTRY(stu_peer_combine),
     ENTRY(stu_peer_exchange),

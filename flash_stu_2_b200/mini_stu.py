@@ -14,7 +14,7 @@ import torch.nn as nn
 
 from . import ops
 from .filters import get_spectral_filters, nearest_power_of_two
-from .modules import STU, _sm_count, new_pos, host_pos
+from .modules import STU, new_pos, host_pos
 
 LDS_PARAMS = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data", "lds_params.pt")
 
@@ -196,15 +196,11 @@ class MiniSTU(nn.Module):
         return Vs.to(device), W.reshape(Ck * F_, -1).contiguous().to(device), R
 
     def _lds_group(self, B: int, T: int, width: int, x) -> int:
-        """Sequences per contraction: as many as leave the fewest waves of 128 x 256 output tiles in all, within 2 GiB of
-        features (16 sequences of 6000 positions to 1024 outputs: groups of 3, 22 waves instead of 32)."""
-        sms = _sm_count(x.device)
-
-        def waves(n):
-            return -(-(-(-n * T // 128) * -(-self.output_dim // 256)) // sms)
-
+        """Sequences per contraction: as many as leave the least time in the GEMM's waves of tiles in all, within 2 GiB of
+        features (16 sequences of 6000 positions to 1024 outputs: groups of 3; one by one they leave the last wave half empty)."""
         most = max(1, min(B, (2 << 30) // max(1, T * width * x.element_size())))
-        return min(range(1, most + 1), key=lambda g: (B // g * waves(g) + (waves(B % g) if B % g else 0), g))
+        cost = lambda n: ops.linear_tile_cost(n * T, self.output_dim) if n else 0
+        return min(range(1, most + 1), key=lambda g: (B // g * cost(g) + cost(B % g), g))
 
     @staticmethod
     def _lds_features(G: int, T: int, padded: int, width: int, x):

@@ -199,6 +199,11 @@ def can_fuse_norm(M: int, N: int, K: int, epilogue: int, dtype: torch.dtype) -> 
     return bool(_lib.native().stu_linear_can_fuse_norm(M, N, K, epilogue, 1))
 
 
+def linear_tile_cost(rows: int, cols: int) -> int:
+    """Time that the tiles of the tcgen05 GEMM take for this many plain outputs, in hundredths of a wave of the smallest."""
+    return int(_lib.native().stu_linear_tile_cost(rows, cols))
+
+
 def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = None,
            resid: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, epilogue: int = EPI_STORE,
            norm_w: Optional[torch.Tensor] = None, eps: float = RMS_EPS, backend: int = BACKEND_AUTO,

@@ -174,6 +174,21 @@ def test_which_linears_fuse_their_norm(M, N, K, epi, fused):
     assert ops.can_fuse_norm(M, N, K, epi, torch.bfloat16) is fused
 
 
+@pytest.mark.parametrize("B,T,out,group", [(16, 6000, 1024, 3), (8, 4700, 1024, 2), (4, 9000, 1024, 1), (16, 700, 1024, 13), (3, 100, 64, 3)])
+def test_lds_contractions_are_grouped_by_the_gemms_own_tiles(monkeypatch, B, T, out, group):
+    """As many sequences as leave the least time in all by the GEMM's plan (8 x 4700 to 1024 outputs: two sequences are two full waves of
+    pairs' tiles, one alone is one of tiles half as high)."""
+    from types import SimpleNamespace
+
+    from flash_stu_2_b200 import ops
+    x = torch.empty(0, dtype=torch.bfloat16)
+    asked = []
+    cost = ops.linear_tile_cost
+    monkeypatch.setattr(ops, "linear_tile_cost", lambda *a: asked.append(a) or cost(*a))
+    assert F.MiniSTU._lds_group(SimpleNamespace(output_dim=out), B, T, 48 * 1024, x) == group
+    assert all(cols == out and rows % T == 0 for rows, cols in asked)
+
+
 def test_captures_of_two_threads_hold_the_collector_until_the_last_is_done():
     import gc
     from flash_stu_2_b200.model import _CollectionHeld
