@@ -50,32 +50,42 @@ class StreamAhead:
         return True
 
     @staticmethod
-    def sms(layers: int, n_stu: int, B: int, d: int, t: int, weight_bytes: int, ring_bytes: int, sm_count: int) -> int:
+    def sms(layers: int, n_stu: int, B: int, d: int, t: int, weight_bytes: int, ring_bytes: int, sm_count: int, norm_apart: bool = True) -> int:
         """SMs for the streams of steps up to position t; 0 where the layers' own kernels are as good.
-        An SM streams about 80 GB/s (10 of them, 12 layers of 32 x 1536 at 2048, 4000 and 7900: 2183, 3379 and 6277 us), in slices of 256
-        positions with an eighth of taps beside them.  The rest of a step takes about 18 us a layer, its weights 2.8 TB/s and its keys
-        and values 5.5 (24 layers of 1536 and 32 sequences 1515 us, measured 1530; 24 of 512: 552, 632; 12 of 1024: 520, 580).  The streams
-        get the SMs that finish them in 0.6 of that: fewer and the step waits for them (2048: 14 SMs 1671 us, 18 to 26 1534 to 1650, 32 and
-        more 1539 to 1630; without 1708 to 1720), more and the chain misses them (64 sequences at 3000: 26 SMs 2336, 50 2556, without
-        2774), a third of the GPU at most (32 at 7900: 40 1954, 50 2036, 32 2334, without 2278).
-        Beside the chain a layer saves its stream at 4.5 TB/s and 2 us, the second branch costs about 8 (2 layers of 512, 16 sequences at 300:
-        146 us without, 152 with)."""
+        Beside a chain an SM streams 45 to 60 GB/s (16, 20, 24, 28 and 32 of them, 12 layers of 32 x 1536 at 7000: 4788, 3818, 3265, 2809 and 2500 us
+        a step), in slices of 256 positions with an eighth of taps beside them.  The rest of a step takes about 18 us a layer, its weights
+        2.8 TB/s (from 1536 channels on more: 4.5 at 2400) and its keys and values 5.5.  The streams get the SMs that finish them well within that
+        time: too few and the step waits for them (6 layers of 3072, 16 sequences at 3000, 8, 11, 14, 20 and 29 SMs: 1131, 737, 631, 679, 665 us, without
+        712), too many and the chain misses them.  Up to 64 sequences its linears are clusters of up to 16 CTAs, which find no room between
+        more than a fifth of the SMs (us, medians of 5 captures, without and with 16, 20, 24, 28, 32, 36, 40: 24 layers of 1536, 32 sequences at 2000 1794:
+        1600, 1636, 1738, 1759, 1796, 1836, 2067; at 3000 1951: 2203, 1824, 1855, 1919, 1914, 2047, 2353; 64 at 3000 3096: 4498, 3519, 3040, 2819, 3039, 4073, 3860);
+        from 65 on they are pairs, which leave a third (8 layers of 1536, 96 at 3000 1365: 32 1147, 40 1035, 49 1078).  Streams that these cannot
+        finish ahead of the step's end are left to the layers (32 at 7000: 2452).
+        Beside the chain a layer saves its stream at 4.5 TB/s and, where the norm behind it is a launch of its own, 2 us; the second branch costs
+        about 8 (12 layers of 256, 16 sequences at 200: 215 us without, 219 with; at 1000 228 and 224)."""
         stream = n_stu * B * d * ((t // 2 + 255) // 256 * 256) * 2 * 1.125
-        if stream / 4.5e12 + n_stu * 2e-6 <= 8e-6:
+        saved = stream / 4.5e12 + n_stu * (2e-6 if norm_apart else 0.5e-6)
+        if saved <= 8e-6:
             return 0
-        rest = 18e-6 * layers + weight_bytes / 2.8e12 + ring_bytes / 5.5e12
-        return max(8, min(sm_count // 3, int(stream / (80e9 * 0.6 * rest)) + 1))
+        rest = 18e-6 * layers + weight_bytes / max(2.8e12, min(4.5e12, 1.9e9 * d)) + ring_bytes / 5.5e12
+        n = max(8, min(sm_count // (5 if B <= 64 else 3), int(stream / (48e9 * rest)) + 1))
+        return n if stream / (60e9 * n) < 0.97 * (rest + saved) else 0
 
     @classmethod
     def plan(cls, layers, past, B: int, last: int, weight_bytes: int):
         """The buffers for steps from here to position `last`, or None."""
         if not cls.supported(layers, past, B):
             return None
-        self = cls(layers, past, B)
         ring = sum(2 * e[0].numel() * e[0].element_size() * min(last, e[0].shape[1]) // e[0].shape[1] for e in past if e is not None and len(e) == 3)
-        device = self.part.device
-        self.n = cls.sms(len(layers), len(self.entries), B, self.part.shape[3], last, weight_bytes, ring, _sm_count(device))
-        return self if self.n else None
+        stus = [(layer, e) for layer, e in zip(layers, past) if hasattr(layer, "stu")]
+        hist, d = stus[0][1][0], stus[0][1][0].shape[1]
+        apart = not all(ops.can_fuse_norm(B, layer.mlp.intermediate_size, d, ops.EPI_GELU_MUL, hist.dtype) for layer, _ in stus)
+        n = cls.sms(len(layers), len(stus), B, d, last, weight_bytes, ring, _sm_count(hist.device), apart)
+        if not n:
+            return None
+        self = cls(layers, past, B)
+        self.n = n
+        return self
 
     def launch(self, sms: int):
         ops.stream_ahead([e[0] for _, e in self.entries], [stu.prepared()[2] for stu, _ in self.entries], self.part, self.ctl, sms)

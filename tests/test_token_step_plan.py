@@ -263,9 +263,24 @@ def test_overridden_parts_of_an_fp32_step_are_called(monkeypatch, where, name):
 
 
 def test_sms_for_the_streams_beside_a_step():
-    """What decides whether and on how many SMs a captured step's history streams run beside it: none for a few short streams, never
-    more than a third of the GPU, more for longer histories."""
-    big = lambda t: StreamAhead.sms(24, 12, 32, 1536, t, 1_800_000_000, 2_400_000_000, 148)
+    """What decides whether and on how many SMs a captured step's history streams run beside it: none for a few short streams or for more than
+    a fifth of the GPU (from 65 sequences on, a third) can finish, more for longer histories up to there."""
+    big = lambda t, B=32: StreamAhead.sms(24, 12, B, 1536, t, 1_800_000_000, 75_000_000 * B, 148)
     assert StreamAhead.sms(4, 2, 16, 512, 300, 60_000_000, 10_000_000, 148) == 0
-    assert 18 <= big(2176) <= 26 and big(500) == 8 and big(8000) == 49
-    assert all(0 < big(t) <= big(t + 512) for t in range(256, 7600, 256))
+    assert 16 <= big(2176) <= 26 and big(500) == 8 and big(4000) == 29 and big(8000) == 0 and big(8000, 16) == 29
+    assert all(0 < big(t) <= big(t + 512) for t in range(256, 4000, 256))
+    assert 29 < big(4000, 65) <= 49 and big(4000, 64) in (0, 29)
+    # narrow layers of 16 sequences, whose norm is fused either way: a launch less is saved
+    small = lambda t, **kw: StreamAhead.sms(12, 6, 16, 256, t, 40_000_000, 50_000_000, 148, **kw)
+    assert small(200, norm_apart=False) == 0 and small(1000, norm_apart=False) == 8 and small(200) == 8
+
+
+def test_nothing_is_allocated_for_steps_that_are_not_streamed(monkeypatch):
+    m = _model().bfloat16()
+    monkeypatch.setattr(STU, "prepared", lambda self: (None, None, True))
+    monkeypatch.setattr(StreamAhead, "__init__", lambda *a: pytest.fail("built"))
+    monkeypatch.setattr("flash_stu_2_b200.stream_ahead._sm_count", lambda dev: 148)
+    pos = torch.zeros(16, 2, dtype=torch.int32)
+    pos._host_t, pos._uniform = 3, True
+    past = [(torch.zeros(16, 64, 2, 8, dtype=torch.bfloat16), pos) for _ in m.layers]
+    assert StreamAhead.plan(m.layers, past, 16, 10, 1_000_000) is None
