@@ -389,6 +389,32 @@ def test_streams_beside_the_captured_step(monkeypatch, B, T0, new, sms):
         assert torch.equal(ids, want_ids) and torch.equal(logits, want)
 
 
+def test_streams_beside_the_captured_step_of_sixteen(monkeypatch):
+    """The smallest batch whose history sums run beside the chain.  Its ordinary step fuses the MLP's norm (which rounds the normalised row
+    as the finish kernel does, but sums its squares and the product in another order): the same tokens up to a near-tie, logits to rounding
+    until then."""
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.stream_ahead import StreamAhead
+    m = _random_model(256, 4, torch.bfloat16)
+    assert ops.can_fuse_norm(16, m.layers[0].mlp.intermediate_size, 256, ops.EPI_GELU_MUL, torch.bfloat16)
+    prompt = torch.randint(0, 1003, (16, 30), device=dev())
+    kw = dict(max_length=64, do_sample=False, return_logits=True)
+    monkeypatch.setattr(StreamAhead, "enabled", False)
+    want_ids, want = m.generate(prompt, **kw)
+    monkeypatch.setattr(StreamAhead, "enabled", True)
+    monkeypatch.setattr(StreamAhead, "sms", staticmethod(lambda *a: 16))
+    launches, ahead = [], ops.stream_ahead
+    monkeypatch.setattr(ops, "stream_ahead", lambda *a: (launches.append(a[-1]), ahead(*a)))
+    ids, logits = m.generate(prompt, **kw)
+    ops.check_status()
+    assert len(launches) == 2
+    for b in range(16):
+        differ = (ids[b] != want_ids[b]).nonzero().flatten()
+        until = int(differ[0]) - 30 + 1 if len(differ) else 34   # (the logits that the first differing token was drawn from are those of one input)
+        assert until > 2
+        close(logits[b, :until], want[b, :until], 2e-2)
+
+
 @pytest.mark.parametrize("half", [0, 1])
 def test_captured_step_without_its_history_sums_is_reported(monkeypatch, half):
     """Sums that a launch beside the step could not finish stay unannounced, and every later step of the call writes nothing: tokens
