@@ -453,6 +453,11 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
     // of the blocks) lanes store single values, side by side.
     const bool unaligned = EPI == EPI_STORE ? ((ep.ldy & 7) || (reinterpret_cast<uintptr_t>(ep.y) & 15))
                                             : EPI == EPI_HIST_T && ((ep.Tseq & 15) || (ep.t0 & 15) || (ep.Lh & 7));
+    // Plain rows off that grid go in shifted pieces (below) unless a main loop that is long enough hides the single stores, which then cost less:
+    // from K = 832 on and with more than six tiles per pair.  us, pieces and single values: 1668 x 50257 (18 tiles per pair), K = 768 / 832 / 960 /
+    // 1024 / 2048 116 / 134 / 139 / 150 / 251 and 123 / 137 / 133 / 140 / 248; 400 x 50257 (5), K = 1024 54.4 and 54.4; 1668 x 5001 (2), K = 1024 / 2048 18.2 / 27.5 and
+    // 19.2 / 28.4; 256 x 32003 (2), K = 1024 / 3072 24.7 / 55.8 and 25.7 / 57.1.
+    const bool in_pieces = EPI == EPI_STORE && unaligned && (K <= 832 || num_tiles <= 6 * pairs);
     // Plain outputs leave by tensor copies where they can: one lane sends the block off, edges clipped by the copy, which runs
     // beside the next block's accumulator reads.
     // Eight warps, two per quarter of the rows and either at every other 64 columns: four took 7400 cycles for a gate/up tile
@@ -519,7 +524,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
 #pragma unroll 1
       for (int nb = n0 + 64 * half; nb < min(n0 + BN, N); nb += 128) {
         const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
-        const bool shifted = EPI == EPI_STORE && unaligned && nb + 64 <= N && K <= 768;
+        const bool shifted = in_pieces && nb + 64 <= N;
 #pragma unroll 1
         for (int h = 0; h < 2; h++) {   // 32 columns of this thread's row
           uint32_t r[32], r2[32];
@@ -567,9 +572,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
         if (shifted) {
           // Plain rows off the 16-byte grid (an odd vocabulary): the 16-byte pieces of the row's memory lie s values into those of the
           // block.  A lane takes its piece and its neighbour's and shifts out the eight values that one store takes; the s values
-          // ahead of the first such piece and the 8 - s behind the last are stored singly.  Logits of 834 x 50257 x 512 67 -> 58 us, 1668
-          // x 50257 x 768 136 -> 132; from K = 1024 on the main loop hides the single stores, which then cost less: 7996 x 50257 x 1024
-          // 724 us with them, 745 without.
+          // ahead of the first such piece and the 8 - s behind the last are stored singly (834 x 50257 x 512 60 -> 52 us).
           const int piece = lane & 7, r0 = lane >> 3;
           const size_t base = (reinterpret_cast<uintptr_t>(ep.y) >> 1) + nb;
 #pragma unroll

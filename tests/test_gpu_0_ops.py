@@ -232,16 +232,17 @@ def test_linear_cuda_core_tiles_skip_what_a_triangular_weight_leaves_out(dt, sha
     ops.check_status()
 
 
-@pytest.mark.parametrize("K", [768, 776])
-@pytest.mark.parametrize("N,ld,at", [(257, 259, 3), (640, 645, 7), (71, 77, 0), (320, 322, 1)])
-def test_linear_odd_rows_by_shifted_pieces_and_singly(N, ld, at, K):
-    """Rows off the 16-byte grid on either side of the K from which they are stored value by value: every phase of a row against the
-    16-byte pieces of memory, blocks of 64 columns and the columns behind the last; nothing is written between the rows."""
+@pytest.mark.parametrize("M,N,ld,at,K", [(300, 257, 259, 3, 768), (300, 640, 645, 7, 840), (300, 71, 77, 0, 776), (300, 320, 322, 1, 2048), (6000, 5121, 5121, 1, 832),
+                                         (6000, 5121, 5121, 5, 840), (300, 12289, 12295, 2, 840)])
+def test_linear_odd_rows_by_shifted_pieces_and_singly(M, N, ld, at, K):
+    """Rows off the 16-byte grid on either side of the K and the number of tiles from which they are stored value by value (the last but
+    one is; single CTAs' tiles): every phase of a row against the 16-byte pieces of memory, blocks of 64 columns and the columns behind the
+    last; nothing is written between the rows."""
     from flash_stu_2_b200 import ops
     g = torch.Generator(device=dev()).manual_seed(N + K)
-    x, W = torch.randn(300, K, device=dev(), generator=g).bfloat16(), (torch.randn(N, K, device=dev(), generator=g) / math.sqrt(K)).bfloat16()
-    buf = torch.full((300 * ld + at,), 7.0, dtype=torch.bfloat16, device=dev())
-    y = buf[at:].view(300, ld)
+    x, W = torch.randn(M, K, device=dev(), generator=g).bfloat16(), (torch.randn(N, K, device=dev(), generator=g) / math.sqrt(K)).bfloat16()
+    buf = torch.full((M * ld + at,), 7.0, dtype=torch.bfloat16, device=dev())
+    y = buf[at:].view(M, ld)
     ops.linear(x, W, out=y[:, :N], backend=ops.BACKEND_TCGEN05)
     ops.check_status()
     close(y[:, :N], _lin_ref(x, W, None, None, 0, torch.bfloat16), 2 ** -7)   # the next value of an output at most
