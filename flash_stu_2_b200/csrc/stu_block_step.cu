@@ -28,17 +28,15 @@
 // Every wait (mbarrier or grid barrier) is bounded: on expiry the CTA raises status 7, stops, lets its outstanding
 // copies land (bounded) and returns; the other CTAs' waits then run out the same way.
 #include "common.cuh"
+#include "history_dot.cuh"
 #include "tma.cuh"
 
 int device_sm_count();  // gemm_tc.cu
 
 namespace {
 
-constexpr int SEG = 256;
 constexpr int STAGES = 3;
-constexpr int HIST_BYTES = 64 * SEG * 2;
-constexpr int TAP_BYTES = 8 * SEG * 2;
-constexpr int STAGE_BYTES = HIST_BYTES + TAP_BYTES;
+constexpr int STAGE_BYTES = HIST_STAGE_BYTES;
 constexpr int MLP_SLOT = 32 * 1024;      // one gate|up unit: 8 gate rows + 8 up rows of d <= 1024 values
 constexpr int MLP_SLOTS = 3;
 constexpr int MLP_BYTES = MLP_SLOTS * MLP_SLOT;   // shared-memory region the MLP weights pass through
@@ -47,13 +45,6 @@ constexpr int NTHREADS = 18 * 32;        // 8 streaming warps, 2 producer warps,
 
 __device__ __forceinline__ void comp_bar() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
 
-__device__ __forceinline__ uint4 lds128(const void* p) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(tma::smem_u32(p)));
-  return v;
-}
 // L2 loads of data another CTA of this launch wrote (L1 is not coherent across SMs)
 __device__ __forceinline__ uint4 ldcg128(const void* p) {
   uint4 v;
@@ -76,25 +67,6 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_rows8(float (&c)[4], const uint4& a, const uint4& b) {
-  mma16816(c, a.x, 0u, a.y, 0u, b.x, b.y);
-  mma16816(c, a.z, 0u, a.w, 0u, b.z, b.w);
-}
-__device__ __forceinline__ uint4 keep_first(const uint4& v, int keep) {
-  uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-    if (2 * j + 1 >= keep) w[j] = (2 * j < keep) ? (w[j] & 0x0000ffffu) : 0u;
-  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // Grid barrier: a monotonic arrival counter in global memory.  Every CTA reads the launch epoch before it arrives
@@ -304,33 +276,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           const bool ok = __all_sync(0xffffffffu,
                                      tma::mbar_wait_bounded(&full_bar[st], ((uint32_t)(n / STAGES)) & 1u, abort_flag));
           if (ok) {
-            const bf16* H = reinterpret_cast<const bf16*>(smem + st * STAGE_BYTES) + (size_t)(g * 8 + ch) * SEG;
-            const bf16* T = reinterpret_cast<const bf16*>(smem + st * STAGE_BYTES + HIST_BYTES) + (size_t)ch * SEG;
-            const bool tail = (sl == nsl - 1);
-#pragma unroll
-            for (int win = 0; win < SEG / 64; win++) {
-#pragma unroll
-              for (int pass = 0; pass < 2; pass++) {
-                const int koff = win * 64 + ((q + 4 * ((g & 1) ^ pass)) << 3);
-                uint4 a = lds128(H + koff);
-                const uint4 b = lds128(T + koff);
-                if (tail) {
-                  const int keep = ss - (sl * SEG + koff);
-                  if (keep <= 0) a = make_uint4(0, 0, 0, 0);
-                  else if (keep < 8) a = keep_first(a, keep);
-                }
-                mma_rows8(acc[win], a, b);
-              }
-            }
+            history_unit(acc, smem + st * STAGE_BYTES, ch, lane, sl == nsl - 1, ss - sl * SEG);
             __syncwarp();
             if (lane == 0) tma::mbar_arrive(&empty_bar[st]);
           }
         }
-        if (q == (g >> 1)) {   // D[g][g] sits in lane (g, q = g/2), register g&1
-          const float even = (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
-          const float odd = (acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]);
-          __stcg(part_out + (size_t)r * 64 + g * 8 + ch, (g & 1) ? odd : even);
-        }
+        if (history_lane(lane)) __stcg(part_out + (size_t)r * 64 + g * 8 + ch, history_sum(acc, lane));
       }
       if (tid == 0) stamp(P, 7);
     } else if (P.mode == 0) {

@@ -28,6 +28,7 @@
 // Every mbarrier wait is bounded; on expiry the CTA raises status 7, lets its outstanding copies land (bounded) and
 // returns.
 #include "common.cuh"
+#include "history_dot.cuh"
 #include "tma.cuh"
 #include "peer.cuh"
 
@@ -35,42 +36,9 @@ int device_sm_count();  // gemm_tc.cu
 
 namespace {
 
-constexpr int SEG = 256;                       // history positions per unit
 constexpr int STAGES = 4;   // 144 KB of the SM's shared memory: CTAs of a neighbouring kernel still fit beside this one
-constexpr int HIST_BYTES = 64 * SEG * 2;       // 8 sequences x 8 channels x SEG bf16
-constexpr int TAP_BYTES = 8 * SEG * 2;
-constexpr int STAGE_BYTES = HIST_BYTES + TAP_BYTES;
+constexpr int STAGE_BYTES = HIST_STAGE_BYTES;
 
-__device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-
-__device__ __forceinline__ uint4 lds128(const void* p) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(tma::smem_u32(p)));
-  return v;
-}
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// rows 8..15 of the A tile are zero
-__device__ __forceinline__ void mma_rows8(float (&c)[4], const uint4& a, const uint4& b) {
-  mma16816(c, a.x, 0u, a.y, 0u, b.x, b.y);
-  mma16816(c, a.z, 0u, a.w, 0u, b.z, b.w);
-}
-// keep the first `keep` (1..7) of the eight bf16 values of a vector
-__device__ __forceinline__ uint4 keep_first(const uint4& v, int keep) {
-  uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-    if (2 * j + 1 >= keep) w[j] = (2 * j < keep) ? (w[j] & 0x0000ffffu) : 0u;
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
 
 struct Params {
   const bf16* x;
@@ -199,26 +167,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           const bool ok = __all_sync(0xffffffffu,
                                      tma::mbar_wait_bounded(&full_bar[st], ((uint32_t)(n / STAGES)) & 1u, abort_flag));
           if (ok) {
-            const bf16* H = reinterpret_cast<const bf16*>(smem + st * STAGE_BYTES) + (size_t)(g * 8 + ch) * SEG;
-            const bf16* T = reinterpret_cast<const bf16*>(smem + st * STAGE_BYTES + HIST_BYTES) + (size_t)ch * SEG;
-            const bool tail = (sl == nsl - 1);
-#pragma unroll
-            for (int win = 0; win < SEG / 64; win++) {
-#pragma unroll
-              for (int pass = 0; pass < 2; pass++) {
-                // row g takes the chunks of its 64-value window in the order that keeps the eight lanes of a
-                // quarter warp (two rows x four chunks) on distinct banks; taps use the same order, only D[g][g] is read
-                const int koff = win * 64 + ((q + 4 * ((g & 1) ^ pass)) << 3);
-                uint4 a = lds128(H + koff);
-                const uint4 b = lds128(T + koff);
-                if (tail) {
-                  const int keep = s - (sl * SEG + koff);   // values of this vector that are stored history
-                  if (keep <= 0) a = make_uint4(0, 0, 0, 0);
-                  else if (keep < 8) a = keep_first(a, keep);
-                }
-                mma_rows8(acc[win], a, b);
-              }
-            }
+            history_unit(acc, smem + st * STAGE_BYTES, ch, lane, sl == nsl - 1, s - sl * SEG);
             __syncwarp();
             if (lane == 0) tma::mbar_arrive(&empty_bar[st]);
           }
@@ -228,12 +177,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const bool okf = __all_sync(0xffffffffu, tma::mbar_wait_bounded(&part_free[slot], (((uint32_t)(k >> 1)) & 1u) ^ 1u,
                                                                        abort_flag));
         if (okf) {
-          // D[g][g] sits in lane (g, q = g/2), register g&1
-          if (q == (g >> 1)) {
-            const float even = (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
-            const float odd = (acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]);
-            s_part[slot][g * 8 + ch] = (g & 1) ? odd : even;
-          }
+          if (history_lane(lane)) s_part[slot][g * 8 + ch] = history_sum(acc, lane);
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&part_full[slot]);
         }

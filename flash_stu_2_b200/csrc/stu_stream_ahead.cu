@@ -11,15 +11,13 @@
 // Control words ctl[4] of a step's buffers: the position that the next launch computes, arrived CTAs, the positions that the two
 // halves of part hold.
 #include "common.cuh"
+#include "history_dot.cuh"
 #include "tma.cuh"
 
 namespace {
 
-constexpr int SEG = 256;                       // history positions per unit
 constexpr int STAGES = 6;                      // 216 KB: the SM is this CTA's alone, and so are its loads in flight
-constexpr int HIST_BYTES = 64 * SEG * 2;       // 8 sequences x 8 channels x SEG bf16
-constexpr int TAP_BYTES = 8 * SEG * 2;
-constexpr int STAGE_BYTES = HIST_BYTES + TAP_BYTES;
+constexpr int STAGE_BYTES = HIST_STAGE_BYTES;
 constexpr int GROUPS = 2;                      // of 8 consumer warps, each with a row of its own
 constexpr int NTHREADS = (8 * GROUPS + 1) * 32;   // and 1 producer warp
 constexpr int MAX_LAYERS = 64;
@@ -35,29 +33,6 @@ struct AheadParams {
   int layers, B, d, Lh;
 };
 
-__device__ __forceinline__ uint4 lds128(const void* p) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(tma::smem_u32(p)));
-  return v;
-}
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// keep the first `keep` (1..7) of the eight bf16 values of a vector
-__device__ __forceinline__ uint4 keep_first(const uint4& v, int keep) {
-  uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-    if (2 * j + 1 >= keep) w[j] = (2 * j < keep) ? (w[j] & 0x0000ffffu) : 0u;
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
 
 // A row is 8 sequences x 8 channels of a layer; CTA i owns rows i, i + grid, ... of all layers.  As in stu_decode_pipe_kernel a unit of
 // 256 positions arrives by two bulk tensor copies, warp w takes channel w, and the dot products are the diagonal of mma.sync products.
@@ -68,7 +43,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) stu_stream_ahead_kernel(const __g
   uint64_t* empty_bar = full_bar + STAGES;
   __shared__ int s_abort, s_issued;
   volatile int* abort_flag = &s_abort;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2;
   const int G = gridDim.x, B = P.B, d = P.d, Lh = P.Lh;
   const int ncg = d >> 3, rows = ((B + 7) >> 3) * ncg, total = rows * P.layers;
   if (tid == 0) {
@@ -123,36 +98,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) stu_stream_ahead_kernel(const __g
         const int n = n0 + sl * here + group, st = n % STAGES;
         ok = tma::warp_wait_bounded(&full_bar[st], (uint32_t)(n / STAGES) & 1u, abort_flag);
         if (!ok) break;
-        const bf16* H = reinterpret_cast<const bf16*>(smem + st * STAGE_BYTES) + (size_t)(g * 8 + ch) * SEG;
-        const bf16* T = reinterpret_cast<const bf16*>(smem + st * STAGE_BYTES + HIST_BYTES) + (size_t)ch * SEG;
-        const bool tail = (sl == nsl - 1);
-#pragma unroll
-        for (int win = 0; win < SEG / 64; win++) {
-#pragma unroll
-          for (int pass = 0; pass < 2; pass++) {
-            // (order of the chunks of a 64-value window: conflict-free for the eight lanes of a quarter warp)
-            const int koff = win * 64 + ((q + 4 * ((g & 1) ^ pass)) << 3);
-            uint4 a = lds128(H + koff);
-            const uint4 b = lds128(T + koff);
-            if (tail) {
-              const int keep = s - (sl * SEG + koff);   // values of this vector that are stored history
-              if (keep <= 0) a = make_uint4(0, 0, 0, 0);
-              else if (keep < 8) a = keep_first(a, keep);
-            }
-            mma16816(acc[win], a.x, 0u, a.y, 0u, b.x, b.y);   // rows 8..15 of the A tile are zero
-            mma16816(acc[win], a.z, 0u, a.w, 0u, b.z, b.w);
-          }
-        }
+        history_unit(acc, smem + st * STAGE_BYTES, ch, lane, sl == nsl - 1, s - sl * SEG);
         __syncwarp();
         if (lane == 0) tma::mbar_arrive(&empty_bar[st]);
       }
       n0 += nsl * here;
-      // D[g][g] sits in lane (g, q = g/2), register g&1
-      if (ok && inside && q == (g >> 1) && bg * 8 + g < B) {
-        const float even = (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
-        const float odd = (acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]);
-        P.part[((size_t)(layer * 2 + p) * B + bg * 8 + g) * d + cg * 8 + ch] = (g & 1) ? odd : even;
-      }
+      if (ok && inside && history_lane(lane) && bg * 8 + g < B)
+        P.part[((size_t)(layer * 2 + p) * B + bg * 8 + g) * d + cg * 8 + ch] = history_sum(acc, lane);
     }
   }
   __syncthreads();
