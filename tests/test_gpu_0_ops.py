@@ -316,6 +316,27 @@ def test_bounded_wait_expiry_is_reported_and_the_context_survives():
     ops.check_status()
 
 
+def test_bounded_wait_expiry_of_single_ctas():
+    """The same for the GEMM's form with a CTA in the place of a pair (300 x 12288 outputs), every CTA of which gives up."""
+    from flash_stu_2_b200 import _lib, ops
+    lib = _lib.load()
+    g = torch.Generator(device=dev()).manual_seed(22)
+    x, W = torch.randn(300, 136, device=dev(), generator=g).bfloat16(), (torch.randn(12288, 136, device=dev(), generator=g) / 12).bfloat16()
+    want = ops.linear(x, W, backend=2)
+    ops.check_status()
+    close(want, _lin_ref(x, W, None, None, 0, torch.bfloat16), 2 ** -7)
+    assert lib.stu_test_inject_wait_expiry(100) == 0
+    try:
+        ops.linear(x, W, backend=2)
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="status 3"):
+            ops.check_status()
+    finally:
+        assert lib.stu_test_inject_wait_expiry(0) == 0
+    assert torch.equal(ops.linear(x, W, backend=2), want)
+    ops.check_status()
+
+
 def test_linear_fused_norm_decode():
     """RMSNorm fused into the mma.sync token-step linears (every row count up to 64; callers use it up to 16 rows)."""
     from flash_stu_2_b200 import ops
