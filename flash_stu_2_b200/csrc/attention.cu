@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256) kv_ring_write_kernel(const T* __restrict_
 // row of one head is TV vectors of 16 bytes, held by 4 lanes (8 for 512-byte rows), so a warp works on 8 keys at a time and a dot
 // product takes two shuffles.  (16 lanes per key took four for two keys, and every copy a division for its ring slot; 16 sequences
 // of 12 heads of 128 over 1025 keys took as long as 32.)  Every group of lanes keeps its own softmax state (reference maximum,
-// sum, weighted values of its slice); the reference moves, and sum and values are rescaled, only where a score outgrows it
+// sum, weighted values of its slice); in bf16 the reference moves, and sum and values are rescaled, only where a score outgrows it
 // by 8, so that the rescale is rare (exp(8) is far from the end of fp32).  Groups are merged by shuffles, warps through shared
 // memory, CTAs of a cluster through distributed shared memory, in a fixed order.
 // The new token's key and value come from the qkv activations; the cluster's first CTA then stores them into ring slot t % W for its
@@ -234,6 +234,10 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
   constexpr int NV = TV / G;                   // vectors of a row per lane: sub, sub + G, ...
   constexpr int U = 4 / NV;                    // keys of a lane per round
   constexpr int KPW = 32 / G, KSTEP = 8 * KPW; // keys at a time: of a warp, of the CTA
+  // How far a score may outgrow the reference before it moves.  bf16: 8, below the rounding of the output; fp32: not at all, an exponent
+  // of up to 8 carries its own rounding into the weights that count (4 heads of 128, 1025 keys, error against float64 2.3e-7; now 1.4e-7,
+  // as with 16 lanes per key; the time is the same).
+  constexpr float LAG = sizeof(T) == 4 ? 0.f : 8.f;
   __shared__ float s_m[8], s_l[8], s_acc[8][HD];
   __shared__ float c_m, c_l, c_acc[HD];        // of this CTA, for the cluster
   const int h = blockIdx.x / splits, part = blockIdx.x - h * splits, b = blockIdx.y;
@@ -324,16 +328,22 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int kk = base + grp + (it * U + u) * KSTEP;
-      float dot = 0.f;
+      float part[NV];   // of each vector, then in pairs: one chain over the lane's values had 1.2 to 1.55 times the error (fp32, heads of 64 and 128)
 #pragma unroll
       for (int i = 0; i < NV; i++) {
         Vec16<T> k;
         float kf[VPL];
         k.raw = ring[(u * 2 * NV + i) * 256];
         k.unpack(kf);
+        part[i] = 0.f;
 #pragma unroll
-        for (int e = 0; e < VPL; e++) dot = fmaf(qv[i * VPL + e], kf[e], dot);
+        for (int e = 0; e < VPL; e++) part[i] = fmaf(qv[i * VPL + e], kf[e], part[i]);
       }
+#pragma unroll
+      for (int n = NV / 2; n > 0; n >>= 1)
+#pragma unroll
+        for (int i = 0; i < n; i++) part[i] += part[i + n];
+      float dot = part[0];
 #pragma unroll
       for (int o = G / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
       if (softcap > 0.f) {
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(256, 3) swa_decode_kernel(const T* __restrict_
       sc[u] = (kk < k_end) ? dot - slope * (float)(nkeys - 1 - kk) : -INFINITY;   // ALiBi: i - j
       mx = fmaxf(mx, sc[u]);
     }
-    const bool grow = mx > m + 8.f || (m == -INFINITY && mx > -INFINITY);
+    const bool grow = mx > m + LAG || (m == -INFINITY && mx > -INFINITY);
     if (__any_sync(0xffffffffu, grow)) {
       const float corr = grow ? __expf(m - mx) : 1.f;   // 0 while the group has seen no key yet
       if (grow) m = mx;
