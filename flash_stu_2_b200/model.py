@@ -287,6 +287,8 @@ class FlashSTU(PreTrainedModel):
                     u_buf.copy_(u)
                 graph.replay()
                 replayed += 1
+                if step == steps - 2 and buffers[-1] is not None:
+                    buffers[-1].note()
                 for e in past:
                     if e is not None and getattr(e[-1], "_host_t", None) is not None:
                         e[-1]._host_t += 1

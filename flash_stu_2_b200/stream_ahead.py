@@ -110,9 +110,16 @@ class StreamAhead:
     def join(self, stream):
         stream.wait_stream(self.stream)
 
+    def note(self):
+        """Behind the last step but one: the sums that the last one needs are there or will not be."""
+        self.noted = torch.empty(4, dtype=torch.int32, pin_memory=True).copy_(self.ctl, non_blocking=True)
+        self.at = torch.cuda.Event()
+        self.at.record()
+
     def check(self):
         """Raises when a launch of the sums has given up on a wait: the steps from the position behind it on wrote nothing.  Waits for
-        the steps so far."""
-        if int(self.ctl[2:].min()) < 0:   # (a half that holds no position stays so)
+        the steps up to note() (a call behind this one is prepared while the last one runs)."""
+        self.at.synchronize()
+        if min(self.noted[2:].tolist()) < 0:   # (a half that holds no position stays so)
             ops.check_status(self.part.device)
             raise RuntimeError(f"flash_stu_2_b200 device status 8: {ops.STATUS_TEXT[8]}")
