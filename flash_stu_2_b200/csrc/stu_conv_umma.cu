@@ -29,6 +29,13 @@
 // a phase's operands - the 64 KB chunk and the 34 KB table of its block distances - form one of two shared-memory
 // stages, filled a phase ahead of the MMAs.
 //
+// Where the outputs end within 16 blocks a unit is one phase of one to two microseconds of MMAs, shorter than the way of
+// its operands from memory.  Then a stage holds the blocks and distances there are and no more (6 KB a block), as many
+// stages as fit (up to 6) are under way, and output blocks in front of the call's first position are left out.
+// us with the transposition behind it, two whole stages and now: 1 x 1536 channels, 333 positions 27.8 and 21.5; 2 x 768, 834
+// positions at 0, 834 and 1666: 20.6, 24.6, 31.0 and 19.9, 23.8, 27.8; 4 x 1024, 1999 positions 37.7 and 35.9.  What is left there
+// is the instructions: 128 x 16 Toeplitz elements out of shared memory for each, 61 cycles however few columns it has.
+//
 // Roles (one persistent CTA per SM, 320 threads):
 //   warp 0      producer: history chunks (2 x 32 KB tensor copies, 128-byte swizzle)
 //   warp 1      allocates tensor memory, issues the MMAs from one thread, commits to the barriers
@@ -51,24 +58,23 @@ int launch_transpose_add(void* x, long long x_bstride, long long x_tstride, cons
 namespace {
 
 constexpr int SUP = 16;                       // 128-position blocks per unit (256 accumulator columns / 16 rows)
-constexpr int PLANE_BYTES = SUP * 16 * 128;   // 16 blocks x 16 rows x 64 positions
-constexpr int HIST_BYTES = 2 * PLANE_BYTES;
-constexpr int TAB_ENTRIES = 16 * SUP + 15;
-constexpr int TAB_BYTES = (TAB_ENTRIES * 128 + 1023) / 1024 * 1024;
-constexpr int STAGE_BYTES = HIST_BYTES + TAB_BYTES;
-constexpr int STG_OFF = 2 * STAGE_BYTES;      // epilogue staging: 4 warps x 32 rows x 80 bytes
-constexpr int STG_BYTES = 4 * 32 * 80;
-constexpr int CTL_OFF = STG_OFF + STG_BYTES;
-constexpr int SMEM_BYTES = CTL_OFF + 256 + 1024;
+constexpr int MAX_STAGES = 6;
+__host__ __device__ constexpr int plane_bytes(int blocks) { return blocks * 16 * 128; }   // blocks x 16 rows x 64 positions
+__host__ __device__ constexpr int tab_bytes(int blocks) { return ((16 * blocks + 15) * 128 + 1023) / 1024 * 1024; }
+__host__ __device__ constexpr int stage_bytes(int blocks) { return 2 * plane_bytes(blocks) + tab_bytes(blocks); }
+constexpr int STG_BYTES = 4 * 32 * 80;        // epilogue staging: 4 warps x 32 rows x 80 bytes
+constexpr int STAGES_BYTES = 2 * stage_bytes(SUP);   // what the stages share
+constexpr int CTL_BYTES = 256;
+constexpr int SMEM_BYTES = STAGES_BYTES + STG_BYTES + CTL_BYTES + 1024;
 constexpr int ACC_COLS = 16 * SUP;
 constexpr int STATUS_CONV_WAIT = 9;
 
 struct Ctl {
-  uint64_t hist_full[2], ready[2], stage_empty[2], tmem_full[2], tmem_empty[2];
+  uint64_t hist_full[MAX_STAGES], ready[MAX_STAGES], stage_empty[MAX_STAGES], tmem_full[2], tmem_empty[2];
   uint32_t tmem_slot;
   int abort_flag, issued_h, consumed_h;
 };
-static_assert(sizeof(Ctl) <= 256, "control block");
+static_assert(sizeof(Ctl) <= CTL_BYTES, "control block");
 
 struct Geom {
   int B, d, Lh, y_Lh, t0, t_end;
@@ -76,18 +82,40 @@ struct Geom {
   int nb_total;   // 128-position blocks that hold outputs
   int msb_first;  // first superblock with outputs of this call
   int n_sup;      // superblocks processed
+  int stages;     // operand stages of stage_bytes(blocks)
+  int blocks;     // blocks of a history chunk, and at most that many block distances >= 0 of a phase
 };
+
+// the stage of phase pc, and whether it is filled for an odd time
+struct Ring {
+  int s = 0;
+  uint32_t turn = 0;
+  __device__ __forceinline__ void next(int stages) {
+    if (++s == stages) s = 0, turn ^= 1u;
+  }
+};
+__device__ __forceinline__ void cp_async_wait(int pending) {
+  switch (pending) {
+    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+    default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+  }
+}
 
 __device__ __forceinline__ int parity_count(int t_end, int p) { return (t_end - p + 1) >> 1; }
 
 // A unit (channel, row group, superblock msb of 16 output blocks) runs 2 msb + 1 phases.  Phase ph < 2 msb works on
 // history chunk ssb = ph / 2 (16 input blocks) and covers the block distances dl = mb - sb (local to the two
 // superblocks) 0 .. nb_m-1 (even ph) or -15 .. -1 (odd ph); the last phase is the chunk on the diagonal, dl >= 0
-// only.  The first phase of a unit starts with dl = 0, which touches every accumulator column, so its first
+// only.  The first phase of a unit starts with dl = 0, which touches every accumulator column that is read, so its first
 // instruction overwrites instead of accumulating.
 struct Phase {
   int ssb, dl_lo, ndl;
 };
+// first output block of superblock msb that the call asks for
+__device__ __forceinline__ int first_block(const Geom& g, int msb) { return max(0, (g.t0 >> 8) - SUP * msb); }
 __device__ __forceinline__ Phase phase_of(int ph, int msb, int nb_m) {
   Phase p;
   if (ph == 2 * msb) {
@@ -162,15 +190,18 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
                                                            unsigned long long* tl) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  Ctl* ctl = reinterpret_cast<Ctl*>(smem + CTL_OFF);
+  Ctl* ctl = reinterpret_cast<Ctl*>(smem + STAGES_BYTES + STG_BYTES);
+  const int PLANE = plane_bytes(g.blocks), HIST = 2 * PLANE, STAGE = stage_bytes(g.blocks), NS = g.stages;
   volatile int* abort_flag = &ctl->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; s++) {
+    for (int s = 0; s < MAX_STAGES; s++) {
       tma::mbar_init(&ctl->hist_full[s], 1);
       tma::mbar_init(&ctl->ready[s], 128);
       tma::mbar_init(&ctl->stage_empty[s], 1);
+    }
+    for (int s = 0; s < 2; s++) {
       tma::mbar_init(&ctl->tmem_full[s], 1);
       tma::mbar_init(&ctl->tmem_empty[s], 128);
     }
@@ -191,19 +222,20 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
     // -------------------------------------------------------------------- producer: the history chunk of each phase
     const bool leader = elect_one();
     int pc = 0;
+    Ring ring;
     bool ok = true;
     FOR_EACH_UNIT(task, msb, c, rg) {
       if (!ok) break;
-      for (int ph = 0; ph <= 2 * msb; ph++, pc++) {
+      for (int ph = 0; ph <= 2 * msb; ph++, pc++, ring.next(NS)) {
         const int ssb = (ph == 2 * msb) ? msb : (ph >> 1);
-        const int s = pc & 1;
-        ok = tma::warp_wait_bounded(&ctl->stage_empty[s], ((uint32_t)(pc >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
+        const int s = ring.s;
+        ok = tma::warp_wait_bounded(&ctl->stage_empty[s], ring.turn ^ 1u, abort_flag, wait_ns);
         if (!ok) break;
         if (leader) {
-          unsigned char* dst = smem + s * STAGE_BYTES;
-          tma::mbar_expect_tx(&ctl->hist_full[s], HIST_BYTES);
+          unsigned char* dst = smem + s * STAGE;
+          tma::mbar_expect_tx(&ctl->hist_full[s], HIST);
           tma::load_5d(dst, &tmH, &ctl->hist_full[s], 0, 0, 8 * rg, SUP * ssb, c);
-          tma::load_5d(dst + PLANE_BYTES, &tmH, &ctl->hist_full[s], 64, 0, 8 * rg, SUP * ssb, c);
+          tma::load_5d(dst + PLANE, &tmH, &ctl->hist_full[s], 64, 0, 8 * rg, SUP * ssb, c);
         }
         __syncwarp();
       }
@@ -213,27 +245,28 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
     // -------------------------------------------------------------------- MMA issuer
     const bool leader = elect_one();
     int pc = 0, uc = 0;
+    Ring ring;
     bool ok = true;
     FOR_EACH_UNIT(task, msb, c, rg) {
       if (!ok) break;
       (void)c; (void)rg;
-      const int nb_m = min(SUP, g.nb_total - SUP * msb);
+      const int nb_m = min(SUP, g.nb_total - SUP * msb), mb_first = first_block(g, msb);
       const int buf = uc & 1;
       ok = tma::warp_wait_bounded(&ctl->tmem_empty[buf], ((uint32_t)(uc >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (leader) TL_STAMP(uc, 0);
-      for (int ph = 0; ph <= 2 * msb; ph++, pc++) {
+      for (int ph = 0; ph <= 2 * msb; ph++, pc++, ring.next(NS)) {
         const Phase P = phase_of(ph, msb, nb_m);
-        const int s = pc & 1;
-        ok = tma::warp_wait_bounded(&ctl->ready[s], (uint32_t)(pc >> 1) & 1u, abort_flag, wait_ns);
+        const int s = ring.s;
+        ok = tma::warp_wait_bounded(&ctl->ready[s], ring.turn, abort_flag, wait_ns);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ph == 0 && leader) TL_STAMP(uc, 1);
-        const uint32_t hist_s = tma::smem_u32(smem + s * STAGE_BYTES), tab_s = hist_s + HIST_BYTES;
+        const uint32_t hist_s = tma::smem_u32(smem + s * STAGE), tab_s = hist_s + HIST;
         for (int st = 0; st < P.ndl; st++) {
           const int dl = P.dl_lo + st;
-          const int mb_lo = max(0, dl), mb_hi = min(nb_m, SUP + dl);
+          const int mb_lo = max(mb_first, dl), mb_hi = min(nb_m, SUP + dl);
           if (mb_hi <= mb_lo) continue;
           const uint32_t dcol = tmem_base + (uint32_t)(buf * ACC_COLS + 16 * mb_lo);
           const uint32_t idesc = idesc_n(16 * (mb_hi - mb_lo));
@@ -245,7 +278,7 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
             for (int kk = 0; kk < 8; kk++) {
               const uint32_t acc = (ph == 0 && st == 0 && kk == 0) ? 0u : 1u;
               umma(dcol, da0 + (uint64_t)(2 * kk * 128 >> 4),
-                   db0 + (uint64_t)(((kk >> 2) * PLANE_BYTES + (kk & 3) * 32) >> 4), idesc, acc);
+                   db0 + (uint64_t)(((kk >> 2) * PLANE + (kk & 3) * 32) >> 4), idesc, acc);
             }
           }
           __syncwarp();
@@ -270,7 +303,7 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
     const int quarter = warp & 3;
     const int pos = 24 - 8 * (lane >> 3) + (lane & 7);   // rank of this lane's position among the warp's 32
     const int i_min = 96 - 32 * quarter;                 // first position (inside a block) of the warp's 32
-    unsigned char* stg = smem + STG_OFF + (warp - 2) * (32 * 80);
+    unsigned char* stg = smem + STAGES_BYTES + (warp - 2) * (32 * 80);
     const int cnt0 = parity_count(g.t_end, 0), cnt1 = parity_count(g.t_end, 1);
     const int lo0 = parity_count(g.t0, 0), lo1 = parity_count(g.t0, 1);
     int uc = 0;
@@ -285,7 +318,7 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (threadIdx.x == 64) TL_STAMP(uc, 3);
 #pragma unroll 1
-      for (int cch = 0; cch < ((nb_m + 1) >> 1); cch++) {   // 32 columns = two blocks
+      for (int cch = first_block(g, msb) >> 1; cch < ((nb_m + 1) >> 1); cch++) {   // 32 columns = two blocks
         uint32_t r[32];
         tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * ACC_COLS + cch * 32), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -324,20 +357,50 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   } else {
     // -------------------------------------------------------------------- generators
-    const int gt = threadIdx.x - 192;
+    // The tables of the phases up to stages - 2 ahead are on their way while a phase is made ready: the stage that a table
+    // goes to was left by the phase before the last one.
+    const int gt = threadIdx.x - 192, ahead = NS - 2;
     const int cnt0 = parity_count(g.t_end, 0), cnt1 = parity_count(g.t_end, 1);
     const size_t pitch = (size_t)g.Lh + 8;
-    int pc = 0;
+    int pc = 0;   // phase whose table is asked for
+    Ring fill, turn;
     bool ok = true;
+    // ---- what is left of phase `done` when its table has landed; its chunk begins at block SUP * ssb (more than two stages: at 0)
+    auto finish = [&](int done, int ssb, int pending) {
+      const int s = turn.s;
+      unsigned char* stage = smem + s * STAGE;
+      // ---- the history chunk: zero what lies past each row's valid count (stale cache contents must not meet the
+      //      zero part of a Toeplitz block as 0 x NaN), up to 129 positions of a row, in whole pieces of 8 behind the first
+      if (!tma::mbar_wait_bounded(&ctl->hist_full[s], turn.turn, abort_flag, wait_ns)) return false;
+      if (gt == 0) TL_STAMP(done, 6);
+      const int base = SUP * 128 * ssb;
+      const int lim = min(g.nb_total * 128, base + SUP * 128) - base, n = gt >> 3;
+      const int from = max((n & 1 ? cnt1 : cnt0) - base, 0);
+      for (int k8 = (from >> 3) + (gt & 7); k8 * 8 < lim; k8 += 8) {
+        const int rr = (k8 >> 4) * 16 + n;
+        unsigned char* ptr = stage + ((k8 >> 3) & 1) * PLANE + (rr >> 3) * 1024 + (rr & 7) * 128 + (((k8 & 7) ^ (rr & 7)) << 4);
+        if (k8 * 8 >= from) {
+          *reinterpret_cast<uint4*>(ptr) = make_uint4(0, 0, 0, 0);
+        } else {
+          for (int w = from & 7; w < 8; w++) reinterpret_cast<unsigned short*>(ptr)[w] = 0;
+        }
+      }
+      cp_async_wait(pending);
+      fence_proxy_async();
+      if (gt == 0) TL_STAMP(done, 7);
+      tma::mbar_arrive(&ctl->ready[s]);
+      turn.next(NS);
+      return true;
+    };
     FOR_EACH_UNIT(task, msb, c, rg) {
       if (!ok) break;
       (void)rg;
       const int nb_m = min(SUP, g.nb_total - SUP * msb);
       for (int ph = 0; ph <= 2 * msb; ph++, pc++) {
         const Phase P = phase_of(ph, msb, nb_m);
-        const int s = pc & 1;
-        unsigned char* stage = smem + s * STAGE_BYTES;
-        ok = tma::mbar_wait_bounded(&ctl->stage_empty[s], ((uint32_t)(pc >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
+        const int s = fill.s;
+        unsigned char* stage = smem + s * STAGE;
+        ok = tma::mbar_wait_bounded(&ctl->stage_empty[s], fill.turn ^ 1u, abort_flag, wait_ns);
         if (!ok) break;
         if (gt == 0) TL_STAMP(pc, 5);
         // ---- core-matrix table of this phase: entry e <-> V = v_lo + e, row r: CM[V][r][w] = g[120 - 8 V + r - w];
@@ -351,40 +414,19 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
             // V >= 16: every tap index of the row is negative (above the diagonal).  A row that straddles tap 0 runs
             // into the table's own zero padding; one that would start before the table only has taps past the filter.
             if (V < 16 && uo >= 0)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tma::smem_u32(stage + HIST_BYTES + it * 16)),
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tma::smem_u32(stage + HIST + it * 16)),
                            "l"(taps8 + ((size_t)(7 - r) * g.d + c) * pitch + uo) : "memory");
             else
-              *reinterpret_cast<uint4*>(stage + HIST_BYTES + it * 16) = make_uint4(0, 0, 0, 0);
+              *reinterpret_cast<uint4*>(stage + HIST + it * 16) = make_uint4(0, 0, 0, 0);
           }
           asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        // ---- the history chunk: zero what lies past each row's valid count (stale cache contents must not meet the
-        //      zero part of a Toeplitz block as 0 x NaN)
-        ok = tma::mbar_wait_bounded(&ctl->hist_full[s], (uint32_t)(pc >> 1) & 1u, abort_flag, wait_ns);
+        fill.next(NS);
+        if (pc >= ahead) ok = finish(pc - ahead, ahead == 0 ? P.ssb : 0, ahead);
         if (!ok) break;
-        if (gt == 0) TL_STAMP(pc, 6);
-        {
-          const int base = SUP * 128 * P.ssb;
-          const int lim = min(g.nb_total * 128, base + SUP * 128);
-          if (lim > cnt1) {
-            for (int el = gt; el < 16 * 129; el += 128) {
-              const int n = el / 129, off = el % 129, p = n & 1;
-              const int sx = max(p ? cnt1 : cnt0, base) + off;
-              if (sx < lim) {
-                const int sl = sx - base, rr = (sl >> 7) * 16 + n, kq = sl & 127, k = kq & 63;
-                unsigned char* ptr = stage + (kq >> 6) * PLANE_BYTES + (rr >> 3) * 1024 + (rr & 7) * 128 +
-                                     (((k >> 3) ^ (rr & 7)) << 4) + (k & 7) * 2;
-                *reinterpret_cast<unsigned short*>(ptr) = 0;
-              }
-            }
-          }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        fence_proxy_async();
-        if (gt == 0) TL_STAMP(pc, 7);
-        tma::mbar_arrive(&ctl->ready[s]);
       }
     }
+    for (int left = min(ahead, pc); ok && left > 0; left--) ok = finish(pc - left, 0, 0);
   }
   __syncthreads();
   if (*abort_flag) {
@@ -395,7 +437,7 @@ __global__ void __launch_bounds__(320, 1) conv_umma_kernel(const __grid_constant
       const uint64_t t_start = tma::global_ns();
       for (int pc = ctl->consumed_h; pc < ctl->issued_h; pc++)
         for (uint32_t w = 0; w < (1u << 22); ++w) {
-          if (tma::mbar_try_wait(&ctl->hist_full[pc & 1], (uint32_t)(pc >> 1) & 1u)) break;
+          if (tma::mbar_try_wait(&ctl->hist_full[pc % NS], (uint32_t)(pc / NS) & 1u)) break;
           if ((w & 255u) == 255u && tma::global_ns() - t_start > wait_ns) break;
         }
     }
@@ -436,13 +478,16 @@ extern "C" int stu_conv_prefill_approx_tc5(const void* hist, const void* taps8, 
   g.msb_first = mlo_min / (SUP * 128);
   g.n_sup = (g.nb_total + SUP - 1) / SUP - g.msb_first;
   if (g.n_sup <= 0) return STU_ERR_SHAPE;
+  g.blocks = g.nb_total < SUP ? g.nb_total : SUP;
+  g.stages = g.nb_total > SUP ? 2 : STAGES_BYTES / stage_bytes(g.blocks);
+  if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
 
   CUtensorMap tmH;
   {
     // history [B][d][2][Lh] seen as (position inside a 128-block, parity, sequence, block, channel)
     cuuint64_t dims[5] = {128, 2, (cuuint64_t)B, (cuuint64_t)(Lh / 128), (cuuint64_t)d};
     cuuint64_t str[4] = {(cuuint64_t)Lh * 2, (cuuint64_t)d * 2 * Lh * 2, 256, (cuuint64_t)2 * Lh * 2};
-    cuuint32_t box[5] = {64, 2, 8, SUP, 1};
+    cuuint32_t box[5] = {64, 2, 8, (cuuint32_t)g.blocks, 1};
     int rc = tma::encode_bf16(&tmH, hist, 5, dims, str, box, true);
     if (rc != STU_OK) return rc;
   }

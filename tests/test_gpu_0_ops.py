@@ -465,6 +465,32 @@ def test_conv_prefill_tcgen05_matches_fft_oracle(shape):
     close(x, x2, 8e-3, row_tol=1.6e-2)
 
 
+@pytest.mark.parametrize("shape", [(1, 256, 1000, 0), (2, 1279, 900, 1270), (3, 1500, 760, 700), (2, 2049, 480, 1800), (9, 2817, 160, 2815),
+                                   (1, 4095, 320, 0)])
+def test_conv_prefill_tcgen05_stages_of_every_depth(shape):
+    """Six to two operand stages (1 to 16 blocks of 128 positions of a parity), each gone round by more channels than it holds, blocks in
+    front of the call's first position left out, NaN in the cache past the valid positions: against the mma.sync kernel on the same
+    operands (the same products, fp32 sums in another order: two roundings to bf16)."""
+    from flash_stu_2_b200 import ops
+    B, T, d, t0 = shape
+    torch.manual_seed(11)
+    L = T + 3
+    Lh = ((L + 1) // 2 + 127) // 128 * 128
+    hist = _hist_from(torch.randn(B, T, d).bfloat16(), Lh)
+    taps = ops.taps_even((torch.randn(L, d) / math.sqrt(L)).bfloat16().to(dev()), Lh)
+    x0 = torch.randn(B, T - t0, d).bfloat16().to(dev())
+    x1, x2 = x0.clone(), x0.clone()
+    y_Lh = ((T + 1) // 2 + 7) // 8 * 8
+    ops.conv_prefill_approx(hist.to(dev()), taps, torch.zeros(B, d, 2, y_Lh, dtype=torch.bfloat16, device=dev()), x2, t0, T, use_tensor_cores=True)
+    for p in range(2):
+        hist[:, :, p, (T - p + 1) // 2:] = float("nan")
+    hist = hist.to(dev())
+    assert ops.conv_prefill_tc5_supported(hist, x1)
+    ops.conv_prefill_approx_tc5(hist, ops.taps_rev8(taps), torch.full((B, d, 2, y_Lh), float("nan"), dtype=torch.bfloat16, device=dev()), x1, t0, T)
+    ops.check_status()
+    close(x1, x2, 8e-3, row_tol=1.6e-2)
+
+
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_history_scatter_epilogue(dt):
     from flash_stu_2_b200 import ops
