@@ -1,6 +1,5 @@
-// General tiled GEMM on CUDA cores with fp32 accumulation: the path for fp32 models (where the
-// 1e-3 / bit-exact-greedy bar rules out tf32 tensor cores) and for shapes the tcgen05 path does
-// not take (tiny K, unaligned strides).  y = epilogue(x @ W^T).
+// General tiled GEMM on CUDA cores with fp32 accumulation: fp32 products that are too small or too short for
+// gemm_f32_umma.cu, or off the 16-byte grid, and bf16 shapes the tcgen05 path does not take (tiny K, unaligned strides).  y = epilogue(x @ W^T).
 //
 // Bound: FFMA issue (74 TFLOP/s), and before that the number of CTAs: the prefill linears of a 512-wide fp32 model are
 // 256 x 512 x 6144.  64 x 64 tiles of 128 threads (8 x 4 outputs each: three 16-byte shared-memory reads per 32 FMAs)

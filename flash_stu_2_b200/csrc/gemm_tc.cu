@@ -1188,7 +1188,7 @@ int device_sm_count() {
   return n;
 }
 
-static int* device_status_word() { return g_status_words[current_device()]; }
+int* device_status_word() { return g_status_words[current_device()]; }
 
 // Test hook for the failure-detection path: the next tcgen05 GEMM launch of this process never issues the copies of
 // its first pipeline stage, and every bounded wait gives up after wait_ms milliseconds (0 restores the default of

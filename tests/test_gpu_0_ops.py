@@ -465,6 +465,51 @@ def test_conv_prefill_tcgen05_matches_fft_oracle(shape):
     close(x, x2, 8e-3, row_tol=1.6e-2)
 
 
+@pytest.mark.parametrize("shape", [(65, 100, 1024), (127, 33, 1028), (129, 1, 2060), (300, 2049, 256), (1000, 700, 516), (8000, 96, 3072), (66, 512, 6144),
+                                   (2000, 1030, 100)])
+@pytest.mark.parametrize("epi", [0, 1, 2, 3])
+def test_fp32_linear_on_tensor_cores(shape, epi):
+    """fp32 products as six bf16 products: edges of tiles, of blocks of 64 of K and of its split over clusters, each epilogue.  Bar:
+    against float64 no further off than the CUDA-core GEMM on the same operands, but for the rounding of the result itself (2^-24)."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    torch.manual_seed(5)
+    x = torch.randn(M, K + 4, device=dev())[:, :K]          # rows that do not follow one another
+    W, W2 = torch.randn(2, N, K, device=dev()) / math.sqrt(K)
+    r = torch.randn(M, N, device=dev())
+    full = x.double() @ W.double().t()
+    Lh = (M // 16 + 1) * 8
+    kw = {0: {}, 1: dict(resid=r), 2: dict(W2=W2), 3: dict(hist_T=M, hist_t0=1, hist_Lh=Lh)}[epi]
+    err = []
+    for backend in (0, 1):
+        out = torch.zeros(1, N, 2, Lh, device=dev()) if epi == 3 else torch.full((M, N), float("nan"), device=dev())
+        ops.linear(x, W, out=out, epilogue=epi, backend=backend, **kw)
+        if epi == 3:
+            t = torch.arange(1, M + 1, device=dev())
+            assert int((out != 0).sum()) <= M * N
+            out = out[0][:, t % 2, t // 2].t()
+        want = {0: full, 1: r.double() + full, 2: torch.nn.functional.gelu(full, approximate="tanh") * (x.double() @ W2.double().t()), 3: full}[epi]
+        err.append(float((out.double() - want).norm() / want.norm()))
+    ops.check_status()
+    assert err[0] <= max(err[1], 2.0 ** -24), err
+
+
+def test_fp32_linear_on_tensor_cores_values_without_a_split():
+    """Infinities, NaN and values whose parts overflow come out as fp32 arithmetic has them."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(6)
+    x, W = torch.randn(200, 1024), torch.randn(70, 1024) / 32
+    x[3, 5], x[7, 9], x[9, 1], x[11, :] = float("inf"), float("nan"), 3e38, 0.0
+    x[11, 4], W[8, 2], W[:, 9] = 1e36, float("-inf"), 0.0
+    got = ops.linear(x.to(dev()), W.to(dev()))
+    want = ops.linear(x.to(dev()), W.to(dev()), backend=1)
+    ops.check_status()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    fin = want.isfinite()
+    assert float(((got - want)[fin].abs() / want[fin].abs().clamp_min(1)).max()) < 2e-5   # (1024 products of order 1/32: rounding of the partial sums)
+
+
 @pytest.mark.parametrize("shape", [(1, 256, 1000, 0), (2, 1279, 900, 1270), (3, 1500, 760, 700), (2, 2049, 480, 1800), (9, 2817, 160, 2815),
                                    (1, 4095, 320, 0)])
 def test_conv_prefill_tcgen05_stages_of_every_depth(shape):
