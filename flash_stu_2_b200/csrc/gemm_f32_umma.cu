@@ -1,9 +1,8 @@
 // fp32 GEMM on the 5th-generation tensor cores: y = epilogue(x @ W^T) for fp32 operands, to fp32 accuracy.
 //
-// Every operand value is split into three bf16 values that add up to it exactly (24 bits of significand: x1 nearest to x, x2 the
-// leading 8 bits of x - x1, x3 the rest), and the product is the sum of the six bf16 products whose order is above 2^-26 of it: x1 y1,
-// x1 y2, x2 y1, x2 y2, x1 y3, x3 y1.  bf16 products are exact in the tensor core; its fp32 sums are not rounded to nearest, so chains of
-// them are kept short: an accumulator takes 32 of K, the smallest products first, and is then added to fp32 sums in registers.  Error
+// Every operand value is split into three bf16 values that add up to it exactly (split3.cuh), and the product is the sum of six of their
+// products.  bf16 products are exact in the tensor core; its fp32 sums are not rounded to nearest, so chains of them are kept short:
+// an accumulator takes 32 of K, the smallest products first, and is then added to fp32 sums in registers.  Error
 // against float64, this kernel and the CUDA-core GEMM (2-norm, normal operands): K = 3072 1.4e-7 and 7.0e-7, 1024 1.2e-7 and 5.7e-7, 256
 // 7.7e-8 and 1.5e-7; positive ones (sums that are not rounded to nearest drift) 9.5e-8 and 4.2e-7, 9.4e-8 and 4.3e-7, 6.7e-8 and
 // 7.0e-8; 64 of K per accumulator 1.25e-7, 1.1e-7, 8.9e-8, positive 9.7e-8, 9.6e-8, 8.7e-8.  (The weight-streaming kernels of up to 64
@@ -24,6 +23,7 @@
 
 #include "common.cuh"
 #include "epilogue.cuh"
+#include "split3.cuh"
 #include "tma.cuh"
 
 int device_sm_count();      // gemm_tc.cu
@@ -58,25 +58,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
         "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
-}
-
-// Two consecutive values as one word of each plane.  The first part comes of a multiplication by 2^16 + 1 and two differences (Dekker's
-// and Veltkamp's splitting: a nearest value of 8 bits; past 2^111 not finite), which stay on the FMA pipe: conversions to bf16 are
-// a sixteenth of its rate.  The second part is cut off and not rounded: behind a nearest first part the signs of the rest are random,
-// and what is cut off is the third part whole.
-__device__ __forceinline__ uint64_t pack2(float a, float b) { return (uint64_t)__float_as_uint(a) | (uint64_t)__float_as_uint(b) << 32; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) { return fma2(b, 0xbf800000bf800000ull, a); }   // a - b
-__device__ __forceinline__ uint32_t upper_halves(uint64_t v) { return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632); }
-__device__ __forceinline__ void split2(float a, float b, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
-  const uint64_t x = pack2(a, b), t = fma2(x, pack2(65537.f, 65537.f), 0ull), x1 = sub2(t, sub2(t, x)), r = sub2(x, x1);
-  w1 = upper_halves(x1);
-  w2 = upper_halves(r);
-  w3 = upper_halves(sub2(r, r & 0xffff0000ffff0000ull));
 }
 
 struct Ctl {
@@ -200,12 +181,11 @@ __global__ void __launch_bounds__(THREADS, 1)
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t acc = tmem_base + ACC_COLS * a;
           if (leader) {
-            constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};   // smallest products first
 #pragma unroll
-            for (int p = 0; p < 6; p++)
+            for (int p = 0; p < SPLIT_PRODUCTS; p++)
 #pragma unroll
               for (int kk = 0; kk < CHAIN; kk++)
-                umma(acc, da + ((PA[p] * PLANE_A + 32 * (h * CHAIN + kk)) >> 4), db + ((PB[p] * PLANE_B + 32 * (h * CHAIN + kk)) >> 4), IDESC, p || kk ? 1u : 0u);
+                umma(acc, da + ((split_a(p) * PLANE_A + 32 * (h * CHAIN + kk)) >> 4), db + ((split_b(p) * PLANE_B + 32 * (h * CHAIN + kk)) >> 4), IDESC, p || kk ? 1u : 0u);
             if (h + 1 == CHAINS) umma_commit(&ctl->empty[s]);
             umma_commit(&ctl->acc_full[a]);
           }

@@ -284,6 +284,7 @@ PyMethodDef methods[] = {
     ENTRY(stu_full_conv),
     ENTRY(stu_full_decode_combine),
     ENTRY(stu_full_conv_tc5),
+    ENTRY(stu_full_conv_f32_tc5),
     ENTRY(stu_full_decode_prepare),
     ENTRY(stu_full_decode_step),
     ENTRY(stu_lds_chunk_scan),

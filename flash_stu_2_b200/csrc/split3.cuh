@@ -1,0 +1,29 @@
+// fp32 values as three bf16 values that add up to them, for products of fp32 accuracy on bf16 tensor cores.
+#pragma once
+#include "common.cuh"
+
+// Two consecutive values as one word of each part: x1 nearest to x, x2 the leading 8 bits of x - x1, x3 the rest, 24 bits of significand
+// in all.  The first part comes of a multiplication by 2^16 + 1 and two differences (Dekker's and Veltkamp's splitting: a nearest value of 8
+// bits; past 2^111 not finite), in pairs on the FMA pipe: conversions to bf16 are a sixteenth of its rate.  (As fused operations: a
+// product and the difference behind it would be fused by the compiler, and the first part not be one.)  The second part is cut off and
+// not rounded: behind a nearest first part the signs of the rest are random, and what is cut off is the third part whole.
+__device__ __forceinline__ uint64_t split_pair(float a, float b) { return (uint64_t)__float_as_uint(a) | (uint64_t)__float_as_uint(b) << 32; }
+__device__ __forceinline__ uint64_t split_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t split_sub2(uint64_t a, uint64_t b) { return split_fma2(b, 0xbf800000bf800000ull, a); }   // a - b
+__device__ __forceinline__ uint32_t split_upper(uint64_t v) { return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632); }
+__device__ __forceinline__ void split2(float a, float b, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
+  const uint64_t x = split_pair(a, b), t = split_fma2(x, split_pair(65537.f, 65537.f), 0ull);
+  const uint64_t x1 = split_sub2(t, split_sub2(t, x)), r = split_sub2(x, x1);
+  w1 = split_upper(x1);
+  w2 = split_upper(r);
+  w3 = split_upper(split_sub2(r, r & 0xffff0000ffff0000ull));
+}
+
+// The products that are formed, part of the one operand by part of the other, smallest first: what is left out is below 2^-26 of the product.
+constexpr int SPLIT_PRODUCTS = 6;
+__host__ __device__ constexpr int split_a(int p) { return p == 0 ? 2 : (p == 2 || p == 3 ? 1 : 0); }   // 2 0 1 1 0 0
+__host__ __device__ constexpr int split_b(int p) { return p == 1 ? 2 : (p == 2 || p == 4 ? 1 : 0); }   // 0 2 1 0 1 0

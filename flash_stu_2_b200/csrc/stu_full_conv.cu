@@ -1,4 +1,4 @@
-// Full variant, fp32: the operand U of the contraction for all K filters in one launch
+// Full variant, fp32, short calls (the others: stu_full_conv_f32_umma.cu): the operand U of the contraction for all K filters in one launch
 // (flash_stu/modules/stu.py:100-118; MiniSTU mini_stu/stu.py:240-269):
 //   U+-[b,t,k,i] = E +- Q,   E = sum_{j even} phi[j,k] x[b,t-j,i],   Q the same over odd j.
 //

@@ -268,9 +268,9 @@ class STU(nn.Module):
         Lh = hist.shape[3]
         ops.to_history(xn, hist, t0)
         U = torch.empty(B * T, nsign * K * d, dtype=xn.dtype, device=xn.device)
-        if xn.dtype == torch.float32:
-            # fp32 sums run on the CUDA cores: all filters in one launch (24 filters, 8 x 1000 positions of 64 channels:
-            # 122 launches, 1.35 ms -> 1 launch, 0.40 ms)
+        if ops.full_conv_f32_tc5_pays(hist, t0 + T):
+            ops.full_conv_f32_tc5(hist, phi, U, nsign == 2, t0, t0 + T)
+        elif xn.dtype == torch.float32:
             ops.full_conv(hist, phi, U, nsign == 2, t0, t0 + T)
         elif ops.full_conv_tc5_supported(hist):
             ops.full_conv_tc5(hist, phi, U, nsign == 2, t0, t0 + T)

@@ -620,6 +620,27 @@ def full_conv_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     _count(2)
 
 
+def full_conv_f32_tc5_pays(hist, t_end: int) -> bool:
+    """Whether full_conv_f32_tc5 takes less time than full_conv: tiles of 128 positions of a parity and 64 or 128 channels have to be worth
+    more than its second launch.  us, full_conv and this, 24 filters: 1 x 8 channels of 500 positions 16 and 15, 1 x 512 of 300 50 and 39,
+    1 x 256 of 300 28 and 28, 2 x 32 of 300 12 and 15, 8 x 64 of 200 29 and 24, 2 x 512 of 60 18 and 29."""
+    B, d, _, _ = hist.shape
+    return hist.dtype == torch.float32 and d % 4 == 0 and (t_end >= 400 or (t_end >= 200 and B * d >= 512))
+
+
+def full_conv_f32_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
+    """full_conv on the tcgen05 tensor cores, to fp32 accuracy."""
+    _cuda(hist, phi, U)
+    B, d, _, Lh = hist.shape
+    L, K = phi.shape
+    assert hist.is_contiguous() and phi.is_contiguous() and U.stride(1) == 1 and U.shape[0] == B * (t_end - t0)
+    scratch = torch.empty(_lib.load().stu_full_conv_f32_tc5_scratch_elems(B, d, K, t_end), dtype=torch.bfloat16, device=hist.device)
+    rc = _lib.native().stu_full_conv_f32_tc5(hist.data_ptr(), Lh, phi.data_ptr(), L, K, scratch.data_ptr(), U.data_ptr(), U.stride(0), B, d,
+                                             int(both_signs), t0, t_end, status_word(hist.device).data_ptr(), _dt(hist), _stream())
+    _lib.check(rc, "stu_full_conv_f32_tc5")
+    _count(2)
+
+
 def full_decode_step_supported(x2d, hist, K: int) -> bool:
     d = x2d.shape[1]
     return (x2d.dtype == torch.bfloat16 and K <= 32 and d % 8 == 0 and hist.shape[3] % 8 == 0 and hist.data_ptr() % 16 == 0

@@ -234,6 +234,12 @@ long long stu_full_conv_tc5_scratch_elems(int K, int t_end);
 int stu_full_conv_tc5(const void* hist, int Lh, const void* phi, int L, int K, void* scratch, void* U, long long ldU, int B,
                       int d, int both_signs, int t0, int t_end, int* status, int dtype, void* stream);
 
+/* The same for fp32 on the tcgen05 tensor cores (products of three bf16 parts of either operand): d and ldU multiples of 4; scratch holds
+ * stu_full_conv_f32_tc5_scratch_elems bf16 values (the parts of the taps and of the history). */
+long long stu_full_conv_f32_tc5_scratch_elems(int B, int d, int K, int t_end);
+int stu_full_conv_f32_tc5(const void* hist, int Lh, const void* phi, int L, int K, void* scratch, void* U, long long ldU, int B,
+                          int d, int both_signs, int t0, int t_end, int* status, int dtype, void* stream);
+
 /* One cached step of the full variant up to the contraction with M_phi, bf16, at most 32 filters: the optional RMSNorm of the
  * rows x, their append at position t = pos[0], U+- [B][(1 or 2) K d] and pos + 1, in one kernel.  taps8 [8][2K][Lh+8]:
  * stu_taps_rev8 of the K filters' even taps and of their odd taps ([2K][Lh], zero past the filters); t < limit <= 2 Lh. */

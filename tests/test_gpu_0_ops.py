@@ -494,6 +494,55 @@ def test_fp32_linear_on_tensor_cores(shape, epi):
     assert err[0] <= max(err[1], 2.0 ** -24), err
 
 
+@pytest.mark.parametrize("case", [(1, 8, 3, 0, 17, True), (3, 20, 5, 5, 257, True), (2, 64, 4, 0, 256, False), (1, 132, 7, 250, 515, True),
+                                  (5, 64, 24, 0, 1000, True)])
+def test_full_variant_fp32_convolutions_on_tensor_cores(case):
+    """Edges of blocks of 128 positions of a parity and of tiles of 64 and 128 channels, a resumed prefill, one sign; NaN in the cache behind
+    the last position.  Bar: against float64 no further off than the CUDA-core kernel, but for the rounding of E and of Q (2^-23)."""
+    from flash_stu_2_b200 import ops
+    B, d, K, t0, T, both = case
+    torch.manual_seed(3)
+    x, phi = torch.randn(B, T, d), torch.randn(T - 2, K) / 8
+    hist = _hist_from(x, (T + 31) // 16 * 8)
+    for p in range(2):
+        hist[:, :, p, (T - p + 1) // 2:] = float("nan")
+    hist, phi = hist.to(dev()), phi.to(dev())
+    U = [torch.full((B * (T - t0), (1 + both) * K * d), float("nan"), device=dev()) for _ in range(2)]
+    ops.full_conv_f32_tc5(hist, phi, U[0], both, t0, T)
+    ops.full_conv(torch.nan_to_num(hist), phi, U[1], both, t0, T)
+    ops.check_status()
+    n = 1 << (2 * T).bit_length()
+    X, sign = torch.fft.rfft(x.double().to(dev()), n=n, dim=1), torch.ones(T - 2, 1, device=dev(), dtype=torch.float64)
+    sign[1::2] = -1
+    want = torch.cat([torch.einsum("bfi,fk->bfki", X, torch.fft.rfft(f, n=n, dim=0)) for f in (phi.double(), phi.double() * sign)[:1 + both]], 2)
+    want = torch.fft.irfft(want, n=n, dim=1)[:, t0:T].reshape(B * (T - t0), -1)
+    err = [float((u.double() - want).norm() / want.norm()) for u in U]
+    assert err[0] <= max(err[1], 2.0 ** -23), err
+
+
+def test_full_variant_fp32_convolutions_of_values_without_a_split():
+    """An infinity, a NaN and a value whose parts overflow reach the results that they reach in fp32 arithmetic, and no others."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(4)
+    B, T, d, K = 1, 300, 8, 3
+    x, phi = torch.randn(B, T, d), torch.rand(T, K) + 0.5
+    x[0, 100, 1], x[0, 200, 2], x[0, 250, 3] = float("inf"), float("nan"), 1e36
+    hist = _hist_from(x, 152).to(dev())
+    U = torch.empty(T, 2 * K * d, device=dev())
+    ops.full_conv_f32_tc5(hist, phi.to(dev()), U, True, 0, T)
+    ops.check_status()
+    lag = torch.arange(T)[:, None] - torch.arange(T)[None]
+    for s in range(2):
+        taps = phi.double() * torch.where(torch.arange(T)[:, None] % 2 == 0, 1.0, 1.0 - 2 * s)
+        got = U.view(T, 2, K, d)[:, s].cpu()
+        for i in (0, 1, 2, 3):
+            start = {1: 100, 2: 200}.get(i, T)
+            assert bool(got[:start, :, i].isfinite().all()) and not bool(got[start:, :, i].isfinite().any())
+            m = torch.where(lag[:start, :start, None] >= 0, taps[lag[:start, :start].clamp_min(0)], torch.zeros((), dtype=torch.float64))
+            want = torch.einsum("tsk,s->tk", m, x[0, :start, i].double())
+            assert float(((got[:start, :, i].double() - want).abs() / want.abs().clamp_min(1)).max()) < 1e-4   # (300 products in one chain)
+
+
 def test_fp32_linear_on_tensor_cores_values_without_a_split():
     """Infinities, NaN and values whose parts overflow come out as fp32 arithmetic has them."""
     from flash_stu_2_b200 import ops
