@@ -400,12 +400,17 @@ bool skinny_wide_takes(int M, int N, int K, int epi, bool norm);
 int skinny_wide_dispatch(const void* A, long long lda, const void* B, long long ldb, int M, int N, int K, int epi,
                          const EpiArgs<bf16>& ep, const void* nw, float eps, cudaStream_t st);
 
+bool skinny_long_takes(int M, int N, int K, int epi, bool norm, bool peer);   // skinny_long.cu
+int skinny_long_dispatch(const void* A, long long lda, const void* B, long long ldb, int M, int N, int K, int epi, const EpiArgs<bf16>& ep,
+                         int pdl, cudaStream_t st);
 bool stream_takes(int M, int N, int K, int epi, int dtype, const void* norm_w, bool peer);   // stream.cu
 int stream_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N, int K,
                     int epi, const EpiArgsAny& ep, const void* norm_w, float eps, int dtype, int pdl, cudaStream_t st);
 
 int skinny_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N, int K,
                     int epi, const EpiArgsAny& ep, const void* norm_w, float eps, int dtype, int pdl, cudaStream_t st) {
+  if (dtype == STU_BF16 && skinny_long_takes(M, N, K, epi, norm_w != nullptr, ep.peer != nullptr))
+    return skinny_long_dispatch(A, lda, B, ldb, M, N, K, epi, ep.as<bf16>(), pdl, st);
   if (stream_takes(M, N, K, epi, dtype, norm_w, ep.peer != nullptr))
     return stream_dispatch(A, lda, B, ldb, B2, M, N, K, epi, ep, norm_w, eps, dtype, pdl, st);
   if (dtype == STU_BF16) {

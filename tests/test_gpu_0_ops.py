@@ -494,6 +494,26 @@ def test_fp32_linear_on_tensor_cores(shape, epi):
     assert err[0] <= max(err[1], 2.0 ** -24), err
 
 
+@pytest.mark.parametrize("shape", [(8, 1024, 49152), (1, 640, 14720), (5, 768, 12296), (7, 1200, 4104), (8, 2049, 4096), (3, 4735, 8192)])
+@pytest.mark.parametrize("epi", [0, 1])
+@pytest.mark.parametrize("early", [False, True])
+def test_linear_of_few_rows_over_long_weights(shape, epi, early):
+    """Up to 8 rows: clusters of one, two and four CTAs, features and K that end inside a tile and a chunk, launched beside the kernel in
+    front that writes its rows.  Bar: one rounding to bf16 of a sum of K products (and of its sum with the residual)."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    torch.manual_seed(9)
+    x, W, r = torch.randn(M, K), torch.randn(N, K) / math.sqrt(K), torch.randn(M, N)
+    x, W, r = (t.bfloat16().to(dev()) for t in (x, W, r))
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev())
+    rows = ops.rmsnorm(x, torch.ones(K, dtype=torch.bfloat16, device=dev()), 1e-6)   # the kernel in front
+    ops.linear(rows, W, resid=r if epi else None, out=out, epilogue=epi | (ops.FLAG_OVERLAP if early else 0))
+    ops.check_status()
+    full = rows.double() @ W.double().t()
+    want = (r.double() + full.bfloat16().double()) if epi else full
+    assert float((out.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-3
+
+
 @pytest.mark.parametrize("case", [(1, 8, 3, 0, 17, True), (3, 20, 5, 5, 257, True), (2, 64, 4, 0, 256, False), (1, 132, 7, 250, 515, True),
                                   (5, 64, 24, 0, 1000, True)])
 def test_full_variant_fp32_convolutions_on_tensor_cores(case):
