@@ -61,6 +61,8 @@ _SIGNATURES = {
                                  _P], c_int),
     "stu_conv_prefill_approx_tc5": ([_P, _P, _P, _P, _LL, _LL, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int,
                                      _P], c_int),
+    "stu_conv_prefill_positions": ([_P, _P, _P, _P, _LL, _LL, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, c_int, _P, c_int, _P],
+                                   c_int),
     "stu_conv_prefill_set_timeline": ([_P], c_int),
     "stu_set_programmatic_launch": ([c_int], c_int),
     "stu_conv_prefill_approx_static": ([_P, _P, _P, _LL, _LL, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],

@@ -265,6 +265,69 @@ PyObject* layer_step_f32(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_RETURN_NONE;
 }
 
+// layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, eps, mlp_eps, t0, fresh, kind, status): new positions of an
+// approx layer, in place on x [B, T, d]: x += STU(norm(x)); x += MLP(norm(x)), seven launches.  kind and taps as in
+// stu_conv_prefill_positions; pos may be None.  Returns 3, or 1 where the MLP was refused (the STU is done), or None where the STU was
+// (x is as it was, and so are the positions).
+PyObject* layer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 16) {
+    PyErr_SetString(PyExc_TypeError, "16 arguments expected");
+    return nullptr;
+  }
+  try {
+    const at::Tensor* t[10];
+    for (int i = 0; i < 10; i++) {
+      if (!plain(args[i], &t[i]) || (!t[i] && i != 5)) Py_RETURN_NONE;
+      if (t[i] && (!t[i]->is_contiguous() || t[i]->device() != t[0]->device() || t[i]->scalar_type() != (i == 5 ? at::kInt : t[0]->scalar_type())))
+        Py_RETURN_NONE;
+    }
+    const at::Tensor &x = *t[0], &hist = *t[3], &gate = *t[7];
+    const int dev = x.device().index(), code = dtype_code(x);
+    if (code < 0 || x.dim() != 3 || x.numel() == 0 || hist.dim() != 4 || gate.dim() != 2 || dev != c10::cuda::current_device() ||
+        !(g_ready.load(std::memory_order_relaxed) >> dev & 1))
+      Py_RETURN_NONE;
+    const int64_t B = x.size(0), T = x.size(1), d = x.size(2), Lh = hist.size(3), I = gate.size(0);
+    const float eps = value_of<float>(args[10]), mlp_eps = value_of<float>(args[11]);
+    const int t0 = value_of<int>(args[12]), fresh = value_of<int>(args[13]), kind = value_of<int>(args[14]);
+    int* status = static_cast<int*>(address_of(args[15]));
+    const auto is = [&](int i, at::IntArrayRef want) { return t[i]->sizes() == want; };
+    if (B * T > INT32_MAX || d > INT32_MAX || I > INT32_MAX || Lh > INT32_MAX || t0 < 0 || t0 + T > 2 * Lh || !is(1, {d}) || !is(2, {d, d}) ||
+        !is(3, {B, d, 2, Lh}) || (kind == 2 ? !is(4, {8, d, Lh + 8}) : !is(4, {d, Lh})) || (t[5] && !is(5, {B, 2})) || !is(6, {d}) ||
+        !is(7, {I, d}) || !is(8, {I, d}) || !is(9, {d, I}))
+      Py_RETURN_NONE;
+    const int64_t yLh = ((t0 + T + 1) / 2 + 7) / 8 * 8;
+    const int M = (int)(B * T), t_end = (int)(t0 + T);
+    at::Tensor xn = at::empty({M, d}, x.options()), yT = at::empty({B, d, 2, yLh}, x.options()), h = at::empty({M, I}, x.options());
+    void* p[10];
+    for (int i = 0; i < 10; i++) p[i] = data_of(t[i]);
+    void *pn = xn.data_ptr(), *py = yT.data_ptr(), *ph = h.data_ptr(), *stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
+    int rc, done = 0;
+    Py_BEGIN_ALLOW_THREADS
+    rc = stu_rmsnorm(p[0], p[1], pn, M, (int)d, d, d, eps, code, stream);
+    if (rc == 0)
+      rc = stu_linear(pn, d, p[2], d, 1, nullptr, nullptr, 0, p[3], 0, M, (int)d, (int)d, 3, (int)T, t0, (int)Lh, nullptr, 0.f, code, 0, stream);
+    if (rc == 0)
+      rc = stu_conv_prefill_positions(p[3], p[4], py, p[0], T * d, d, (int)B, (int)d, (int)Lh, (int)yLh, t0, t_end, (int*)p[5], fresh, kind,
+                                      status, code, stream);
+    if (rc == 0) {
+      done = 1;
+      rc = stu_rmsnorm(p[0], p[6], pn, M, (int)d, d, d, mlp_eps, code, stream);
+    }
+    if (rc == 0)
+      rc = stu_linear(pn, d, p[7], d, 1, p[8], nullptr, 0, ph, I, M, (int)I, (int)d, 2, 0, 0, 0, nullptr, 0.f, code, 0, stream);
+    if (rc == 0)
+      rc = stu_linear(ph, I, p[9], I, 1, nullptr, p[0], d, p[0], d, M, (int)d, (int)I, 1, 0, 0, 0, nullptr, 0.f, code, 0, stream);
+    Py_END_ALLOW_THREADS
+    if (raised(rc, "layer_prefill")) return nullptr;
+    if (rc == 0) done = 3;
+    if (done) return PyLong_FromLong(done);
+  } catch (const BadArgument&) {
+    PyErr_Clear();
+  } catch (const std::exception&) {
+  }
+  Py_RETURN_NONE;
+}
+
 // what ops.py launches
 #define ENTRY(name) {#name, (PyCFunction)(void (*)(void))Call<&name>::call, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
@@ -308,6 +371,7 @@ PyMethodDef methods[] = {
     {"status_ready", (PyCFunction)(void (*)(void))status_ready, METH_FASTCALL, nullptr},
     {"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, nullptr},
     {"layer_step_f32", (PyCFunction)(void (*)(void))layer_step_f32, METH_FASTCALL, nullptr},
+    {"layer_prefill", (PyCFunction)(void (*)(void))layer_prefill, METH_FASTCALL, nullptr},
     {"rmsnorm", (PyCFunction)(void (*)(void))rmsnorm, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

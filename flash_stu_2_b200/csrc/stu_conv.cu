@@ -260,7 +260,12 @@ __global__ void __launch_bounds__(256) conv_mma_kernel(const bf16* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) transpose_add_kernel(T* __restrict__ x, long long x_bstride,
                                                             long long x_tstride, const T* __restrict__ yT, int d,
-                                                            int Lh, int t0, int t_end) {
+                                                            int Lh, int t0, int t_end, int* __restrict__ pos, int B, int fresh) {
+  if (pos && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)   // the sequences' positions move on with the last kernel of the call
+    for (int i = threadIdx.x; i < B; i += 256) {
+      pos[2 * i] = fresh ? t_end : pos[2 * i] + (t_end - t0);
+      if (fresh) pos[2 * i + 1] = 0;
+    }
   constexpr int V = Elem<T>::VEC;           // elements per 16 bytes
   constexpr int TC = 8 * V;                 // channels per CTA (64 bf16 / 32 fp32)
   constexpr int TS = 64;                    // time indices per parity per CTA
@@ -304,17 +309,17 @@ __global__ void __launch_bounds__(256) transpose_add_kernel(T* __restrict__ x, l
 
 // Residual add of a finished convolution: x[b, t - t0, :] += yT[b][:][t&1][t>>1] for t in [t0, t_end).
 int launch_transpose_add(void* x, long long x_bstride, long long x_tstride, const void* yT, int B, int d, int y_Lh,
-                         int t0, int t_end, int dtype, cudaStream_t st) {
+                         int t0, int t_end, int* pos, int fresh, int dtype, cudaStream_t st) {
   const int v2 = (dtype == STU_F32) ? 8 : 16;  // 2V: the kernel aligns its first tile to this
   int tb = t0 - t0 % v2;
   const int tc = (dtype == STU_F32) ? 32 : 64;
   dim3 g2((t_end - tb + 127) / 128, (d + tc - 1) / tc, B);
   if (dtype == STU_F32)
     transpose_add_kernel<float><<<g2, 256, 0, st>>>((float*)x, x_bstride, x_tstride, (const float*)yT, d, y_Lh, t0,
-                                                    t_end);
+                                                    t_end, pos, B, fresh);
   else
     transpose_add_kernel<bf16><<<g2, 256, 0, st>>>((bf16*)x, x_bstride, x_tstride, (const bf16*)yT, d, y_Lh, t0,
-                                                   t_end);
+                                                   t_end, pos, B, fresh);
   STU_CHECK_LAUNCH();
   return STU_OK;
 }
@@ -322,9 +327,8 @@ int launch_transpose_add(void* x, long long x_bstride, long long x_tstride, cons
 // Prefill convolution entry point: hist holds projected inputs for times [0, t_end); computes the
 // convolution outputs for times [t0, t_end) into yT (same layout as hist, y_Lh elements per parity row) and adds them to x
 // ([B, t_end - t0, d] with the given strides).  use_tensor_cores selects conv_mma_kernel (bf16).
-extern "C" int stu_conv_prefill_approx(const void* hist, const void* taps, void* yT, void* x, long long x_bstride,
-                                       long long x_tstride, int B, int d, int Lh, int y_Lh, int t0, int t_end,
-                                       int dtype, int use_tensor_cores, void* stream) {
+static int conv_prefill_approx(const void* hist, const void* taps, void* yT, void* x, long long x_bstride, long long x_tstride, int B, int d,
+                               int Lh, int y_Lh, int t0, int t_end, int* pos, int fresh, int dtype, int use_tensor_cores, void* stream) {
   if (!hist || !taps || !yT || !x) return STU_ERR_NULL;
   if (B <= 0 || d <= 0 || Lh <= 0 || t0 < 0 || t_end <= t0 || t_end > 2 * Lh || t_end > 2 * y_Lh)
     return STU_ERR_SHAPE;
@@ -361,7 +365,27 @@ extern "C" int stu_conv_prefill_approx(const void* hist, const void* taps, void*
     }
   }
   STU_CHECK_LAUNCH();
-  return launch_transpose_add(x, x_bstride, x_tstride, yT, B, d, y_Lh, t0, t_end, dtype, st);
+  return launch_transpose_add(x, x_bstride, x_tstride, yT, B, d, y_Lh, t0, t_end, pos, fresh, dtype, st);
+}
+
+extern "C" int stu_conv_prefill_approx(const void* hist, const void* taps, void* yT, void* x, long long x_bstride,
+                                       long long x_tstride, int B, int d, int Lh, int y_Lh, int t0, int t_end,
+                                       int dtype, int use_tensor_cores, void* stream) {
+  return conv_prefill_approx(hist, taps, yT, x, x_bstride, x_tstride, B, d, Lh, y_Lh, t0, t_end, nullptr, 0, dtype, use_tensor_cores, stream);
+}
+
+int conv_prefill_approx_tc5(const void* hist, const void* taps8, void* yT, void* x, long long x_bstride, long long x_tstride, int B, int d, int Lh,
+                            int y_Lh, int t0, int t_end, int* pos, int fresh, int* status, int dtype, void* stream);   // stu_conv_umma.cu
+
+// One of the three forms (kind 0: CUDA cores, 1: mma.sync, 2: tcgen05, whose taps are the reversed table), and the positions pos [B][2]
+// (NULL: none) behind it: t_end, and a cleared counter, where the cache is fresh, else t_end - t0 more than they were.
+extern "C" int stu_conv_prefill_positions(const void* hist, const void* taps, void* yT, void* x, long long x_bstride, long long x_tstride, int B,
+                                          int d, int Lh, int y_Lh, int t0, int t_end, int* pos, int fresh, int kind, int* status, int dtype,
+                                          void* stream) {
+  if (kind < 0 || kind > 2 || (fresh && t0 != 0)) return STU_ERR_SHAPE;
+  if (kind == 2)
+    return conv_prefill_approx_tc5(hist, taps, yT, x, x_bstride, x_tstride, B, d, Lh, y_Lh, t0, t_end, pos, fresh, status, dtype, stream);
+  return conv_prefill_approx(hist, taps, yT, x, x_bstride, x_tstride, B, d, Lh, y_Lh, t0, t_end, pos, fresh, dtype, kind, stream);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -53,7 +53,7 @@
 
 int device_sm_count();
 int launch_transpose_add(void* x, long long x_bstride, long long x_tstride, const void* yT, int B, int d, int y_Lh,
-                         int t0, int t_end, int dtype, cudaStream_t st);
+                         int t0, int t_end, int* pos, int fresh, int dtype, cudaStream_t st);
 
 namespace {
 
@@ -461,9 +461,8 @@ extern "C" int stu_conv_prefill_set_timeline(void* device_words) {
   return STU_OK;
 }
 
-extern "C" int stu_conv_prefill_approx_tc5(const void* hist, const void* taps8, void* yT, void* x, long long x_bstride,
-                                           long long x_tstride, int B, int d, int Lh, int y_Lh, int t0, int t_end,
-                                           int* status, int dtype, void* stream) {
+int conv_prefill_approx_tc5(const void* hist, const void* taps8, void* yT, void* x, long long x_bstride, long long x_tstride, int B, int d, int Lh,
+                            int y_Lh, int t0, int t_end, int* pos, int fresh, int* status, int dtype, void* stream) {
   if (!hist || !taps8 || !yT || !x) return STU_ERR_NULL;
   if (B <= 0 || d <= 0 || Lh <= 0 || t0 < 0 || t_end <= t0 || t_end > 2 * Lh || t_end > 2 * y_Lh) return STU_ERR_SHAPE;
   if (dtype != STU_BF16) return STU_ERR_DTYPE;
@@ -501,5 +500,11 @@ extern "C" int stu_conv_prefill_approx_tc5(const void* hist, const void* taps8, 
                                                                       status, 2000000000ull,
                                                                       g_timeline);
   STU_CHECK_LAUNCH();
-  return launch_transpose_add(x, x_bstride, x_tstride, yT, B, d, y_Lh, t0, t_end, dtype, st);
+  return launch_transpose_add(x, x_bstride, x_tstride, yT, B, d, y_Lh, t0, t_end, pos, fresh, dtype, st);
+}
+
+extern "C" int stu_conv_prefill_approx_tc5(const void* hist, const void* taps8, void* yT, void* x, long long x_bstride,
+                                           long long x_tstride, int B, int d, int Lh, int y_Lh, int t0, int t_end,
+                                           int* status, int dtype, void* stream) {
+  return conv_prefill_approx_tc5(hist, taps8, yT, x, x_bstride, x_tstride, B, d, Lh, y_Lh, t0, t_end, nullptr, 0, status, dtype, stream);
 }

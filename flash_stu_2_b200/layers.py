@@ -157,12 +157,18 @@ class STULayer(nn.Module):
         elif T == 1 and past_key_value is not None:
             entry = self._decode(xc, past_key_value)
         else:
+            stu, mlp = child(self, "stu"), child(self, "mlp")
             stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
-            xn = ops.rmsnorm(xc, param(stu_norm, "weight"), stu_norm.eps)
-            entry = child(self, "stu").add_to_residual(xn, xc, past_key_value, use_cache)
-            x2 = xc.view(B * T, d)
-            xn2 = ops.rmsnorm(x2, param(mlp_norm, "weight"), mlp_norm.eps)
-            child(self, "mlp").apply_residual(xn2, x2, x2)
+            done, entry = 0, past_key_value
+            if stu.use_approx and not stu.use_hankel_L and own(stu, STU, "add_to_residual") and own(mlp, MLP, "apply_residual"):
+                done, entry = stu.layer_prefill(xc, entry, use_cache, stu_norm, mlp_norm, mlp)
+            if not done:
+                xn = ops.rmsnorm(xc, param(stu_norm, "weight"), stu_norm.eps)
+                entry = stu.add_to_residual(xn, xc, entry, use_cache)
+            if done != 3:
+                x2 = xc.view(B * T, d)
+                xn2 = ops.rmsnorm(x2, param(mlp_norm, "weight"), mlp_norm.eps)
+                mlp.apply_residual(xn2, x2, x2)
         if xc is not x:
             x.copy_(xc)
         if use_cache:

@@ -40,6 +40,14 @@ def new_pos(batch: int, device) -> torch.Tensor:
     return p
 
 
+def unwritten_pos(batch: int, device) -> torch.Tensor:
+    """new_pos for a call whose kernels write the positions."""
+    p = torch.empty(batch, 2, dtype=torch.int32, device=device)
+    p._host_t = 0
+    p._uniform = True
+    return p
+
+
 def host_pos(pos: torch.Tensor) -> int:
     """Host-side mirror of pos[0,0]; falls back to a device read when the tensor was re-created
     (e.g. by _reorder_cache), which also re-checks whether all sequences share one position."""
@@ -234,16 +242,18 @@ class STU(nn.Module):
         return (self.M_inputs if self.use_approx else self.M_phi_plus).dtype
 
     def new_cache(self, batch: int, device, filled: int = 0) -> Tuple[torch.Tensor, torch.Tensor]:
-        """An empty cache; the first `filled` positions are about to be written and need not be zeroed.  (Zeros over most of a row
-        are written faster over all of it.)"""
+        """An empty cache; the first `filled` positions are about to be written and need not be zeroed."""
+        return self._new_history(batch, device, filled), new_pos(batch, device)
+
+    def _new_history(self, batch: int, device, filled: int):
+        """(Zeros over most of a row are written faster over all of it.)"""
         kept = filled // 2
         if 4 * kept < 3 * self.Lh:
-            hist = torch.zeros(batch, self.d_in, 2, self.Lh, dtype=self.param_dtype, device=device)
-        else:
-            hist = torch.empty(batch, self.d_in, 2, self.Lh, dtype=self.param_dtype, device=device)
-            if kept < self.Lh:
-                hist[..., kept:].zero_()
-        return hist, new_pos(batch, device)
+            return torch.zeros(batch, self.d_in, 2, self.Lh, dtype=self.param_dtype, device=device)
+        hist = torch.empty(batch, self.d_in, 2, self.Lh, dtype=self.param_dtype, device=device)
+        if kept < self.Lh:
+            hist[..., kept:].zero_()
+        return hist
 
     # ------------------------------------------------------------------ full variant
     def full_forward(self, xn: torch.Tensor, resid: Optional[torch.Tensor], out: torch.Tensor, entry=None,
@@ -345,6 +355,38 @@ class STU(nn.Module):
         ops.linear(U, Mcat, resid=resid2d, out=out2d, epilogue=ops.EPI_RESID | (ops.FLAG_OVERLAP if ops.overlap_decode else 0))
         pos._host_t = t + 1
         return hist, pos
+
+    def layer_prefill(self, x: torch.Tensor, entry, use_cache: bool, stu_norm, mlp_norm, mlp):
+        """(done, entry): add_to_residual of the normalised x [B,T,d] (contiguous) and the MLP behind it as one native call; see
+        ops.layer_prefill.  Where it does nothing, entry is what add_to_residual is to be given."""
+        B, T, d = x.shape
+        MinT, taps, taps8 = self.prepared()
+        t0, fresh = 0, False
+        if entry is not None:
+            hist, pos = entry
+            t0 = host_pos(pos)
+        if t0 + T > self.capacity:
+            raise ValueError(f"sequence position {t0 + T} exceeds the capacity {self.capacity} (seq_len={self.seq_len}: "
+                             f"the filters have seq_len taps; cache_len={self.cache_len})")
+        if entry is None:
+            if use_cache and own(self, STU, "new_cache"):
+                hist, pos, fresh = self._new_history(B, x.device, T), unwritten_pos(B, x.device), True
+            elif use_cache:
+                hist, pos = self.new_cache(B, x.device)
+            else:
+                hist, pos = torch.empty(B, d, 2, self.Lh, dtype=x.dtype, device=x.device), None
+        kind = (0 if x.dtype != torch.bfloat16 or not STU.tensor_core_conv
+                else 2 if STU.tcgen05_conv and taps8 is not None and ops.conv_prefill_tc5_supported(hist, x) else 1)
+        done = ops.layer_prefill(x, param(stu_norm, "weight"), MinT, hist, taps8 if kind == 2 else taps, pos, param(mlp_norm, "weight"),
+                                 param(child(mlp, "gate_proj"), "weight"), param(child(mlp, "up_proj"), "weight"),
+                                 param(child(mlp, "down_proj"), "weight"), stu_norm.eps, mlp_norm.eps, t0, fresh, kind)
+        if pos is None:
+            return done, None
+        if done:
+            pos._host_t = t0 + T
+        elif fresh:
+            pos.zero_()
+        return done, (hist, pos)
 
     def add_to_residual(self, xn: torch.Tensor, x: torch.Tensor, entry=None, use_cache: bool = False):
         """x += STU(xn) for xn, x [B,T,d] (x contiguous).  Returns the cache entry when use_cache."""

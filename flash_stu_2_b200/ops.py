@@ -378,6 +378,21 @@ def layer_step_f32(x, norm_w, MinT, hist, taps, pos, mid, mlp_norm_w, gate, up, 
     return done
 
 
+def layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, eps: float, mlp_eps: float, t0: int, fresh: bool,
+                  kind: int) -> int:
+    """New positions of an approx layer, in place on x [B,T,d], seven launches in one native call; the positions move on in the last kernel
+    of the convolution (fresh: they need not have been written before).  kind 2 (taps: the reversed table): tcgen05, 1: mma.sync,
+    0: CUDA cores.  3: done; 1: the MLP is left to the caller; 0: all of it is."""
+    if getattr(_local, "arena", None) is not None:
+        return 0
+    done = _lib.native().layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, eps, mlp_eps, t0, int(fresh), kind,
+                                       status_word(x.device))
+    if done is None:
+        return 0
+    _count(7 if done == 3 else 4)
+    return done
+
+
 def decode_approx_shard(x, norm_w, MinT, hist, taps8, pos, out, eps: float = RMS_EPS, add_residual: bool = False,
                         flags: int = 0):
     """Fused decode step for the d_ch channels of a tensor-parallel rank: x [B,d_in] (full layer input), MinT

@@ -128,6 +128,13 @@ int stu_conv_prefill_approx_tc5(const void* hist, const void* taps8, void* yT, v
                                 long long x_tstride, int B, int d, int Lh, int y_Lh, int t0, int t_end, int* status,
                                 int dtype, void* stream);
 
+/* stu_conv_prefill_approx (kind 0: CUDA cores, 1: tensor cores) or stu_conv_prefill_approx_tc5 (kind 2; taps is taps8 there), and the
+ * positions behind it, in its last kernel: pos [B][2] (NULL: none) become (t_end, 0) where the cache is fresh (then t0 = 0), else the first
+ * of either pair t_end - t0 more than it was. */
+int stu_conv_prefill_positions(const void* hist, const void* taps, void* yT, void* x, long long x_bstride, long long x_tstride, int B,
+                               int d, int Lh, int y_Lh, int t0, int t_end, int* pos, int fresh, int kind, int* status, int dtype,
+                               void* stream);
+
 /* The token-step kernels (RMSNorm, the decode linears, the attention and STU decode kernels) are launched with the
  * programmatic-stream-serialization attribute: each fetches its weights while the kernel before it drains and waits
  * (griddepcontrol.wait) before it touches anything that kernel writes.  stu_set_programmatic_launch(0) turns the

@@ -460,3 +460,41 @@ def test_a_new_cache_is_zero_behind_the_prefill(T):
             for parity in (0, 1):
                 n = (T + 1 - parity) // 2
                 assert bool((cache[0][:, :, parity, n:] == 0).all()) and bool(torch.isfinite(cache[0][:, :, parity, :n]).all())
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,first,second", [(1, 1, 2), (3, 50, 1), (2, 300, 211), (9, 17, 64)])
+def test_prefill_in_one_native_call_equals_the_parts(dt, B, first, second, monkeypatch):
+    """Two calls on one cache, the second resumed: outputs, history and positions are those of the kernels called one by one, with every
+    form of the convolution, without a cache, and where the call is refused."""
+    import flash_stu_2_b200 as F
+    from flash_stu_2_b200 import ops
+    from flash_stu_2_b200.modules import STU
+    torch.manual_seed(2)
+    cfg = F.FlashSTUConfig(n_embd=64, n_layers=1, n_heads=1, seq_len=600, vocab_size=1, mlp_scale=4, num_eigh=8, torch_dtype=dt, use_attn=False)
+    blk = F.FlashSTUBlock(config=cfg).cuda().eval()
+    for name, p in blk.named_parameters():
+        torch.nn.init.normal_(p, 1.0 if name.endswith("norm.weight") else 0.0, 0.1)
+    x = torch.randn(B, first + second, 64, device="cuda").to(dt)
+
+    def run():
+        with torch.no_grad():
+            a, b, c = (t.clone(memory_format=torch.contiguous_format) for t in (x[:, :first], x[:, first:], x[:, :first]))
+            _, past = blk(a, use_cache=True)
+            _, past = blk(b, past_key_value=past, use_cache=True)
+            blk(c)
+            ops.check_status()
+            return a, b, c, past[0].clone(), past[1].clone(), past[1]._host_t
+
+    calls, whole = [], ops.layer_prefill
+    monkeypatch.setattr(ops, "layer_prefill", lambda *a: calls.append(whole(*a)) or calls[-1])
+    for tc, tc5 in [(True, True), (True, False), (False, False)]:
+        monkeypatch.setattr(STU, "tensor_core_conv", tc)
+        monkeypatch.setattr(STU, "tcgen05_conv", tc5)
+        del calls[:]
+        one = run()
+        assert calls == [3] * (3 - (second == 1))   # (a single cached position is a token step)
+        with monkeypatch.context() as m:
+            m.setattr(ops, "layer_prefill", lambda *a: 0)
+            parts = run()
+        assert all(torch.equal(p, q) for p, q in zip(one[:5], parts[:5])) and one[5] == parts[5] == first + second
