@@ -21,6 +21,8 @@
 // Every wait is bounded: on expiry the CTA raises status 3, frees its tensor memory and returns.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "split3.cuh"
@@ -273,6 +275,38 @@ struct Operands {
   int M, N, K, causal;
 };
 
+// How many clusters of KS CTAs the GPU holds at a time (the SMs of a GPC are no multiple of 8: 8 leave some of them out)
+template <int EPI, int KS, int BN>
+int clusters_at_once() {
+  static std::atomic<int> known[STU_MAX_DEVICES] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= STU_MAX_DEVICES) dev = 0;
+  int n = KS == 1 ? device_sm_count() : known[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  auto kern = gemm_f32_umma_kernel<EPI, KS, BN>;
+  static SmemLimit limit;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, 1, KS);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem_bytes<BN>();
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = KS;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (allow_smem((const void*)kern, smem_bytes<BN>(), limit) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = 1;
+  }
+  known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+template <int EPI, int BN>
+int clusters_at_once(int ks) {
+  return ks == 1 ? clusters_at_once<EPI, 1, BN>() : ks == 2 ? clusters_at_once<EPI, 2, BN>() : ks == 4 ? clusters_at_once<EPI, 4, BN>() : clusters_at_once<EPI, 8, BN>();
+}
+
 template <int EPI, int KS, int BN>
 int launch_tile(const Operands& o, const EpiArgs<float>& ep, cudaStream_t st) {
   constexpr int COLS = EPI == EPI_GELU_MUL ? BN / 2 : BN;
@@ -315,20 +349,21 @@ int launch_split(const Operands& o, int ks, const EpiArgs<float>& ep, cudaStream
   }
 }
 
-// The tile width and the split of K that take the least time: waves of CTAs, one per SM, of 4.2 us and 1.05, 1.5 or 1.95 us per block of 64 of
-// K (32, 64 or 128 columns), 0.8 us and a tenth per CTA of a cluster (fitted to 26 shapes of 20 to 8192 rows; within 10 % of the best of all
-// in each).
+// The tile width and the split of K that take the least time: waves of clusters, a CTA per SM, of 4.2 us and 1.05, 1.5 or 1.95 us per block of
+// 64 of K (32, 64 or 128 columns), 0.8 us and a tenth per CTA of a cluster (fitted to 26 shapes of 20 to 8192 rows; within 10 % of the best of
+// all in each).
 template <int EPI>
 int launch_epi(const Operands& o, const EpiArgs<float>& ep, cudaStream_t st) {
-  const int sms = device_sm_count(), blocks = (o.K + BK - 1) / BK;
+  const int blocks = (o.K + BK - 1) / BK;
   double best = 1e30;
   int best_bn = 128, best_ks = 1;
   for (int bn = 128; bn >= 32; bn /= 2)
     for (int ks = 1; ks <= 8 && (ks == 1 || blocks >= ks); ks *= 2) {
       const int cols = EPI == EPI_GELU_MUL ? bn / 2 : bn;
-      const long long ctas = (long long)((o.M + BM - 1) / BM) * ((o.N + cols - 1) / cols) * ks;
+      const long long tiles = (long long)((o.M + BM - 1) / BM) * ((o.N + cols - 1) / cols);
+      const int room = bn == 128 ? clusters_at_once<EPI, 128>(ks) : bn == 64 ? clusters_at_once<EPI, 64>(ks) : clusters_at_once<EPI, 32>(ks);
       const double block = bn == 128 ? 1.95 : bn == 64 ? 1.5 : 1.05;
-      const double t = (double)((ctas + sms - 1) / sms) * (4.2 + (blocks + ks - 1) / ks * block + (ks > 1 ? 0.8 + 0.1 * ks : 0.0));
+      const double t = (double)((tiles + room - 1) / room) * (4.2 + (blocks + ks - 1) / ks * block + (ks > 1 ? 0.8 + 0.1 * ks : 0.0));
       if (t < best) best = t, best_bn = bn, best_ks = ks;
     }
   switch (best_bn) {
