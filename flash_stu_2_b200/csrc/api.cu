@@ -38,11 +38,11 @@ bool skinny_umma_takes(int M, int N, int K, int epi, bool norm, bool peer);   //
 // Small-M shapes for which the tcgen05 GEMM beats the weight-streaming kernel.
 static bool prefers_tensor_gemm(int M, int N) { return (M >= 32 && N >= 5120) || (M >= 16 && N >= 32768); }
 
-extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, long long w_row_stride,
-                          long long w_k_stride, const void* W2, const void* resid, long long resid_row_stride,
-                          void* y, long long y_row_stride, int M, int N, int K, int epilogue, int hist_T,
-                          int hist_t0, int hist_Lh, const void* norm_w, float eps, int dtype, int backend,
-                          void* stream) {
+extern "C" int stu_linear_split(const void* x, long long x_row_stride, const void* W, long long w_row_stride,
+                                long long w_k_stride, const void* W2, const void* resid, long long resid_row_stride,
+                                void* y, long long y_row_stride, int M, int N, int K, int epilogue, int hist_T,
+                                int hist_t0, int hist_Lh, const void* norm_w, float eps, int dtype, int backend,
+                                float* workspace, long long workspace_elems, void* stream) {
   if (!x || !W || !y) return STU_ERR_NULL;
   if (M < 0 || N <= 0 || K <= 0) return STU_ERR_SHAPE;
   if (M == 0) return STU_OK;
@@ -107,11 +107,20 @@ extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, 
       return skinny_dispatch(x, x_row_stride, W, w_row_stride, W2, M, N, K, epilogue, ep, nullptr, eps, dtype, pdl, st);
     case BACKEND_TCGEN05:
       if (!tc_ok) return STU_ERR_UNSUPPORTED;
-      return gemm_tc_dispatch(x, x_row_stride, W, w_row_stride, W2, M, N, K, epilogue, causal, ep, st);
+      return gemm_tc_dispatch(x, x_row_stride, W, w_row_stride, W2, M, N, K, epilogue, causal, ep, st, workspace, workspace_elems);
     case BACKEND_SIMT:
       return gemm_simt_dispatch(x, x_row_stride, W, w_row_stride, w_k_stride, W2, M, N, K, epilogue, causal, ep, dtype, st);
   }
   return STU_ERR_UNSUPPORTED;
+}
+
+extern "C" int stu_linear(const void* x, long long x_row_stride, const void* W, long long w_row_stride,
+                          long long w_k_stride, const void* W2, const void* resid, long long resid_row_stride,
+                          void* y, long long y_row_stride, int M, int N, int K, int epilogue, int hist_T,
+                          int hist_t0, int hist_Lh, const void* norm_w, float eps, int dtype, int backend,
+                          void* stream) {
+  return stu_linear_split(x, x_row_stride, W, w_row_stride, w_k_stride, W2, resid, resid_row_stride, y, y_row_stride, M, N, K, epilogue, hist_T,
+                          hist_t0, hist_Lh, norm_w, eps, dtype, backend, nullptr, 0, stream);
 }
 
 // y = x[M,K] @ W[N,K]^T for M <= 64 rows (bf16) with the exchange fused in: the rows are stored into every rank's inbox

@@ -94,7 +94,8 @@ int gemm_f32_umma_dispatch(const void* A, long long lda, const void* B, long lon
 bool gemm_f32_umma_takes(const void* A, long long lda, const void* B, long long ldb, long long skb, const void* B2, int M, int N, int K,
                          int epi, int dtype);
 int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N,
-                     int K, int epi, int causal, const EpiArgsAny& ep, cudaStream_t st);
+                     int K, int epi, int causal, const EpiArgsAny& ep, cudaStream_t st, float* workspace = nullptr,
+                     long long workspace_elems = 0);
 bool gemm_tc_supported(const void* A, long long lda, const void* B, long long ldb, long long skb, const void* B2,
                        int M, int N, int K, int epi, const EpiArgsAny& ep, int dtype);
 int skinny_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N, int K,

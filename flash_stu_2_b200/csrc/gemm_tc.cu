@@ -10,7 +10,7 @@
 // scatter into the projected history).  The kernel is persistent (one pair per two SMs walks the tile list) and the accumulator is
 // double-buffered in TMEM, so one tile's epilogue overlaps the next tile's main loop.  Every load is a plain load of this GPU's
 // own memory into the loading CTA's shared memory.  Where tiles of 256 rows would fill their last wave badly, CTAs alone on tiles of
-// 128 x 256 take their place (tile_form).
+// 128 x 256 take their place (tile_form); where long K keeps few of them busy, it is cut (split_plan).
 // One CTA per 128 x 256 or 128 x 128 tile, as it was before, and now (us, all back to back): 65536 x 1536 x 6144 938 -> 880,
 // gate/up 65536 x 6144 x 1536 1998 -> 1874, 65536 x 4608 x 1536 771 -> 656, 7996 x 3072 x 1024 47.3 -> 43.0, 1668 x 768 x 3072
 // 18.1 -> 12.0, 333 x 1536 x 6144 32.0 -> 18.3; smallest 4.3 -> 4.7 (256 x 256 x 64), before the launch became programmatic: barriers and tensor memory
@@ -270,12 +270,19 @@ __host__ __device__ constexpr int stage_blocks(int mma_n) { return mma_n > 128 ?
 // tile while the epilogue warps drain the previous one.
 // CTAS = 1: the same with a CTA in the place of a pair, tiles of 128 rows (cta_group::1, all rows of B in its shared memory), for
 // products whose tiles of 256 rows would fill their last wave badly (see tile_form).
-template <int EPI, int STAGES, int TN, int CTAS>
+// SPLIT: K of the tiles behind the first `whole` is cut into `parts` (split_plan); what a pair works on are then those tiles' parts, and their
+// sums go to `partials` in fp32: per part [CTA][32 rows][4 columns], every store of a warp 512 bytes in a row.  split_sum_kernel adds them up.
+struct SplitK {
+  int whole, parts;
+  float* partials;
+};
+constexpr int SPLIT_TILE = 256 * 256;   // values of a part
+template <int EPI, int STAGES, int TN, int CTAS, bool SPLIT>
 __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmY, int by_copy, int M, int N,
                    int K, int tiles_m, int tiles_n, int group_m, int causal, EpiArgs<bf16> ep, int* status,
-                   int drop_first_copy, unsigned long long wait_ns) {
+                   int drop_first_copy, unsigned long long wait_ns, SplitK split) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
   constexpr bool COPIES = (EPI == EPI_STORE || EPI == EPI_GELU_MUL || EPI == EPI_BLOCKCOL);   // outputs that nothing is added to
   constexpr int BN = TN;                       // output columns of a tile
@@ -300,8 +307,18 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = PAIR ? blockIdx.x & 1 : 0, pair = blockIdx.x / CTAS, pairs = gridDim.x / CTAS;
-  const int num_tiles = tiles_m * tiles_n;
+  const int num_tiles = SPLIT ? split.whole + (tiles_m * tiles_n - split.whole) * split.parts : tiles_m * tiles_n;
   int num_kb = (K + BK - 1) / BK;
+  // tile and k-blocks of a part.  All tiles' first parts come first: what works on them at a time shares its k-blocks in L2.
+  const int rest = SPLIT ? tiles_m * tiles_n - split.whole : 1;
+  const auto whole_tile = [&](int tile) { return SPLIT && tile >= split.whole ? split.whole + (tile - split.whole) % rest : tile; };
+  const auto k_range = [&](int tile, int& kb0, int& kb_end) {
+    if (SPLIT && tile >= split.whole) {
+      const int part = (tile - split.whole) / rest;
+      kb0 = (int)((long long)num_kb * part / split.parts);
+      kb_end = (int)((long long)num_kb * (part + 1) / split.parts);
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -347,10 +364,11 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
     bool ok = true, ready = false;
     for (int tile = pair; ok && tile < num_tiles; tile += pairs) {
       int tm, tn;
-      tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
+      tile_coords(whole_tile(tile), tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = (CTAS * tm + rank) * BM, n0 = tn * BN + (DUAL ? 0 : rank * (BN / 2));
-      const int kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, min((tm + 1) * CTAS * BM, M) - 1, K);
-      for (int kb = 0; kb < kb_end; kb += KBS, g++) {
+      int kb0 = 0, kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, min((tm + 1) * CTAS * BM, M) - 1, K);
+      k_range(tile, kb0, kb_end);
+      for (int kb = kb0; kb < kb_end; kb += KBS, g++) {
         if (!ready) ok = warp_wait(&empty_bar[s], ph, abort_flag, wait_ns);
         if (!ok) break;
         const int s1 = s + 1 == STAGES ? 0 : s + 1;
@@ -399,11 +417,12 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
         const int buf = it & 1;
         const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
         int tm, tn;
-        tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
-        const int kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, min((tm + 1) * CTAS * BM, M) - 1, K);
+        tile_coords(whole_tile(tile), tiles_m, tiles_n, group_m, tm, tn);
+        int kb0 = 0, kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, min((tm + 1) * CTAS * BM, M) - 1, K);
+        k_range(tile, kb0, kb_end);
         ok = warp_wait(&tmem_empty[buf], (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
         if (!ok) break;
-        for (int kb = 0; kb < kb_end; kb += KBS, g++) {
+        for (int kb = kb0; kb < kb_end; kb += KBS, g++) {
           if (!ready) ok = warp_wait(&full_bar[s], ph, abort_flag, wait_ns);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -421,8 +440,8 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; kk++) {
                   const uint64_t dak = da + j * (KB_BYTES >> 4) + 2 * kk, dbk = db + j * (KB_BYTES >> 4) + 2 * kk;
-                  if constexpr (PAIR) umma_pair<MMA_N>(acc_addr, dak, dbk, (kb | j | kk) ? 1u : 0u);
-                  else umma<MMA_N>(acc_addr, dak, dbk, (kb | j | kk) ? 1u : 0u);
+                  if constexpr (PAIR) umma_pair<MMA_N>(acc_addr, dak, dbk, ((kb - kb0) | j | kk) ? 1u : 0u);
+                  else umma<MMA_N>(acc_addr, dak, dbk, ((kb - kb0) | j | kk) ? 1u : 0u);
                 }
               }
             // arrives when the MMAs above have finished reading this stage
@@ -469,7 +488,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
     int it = 0;
     for (int tile = pair; tile < num_tiles; tile += pairs, it++) {
       int tm, tn;
-      tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn);
+      tile_coords(whole_tile(tile), tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = (CTAS * tm + rank) * BM, n0 = tn * BN;
       const int first = m0 + quarter * 32, rows = min(32, M - first);   // this warp's rows
       const int buf = it & 1;
@@ -478,6 +497,25 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (SPLIT && tile >= split.whole) {
+        float4* part = reinterpret_cast<float4*>(split.partials + (size_t)(tile - split.whole) * SPLIT_TILE) + (rank * 4 + quarter) * (BN / 4) * 32 + lane;
+#pragma unroll 1
+        for (int nb = n0 + 64 * half; nb < (rows > 0 ? min(n0 + BN, N) : 0); nb += 128) {
+          const uint32_t taddr = acc_addr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(nb - n0);
+          uint32_t r[2][32];
+          tmem_ld32(taddr, r[0]);
+          tmem_ld32(taddr + 32, r[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 16; j++)
+            part[((nb - n0) / 4 + j) * 32] = make_float4(__uint_as_float(r[j >> 3][4 * (j & 7)]), __uint_as_float(r[j >> 3][4 * (j & 7) + 1]),
+                                                         __uint_as_float(r[j >> 3][4 * (j & 7) + 2]), __uint_as_float(r[j >> 3][4 * (j & 7) + 3]));
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(hand_back + buf * (uint32_t)sizeof(uint64_t));
+        continue;
+      }
       if (COPIES && by_copy) {
 #pragma unroll 1
         for (int nb = n0 + 64 * half; nb < min(n0 + BN, N); nb += 128) {
@@ -704,6 +742,49 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
   }
 }
 
+// The split tiles' sums over their parts, first to last, and the epilogue.  A CTA: 8 rows x 128 columns of a tile, a thread 4 columns (8 rows x 16 bytes of a
+// part are 128 bytes in a row, 4 threads' outputs 32 bytes of theirs).
+template <int EPI>
+__global__ void __launch_bounds__(256) split_sum_kernel(const float* __restrict__ partials, int whole, int parts, int M, int N, int tiles_m, int tiles_n,
+                                                        int group_m, EpiArgs<bf16> ep) {
+  pdl_wait();
+  pdl_trigger();
+  int tm, tn;
+  tile_coords(whole + blockIdx.y, tiles_m, tiles_n, group_m, tm, tn);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = (blockIdx.x >> 1) * 8 + (lane & 7), c4 = (blockIdx.x & 1) * 32 + warp * 4 + (lane >> 3);
+  const int m = tm * 256 + row, n = tn * 256 + c4 * 4;
+  if (m >= M || n >= N) return;
+  const float4* p = reinterpret_cast<const float4*>(partials + (size_t)blockIdx.y * SPLIT_TILE) + ((row >> 5) * 64 + c4) * 32 + (row & 31);
+  float4 acc = __ldcs(p);
+#pragma unroll 8
+  for (int i = 1; i < parts; i++) {
+    const float4 v = __ldcs(p + (size_t)i * gridDim.y * (SPLIT_TILE / 4));
+    acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
+  }
+  const float o[4] = {acc.x, acc.y, acc.z, acc.w};
+  const bool vec = n + 4 <= N && ep.ldy % 4 == 0 && (reinterpret_cast<uintptr_t>(ep.y) & 7) == 0;
+  bf16* y = ep.y + (size_t)m * ep.ldy + n;
+  if (EPI == EPI_RESID) {   // rows of resid and y on the 16-byte grid (gemm_tc_supported)
+    const bf16* rr = ep.resid + (size_t)m * ep.ldr + n;
+    for (int j = 0; j < min(4, N - n); j++)
+      if (!vec) y[j] = __float2bfloat16_rn(__bfloat162float(rr[j]) + round_to<bf16>(o[j]));
+    if (vec) {
+      const uint2 rv = *reinterpret_cast<const uint2*>(rr);
+      const float r[4] = {__uint_as_float(rv.x << 16), __uint_as_float(rv.x & 0xffff0000u), __uint_as_float(rv.y << 16),
+                          __uint_as_float(rv.y & 0xffff0000u)};
+      const __nv_bfloat162 a = __floats2bfloat162_rn(r[0] + round_to<bf16>(o[0]), r[1] + round_to<bf16>(o[1]));
+      const __nv_bfloat162 b = __floats2bfloat162_rn(r[2] + round_to<bf16>(o[2]), r[3] + round_to<bf16>(o[3]));
+      *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+  } else if (vec) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(o[0], o[1]), b = __floats2bfloat162_rn(o[2], o[3]);
+    *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  } else {
+    for (int j = 0; j < min(4, N - n); j++) y[j] = __float2bfloat16_rn(o[j]);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------- host
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -816,7 +897,7 @@ int device_pairs() {
   static std::atomic<int> found[STU_MAX_DEVICES] = {};
   std::atomic<int>& n = found[current_device()];
   if (n.load(std::memory_order_relaxed) == 0) {
-    const void* kernel = (const void*)gemm_tc_kernel<EPI_STORE, 6, 256, 2>;
+    const void* kernel = (const void*)gemm_tc_kernel<EPI_STORE, 6, 256, 2, false>;
     constexpr size_t smem = tc_smem<EPI_STORE, 6, 256, 2>();
     static SmemLimit limit;
     cudaLaunchConfig_t cfg = {};
@@ -839,9 +920,9 @@ int device_pairs() {
   return n.load(std::memory_order_relaxed);
 }
 
-template <int EPI, int STAGES, int TN, int CTAS = 2>
+template <int EPI, int STAGES, int TN, int CTAS = 2, bool SPLIT = false>
 int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2, int M, int N, int K, int m_fast,
-              int causal, const EpiArgs<bf16>& ep, int* status, cudaStream_t st) {
+              int causal, const EpiArgs<bf16>& ep, int* status, cudaStream_t st, SplitK split = {}) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL);
   constexpr bool COPIES = (EPI == EPI_STORE || EPI == EPI_GELU_MUL || EPI == EPI_BLOCKCOL);
   constexpr size_t smem = tc_smem<EPI, STAGES, TN, CTAS>();
@@ -852,23 +933,28 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   int by_copy = 0;
   if (COPIES && !ep.peer && ep.ldy % 8 == 0 && N % 8 == 0 && aligned16(ep.y) && (EPI != EPI_BLOCKCOL || (ep.Tseq % 64 == 0 && N % ep.Tseq == 0)))
     by_copy = make_output_map(&y, ep, EPI == EPI_BLOCKCOL, M, N) == STU_OK;
-  auto k = gemm_tc_kernel<EPI, STAGES, TN, CTAS>;
+  auto k = gemm_tc_kernel<EPI, STAGES, TN, CTAS, SPLIT>;
   static SmemLimit limit;
   cudaError_t e = allow_smem((const void*)k, smem, limit);
   if (e != cudaSuccess) return (int)e;
   const int tiles_m = (M + CTAS * BM - 1) / (CTAS * BM), tiles_n = (N + TN - 1) / TN;
-  const int tiles = tiles_m * tiles_n, most = CTAS == 2 ? device_pairs() : device_sm_count();
+  const int tiles = SPLIT ? split.whole + (tiles_m * tiles_n - split.whole) * split.parts : tiles_m * tiles_n, most = CTAS == 2 ? device_pairs() : device_sm_count();
   const int grid = CTAS * (tiles < most ? tiles : most);  // one persistent CTA per SM
   const int drop = g_drop_first_copy;
   g_drop_first_copy = 0;   // the injected fault applies to one launch
   const int group_m = m_fast ? tiles_m : gemm_group_m(tiles_n, N, K, DUAL);
   e = launch_maybe_overlapped(k, dim3(grid), dim3(64 + 32 * EPI_WARPS), smem, st, true, a, b, b2, y, by_copy, M, N, K, tiles_m, tiles_n, group_m,
-                              causal, ep, status, drop, g_wait_ns);
+                              causal, ep, status, drop, g_wait_ns, split);
   if (e != cudaSuccess) return (int)e;
   STU_CHECK_LAUNCH();
+  if constexpr (SPLIT) {
+    e = launch_maybe_overlapped(split_sum_kernel<EPI>, dim3(64, tiles_m * tiles_n - split.whole), dim3(256), 0, st, true, (const float*)split.partials,
+                                split.whole, split.parts, M, N, tiles_m, tiles_n, group_m, ep);
+    if (e != cudaSuccess) return (int)e;
+    STU_CHECK_LAUNCH();
+  }
   return STU_OK;
 }
-
 
 // ------------------------------------------------------------------------------------------------
 // Token-step linear layers for 9..64 activation rows on the tensor cores, operands swapped: the WEIGHTS are the
@@ -1261,8 +1347,38 @@ extern "C" long long stu_linear_tile_cost(int M, int N) {
   return cost;
 }
 
+// Plain and residual products that leave pairs idle for long: the tiles that do not fill a wave (all of them where there are fewer than pairs) are
+// 256 x 256 whatever the rows, their K is cut into parts of the same length, and split_sum_kernel adds the parts up.  A pair working alone on
+// K = 49152 takes 200 us, so what counts is long K: us, as tile_form has it and split, 24000 x 1024 x 49152 (6 of 376 tiles in the last wave) 1784 -> 1637,
+// 8192 x 768 x 24576 349 -> 312, 1180 x 1024 x 24576 80.9 -> 54.4, 251 x 2048 x 98304 327 -> 96, 74 x 512 x 24576 61.1 -> 15.7, 16384 x 1536 x 6144 207 -> 187,
+// 4096 x 1536 x 6144 64.7 -> 56.3, 333 x 1536 x 6144 30.5 -> 26.3 (weights from HBM).  The parts' way through L2 and the second launch cost what short K
+// gains: 834 x 768 x 3072 in 4 parts 20.5 -> 21.5, 1337 x 1024 x 2048 in 3 12.6 -> 17.6, 8192 x 1536 x 6144 in 3 106 -> 107.  The line, in us: a k-block
+// of 64 takes 0.31 in a wide tile (0.18 in a narrow one; 0.27 and 0.155 where few SMs work), a wave of parts 1 more, each part 0.05 (256 KB
+// written and read), the second launch 4; 105 products of 65 to 24000 rows, K = 512 to 98304: 0.97 (noise, not split) to 4.0 times as fast.
+static SplitK split_plan(long long M, long long N, long long K) {
+  SplitK s = {0, 1, nullptr};
+  if (M <= 64 || K < 1024) return s;   // token steps' kernels, or never worth it
+  const long long tiles = (M + 255) / 256 * ((N + 255) / 256), pairs = device_pairs(), kb = (K + BK - 1) / BK, rest = tiles % pairs;
+  if (rest == 0) return s;
+  long long cost = 0;
+  tile_form(M, N, false, true, &cost);
+  double best = 0.95 * 0.0018 * cost * kb;
+  for (long long parts = 2; parts <= std::min(kb, 32ll) && rest * parts <= 5 * pairs; parts++) {   // up to 97 MB of parts
+    const double us = tiles / pairs * kb * 0.31 + (rest * parts + pairs - 1) / pairs * ((kb + parts - 1) / parts * 0.31 + 1) + 4 + rest * parts * 0.05;
+    if (us < best) best = us, s.parts = (int)parts;
+  }
+  s.whole = (int)(tiles - rest);
+  return s;
+}
+// fp32 values that stu_linear_split wants for its parts; 0: nothing is split.
+extern "C" long long stu_linear_workspace_elems(int M, int N, int K, int epilogue, int dtype) {
+  if (dtype != STU_BF16 || (epilogue & ~(STU_FLAG_OVERLAP | STU_FLAG_EARLY_TRIGGER)) > EPI_RESID || M <= 0 || N <= 0 || K <= 0) return 0;
+  const SplitK s = split_plan(M, N, K);
+  return s.parts > 1 ? ((M + 255ll) / 256 * ((N + 255ll) / 256) - s.whole) * s.parts * SPLIT_TILE : 0;
+}
+
 int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N,
-                     int K, int epi, int causal, const EpiArgsAny& epa, cudaStream_t st) {
+                     int K, int epi, int causal, const EpiArgsAny& epa, cudaStream_t st, float* workspace, long long workspace_elems) {
   CUtensorMap ma, mb, mb2;
   EpiArgs<bf16> ep = epa.as<bf16>();
   int rc;
@@ -1275,6 +1391,17 @@ int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb,
     ep.ldy = N;  // channel count
     if (wide) return launch_tc<EPI_HIST_T, 6, 256>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
     return launch_tc<EPI_HIST_T, 4, 128>(ma, mb, mb, N, M, K, /*m_fast=*/1, 0, ep, device_status_word(), st);
+  }
+  if (workspace && !causal && !ep.kpos && !ep.peer && (epi == EPI_STORE || epi == EPI_RESID)) {
+    const long long want = stu_linear_workspace_elems(M, N, K, epi, STU_BF16);
+    if (want > 0 && want <= workspace_elems) {
+      SplitK split = split_plan(M, N, K);
+      split.partials = workspace;
+      if ((rc = make_map(&ma, A, M, K, lda)) != STU_OK) return rc;
+      if ((rc = make_map(&mb, B, N, K, ldb, 128)) != STU_OK) return rc;
+      if (epi == EPI_STORE) return launch_tc<EPI_STORE, 6, 256, 2, true>(ma, mb, mb, M, N, K, 0, 0, ep, device_status_word(), st, split);
+      return launch_tc<EPI_RESID, 6, 256, 2, true>(ma, mb, mb, M, N, K, 0, 0, ep, device_status_word(), st, split);
+    }
   }
   const bool dual = epi == EPI_GELU_MUL;
   const int form = tile_form(M, dual ? 2ll * N : N, dual, epi != EPI_BLOCKCOL);

@@ -166,9 +166,14 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     void *px = data_of(x), *pW = data_of(W), *pW2 = data_of(W2), *pr = data_of(resid), *py = data_of(out), *pn = data_of(norm_w);
     const long long lda = x->stride(0), r_rs = resid ? resid->stride(0) : 0;
     void* stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
+    // backends that may come to the tcgen05 GEMM: 0 and 2
+    const long long parts = backend == 0 || backend == 2 ? stu_linear_workspace_elems((int)M, (int)N, (int)K, epi, code) : 0;
+    at::Tensor workspace;
+    if (parts > 0) workspace = at::empty({parts}, x->options().dtype(at::kFloat));
+    float* pw = parts > 0 ? workspace.data_ptr<float>() : nullptr;
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = stu_linear(px, lda, pW, w_rs, w_ks, pW2, pr, r_rs, py, y_rs, (int)M, (int)N, (int)K, epi, hT, ht0, hLh, pn, eps, code, backend, stream);
+    rc = stu_linear_split(px, lda, pW, w_rs, w_ks, pW2, pr, r_rs, py, y_rs, (int)M, (int)N, (int)K, epi, hT, ht0, hLh, pn, eps, code, backend, pw, parts, stream);
     Py_END_ALLOW_THREADS
     if (raised(rc, "stu_linear")) return nullptr;
     if (rc != 0) Py_RETURN_NONE;
@@ -298,6 +303,10 @@ PyObject* layer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int64_t yLh = ((t0 + T + 1) / 2 + 7) / 8 * 8;
     const int M = (int)(B * T), t_end = (int)(t0 + T);
     at::Tensor xn = at::empty({M, d}, x.options()), yT = at::empty({B, d, 2, yLh}, x.options()), h = at::empty({M, I}, x.options());
+    const long long parts = stu_linear_workspace_elems(M, (int)d, (int)I, 1, code);
+    at::Tensor workspace;
+    if (parts > 0) workspace = at::empty({parts}, x.options().dtype(at::kFloat));
+    float* pw = parts > 0 ? workspace.data_ptr<float>() : nullptr;
     void* p[10];
     for (int i = 0; i < 10; i++) p[i] = data_of(t[i]);
     void *pn = xn.data_ptr(), *py = yT.data_ptr(), *ph = h.data_ptr(), *stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
@@ -316,7 +325,7 @@ PyObject* layer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (rc == 0)
       rc = stu_linear(pn, d, p[7], d, 1, p[8], nullptr, 0, ph, I, M, (int)I, (int)d, 2, 0, 0, 0, nullptr, 0.f, code, 0, stream);
     if (rc == 0)
-      rc = stu_linear(ph, I, p[9], I, 1, nullptr, p[0], d, p[0], d, M, (int)d, (int)I, 1, 0, 0, 0, nullptr, 0.f, code, 0, stream);
+      rc = stu_linear_split(ph, I, p[9], I, 1, nullptr, p[0], d, p[0], d, M, (int)d, (int)I, 1, 0, 0, 0, nullptr, 0.f, code, 0, pw, parts, stream);
     Py_END_ALLOW_THREADS
     if (raised(rc, "layer_prefill")) return nullptr;
     if (rc == 0) done = 3;

@@ -88,6 +88,15 @@ int stu_linear_can_fuse_norm(int M, int N, int K, int epilogue, int dtype);
 /* Time of the tcgen05 GEMM's tiles for M x N plain outputs, in hundredths of a wave of its smallest ones (per k-block): for callers that
  * choose how many rows a product has.  No counterpart in the reference. */
 long long stu_linear_tile_cost(int M, int N);
+/* stu_linear with a workspace (device, 16-byte aligned): epilogues 0 and 1 of the tcgen05 GEMM whose last wave of tiles would leave SMs idle
+ * for long cut K of those tiles, keep the parts' sums there in fp32 and add them up in a second launch.  ..._workspace_elems: fp32 values that
+ * this takes for a product, 0 where it does not pay (any dtype or epilogue may be asked for).  With less than that, or NULL, the
+ * call is stu_linear.  The contents need not be set and are not kept.  No counterpart in the reference. */
+long long stu_linear_workspace_elems(int M, int N, int K, int epilogue, int dtype);
+int stu_linear_split(const void* x, long long x_row_stride, const void* W, long long w_row_stride, long long w_k_stride,
+                     const void* W2, const void* resid, long long resid_row_stride, void* y, long long y_row_stride,
+                     int M, int N, int K, int epilogue, int hist_T, int hist_t0, int hist_Lh, const void* norm_w,
+                     float eps, int dtype, int backend, float* workspace, long long workspace_elems, void* stream);
 
 /* taps[c][j] = fp[2j][c] for fp = phi @ M_filters ([L,d], model dtype): the even taps that survive when the
  * plus and minus branches of flash_stu/utils/stu_utils.py:223-227 are added (flash_stu/modules/stu.py:88,120). */

@@ -494,6 +494,44 @@ def test_fp32_linear_on_tensor_cores(shape, epi):
     assert err[0] <= max(err[1], 2.0 ** -24), err
 
 
+# (rows, outputs, K, distance of the outputs' rows): one tile in parts of unequal length, edges of tiles, odd row strides, whole tiles ahead of the split ones
+@pytest.mark.parametrize("shape", [(65, 64, 24576, 64), (257, 513, 12296, 513), (333, 1536, 6144, 1540), (70, 1030, 49152, 1033), (140, 1001, 8200, 1002),
+                                   (5193, 1000, 4096, 1000), (19851, 512, 3072, 512)])
+@pytest.mark.parametrize("epi", [0, 1])
+def test_linear_of_long_weights_in_parts(shape, epi):
+    """bf16 products whose K is cut over the SMs.  Bars: a plain result is the float64 one rounded once, but for fp32 sums of K products; a
+    residual is added to the rounded product; without the workspace the call is the product in one piece."""
+    from flash_stu_2_b200 import _lib, ops
+    M, N, K, ld = shape
+    if epi and (N % 8 or ld % 8):
+        ld = N = N // 8 * 8      # residual rows lie on the 16-byte grid
+    assert _lib.load().stu_linear_workspace_elems(M, N, K, epi, 1) >= 2 * 65536
+    torch.manual_seed(8)
+    x = torch.randn(M, K, device=dev()).bfloat16()
+    W = (torch.randn(N, K, device=dev()) / math.sqrt(K)).bfloat16()
+    r = torch.randn(M, ld, device=dev()).bfloat16()[:, :N]
+    buf = torch.full((M + 1, ld), 7.0, device=dev(), dtype=torch.bfloat16)
+    out = buf[:M, :N]
+    ops.linear(x, W, out=out, epilogue=epi, resid=r if epi else None)
+    ops.check_status()
+    assert bool((buf[M] == 7).all()) and bool((buf[:, N:] == 7).all())
+    full = torch.cat([x[i:i + 2048].double() @ W.double().t() for i in range(0, M, 2048)])
+    # sums of K products of order 1/sqrt(K): 2^-24 * sqrt(K) * a few, well below 1e-4 for every K here
+    lo, hi = (full - 1e-4).bfloat16(), (full + 1e-4).bfloat16()
+    if epi:
+        lo, hi = (r.float() + lo.float()).bfloat16(), (r.float() + hi.float()).bfloat16()
+    assert bool(((out >= lo) & (out <= hi)).all())
+    if epi == 0:
+        short = torch.empty(M, N, device=dev(), dtype=torch.bfloat16)
+        work = torch.full((64,), float("nan"), device=dev())
+        rc = _lib.load().stu_linear_split(x.data_ptr(), K, W.data_ptr(), K, 1, None, None, 0, short.data_ptr(), N, M, N, K, 0, 0, 0, 0, None, 0.0, 1, 0,
+                                          work.data_ptr(), 64, torch.cuda.current_stream().cuda_stream)
+        whole = torch.empty_like(short)
+        rc2 = _lib.load().stu_linear(x.data_ptr(), K, W.data_ptr(), K, 1, None, None, 0, whole.data_ptr(), N, M, N, K, 0, 0, 0, 0, None, 0.0, 1, 0,
+                                     torch.cuda.current_stream().cuda_stream)
+        assert rc == rc2 == 0 and torch.equal(short, whole) and bool(work.isnan().all())
+
+
 @pytest.mark.parametrize("shape", [(8, 1024, 49152), (1, 640, 14720), (5, 768, 12296), (7, 1200, 4104), (8, 2049, 4096), (3, 4735, 8192)])
 @pytest.mark.parametrize("epi", [0, 1])
 @pytest.mark.parametrize("early", [False, True])
