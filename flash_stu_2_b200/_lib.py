@@ -96,6 +96,7 @@ _SIGNATURES = {
     "stu_full_conv_tc5_scratch_elems": ([c_int, c_int], c_longlong),
     "stu_full_conv_tc5": ([_P, c_int, _P, c_int, c_int, _P, _P, _LL, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P], c_int),
     "stu_full_decode_step": ([_P, _LL, _P, c_float, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P], c_int),
+    "stu_full_decode_step_tc5": ([_P, _LL, _P, c_float, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P], c_int),
     "stu_full_decode_prepare": ([_P, _LL, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P], c_int),
     "stu_full_decode_combine": ([_P, _LL, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_lds_final_state": ([_P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),

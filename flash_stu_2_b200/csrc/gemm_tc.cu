@@ -1292,6 +1292,11 @@ extern "C" int stu_test_inject_wait_expiry(int wait_ms) {
   return STU_OK;
 }
 
+// make_map for the other tensor-core kernels of K-major bf16 operands.
+int operand_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows) {
+  return make_map(map, base, rows, cols, ld, box_rows);
+}
+
 extern "C" int stu_set_status_word(int* device_status) {
   g_status_words[current_device()] = device_status;
   return STU_OK;

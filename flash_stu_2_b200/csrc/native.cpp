@@ -359,6 +359,7 @@ PyMethodDef methods[] = {
     ENTRY(stu_full_conv_f32_tc5),
     ENTRY(stu_full_decode_prepare),
     ENTRY(stu_full_decode_step),
+    ENTRY(stu_full_decode_step_tc5),
     ENTRY(stu_lds_chunk_scan),
     ENTRY(stu_lds_decode_step),
     ENTRY(stu_lds_final_state),

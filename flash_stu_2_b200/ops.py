@@ -673,16 +673,30 @@ def full_decode_step_pays(batch: int, d: int, K: int, t: int) -> bool:
     return batch * d * tiles <= 49152 and (batch * tiles) ** 2 * d * t <= 3.8e9
 
 
-def full_decode_step(x2d, norm_w, eps: float, hist, taps8, pos, U, limit: int, both_signs: bool):
+def full_decode_step_tc5_pays(batch: int, d: int, K: int, t: int) -> bool:
+    """Whether the step at position t takes less time with its sums on tcgen05 (64 channels per CTA).  With more than a CTA per SM always; with
+    half of the SMs busy or more from some position on, which depends on how many tiles of 8 filters the other kernel loads the
+    taps of.  Layer step of 24 filters, us, mma.sync and tcgen05: 8 x 1024 at 1000 44.5 and 45.5, at 3000 52.9 and 50.4, at 6000 69.6 and
+    59.3, 16 x 1024 at 1000 65.0 and 54.0.  The kernel alone, from L2: 8 x 1024, 8 filters, at 4000 16.5 and 15.0; 16 filters, at 2000 12.1 and
+    11.0; 32 filters, at 600 13.9 and 9.3; 16 x 1024, 8 filters, at 300 10.7 and 8.6.  4 x 1024 at 4000, 24 filters: 14.2 and 15.5."""
+    if d % 64 or K > 32:
+        return False
+    ctas = batch * (d // 64)
+    return ctas > 148 or (ctas >= 74 and t >= (3000, 3000, 1500, 500)[(K + 7) // 8 - 1])
+
+
+def full_decode_step(x2d, norm_w, eps: float, hist, taps8, pos, U, limit: int, both_signs: bool, t: int = 0):
     """U+- [B, (1 or 2)*K*d] of the position after the cached ones: x2d [B,d] (normalised first with norm_w) is appended to
-    hist [B,d,2,Lh], taps8 [8, 2K, Lh+8] holds the even and the odd taps of the filters; pos moves on."""
+    hist [B,d,2,Lh], taps8 [8, 2K, Lh+8] holds the even and the odd taps of the filters; pos moves on.  t: about where pos is (it tells
+    which kernel is launched)."""
     _cuda(x2d, norm_w, hist, taps8, pos, U)
     B, d, _, Lh = hist.shape
     K = taps8.shape[1] // 2
     assert taps8.shape == (8, 2 * K, Lh + 8) and x2d.stride(1) == 1 and U.is_contiguous() and U.numel() == B * (1 + both_signs) * K * d
-    rc = _lib.native().stu_full_decode_step(x2d.data_ptr(), x2d.stride(0), norm_w.data_ptr() if norm_w is not None else None, eps,
-                                            hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), U.data_ptr(), B, d, K, Lh, limit,
-                                            int(both_signs), status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
+    step = _lib.native().stu_full_decode_step_tc5 if full_decode_step_tc5_pays(B, d, K, t) else _lib.native().stu_full_decode_step
+    rc = step(x2d.data_ptr(), x2d.stride(0), norm_w.data_ptr() if norm_w is not None else None, eps,
+              hist.data_ptr(), taps8.data_ptr(), pos.data_ptr(), U.data_ptr(), B, d, K, Lh, limit,
+              int(both_signs), status_word(x2d.device).data_ptr(), _dt(x2d), _stream())
     _lib.check(rc, "stu_full_decode_step")
     _count()
 

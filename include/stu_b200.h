@@ -262,6 +262,10 @@ int stu_full_conv_f32_tc5(const void* hist, int Lh, const void* phi, int L, int 
 int stu_full_decode_step(const void* x, long long x_rstride, const void* norm_w, float eps, void* hist, const void* taps8,
                          int* pos, void* U, int B, int d, int K, int Lh, int limit, int both_signs, int* status, int dtype,
                          void* stream);
+/* The same with the sums on tcgen05 (another order of fp32 sums), d a multiple of 64; status 9 where a bounded wait ran out. */
+int stu_full_decode_step_tc5(const void* x, long long x_rstride, const void* norm_w, float eps, void* hist, const void* taps8,
+                             int* pos, void* U, int B, int d, int K, int Lh, int limit, int both_signs, int* status, int dtype,
+                             void* stream);
 
 /* One cached decode step of the full variant, around one GEMM G = hist_rows @ PhiT^T (stu_linear, M = B*d*2,
  * N = 2K, K = Lh): prepare appends x_t at time pos[0] and rebuilds PhiT [2K][Lh] (time-reversed even / odd

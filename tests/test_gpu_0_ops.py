@@ -1580,6 +1580,41 @@ def test_full_variant_step_kernel(B, d, K, L, signs):
     assert int(pos[0, 0]) == L
 
 
+@pytest.mark.parametrize("B,d,K,L,signs", [(1, 64, 5, 64, 2), (3, 128, 24, 260, 2), (2, 192, 32, 96, 1), (1, 128, 9, 1100, 2), (3, 3200, 8, 40, 2)])
+def test_full_variant_step_kernel_on_tensor_cores(monkeypatch, B, d, K, L, signs):
+    """The same on tcgen05: filters that fill no 8, positions around whole stages of 128 and past the ring's depth, both depths of the ring."""
+    from flash_stu_2_b200 import ops
+    monkeypatch.setattr(ops, "full_decode_step_tc5_pays", lambda *a: True)
+    torch.manual_seed(17)
+    Lh = ((L + 1) // 2 + 7) // 8 * 8
+    x, phi = (3 * torch.randn(B, L, d)).bfloat16(), (torch.randn(L, K) / 4).bfloat16()
+    w = (1 + 0.1 * torch.randn(d)).bfloat16()
+    xn = O.rmsnorm(x, w)
+    f = phi.to(dev())
+    taps8 = ops.taps_rev8(torch.cat([ops.taps_even(f, Lh), ops.taps_even(f[1:], Lh)]))
+    for t in sorted({t for t in (0, 1, 2, 15, 16, 33, 126, 127, 128, 129, 130, 255, 256, 257, 767, 768, 769, 900, L - 2, L - 1) if t < L}):
+        hist = torch.full((B, d, 2, Lh), float("nan"), dtype=torch.bfloat16, device=dev())
+        if t:
+            ops.to_history(xn[:, :t].to(dev()), hist, 0)
+        pos = torch.zeros(B, 2, dtype=torch.int32, device=dev())
+        pos[:, 0] = t
+        U = torch.full((B, signs * K * d), 7.0, dtype=torch.bfloat16, device=dev())
+        ops.full_decode_step(x[:, t].to(dev()), w.to(dev()), ops.RMS_EPS, hist, taps8, pos, U, L, signs == 2, t)
+        ops.check_status()
+        assert pos.tolist() == [[t + 1, 0]] * B
+        close(hist[:, :, t & 1, t >> 1], xn[:, t], 2 ** -7)
+        past = xn[:, :t + 1].double().flip(1)
+        past[:, 0] = hist[:, :, t & 1, t >> 1].cpu().double()   # (its rounding may differ by one unit)
+        taps = phi[:t + 1].double()
+        want = [torch.einsum("tk,bti->bki", taps * (s ** torch.arange(t + 1))[:, None], past).reshape(B, K * d) for s in (1.0, -1.0)]
+        close(U, torch.cat(want[:signs], 1), 4 * 2 ** -9)
+    pos[:, 0] = L
+    ops.full_decode_step(x[:, 0].to(dev()), w.to(dev()), ops.RMS_EPS, hist, taps8, pos, U, L, signs == 2, L)
+    with pytest.raises(RuntimeError, match="status 2"):
+        ops.check_status()
+    assert int(pos[0, 0]) == L
+
+
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,d", [(2368, 64), (2401, 264), (5000, 1024), (2500, 1536), (2400, 3072), (2999, 1000)])
 def test_rmsnorm_of_many_rows(dt, rows, d):
