@@ -335,7 +335,8 @@ class STU(nn.Module):
         t = host_pos(pos)
         if t + 1 > self.capacity:
             raise ValueError(f"sequence position {t + 1} exceeds the capacity {self.capacity} (seq_len={self.seq_len})")
-        if Lh == self.Lh and ops.full_decode_step_supported(x2d, hist, K) and ops.full_decode_step_pays(B, d, K, t):
+        if (Lh == self.Lh and ops.full_decode_step_supported(x2d, hist, K)
+                and (ops.full_decode_step_pays(B, d, K, t) or ops.full_decode_step_tc5_pays(B, d, K, t))):
             U = ops.empty((B, nsign * K * d), x2d.dtype, x2d.device)
             ops.full_decode_step(x2d, norm_w, eps, hist, self.step_taps(), pos, U, self.capacity, nsign == 2, t)
         else:   # fp32, more filters or rows, rows off the 16-byte grid: tap matrices, a GEMM over all history rows, their combination

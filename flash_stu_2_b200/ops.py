@@ -663,7 +663,7 @@ def full_decode_step_supported(x2d, hist, K: int) -> bool:
 
 
 def full_decode_step_pays(batch: int, d: int, K: int, t: int) -> bool:
-    """Whether the one-kernel step takes less time at position t than tap matrices, a GEMM over all history rows and a combine.  It
+    """Whether the one-kernel step on mma.sync takes less time at position t than tap matrices, a GEMM over all history rows and a combine.  It
     saves five launches and the tap matrices, but reads the taps in every CTA, on mma.sync: rows, filters and positions tell, and
     with more sequences the rest of the step gains less from the launches that are saved (the lines are fits).  Layer step of 24
     filters, us, replayed from a graph: 8 x 1024 at 1000 47.5 and 54.1, at 7000 72 and 76; 16 x 1024 at 1000 64 and 68, at 2000 77
@@ -674,7 +674,10 @@ def full_decode_step_pays(batch: int, d: int, K: int, t: int) -> bool:
 
 
 def full_decode_step_tc5_pays(batch: int, d: int, K: int, t: int) -> bool:
-    """Whether the step at position t takes less time with its sums on tcgen05 (64 channels per CTA).  With more than a CTA per SM always; with
+    """Whether the step at position t takes less time with its sums on tcgen05 (64 channels per CTA) than in either other form.  Against a
+    GEMM over all history rows it does wherever it does against mma.sync (layer step of 24 filters, us, GEMM and tcgen05: 12 x 1024
+    at 3000 77.1 and 61.8, 16 x 1024 at 7000 119.6 and 104.4, 24 x 1024 at 3000 105.2 and 97.6, 32 x 512 at 2800 70.2 and 54.4, 64 x 512 at
+    1000 70.1 and 55.1, 32 x 1536 at 60 104.0 and 92.8); against that, with more than a CTA per SM always, and with
     half of the SMs busy or more from some position on, which depends on how many tiles of 8 filters the other kernel loads the
     taps of.  Layer step of 24 filters, us, mma.sync and tcgen05: 8 x 1024 at 1000 44.5 and 45.5, at 3000 52.9 and 50.4, at 6000 69.6 and
     59.3, 16 x 1024 at 1000 65.0 and 54.0.  The kernel alone, from L2: 8 x 1024, 8 filters, at 4000 16.5 and 15.0; 16 filters, at 2000 12.1 and

@@ -226,3 +226,11 @@ def test_which_attention_kernel_takes_a_prefill(hd, B, H, T, window, t0, takes):
 def test_which_form_the_full_variants_step_takes(batch, d, K, t, pays):
     from flash_stu_2_b200 import ops
     assert ops.full_decode_step_pays(batch, d, K, t) is pays
+
+
+@pytest.mark.parametrize("batch,d,K,t,pays", [(8, 1024, 24, 1499, False), (8, 1024, 24, 1500, True), (8, 1024, 8, 2999, False), (8, 1024, 32, 500, True),
+                                             (5, 960, 24, 1500, True), (4, 1152, 24, 8000, False), (16, 1024, 24, 0, True), (16, 1024, 33, 4000, False),
+                                             (19, 512, 1, 0, True), (40, 520, 24, 8000, False)])
+def test_when_the_full_variants_step_goes_to_tcgen05(batch, d, K, t, pays):
+    from flash_stu_2_b200 import ops
+    assert ops.full_decode_step_tc5_pays(batch, d, K, t) is pays
