@@ -11,7 +11,8 @@
 // turn, their sums meet in shared memory.  As a kernel that rebuilt the K x Lh tap matrices, a GEMM against them (both
 // tap sets for both parities) and a kernel each to combine and to advance, behind the norm kernel, this was 5 launches: 8
 // sequences of 1024 channels near position 2800, the whole layer step, replayed from a graph, 63.6 us; this form 55.9 (layer
-// prefill and 64 steps 8.42 -> 7.94 ms).  ops.full_decode_step_pays says where that form stays the faster one.
+// prefill and 64 steps 8.42 -> 7.94 ms).  ops.full_decode_step_pays says where that form stays the faster one, ops.full_decode_step_tc5_pays
+// where the kernel of stu_full_step_umma.cu is.
 #include "common.cuh"
 
 int device_sm_count();   // gemm_tc.cu

@@ -507,8 +507,8 @@ def test_linear_of_long_weights_in_parts(shape, epi):
         ld = N = N // 8 * 8      # residual rows lie on the 16-byte grid
     assert _lib.load().stu_linear_workspace_elems(M, N, K, epi, 1) >= 2 * 65536
     torch.manual_seed(8)
-    x = torch.randn(M, K, device=dev()).bfloat16()
-    W = (torch.randn(N, K, device=dev()) / math.sqrt(K)).bfloat16()
+    x = torch.randn(M, K + 8, device=dev()).bfloat16()[:, :K]
+    W = (torch.randn(N, K + 16, device=dev()) / math.sqrt(K)).bfloat16()[:, :K]
     r = torch.randn(M, ld, device=dev()).bfloat16()[:, :N]
     buf = torch.full((M + 1, ld), 7.0, device=dev(), dtype=torch.bfloat16)
     out = buf[:M, :N]
@@ -524,10 +524,10 @@ def test_linear_of_long_weights_in_parts(shape, epi):
     if epi == 0:
         short = torch.empty(M, N, device=dev(), dtype=torch.bfloat16)
         work = torch.full((64,), float("nan"), device=dev())
-        rc = _lib.load().stu_linear_split(x.data_ptr(), K, W.data_ptr(), K, 1, None, None, 0, short.data_ptr(), N, M, N, K, 0, 0, 0, 0, None, 0.0, 1, 0,
+        rc = _lib.load().stu_linear_split(x.data_ptr(), K + 8, W.data_ptr(), K + 16, 1, None, None, 0, short.data_ptr(), N, M, N, K, 0, 0, 0, 0, None, 0.0, 1, 0,
                                           work.data_ptr(), 64, torch.cuda.current_stream().cuda_stream)
         whole = torch.empty_like(short)
-        rc2 = _lib.load().stu_linear(x.data_ptr(), K, W.data_ptr(), K, 1, None, None, 0, whole.data_ptr(), N, M, N, K, 0, 0, 0, 0, None, 0.0, 1, 0,
+        rc2 = _lib.load().stu_linear(x.data_ptr(), K + 8, W.data_ptr(), K + 16, 1, None, None, 0, whole.data_ptr(), N, M, N, K, 0, 0, 0, 0, None, 0.0, 1, 0,
                                      torch.cuda.current_stream().cuda_stream)
         assert rc == rc2 == 0 and torch.equal(short, whole) and bool(work.isnan().all())
 
@@ -1608,6 +1608,12 @@ def test_full_variant_step_kernel_on_tensor_cores(monkeypatch, B, d, K, L, signs
         taps = phi[:t + 1].double()
         want = [torch.einsum("tk,bti->bki", taps * (s ** torch.arange(t + 1))[:, None], past).reshape(B, K * d) for s in (1.0, -1.0)]
         close(U, torch.cat(want[:signs], 1), 4 * 2 ** -9)
+    # the row as it was appended, without a norm: the same bits
+    new, again = hist[:, :, t & 1, t >> 1].clone(), torch.empty_like(U)
+    hist[:, :, t & 1, t >> 1], pos[:, 0] = float("inf"), t
+    ops.full_decode_step(new, None, 0.0, hist, taps8, pos, again, L, signs == 2, t)
+    ops.check_status()
+    assert torch.equal(again, U) and torch.equal(hist[:, :, t & 1, t >> 1], new)
     pos[:, 0] = L
     ops.full_decode_step(x[:, 0].to(dev()), w.to(dev()), ops.RMS_EPS, hist, taps8, pos, U, L, signs == 2, L)
     with pytest.raises(RuntimeError, match="status 2"):
