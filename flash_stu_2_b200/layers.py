@@ -160,7 +160,7 @@ class STULayer(nn.Module):
             stu, mlp = child(self, "stu"), child(self, "mlp")
             stu_norm, mlp_norm = child(self, "stu_norm"), child(self, "mlp_norm")
             done, entry = 0, past_key_value
-            if stu.use_approx and not stu.use_hankel_L and own(stu, STU, "add_to_residual") and own(mlp, MLP, "apply_residual"):
+            if own(stu, STU, "add_to_residual") and own(mlp, MLP, "apply_residual") and stu.use_approx and not stu.use_hankel_L:
                 done, entry = stu.layer_prefill(xc, entry, use_cache, stu_norm, mlp_norm, mlp)
             if not done:
                 xn = ops.rmsnorm(xc, param(stu_norm, "weight"), stu_norm.eps)

@@ -234,3 +234,23 @@ def test_which_form_the_full_variants_step_takes(batch, d, K, t, pays):
 def test_when_the_full_variants_step_goes_to_tcgen05(batch, d, K, t, pays):
     from flash_stu_2_b200 import ops
     assert ops.full_decode_step_tc5_pays(batch, d, K, t) is pays
+
+
+def test_a_prefill_calls_another_modules_sub_layers(monkeypatch):
+    """A layer whose STU is of another class, with no more of its interface than the prefill called: add_to_residual."""
+    import flash_stu_2_b200 as F
+    from flash_stu_2_b200 import ops
+
+    class Other(torch.nn.Module):
+        def add_to_residual(self, xn, x, entry=None, use_cache=False):
+            x += 2 * xn
+            return "entry" if use_cache else None
+
+    cfg = F.FlashSTUConfig(n_embd=8, n_layers=1, n_heads=1, seq_len=16, vocab_size=1, mlp_scale=2, num_eigh=2, torch_dtype=torch.float32, use_attn=False)
+    layer = F.FlashSTUBlock(config=cfg, phi=torch.zeros(16, 2)).layer
+    layer.stu = Other()
+    monkeypatch.setattr(ops, "rmsnorm", lambda x, *a: x.clone())
+    layer.mlp.apply_residual = lambda xn, resid, out, **kw: out.add_(xn)
+    x = torch.randn(2, 5, 8)
+    y, entry = layer(x.clone(), use_cache=True)
+    assert torch.equal(y, 2 * (x + 2 * x)) and entry == "entry"
