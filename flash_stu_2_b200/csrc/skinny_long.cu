@@ -8,6 +8,8 @@
 // weight row and of an activation row per lane and chunk of 32, the k order permuted alike in both.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "epilogue.cuh"
 
@@ -157,6 +159,34 @@ int launch_long(const void* A, long long lda, const void* B, long long ldb, int 
   return STU_OK;
 }
 
+// Whether the GPU holds this many clusters of KS CTAs at a time (the SMs of a GPC are no multiple of 4)
+template <int KS>
+bool clusters_fit(int clusters) {
+  static std::atomic<int> known[STU_MAX_DEVICES] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= STU_MAX_DEVICES) dev = 0;
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n > 0) return clusters <= n;
+  auto kern = skinny_long_kernel<EPI_STORE, KS>;
+  static SmemLimit limit;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, KS);
+  cfg.blockDim = dim3(NW * 32);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = at.val.clusterDim.z = 1;
+  at.val.clusterDim.y = KS;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (allow_smem((const void*)kern, SMEM_BYTES, limit) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  known[dev].store(n, std::memory_order_relaxed);
+  return clusters <= n;
+}
+
 template <int EPI>
 int launch_long_split(int ks, const void* A, long long lda, const void* B, long long ldb, int M, int N, int K, const EpiArgs<bf16>& ep,
                       int pdl, cudaStream_t st) {
@@ -169,22 +199,23 @@ int launch_long_split(int ks, const void* A, long long lda, const void* B, long 
 
 }  // namespace
 
-// Up to 8 rows of 4096 weights and more, where the kernels of 8 features per CTA would need a second wave or there are 9.4 M weights and
-// more.  us, 8 rows, those kernels and this one: 1024 x 49152 26.7 and 21.5, 768 x 24576 17.3 and 10.7, 768 x 12288 12.1 and 7.0, 1024 x 12288 8.5
-// and 8.0, 1024 x 8192 6.6 and 6.8, 1024 x 4096 3.7 and 4.4, 512 x 49152 15.5 and 16.0, 1280 x 5120 9.1 and 5.9, 1536 x 4096 6.7 and 5.6, 2048 x 8192
-// 11.9 and 9.2, 4096 x 16384 39 and 25 (1 and 4 rows alike).
+// Up to 8 rows of 4096 weights and more, where the kernels of 8 features per CTA would need a second wave (from 4104 weights or 16 features per SM
+// on) or there are 9.4 M weights and more and the clusters of four run at a time (B200: up to 33 of them, N = 1056; in two waves 4 x 1128 x
+// 8368 took 13.7 us where those kernels take 8.6).  us, 8 rows, those kernels and this one: 1024 x 49152 26.7 and 21.5, 768 x 24576 17.3 and 10.7, 768 x 12288
+// 12.1 and 7.0, 1024 x 12288 8.5 and 8.0, 1024 x 8192 6.6 and 6.8, 1024 x 4096 3.7 and 4.4, 512 x 49152 15.5 and 16.0, 1280 x 5120 9.1 and 5.9, 2048 x 4096 7.3
+// and 7.8, 2048 x 8192 11.9 and 9.2, 4096 x 16384 39 and 25 (1 and 4 rows alike).
 bool skinny_long_takes(int M, int N, int K, int epi, bool norm, bool peer) {
   const int sms = device_sm_count();
-  return M <= 8 && (epi == EPI_STORE || epi == EPI_RESID) && !norm && !peer && K >= 4096 && N <= 32 * sms &&
-         (N > 8 * sms || (N >= 640 && (long long)N * K >= 9400000));
+  if (M > 8 || (epi != EPI_STORE && epi != EPI_RESID) || norm || peer || K < 4096 || N > 32 * sms) return false;
+  if (N > 8 * sms) return K > 4096 || N > 16 * sms;
+  return N >= 640 && (long long)N * K >= 9400000 && clusters_fit<4>((N + 8 * NT - 1) / (8 * NT));
 }
 
 int skinny_long_dispatch(const void* A, long long lda, const void* B, long long ldb, int M, int N, int K, int epi, const EpiArgs<bf16>& ep,
                          int pdl, cudaStream_t st) {
-  // K is split until there is about one CTA per SM (1536 x 8192: one CTA per tile 9.6 us, two 8.2, four 10.8)
-  const int ctas = (N + 8 * NT - 1) / (8 * NT), sms = device_sm_count();
-  int ks = 1;
-  while (ks < 4 && ctas * ks * 2 <= sms) ks *= 2;
+  // K is split until there is about one CTA per SM (1536 x 8192: one CTA per tile 9.6 us, two 8.2, four 10.8), in clusters that run at a time
+  const int ctas = (N + 8 * NT - 1) / (8 * NT);
+  const int ks = clusters_fit<4>(ctas) ? 4 : clusters_fit<2>(ctas) ? 2 : 1;
   if (epi == EPI_STORE) return launch_long_split<EPI_STORE>(ks, A, lda, B, ldb, M, N, K, ep, pdl, st);
   return launch_long_split<EPI_RESID>(ks, A, lda, B, ldb, M, N, K, ep, pdl, st);
 }
