@@ -6,7 +6,7 @@
 // against float64, this kernel and the CUDA-core GEMM (2-norm, normal operands): K = 3072 1.4e-7 and 7.0e-7, 1024 1.2e-7 and 5.7e-7, 256
 // 7.7e-8 and 1.5e-7; positive ones (sums that are not rounded to nearest drift) 9.5e-8 and 4.2e-7, 9.4e-8 and 4.3e-7, 6.7e-8 and
 // 7.0e-8; 64 of K per accumulator 1.25e-7, 1.1e-7, 8.9e-8, positive 9.7e-8, 9.6e-8, 8.7e-8.  (The weight-streaming kernels of up to 64
-// rows are below either and keep those.)  Values below 2^-110 have third parts that bf16 does not hold.
+// rows are below either and keep those.)
 //
 // Bound: shared memory, through which a block of 64 of K passes three times as planes and six times as operands, and the splitting, about
 // 6 instructions a value.  us, the CUDA-core GEMM and this kernel: 8000 x 96 x 3072 159 and 50, 256 x 512 x 6144 56 and 28, gate/up 256 x 6144 x
@@ -16,8 +16,9 @@
 // shared memory, in rank order.  Warps 0..10 fetch 64 of K of both operands into registers, one block ahead, split them and store the
 // three planes in the 128-byte swizzle that the operand descriptors expect, into one of two or three stages; warp 11 issues 24
 // tcgen05.mma per block; warps 12..19 drain the accumulators in tensor memory (tcgen05.ld) into their sums.
-// A sum that is not finite is computed again on the CUDA cores: operands that are not finite, or above 2^111, have no
-// such split.
+// Sums that are not finite are computed again on the CUDA cores, 32 rows and half of a tile's columns at a time: operands that are not finite, or
+// above 2^87, have no such split, and sums above 2^79 overflow.  4000 x 8192 x 1024, all of them, 6.4 ms (a thread's chain for each, 125 ms; the
+// CUDA-core GEMM 1.6), 1000 x 1536 x 512 with a NaN in one row 157 us (36 without).
 // Every wait is bounded: on expiry the CTA raises status 3, frees its tensor memory and returns.
 #include <cooperative_groups.h>
 
@@ -71,6 +72,64 @@ struct Ctl {
 template <int BN> __host__ __device__ constexpr int stage_bytes() { return 3 * (PLANE_A + BN * BK * 2); }
 template <int BN> __host__ __device__ constexpr int stages() { return BN <= 64 ? 3 : 2; }
 template <int BN> __host__ __device__ constexpr int smem_bytes() { return stages<BN>() * stage_bytes<BN>() + (int)sizeof(Ctl) + 1024; }
+
+// One warp's 32 rows and HALF columns of a tile once more, on the CUDA cores: sums over k in [k0, k1) into part (lane: a row; columns `step` apart).
+// room: again_floats() values of shared memory.  Of A there are `rows` rows; B (and B2: gate/up) are those of the tile's columns, of which there are `cols`.
+constexpr int AGAIN_K = 32;
+template <int HALF> __host__ __device__ constexpr int again_floats() { return 32 * (AGAIN_K + 1) + AGAIN_K * (HALF + 4); }
+template <int HALF, int COLS, bool DUAL>
+__device__ __noinline__ void sums_again(const float* A, long long lda, int rows, const float* B, const float* B2, long long ldb, int c0, int cols,
+                                        int k0, int k1, float* room, float* part, int step) {
+  const int lane = threadIdx.x & 31, piece = 4 * (lane & 7);   // 16-byte pieces of a row: K and k0 are multiples of 4 values, rows lie on the grid
+  float *a_s = room, *b_s = room + 32 * (AGAIN_K + 1);
+  for (int c = 0; c < HALF; c++) part[c * step] = 0.f;
+  for (int k = k0; k < k1; k += AGAIN_K) {
+    const bool in = k + piece < k1;
+    float4 v[8];   // (eight on their way at once)
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int r = 4 * i + (lane >> 3);
+      v[i] = in && r < rows ? *reinterpret_cast<const float4*>(A + (size_t)r * lda + k + piece) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      float* at = a_s + (4 * i + (lane >> 3)) * (AGAIN_K + 1) + piece;
+      at[0] = v[i].x, at[1] = v[i].y, at[2] = v[i].z, at[3] = v[i].w;
+    }
+#pragma unroll 1
+    for (int c8 = 0; c8 < HALF; c8 += 32) {
+#pragma unroll
+      for (int i = 0; i < (HALF < 32 ? HALF / 4 : 8); i++) {
+        const int c = c0 + c8 + 4 * i + (lane >> 3), n = DUAL ? c % COLS : c;
+        v[i] = in && n < cols ? *reinterpret_cast<const float4*>((DUAL && c >= COLS ? B2 : B) + (size_t)n * ldb + k + piece) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < (HALF < 32 ? HALF / 4 : 8); i++) {
+        float* at = b_s + piece * (HALF + 4) + c8 + 4 * i + (lane >> 3);
+        at[0] = v[i].x, at[HALF + 4] = v[i].y, at[2 * (HALF + 4)] = v[i].z, at[3 * (HALF + 4)] = v[i].w;
+      }
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int h = 0; h < HALF; h += 16) {
+      float s[16];
+#pragma unroll
+      for (int c = 0; c < 16; c++) s[c] = 0.f;
+#pragma unroll 4
+      for (int i = 0; i < AGAIN_K; i++) {
+        const float a = a_s[lane * (AGAIN_K + 1) + i];
+#pragma unroll
+        for (int c = 0; c < 16; c += 4) {
+          const float4 b = *reinterpret_cast<const float4*>(b_s + i * (HALF + 4) + h + c);
+          s[c] = fmaf(a, b.x, s[c]), s[c + 1] = fmaf(a, b.y, s[c + 1]), s[c + 2] = fmaf(a, b.z, s[c + 2]), s[c + 3] = fmaf(a, b.w, s[c + 3]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 16; c++) part[(h + c) * step] += s[c];
+    }
+  }
+}
 
 template <int EPI, int KS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -225,9 +284,22 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     __syncwarp();
     __syncthreads();
-    float* p = part + ((warp & 3) * 32 + lane) * PITCH + c0;
+    const int r0 = (warp & 3) * 32;
+    float* p = part + (r0 + lane) * PITCH + c0;
+    bool fine = true;
+#pragma unroll
+    for (int c = 0; c < HALF; c++) {
+      sum[c] *= SPLIT_UNSCALE;
+      fine = fine && isfinite(sum[c]);
+    }
 #pragma unroll
     for (int c = 0; c < HALF; c += 4) *reinterpret_cast<float4*>(p + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+    if (!__all_sync(0xffffffffu, fine)) {
+      constexpr int ROOM = (BM * PITCH + 31) / 32 * 32;   // behind the tile's sums
+      static_assert(4 * (ROOM + DRAIN_WARPS * again_floats<HALF>()) <= STAGES * STAGE, "room for the sums made again");
+      sums_again<HALF, COLS, DUAL>(A + (size_t)min(m0 + r0, M - 1) * lda, lda, min(32, M - m0 - r0), B + (size_t)n0 * ldb, DUAL ? B2 + (size_t)n0 * ldb : nullptr, ldb, c0,
+                                   N - n0, kb0 * BK, min(kb1 * BK, k_end), part + ROOM + (warp - DRAIN0) * again_floats<HALF>(), p, 1);
+    }
   }
   cg::cluster_group cluster = cg::this_cluster();
   if constexpr (KS > 1) cluster.sync(); else __syncthreads();
@@ -247,15 +319,6 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int r = 0; r < KS; r++) {
         s += parts[r][row * PITCH + c];
         if (DUAL) s2 += parts[r][row * PITCH + COLS + c];
-      }
-      if (!isfinite(s) || (DUAL && !isfinite(s2))) {
-        s = s2 = 0.f;
-#pragma unroll 1
-        for (int k = 0; k < k_end; k++) {
-          const float a = A[(size_t)m * lda + k];
-          s = fmaf(a, B[(size_t)n * ldb + k], s);
-          if (DUAL) s2 = fmaf(a, B2[(size_t)n * ldb + k], s2);
-        }
       }
       epilogue_store<float, EPI>(ep, m, n, s, s2);
     }

@@ -2,11 +2,14 @@
 #pragma once
 #include "common.cuh"
 
-// Two consecutive values as one word of each part: x1 nearest to x, x2 the leading 8 bits of x - x1, x3 the rest, 24 bits of significand
-// in all.  The first part comes of a multiplication by 2^16 + 1 and two differences (Dekker's and Veltkamp's splitting: a nearest value of 8
-// bits; past 2^111 not finite), in pairs on the FMA pipe: conversions to bf16 are a sixteenth of its rate.  (As fused operations: a
+// Two consecutive values, times SPLIT_SCALE, as one word of each part: x1 nearest to x, x2 the leading 8 bits of x - x1, x3 the rest, 24 bits of
+// significand in all.  The first part comes of a multiplication by 2^16 + 1 and two differences (Dekker's and Veltkamp's splitting: a nearest value of 8
+// bits; past 2^111, here 2^87, not finite), in pairs on the FMA pipe: conversions to bf16 are a sixteenth of its rate.  (As fused operations: a
 // product and the difference behind it would be fused by the compiler, and the first part not be one.)  The second part is cut off and
 // not rounded: behind a nearest first part the signs of the rest are random, and what is cut off is the third part whole.
+// The scale keeps the third part of every fp32 value, subnormal ones among them, a normal bf16 value (from 2^-125 on), and the small
+// products of results that fp32 holds above the accumulators' subnormal range; a sum past 2^79 is not finite.
+constexpr float SPLIT_SCALE = 16777216.f, SPLIT_UNSCALE = 1.f / (SPLIT_SCALE * SPLIT_SCALE);   // of an operand; of a sum of products
 __device__ __forceinline__ uint64_t split_pair(float a, float b) { return (uint64_t)__float_as_uint(a) | (uint64_t)__float_as_uint(b) << 32; }
 __device__ __forceinline__ uint64_t split_fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
@@ -16,7 +19,7 @@ __device__ __forceinline__ uint64_t split_fma2(uint64_t a, uint64_t b, uint64_t 
 __device__ __forceinline__ uint64_t split_sub2(uint64_t a, uint64_t b) { return split_fma2(b, 0xbf800000bf800000ull, a); }   // a - b
 __device__ __forceinline__ uint32_t split_upper(uint64_t v) { return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632); }
 __device__ __forceinline__ void split2(float a, float b, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
-  const uint64_t x = split_pair(a, b), t = split_fma2(x, split_pair(65537.f, 65537.f), 0ull);
+  const uint64_t x = split_fma2(split_pair(a, b), split_pair(SPLIT_SCALE, SPLIT_SCALE), 0ull), t = split_fma2(x, split_pair(65537.f, 65537.f), 0ull);
   const uint64_t x1 = split_sub2(t, split_sub2(t, x)), r = split_sub2(x, x1);
   w1 = split_upper(x1);
   w2 = split_upper(r);

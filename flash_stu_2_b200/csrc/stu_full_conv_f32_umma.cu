@@ -16,8 +16,9 @@
 //
 // Roles (one persistent CTA per SM, 320 threads): warp 0 producer, warp 1 MMA issuer, warps 2-9 sums and outputs (a quarter of the
 // rows and half of the channels each).  Tiles run from the latest positions (the most work) down, the filters of a channel block side by
-// side, so that its history rows are read from L2.  A result that is not finite is computed again on the CUDA cores: values that are
-// not finite, or above 2^111, have no such parts.
+// side, so that its history rows are read from L2.  Sums that are not finite are computed again on the CUDA cores, a warp's part of a
+// tile at a time: values that are not finite, or above 2^87, have no such parts, and sums above 2^79 overflow.  24 filters, 8 x 1000 positions of 64
+// channels, all of them, 2.2 ms (a thread's chain for each, 39 ms; the CUDA-core kernel 0.29), with one NaN in a channel 0.8 (7.9).
 // Every load is a plain single-CTA copy of this GPU's own memory.  Every wait is bounded: on expiry the CTA raises status 9, lets issued
 // copies land (bounded), frees its tensor memory and returns.
 #include <cuda.h>
@@ -149,17 +150,78 @@ __device__ __forceinline__ Tile tile_at(const Geom& g, int i) {
   return t;
 }
 
-// U+ (sign 0) or U- of one position, filter and channel row, product by product
-__device__ __noinline__ float one_result(const float* hist, const float* phi, const Geom& g, int row, int k, int tt, int sign) {
-  const int m = tt >> 1, p = tt & 1;
-  const float *same = hist + ((size_t)row * 2 + p) * g.Lh, *other = hist + ((size_t)row * 2 + (p ^ 1)) * g.Lh;
-  float e = 0.f, q = 0.f;
-  for (int s = 0; s <= m; s++) {
-    const int j = 2 * (m - s), jo = j + (p ? 1 : -1);
-    if (j < g.L) e = fmaf(phi[(size_t)j * g.K + k], same[s], e);
-    if (jo >= 0 && jo < g.L) q = fmaf(phi[(size_t)jo * g.K + k], other[s], q);
+// A warp's outputs of a tile once more, on the CUDA cores, and stored: lane = position 2 m + p (the warp's 32 m are m_min .. m_min + 31), `half` channels
+// from col0 on (16 at a time), filter k.  Entries in steps of AGAIN_S through the warp's staging block; an output meets those that its sum has
+// and no others.
+constexpr int AGAIN_S = 32, AGAIN_C = 16, AGAIN_TAPS = 32 + AGAIN_S;
+static_assert(4 * (2 * AGAIN_S * AGAIN_C + 2 * AGAIN_TAPS) <= STG_BYTES, "staging block");
+__device__ __noinline__ void outputs_again(const float* hist, const float* phi, float* U, const Geom& g, int k, int p, int m_min, int m, int col0,
+                                           int half, float* st) {
+  const int lane = threadIdx.x & 31, rows = g.B * g.d, back = p ? 0 : 1;   // Q: odd taps 2 (m - s - back) + 1
+  float *same = st, *other = st + AGAIN_S * AGAIN_C, *te = st + 2 * AGAIN_S * AGAIN_C, *tq = te + AGAIN_TAPS;
+  for (; half > 0 && col0 < rows; col0 += AGAIN_C, half -= AGAIN_C) {
+    float e[AGAIN_C], q[AGAIN_C];
+#pragma unroll
+    for (int c = 0; c < AGAIN_C; c++) e[c] = q[c] = 0.f;
+    for (int s0 = 0; s0 <= m_min + 31; s0 += AGAIN_S) {
+      __syncwarp();
+      float v[2][AGAIN_C];   // (all on their way at once)
+#pragma unroll
+      for (int c = 0; c < AGAIN_C; c++) {
+        const int s = s0 + lane;
+        const float* h = hist + (size_t)(col0 + c) * 2 * g.Lh + s;
+        v[0][c] = col0 + c < rows && 2 * s + p < g.t_end ? h[p ? g.Lh : 0] : 0.f;
+        v[1][c] = col0 + c < rows && 2 * s + (p ^ 1) < g.t_end ? h[p ? 0 : g.Lh] : 0.f;
+      }
+#pragma unroll
+      for (int c = 0; c < AGAIN_C; c += 4) {
+        *reinterpret_cast<float4*>(same + lane * AGAIN_C + c) = make_float4(v[0][c], v[0][c + 1], v[0][c + 2], v[0][c + 3]);
+        *reinterpret_cast<float4*>(other + lane * AGAIN_C + c) = make_float4(v[1][c], v[1][c + 1], v[1][c + 2], v[1][c + 3]);
+      }
+      const int d0 = m_min - s0 - (AGAIN_S - 1);   // distance that the staged taps begin with
+#pragma unroll
+      for (int i = lane; i < AGAIN_TAPS; i += 32) {
+        const int je = 2 * (d0 + i), jq = 2 * (d0 + i - back) + 1;
+        te[i] = je >= 0 && je < g.L ? phi[(size_t)je * g.K + k] : 0.f;
+        tq[i] = jq >= 0 && jq < g.L ? phi[(size_t)jq * g.K + k] : 0.f;
+      }
+      __syncwarp();
+      const auto add = [&](float (&sum)[AGAIN_C], float tap, const float* x, int i) {
+#pragma unroll
+        for (int c = 0; c < AGAIN_C; c += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(x + i * AGAIN_C + c);
+          sum[c] = fmaf(tap, w.x, sum[c]), sum[c + 1] = fmaf(tap, w.y, sum[c + 1]);
+          sum[c + 2] = fmaf(tap, w.z, sum[c + 2]), sum[c + 3] = fmaf(tap, w.w, sum[c + 3]);
+        }
+      };
+      const int at = m - m_min + AGAIN_S - 1;   // tap of entry s0
+      if (d0 >= back && 2 * (d0 + AGAIN_TAPS) < g.L) {   // every tap of every lane
+#pragma unroll 4
+        for (int i = 0; i < AGAIN_S; i++) {
+          add(e, te[at - i], same, i);
+          add(q, tq[at - i], other, i);
+        }
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < AGAIN_S; i++) {
+          const int dist = m - s0 - i;
+          if (dist >= 0 && 2 * dist < g.L) add(e, te[at - i], same, i);
+          if (dist >= back && 2 * (dist - back) + 1 < g.L) add(q, tq[at - i], other, i);
+        }
+      }
+    }
+    const int t = 2 * m + p;
+    if (t >= g.t0 && t < g.t_end)
+#pragma unroll
+      for (int c = 0; c < AGAIN_C; c++) {
+        const int col = col0 + c, b = col / g.d;
+        if (col >= rows) continue;
+        float* at = U + ((size_t)b * g.Tn + (t - g.t0)) * g.ldU + (size_t)k * g.d + (col - b * g.d);
+        at[0] = e[c] + q[c];
+        if (g.both) at[(size_t)g.K * g.d] = e[c] - q[c];
+      }
   }
-  return sign ? e - q : e + q;
+  __syncwarp();
 }
 
 template <int TN>
@@ -293,6 +355,18 @@ __global__ void __launch_bounds__(THREADS, 1)
       };
       ok = add(e) && add(q);
       if (!ok) break;
+      bool fine = true;
+#pragma unroll
+      for (int c = 0; c < HALF; c++) {
+        e[c] *= SPLIT_UNSCALE, q[c] *= SPLIT_UNSCALE;
+        fine = fine && isfinite(e[c]) && isfinite(q[c]);
+      }
+      if (!__all_sync(0xffffffffu, fine)) {
+        // row `lane` of the warp's 32 is position 120 - 8 (L / 8) + L % 8 of the block, L = 32 quarter + lane
+        const int m_min = t.mb * BM + 96 - 32 * quarter;
+        outputs_again(hist, phi, U, g, t.k, t.p, m_min, m_min + 24 - 8 * (lane >> 3) + (lane & 7), t.ct * TN + half * HALF, HALF, st);
+        continue;
+      }
 #pragma unroll
       for (int sign = 0; sign < 2; sign++) {
         if (sign && !g.both) break;
@@ -309,12 +383,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             const int b = col / g.d, c = col - b * g.d;
             float* base = U + (size_t)b * g.Tn * g.ldU + (size_t)(sign * g.K + t.k) * g.d + c;
             float4 v[8];
-            bool fine = true;
 #pragma unroll
-            for (int x = 0; x < 8; x++) {
-              v[x] = *reinterpret_cast<const float4*>(st + (r0 + 4 * x) * SROW + piece * 4);
-              fine = fine && isfinite(v[x].x) && isfinite(v[x].y) && isfinite(v[x].z) && isfinite(v[x].w);
-            }
+            for (int x = 0; x < 8; x++) v[x] = *reinterpret_cast<const float4*>(st + (r0 + 4 * x) * SROW + piece * 4);
             // row r0 + 4 x of the warp's 32 is position 120 - 8 (L / 8) + L % 8 of the block, L = 32 quarter + r0 + 4 x
             auto time_of = [&](int x) { return 2 * (t.mb * BM + 120 - 32 * quarter - 8 * (x >> 1) + r0 + 4 * (x & 1)) + t.p; };
 #pragma unroll
@@ -322,12 +392,6 @@ __global__ void __launch_bounds__(THREADS, 1)
               const int tt = time_of(x);
               if (tt >= g.t0 && tt < g.t_end) *reinterpret_cast<float4*>(base + (size_t)(tt - g.t0) * g.ldU) = v[x];
             }
-            if (!fine)
-              for (int x = 0; x < 8; x++) {
-                const int tt = time_of(x);
-                if (tt < g.t0 || tt >= g.t_end) continue;
-                for (int j = 0; j < 4; j++) base[(size_t)(tt - g.t0) * g.ldU + j] = one_result(hist, phi, g, col + j, t.k, tt, sign);
-              }
           }
           __syncwarp();
         }

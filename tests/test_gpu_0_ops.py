@@ -576,6 +576,10 @@ def test_full_variant_fp32_convolutions_on_tensor_cores(case):
     want = torch.fft.irfft(want, n=n, dim=1)[:, t0:T].reshape(B * (T - t0), -1)
     err = [float((u.double() - want).norm() / want.norm()) for u in U]
     assert err[0] <= max(err[1], 2.0 ** -23), err
+    again = torch.full_like(U[0], float("nan"))   # operands past 2^87: every sum made again on the CUDA cores, the other kernel's chains
+    ops.full_conv_f32_tc5(hist * 2.0 ** 90, phi * 2.0 ** -90, again, both, t0, T)
+    ops.check_status()
+    assert torch.equal(again, U[1])
 
 
 def test_full_variant_fp32_convolutions_of_values_without_a_split():
@@ -615,6 +619,60 @@ def test_fp32_linear_on_tensor_cores_values_without_a_split():
     assert torch.equal(got[got.isinf()], want[want.isinf()])
     fin = want.isfinite()
     assert float(((got - want)[fin].abs() / want[fin].abs().clamp_min(1)).max()) < 2e-5   # (1024 products of order 1/32: rounding of the partial sums)
+
+
+@pytest.mark.parametrize("shape", [(65, 100, 1024), (129, 1, 2060), (300, 2049, 256), (1000, 700, 516), (66, 512, 6144)])
+@pytest.mark.parametrize("epi", [0, 1, 2, 3])
+def test_fp32_sums_on_tensor_cores_made_again(shape, epi):
+    """Operands past 2^87 have no split: every sum is made on the CUDA cores behind the instructions.  Edges of tiles, of K and of its split, each
+    epilogue, several sequences of a history that begin at an odd position.  Bar: against float64 no further off than the CUDA-core GEMM."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    torch.manual_seed(7)
+    x = 3e26 * torch.randn(M, K + 4, device=dev())[:, :K]
+    W, W2 = 1e-26 * torch.randn(2, N, K, device=dev()) / math.sqrt(K)
+    x[M // 2, K - 1], r = float("inf"), torch.randn(M, N, device=dev())
+    full, T = x.double() @ W.double().t(), M // 3 if M % 3 == 0 else M // 5 if M % 5 == 0 else M
+    Lh = (T + 20) // 16 * 8
+    kw = {0: {}, 1: dict(resid=r), 2: dict(W2=W2), 3: dict(hist_T=T, hist_t0=3, hist_Lh=Lh)}[epi]
+    want = {0: full, 1: r.double() + full, 2: torch.nn.functional.gelu(full, approximate="tanh") * (x.double() @ W2.double().t()), 3: full}[epi]
+    err, fin = [], want.isfinite()
+    for backend in (0, 1):
+        out = torch.full((M // T, N, 2, Lh) if epi == 3 else (M, N), float("nan"), device=dev())
+        ops.linear(x, W, out=out, epilogue=epi, backend=backend, **kw)
+        if epi == 3:
+            t = torch.arange(3, T + 3, device=dev())
+            assert int((~out.isnan()).sum()) == M * N
+            out = out[:, :, t % 2, t // 2].permute(0, 2, 1).reshape(M, N)
+        assert torch.equal(out.isfinite(), fin) and torch.equal(out.isnan(), want.isnan())
+        err.append(float((out.double() - want)[fin].norm() / want[fin].norm()))
+    ops.check_status()
+    assert err[0] <= max(err[1], 2.0 ** -24), err
+
+
+@pytest.mark.parametrize("rows,weights", [(1e-36, 1.0), (1.0, 1e-36), (1e-35, 1e30), (3e-19, 3e-19), (1e-42, 1e6), (1e20, 1e4)])
+def test_fp32_products_on_tensor_cores_of_small_and_large_operands(rows, weights):
+    """Operands whose third parts bf16 would hold only as subnormals, or not at all, and products near the end of fp32's range.  Bars: against
+    float64 no further off than the CUDA-core kernels on the same operands, but for the rounding of the result (E and Q: 2^-23)."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(12)
+    x, W = rows * torch.randn(300, 512, device=dev()), weights * torch.randn(2000, 512, device=dev())
+    want = x.double() @ W.double().t()
+    err = [float((ops.linear(x, W, backend=b).double() - want).norm() / want.norm()) for b in (0, 1)]
+    assert err[0] <= max(err[1], 2.0 ** -24), err
+    B, T, d, K = 2, 500, 8, 3
+    x, phi = rows * torch.randn(B, T, d), weights * torch.randn(T, K)
+    hist = _hist_from(x, 256).to(dev())
+    U = [torch.empty(B * T, 2 * K * d, device=dev()) for _ in range(2)]
+    ops.full_conv_f32_tc5(hist, phi.to(dev()), U[0], True, 0, T)
+    ops.full_conv(hist, phi.to(dev()), U[1], True, 0, T)
+    ops.check_status()
+    lag = torch.arange(T)[:, None] - torch.arange(T)[None]
+    m = torch.where(lag[:, :, None] >= 0, phi.double()[lag.clamp_min(0)], torch.zeros((), dtype=torch.float64))
+    want = [torch.einsum("tsk,bsi->btki", m * s, x.double()) for s in (torch.ones(()), (1.0 - 2 * (lag.abs() % 2))[:, :, None])]
+    want = torch.stack(want, 2).reshape(B * T, -1)
+    err = [float((u.cpu().double() - want).norm() / want.norm()) for u in U]
+    assert err[0] <= max(err[1], 2.0 ** -23), err
 
 
 @pytest.mark.parametrize("shape", [(1, 256, 1000, 0), (2, 1279, 900, 1270), (3, 1500, 760, 700), (2, 2049, 480, 1800), (9, 2817, 160, 2815),
