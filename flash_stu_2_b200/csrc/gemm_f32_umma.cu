@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (int p = 0; p < SPLIT_PRODUCTS; p++)
 #pragma unroll
               for (int kk = 0; kk < CHAIN; kk++)
-                umma(acc, da + ((split_a(p) * PLANE_A + 32 * (h * CHAIN + kk)) >> 4), db + ((split_b(p) * PLANE_B + 32 * (h * CHAIN + kk)) >> 4), IDESC, p || kk ? 1u : 0u);
+                umma(acc, da + ((split_a(p) * PLANE_A + 32 * (h * CHAIN + kk)) >> 4), db + ((split_b(p) * PLANE_B + 32 * (h * CHAIN + kk)) >> 4), IDESC | split_sign(p), p || kk ? 1u : 0u);
             if (h + 1 == CHAINS) umma_commit(&ctl->empty[s]);
             umma_commit(&ctl->acc_full[a]);
           }

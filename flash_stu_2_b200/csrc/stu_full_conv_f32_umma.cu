@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
             for (int kk = 0; kk < BK / 16; kk++)   // 16 positions: two core matrices of the table, 32 bytes of a history row
               umma(tmem_base + 128 * a, da + (uint64_t)((2 * kk * CM + split_a(p) * 128) >> 4),
-                   db + (uint64_t)((split_b(p) * PLANE_B + kk * 32) >> 4), IDESC, p || kk ? 1u : 0u);
+                   db + (uint64_t)((split_b(p) * PLANE_B + kk * 32) >> 4), IDESC | split_sign(p), p || kk ? 1u : 0u);
           umma_commit(&ctl->empty[s]);
           umma_commit(&ctl->acc_full[a]);
         }
