@@ -124,6 +124,11 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // STU_B200_DISABLE_PDL=1 turns every launch back into a plain stream-ordered one.
 bool pdl_enabled();
 
+// What stu_test_inject_wait_expiry set (gemm_tc.cu): the bound of the waits of the next launches, and whether the launch that asks is the one
+// whose first stage is never filled.
+unsigned long long wait_bound_ns();
+bool take_dropped_stage();
+
 // Launch with or without the programmatic attribute.
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_maybe_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,

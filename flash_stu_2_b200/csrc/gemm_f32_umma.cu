@@ -19,7 +19,7 @@
 // Sums that are not finite are computed again on the CUDA cores, 32 rows and half of a tile's columns at a time: operands that are not finite, or
 // above 2^87, have no such split, and sums above 2^79 overflow.  4000 x 8192 x 1024, all of them, 6.4 ms (a thread's chain for each, 125 ms; the
 // CUDA-core GEMM 1.6), 1000 x 1536 x 512 with a NaN in one row 157 us (36 without).
-// Every wait is bounded: on expiry the CTA raises status 3, frees its tensor memory and returns.
+// Every wait is bounded: on expiry the CTA raises status 3, frees its tensor memory and returns, and no CTA of its cluster stores anything.
 #include <cooperative_groups.h>
 
 #include <atomic>
@@ -135,7 +135,7 @@ template <int EPI, int KS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_f32_umma_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ B, long long ldb,
                          const float* __restrict__ B2, int M, int N, int K, int causal, EpiArgs<float> ep, int* status,
-                         unsigned long long wait_ns) {
+                         int drop_first_stage, unsigned long long wait_ns) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL), HIST = (EPI == EPI_HIST);
   constexpr int COLS = DUAL ? BN / 2 : BN, STAGE = stage_bytes<BN>(), PLANE_B = BN * BK * 2, PITCH = BN + 4;
   constexpr int STAGES = stages<BN>(), ACCS = BN <= 64 ? 4 : 2, ACC_COLS = BN <= 64 ? 64 : 128;
@@ -223,7 +223,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&ctl->full[s]);
+        // (drop_first_stage, a test: the last CTA of a cluster never has its first block)
+        if (lane == 0 && !(drop_first_stage && n == 0 && (KS == 1 || blockIdx.z == KS - 1))) tma::mbar_arrive(&ctl->full[s]);
         if (++s == STAGES) s = 0, turn ^= 1u;
       }
     } else {
@@ -305,6 +306,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   }
   cg::cluster_group cluster = cg::this_cluster();
+  if (KS > 1 && tid == 0 && *abort_flag) {   // nobody adds up sums that one of the cluster has not got
+    if (status) atomicExch(status, 3);
+    for (int r = 0; r < KS; r++) *cluster.map_shared_rank(&ctl->abort_flag, r) = 1;
+  }
   if constexpr (KS > 1) cluster.sync(); else __syncthreads();
   const int rank = KS > 1 ? (int)cluster.block_rank() : 0;
   const float* parts[KS];
@@ -416,7 +421,7 @@ int launch_tile(const Operands& o, const EpiArgs<float>& ep, cudaStream_t st) {
   }
   cfg.attrs = at;
   cfg.numAttrs = n;
-  e = cudaLaunchKernelEx(&cfg, kern, o.A, o.lda, o.B, o.ldb, o.B2, o.M, o.N, o.K, o.causal, ep, device_status_word(), 2000000000ull);
+  e = cudaLaunchKernelEx(&cfg, kern, o.A, o.lda, o.B, o.ldb, o.B2, o.M, o.N, o.K, o.causal, ep, device_status_word(), (int)take_dropped_stage(), wait_bound_ns());
   if (e != cudaSuccess) return (int)e;
   STU_CHECK_LAUNCH();
   return STU_OK;

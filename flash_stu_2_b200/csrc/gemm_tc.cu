@@ -940,8 +940,7 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
   const int tiles_m = (M + CTAS * BM - 1) / (CTAS * BM), tiles_n = (N + TN - 1) / TN;
   const int tiles = SPLIT ? split.whole + (tiles_m * tiles_n - split.whole) * split.parts : tiles_m * tiles_n, most = CTAS == 2 ? device_pairs() : device_sm_count();
   const int grid = CTAS * (tiles < most ? tiles : most);  // one persistent CTA per SM
-  const int drop = g_drop_first_copy;
-  g_drop_first_copy = 0;   // the injected fault applies to one launch
+  const int drop = take_dropped_stage();
   const int group_m = m_fast ? tiles_m : gemm_group_m(tiles_n, N, K, DUAL);
   e = launch_maybe_overlapped(k, dim3(grid), dim3(64 + 32 * EPI_WARPS), smem, st, true, a, b, b2, y, by_copy, M, N, K, tiles_m, tiles_n, group_m,
                               causal, ep, status, drop, g_wait_ns, split);
@@ -1276,9 +1275,9 @@ int device_sm_count() {
 
 int* device_status_word() { return g_status_words[current_device()]; }
 
-// Test hook for the failure-detection path: the next tcgen05 GEMM launch of this process never issues the copies of
-// its first pipeline stage, and every bounded wait gives up after wait_ms milliseconds (0 restores the default of
-// two seconds without arming a fault).  The kernel then reports status 3, drains what it did issue, frees its tensor
+// Test hook for the failure-detection path: the next launch of this process of a tcgen05 GEMM (bf16 or fp32), of the full variant's fp32 convolutions or of
+// its token step on tcgen05 never fills its first pipeline stage, and every bounded wait of theirs gives up after wait_ms milliseconds (0 restores
+// the default of two seconds without arming a fault).  The kernel then reports its status, drains what it did issue, frees its tensor
 // memory and returns; nothing faults and the context stays usable.
 extern "C" int stu_test_inject_wait_expiry(int wait_ms) {
   if (wait_ms < 0 || wait_ms > 10000) return STU_ERR_SHAPE;
@@ -1290,6 +1289,13 @@ extern "C" int stu_test_inject_wait_expiry(int wait_ms) {
     g_wait_ns = (unsigned long long)wait_ms * 1000000ull;
   }
   return STU_OK;
+}
+
+unsigned long long wait_bound_ns() { return g_wait_ns; }
+bool take_dropped_stage() {   // the injected fault applies to one launch
+  const bool drop = g_drop_first_copy != 0;
+  g_drop_first_copy = 0;
+  return drop;
 }
 
 // make_map for the other tensor-core kernels of K-major bf16 operands.

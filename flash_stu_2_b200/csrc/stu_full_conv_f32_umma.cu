@@ -228,7 +228,7 @@ template <int TN>
 __global__ void __launch_bounds__(THREADS, 1)
     full_conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmH, const bf16* __restrict__ tab, const float* __restrict__ hist,
                               const float* __restrict__ phi, float* __restrict__ U, const __grid_constant__ Geom g, int* status,
-                              unsigned long long wait_ns) {
+                              int drop_first_stage, unsigned long long wait_ns) {
   constexpr int PLANE_B = plane_b<TN>(), B_PITCH = 3 * PLANE_B, HALF = TN / 2;
   constexpr int A_OFF = STAGES * B_PITCH, STG_OFF = stages_bytes<TN>(), CTL_OFF = STG_OFF + EPI_WARPS * STG_BYTES;
   extern __shared__ unsigned char smem_raw[];
@@ -274,8 +274,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int kb = 0; kb <= 2 * t.mb + 1; kb++, it++) {
           ok = tma::warp_wait_bounded(&ctl->empty[s], ph, abort_flag, wait_ns);
           if (!ok) break;
-          if (leader) {
-            tma::mbar_expect_tx(&ctl->full[s], B_PITCH + A_BYTES);
+          if (leader) tma::mbar_expect_tx(&ctl->full[s], B_PITCH + A_BYTES);
+          if (leader && !(drop_first_stage && it == 0)) {   // (a test: these copies are never issued)
             tma::load_4d(smem + s * B_PITCH, &tmH, &ctl->full[s], kb * BK, t.p ^ acc, t.ct * TN, 0);
             const int e0 = 16 * (g.nb - 1) - 16 * t.mb + 8 * kb;   // X = -(m0 - s0) / 8
             tma::bulk_load(smem + A_OFF + s * A_PITCH, tk + (size_t)e0 * (CM / 2), A_BYTES, &ctl->full[s]);
@@ -430,7 +430,8 @@ int launch_conv(const CUtensorMap& tmH, const bf16* tab, const float* hist, cons
   const cudaError_t e = allow_smem((const void*)full_conv_f32_umma_kernel<TN>, smem_bytes<TN>(), limit);
   if (e != cudaSuccess) return (int)e;
   const int sms = device_sm_count(), tiles = (g.nb - g.mb_first) * g.n_ct * 2 * g.K;
-  full_conv_f32_umma_kernel<TN><<<tiles < sms ? tiles : sms, THREADS, smem_bytes<TN>(), st>>>(tmH, tab, hist, phi, U, g, status, 2000000000ull);
+  full_conv_f32_umma_kernel<TN><<<tiles < sms ? tiles : sms, THREADS, smem_bytes<TN>(), st>>>(tmH, tab, hist, phi, U, g, status, (int)take_dropped_stage(),
+                                                                                                            wait_bound_ns());
   STU_CHECK_LAUNCH();
   return STU_OK;
 }

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     full_step_umma_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmT, const bf16* __restrict__ x,
                           long long x_rstride, const bf16* __restrict__ nw, float eps, bf16* __restrict__ hist, const bf16* __restrict__ taps,
                           int* __restrict__ pos, bf16* __restrict__ U, int B, int d, int K, int Lh, int limit, int both,
-                          int stages, int* __restrict__ status, unsigned long long wait_ns) {
+                          int stages, int* __restrict__ status, int drop_first_stage, unsigned long long wait_ns) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int K8 = (K + 7) & ~7, stage = stage_bytes(K8);
@@ -125,9 +125,11 @@ __global__ void __launch_bounds__(THREADS, 2)
         uint64_t* bar = it == n - 1 ? &ctl->last : &ctl->full[s];
         tma::mbar_expect_tx(bar, A_BYTES + 2 * K * BK * 2);
         const int e0 = it * BK;
-        load_2d(a, &tmH, bar, e0, (b * d + i0) * 2);
-        load_2d(a + A_BYTES, &tmT, bar, (oE & ~7) + e0, (oE & 7) * 2 * K);
-        load_2d(a + A_BYTES + K8 * BK * 2, &tmT, bar, (oQ & ~7) + e0, (oQ & 7) * 2 * K + K);
+        if (!(drop_first_stage && it == 0)) {   // (a test: these copies are never issued)
+          load_2d(a, &tmH, bar, e0, (b * d + i0) * 2);
+          load_2d(a + A_BYTES, &tmT, bar, (oE & ~7) + e0, (oE & 7) * 2 * K);
+          load_2d(a + A_BYTES + K8 * BK * 2, &tmT, bar, (oQ & ~7) + e0, (oQ & 7) * 2 * K + K);
+        }
       }
       __syncwarp();
       if (++s == stages) s = 0, ph ^= 1u;
@@ -289,7 +291,7 @@ extern "C" int stu_full_decode_step_tc5(const void* x, long long x_rstride, cons
   const int tiles = B * (d / CH), stages = tiles > device_sm_count() ? 4 : MAX_STAGES;
   e = launch_maybe_overlapped(full_step_umma_kernel, dim3(tiles), dim3(THREADS), smem_bytes((K + 7) & ~7, stages), (cudaStream_t)stream, true, h, tp,
                               (const bf16*)x, x_rstride, (const bf16*)norm_w, eps, (bf16*)hist, (const bf16*)taps8, pos, (bf16*)U, B, d, K, Lh, limit,
-                              both_signs, stages, status, 2000000000ull);
+                              both_signs, stages, status, (int)take_dropped_stage(), wait_bound_ns());
   if (e != cudaSuccess) return (int)e;
   STU_CHECK_LAUNCH();
   return STU_OK;

@@ -86,13 +86,13 @@ def status_word(device) -> torch.Tensor:
 
 
 STATUS_TEXT = {1: "token id outside the vocabulary", 2: "position outside the cache capacity (seq_len)",
-               3: "a bounded mbarrier wait ran out inside the tcgen05 GEMM", 4: "more top-k ties than the candidate list holds and the vocabulary does not fit in shared memory",
+               3: "a bounded mbarrier wait ran out inside a tcgen05 GEMM", 4: "more top-k ties than the candidate list holds and the vocabulary does not fit in shared memory",
                5: "top_p without top_k (<= 1024) needs the vocabulary row in shared memory (at most 51712 entries)",
                6: "decode step told that all sequences share one position, but the cached positions differ",
                7: "a bounded pipeline wait ran out inside the decode kernel",
                8: "a token step found no history sums for its position in its workspace (fused token-step kernel, or a captured step "
                   "whose sums are computed beside the step before)",
-               9: "a bounded pipeline wait ran out inside the tcgen05 prefill convolution",
+               9: "a bounded pipeline wait ran out inside a tcgen05 kernel of the STU (prefill convolutions, the full variant's token step)",
                10: "a tensor-parallel rank waited in vain for another rank's sub-layer output",
                11: "tcgen05 attention prefill: a bounded wait ran out, or a sequence was not at position 0",
                12: "a bounded wait ran out inside the token-step kernel"}

@@ -37,9 +37,9 @@ int stu_b200_version(void);
 int stu_set_status_word(int* device_status);
 
 /* Failure-detection test hook (no counterpart in the reference): arms ONE injected fault for the next tcgen05 GEMM
- * launched by stu_linear -- the copies of its first pipeline stage are never issued -- and shortens every bounded
- * device-side wait to wait_ms milliseconds.  That launch must report status 3 and return; the GPU context stays
- * usable.  wait_ms = 0 disarms and restores the two-second bound. */
+ * launched by stu_linear, stu_full_conv_f32_tc5 or stu_full_decode_step_tc5 -- its first pipeline stage is never filled -- and shortens every
+ * bounded device-side wait of theirs to wait_ms milliseconds.  That launch must report status 3 (GEMM) or 9 and return; the GPU context
+ * stays usable.  wait_ms = 0 disarms and restores the two-second bound. */
 int stu_test_inject_wait_expiry(int wait_ms);
 
 /* y[r,:] = x[r,:] * rsqrt(mean(x[r,:]^2) + eps) * w.

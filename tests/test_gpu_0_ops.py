@@ -362,6 +362,76 @@ def test_bounded_wait_expiry_of_single_ctas():
     ops.check_status()
 
 
+def _gives_up(call, status):
+    """The next launch never has its first stage: it returns within its shortened bound and says so."""
+    import time
+    from flash_stu_2_b200 import _lib, ops
+    lib = _lib.load()
+    ops.check_status()
+    assert lib.stu_test_inject_wait_expiry(100) == 0
+    try:
+        t0 = time.monotonic()
+        call()
+        torch.cuda.synchronize()
+        assert time.monotonic() - t0 < 5.0
+        with pytest.raises(RuntimeError, match=f"status {status}"):
+            ops.check_status()
+    finally:
+        assert lib.stu_test_inject_wait_expiry(0) == 0
+
+
+@pytest.mark.parametrize("shape", [(2500, 1000, 96), (100, 96, 4096), (300, 2000, 512)])
+def test_bounded_wait_expiry_of_the_fp32_gemm(shape):
+    """Two blocks of K, K split over a cluster of which one CTA gives up, eight blocks: nothing is stored by a cluster that lacks a part, and the next call is
+    correct."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    g = torch.Generator(device=dev()).manual_seed(23)
+    x, W = torch.randn(M, K, device=dev(), generator=g), torch.randn(N, K, device=dev(), generator=g)
+    want, out = ops.linear(x, W), torch.full((M, N), 7.0, device=dev())
+    _gives_up(lambda: ops.linear(x, W, out=out), 3)
+    assert bool((out == 7.0).all())
+    assert torch.equal(ops.linear(x, W, out=out), want)
+    ops.check_status()
+
+
+def test_bounded_wait_expiry_of_the_fp32_convolutions():
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(24)
+    hist, phi = torch.randn(2, 8, 2, 256, device=dev()), torch.randn(500, 3, device=dev())
+    U = [torch.empty(2 * 500, 2 * 3 * 8, device=dev()) for _ in range(3)]
+    ops.full_conv_f32_tc5(hist, phi, U[0], True, 0, 500)
+    _gives_up(lambda: ops.full_conv_f32_tc5(hist, phi, U[1], True, 0, 500), 9)
+    ops.full_conv_f32_tc5(hist, phi, U[2], True, 0, 500)
+    ops.check_status()
+    assert torch.equal(U[0], U[2])
+
+
+@pytest.mark.parametrize("t", [100, 1001])
+def test_bounded_wait_expiry_of_the_full_variants_step(monkeypatch, t):
+    """One stage (the position's) and more stages than the ring holds."""
+    from flash_stu_2_b200 import ops
+    monkeypatch.setattr(ops, "full_decode_step_tc5_pays", lambda *a: True)
+    torch.manual_seed(25)
+    B, d, K, Lh = 2, 64, 24, 512
+    hist, x, w = (torch.randn(*s, device=dev()).bfloat16() for s in ((B, d, 2, Lh), (B, d), (d,)))
+    phi = (torch.randn(2 * Lh, K, device=dev()) / 4).bfloat16()
+    taps8 = ops.taps_rev8(torch.cat([ops.taps_even(phi, Lh), ops.taps_even(phi[1:], Lh)]))
+    pos = torch.zeros(B, 2, dtype=torch.int32, device=dev())
+
+    def step():
+        pos[:, 0] = t
+        U = torch.full((B, 2 * K * d), 7.0, device=dev()).bfloat16()
+        ops.full_decode_step(x, w, ops.RMS_EPS, hist, taps8, pos, U, 2 * Lh, True, t)
+        return U
+
+    want, given_up = step(), []
+    _gives_up(lambda: given_up.append(step()), 9)
+    assert bool((given_up[0] == 7.0).all()) and pos[:, 1].tolist() == [0] * B
+    assert torch.equal(step(), want) and pos.tolist() == [[t + 1, 0]] * B
+    ops.check_status()
+
+
 def test_linear_fused_norm_decode():
     """RMSNorm fused into the mma.sync token-step linears (every row count up to 64; callers use it up to 16 rows)."""
     from flash_stu_2_b200 import ops
