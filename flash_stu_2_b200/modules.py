@@ -278,7 +278,7 @@ class STU(nn.Module):
         Lh = hist.shape[3]
         ops.to_history(xn, hist, t0)
         U = torch.empty(B * T, nsign * K * d, dtype=xn.dtype, device=xn.device)
-        if ops.full_conv_f32_tc5_pays(hist, t0 + T):
+        if xn.dtype == torch.float32 and ops.full_conv_f32_tc5_pays(B, d, K, t0, t0 + T):
             ops.full_conv_f32_tc5(hist, phi, U, nsign == 2, t0, t0 + T)
         elif xn.dtype == torch.float32:
             ops.full_conv(hist, phi, U, nsign == 2, t0, t0 + T)

@@ -39,6 +39,7 @@ BACKEND_AUTO, BACKEND_SIMT, BACKEND_TCGEN05, BACKEND_SKINNY = 0, 1, 2, 3
 RMS_EPS = float(torch.finfo(torch.float32).eps)  # what torch.nn.RMSNorm(eps=None) resolves to
 
 _status = {}
+_sms = {}
 launch_count = 0  # kernels launched through this module (bench.py reports it)
 
 
@@ -635,12 +636,41 @@ def full_conv_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
     _count(2)
 
 
-def full_conv_f32_tc5_pays(hist, t_end: int) -> bool:
-    """Whether full_conv_f32_tc5 takes less time than full_conv: tiles of 128 positions of a parity and 64 or 128 channels have to be worth
-    more than its second launch.  us, full_conv and this, 24 filters: 1 x 8 channels of 500 positions 16 and 15, 1 x 512 of 300 50 and 39,
-    1 x 256 of 300 28 and 28, 2 x 32 of 300 12 and 15, 8 x 64 of 200 29 and 24, 2 x 512 of 60 18 and 29."""
-    B, d, _, _ = hist.shape
-    return hist.dtype == torch.float32 and d % 4 == 0 and (t_end >= 400 or (t_end >= 200 and B * d >= 512))
+def sm_count() -> int:
+    """SMs of the current device (before there is one: a B200's)."""
+    if not torch.cuda.is_initialized():
+        return 148
+    dev = torch._C._cuda_getDevice()
+    if dev not in _sms:
+        _sms[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
+    return _sms[dev]
+
+
+def full_conv_f32_tc5_pays(B: int, d: int, K: int, t0: int, t_end: int) -> bool:
+    """Whether full_conv_f32_tc5 takes less time than full_conv for outputs t0 .. t_end - 1 of fp32 histories [B, d].  Both are waves of tiles: of 64 entries
+    of both parities and 32 (16) channels, 1.3 us per 32 entries where the SMs have three tiles each and 1.6 for one, and of 128 entries of a parity
+    and 128 (64) channels, 1.1 (0.9) us per 64 entries, behind a launch that splits the operands.  Fitted to 5461 calls of 1 to 32 sequences,
+    4 to 1024 channels, 1 to 32 filters and up to 6000 positions: half a percent of them are taken and more than 3 % slower (at most 1.26), where the positions
+    alone decided it was a ninth (up to 1.7: 4 x 144 channels of 219 positions, one filter, 10.8 us and 15.8)."""
+    rows, hi, lo, sms = B * d, (t_end + 1) // 2, t0 // 2, sm_count()
+    if d % 4 or not (t_end >= 400 or (t_end >= 200 and rows >= 512)):
+        return False
+    # tensor cores: tiles of the last block come first, the SM with one more than the others has about the mean of first and last
+    blocks, wide = -(-hi // 128), rows > 64
+    per_block = -(-rows // (128 if wide else 64)) * 2 * K
+    tiles = (blocks - lo // 128) * per_block
+    waves = -(-tiles // sms)
+    last = blocks - 1 - (waves - 1) * sms // per_block
+    stages = waves * (2 * (blocks - 1 + last) + 4)
+    tensor = 7.15 + stages * (1.09 + 0.067 * min(tiles, sms) / sms if wide else 0.907) + (2.67 * waves if wide else 0.0) \
+        + 12.5e-6 * (384 * blocks * K + rows * hi / 4)
+    # CUDA cores
+    channels, tall = (16 if rows <= 16 else 32), -(-(hi - lo) // 64)
+    columns = K * -(-rows // channels)
+    steps = columns * ((tall - 1) * -(-lo // 32) + tall * (tall - 1) + -(-hi // 32) + tall)
+    longest = -(-hi // 32)
+    cores = 3.5 + max(1.6 * longest, (0.79 if rows <= 16 else 1.3) * steps / sms + 0.85 * longest)
+    return tensor < 0.98 * cores
 
 
 def full_conv_f32_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):

@@ -254,3 +254,11 @@ def test_a_prefill_calls_another_modules_sub_layers(monkeypatch):
     x = torch.randn(2, 5, 8)
     y, entry = layer(x.clone(), use_cache=True)
     assert torch.equal(y, 2 * (x + 2 * x)) and entry == "entry"
+
+
+@pytest.mark.parametrize("B,d,K,t0,t_end,pays", [(8, 64, 24, 0, 1000, True), (4, 512, 24, 0, 600, True), (8, 96, 16, 0, 2048, True), (4, 144, 1, 0, 219, False),
+                                                 (8, 16, 1, 0, 415, False), (1, 988, 4, 265, 266, False), (3, 36, 4, 0, 867, False), (1, 16, 24, 0, 2000, True),
+                                                 (2, 66, 24, 0, 2000, False), (8, 64, 24, 0, 199, False)])
+def test_which_kernel_takes_the_full_variants_fp32_convolutions(B, d, K, t0, t_end, pays):
+    from flash_stu_2_b200 import ops
+    assert ops.full_conv_f32_tc5_pays(B, d, K, t0, t_end) is pays
