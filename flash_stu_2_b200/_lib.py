@@ -57,6 +57,7 @@ _SIGNATURES = {
     "stu_linear_split": ([_P, _LL, _P, _LL, _LL, _P, _P, _LL, _P, _LL, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                           _P, c_float, c_int, c_int, _P, _LL, _P], c_int),
     "stu_linear_workspace_elems": ([c_int, c_int, c_int, c_int, c_int], c_longlong),
+    "stu_linear_launches": ([], c_int),
     "stu_linear_can_fuse_norm": ([c_int, c_int, c_int, c_int, c_int], c_int),
     "stu_linear_tile_cost": ([c_int, c_int], c_longlong),
     "stu_taps_even": ([_P, _P, c_int, c_int, c_int, c_int, _P], c_int),

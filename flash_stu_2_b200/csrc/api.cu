@@ -35,6 +35,9 @@ extern "C" int stu_set_programmatic_launch(int on) {
 int device_sm_count();   // gemm_tc.cu
 bool skinny_umma_takes(int M, int N, int K, int epi, bool norm, bool peer);   // gemm_tc.cu
 
+thread_local int t_linear_launches = 0;   // (gemm_tc.cu: 2 for a product whose K is cut)
+extern "C" int stu_linear_launches(void) { return t_linear_launches; }
+
 // Small-M shapes for which the tcgen05 GEMM beats the weight-streaming kernel.
 static bool prefers_tensor_gemm(int M, int N) { return (M >= 32 && N >= 5120) || (M >= 16 && N >= 32768); }
 
@@ -43,6 +46,7 @@ extern "C" int stu_linear_split(const void* x, long long x_row_stride, const voi
                                 void* y, long long y_row_stride, int M, int N, int K, int epilogue, int hist_T,
                                 int hist_t0, int hist_Lh, const void* norm_w, float eps, int dtype, int backend,
                                 float* workspace, long long workspace_elems, void* stream) {
+  t_linear_launches = 1;
   if (!x || !W || !y) return STU_ERR_NULL;
   if (M < 0 || N <= 0 || K <= 0) return STU_ERR_SHAPE;
   if (M == 0) return STU_OK;

@@ -29,6 +29,7 @@
 
 int device_sm_count();   // SM count of the current device (cached per device)
 static int current_device();
+extern thread_local int t_linear_launches;   // api.cu: kernels of this thread's last linear
 
 namespace cg = cooperative_groups;
 
@@ -951,6 +952,7 @@ int launch_tc(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2,
                                 split.whole, split.parts, M, N, tiles_m, tiles_n, group_m, ep);
     if (e != cudaSuccess) return (int)e;
     STU_CHECK_LAUNCH();
+    t_linear_launches = 2;
   }
   return STU_OK;
 }

@@ -272,8 +272,8 @@ PyObject* layer_step_f32(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, eps, mlp_eps, t0, fresh, kind, status): new positions of an
 // approx layer, in place on x [B, T, d]: x += STU(norm(x)); x += MLP(norm(x)), seven launches.  kind and taps as in
-// stu_conv_prefill_positions; pos may be None.  Returns 3, or 1 where the MLP was refused (the STU is done), or None where the STU was
-// (x is as it was, and so are the positions).
+// stu_conv_prefill_positions; pos may be None.  Returns 3 (7: the last product took two launches), or 1 where the MLP was refused (the STU
+// is done), or None where the STU was (x is as it was, and so are the positions).
 PyObject* layer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 16) {
     PyErr_SetString(PyExc_TypeError, "16 arguments expected");
@@ -328,7 +328,7 @@ PyObject* layer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
       rc = stu_linear_split(ph, I, p[9], I, 1, nullptr, p[0], d, p[0], d, M, (int)d, (int)I, 1, 0, 0, 0, nullptr, 0.f, code, 0, pw, parts, stream);
     Py_END_ALLOW_THREADS
     if (raised(rc, "layer_prefill")) return nullptr;
-    if (rc == 0) done = 3;
+    if (rc == 0) done = stu_linear_launches() == 2 ? 7 : 3;
     if (done) return PyLong_FromLong(done);
   } catch (const BadArgument&) {
     PyErr_Clear();
@@ -365,6 +365,7 @@ PyMethodDef methods[] = {
     ENTRY(stu_lds_final_state),
     ENTRY(stu_linear),
     ENTRY(stu_linear_can_fuse_norm),
+    ENTRY(stu_linear_launches),
     ENTRY(stu_linear_tile_cost),
     ENTRY(stu_linear_push),
     ENTRY(stu_peer_combine),

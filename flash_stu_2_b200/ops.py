@@ -215,7 +215,7 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
         # checks, output and launch in one native call; None: whatever is out of the ordinary is looked at below
         y = _lib.native().linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed_weight, hist_T, hist_t0, hist_Lh)
         if y is not None:
-            _count()
+            _count(1 if x.shape[0] <= 64 else _lib.native().stu_linear_launches())   # (two where K is cut: more rows than a token step's)
             return y
     _cuda(x, W, W2, resid, out, norm_w)
     assert x.dim() == 2 and W.dim() == 2 and x.stride(1) == 1
@@ -390,8 +390,8 @@ def layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, 
                                        status_word(x.device))
     if done is None:
         return 0
-    _count(7 if done == 3 else 4)
-    return done
+    _count({1: 4, 3: 7, 7: 8}[done])
+    return done & 3
 
 
 def decode_approx_shard(x, norm_w, MinT, hist, taps8, pos, out, eps: float = RMS_EPS, add_residual: bool = False,

@@ -85,6 +85,8 @@ int stu_linear(const void* x, long long x_row_stride, const void* W, long long w
                int M, int N, int K, int epilogue, int hist_T, int hist_t0, int hist_Lh, const void* norm_w,
                float eps, int dtype, int backend, void* stream);
 int stu_linear_can_fuse_norm(int M, int N, int K, int epilogue, int dtype);
+/* Kernels that the calling thread's last stu_linear or stu_linear_split launched: 1, or 2 where K was cut. */
+int stu_linear_launches(void);
 /* Time of the tcgen05 GEMM's tiles for M x N plain outputs, in hundredths of a wave of its smallest ones (per k-block): for callers that
  * choose how many rows a product has.  No counterpart in the reference. */
 long long stu_linear_tile_cost(int M, int N);

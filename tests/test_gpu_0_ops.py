@@ -602,6 +602,20 @@ def test_linear_of_long_weights_in_parts(shape, epi):
         assert rc == rc2 == 0 and torch.equal(short, whole) and bool(work.isnan().all())
 
 
+@pytest.mark.parametrize("shape,launches", [((333, 1536, 6144), 2), ((65, 64, 24576), 2), ((333, 1536, 512), 1), ((64, 64, 24576), 1)])
+def test_launches_of_a_linear_are_counted(shape, launches):
+    """A product whose K is cut is added up in a launch of its own; on the CUDA cores (asked for, or rows that the tensor cores do not take) it is one launch."""
+    from flash_stu_2_b200 import _lib, ops
+    M, N, K = shape
+    assert (_lib.load().stu_linear_workspace_elems(M, N, K, 0, 1) > 0) == (launches == 2)
+    x, W = torch.ones(M, K, device=dev(), dtype=torch.bfloat16), torch.ones(N, K, device=dev(), dtype=torch.bfloat16)
+    odd = torch.ones(M, K + 1, device=dev(), dtype=torch.bfloat16)[:, :K]   # rows off the 16-byte grid: not on the tensor cores
+    for rows, backend, want in ((x, 0, launches), (x, 1, 1), (odd, 0, 1), (x, 0, launches)):
+        before = ops.launch_count
+        ops.linear(rows, W, backend=backend)
+        assert ops.launch_count - before == want
+
+
 @pytest.mark.parametrize("shape", [(8, 1024, 49152), (1, 640, 14720), (5, 768, 12296), (7, 1200, 4104), (8, 2049, 4096), (3, 4735, 8192)])
 @pytest.mark.parametrize("epi", [0, 1])
 @pytest.mark.parametrize("early", [False, True])

@@ -498,3 +498,25 @@ def test_prefill_in_one_native_call_equals_the_parts(dt, B, first, second, monke
             m.setattr(ops, "layer_prefill", lambda *a: 0)
             parts = run()
         assert all(torch.equal(p, q) for p, q in zip(one[:5], parts[:5])) and one[5] == parts[5] == first + second
+
+
+def test_launches_of_a_layers_prefill_are_counted(monkeypatch):
+    """In one native call as many launches are counted as in calls apart, also where the down projection takes two."""
+    import flash_stu_2_b200 as F
+    from flash_stu_2_b200 import _lib, ops
+    cfg = F.FlashSTUConfig(n_embd=64, n_layers=1, n_heads=1, seq_len=128, vocab_size=1, mlp_scale=64, num_eigh=8, torch_dtype=torch.bfloat16, use_attn=False)
+    blk = F.FlashSTUBlock(config=cfg).cuda().eval()
+    with torch.no_grad():
+        blk(torch.zeros(1, 8, 64, device="cuda", dtype=torch.bfloat16))   # (the taps are laid out)
+    counts = []
+    for apart in (False, True):
+        if apart:
+            monkeypatch.setattr(ops, "layer_prefill", lambda *a: 0)
+        for T in (80, 40):   # (40: no cut)
+            before = ops.launch_count
+            with torch.no_grad():
+                blk(torch.zeros(1, T, 64, device="cuda", dtype=torch.bfloat16))
+            counts.append(ops.launch_count - before)
+    ops.check_status()
+    assert _lib.load().stu_linear_workspace_elems(80, 64, 4096, 1, 1) > 0
+    assert counts[:2] == counts[2:] and counts[0] == counts[1] + 1
