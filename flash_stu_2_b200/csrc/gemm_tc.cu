@@ -1334,11 +1334,18 @@ bool gemm_tc_supported(const void* A, long long lda, const void* B, long long ld
 // 24.6, 300 x 12288 x 3072 55.6 and 51.6 (2 for 3), 1030 x 6144 x 1536 43.4 and 40.4 (3 for 4), 1030 x 12288 x 3072 127 and 137 (6 for 7: pairs);
 // plain 300 x 12288 x 4096 45.9 and 34.8, 1030 x 7680 x 2560 42.7 and 36.9, 300 x 50257 x 2560 102 and 92; residual 3661 x 2560 x 10240 196 and 152;
 // with as many waves 7996 x 4096 x 1024 gate/up 108 and 129.  (16.7, 26.6, 50.9, 41.0, 130; 34.3, 37.4, 94; 147; 120 when all tiles were single CTAs'.)
-// STU_B200_TILE_N=128 and 256 force either, STU_B200_TILE_CTAS=1 and 2 the last form or the others.
+// STU_B200_TILE_N=128 and 256 force either, STU_B200_TILE_CTAS=1 and 2 the last form or the others; with any of them no K is cut.
 enum { TILE_NARROW, TILE_WIDE, TILE_SINGLE };
+static const char* tile_n_asked() {
+  static const char* env = getenv("STU_B200_TILE_N");
+  return env;
+}
+static const char* tile_ctas_asked() {
+  static const char* env = getenv("STU_B200_TILE_CTAS");
+  return env;
+}
 static int tile_form(long long rows, long long cols, bool dual, bool single_built, long long* cost = nullptr) {
-  static const char* env_n = getenv("STU_B200_TILE_N");
-  static const char* env_c = getenv("STU_B200_TILE_CTAS");
+  const char *env_n = tile_n_asked(), *env_c = tile_ctas_asked();
   const long long pairs = device_pairs(), sms = device_sm_count(), rows2 = (rows + 2 * BM - 1) / (2 * BM);
   const auto waves = [](long long tiles, long long at_a_time) { return (tiles + at_a_time - 1) / at_a_time; };
   const long long wide = 174 * waves(rows2 * ((cols + 255) / 256), pairs);
@@ -1370,7 +1377,7 @@ extern "C" long long stu_linear_tile_cost(int M, int N) {
 // written and read), the second launch 4; 105 products of 65 to 24000 rows, K = 512 to 98304: 0.97 (noise, not split) to 4.0 times as fast.
 static SplitK split_plan(long long M, long long N, long long K) {
   SplitK s = {0, 1, nullptr};
-  if (M <= 64 || K < 1024) return s;   // token steps' kernels, or never worth it
+  if (M <= 64 || K < 1024 || tile_n_asked() || tile_ctas_asked()) return s;   // token steps' kernels, never worth it, or another form asked for
   const long long tiles = (M + 255) / 256 * ((N + 255) / 256), pairs = device_pairs(), kb = (K + BK - 1) / BK, rest = tiles % pairs;
   if (rest == 0) return s;
   long long cost = 0;

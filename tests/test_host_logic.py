@@ -262,3 +262,17 @@ def test_a_prefill_calls_another_modules_sub_layers(monkeypatch):
 def test_which_kernel_takes_the_full_variants_fp32_convolutions(B, d, K, t0, t_end, pays):
     from flash_stu_2_b200 import ops
     assert ops.full_conv_f32_tc5_pays(B, d, K, t0, t_end) is pays
+
+
+def test_a_tile_form_that_is_asked_for_cuts_no_k():
+    """The environment is read once, so each setting has a process of its own."""
+    import os
+    import subprocess
+    import sys
+    from flash_stu_2_b200 import _build
+    code = ("import ctypes, sys; f = ctypes.CDLL(sys.argv[1]).stu_linear_workspace_elems; f.restype = ctypes.c_longlong; "
+            "print(f(333, 1536, 6144, 0, 1))")
+    env = {k: v for k, v in os.environ.items() if not k.startswith("STU_B200_TILE")}
+    for asked in ({}, {"STU_B200_TILE_N": "128"}, {"STU_B200_TILE_N": "256"}, {"STU_B200_TILE_CTAS": "1"}, {"STU_B200_TILE_CTAS": "2"}):
+        out = subprocess.run([sys.executable, "-c", code, _build.build_library()], env={**env, **asked}, capture_output=True, text=True, check=True).stdout
+        assert (int(out) == 0) is bool(asked), asked
