@@ -714,8 +714,8 @@ def full_decode_step_tc5_pays(batch: int, d: int, K: int, t: int) -> bool:
     11.0; 32 filters, at 600 13.9 and 9.3; 16 x 1024, 8 filters, at 300 10.7 and 8.6.  4 x 1024 at 4000, 24 filters: 14.2 and 15.5."""
     if d % 64 or K > 32:
         return False
-    ctas = batch * (d // 64)
-    return ctas > 148 or (ctas >= 74 and t >= (3000, 3000, 1500, 500)[(K + 7) // 8 - 1])
+    ctas, sms = batch * (d // 64), sm_count()
+    return ctas > sms or (2 * ctas >= sms and t >= (3000, 3000, 1500, 500)[(K + 7) // 8 - 1])
 
 
 def full_decode_step(x2d, norm_w, eps: float, hist, taps8, pos, U, limit: int, both_signs: bool, t: int = 0):

@@ -276,3 +276,11 @@ def test_a_tile_form_that_is_asked_for_cuts_no_k():
     for asked in ({}, {"STU_B200_TILE_N": "128"}, {"STU_B200_TILE_N": "256"}, {"STU_B200_TILE_CTAS": "1"}, {"STU_B200_TILE_CTAS": "2"}):
         out = subprocess.run([sys.executable, "-c", code, _build.build_library()], env={**env, **asked}, capture_output=True, text=True, check=True).stdout
         assert (int(out) == 0) is bool(asked), asked
+
+
+@pytest.mark.parametrize("sms,batch,t,pays", [(148, 9, 0, False), (132, 9, 0, True), (148, 4, 5000, False), (132, 4, 5000, False), (128, 4, 5000, True), (148, 5, 5000, True), (162, 5, 5000, False)])
+def test_the_full_variants_step_asks_how_many_sms_there_are(monkeypatch, sms, batch, t, pays):
+    """16 CTAs per sequence: more than there are SMs, or half of them and more from position 1500 on (24 filters)."""
+    from flash_stu_2_b200 import ops
+    monkeypatch.setattr(ops, "sm_count", lambda: sms)
+    assert ops.full_decode_step_tc5_pays(batch, 1024, 24, t) is pays
