@@ -363,14 +363,14 @@ struct Operands {
   int M, N, K, causal;
 };
 
-// How many clusters of KS CTAs the GPU holds at a time (the SMs of a GPC are no multiple of 8: 8 leave some of them out)
+// How many clusters of KS CTAs the GPU holds at a time (the SMs of a GPC are no multiple of 8: 8 leave some of them out); 0: none, or it cannot say now
 template <int EPI, int KS, int BN>
 int clusters_at_once() {
   static std::atomic<int> known[STU_MAX_DEVICES] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= STU_MAX_DEVICES) dev = 0;
   int n = KS == 1 ? device_sm_count() : known[dev].load(std::memory_order_relaxed);
-  if (n > 0) return n;
+  if (n != 0) return n < 0 ? 0 : n;
   auto kern = gemm_f32_umma_kernel<EPI, KS, BN>;
   static SmemLimit limit;
   cudaLaunchConfig_t cfg = {};
@@ -383,11 +383,11 @@ int clusters_at_once() {
   at.val.clusterDim.z = KS;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  if (allow_smem((const void*)kern, smem_bytes<BN>(), limit) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-    (void)cudaGetLastError();
-    n = 1;
+  if (allow_smem((const void*)kern, smem_bytes<BN>(), limit) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();   // (asked again by the next call)
+    return 0;
   }
-  known[dev].store(n, std::memory_order_relaxed);
+  known[dev].store(n > 0 ? n : -1, std::memory_order_relaxed);
   return n;
 }
 template <int EPI, int BN>
@@ -439,21 +439,29 @@ int launch_split(const Operands& o, int ks, const EpiArgs<float>& ep, cudaStream
 
 // The tile width and the split of K that take the least time: waves of clusters, a CTA per SM, of 4.2 us and 1.05, 1.5 or 1.95 us per block of
 // 64 of K (32, 64 or 128 columns), 0.8 us and a tenth per CTA of a cluster (fitted to 26 shapes of 20 to 8192 rows; within 10 % of the best of
-// all in each).
-template <int EPI>
-int launch_epi(const Operands& o, const EpiArgs<float>& ep, cudaStream_t st) {
-  const int blocks = (o.K + BK - 1) / BK;
+// all in each).  clusters(columns, ks): how many the GPU holds at a time; a split of which it holds none is not taken, and of single CTAs it holds some.
+template <typename Clusters>
+void choose_tile(int M, int N, int K, bool dual, const Clusters& clusters, int* best_bn, int* best_ks) {
+  const int blocks = (K + BK - 1) / BK;
   double best = 1e30;
-  int best_bn = 128, best_ks = 1;
+  *best_bn = 128, *best_ks = 1;
   for (int bn = 128; bn >= 32; bn /= 2)
     for (int ks = 1; ks <= 8 && (ks == 1 || blocks >= ks); ks *= 2) {
-      const int cols = EPI == EPI_GELU_MUL ? bn / 2 : bn;
-      const long long tiles = (long long)((o.M + BM - 1) / BM) * ((o.N + cols - 1) / cols);
-      const int room = bn == 128 ? clusters_at_once<EPI, 128>(ks) : bn == 64 ? clusters_at_once<EPI, 64>(ks) : clusters_at_once<EPI, 32>(ks);
+      const int cols = dual ? bn / 2 : bn, room = clusters(bn, ks);
+      if (room < 1) continue;
+      const long long tiles = (long long)((M + BM - 1) / BM) * ((N + cols - 1) / cols);
       const double block = bn == 128 ? 1.95 : bn == 64 ? 1.5 : 1.05;
       const double t = (double)((tiles + room - 1) / room) * (4.2 + (blocks + ks - 1) / ks * block + (ks > 1 ? 0.8 + 0.1 * ks : 0.0));
-      if (t < best) best = t, best_bn = bn, best_ks = ks;
+      if (t < best) best = t, *best_bn = bn, *best_ks = ks;
     }
+}
+
+template <int EPI>
+int launch_epi(const Operands& o, const EpiArgs<float>& ep, cudaStream_t st) {
+  int best_bn, best_ks;
+  choose_tile(o.M, o.N, o.K, EPI == EPI_GELU_MUL, [](int bn, int ks) {
+    return bn == 128 ? clusters_at_once<EPI, 128>(ks) : bn == 64 ? clusters_at_once<EPI, 64>(ks) : clusters_at_once<EPI, 32>(ks);
+  }, &best_bn, &best_ks);
   switch (best_bn) {
     case 32: return launch_split<EPI, 32>(o, best_ks, ep, st);
     case 64: return launch_split<EPI, 64>(o, best_ks, ep, st);
@@ -462,6 +470,13 @@ int launch_epi(const Operands& o, const EpiArgs<float>& ep, cudaStream_t st) {
 }
 
 }  // namespace
+
+// Test hook: columns * 16 + CTAs per cluster of the tiles of a product on a GPU that holds room[i] clusters of 2^i CTAs at a time.
+extern "C" int stu_test_f32_tile(int M, int N, int K, int gate_up, const int* room) {
+  int bn, ks;
+  choose_tile(M, N, K, gate_up != 0, [room](int, int of) { return room[of == 1 ? 0 : of == 2 ? 1 : of == 4 ? 2 : 3]; }, &bn, &ks);
+  return bn * 16 + ks;
+}
 
 // Both operands K-major with rows on the 16-byte grid; from 256 of K on, or from 96 where the tiles of 64 x 64 are four per SM and more (us, the
 // CUDA-core GEMM and this one: 4000 x 4096 x 64 62 and 64, x 96 87 and 74; 8000 x 96 x 96 9.2 and 10.9; 300 x 512 x 128 7.8 and 8.4).  Where

@@ -41,6 +41,8 @@ int stu_set_status_word(int* device_status);
  * bounded device-side wait of theirs to wait_ms milliseconds.  That launch must report status 3 (GEMM) or 9 and return; the GPU context
  * stays usable.  wait_ms = 0 disarms and restores the two-second bound. */
 int stu_test_inject_wait_expiry(int wait_ms);
+/* Test hook: columns * 16 + CTAs per cluster of an fp32 product's tiles where the GPU held room[i] clusters of 2^i CTAs at a time (i < 4). */
+int stu_test_f32_tile(int M, int N, int K, int gate_up, const int* room);
 
 /* y[r,:] = x[r,:] * rsqrt(mean(x[r,:]^2) + eps) * w.
  * Replaces torch.nn.RMSNorm / LigerRMSNorm as used in flash_stu/layers/stu_layer.py:32-36,67-71,

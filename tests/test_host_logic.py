@@ -284,3 +284,16 @@ def test_the_full_variants_step_asks_how_many_sms_there_are(monkeypatch, sms, ba
     from flash_stu_2_b200 import ops
     monkeypatch.setattr(ops, "sm_count", lambda: sms)
     assert ops.full_decode_step_tc5_pays(batch, 1024, 24, t) is pays
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 30, 3072), (256, 512, 6144), (1000, 1536, 512), (65, 8, 256)])
+@pytest.mark.parametrize("gate_up", [0, 1])
+def test_an_fp32_product_is_not_split_over_clusters_that_the_gpu_does_not_hold(M, N, K, gate_up):
+    import ctypes
+    from flash_stu_2_b200 import _lib
+    hook = _lib.load().stu_test_f32_tile
+    for most in range(4):   # clusters of more than 2^most CTAs: none at a time
+        room = (ctypes.c_int * 4)(*([148, 74, 33, 16][:most + 1] + [0] * (3 - most)))
+        tile = hook(M, N, K, gate_up, room)
+        assert tile // 16 in (32, 64, 128) and tile % 16 <= 2 ** most
+    assert tile % 16 == 8 or K < 3072 or M > 256   # (with all of them long K over few tiles is split eightfold)
