@@ -364,6 +364,8 @@ PyMethodDef methods[] = {
     ENTRY(stu_lds_decode_step),
     ENTRY(stu_lds_final_state),
     ENTRY(stu_linear),
+    ENTRY(stu_linear_split),
+    ENTRY(stu_linear_workspace_elems),
     ENTRY(stu_linear_can_fuse_norm),
     ENTRY(stu_linear_launches),
     ENTRY(stu_linear_tile_cost),

@@ -330,6 +330,11 @@ class FlashSTU(PreTrainedModel):
                    if hasattr(layer, "stu") and not layer.stu.use_approx)
         nbytes = (B * (6 * d + 2 * row) * (self.n_layers + 1) + B * full + B * (self.lm_head.weight.shape[0] + 64)) \
             * self.lm_head.weight.element_size() + 4096 * (self.n_layers + 1)
+        if B > 64:   # products that may cut K: the parts' sums of one at a time
+            shapes = {shape for p in self.parameters() if p.dim() == 2 for shape in (tuple(p.shape), tuple(p.shape[::-1]))}
+            shapes |= {(layer.stu.d_out, layer.stu.K * layer.stu.d_in * (1 if layer.stu.use_hankel_L else 2)) for layer in self.layers
+                       if hasattr(layer, "stu") and not layer.stu.use_approx}
+            nbytes += 4 * max(ops.linear_workspace(B, *shape, ops.EPI_RESID, self.lm_head.weight.dtype) for shape in shapes)
         buffer = torch.empty(nbytes, dtype=torch.uint8, device=tok.device)
         host_t = [getattr(e[-1], "_host_t", None) if e is not None else None for e in past]
         graph = torch.cuda.CUDAGraph()

@@ -205,13 +205,19 @@ def linear_tile_cost(rows: int, cols: int) -> int:
     return int(_lib.native().stu_linear_tile_cost(rows, cols))
 
 
+def linear_workspace(rows: int, cols: int, K: int, epilogue: int, dtype: torch.dtype) -> int:
+    """fp32 values that a product of this size keeps the parts of its sums in (0: its K is not cut)."""
+    return int(_lib.native().stu_linear_workspace_elems(rows, cols, K, epilogue, 1)) if dtype == torch.bfloat16 else 0
+
+
 def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = None,
            resid: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, epilogue: int = EPI_STORE,
            norm_w: Optional[torch.Tensor] = None, eps: float = RMS_EPS, backend: int = BACKEND_AUTO,
            transposed_weight: bool = False, hist_T: int = 0, hist_t0: int = 0, hist_Lh: int = 0,
            kpos: Optional[torch.Tensor] = None):
     """y = epilogue(x @ W^T) for x [M,K] and W [N,K] (or W [K,N] with transposed_weight=True)."""
-    if kpos is None and (out is not None or getattr(_local, "arena", None) is None):
+    pieces = getattr(_local, "arena", None)
+    if kpos is None and (pieces is None or (out is not None and x.shape[0] <= 64)):   # (more rows: K may be cut, and the workspace is a piece)
         # checks, output and launch in one native call; None: whatever is out of the ordinary is looked at below
         y = _lib.native().linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed_weight, hist_T, hist_t0, hist_Lh)
         if y is not None:
@@ -244,14 +250,19 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
         assert resid is None and epilogue == EPI_STORE and kpos.is_cuda and kpos.dtype == torch.int32
         resid, epilogue = kpos, EPI_STORE | EPI_FLAG_KPOS
     status_word(x.device)   # the tcgen05 GEMM reports an expired device-side wait through the registered word
-    rc = _lib.native().stu_linear(x.data_ptr(), x.stride(0), W.data_ptr(), w_rs, w_ks, _p(W2), _p(resid), r_rs,
-                                  out.data_ptr(), y_rs, M, N, K, epilogue, hist_T, hist_t0, hist_Lh, _p(norm_w), eps,
-                                  _dt(x), backend, _stream())
+    parts = linear_workspace(M, N, K, epilogue, x.dtype) if backend in (BACKEND_AUTO, BACKEND_TCGEN05) and w_ks == 1 else 0
+    used = pieces.used if pieces is not None else 0
+    work = empty((parts,), torch.float32, x.device) if parts else None
+    rc = _lib.native().stu_linear_split(x.data_ptr(), x.stride(0), W.data_ptr(), w_rs, w_ks, _p(W2), _p(resid), r_rs,
+                                        out.data_ptr(), y_rs, M, N, K, epilogue, hist_T, hist_t0, hist_Lh, _p(norm_w), eps,
+                                        _dt(x), backend, _p(work), parts, _stream())
+    if pieces is not None:
+        pieces.used = used   # (what takes its place is written behind this product, on the same stream)
     if rc == _lib.ERR_UNSUPPORTED and norm_w is not None and x.dtype == torch.float32 and backend == BACKEND_AUTO:
         # rows or weights off the 16-byte grid: the norm in a launch of its own, the product on the kernels that take them
         return linear(rmsnorm(x, norm_w, eps), W, W2=W2, resid=resid, out=out, epilogue=epilogue)
     _lib.check(rc, "stu_linear")
-    _count()
+    _count(_lib.native().stu_linear_launches())
     return out
 
 

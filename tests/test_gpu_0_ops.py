@@ -616,6 +616,28 @@ def test_launches_of_a_linear_are_counted(shape, launches):
         assert ops.launch_count - before == want
 
 
+@pytest.mark.parametrize("shape", [(128, 1024, 4096), (333, 1536, 6144), (65, 64, 24576)])
+@pytest.mark.parametrize("given", [False, True])
+def test_a_linear_in_parts_takes_its_workspace_from_the_arena(shape, given):
+    """The buffer that a caller gives for a captured step holds the parts of K as well, for one product at a time; the sums are those of a call outside."""
+    from flash_stu_2_b200 import _lib, ops
+    M, N, K = shape
+    torch.manual_seed(4)
+    x, W = (torch.randn(r, K, device=dev()).bfloat16() for r in (M, N))
+    parts = _lib.load().stu_linear_workspace_elems(M, N, K, 0, 1)
+    assert parts > 0
+    want = ops.linear(x, W)
+    room = (2 * M * N + 255) // 256 * 256
+    buffer = torch.empty(4 * parts + 3 * room, dtype=torch.uint8, device=dev())
+    outs = [torch.empty_like(want) for _ in range(3)] if given else [None] * 3
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    with ops.arena(buffer):
+        got = [ops.linear(x, W, out=out) for out in outs]
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+    ops.check_status()
+    assert all(torch.equal(g, want) for g in got)
+
+
 @pytest.mark.parametrize("shape", [(8, 1024, 49152), (1, 640, 14720), (5, 768, 12296), (7, 1200, 4104), (8, 2049, 4096), (3, 4735, 8192)])
 @pytest.mark.parametrize("epi", [0, 1])
 @pytest.mark.parametrize("early", [False, True])

@@ -364,6 +364,43 @@ def test_the_three_forms_of_the_token_loop_agree(monkeypatch, dt, kw):
         close(logits[:, :same], eager_logits[:, :same], 2e-2)
 
 
+@pytest.mark.parametrize("approx", [True, False])
+def test_a_captured_step_of_many_sequences_keeps_its_parts_in_its_buffer(monkeypatch, approx):
+    """80 sequences and long products (the down projection; without approx the contraction of all filters): K is cut, the parts' place is
+    in the step's buffer, and the logits are those of the eager loop.  (What capturing does allocate is an attention's output and two words.)"""
+    import flash_stu_2_b200 as F
+    from flash_stu_2_b200 import _lib, ops
+    torch.manual_seed(3)
+    cfg = F.FlashSTUConfig(n_embd=256, n_layers=2, n_heads=4, seq_len=64, window_size=40, vocab_size=1003, mlp_scale=16, num_eigh=8,
+                           torch_dtype=torch.bfloat16, use_approx=approx)
+    with torch.device(dev()):
+        m = F.FlashSTU(cfg).eval()
+    with torch.no_grad():
+        for name, p in m.named_parameters():
+            if not name.endswith("norm.weight"):
+                p.normal_(0.0, 0.5 * p.shape[-1] ** -0.5)
+    parts = _lib.load().stu_linear_workspace_elems(80, 256, 4096, 1, 1)
+    assert parts > 0
+    allocated = []
+
+    class Counted(ops.arena):
+        def __enter__(self):
+            allocated.append(torch.cuda.memory_stats()["requested_bytes.all.allocated"])
+            return super().__enter__()
+
+        def __exit__(self, *exc):
+            allocated.append(torch.cuda.memory_stats()["requested_bytes.all.allocated"])
+            return super().__exit__(*exc)
+
+    monkeypatch.setattr(ops, "arena", Counted)
+    prompt = torch.randint(0, 1003, (80, 5), device=dev())
+    ids, logits = m.generate(prompt, max_length=13, do_sample=False, return_logits=True)
+    assert len(allocated) == 2 and allocated[1] - allocated[0] < 4 * parts
+    eager_ids, eager_logits = m.generate(prompt, max_length=13, do_sample=False, return_logits=True, cuda_graph=False)
+    ops.check_status()
+    assert torch.equal(ids, eager_ids) and torch.equal(logits, eager_logits)
+
+
 @pytest.mark.parametrize("B,T0,new,sms", [(17, 30, 34, 9), (19, 1, 63, 40), (32, 33, 12, 148)])
 def test_streams_beside_the_captured_step(monkeypatch, B, T0, new, sms):
     """The captured step with its STU layers' history sums on a branch of their own draws the same tokens from the same logits as the
