@@ -564,6 +564,37 @@ def test_fp32_linear_on_tensor_cores(shape, epi):
     assert err[0] <= max(err[1], 2.0 ** -24), err
 
 
+# The largest second and third parts, of one sign: what the six products leave out of each is 2^-23.03 of it, and adds up
+WORST = 1 + 2.0 ** -8 - 2.0 ** -23
+
+
+@pytest.mark.parametrize("shape", [(640, 512, 256), (129, 96, 1024), (300, 640, 3072)])
+@pytest.mark.parametrize("signs", [(1, 1), (-1, 1), (-1, -1)])
+def test_fp32_linear_on_tensor_cores_largest_parts(shape, signs):
+    """Bar: 2^-23 for what is left out, as much for either of the two instructions with an accumulator's largest products (their sums are cut off), and half an ulp
+    for each of the K / 32 accumulators that are added up."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    x, W = torch.full((M, K), signs[0] * WORST, device=dev()), torch.full((N, K), signs[1] * WORST, device=dev())
+    err = [float((ops.linear(x, W, backend=b).double() / (signs[0] * signs[1] * K * WORST ** 2) - 1).abs().max()) for b in (0, 1)]
+    ops.check_status()
+    assert err[0] <= (3 + K / 64) * 2.0 ** -23, err
+
+
+@pytest.mark.parametrize("B,T,d,K", [(2, 900, 64, 3), (1, 513, 132, 2)])
+def test_full_variant_fp32_convolutions_of_the_largest_parts(B, T, d, K):
+    """As above with an accumulator for 64 positions of a parity, and one sum of the two parities' sums."""
+    from flash_stu_2_b200 import ops
+    Lh = (T // 2 + 8) // 8 * 8
+    hist, phi = torch.full((B, d, 2, Lh), WORST, device=dev()), torch.full((T, K), WORST, device=dev())
+    U = torch.full((B * T, K * d), float("nan"), device=dev())
+    ops.full_conv_f32_tc5(hist, phi, U, False, 0, T)
+    ops.check_status()
+    terms = torch.arange(1, T + 1, device=dev(), dtype=torch.float64).view(1, T, 1)
+    err = (U.double().view(B, T, K * d) / (terms * WORST ** 2) - 1).abs()
+    assert bool((err <= (4 + 2 * math.ceil(T / 128)) * 2.0 ** -23).all()), float(err.max())
+
+
 # (rows, outputs, K, distance of the outputs' rows): one tile in parts of unequal length, edges of tiles, odd row strides, whole tiles ahead of the split ones
 @pytest.mark.parametrize("shape", [(65, 64, 24576, 64), (257, 513, 12296, 513), (333, 1536, 6144, 1540), (70, 1030, 49152, 1033), (140, 1001, 8200, 1002),
                                    (5193, 1000, 4096, 1000), (19851, 512, 3072, 512)])
