@@ -102,8 +102,8 @@ extern "C" int stu_linear_split(const void* x, long long x_row_stride, const voi
     if (sk_ok && tc_ok && prefers_tensor_gemm(M, N) && !skinny_umma_takes(M, N, K, epilogue, false, false))
       sk_ok = false;
     backend = sk_ok ? BACKEND_SKINNY : (tc_ok ? BACKEND_TCGEN05 : BACKEND_SIMT);
-    if (backend == BACKEND_SIMT && gemm_f32_umma_takes(x, x_row_stride, W, w_row_stride, w_k_stride, W2, M, N, K, epilogue, dtype))
-      return gemm_f32_umma_dispatch(x, x_row_stride, W, w_row_stride, W2, M, N, K, epilogue, causal, ep, st);
+    if (backend == BACKEND_SIMT && gemm_f32_umma_takes(x, x_row_stride, W, w_row_stride, w_k_stride, W2, M, N, K, causal, dtype))
+      return gemm_f32_umma_dispatch(x, x_row_stride, W, w_row_stride, W2, M, N, K, epilogue, ep, st);
   }
   switch (backend) {
     case BACKEND_SKINNY:

@@ -90,9 +90,9 @@ __device__ __forceinline__ void epilogue_store(const EpiArgs<T>& ep, int m, int 
 int gemm_simt_dispatch(const void* A, long long lda, const void* B, long long ldb, long long skb, const void* B2,
                        int M, int N, int K, int epi, int causal, const EpiArgsAny& ep, int dtype, cudaStream_t st);
 int gemm_f32_umma_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N, int K, int epi,
-                           int causal, const EpiArgsAny& ep, cudaStream_t st);
+                           const EpiArgsAny& ep, cudaStream_t st);
 bool gemm_f32_umma_takes(const void* A, long long lda, const void* B, long long ldb, long long skb, const void* B2, int M, int N, int K,
-                         int epi, int dtype);
+                         int causal, int dtype);
 int gemm_tc_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N,
                      int K, int epi, int causal, const EpiArgsAny& ep, cudaStream_t st, float* workspace = nullptr,
                      long long workspace_elems = 0);

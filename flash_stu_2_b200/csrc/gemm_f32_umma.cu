@@ -134,7 +134,7 @@ __device__ __noinline__ void sums_again(const float* A, long long lda, int rows,
 template <int EPI, int KS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_f32_umma_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ B, long long ldb,
-                         const float* __restrict__ B2, int M, int N, int K, int causal, EpiArgs<float> ep, int* status,
+                         const float* __restrict__ B2, int M, int N, int K, EpiArgs<float> ep, int* status,
                          int drop_first_stage, unsigned long long wait_ns) {
   constexpr bool DUAL = (EPI == EPI_GELU_MUL), HIST = (EPI == EPI_HIST);
   constexpr int COLS = DUAL ? BN / 2 : BN, STAGE = stage_bytes<BN>(), PLANE_B = BN * BK * 2, PITCH = BN + 4;
@@ -152,8 +152,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   volatile int* abort_flag = &ctl->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * COLS;
-  const int k_end = causal ? min(K, n0 + COLS) : K;   // a lower-triangular B has nothing beyond the tile's last column
-  const int nkb = (k_end + BK - 1) / BK, per = (nkb + KS - 1) / KS;
+  const int nkb = (K + BK - 1) / BK, per = (nkb + KS - 1) / KS;
   const int kb0 = KS > 1 ? min(nkb, (int)blockIdx.z * per) : 0, kb1 = KS > 1 ? min(nkb, kb0 + per) : nkb;
 
   if (tid == 0) {
@@ -302,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       constexpr int ROOM = (BM * PITCH + 31) / 32 * 32;   // behind the tile's sums
       static_assert(4 * (ROOM + DRAIN_WARPS * again_floats<HALF>()) <= STAGES * STAGE, "room for the sums made again");
       sums_again<HALF, COLS, DUAL>(A + (size_t)min(m0 + r0, M - 1) * lda, lda, min(32, M - m0 - r0), B + (size_t)n0 * ldb, DUAL ? B2 + (size_t)n0 * ldb : nullptr, ldb, c0,
-                                   N - n0, kb0 * BK, min(kb1 * BK, k_end), part + ROOM + (warp - DRAIN0) * again_floats<HALF>(), p, HIST ? BM : 1);
+                                   N - n0, kb0 * BK, min(kb1 * BK, K), part + ROOM + (warp - DRAIN0) * again_floats<HALF>(), p, HIST ? BM : 1);
     }
   }
   cg::cluster_group cluster = cg::this_cluster();
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 struct Operands {
   const float *A, *B, *B2;
   long long lda, ldb;
-  int M, N, K, causal;
+  int M, N, K;
 };
 
 // How many clusters of KS CTAs the GPU holds at a time (the SMs of a GPC are no multiple of 8: 8 leave some of them out); 0: none, or it cannot say now
@@ -421,7 +420,7 @@ int launch_tile(const Operands& o, const EpiArgs<float>& ep, cudaStream_t st) {
   }
   cfg.attrs = at;
   cfg.numAttrs = n;
-  e = cudaLaunchKernelEx(&cfg, kern, o.A, o.lda, o.B, o.ldb, o.B2, o.M, o.N, o.K, o.causal, ep, device_status_word(), (int)take_dropped_stage(), wait_bound_ns());
+  e = cudaLaunchKernelEx(&cfg, kern, o.A, o.lda, o.B, o.ldb, o.B2, o.M, o.N, o.K, ep, device_status_word(), (int)take_dropped_stage(), wait_bound_ns());
   if (e != cudaSuccess) return (int)e;
   STU_CHECK_LAUNCH();
   return STU_OK;
@@ -480,10 +479,11 @@ extern "C" int stu_test_f32_tile(int M, int N, int K, int gate_up, const int* ro
 
 // Both operands K-major with rows on the 16-byte grid; from 256 of K on, or from 96 where the tiles of 64 x 64 are four per SM and more (us, the
 // CUDA-core GEMM and this one: 4000 x 4096 x 64 62 and 64, x 96 87 and 74; 8000 x 96 x 96 9.2 and 10.9; 300 x 512 x 128 7.8 and 8.4).  Where
-// the CUDA-core GEMM splits K into eight chains of less than 128 it is as fast and, for positive operands, a tenth more exact.
+// the CUDA-core GEMM splits K into eight chains of less than 128 it is as fast and, for positive operands, a tenth more exact.  Lower-triangular weights stay there: their
+// short rows are such sums, and it reads nothing past blocks of 64 columns (what lies there need not be finite).
 bool gemm_f32_umma_takes(const void* A, long long lda, const void* B, long long ldb, long long skb, const void* B2, int M, int N, int K,
-                         int epi, int dtype) {
-  if (dtype != STU_F32 || skb != 1 || lda % 4 || ldb % 4 || K % 4 || !aligned16(A) || !aligned16(B) || (B2 && !aligned16(B2))) return false;
+                         int causal, int dtype) {
+  if (causal || dtype != STU_F32 || skb != 1 || lda % 4 || ldb % 4 || K % 4 || !aligned16(A) || !aligned16(B) || (B2 && !aligned16(B2))) return false;
   if (M <= 64 || N < 1) return false;
   const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64), sms = device_sm_count();
   if (K < 256) return K >= 96 && tiles >= 4 * sms;
@@ -491,8 +491,8 @@ bool gemm_f32_umma_takes(const void* A, long long lda, const void* B, long long 
 }
 
 int gemm_f32_umma_dispatch(const void* A, long long lda, const void* B, long long ldb, const void* B2, int M, int N, int K, int epi,
-                           int causal, const EpiArgsAny& ep, cudaStream_t st) {
-  const Operands o{(const float*)A, (const float*)B, (const float*)B2, lda, ldb, M, N, K, causal};
+                           const EpiArgsAny& ep, cudaStream_t st) {
+  const Operands o{(const float*)A, (const float*)B, (const float*)B2, lda, ldb, M, N, K};
   switch (epi) {
     case EPI_STORE: return launch_epi<EPI_STORE>(o, ep.as<float>(), st);
     case EPI_RESID: return launch_epi<EPI_RESID>(o, ep.as<float>(), st);

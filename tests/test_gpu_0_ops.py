@@ -564,6 +564,41 @@ def test_fp32_linear_on_tensor_cores(shape, epi):
     assert err[0] <= max(err[1], 2.0 ** -24), err
 
 
+@pytest.mark.parametrize("shape", [(4000, 2500, 2500), (70, 1100, 1100), (300, 2049, 1024), (66, 40, 3072)])
+@pytest.mark.parametrize("epi", [0, 1, 2])
+def test_fp32_linear_of_triangular_weights_stays_on_the_cuda_cores(shape, epi):
+    """NaN past the blocks of 64 columns, of which that GEMM reads nothing; short rows are sums that it makes more exactly."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    torch.manual_seed(7)
+    x, r = torch.randn(M, K, device=dev()), torch.randn(M, N, device=dev())
+    hole = torch.arange(K, device=dev())[None, :] >= (torch.arange(N, device=dev())[:, None] // 64 + 1) * 64
+    W, W2 = torch.tril(torch.randn(2, N, K, device=dev()) / math.sqrt(K)).masked_fill(hole, float("nan"))
+    kw = {0: {}, 1: dict(resid=r), 2: dict(W2=W2)}[epi]
+    y = [ops.linear(x, W, epilogue=epi | ops.EPI_FLAG_CAUSAL, backend=b, **kw) for b in (0, 1)]
+    ops.check_status()
+    assert bool(y[0].isfinite().all()) and torch.equal(*y)
+
+
+@pytest.mark.parametrize("B,T,t0,N,K", [(3, 100, 5, 200, 1024), (7, 33, 0, 130, 2048), (2, 1000, 301, 72, 1028)])
+def test_fp32_histories_of_several_sequences_on_tensor_cores(B, T, t0, N, K):
+    """Tiles that end inside a sequence's positions and hold several, behind positions that are there and stay as they are."""
+    from flash_stu_2_b200 import ops
+    torch.manual_seed(6)
+    x, W = torch.randn(B * T, K, device=dev()), torch.randn(N, K, device=dev()) / math.sqrt(K)
+    Lh = (t0 + T) // 2 + 9
+    full = (x.double() @ W.double().t()).view(B, T, N)
+    t, err = torch.arange(t0, t0 + T, device=dev()), []
+    for backend in (0, 1):
+        hist = torch.full((B, N, 2, Lh), 7.0, device=dev())
+        ops.linear(x, W, out=hist, epilogue=ops.EPI_HIST, hist_T=T, hist_t0=t0, hist_Lh=Lh, backend=backend)
+        got = hist[:, :, t % 2, t // 2].transpose(1, 2)
+        assert int((hist != 7.0).sum()) == B * T * N
+        err.append(float((got.double() - full).norm() / full.norm()))
+    ops.check_status()
+    assert err[0] <= max(err[1], 2.0 ** -24), err
+
+
 # The largest second and third parts, of one sign: what the six products leave out of each is 2^-23.03 of it, and adds up
 WORST = 1 + 2.0 ** -8 - 2.0 ** -23
 
