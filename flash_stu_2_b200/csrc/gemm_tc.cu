@@ -197,6 +197,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
 
 // A barrier of this pair (shared::cluster address).  At the default scope: a release for the cluster waits for all of the
 // thread's stores so far to arrive, which nothing here needs (the reads of tensor memory are done and fenced).
@@ -273,6 +283,8 @@ __host__ __device__ constexpr int stage_blocks(int mma_n) { return mma_n > 128 ?
 // products whose tiles of 256 rows would fill their last wave badly (see tile_form).
 // SPLIT: K of the tiles behind the first `whole` is cut into `parts` (split_plan); what a pair works on are then those tiles' parts, and their
 // sums go to `partials` in fp32: per part [CTA][32 rows][4 columns], every store of a warp 512 bytes in a row.  split_sum_kernel adds them up.
+// The first `whole` tiles' sums are made of the same parts, one accumulator behind the other and added up in the epilogue's registers in the same order:
+// equal rows of x give equal results wherever they stand.
 struct SplitK {
   int whole, parts;
   float* partials;
@@ -313,11 +325,15 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
   // tile and k-blocks of a part.  All tiles' first parts come first: what works on them at a time shares its k-blocks in L2.
   const int rest = SPLIT ? tiles_m * tiles_n - split.whole : 1;
   const auto whole_tile = [&](int tile) { return SPLIT && tile >= split.whole ? split.whole + (tile - split.whole) % rest : tile; };
+  const auto part_range = [&](int part, int& kb0, int& kb_end) {
+    kb0 = (int)((long long)num_kb * part / split.parts);
+    kb_end = (int)((long long)num_kb * (part + 1) / split.parts);
+  };
+  const auto chains = [&](int tile) { return SPLIT && tile < split.whole ? split.parts : 1; };   // accumulators of a tile
   const auto k_range = [&](int tile, int& kb0, int& kb_end) {
     if (SPLIT && tile >= split.whole) {
       const int part = (tile - split.whole) / rest;
-      kb0 = (int)((long long)num_kb * part / split.parts);
-      kb_end = (int)((long long)num_kb * (part + 1) / split.parts);
+      part_range(part, kb0, kb_end);
     }
   };
 
@@ -414,13 +430,15 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
       int g = 0, s = 0, it = 0;
       uint32_t ph = 0;
       bool ok = true, ready = false;
-      for (int tile = pair; ok && tile < num_tiles; tile += pairs, it++) {
+      for (int tile = pair, chain = 0; ok && tile < num_tiles; it++) {
         const int buf = it & 1;
         const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
         int tm, tn;
         tile_coords(whole_tile(tile), tiles_m, tiles_n, group_m, tm, tn);
         int kb0 = 0, kb_end = row_kb<EPI>(tile_kb(num_kb, tn * BN, causal, BN), ep, min((tm + 1) * CTAS * BM, M) - 1, K);
-        k_range(tile, kb0, kb_end);
+        if (chains(tile) > 1) part_range(chain, kb0, kb_end);
+        else k_range(tile, kb0, kb_end);
+        if (++chain >= chains(tile)) tile += pairs, chain = 0;   // (of the next turn)
         ok = warp_wait(&tmem_empty[buf], (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, wait_ns);
         if (!ok) break;
         for (int kb = kb0; kb < kb_end; kb += KBS, g++) {
@@ -492,12 +510,47 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(64 + 32 * EPI_WAR
       tile_coords(whole_tile(tile), tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = (CTAS * tm + rank) * BM, n0 = tn * BN;
       const int first = m0 + quarter * 32, rows = min(32, M - first);   // this warp's rows
+      bool ok = true;
+      if constexpr (SPLIT) {
+        if (tile < split.whole) {   // this warp's part of the tile, 32 rows and 64 of every 128 columns, over all accumulators but the last, and that one's on top
+          float sum[128];
+#pragma unroll
+          for (int i = 0; i < 128; i++) sum[i] = -0.f;   // (the zero that leaves the sign of another alone)
+          for (int chain = 0;; chain++, it++) {
+            ok = mbar_wait(&tmem_full[it & 1], ((uint32_t)it >> 1) & 1u, abort_flag, wait_ns);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t taddr = tmem_base + (uint32_t)(it & 1) * ACC_COLS + ((uint32_t)(quarter * 32) << 16) + 64 * half;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+              uint32_t r[8];
+              tmem_ld8(taddr + (i >> 3) * 128 + (i & 7) * 8, r);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int j = 0; j < 8; j++) sum[8 * i + j] += __uint_as_float(r[j]);
+            }
+            if (chain + 1 == split.parts) {
+#pragma unroll
+              for (int i = 0; i < 16; i++) tmem_st8(taddr + (i >> 3) * 128 + (i & 7) * 8, sum + 8 * i);
+              break;
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(hand_back + (it & 1) * (uint32_t)sizeof(uint64_t));
+          }
+          if (!ok) break;
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");   // read again below, by this warp
+        }
+      }
       const int buf = it & 1;
       const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS;
-      bool ok = mbar_wait(&tmem_full[buf], ((uint32_t)it >> 1) & 1u, abort_flag, wait_ns);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!SPLIT || tile >= split.whole) {
+        ok = mbar_wait(&tmem_full[buf], ((uint32_t)it >> 1) & 1u, abort_flag, wait_ns);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
       if (SPLIT && tile >= split.whole) {
         float4* part = reinterpret_cast<float4*>(split.partials + (size_t)(tile - split.whole) * SPLIT_TILE) + (rank * 4 + quarter) * (BN / 4) * 32 + lane;
 #pragma unroll 1
@@ -1369,9 +1422,10 @@ extern "C" long long stu_linear_tile_cost(int M, int N) {
 
 // Plain and residual products that leave pairs idle for long: the tiles that do not fill a wave (all of them where there are fewer than pairs) are
 // 256 x 256 whatever the rows, their K is cut into parts of the same length, and split_sum_kernel adds the parts up.  A pair working alone on
-// K = 49152 takes 200 us, so what counts is long K: us, as tile_form has it and split, 24000 x 1024 x 49152 (6 of 376 tiles in the last wave) 1784 -> 1637,
-// 8192 x 768 x 24576 349 -> 312, 1180 x 1024 x 24576 80.9 -> 54.4, 251 x 2048 x 98304 327 -> 96, 74 x 512 x 24576 61.1 -> 15.7, 16384 x 1536 x 6144 207 -> 187,
-// 4096 x 1536 x 6144 64.7 -> 56.3, 333 x 1536 x 6144 30.5 -> 26.3 (weights from HBM).  The parts' way through L2 and the second launch cost what short K
+// K = 49152 takes 200 us, so what counts is long K: us, as tile_form has it and split, single calls on operands from HBM, 24000 x 1024 x 49152 (6 of
+// 376 tiles in the last wave) 1750 -> 1566, 8192 x 768 x 24576 264 -> 204, 1180 x 1024 x 24576 94 -> 62, 251 x 2048 x 98304 322 -> 106, 74 x 512 x 24576 82 -> 24,
+// 16384 x 1536 x 6144 213 -> 200, 4096 x 1536 x 6144 74 -> 64, 333 x 1536 x 6144 29 -> 24.  (That the whole tiles add up the same parts costs, back to back,
+// 24000 x 1024 x 8192 269 -> 274, 16384 x 1536 x 6144 201.5 -> 203.4, 19851 x 512 x 3072 50.0 -> 53.4.)  The parts' way through L2 and the second launch cost what short K
 // gains: 834 x 768 x 3072 in 4 parts 20.5 -> 21.5, 1337 x 1024 x 2048 in 3 12.6 -> 17.6, 8192 x 1536 x 6144 in 3 106 -> 107.  The line, in us: a k-block
 // of 64 takes 0.31 in a wide tile (0.18 in a narrow one; 0.27 and 0.155 where few SMs work), a wave of parts 1 more, each part 0.05 (256 KB
 // written and read), the second launch 4; 105 products of 65 to 24000 rows, K = 512 to 98304: 0.97 (noise, not split) to 4.0 times as fast.

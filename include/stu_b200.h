@@ -95,7 +95,8 @@ long long stu_linear_tile_cost(int M, int N);
 /* stu_linear with a workspace (device, 16-byte aligned): epilogues 0 and 1 of the tcgen05 GEMM whose last wave of tiles would leave SMs idle
  * for long cut K of those tiles, keep the parts' sums there in fp32 and add them up in a second launch.  ..._workspace_elems: fp32 values that
  * this takes for a product, 0 where it does not pay (any dtype or epilogue may be asked for).  With less than that, or NULL, the
- * call is stu_linear.  The contents need not be set and are not kept.  No counterpart in the reference. */
+ * call is stu_linear.  Every row's sums are cut alike, so equal rows of a call give equal results; how they are cut depends on M, N and K, so a row
+ * may be rounded otherwise in a call of another size (a prefill in chunks, another batch).  The contents need not be set and are not kept.  No counterpart in the reference. */
 long long stu_linear_workspace_elems(int M, int N, int K, int epilogue, int dtype);
 int stu_linear_split(const void* x, long long x_row_stride, const void* W, long long w_row_stride, long long w_k_stride,
                      const void* W2, const void* resid, long long resid_row_stride, void* y, long long y_row_stride,

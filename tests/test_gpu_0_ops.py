@@ -395,6 +395,19 @@ def test_bounded_wait_expiry_of_the_fp32_gemm(shape):
     ops.check_status()
 
 
+@pytest.mark.parametrize("shape", [(333, 1536, 6144), (5193, 1000, 4096)])   # parts alone; whole tiles of several accumulators ahead of them
+def test_bounded_wait_expiry_of_a_linear_in_parts(shape):
+    from flash_stu_2_b200 import _lib, ops
+    M, N, K = shape
+    assert _lib.load().stu_linear_workspace_elems(M, N, K, 0, 1) > 0
+    g = torch.Generator(device=dev()).manual_seed(26)
+    x, W = torch.randn(M, K, device=dev(), generator=g).bfloat16(), torch.randn(N, K, device=dev(), generator=g).bfloat16()
+    want = ops.linear(x, W)
+    _gives_up(lambda: ops.linear(x, W), 3)
+    assert torch.equal(ops.linear(x, W), want)
+    ops.check_status()
+
+
 def test_bounded_wait_expiry_of_the_fp32_convolutions():
     from flash_stu_2_b200 import ops
     torch.manual_seed(24)
@@ -666,6 +679,26 @@ def test_linear_of_long_weights_in_parts(shape, epi):
         rc2 = _lib.load().stu_linear(x.data_ptr(), K + 8, W.data_ptr(), K + 16, 1, None, None, 0, whole.data_ptr(), N, M, N, K, 0, 0, 0, 0, None, 0.0, 1, 0,
                                      torch.cuda.current_stream().cuda_stream)
         assert rc == rc2 == 0 and torch.equal(short, whole) and bool(work.isnan().all())
+
+
+@pytest.mark.parametrize("shape", [(5193, 1000, 4096), (19851, 512, 3072), (16384, 1536, 6144), (5193, 1001, 4104), (2100, 200, 24576)])
+@pytest.mark.parametrize("epi", [0, 1])
+def test_equal_rows_of_a_linear_in_parts_are_equal(shape, epi):
+    """Tiles of which K is cut and, ahead of them, whole ones: an output is the same sum in either, so sequences of a batch do not differ by where they stand."""
+    from flash_stu_2_b200 import _lib, ops
+    M, N, K = shape
+    if epi:
+        N = N // 8 * 8
+    assert _lib.load().stu_linear_workspace_elems(M, N, K, epi, 1) > 0
+    torch.manual_seed(11)
+    three = torch.randn(3, K, device=dev()).bfloat16()
+    x, W = three.repeat(-(-M // 3), 1)[:M], (torch.randn(N, K, device=dev()) / math.sqrt(K)).bfloat16()
+    r = torch.randn(3, N, device=dev()).bfloat16().repeat(-(-M // 3), 1)[:M] if epi else None
+    y = ops.linear(x, W, resid=r, epilogue=epi)
+    ops.check_status()
+    assert torch.equal(y, y[:3].repeat(-(-M // 3), 1)[:M])
+    full = three.double() @ W.double().t() + (r[:3].double() if epi else 0.0)
+    assert float((y[:3].double() - full).abs().max()) <= 2.0 ** -7 * max(1.0, float(full.abs().max()))
 
 
 @pytest.mark.parametrize("shape,launches", [((333, 1536, 6144), 2), ((65, 64, 24576), 2), ((333, 1536, 512), 1), ((64, 64, 24576), 1)])
