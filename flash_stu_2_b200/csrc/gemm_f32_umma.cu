@@ -316,9 +316,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   for (int r = 0; r < KS; r++) parts[r] = KS > 1 ? cluster.map_shared_rank(part, r) : part;
   if (!*abort_flag) {
     // This CTA's outputs are the tile's rows rank, rank + KS, ...; of a history, which is time-major, its columns rank, rank + KS, ..., whose sums lie one
-    // behind the other (in rows, four to 32 lanes met in a bank: 114 x 2912 x 292 29 us, now 14).  Residuals are read four at a time (4944 x 3891 x 96
-    // 190 -> 121 us).
-    constexpr int OUTS = BM / KS * COLS, AT_A_TIME = 4;
+    // behind the other (in rows, four to 32 lanes met in a bank: 114 x 2912 x 292 29 us, now 11).  Residuals are read four at a time (4944 x 3891 x 96
+    // 190 -> 124 us), over a cluster singly: a CTA has few of them, and with four (or two) the compiler's main loop is 6 % slower (388 x 256 x 12288 53.3, now 49.9).
+    constexpr int OUTS = BM / KS * COLS, AT_A_TIME = EPI == EPI_RESID && KS > 1 ? 1 : 4;
     const auto output = [&](int e, int& m, int& n, float& s, float& s2) {
       const int row = HIST ? e % BM : rank + e / COLS * KS, c = HIST ? rank + e / BM * KS : e % COLS;
       m = m0 + row, n = n0 + c, s = s2 = 0.f;
