@@ -94,6 +94,7 @@ _SIGNATURES = {
     "stu_full_combine": ([_P, _P, _LL, _P, _LL, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_full_conv": ([_P, c_int, _P, c_int, c_int, _P, _LL, c_int, c_int, c_int, c_int, c_int, c_int, _P], c_int),
     "stu_full_conv_f32_tc5_scratch_elems": ([c_int, c_int, c_int, c_int], c_longlong),
+    "stu_full_conv_f32_tc5_pays": ([c_int, c_int, c_int, c_int, c_int], c_int),
     "stu_full_conv_f32_tc5": ([_P, c_int, _P, c_int, c_int, _P, _P, _LL, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P], c_int),
     "stu_full_conv_tc5_scratch_elems": ([c_int, c_int], c_longlong),
     "stu_full_conv_tc5": ([_P, c_int, _P, c_int, c_int, _P, _P, _LL, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P], c_int),

@@ -11,7 +11,7 @@
 //
 // Bound: L2, from which a stage of 24 instructions (66 cycles each at 128 channels) takes 57 KB: 1.4 us a stage on all SMs are 6 TB/s.  24
 // filters, the CUDA-core kernel (stu_full_conv.cu) and this one, us: 8 x 1000 positions of 64 channels 277 and 101, 4 x 600 of 512 478 and 200, 16
-// filters, 8 x 2048 of 96 1074 and 276 (ops.full_conv_f32_tc5_pays says where that one stays the faster).  Error against float64: 3.3e-7 and
+// filters, 8 x 2048 of 96 1074 and 276 (stu_full_conv_f32_tc5_pays says where that one stays the faster).  Error against float64: 3.3e-7 and
 // 9.6e-8, 2.6e-7 and 9.1e-8, 4.7e-7 and 1.1e-7 (32 positions per accumulator: the same, and twice the reads of tensor memory, 121 us for the first).
 //
 // Roles (one persistent CTA per SM, 320 threads): warp 0 producer, warp 1 MMA issuer, warps 2-9 sums and outputs (a quarter of the
@@ -22,6 +22,8 @@
 // Every load is a plain single-CTA copy of this GPU's own memory.  Every wait is bounded: on expiry the CTA raises status 9, lets issued
 // copies land (bounded), frees its tensor memory and returns.
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "split3.cuh"
@@ -445,6 +447,29 @@ extern "C" long long stu_full_conv_f32_tc5_scratch_elems(int B, int d, int K, in
 }
 
 // U[b][t - t0][sign][k][i] (row stride ldU) of positions [t0, t_end) from the history [B][d][2][Lh]; phi [L][K]; all fp32.
+// Whether this takes less time than the kernel of stu_full_conv.cu.  Both are waves of tiles: there of 64 entries of both parities and 32 (16) channels, 1.3 us per
+// 32 entries where the SMs have three tiles each and 1.6 for one, here of 128 entries of a parity and 128 (64) channels, 1.1 (0.9) us per 64 entries, behind a
+// launch that splits the operands.  Fitted to 5461 calls of 1 to 32 sequences, 4 to 1024 channels, 1 to 32 filters and up to 6000 positions: half a percent of
+// them are taken and more than 3 % slower (at most 1.26), where the positions alone decided it was a ninth (up to 1.7: 4 x 144 channels of 219 positions, one
+// filter, 10.8 us and 15.8).
+extern "C" int stu_full_conv_f32_tc5_pays(int B, int d, int K, int t0, int t_end) {
+  if (B <= 0 || d <= 0 || K <= 0 || t0 < 0 || t_end <= t0) return 0;
+  const long long rows = (long long)B * d, hi = (t_end + 1) / 2, lo = t0 / 2, sms = device_sm_count();
+  if (d % 4 || !(t_end >= 400 || (t_end >= 200 && rows >= 512))) return 0;
+  const auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  // tensor cores: tiles of the last block come first, the SM with one more than the others has about the mean of first and last
+  const bool wide = rows > 64;
+  const long long blocks = up(hi, 128), per_block = up(rows, wide ? 128 : 64) * 2 * K, tiles = (blocks - lo / 128) * per_block, waves = up(tiles, sms);
+  const long long last = blocks - 1 - (waves - 1) * sms / per_block, stages = waves * (2 * (blocks - 1 + last) + 4);
+  const double tensor = 7.15 + stages * (wide ? 1.09 + 0.067 * std::min(tiles, sms) / sms : 0.907) + (wide ? 2.67 * waves : 0.0) +
+                        12.5e-6 * (384.0 * blocks * K + rows * hi / 4.0);
+  // CUDA cores
+  const long long tall = up(hi - lo, 64), columns = K * up(rows, rows <= 16 ? 16 : 32), longest = up(hi, 32);
+  const long long steps = columns * ((tall - 1) * up(lo, 32) + tall * (tall - 1) + longest + tall);
+  const double cores = 3.5 + std::max(1.6 * longest, (rows <= 16 ? 0.79 : 1.3) * steps / sms + 0.85 * longest);
+  return tensor < 0.98 * cores;
+}
+
 extern "C" int stu_full_conv_f32_tc5(const void* hist, int Lh, const void* phi, int L, int K, void* scratch, void* U, long long ldU, int B,
                                      int d, int both_signs, int t0, int t_end, int* status, int dtype, void* stream) {
   if (!hist || !phi || !scratch || !U) return STU_ERR_NULL;

@@ -40,12 +40,19 @@ RMS_EPS = float(torch.finfo(torch.float32).eps)  # what torch.nn.RMSNorm(eps=Non
 
 _status = {}
 _sms = {}
-launch_count = 0  # kernels launched through this module (bench.py reports it)
+_launches = 0
 
 
 def _count(n=1):
-    global launch_count
-    launch_count += n
+    global _launches
+    _launches += n
+
+
+def __getattr__(name):
+    """launch_count: kernels launched through this module (bench.py reports it); the native linear counts its own."""
+    if name == "launch_count":
+        return _launches + (_lib._native.linear_launches() if _lib._native is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -221,7 +228,6 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
         # checks, output and launch in one native call; None: whatever is out of the ordinary is looked at below
         y = _lib.native().linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed_weight, hist_T, hist_t0, hist_Lh)
         if y is not None:
-            _count(1 if x.shape[0] <= 64 else _lib.native().stu_linear_launches())   # (two where K is cut: more rows than a token step's)
             return y
     _cuda(x, W, W2, resid, out, norm_w)
     assert x.dim() == 2 and W.dim() == 2 and x.stride(1) == 1
@@ -649,39 +655,18 @@ def full_conv_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):
 
 def sm_count() -> int:
     """SMs of the current device (before there is one: a B200's)."""
-    if not torch.cuda.is_initialized():
+    if not _sms and not torch.cuda.is_initialized():
         return 148
     dev = torch._C._cuda_getDevice()
-    if dev not in _sms:
-        _sms[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
-    return _sms[dev]
+    n = _sms.get(dev)
+    if n is None:
+        n = _sms[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
+    return n
 
 
 def full_conv_f32_tc5_pays(B: int, d: int, K: int, t0: int, t_end: int) -> bool:
-    """Whether full_conv_f32_tc5 takes less time than full_conv for outputs t0 .. t_end - 1 of fp32 histories [B, d].  Both are waves of tiles: of 64 entries
-    of both parities and 32 (16) channels, 1.3 us per 32 entries where the SMs have three tiles each and 1.6 for one, and of 128 entries of a parity
-    and 128 (64) channels, 1.1 (0.9) us per 64 entries, behind a launch that splits the operands.  Fitted to 5461 calls of 1 to 32 sequences,
-    4 to 1024 channels, 1 to 32 filters and up to 6000 positions: half a percent of them are taken and more than 3 % slower (at most 1.26), where the positions
-    alone decided it was a ninth (up to 1.7: 4 x 144 channels of 219 positions, one filter, 10.8 us and 15.8)."""
-    rows, hi, lo, sms = B * d, (t_end + 1) // 2, t0 // 2, sm_count()
-    if d % 4 or not (t_end >= 400 or (t_end >= 200 and rows >= 512)):
-        return False
-    # tensor cores: tiles of the last block come first, the SM with one more than the others has about the mean of first and last
-    blocks, wide = -(-hi // 128), rows > 64
-    per_block = -(-rows // (128 if wide else 64)) * 2 * K
-    tiles = (blocks - lo // 128) * per_block
-    waves = -(-tiles // sms)
-    last = blocks - 1 - (waves - 1) * sms // per_block
-    stages = waves * (2 * (blocks - 1 + last) + 4)
-    tensor = 7.15 + stages * (1.09 + 0.067 * min(tiles, sms) / sms if wide else 0.907) + (2.67 * waves if wide else 0.0) \
-        + 12.5e-6 * (384 * blocks * K + rows * hi / 4)
-    # CUDA cores
-    channels, tall = (16 if rows <= 16 else 32), -(-(hi - lo) // 64)
-    columns = K * -(-rows // channels)
-    steps = columns * ((tall - 1) * -(-lo // 32) + tall * (tall - 1) + -(-hi // 32) + tall)
-    longest = -(-hi // 32)
-    cores = 3.5 + max(1.6 * longest, (0.79 if rows <= 16 else 1.3) * steps / sms + 0.85 * longest)
-    return tensor < 0.98 * cores
+    """Whether full_conv_f32_tc5 takes less time than full_conv for outputs t0 .. t_end - 1 of fp32 histories [B, d]."""
+    return bool(_lib.native().stu_full_conv_f32_tc5_pays(B, d, K, t0, t_end))
 
 
 def full_conv_f32_tc5(hist, phi, U, both_signs: bool, t0: int, t_end: int):

@@ -258,6 +258,7 @@ int stu_full_conv_tc5(const void* hist, int Lh, const void* phi, int L, int K, v
 /* The same for fp32 on the tcgen05 tensor cores (products of three bf16 parts of either operand): d and ldU multiples of 4; scratch holds
  * stu_full_conv_f32_tc5_scratch_elems bf16 values (the parts of the taps and of the history). */
 long long stu_full_conv_f32_tc5_scratch_elems(int B, int d, int K, int t_end);
+int stu_full_conv_f32_tc5_pays(int B, int d, int K, int t0, int t_end);   /* 1 where it takes less time than stu_full_conv */
 int stu_full_conv_f32_tc5(const void* hist, int Lh, const void* phi, int L, int K, void* scratch, void* U, long long ldU, int B,
                           int d, int both_signs, int t0, int t_end, int* status, int dtype, void* stream);
 
