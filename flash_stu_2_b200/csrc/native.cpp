@@ -126,12 +126,8 @@ bool raised(int rc, const char* what) {
   return true;
 }
 
-// Kernels that linear() has launched: counted here, in calls of a few microseconds
-std::atomic<long long> g_linear_launches{0};
-PyObject* linear_launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_FromLongLong(g_linear_launches.load(std::memory_order_relaxed)); }
-
-// linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed, hist_T, hist_t0, hist_Lh) -> y, or None where a check
-// fails or the library refuses: ops.linear then goes through its own checks, which raise what they raise.
+// linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed, hist_T, hist_t0, hist_Lh) -> y, or (y,) where K was cut
+// and there were two launches, or None where a check fails or the library refuses: ops.linear then goes through its own checks, which raise what they raise.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 13) {
     PyErr_SetString(PyExc_TypeError, "13 arguments expected");
@@ -181,10 +177,13 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_END_ALLOW_THREADS
     if (raised(rc, "stu_linear")) return nullptr;
     if (rc != 0) Py_RETURN_NONE;
-    if (M > 0) g_linear_launches.fetch_add(stu_linear_launches(), std::memory_order_relaxed);
-    if (made.defined()) return THPVariable_Wrap(std::move(made));
-    Py_INCREF(args[4]);
-    return args[4];
+    PyObject* y = made.defined() ? THPVariable_Wrap(std::move(made)) : Py_NewRef(args[4]);
+    if (parts > 0 && y && stu_linear_launches() == 2) {
+      PyObject* pair = PyTuple_Pack(1, y);
+      Py_DECREF(y);
+      y = pair;
+    }
+    return y;
   } catch (const BadArgument&) {
     PyErr_Clear();
   } catch (const std::exception&) {
@@ -388,7 +387,6 @@ PyMethodDef methods[] = {
     ENTRY(stu_to_history),
     ENTRY(stu_toeplitz),
     {"status_ready", (PyCFunction)(void (*)(void))status_ready, METH_FASTCALL, nullptr},
-    {"linear_launches", (PyCFunction)(void (*)(void))linear_launches, METH_FASTCALL, nullptr},
     {"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, nullptr},
     {"layer_step_f32", (PyCFunction)(void (*)(void))layer_step_f32, METH_FASTCALL, nullptr},
     {"layer_prefill", (PyCFunction)(void (*)(void))layer_prefill, METH_FASTCALL, nullptr},

@@ -40,19 +40,12 @@ RMS_EPS = float(torch.finfo(torch.float32).eps)  # what torch.nn.RMSNorm(eps=Non
 
 _status = {}
 _sms = {}
-_launches = 0
+launch_count = 0  # kernels launched through this module (bench.py reports it)
 
 
 def _count(n=1):
-    global _launches
-    _launches += n
-
-
-def __getattr__(name):
-    """launch_count: kernels launched through this module (bench.py reports it); the native linear counts its own."""
-    if name == "launch_count":
-        return _launches + (_lib._native.linear_launches() if _lib._native is not None else 0)
-    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+    global launch_count
+    launch_count += n
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -116,6 +109,7 @@ def check_status(device=None):
 
 
 _local = threading.local()   # .arena: where this thread's outputs come from while an `arena` block is open
+_arenas, _arenas_lock = 0, threading.Lock()   # blocks that are open in any thread: where there is none, no thread's own is looked for
 
 
 class arena:
@@ -127,11 +121,17 @@ class arena:
         self.buffer, self.used = buffer, 0
 
     def __enter__(self):
+        global _arenas
+        with _arenas_lock:
+            _arenas += 1
         self.outer, _local.arena = getattr(_local, "arena", None), self
         return self
 
     def __exit__(self, *exc):
+        global _arenas
         _local.arena = self.outer
+        with _arenas_lock:
+            _arenas -= 1
 
     def take(self, shape, dtype):
         n = math.prod(shape) * dtype.itemsize
@@ -223,11 +223,15 @@ def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = Non
            transposed_weight: bool = False, hist_T: int = 0, hist_t0: int = 0, hist_Lh: int = 0,
            kpos: Optional[torch.Tensor] = None):
     """y = epilogue(x @ W^T) for x [M,K] and W [N,K] (or W [K,N] with transposed_weight=True)."""
-    pieces = getattr(_local, "arena", None)
+    pieces = getattr(_local, "arena", None) if _arenas else None
     if kpos is None and (pieces is None or (out is not None and x.shape[0] <= 64)):   # (more rows: K may be cut, and the workspace is a piece)
         # checks, output and launch in one native call; None: whatever is out of the ordinary is looked at below
         y = _lib.native().linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed_weight, hist_T, hist_t0, hist_Lh)
         if y is not None:
+            if type(y) is tuple:   # K was cut: two launches
+                _count(2)
+                return y[0]
+            _count()
             return y
     _cuda(x, W, W2, resid, out, norm_w)
     assert x.dim() == 2 and W.dim() == 2 and x.stride(1) == 1
