@@ -411,7 +411,7 @@ def layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, 
                                        status_word(x.device))
     if done is None:
         return 0
-    _count({1: 4, 3: 7, 7: 8}[done])
+    _count(7 if done == 3 else 8 if done == 7 else 4)
     return done & 3
 
 

@@ -757,6 +757,25 @@ def test_linear_of_few_rows_over_long_weights(shape, epi, early):
     assert float((out.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-3
 
 
+@pytest.mark.parametrize("shape", [(8, 1024, 49152), (1, 640, 14720), (5, 768, 12296), (7, 1200, 4104), (3, 4735, 8192)])
+@pytest.mark.parametrize("epi", [0, 1])
+def test_linear_of_few_rows_over_long_weights_output_by_output(shape, epi):
+    """Each output by itself: the float64 sum rounded once, but for fp32 sums of K products of order 1 / sqrt(K) (2^-24 * sqrt(K) * a few, well below
+    1e-4), and the residual added to that."""
+    from flash_stu_2_b200 import ops
+    M, N, K = shape
+    torch.manual_seed(12)
+    x, W, r = torch.randn(M, K, device=dev()), torch.randn(N, K, device=dev()) / math.sqrt(K), torch.randn(M, N, device=dev())
+    x, W, r = (t.bfloat16() for t in (x, W, r))
+    out = ops.linear(x, W, resid=r if epi else None, epilogue=epi)
+    ops.check_status()
+    full = x.double() @ W.double().t()
+    lo, hi = (full - 1e-4).bfloat16(), (full + 1e-4).bfloat16()
+    if epi:
+        lo, hi = (r.float() + lo.float()).bfloat16(), (r.float() + hi.float()).bfloat16()
+    assert bool(((out >= lo) & (out <= hi)).all())
+
+
 @pytest.mark.parametrize("case", [(1, 8, 3, 0, 17, True), (3, 20, 5, 5, 257, True), (2, 64, 4, 0, 256, False), (1, 132, 7, 250, 515, True),
                                   (5, 64, 24, 0, 1000, True)])
 def test_full_variant_fp32_convolutions_on_tensor_cores(case):
