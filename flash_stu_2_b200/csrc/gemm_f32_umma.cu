@@ -9,7 +9,7 @@
 // rows are below either and keep those.)
 //
 // Bound: shared memory, through which a block of 64 of K passes three times as planes and six times as operands, and the splitting, about
-// 6 instructions a value.  us, the CUDA-core GEMM and this kernel: 8000 x 96 x 3072 159 and 50, 256 x 512 x 6144 56 and 28, gate/up 256 x 6144 x
+// 6 instructions a value.  us, the CUDA-core GEMM and this kernel: 8000 x 96 x 3072 159 and 53, 256 x 512 x 6144 56 and 28, gate/up 256 x 6144 x
 // 512 86 and 43, 1000 x 1536 x 512 51 and 23, 4000 x 8192 x 1024 1603 and 487 (138 TFLOP/s of fp32 products, the CUDA cores' peak is 74).
 //
 // One 128 x BN tile per CTA (gate/up: BN / 2 columns of either), K split over a cluster of KS CTAs whose sums meet in distributed

@@ -6,7 +6,8 @@
 // the 128 x 2K sums a row needs the even taps (its parity is the position's) or the odd ones: the other half is work that costs nothing
 // beside the history's bytes.  What the cache holds past the position is set to zero in shared memory ahead of the last stage's instructions.
 //
-// Bound: HBM, the history once, behind a chain of 7 us (position, first copies, last instructions, outputs).  full_step_kernel is bound by its load
+// Bound: HBM, the history once, behind a chain of 7 us back to back (position, first copies, last instructions, outputs) and of 14 behind a kernel that
+// it was not launched beside (8 x 1024, history from HBM, at 3000 22.5 us, at 6000 30.7: 49 MB more in 8.2).  full_step_kernel is bound by its load
 // units: 16-byte loads of 64-byte pieces of rows, for the taps as many as for the history, 1.9 us for every 256 entries whether they come from
 // L1 or from HBM.  us, that one and this one, 24 filters, history from L2: 8 x 1024 channels at position 1000 10.7 and 9.5, at 3000 19.6 and 14.1, at
 // 8000 40 and 31; 16 x 1024 at 2000 28.2 and 15.7.  ops.full_decode_step_tc5_pays says where that one stays the faster.
@@ -285,7 +286,7 @@ extern "C" int stu_full_decode_step_tc5(const void* x, long long x_rstride, cons
   static SmemLimit lim;
   cudaError_t e = allow_smem((const void*)full_step_umma_kernel, smem_bytes(MAX_K, MAX_STAGES), lim);
   if (e != cudaSuccess) return (int)e;
-  // Four stages where the grid fills more than one CTA per SM, so that two fit (16 x 1024 at position 2000 15.7 us, with eight 24.6); six below that (the
+  // Four stages where the grid fills more than one CTA per SM, so that two fit (16 x 1024 at position 2000 15.0 us, with six 21.9); six below that (the
   // layer step of 8 x 1024 at 3000 in a chain 51.4 with four, 50.4 with six; two and three, beside which the next kernel's CTAs fit and take the
   // bandwidth early, 57).
   const int tiles = B * (d / CH), stages = tiles > device_sm_count() ? 4 : MAX_STAGES;
