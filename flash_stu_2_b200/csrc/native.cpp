@@ -126,6 +126,11 @@ bool raised(int rc, const char* what) {
   return true;
 }
 
+// K from which the layers let a product's K be cut (stu_linear_split): the contractions of all filters' features (filters * d), not an MLP's.  A cut sum is
+// rounded other than one chain, and how K is cut depends on the rows of the call: with it a model drew other tokens in another batch or a prefill in chunks
+// (28 prompts of 1033 tokens, 512 channels: 3 of 1036), for 1 % of a prefill.
+constexpr long long CUT_K = 16384;
+
 // linear(x, W, W2, resid, out, epilogue, norm_w, eps, backend, transposed, hist_T, hist_t0, hist_Lh) -> y, or (y,) where K was cut
 // and there were two launches, or None where a check fails or the library refuses: ops.linear then goes through its own checks, which raise what they raise.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -167,7 +172,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const long long lda = x->stride(0), r_rs = resid ? resid->stride(0) : 0;
     void* stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
     // backends that may come to the tcgen05 GEMM: 0 and 2
-    const long long parts = backend == 0 || backend == 2 ? stu_linear_workspace_elems((int)M, (int)N, (int)K, epi, code) : 0;
+    const long long parts = K >= CUT_K && (backend == 0 || backend == 2) ? stu_linear_workspace_elems((int)M, (int)N, (int)K, epi, code) : 0;
     at::Tensor workspace;
     if (parts > 0) workspace = at::empty({parts}, x->options().dtype(at::kFloat));
     float* pw = parts > 0 ? workspace.data_ptr<float>() : nullptr;
@@ -307,7 +312,7 @@ PyObject* layer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int64_t yLh = ((t0 + T + 1) / 2 + 7) / 8 * 8;
     const int M = (int)(B * T), t_end = (int)(t0 + T);
     at::Tensor xn = at::empty({M, d}, x.options()), yT = at::empty({B, d, 2, yLh}, x.options()), h = at::empty({M, I}, x.options());
-    const long long parts = stu_linear_workspace_elems(M, (int)d, (int)I, 1, code);
+    const long long parts = I >= CUT_K ? stu_linear_workspace_elems(M, (int)d, (int)I, 1, code) : 0;
     at::Tensor workspace;
     if (parts > 0) workspace = at::empty({parts}, x.options().dtype(at::kFloat));
     float* pw = parts > 0 ? workspace.data_ptr<float>() : nullptr;

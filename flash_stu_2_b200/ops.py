@@ -213,8 +213,8 @@ def linear_tile_cost(rows: int, cols: int) -> int:
 
 
 def linear_workspace(rows: int, cols: int, K: int, epilogue: int, dtype: torch.dtype) -> int:
-    """fp32 values that a product of this size keeps the parts of its sums in (0: its K is not cut)."""
-    return int(_lib.native().stu_linear_workspace_elems(rows, cols, K, epilogue, 1)) if dtype == torch.bfloat16 else 0
+    """fp32 values that a product of this size keeps the parts of its sums in (0: its K is not cut; CUT_K of native.cpp says why short ones are not)."""
+    return int(_lib.native().stu_linear_workspace_elems(rows, cols, K, epilogue, 1)) if dtype == torch.bfloat16 and K >= 16384 else 0
 
 
 def linear(x: torch.Tensor, W: torch.Tensor, *, W2: Optional[torch.Tensor] = None,

@@ -397,14 +397,13 @@ def test_bounded_wait_expiry_of_the_fp32_gemm(shape):
 
 @pytest.mark.parametrize("shape", [(333, 1536, 6144), (5193, 1000, 4096)])   # parts alone; whole tiles of several accumulators ahead of them
 def test_bounded_wait_expiry_of_a_linear_in_parts(shape):
-    from flash_stu_2_b200 import _lib, ops
+    from flash_stu_2_b200 import ops
     M, N, K = shape
-    assert _lib.load().stu_linear_workspace_elems(M, N, K, 0, 1) > 0
     g = torch.Generator(device=dev()).manual_seed(26)
     x, W = torch.randn(M, K, device=dev(), generator=g).bfloat16(), torch.randn(N, K, device=dev(), generator=g).bfloat16()
-    want = ops.linear(x, W)
-    _gives_up(lambda: ops.linear(x, W), 3)
-    assert torch.equal(ops.linear(x, W), want)
+    want = _linear_in_parts(x, W)
+    _gives_up(lambda: _linear_in_parts(x, W), 3)
+    assert torch.equal(_linear_in_parts(x, W), want)
     ops.check_status()
 
 
@@ -681,27 +680,54 @@ def test_linear_of_long_weights_in_parts(shape, epi):
         assert rc == rc2 == 0 and torch.equal(short, whole) and bool(work.isnan().all())
 
 
+def _linear_in_parts(x, W, r=None):
+    """stu_linear_split with the workspace that it wants: the op asks for one from 16384 of K on alone."""
+    from flash_stu_2_b200 import _lib, ops
+    (M, K), N = x.shape, W.shape[0]
+    elems = _lib.load().stu_linear_workspace_elems(M, N, K, int(r is not None), 1)
+    assert elems > 0
+    work, y = torch.empty(elems, device=dev()), torch.empty(M, N, device=dev(), dtype=torch.bfloat16)
+    ops.status_word(x.device)
+    rc = _lib.load().stu_linear_split(x.data_ptr(), K, W.data_ptr(), K, 1, None, r.data_ptr() if r is not None else None, N, y.data_ptr(), N, M, N, K,
+                                      int(r is not None), 0, 0, 0, None, 0.0, 1, 0, work.data_ptr(), elems, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and _lib.load().stu_linear_launches() == 2
+    return y
+
+
 @pytest.mark.parametrize("shape", [(5193, 1000, 4096), (19851, 512, 3072), (16384, 1536, 6144), (5193, 1001, 4104), (2100, 200, 24576)])
 @pytest.mark.parametrize("epi", [0, 1])
 def test_equal_rows_of_a_linear_in_parts_are_equal(shape, epi):
     """Tiles of which K is cut and, ahead of them, whole ones: an output is the same sum in either, so sequences of a batch do not differ by where they stand."""
-    from flash_stu_2_b200 import _lib, ops
     M, N, K = shape
     if epi:
         N = N // 8 * 8
-    assert _lib.load().stu_linear_workspace_elems(M, N, K, epi, 1) > 0
+    from flash_stu_2_b200 import ops
     torch.manual_seed(11)
     three = torch.randn(3, K, device=dev()).bfloat16()
     x, W = three.repeat(-(-M // 3), 1)[:M], (torch.randn(N, K, device=dev()) / math.sqrt(K)).bfloat16()
     r = torch.randn(3, N, device=dev()).bfloat16().repeat(-(-M // 3), 1)[:M] if epi else None
-    y = ops.linear(x, W, resid=r, epilogue=epi)
+    y = _linear_in_parts(x, W, r)
     ops.check_status()
     assert torch.equal(y, y[:3].repeat(-(-M // 3), 1)[:M])
     full = three.double() @ W.double().t() + (r[:3].double() if epi else 0.0)
     assert float((y[:3].double() - full).abs().max()) <= 2.0 ** -7 * max(1.0, float(full.abs().max()))
 
 
-@pytest.mark.parametrize("shape,launches", [((333, 1536, 6144), 2), ((65, 64, 24576), 2), ((333, 1536, 512), 1), ((64, 64, 24576), 1)])
+@pytest.mark.parametrize("shape", [(333, 1536, 6144), (28924, 512, 2048), (16384, 1536, 6144), (900, 3072, 12288)])
+def test_a_models_products_have_one_chain_whatever_the_batch(shape):
+    """The rows of a prefill in one call and in calls of other sizes, through the tiles' forms and edges: the same results (an MLP's K)."""
+    from flash_stu_2_b200 import _lib, ops
+    M, N, K = shape
+    assert _lib.load().stu_linear_workspace_elems(M, N, K, 1, 1) > 0   # (a cut would pay)
+    torch.manual_seed(13)
+    x, W, r = torch.randn(M, K, device=dev()).bfloat16(), (torch.randn(N, K, device=dev()) / math.sqrt(K)).bfloat16(), torch.randn(M, N, device=dev()).bfloat16()
+    whole = ops.linear(x, W, resid=r, epilogue=1)
+    for n in (72, M // 3, M - 72):   # (more rows than a token step's)
+        assert torch.equal(ops.linear(x[:n], W, resid=r[:n], epilogue=1), whole[:n])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("shape,launches", [((333, 1536, 24576), 2), ((65, 64, 24576), 2), ((333, 1536, 512), 1), ((64, 64, 24576), 1)])
 def test_launches_of_a_linear_are_counted(shape, launches):
     """A product whose K is cut is added up in a launch of its own; on the CUDA cores (asked for, or rows that the tensor cores do not take) it is one launch."""
     from flash_stu_2_b200 import _lib, ops
@@ -715,7 +741,7 @@ def test_launches_of_a_linear_are_counted(shape, launches):
         assert ops.launch_count - before == want
 
 
-@pytest.mark.parametrize("shape", [(128, 1024, 4096), (333, 1536, 6144), (65, 64, 24576)])
+@pytest.mark.parametrize("shape", [(128, 1024, 16384), (333, 1536, 24576), (65, 64, 24576)])
 @pytest.mark.parametrize("given", [False, True])
 def test_a_linear_in_parts_takes_its_workspace_from_the_arena(shape, given):
     """The buffer that a caller gives for a captured step holds the parts of K as well, for one product at a time; the sums are those of a call outside."""

@@ -504,7 +504,7 @@ def test_launches_of_a_layers_prefill_are_counted(monkeypatch):
     """In one native call as many launches are counted as in calls apart, also where the down projection takes two."""
     import flash_stu_2_b200 as F
     from flash_stu_2_b200 import _lib, ops
-    cfg = F.FlashSTUConfig(n_embd=64, n_layers=1, n_heads=1, seq_len=128, vocab_size=1, mlp_scale=64, num_eigh=8, torch_dtype=torch.bfloat16, use_attn=False)
+    cfg = F.FlashSTUConfig(n_embd=64, n_layers=1, n_heads=1, seq_len=128, vocab_size=1, mlp_scale=256, num_eigh=8, torch_dtype=torch.bfloat16, use_attn=False)
     blk = F.FlashSTUBlock(config=cfg).cuda().eval()
     with torch.no_grad():
         blk(torch.zeros(1, 8, 64, device="cuda", dtype=torch.bfloat16))   # (the taps are laid out)
@@ -518,5 +518,5 @@ def test_launches_of_a_layers_prefill_are_counted(monkeypatch):
                 blk(torch.zeros(1, T, 64, device="cuda", dtype=torch.bfloat16))
             counts.append(ops.launch_count - before)
     ops.check_status()
-    assert _lib.load().stu_linear_workspace_elems(80, 64, 4096, 1, 1) > 0
+    assert _lib.load().stu_linear_workspace_elems(80, 64, 16384, 1, 1) > 0
     assert counts[:2] == counts[2:] and counts[0] == counts[1] + 1

@@ -366,12 +366,12 @@ def test_the_three_forms_of_the_token_loop_agree(monkeypatch, dt, kw):
 
 @pytest.mark.parametrize("approx", [True, False])
 def test_a_captured_step_of_many_sequences_keeps_its_parts_in_its_buffer(monkeypatch, approx):
-    """80 sequences and long products (the down projection; without approx the contraction of all filters): K is cut, the parts' place is
+    """80 sequences and long products (the down projection of a wide MLP): K is cut, the parts' place is
     in the step's buffer, and the logits are those of the eager loop.  (What capturing does allocate is an attention's output and two words.)"""
     import flash_stu_2_b200 as F
     from flash_stu_2_b200 import _lib, ops
     torch.manual_seed(3)
-    cfg = F.FlashSTUConfig(n_embd=256, n_layers=2, n_heads=4, seq_len=64, window_size=40, vocab_size=1003, mlp_scale=16, num_eigh=8,
+    cfg = F.FlashSTUConfig(n_embd=256, n_layers=2, n_heads=4, seq_len=64, window_size=40, vocab_size=1003, mlp_scale=64, num_eigh=8,
                            torch_dtype=torch.bfloat16, use_approx=approx)
     with torch.device(dev()):
         m = F.FlashSTU(cfg).eval()
@@ -379,7 +379,7 @@ def test_a_captured_step_of_many_sequences_keeps_its_parts_in_its_buffer(monkeyp
         for name, p in m.named_parameters():
             if not name.endswith("norm.weight"):
                 p.normal_(0.0, 0.5 * p.shape[-1] ** -0.5)
-    parts = _lib.load().stu_linear_workspace_elems(80, 256, 4096, 1, 1)
+    parts = _lib.load().stu_linear_workspace_elems(80, 256, 16384, 1, 1)
     assert parts > 0
     allocated = []
 
