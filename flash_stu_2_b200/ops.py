@@ -143,7 +143,7 @@ class arena:
 
 
 def empty(shape, dtype: torch.dtype, device) -> torch.Tensor:
-    a = getattr(_local, "arena", None)
+    a = getattr(_local, "arena", None) if _arenas else None
     if a is not None:
         t = a.take(shape, dtype)
         if t is not None:
@@ -152,7 +152,7 @@ def empty(shape, dtype: torch.dtype, device) -> torch.Tensor:
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = RMS_EPS, out: Optional[torch.Tensor] = None):
-    if out is None and getattr(_local, "arena", None) is None:
+    if out is None and (not _arenas or getattr(_local, "arena", None) is None):
         y = _lib.native().rmsnorm(x, weight, eps)
         if y is not None:
             _count()
@@ -387,7 +387,7 @@ def layer_step_f32(x, norm_w, MinT, hist, taps, pos, mid, mlp_norm_w, gate, up, 
     """One cached token of an approx layer in fp32, up to 8 sequences: decode_approx into `mid`, then the MLP from there into x, issued in
     one native call (the interpreter takes as long for the three calls apart as the kernels do).  3: done; 1: the MLP is left to the
     caller; 0: nothing was launched."""
-    if getattr(_local, "arena", None) is not None:
+    if _arenas and getattr(_local, "arena", None) is not None:
         return 0
     ov = FLAG_OVERLAP if overlap_decode else 0
     early = FLAG_EARLY_TRIGGER if overlap_decode else 0
@@ -405,7 +405,7 @@ def layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, 
     """New positions of an approx layer, in place on x [B,T,d], seven launches in one native call; the positions move on in the last kernel
     of the convolution (fresh: they need not have been written before).  kind 2 (taps: the reversed table): tcgen05, 1: mma.sync,
     0: CUDA cores.  3: done; 1: the MLP is left to the caller; 0: all of it is."""
-    if getattr(_local, "arena", None) is not None:
+    if _arenas and getattr(_local, "arena", None) is not None:
         return 0
     done = _lib.native().layer_prefill(x, norm_w, MinT, hist, taps, pos, mlp_norm_w, gate, up, down, eps, mlp_eps, t0, int(fresh), kind,
                                        status_word(x.device))
